@@ -6,7 +6,7 @@
 #include <mutex>
 #include <utility>
 
-#include "common.cuh"
+#include "tc5.cuh"
 
 __device__ int g_cn_status = 0;
 
@@ -40,6 +40,28 @@ cudaError_t cn_allow_smem(const void* kernel, int bytes) {
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) cn_smem_book(kernel, dev, bytes, 1);
     return e;
+}
+
+int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
+               unsigned box_cols, unsigned box_rows) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode encode = nullptr;
+    if (!encode) {  // the driver's entry point, looked up once (two threads may both look: the same answer)
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        CN_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
+        if (!fn) CN_FAIL(CN_ERR_CUDA, "cuTensorMapEncodeTiled is not in this driver");
+        encode = (Encode)fn;
+    }
+    const CUtensorMapDataType type = elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : elem == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {row_bytes};
+    const cuuint32_t box[2] = {box_cols, box_rows}, es[2] = {1, 1};
+    const CUresult r = encode(map, type, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              elem == 4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) CN_FAIL(CN_ERR_CUDA, "tensor map of [%llu x %llu]: driver error %d", rows, cols, (int)r);
+    return CN_OK;
 }
 
 extern "C" const char* cn_last_error_string(void) { return t_err; }

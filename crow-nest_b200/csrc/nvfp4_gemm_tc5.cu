@@ -26,6 +26,7 @@
 // Every wait is bounded; tensor memory (TN columns) is allocated by warp 12 and freed by it after the CTA has
 // met again, whatever happened in between.
 #include "common.cuh"
+#include "nvfp4_gemm.cuh"
 
 namespace {
 
@@ -368,11 +369,21 @@ extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void
         CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_gemm: workspace of %zu B, %zu B needed", workspace_bytes, cn_nvfp4_gemm_workspace_bytes(k, m));
     uint16_t* xh = (uint16_t*)workspace;
     float* rs = (float*)((char*)workspace + (((size_t)m * k * 2 + 255) & ~(size_t)255));
-    if (dtype == CN_BF16)
-        gemm_prep_x_kernel<1><<<m, 256, 0, stream>>>(x, xh, rs, k);
-    else
-        gemm_prep_x_kernel<0><<<m, 256, 0, stream>>>(x, xh, rs, k);
-    CN_CUDA(cudaGetLastError());
+    // more than 128 rows of bf16 go to the tensor cores as they are; everything else as f16 x 2^k per row
+    const bool pair = m > 128;
+    if (!pair || dtype != CN_BF16) {
+        if (dtype == CN_BF16)
+            gemm_prep_x_kernel<1><<<m, 256, 0, stream>>>(x, xh, rs, k);
+        else
+            gemm_prep_x_kernel<0><<<m, 256, 0, stream>>>(x, xh, rs, k);
+        CN_CUDA(cudaGetLastError());
+    }
+    if (pair) {
+        GemmCall c = {};
+        c.w = w, c.gs = gs, c.x_f16 = dtype != CN_BF16, c.x = c.x_f16 ? (const void*)xh : x, c.rs = rs, c.y = y;
+        c.rows = rows, c.k = k, c.m = m, c.ldy = ldy;
+        return cn_gemm_pair_launch(c, stream);
+    }
     CN_ALLOW_SMEM(nvfp4_gemm_tc5_kernel<128>, (int)smem_of(128));
     CN_ALLOW_SMEM(nvfp4_gemm_tc5_kernel<256>, (int)smem_of(256));
     GemmParams p;

@@ -1,0 +1,30 @@
+"""The CTA-pair GEMM (more than 128 rows) at the edges of its tiles: row counts around 256-row tiles (odd ones take the
+one-row stores), token counts around the tile widths it chooses (one and two accumulators, 4 to 8 weight slots), k = 256,
+every scale byte in the bf16 decode (subnormal scales ride as subnormal bf16)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import oracle
+from crownest_b200 import device_status, ops, synth
+from test_gpu_nvfp4_gemv import check_close, from_dev_bf16, to_dev_bf16
+
+
+@pytest.mark.parametrize("rows,k,m", [(256, 256, 129), (333, 256, 160), (255, 512, 193), (258, 768, 449), (1030, 1280, 225), (2, 2048, 513)])
+def test_pair_gemm_matches_the_cpu_reference(rows, k, m):
+    rng = np.random.default_rng(rows + m)
+    w = synth.nvfp4_matrix(rows, k, rng).copy()
+    if k == 256:  # every scale byte, bit 7 and 0x7F included
+        w.reshape(-1, 36)[:, :4] = np.arange(rows * (k // 64) * 4, dtype=np.uint32).astype(np.uint8).reshape(-1, 4)
+    xb, xf = synth.activations(m, k, rng)
+    fw = ops.Fp4.from_host(w, rows, k, np.float32(0.37))
+    ref = np.concatenate([oracle.nvfp4_gemv(w, rows, k, np.float32(0.37), xf[t:t + 8], threads=8, path=1) for t in range(0, m, 8)])
+    # bf16 rows as they are; the ulp no lower than rms / 64 (f32 accumulation error of either side, as for the other GEMMs)
+    check_close(from_dev_bf16(ops.launch_gemm(fw, to_dev_bf16(xb))), ref, f"pair gemm {rows}x{k} m={m}", ulp_floor=1.0 / 64)
+    # f32 rows ride as f16 (exact for these bf16 values): the f32 accumulator itself
+    yf = ops.launch_gemm(fw, torch.from_numpy(xf).cuda()).cpu().numpy()
+    scale = np.sqrt(np.mean(ref.astype(np.float64) ** 2, axis=1, keepdims=True))
+    assert np.max(np.abs(yf - ref) / scale) <= 1e-4
+    assert device_status() == 0
