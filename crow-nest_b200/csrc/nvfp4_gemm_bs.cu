@@ -20,7 +20,7 @@
 // one lane of warp 5 copies the scale chunks to tensor memory (tcgen05.cp) and issues the MMAs, warps 0-3 read the
 // accumulator (tcgen05.ld), add the five levels of every token and store. When the row tiles alone cannot fill the GPU the
 // column range is split over blockIdx.z and a second kernel adds the partial sums in split order.
-#include "common.cuh"
+#include "tc5.cuh"
 
 namespace {
 
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) nvfp4_gemm_bs_kernel(const BsPa
     volatile int* failed = (volatile int*)(tmem_slot + 1);
     const uint32_t ring_addr = (smem_u32(smem_raw) + 2048u + 1023u) & ~1023u;
     uint8_t* ring = smem_raw + (ring_addr - smem_u32(smem_raw));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
     const int kts = p.k / KT;
     const int rt = blockIdx.x, tb0 = blockIdx.y * NB;
     const int ntb = (p.m + TB - 1) / TB;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(BS_THREADS, 1) nvfp4_gemm_bs_kernel(const BsPa
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot);
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer: one bulk copy per operand and stage
@@ -340,44 +340,51 @@ __global__ void __launch_bounds__(BS_THREADS, 1) nvfp4_gemm_bs_kernel(const BsPa
             }
         }
     } else if (warp == 5) {
-        // ------------------------------------------------------------ scale copies and MMAs, one lane
-        if (lane == 0) {
-            bool ok = true;
-            for (int i = 0; i < nst && ok; i++) {
-                const int s = i % STAGES;
-                if (!mbar_wait(&full[s], (i / STAGES) & 1)) {
-                    cn_dev_fail(CN_DEV_WAIT_FULL);
-                    *failed = 1;
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a_addr = ring_addr + (uint32_t)s * STAGE;
+        // ------------------------------------------------------------ scale copies and MMAs, issued by an elected lane of the
+        // converged warp (see elect_lane)
+        const uint32_t ring_u = warp_uniform(ring_addr);
+        const uint64_t sw0 = desc_sw128(ring_u), sf0 = desc_sf(ring_u);
+        const bool two = NB == 2 && tb0 + 1 < ntb;
+        bool ok = true;
+        int s = 0;
+        uint32_t par = 0;
+        for (int i = 0; i < nst; i++) {
+            if (!mbar_wait(&full[s], par)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                *failed = 1;
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint64_t a_sw = sw0 + (uint32_t)(s * (STAGE >> 4)), a_sf = sf0 + (uint32_t)(s * (STAGE >> 4));
+            if (elect_lane()) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    cp_sf(tmem + SFA_COL + 4 * j, desc_sf(a_addr + A_IMG + 512 * j));
+                    cp_sf(tmem + SFA_COL + 4 * j, a_sf + ((A_IMG + 512 * j) >> 4));
 #pragma unroll
                     for (int nb = 0; nb < NB; nb++) {
-                        if (tb0 + nb >= ntb) continue;
-                        const uint32_t b_addr = a_addr + A_STAGE + nb * B_STAGE;
-                        cp_sf(tmem + SFB_COL + nb * 32 + 8 * j, desc_sf(b_addr + B_IMG + (2 * j) * 512));
-                        cp_sf(tmem + SFB_COL + nb * 32 + 8 * j + 4, desc_sf(b_addr + B_IMG + (2 * j + 1) * 512));
+                        if (nb == 1 && !two) continue;
+                        const uint64_t b_sf = a_sf + ((A_STAGE + nb * B_STAGE + B_IMG) >> 4);
+                        cp_sf(tmem + SFB_COL + nb * 32 + 8 * j, b_sf + ((2 * j) * 512 >> 4));
+                        cp_sf(tmem + SFB_COL + nb * 32 + 8 * j + 4, b_sf + ((2 * j + 1) * 512 >> 4));
                     }
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
 #pragma unroll
                     for (int nb = 0; nb < NB; nb++) {
-                        if (tb0 + nb >= ntb) continue;
-                        const uint32_t b_addr = a_addr + A_STAGE + nb * B_STAGE;
-                        umma_bs(tmem + nb * NCOL, desc_sw128(a_addr + 32u * j), desc_sw128(b_addr + 32u * j), IDESC, tmem + SFA_COL + 4 * j,
+                        if (nb == 1 && !two) continue;
+                        umma_bs(tmem + nb * NCOL, a_sw + 2 * j, a_sw + ((A_STAGE + nb * B_STAGE) >> 4) + 2 * j, IDESC, tmem + SFA_COL + 4 * j,
                                 tmem + SFB_COL + nb * 32 + 8 * j, (i > 0 || j > 0) ? 1u : 0u);
                     }
                 }
                 umma_commit(&empty[s]);
             }
-            if (ok) umma_commit(accbar);
+            __syncwarp();
+            if (++s == STAGES) s = 0, par ^= 1u;
         }
+        if (ok && elect_lane()) umma_commit(accbar);
+        __syncwarp();
     } else {
         // ------------------------------------------------------------ epilogue: lane = weight row, the five levels of a token added
         bool ok = true;
