@@ -39,6 +39,15 @@ struct Mul1Spec {
     long long tr_off, suh_off, svh_off;  // byte offsets into the record
 };
 
+// What differs between the matrices of one launch (gate and up read the same rows): the staged activations of the matrix, its
+// partial sums, and where its trellis and input scales lie in a record.
+struct Mul1Side {
+    uint16_t* xh;
+    float* xinv;
+    float* part;
+    long long tr_off, suh_off;
+};
+
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 
 // natural-order FWHT of 128 values over one warp, element 4*lane + j in v[j]; stages (a+b, a-b)
@@ -81,17 +90,19 @@ __device__ __forceinline__ void store_hi_lo(uint16_t* xh, size_t plane, size_t a
 }
 
 // xh16[slot][t][k] = the hi / lo planes of H128(x * suh) * mul, xinv[slot][t][k/128] = 1/mul.
-// grid (k/128, 1, slots), block 32 T (warp t = activation row t). XT: 0 f32, 1 bf16 input. x row of slot: x + (slot / x_div) * T * k.
+// grid (k/128, matrices, slots), block 32 T (warp t = activation row t). XT: 0 f32, 1 bf16 input. x row of slot: x + (slot / x_div) * T * k.
 // rowsrc (optional): the x row of (slot, t) as an index into x [rows][k], negative = an unused row slot (stored as zeros)
 template <int XT>
-__global__ void mul1_had_in_kernel(const unsigned long long* __restrict__ ptrs, const void* __restrict__ x, uint16_t* __restrict__ xh,
-                                   float* __restrict__ xinv, int k, int T, long long suh_off, int x_div, size_t plane,
-                                   const int* __restrict__ rowsrc) {
+__global__ void mul1_had_in_kernel(const unsigned long long* __restrict__ ptrs, const void* __restrict__ x, Mul1Side sa, Mul1Side sb, int k, int T,
+                                   int x_div, size_t plane, const int* __restrict__ rowsrc) {
     pdl_launch_dependents();
     pdl_wait();  // everything below may read what earlier kernels of the stream wrote
     const int slot = blockIdx.z, t = threadIdx.x >> 5, blk = blockIdx.x, lane = threadIdx.x & 31;  // one warp per activation row
     if (ptrs[slot] == 0ull) return;  // a null record: nothing to read or write
-    const uint16_t* suh = (const uint16_t*)(ptrs[slot] + (unsigned long long)suh_off);
+    const Mul1Side& sd = blockIdx.y ? sb : sa;
+    uint16_t* xh = sd.xh;
+    float* xinv = sd.xinv;
+    const uint16_t* suh = (const uint16_t*)(ptrs[slot] + (unsigned long long)sd.suh_off);
     const int src = rowsrc ? rowsrc[slot * T + t] : 0;
     const size_t xrow = rowsrc ? (size_t)(src < 0 ? 0 : src) * k : ((size_t)(slot / x_div) * T + t) * k, row = ((size_t)slot * T + t) * k;
     const int c0 = blk * 128 + 4 * lane;
@@ -148,13 +159,12 @@ __device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const
     }
 }
 
-// y' partials of one k-split. grid (n/128, S, slots), block 288 = 8 decode warps + 1 copy warp.
+// y' partials of one k-split. grid (matrices n/128, S, slots), block 288 = 8 decode warps + 1 copy warp.
 // part[slot][sp][t][n]; xh16 [slot][T][k] f16, xinv [slot][T][k/128].
 // MT: activation rows the register allocation is built for (1, 2, 4 or 8; T <= MT of them live)
 template <bool K3, int MT>
-__global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long long* __restrict__ ptrs, const uint16_t* __restrict__ xh,
-                                                        const float* __restrict__ xinv, float* __restrict__ part, Mul1Spec sp_, int S, int T,
-                                                        size_t plane, int SPC) {
+__global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, Mul1Spec sp_,
+                                                        int S, int T, size_t plane, int SPC) {
     pdl_launch_dependents();
     pdl_wait();  // everything below may read what earlier kernels of the stream wrote
     // SPC consecutive k-splits per CTA (blockIdx.y walks groups of SPC): the splits keep their own partial sums, so
@@ -166,7 +176,12 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
     const int k = sp_.k, n = sp_.n, n32 = sp_.n32;
     const int tiles_n = n >> 4, tps = (k >> 4) / S, kb0 = sp0 * tps, rows = SPC * tps * 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb0 = blockIdx.x * 8;
+    const bool second = (int)blockIdx.x >= (n >> 7);  // the CTAs of the second matrix follow those of the first
+    const Mul1Side& sd = second ? side_b : side_a;
+    const uint16_t* __restrict__ xh = sd.xh;
+    const float* __restrict__ xinv = sd.xinv;
+    float* __restrict__ part = sd.part;
+    const int nb0 = ((int)blockIdx.x - (second ? n >> 7 : 0)) * 8;
     const int run_bytes = 32 * n32;  // 8 tiles of one tile row
     uint64_t* full = (uint64_t*)smem;
     uint64_t* empty = full + RING;
@@ -187,7 +202,7 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
     const int nst1 = (tps + UROWS - 1) / UROWS;  // stages of one split
     const int nst = SPC * nst1;
     if (warp == 8) {
-        const uint8_t* base = (const uint8_t*)(rec + (unsigned long long)sp_.tr_off);
+        const uint8_t* base = (const uint8_t*)(rec + (unsigned long long)sd.tr_off);
         if (((uintptr_t)base & 15) != 0) {
             cn_dev_fail(103);  // a trellis that is not 16-byte aligned cannot be bulk-copied
             return;
@@ -333,12 +348,21 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
 __device__ __forceinline__ void out_block(float v[4], const float* __restrict__ part, const uint16_t* __restrict__ svh, int slot, int S, int T,
                                           int t, int n, int blk, int lane) {
     const int c0 = blk * 128 + 4 * lane;
+    // the splits are added one after the other, but eight 16-byte loads are in flight at a time (one trip to L2 for each split
+    // of each value made this the longest step of a one-token FFN after the GEMVs: 13 us of 64 with sixteen splits twice)
+    const float4* src = (const float4*)(part + ((size_t)slot * S * T + t) * n + c0);
+    const size_t step = (size_t)T * n / 4;
+    float4 a = src[0];
+    for (int q0 = 1; q0 < S; q0 += 8) {
+        float4 r[8];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        float s = part[(((size_t)slot * S + 0) * T + t) * n + c0 + j];
-        for (int q = 1; q < S; q++) s = __fadd_rn(s, part[(((size_t)slot * S + q) * T + t) * n + c0 + j]);
-        v[j] = s;
+        for (int i = 0; i < 8; i++)
+            if (q0 + i < S) r[i] = src[(size_t)(q0 + i) * step];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (q0 + i < S) a.x = __fadd_rn(a.x, r[i].x), a.y = __fadd_rn(a.y, r[i].y), a.z = __fadd_rn(a.z, r[i].z), a.w = __fadd_rn(a.w, r[i].w);
     }
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
     fwht128(v, lane);
 #pragma unroll
     for (int j = 0; j < 4; j++) v[j] = __fmul_rn(__fmul_rn(v[j], 0.0078125f), h2f(svh[c0 + j]));
@@ -442,9 +466,6 @@ struct Mul1Plan {
     int* rowdst;               // [slots * MUL1_GT] combo (output row) of every (group slot, row), -1 = unused
     int grp_rows;              // rows the scratch holds per slot: max(max_t, 4)
     float* eo;                 // [slots][T][hidden] expert outputs (MoE form)
-    // the up projection does not depend on the gate projection: it runs on a side stream between two events
-    cudaStream_t side;
-    cudaEvent_t fork, join;
 };
 
 int ksplit(int k) {
@@ -467,21 +488,23 @@ Mul1Spec spec_of(const Mul1Plan* p, int which) {
     return s;
 }
 
-int launch_had_in(const unsigned long long* ptrs, const void* x, uint16_t* xh, float* xinv, const Mul1Spec& s, int slots, int T, int x_div,
-                  int dtype, size_t plane, cudaStream_t st, const int* rowsrc = nullptr) {
-    dim3 grid(s.k / 128, 1, slots);
+// sb: the second matrix of the launch (up beside gate), or null
+int launch_had_in(const unsigned long long* ptrs, const void* x, const Mul1Side& sa, const Mul1Side* sb, int k, int slots, int T, int x_div, int dtype,
+                  size_t plane, cudaStream_t st, const int* rowsrc = nullptr) {
+    dim3 grid(k / 128, sb ? 2 : 1, slots);
     if (dtype == CN_BF16)
-        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<1>), dim3(grid), dim3(32 * T), 0, st, ptrs, x, xh, xinv, s.k, T, s.suh_off, x_div, plane, rowsrc));
+        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<1>), grid, dim3(32 * T), 0, st, ptrs, x, sa, sb ? *sb : sa, k, T, x_div, plane, rowsrc));
     else
-        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<0>), dim3(grid), dim3(32 * T), 0, st, ptrs, x, xh, xinv, s.k, T, s.suh_off, x_div, plane, rowsrc));
+        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<0>), grid, dim3(32 * T), 0, st, ptrs, x, sa, sb ? *sb : sa, k, T, x_div, plane, rowsrc));
     CN_CUDA(cudaGetLastError());
     return CN_OK;
 }
 
 // live: how many of the slots are expected to hold a record (the grouped MoE form launches more slots than it fills)
-int launch_gemv(const unsigned long long* ptrs, const uint16_t* xh, const float* xinv, float* part, const Mul1Spec& s, int slots, int T,
-                size_t plane, cudaStream_t st, int live = 0) {
+int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Side* sb, const Mul1Spec& s, int slots, int T, size_t plane,
+                cudaStream_t st, int live = 0) {
     if (live < 1 || live > slots) live = slots;
+    const int mats = sb ? 2 : 1;
     const int S = ksplit(s.k), tps = (s.k / 16) / S;
     if (tps % 8 != 0) CN_FAIL(CN_ERR_SHAPE, "mul1 gemv: k = %d does not split into whole 128-row blocks", s.k);  // the kernel's stage / block counters rely on it
     // k-splits per CTA: as many as still leave about four CTAs per SM (the splits keep separate partial sums, so
@@ -489,7 +512,7 @@ int launch_gemv(const unsigned long long* ptrs, const uint16_t* xh, const float*
     int spc = 1;
     for (int c = S; c > 1; c--) {
         if (S % c) continue;
-        const long long ctas = (long long)(s.n / 128) * (S / c) * live;
+        const long long ctas = (long long)mats * (s.n / 128) * (S / c) * live;
         const size_t need = 128 + (size_t)RING * UROWS * 32 * s.n32 + (size_t)2 * T * (c * tps * 16 + XPAD) * 2 + 8 + (size_t)T * (c * tps / 8) * 4;
         if (ctas >= 592 && need <= 160 * 1024) {
             spc = c;
@@ -498,14 +521,14 @@ int launch_gemv(const unsigned long long* ptrs, const uint16_t* xh, const float*
     }
     const int rows = spc * tps * 16;
     const size_t smem = 128 + (size_t)RING * UROWS * 32 * s.n32 + (size_t)2 * T * (rows + XPAD) * 2 + 8 + (size_t)T * (rows / 128) * 4;
-    dim3 grid(s.n / 128, S / spc, slots);
+    dim3 grid(mats * (s.n / 128), S / spc, slots);
     if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "mul1 gemv: %zu B of shared memory per block", smem);
     const bool k3 = s.bits == 3 && !s.half;
     const int mt = T == 1 ? 1 : (T == 2 ? 2 : (T <= 4 ? 4 : 8));
 #define CN_MUL1_CASE(K3V, MTV)                                                                                                      \
     if (k3 == K3V && mt == MTV) {                                                                                                   \
         CN_ALLOW_SMEM((mul1_gemv_kernel<K3V, MTV>), 160 * 1024);                                                                    \
-        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K3V, MTV>), grid, dim3(288), smem, st, ptrs, xh, xinv, part, s, S, T, plane, spc));        \
+        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K3V, MTV>), grid, dim3(288), smem, st, ptrs, sa, sb ? *sb : sa, s, S, T, plane, spc));             \
     }
     CN_MUL1_CASE(true, 1) CN_MUL1_CASE(true, 2) CN_MUL1_CASE(true, 4) CN_MUL1_CASE(true, 8)
     CN_MUL1_CASE(false, 1) CN_MUL1_CASE(false, 2) CN_MUL1_CASE(false, 4) CN_MUL1_CASE(false, 8)
@@ -583,9 +606,6 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
     step(cudaMalloc(&p->rowsrc, (size_t)max_slots * MUL1_GT * 4));
     step(cudaMalloc(&p->rowdst, (size_t)max_slots * MUL1_GT * 4));
     step(cudaMalloc(&p->eo, rows * hidden * 4));
-    step(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
-    step(cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming));
-    step(cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming));
     if (e != cudaSuccess) {
         cn_mul1_plan_destroy(p);
         CN_FAIL(CN_ERR_CUDA, "cn_mul1_plan_create: %s", cudaGetErrorString(e));
@@ -599,9 +619,6 @@ extern "C" int cn_mul1_plan_destroy(void* plan) {
     if (!p) return CN_OK;
     cudaFree(p->xh_a), cudaFree(p->xh_b), cudaFree(p->xinv_a), cudaFree(p->xinv_b), cudaFree(p->part_a), cudaFree(p->part_b), cudaFree(p->ptrs),
         cudaFree(p->eo), cudaFree(p->order), cudaFree(p->groups), cudaFree(p->rowsrc), cudaFree(p->rowdst);
-    if (p->side) cudaStreamDestroy(p->side);
-    if (p->fork) cudaEventDestroy(p->fork);
-    if (p->join) cudaEventDestroy(p->join);
     delete p;
     return CN_OK;
 }
@@ -614,8 +631,9 @@ extern "C" int cn_mul1_gemv(void* plan, int which, const unsigned long long* ptr
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_mul1_gemv: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     cudaStream_t st = (cudaStream_t)stream;
     const Mul1Spec s = spec_of(p, which);
-    if (int rc = launch_had_in(ptrs, x, p->xh_a, p->xinv_a, s, slots, t, x_div, dtype, p->plane, st)) return rc;
-    if (int rc = launch_gemv(ptrs, p->xh_a, p->xinv_a, p->part_a, s, slots, t, p->plane, st)) return rc;
+    const Mul1Side side = {p->xh_a, p->xinv_a, p->part_a, s.tr_off, s.suh_off};
+    if (int rc = launch_had_in(ptrs, x, side, nullptr, s.k, slots, t, x_div, dtype, p->plane, st)) return rc;
+    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, p->plane, st)) return rc;
     dim3 grid(s.n / 128, 1, slots);
     if (dtype == CN_BF16)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, s.n, ksplit(s.k), t, s.svh_off, (const int*)nullptr));
@@ -629,20 +647,16 @@ extern "C" int cn_mul1_gemv(void* plan, int which, const unsigned long long* ptr
 static int mul1_ffn(Mul1Plan* p, const unsigned long long* ptrs, const void* x, void* y, int slots, int t, int x_div, float limit, int dtype,
                     int out_f32, cudaStream_t st, const int* rowsrc = nullptr, const int* rowdst = nullptr, int live = 0) {
     const Mul1Spec g = spec_of(p, 0), u = spec_of(p, 1), d = spec_of(p, 2);
-    // up branch on the side stream; it is joined again on every path, so a capture of `st` stays valid
-    CN_CUDA(cudaEventRecord(p->fork, st));
-    CN_CUDA(cudaStreamWaitEvent(p->side, p->fork, 0));
-    int rc = launch_had_in(ptrs, x, p->xh_b, p->xinv_b, u, slots, t, x_div, dtype, p->plane, p->side, rowsrc);
-    if (rc == CN_OK) rc = launch_gemv(ptrs, p->xh_b, p->xinv_b, p->part_b, u, slots, t, p->plane, p->side, live);
-    CN_CUDA(cudaEventRecord(p->join, p->side));
-    if (rc == CN_OK) rc = launch_had_in(ptrs, x, p->xh_a, p->xinv_a, g, slots, t, x_div, dtype, p->plane, st, rowsrc);
-    if (rc == CN_OK) rc = launch_gemv(ptrs, p->xh_a, p->xinv_a, p->part_a, g, slots, t, p->plane, st, live);
-    CN_CUDA(cudaStreamWaitEvent(st, p->join, 0));
-    if (rc != CN_OK) return rc;
+    // gate and up share each launch: two small grids on two streams cost an event fork and join and ran one after the other
+    // anyway (one token, four experts of 4096 x 1536: 65 -> 55 us with out_block's wide loads; 16 tokens: 298 -> 289)
+    const Mul1Side ga = {p->xh_a, p->xinv_a, p->part_a, g.tr_off, g.suh_off}, up = {p->xh_b, p->xinv_b, p->part_b, u.tr_off, u.suh_off};
+    const Mul1Side dn = {p->xh_a, p->xinv_a, p->part_a, d.tr_off, d.suh_off};
+    if (int rc = launch_had_in(ptrs, x, ga, &up, g.k, slots, t, x_div, dtype, p->plane, st, rowsrc)) return rc;
+    if (int rc = launch_gemv(ptrs, ga, &up, g, slots, t, p->plane, st, live)) return rc;
     CN_CUDA(cn_launch_pdl(mul1_act_had_in_kernel, dim3(p->inter / 128, 1, slots), dim3(32 * t), 0, st, ptrs, p->part_a, p->part_b, p->xh_a, p->xinv_a, p->inter, ksplit(p->hidden), t,
                                                                          g.svh_off, u.svh_off, d.suh_off, limit, p->plane));
     CN_CUDA(cudaGetLastError());
-    if (int rc = launch_gemv(ptrs, p->xh_a, p->xinv_a, p->part_a, d, slots, t, p->plane, st, live)) return rc;
+    if (int rc = launch_gemv(ptrs, dn, nullptr, d, slots, t, p->plane, st, live)) return rc;
     dim3 grid(d.n / 128, 1, slots);
     if (dtype == CN_BF16 && !out_f32)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, d.n, ksplit(d.k), t, d.svh_off, rowdst));
@@ -783,8 +797,9 @@ extern "C" int cn_mul1_gemv_noalloc(int which, int hidden, int inter, int bits, 
     cudaStream_t st = (cudaStream_t)stream;
     // every region is written before it is read within one call (had_in fills xh / xinv of the live
     // slots, the GEMV fills every partial that had_out sums), so nothing has to start at zero
-    if (int rc = launch_had_in(ptrs, x, xh, xinv, s, slots, t, x_div, dtype, plane, st)) return rc;
-    if (int rc = launch_gemv(ptrs, xh, xinv, part, s, slots, t, plane, st)) return rc;
+    const Mul1Side side = {xh, xinv, part, s.tr_off, s.suh_off};
+    if (int rc = launch_had_in(ptrs, x, side, nullptr, s.k, slots, t, x_div, dtype, plane, st)) return rc;
+    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, plane, st)) return rc;
     dim3 grid(s.n / 128, 1, slots);
     if (dtype == CN_BF16)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, part, y, s.n, ksplit(s.k), t, s.svh_off, (const int*)nullptr));
