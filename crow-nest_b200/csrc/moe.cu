@@ -307,7 +307,19 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
     CN_CUDA(cudaStreamWaitEvent(p->side, p->fork, 0));
     const size_t es = dtype == CN_BF16 ? 2 : 4;
     int rc = CN_OK;
-    for (int t0 = 0; t0 < tokens && rc == CN_OK; t0 += CN_MAX_M) {
+    // More rows than a GEMV takes: both projections as one launch each over groups of rows (64 tokens, 512 x 2048: sixteen launches of
+    // 8 us each before, two of 24 and 11 us now; the step with the shared expert 297 -> 246 us).
+    RowsCall u = {}, d = {};
+    u.w0 = shared_gate, u.w1 = shared_up, u.m = tokens, u.gs0 = shared_gs, u.gs1 = shared_gs + 1, u.x = x, u.x_div = 1, u.x_f32 = dtype == CN_F32;
+    u.y = p->hs, u.ldy = p->shared_inter, u.rows = p->shared_inter, u.k = p->hidden, u.limit = limit, u.max_groups = (tokens + (u.x_f32 ? 1 : 7)) / (u.x_f32 ? 2 : 8);
+    d.w0 = shared_down, d.m = tokens, d.gs0 = shared_gs + 2, d.x = p->hs, d.x_div = 1, d.x_f32 = 1, d.y = p->ys, d.ldy = p->hidden, d.rows = p->hidden;
+    d.k = p->shared_inter, d.max_groups = (tokens + 1) / 2;
+    const bool grouped = tokens > CN_MAX_M && cn_rows_fits(u) && cn_rows_fits(d);
+    if (grouped) {
+        rc = cn_rows_launch(u, p->side, "cn_moe_nvfp4_run (shared gate/up)");
+        if (rc == CN_OK) rc = cn_rows_launch(d, p->side, "cn_moe_nvfp4_run (shared down)");
+    }
+    for (int t0 = 0; !grouped && t0 < tokens && rc == CN_OK; t0 += CN_MAX_M) {
         const int m = tokens - t0 < CN_MAX_M ? tokens - t0 : CN_MAX_M;
         GemvCall g = {};
         g.w0 = shared_gate, g.w1 = shared_up, g.gs0 = shared_gs, g.gs1 = shared_gs + 1, g.x = (const char*)x + (size_t)t0 * p->hidden * es;
@@ -329,49 +341,48 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
 int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigned long long* table_up, const unsigned long long* table_dn,
                    const float* gs_gu, const float* gs_up, const float* gs_dn, const int32_t* ids, const void* x, float* eo,
                    const unsigned long long* eo_ptrs, int combos, int x_div, float limit, int dtype, cudaStream_t stream) {
-    if (combos > 96 && combos >= 2 * p->experts) {
-        // At least two combo slots per expert (a long batch, or the inbox of an expert-parallel rank, whose few resident
-        // experts take all its rows): sort by expert, cut into groups of up to four rows of one expert, and stream every
-        // expert once per group (persistent CTAs over a device-side group list; empty slots cost nothing). One-row
-        // groups and larger groups are separate launches.
-        const size_t smem = (size_t)(3 * (p->experts + 1) + combos) * sizeof(int);
-        if (smem <= 160 * 1024) {
-            int* ga = p->groups;
-            int* gb = ga + combos;
-            int* gbrows = gb + combos;
-            int* gd = gbrows + combos;
-            int* gdrows = gd + combos;
-            int* counts = gdrows + combos;
-            if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, gd, gdrows, counts, 4, stream)) return rc;
-            RoutedCall a = {};
-            a.ids = ids, a.order = p->order, a.tab0 = table_gu, a.tab1 = table_up, a.fused_up_rows = table_up ? 0 : p->inter, a.gs0 = gs_gu;
-            a.gs1 = gs_up ? gs_up : gs_gu, a.x = x, a.x_div = x_div, a.x_f32 = dtype == CN_F32, a.y = p->h, a.ldy = p->inter, a.rows = p->inter, a.k = p->hidden;
-            a.limit = limit;
-            RoutedCall d = {};
-            d.ids = ids, d.order = p->order, d.tab0 = table_dn, d.gs0 = gs_dn, d.x = p->h, d.x_div = 1, d.x_f32 = 1, d.y = eo, d.yptrs = eo_ptrs, d.ldy = p->hidden;
-            d.rows = p->hidden, d.k = p->inter;
-            if (a.x_f32) {
-                // f32 rows take two row slots each (high and low f16 plane): groups of one or two rows, one launch
-                a.mt = 4, a.gcount = counts + 2, a.gpos = gd, a.grows = gdrows, a.max_groups = combos;
-                if (int rc = cn_routed_launch(a, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
-            } else {
-                for (int cls = 0; cls < 2; cls++) {
-                    a.mt = cls ? 4 : 1, a.gcount = counts + cls, a.gpos = cls ? gb : ga, a.grows = cls ? gbrows : nullptr, a.max_groups = cls ? combos / 2 : combos;
-                    if (int rc = cn_routed_launch(a, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
-                }
-            }
-            // the intermediate rows are f32
-            d.mt = 4, d.gcount = counts + 2, d.gpos = gd, d.grows = gdrows, d.max_groups = combos;
-            if (int rc = cn_routed_launch(d, stream, "cn_moe_nvfp4 (down, grouped)")) return rc;
-            return CN_OK;
-        }
-    }
-    // Few combos: one launch each for gate|up and down over the combos as they come (nearly every CTA of the step is
-    // resident at once and L2 serves an expert's second reader).
+    // Routed gate|up of the combos as they come (nearly every CTA of a small step is resident at once and L2 serves an
+    // expert's second reader).
     GemvCall a = {};
     a.gs0 = gs_gu, a.gs1 = gs_up ? gs_up : gs_gu, a.x = x, a.y = p->h, a.rows = p->inter, a.k = p->hidden, a.m = 1, a.ldy = p->inter;
     a.limit = limit, a.dtype = dtype, a.out_f32 = 1, a.ids = ids, a.order = nullptr, a.tab0 = table_gu, a.tab1 = table_up;
     a.fused_up_rows = table_up ? 0 : p->inter, a.x_div = x_div, a.combos = combos, a.experts = p->experts;
+    // From 48 combos on the combos are sorted by expert and cut into groups that share one decode of the expert's weights
+    // (nvfp4_rows.cu): the down projection in groups of up to two rows (its rows are f32), gate|up in groups of up to eight bf16 rows
+    // where enough of them share an expert (three combo slots for four experts), two f32 rows always. Measured, us per step of
+    // ungrouped / down grouped / both: 512 experts of 2048 x 512, top 10: 16 tokens 122 / 113 / 120, 64 tokens 444 / 325 / 297; 128
+    // experts of 2560 x 1280, top 6: 8 tokens 117 / 106 / 132, 32 tokens 390 / 306 / 267; 288 experts of 4096 x 2048, top 8: 16 tokens
+    // 515 / 401 / 440, 32 tokens 956 / 693 / 590; 64 tokens of f32 rows, 512 experts: 614 / 500 / 343. With 40 combos nothing is gained
+    // (48 / 48 / 59): the grouping is a launch of its own.
+    if (combos >= 48 && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
+        int* ga = p->groups;
+        int* gb = ga + combos;
+        int* gbrows = gb + combos;
+        int* gd = gbrows + combos;
+        int* gdrows = gd + combos;
+        int* counts = gdrows + combos;
+        auto bound = [&](int rows) { return combos < p->experts + combos / rows ? combos : p->experts + combos / rows; };  // an expert ends in one short group
+        RowsCall u = {};
+        u.ids = ids, u.order = p->order, u.tab0 = table_gu, u.tab1 = table_up, u.fused_up_rows = a.fused_up_rows, u.gs0 = a.gs0, u.gs1 = a.gs1;
+        u.x = x, u.x_div = x_div, u.x_f32 = dtype == CN_F32, u.y = p->h, u.ldy = p->inter, u.rows = p->inter, u.k = p->hidden, u.limit = limit;
+        u.max_groups = bound(u.x_f32 ? 2 : 8);
+        if (u.x_f32)
+            u.count2 = counts + 2, u.pos2 = gd, u.rows2 = gdrows;
+        else
+            u.count1 = counts, u.pos1 = ga, u.count2 = counts + 1, u.pos2 = gb, u.rows2 = gbrows;
+        RowsCall d = {};
+        d.ids = ids, d.order = p->order, d.tab0 = table_dn, d.gs0 = gs_dn, d.x = p->h, d.x_div = 1, d.x_f32 = 1, d.y = eo, d.yptrs = eo_ptrs, d.ldy = p->hidden;
+        d.rows = p->hidden, d.k = p->inter, d.count2 = counts + 2, d.pos2 = gd, d.rows2 = gdrows, d.max_groups = bound(2);
+        if (cn_rows_fits(d)) {
+            if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, gd, gdrows, counts, 8, stream)) return rc;
+            if ((u.x_f32 || 4LL * combos >= 3LL * p->experts) && cn_rows_fits(u)) {
+                if (int rc = cn_rows_launch(u, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
+            } else if (int rc = cn_gemv_launch(a, stream, "cn_moe_nvfp4 (gate/up)")) {
+                return rc;
+            }
+            return cn_rows_launch(d, stream, "cn_moe_nvfp4 (down, grouped)");
+        }
+    }
     if (int rc = cn_gemv_launch(a, stream, "cn_moe_nvfp4 (gate/up)")) return rc;
     GemvCall d = {};
     d.gs0 = gs_dn, d.x = p->h, d.y = eo, d.yptrs = eo_ptrs, d.rows = p->hidden, d.k = p->inter, d.m = 1, d.ldy = p->hidden, d.dtype = CN_F32, d.out_f32 = 1;

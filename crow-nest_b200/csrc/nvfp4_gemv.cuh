@@ -36,29 +36,6 @@ struct GemvCall {
 
 int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
-// One class of routed-expert groups (nvfp4_routed.cu): combos sorted by expert (order), groups of `mt` = 1 or up to 4
-// consecutive positions of one expert (gpos, grows; grows null for one-row groups), their number on the device (gcount).
-struct RoutedCall {
-    const int32_t* ids;
-    const int32_t* order;
-    const int* gcount;
-    const int* gpos;
-    const int* grows;
-    const unsigned long long* tab0;
-    const unsigned long long* tab1;
-    int fused_up_rows;
-    const float* gs0;
-    const float* gs1;
-    const void* x;  // activation row of combo c: row c / x_div, bf16 (or f32 when x_f32)
-    int x_div, x_f32;
-    float* y;  // f32 row of combo c at y + c * ldy, or at yptrs[c]
-    const unsigned long long* yptrs;
-    int ldy, rows, k;
-    float limit;
-    int mt, max_groups;
-};
-int cn_routed_launch(const RoutedCall& a, cudaStream_t stream, const char* who);
-
 // Sort combos by expert and cut every expert's run into groups (moe.cu): order [combos]; ga = positions (in order) of the
 // one-row groups, counts[0] of them; gb / gbrows = positions and row counts (2..gmax, gmax 4 or 8) of the larger groups,
 // counts[1]; gd / gdrows = the same runs cut into groups of one or two rows, counts[2]. Combos without a resident expert
@@ -120,3 +97,28 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
 // f32 activation rows (1..8) as columns of the tensor-core tile, three f16 planes each (nvfp4_gemv_col.cu)
 int cn_gemv_col_launch(const GemvCall& a, cudaStream_t stream, const char* who);
+
+// Rows of activations in groups that share a matrix (nvfp4_rows.cu). Routed form: the *count1 one-row groups at pos1 (none when
+// count1 is null), then *count2 groups at pos2 of rows2 rows (up to eight bf16 or two f32 rows of one expert); positions are into
+// `order`. Dense form (w0 set): m rows of one matrix, or of a gate / up pair.
+struct RowsCall {
+    const void *w0, *w1;
+    int m;
+    const int32_t* ids;
+    const int32_t* order;
+    const int *count1, *pos1, *count2, *pos2, *rows2;
+    const unsigned long long* tab0;
+    const unsigned long long* tab1;
+    int fused_up_rows;
+    const float* gs0;
+    const float* gs1;
+    const void* x;  // activation row of combo c: row c / x_div, bf16 (or f32 when x_f32)
+    int x_div, x_f32;
+    float* y;  // f32 row of combo c at y + c * ldy, or at yptrs[c]
+    const unsigned long long* yptrs;
+    int ldy, rows, k;
+    float limit;
+    int max_groups;  // bound of the groups
+};
+bool cn_rows_fits(const RowsCall& a);
+int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who);

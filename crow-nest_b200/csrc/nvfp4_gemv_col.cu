@@ -23,6 +23,7 @@
 // What bounds it: issue slots (about 200 warp instructions per unit whatever the rows, 88 of them the decode and its scaling;
 // 0.63 of the issue slots used). The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
 #include "common.cuh"
+#include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"
 
 namespace {
@@ -82,40 +83,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         if (clock64() - t0 > 2000000000LL) return false;
     }
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float2 lds64f(uint32_t a) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-    return v;
-}
-// Scale byte i of a word (sel = 0x4i4i) as f16x2 of scale x 2^-8, in both halves: an E4M3 byte shifted left by seven is that
-// f16 as it stands, subnormals included. The engine's reading: bit 7 ignored, 0x7F read as 0x7E.
-__device__ __forceinline__ uint32_t scale_f16x2(uint32_t w, uint32_t sel) {
-    const uint32_t b = __byte_perm(w, 0u, sel) & 0x007f007fu;
-    uint32_t r;
-    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(b), "r"(0x007e007eu));
-    return r << 7;
-}
-__device__ __forceinline__ uint32_t hmul2u(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-// the power of two of a tensor scale (1 where it has none)
-__device__ __forceinline__ float gs_pow2(float gs) {
-    const uint32_t e = (__float_as_uint(gs) >> 23) & 0xFF;
-    return e > 0 && e < 255 ? __uint_as_float(e << 23) : 1.0f;
-}
-
 // NP: MMA column groups, 8 NP >= 3 m. CPS: CTAs per SM the register allocation must allow.
 template <int NP, int CPS>
 __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_col_kernel(const ColParams cp) {
@@ -216,34 +183,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_col_kernel(const Col
                     const int task = t0 + i * (NW * 32);
                     if (task >= ntask) break;  // uniform over eight lanes
                     const int b = task >> 3, ch = task & 7;
-                    const uint32_t u[8] = {raw[i][0].x, raw[i][0].y, raw[i][0].z, raw[i][0].w, raw[i][1].x, raw[i][1].y, raw[i][1].z, raw[i][1].w};
-                    uint32_t e = 0;  // largest exponent of the block's finite values
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const uint32_t ev = (u[q] >> 23) & 0xFF;
-                        e = max(e, ev == 255u ? 0u : ev);
-                    }
-                    const uint32_t gm = 0xffu << (lane & 24);
-                    e = max(e, __shfl_xor_sync(gm, e, 1));
-                    e = max(e, __shfl_xor_sync(gm, e, 2));
-                    e = max(e, __shfl_xor_sync(gm, e, 4));
-                    e = e < 15 ? 15 : e;
-                    const float mul = __uint_as_float((268u - e) << 23), inv = __uint_as_float((e - 6u) << 23);  // 2^8 of scale_f16x2
                     uint32_t h[NPL][4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        float a = __uint_as_float(u[2 * q]) * mul, c = __uint_as_float(u[2 * q + 1]) * mul;  // below 2^15
-                        // the first plane on the block's own grid of 2^5, then what is left as f16, twice; an infinity or a NaN
-                        // goes into the first plane and leaves nothing
-                        const bool fa = fabsf(a) < 65536.0f, fc = fabsf(c) < 65536.0f;
-                        const float ga = fa ? __fsub_rn(__fadd_rn(a, 402653184.0f), 402653184.0f) : a;  // 1.5 x 2^28
-                        const float gc = fc ? __fsub_rn(__fadd_rn(c, 402653184.0f), 402653184.0f) : c;
-                        const __half2 h0 = __floats2half2_rn(ga, gc);
-                        a = fa ? (a - ga) * 2048.0f : 0.0f, c = fc ? (c - gc) * 2048.0f : 0.0f;
-                        const __half2 h1 = __floats2half2_rn(a, c);
-                        const __half2 h2 = __floats2half2_rn((a - __low2float(h1)) * 2048.0f, (c - __high2float(h1)) * 2048.0f);
-                        h[0][q] = *(const uint32_t*)&h0, h[1][q] = *(const uint32_t*)&h1, h[2][q] = *(const uint32_t*)&h2;
-                    }
+                    const float inv = f32_planes(raw[i][0], raw[i][1], lane, h);
 #pragma unroll
                     for (int pl = 0; pl < NPL; pl++) {
                         const int c = r * NPL + pl;

@@ -1,0 +1,256 @@
+// Routed-expert NVFP4 rows: groups of activation rows of one expert as the columns of the tensor-core tile, one warp per tile.
+//
+// Supersedes gemv_fp4_ptrb over the pointer tables (engine/src/kernels.rs:195-233) together with the grouping idea of the
+// reference's prefill path (moe_count / moe_plan / moe_scatter, engine/src/kernels.rs:3334-3420). Arithmetic as in
+// nvfp4_gemv_col.cu: weights with their scale in f16 (exact), f32 rows as three f16 planes, f32 sums.
+//
+// An expert's matrices are small (2048 x 512: a row is 288 bytes), so what a GEMV kernel spends per tile - handing sums between
+// warps, staging and scale tables per CTA - outweighs the tile. Here a warp keeps a 16-row tile to itself: it brings the tile in
+// by its own bulk copies (16 row pieces of up to eight blocks, two to four chunks ahead), holds all its sums in registers and stores
+// them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
+// columns) share one decode of its weights; a row's sum does not depend on the rows it is grouped with. Bound by issue slots:
+// about 180 warp instructions per 16 x 128 values. Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under the profiler): gate/up
+// 157 -> 129 us, down 203 -> 86 us against one CTA set per combo.
+#include "nvfp4_col.cuh"
+#include "nvfp4_gemv.cuh"
+
+namespace {
+
+constexpr int NW = 8;
+constexpr int CB = 8;  // blocks per row and chunk
+constexpr int PITCH = CB * 36 + 16;
+constexpr int CHUNK = 16 * PITCH;
+constexpr int MAX_D = 4;
+constexpr int HDR = NW * MAX_D * 8;
+
+struct RowsParams {
+    RowsCall c;
+    int parts, depth;
+    uint32_t inv_off, x_off, ring_off;
+};
+
+// NPL: columns per activation row (1: bf16, 3: f32)
+template <int NPL, int CPS>
+__global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int XE = NPL == 1 ? 2 : 4;
+    const RowsCall& c = p.c;
+    pdl_launch_dependents();
+    pdl_wait();  // the groups, ids and activations come from the kernels before this one
+    constexpr int RG = NPL == 1 ? 8 : 2;  // most rows of a group
+    const int bpr = c.k >> 6;
+    const size_t row_bytes = (size_t)bpr * 36;
+    const bool gu = c.tab1 || c.w1 || c.fused_up_rows > 0;
+    const float gs0 = __ldg(c.gs0), gs1 = __ldg(c.gs1), gp = gs_pow2(gs0);
+    const float f0 = gs0 / gp, f1 = gs1 / gp;  // exact: gp is a power of two
+    const int per_tile = gu ? 8 : 16, T = (c.rows + per_tile - 1) / per_tile;  // gate/up: row slots 0-7 gate, 8-15 up
+    const int t0 = (int)((long long)blockIdx.x * T / p.parts), t1 = (int)((long long)(blockIdx.x + 1) * T / p.parts);
+    const int nch = (bpr + CB - 1) / CB, D = p.depth;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t* full = (uint64_t*)smem + warp * MAX_D;
+    const uint32_t base = smem_u32(smem);
+    uint8_t* ring = smem + p.ring_off + (size_t)warp * D * CHUNK;
+    const int mytiles = t0 + warp < t1 ? (t1 - t0 - warp + NW - 1) / NW : 0, total = mytiles * nch;
+    if (lane == 0) {
+        for (int i = 0; i < D; i++) mbar_init(&full[i], 1);
+        mbar_fence_init();
+    }
+    __syncwarp();
+    const uint64_t pol = l2_policy_evict_first();
+    const int n1 = c.count1 ? *c.count1 : 0, ngroups = c.w0 ? (c.m + RG - 1) / RG : n1 + *c.count2;
+    int s = 0, pstage = 0;  // stage read next, stage filled next: they meet again at the end of every group
+    uint32_t par = 0;
+    for (int grp = blockIdx.y; grp < ngroups; grp += gridDim.y) {
+        // the group's rows and matrices: one-row groups, larger groups, or (dense form) RG rows after one another
+        int pos = grp * RG, nrows = min(RG, c.m - pos);
+        const uint8_t *w0 = (const uint8_t*)c.w0, *w1 = (const uint8_t*)c.w1;
+        if (!c.w0) {
+            pos = grp < n1 ? c.pos1[grp] : c.pos2[grp - n1], nrows = grp < n1 ? 1 : c.rows2[grp - n1];
+            const int e = c.ids[c.order[pos]];
+            w0 = (const uint8_t*)c.tab0[e];
+            w1 = c.tab1 ? (const uint8_t*)c.tab1[e] : (c.fused_up_rows > 0 ? w0 + (size_t)c.fused_up_rows * row_bytes : nullptr);
+            if (!w0 || (gu && !w1)) continue;  // this matrix of the expert is not resident
+        }
+        auto member = [&](int r) { return c.w0 ? pos + r : c.order[pos + r]; };
+        // chunk i of this warp in turn -> the next stage
+        int ptile = t0 + warp, pch = 0;
+        auto issue = [&]() {
+            const int row = gu ? ptile * 8 + (lane & 7) : ptile * 16 + lane;
+            const uint8_t* wb = (gu && ((lane >> 3) & 1)) ? w1 : w0;
+            const bool have = lane < 16 && row < c.rows;
+            const uint32_t piece = (uint32_t)min(CB, bpr - pch * CB) * 36u;
+            const uint32_t n = (uint32_t)__popc(__ballot_sync(0xffffffffu, have));
+            if (lane == 0) {
+                mbar_expect_tx(&full[pstage], n * piece);
+                mbar_arrive(&full[pstage]);
+            }
+            __syncwarp();
+            if (have) bulk_g2s_stream(ring + (size_t)pstage * CHUNK + (size_t)lane * PITCH, wb + (size_t)row * row_bytes + (size_t)pch * (CB * 36), piece, &full[pstage], pol);
+            if (++pch == nch) pch = 0, ptile += NW;
+            if (++pstage == D) pstage = 0;
+        };
+        for (int i = 0; i < D && i < total; i++) issue();
+
+        // the group's rows: eight lanes per 64-value block; column, block and chunk order as in nvfp4_gemv_col.cu
+        const int ncol = NPL * nrows;
+        for (int r = 0; r < nrows; r++) {
+            const int combo = member(r);
+            const uint4* xr = (const uint4*)((const char*)c.x + (size_t)(combo / c.x_div) * c.k * XE);
+            for (int task = threadIdx.x; task < bpr * 8; task += NW * 32) {  // uniform over eight lanes
+                const int b = task >> 3, ch = task & 7;
+                uint32_t h[NPL][4];
+                float inv;
+                if constexpr (NPL == 1)
+                    inv = bf16_plane(__ldcg(xr + task), lane, h);
+                else
+                    inv = f32_planes(__ldcg(xr + 2 * task), __ldcg(xr + 2 * task + 1), lane, h);
+#pragma unroll
+                for (int pl = 0; pl < NPL; pl++) {
+                    const int col = r * NPL + pl;
+                    *(uint4*)(smem + p.x_off + ((size_t)(col * bpr + b) * 8 + (ch ^ (4 * (col & 1)))) * 16) = make_uint4(h[pl][0], h[pl][1], h[pl][2], h[pl][3]);
+                    if (ch == pl) *(float*)(smem + p.inv_off + ((size_t)b * 8 + col) * 4) = inv * gp;
+                }
+            }
+        }
+        __syncthreads();
+
+        const int g = lane >> 2, t = lane & 3;
+        const int col = g < ncol ? g : (ncol > 1 ? g & 1 : 0);  // a column beyond the live ones repeats one of them and is not read
+        const uint32_t xa = base + p.x_off + (uint32_t)(col * bpr * 128 + (col & 1) * 64 + t * 16);
+        const uint32_t xflip = (col & 1) ? (uint32_t)-64 : 64u;
+        const uint32_t xi0 = base + p.inv_off + 8u * (uint32_t)t;
+        const uint32_t sel0 = (t >> 1) ? 0x4141u : 0x4040u, sel1 = sel0 + 0x0202u;
+        const uint32_t rbase = smem_u32(ring) + (uint32_t)(g * PITCH + 4 * t);
+        int done = 0;
+        bool ok = true;
+        for (int tile = t0 + warp; tile < t1 && ok; tile += NW) {
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int ch = 0; ch < nch; ch++) {
+                if (!mbar_wait(&full[s], par)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                    break;
+                }
+                const int nb = min(CB, bpr - ch * CB);
+                const uint32_t cbase = rbase + (uint32_t)(s * CHUNK), xc = xa + (uint32_t)(ch * CB * 128), xic = xi0 + (uint32_t)(ch * CB * 32);
+                auto block = [&](int b) {
+                    const uint32_t pw = cbase + 36u * b, pw8 = pw + 8u * PITCH;
+                    const uint32_t sa = lds32(pw - 4u * t), sb = lds32(pw8 - 4u * t);
+                    float cc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        uint32_t ha[4], hb[4];
+                        e2m1x8_to_f16x2(lds32(pw + 4u + 16u * hf), ha);
+                        e2m1x8_to_f16x2(lds32(pw8 + 4u + 16u * hf), hb);
+                        const uint32_t fa = scale_f16x2(sa, hf ? sel1 : sel0), fb = scale_f16x2(sb, hf ? sel1 : sel0);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) ha[i] = hmul2u(ha[i], fa), hb[i] = hmul2u(hb[i], fb);
+                        const uint4 xv = lds128(xc + b * 128u + (hf ? xflip : 0u));
+                        mma16816(cc, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
+                        mma16816(cc, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
+                    }
+                    const float2 xi = lds64f(xic + b * 32u);
+                    acc[0] = fmaf(cc[0], xi.x, acc[0]);
+                    acc[1] = fmaf(cc[1], xi.y, acc[1]);
+                    acc[2] = fmaf(cc[2], xi.x, acc[2]);
+                    acc[3] = fmaf(cc[3], xi.y, acc[3]);
+                };
+                if (nb == CB) {
+#pragma unroll
+                    for (int b = 0; b < CB; b++) block(b);
+                } else {
+                    for (int b = 0; b < nb; b++) block(b);
+                }
+                __syncwarp();  // every lane has read the stage
+                if (++done + D <= total) issue();
+                if (++s == D) s = 0, par ^= 1u;
+            }
+            if (!ok) break;
+            // lane (g, t): row slots g and g + 8, columns 2 t and 2 t + 1
+            float v[2][2];  // [row slot][activation row of this lane]
+            int r0;
+            if constexpr (NPL == 1) {
+                v[0][0] = acc[0], v[0][1] = acc[1], v[1][0] = acc[2], v[1][1] = acc[3];
+                r0 = 2 * t;
+            } else {
+                // columns 0-2 are the planes of row 0, 3-5 those of row 1: lane t = 0 ends up with row 0, lane t = 1 with row 1
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const float na = __shfl_down_sync(0xffffffffu, acc[2 * i], 1), nb = __shfl_down_sync(0xffffffffu, acc[2 * i + 1], 1);
+                    v[i][0] = t == 0 ? fmaf(na, 0x1p-22f, fmaf(acc[2 * i + 1], 0x1p-11f, acc[2 * i])) : fmaf(nb, 0x1p-22f, fmaf(na, 0x1p-11f, acc[2 * i + 1]));
+                }
+                r0 = t;
+            }
+#pragma unroll
+            for (int j = 0; j < (NPL == 1 ? 2 : 1); j++) {
+                if (r0 + j >= nrows) continue;
+                const int combo = member(r0 + j);
+                float* y = c.yptrs ? (float*)c.yptrs[combo] : c.y + (size_t)combo * c.ldy;
+                if (gu) {
+                    const int idx = tile * 8 + g;
+                    if (idx < c.rows) y[idx] = act_gu(v[0][j] * f0, v[1][j] * f1, c.limit);
+                } else {
+                    const int row = tile * 16 + g;
+                    if (row < c.rows) y[row] = v[0][j] * f0;
+                    if (row + 8 < c.rows) y[row + 8] = v[1][j] * f0;
+                }
+            }
+        }
+        if (__syncthreads_or(!ok)) return;  // also: every warp has read this group's rows
+    }
+}
+
+bool layout(const RowsCall& a, int cps, RowsParams& p, size_t& smem) {
+    const int bpr = a.k / 64, cols = 8;
+    p.inv_off = HDR;
+    p.x_off = (p.inv_off + (uint32_t)(bpr * 32) + 127u) & ~127u;
+    p.ring_off = p.x_off + (uint32_t)((a.x_f32 ? 6 : cols) * bpr * 128);
+    const long long room = (227 * 1024) / cps - 1024 - (long long)p.ring_off;
+    long long d = room / (NW * CHUNK);
+    if (d > MAX_D) d = MAX_D;
+    p.depth = (int)d;
+    smem = (size_t)p.ring_off + (size_t)(d > 0 ? d : 0) * NW * CHUNK;
+    return d >= 2;
+}
+
+}  // namespace
+
+bool cn_rows_fits(const RowsCall& a) {
+    RowsParams p = {};
+    size_t smem;
+    return a.k > 0 && a.k % 256 == 0 && layout(a, 1, p, smem);
+}
+
+int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
+    RowsParams p = {};
+    size_t smem;
+    if (a.rows <= 0 || a.k <= 0 || a.k % 256 != 0) CN_FAIL(CN_ERR_SHAPE, "%s: k = %d must be a positive multiple of 256", who, a.k);
+    if ((uintptr_t)a.x & 15) CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
+    int cps = 2;
+    if (!layout(a, 2, p, smem)) {
+        cps = 1;
+        if (!layout(a, 1, p, smem)) CN_FAIL(CN_ERR_LIMIT, "%s: k = %d leaves no room for a weight ring beside the activation rows", who, a.k);
+    }
+    p.c = a;
+    if (!p.c.gs1) p.c.gs1 = a.gs0;
+    const bool gu = a.tab1 || a.w1 || a.fused_up_rows > 0;
+    const int T = (a.rows + (gu ? 8 : 16) - 1) / (gu ? 8 : 16);
+    // CTAs per group: four rounds of CTAs if every group were there, but at least two tiles for each warp
+    p.parts = (4 * 148 * cps + a.max_groups - 1) / a.max_groups;
+    if (p.parts > T / (2 * NW)) p.parts = T / (2 * NW);
+    if (p.parts < 1) p.parts = 1;
+    // CTAs walk the groups: four rounds of CTAs at most, so that a list much shorter than its bound (the inbox of an
+    // expert-parallel rank) costs no more than that
+    int gy = (4 * 148 * cps + p.parts - 1) / p.parts;
+    if (gy > a.max_groups) gy = a.max_groups;
+    const dim3 grid((unsigned)p.parts, (unsigned)gy);
+#define CN_ROWS_CASE(NPLV, CPSV)                                                                                   \
+    if (a.x_f32 == (NPLV == 3) && cps == CPSV) {                                                                   \
+        CN_ALLOW_SMEM((nvfp4_rows_kernel<NPLV, CPSV>), 226 * 1024);                                                \
+        CN_CUDA(cn_launch_pdl((nvfp4_rows_kernel<NPLV, CPSV>), grid, dim3(NW * 32), smem, stream, p));             \
+        return CN_OK;                                                                                              \
+    }
+    CN_ROWS_CASE(1, 1) CN_ROWS_CASE(1, 2) CN_ROWS_CASE(3, 1) CN_ROWS_CASE(3, 2)
+#undef CN_ROWS_CASE
+    return CN_OK;
+}

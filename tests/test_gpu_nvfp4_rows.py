@@ -1,0 +1,53 @@
+"""Experts with their rows in groups (48 combos and more): k that ends in a part of a chunk, row counts that end in a part of a tile,
+groups of one, two and eight rows and what is left over, f32 and bf16 rows, the shared expert beyond eight rows."""
+import numpy as np
+import pytest
+import torch
+
+from crownest_b200 import device_status, moe, ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden,inter,experts,topk,tokens,shared", [(256, 256, 3, 2, 24, 256), (768, 1280, 5, 2, 33, 512), (2048, 512, 64, 4, 40, 0),
+                                                                   (1280, 768, 200, 6, 8, 256), (4096, 256, 2, 2, 60, 1024)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_grouped_experts_against_64_bits(hidden, inter, experts, topk, tokens, shared, dtype):
+    rng = np.random.default_rng(hidden + inter + tokens)
+
+    def matrix(rows, k):
+        return torch.from_numpy(synth.nvfp4_matrix(rows, k, rng)).cuda()
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(experts)], [matrix(hidden, inter) for _ in range(experts)]
+    sh = [matrix(shared, hidden), matrix(shared, hidden), matrix(hidden, shared)] if shared else None
+    gs_gu, gs_dn = 0.03, 0.7
+    w = moe.GpuMoeWeights(hidden, inter, experts, gs_gu, gs_dn, gate_up=gu, down=dn, shared=sh, shared_gs=[0.03, 0.03, 0.7], device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, topk, tokens, shared_inter=shared)
+    x = torch.from_numpy(rng.standard_normal((tokens, hidden)).astype(np.float32)).cuda().to(dtype)
+    logits = torch.from_numpy(rng.standard_normal((tokens, experts)).astype(np.float32)).cuda()
+    y = torch.empty_like(x)
+    plan.run(w, logits, x, y, router="softmax")
+    again = torch.empty_like(y)
+    plan.run(w, logits, x, again, router="softmax")
+    assert torch.equal(y, again)
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m.view(-1), torch.tensor([gs], dtype=torch.float32, device="cuda"), rows, k)).double().view(rows, k)
+
+    def ffn(g, u, d, xs):
+        a = xs @ g.t()
+        return (a / (1 + torch.exp(-a)) * (xs @ u.t())) @ d.t()
+
+    ids, wts = plan.ids.view(tokens, topk), plan.wts.view(tokens, topk).double()
+    x64, want = x.double(), torch.zeros((tokens, hidden), dtype=torch.float64, device="cuda")
+    for e in range(experts):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        if len(t):
+            full = deq(gu[e], 2 * inter, hidden, gs_gu)
+            want.index_add_(0, t, wts[t, j, None] * ffn(full[:inter], full[inter:], deq(dn[e], hidden, inter, gs_dn), x64[t]))
+    if shared:
+        want += ffn(deq(sh[0], shared, hidden, 0.03), deq(sh[1], shared, hidden, 0.03), deq(sh[2], hidden, shared, 0.7), x64)
+    # f32 throughout: two long sums of 1.2e-7 each, a dozen f32 roundings; a bf16 result adds its own rounding of at most 2^-9
+    bound = 2e-6 if dtype == torch.float32 else 2.0 ** -9 + 2e-6
+    assert (y.double() - want).norm() <= bound * want.norm()
+    assert device_status() == 0
