@@ -100,7 +100,7 @@ int cn_gemv_col_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
 // Rows of activations in groups that share a matrix (nvfp4_rows.cu). Routed form: the *count1 one-row groups at pos1 (none when
 // count1 is null), then *count2 groups at pos2 of rows2 rows (up to eight bf16 or two f32 rows of one expert); positions are into
-// `order`. Dense form (w0 set): m rows of one matrix, or of a gate / up pair.
+// `order`; without `order`, m combos one by one. Dense form (w0 set): m rows of one matrix, or of a gate / up pair.
 struct RowsCall {
     const void *w0, *w1;
     int m;
@@ -119,6 +119,7 @@ struct RowsCall {
     int ldy, rows, k;
     float limit;
     int max_groups;  // bound of the groups
+    int experts;     // entries of the tables (0 = unknown: ids are trusted); an id beyond them skips the combo
 };
 bool cn_rows_fits(const RowsCall& a);
 int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who);

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
     }
     __syncwarp();
     const uint64_t pol = l2_policy_evict_first();
-    const int n1 = c.count1 ? *c.count1 : 0, ngroups = c.w0 ? (c.m + RG - 1) / RG : n1 + *c.count2;
+    const int n1 = c.count1 ? *c.count1 : 0, ngroups = c.w0 ? (c.m + RG - 1) / RG : (c.order ? n1 + *c.count2 : c.m);
     int s = 0, pstage = 0;  // stage read next, stage filled next: they meet again at the end of every group
     uint32_t par = 0;
     for (int grp = blockIdx.y; grp < ngroups; grp += gridDim.y) {
@@ -65,13 +65,17 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
         int pos = grp * RG, nrows = min(RG, c.m - pos);
         const uint8_t *w0 = (const uint8_t*)c.w0, *w1 = (const uint8_t*)c.w1;
         if (!c.w0) {
-            pos = grp < n1 ? c.pos1[grp] : c.pos2[grp - n1], nrows = grp < n1 ? 1 : c.rows2[grp - n1];
-            const int e = c.ids[c.order[pos]];
+            if (c.order)
+                pos = grp < n1 ? c.pos1[grp] : c.pos2[grp - n1], nrows = grp < n1 ? 1 : c.rows2[grp - n1];
+            else
+                pos = grp, nrows = 1;  // the combos as they come
+            const int e = c.ids[c.order ? c.order[pos] : pos];
+            if (e < 0 || (c.experts > 0 && e >= c.experts)) continue;
             w0 = (const uint8_t*)c.tab0[e];
             w1 = c.tab1 ? (const uint8_t*)c.tab1[e] : (c.fused_up_rows > 0 ? w0 + (size_t)c.fused_up_rows * row_bytes : nullptr);
             if (!w0 || (gu && !w1)) continue;  // this matrix of the expert is not resident
         }
-        auto member = [&](int r) { return c.w0 ? pos + r : c.order[pos + r]; };
+        auto member = [&](int r) { return c.order ? c.order[pos + r] : pos + r; };
         // chunk i of this warp in turn -> the next stage
         int ptile = t0 + warp, pch = 0;
         auto issue = [&]() {
