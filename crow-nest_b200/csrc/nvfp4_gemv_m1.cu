@@ -51,7 +51,9 @@ constexpr int ROWS = 16;
 // ---- two-CTA cluster helpers (K range of a tile shared between the CTAs of a pair)
 // f32 [8 slots][up to 3 senders][16] sums from the other CTAs of a cluster of two or four, then a barrier per slot
 constexpr int XCH_OFF = 256, XCH_SLOTS = 8, XBAR_OFF = XCH_OFF + XCH_SLOTS * 3 * 64;
-static_assert(XBAR_OFF + XCH_SLOTS * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
+// tiles of a CTA that have a slot of their own (slots are not used twice); with more than one activation row they lie behind the tile sums
+__host__ __device__ constexpr int xch_slots(int mt) { return mt == 1 ? XCH_SLOTS : 16; }
+static_assert(XBAR_OFF + xch_slots(2) * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -114,7 +116,7 @@ __device__ __forceinline__ void push_lines(const GemvParams& p, int row0, int nr
 
 // TX: 36-byte blocks per row and stage (32 or 16); the last chunk of a row may be shorter
 // CPS: CTAs per SM the register allocation must allow; MT: activation rows (1, 2, 4 or 8; p.m of them live)
-// KS: 1, or 2 = launched as two-CTA clusters, the CTAs of a pair sharing every tile's K range (MT = 1 only)
+// KS: 1, or 2 / 4 = launched as clusters of so many CTAs that share the K range of every tile
 // LN: tensor-parallel line output compiled in (one activation row only); without it the kernel carries none of that code
 template <int TX, int CPS, int MT, int KS = 1, bool LN = false>
 __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const GemvParams p) {
@@ -125,8 +127,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     constexpr int pstride = TX * 36 + 16;  // padded: the eight rows of a quad column hit distinct banks
     constexpr int stage_bytes = ROWS * pstride;
     constexpr int GPW = TX / 2 / NW > 0 ? TX / 2 / NW : 1;  // groups per warp and full chunk
-    // KS = 2 (one activation row only): the CTAs of a cluster pair walk the same tiles, each over half of K
-    static_assert(KS == 1 || MT == 1, "the K range is shared between CTAs for one activation row only");
+    // KS > 1: the CTAs of a cluster walk the same tiles, each over its part of K
     const int crank = KS > 1 ? (int)(blockIdx.x % KS) : 0;
     const int cid = KS > 1 ? (int)(blockIdx.x / KS) : (int)blockIdx.x, ncl = KS > 1 ? (int)(gridDim.x / KS) : (int)gridDim.x;
     const int bpr_all = p.k >> 6;
@@ -161,7 +162,9 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     float* lut = (float*)(smem + LUT_OFF);  // [2][256] ue4m3 * gs
     float* red = (float*)(smem + RED_OFF);  // [red_depth][NW][MT][16] partial sums of a tile
     const int RD = p.red_depth;             // tile sums in flight (<= RED_DEPTH)
-    const uint32_t xs_off = (uint32_t)(RED_OFF + RD * NW * MT * 64);
+    // the sums handed over inside a cluster: in the header for one activation row, behind the tile sums for more
+    const uint32_t xch_off = MT == 1 ? (uint32_t)XCH_OFF : (uint32_t)(RED_OFF + RD * NW * MT * 64);
+    const uint32_t xs_off = (uint32_t)(RED_OFF + RD * NW * MT * 64) + (KS > 1 && MT > 1 ? (uint32_t)(xch_slots(MT) * (KS - 1) * MT * 64) : 0u);
     uint8_t* xs0 = smem + xs_off;           // [MT][bpr][128] f16 activations
     const uint32_t XS = (uint32_t)bpr * XB;  // bytes of one activation row
     float* xinv0 = (float*)(xs0 + (size_t)MT * XS);  // [MT][bpr]
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     // depend on the previous kernel); the consumers meet it on named barrier 2 before their first wait.
     if (warp == NW) {
         // one barrier per lane and round: S full + S empty + RD tile-sum (+ the pair's exchange slots), side by side
-        for (int i = lane; i < 2 * S + RD + (KS > 1 ? XCH_SLOTS : 0); i += 32) {
+        for (int i = lane; i < 2 * S + RD + (KS > 1 ? xch_slots(MT) : 0); i += 32) {
             if (i < S) mbar_init(&full[i], 1);
             else if (i < 2 * S) mbar_init(&empty[i - S], NW);
             else if (i < 2 * S + RD) mbar_init(&tbar[i - 2 * S], NW);
@@ -250,7 +253,10 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     const int ntask = MT * bpr * 8;
     auto load_x = [&](int task) -> uint4 {
         // task = (row * bpr + block) * 8 + chunk; rows beyond p.m read as zero
-        return (task < ntask && (MT == 1 || (task >> 3) < p.m * bpr)) ? __ldcg((const uint4*)xbase + task) : make_uint4(0u, 0u, 0u, 0u);
+        if (task >= ntask || (MT > 1 && (task >> 3) >= p.m * bpr)) return make_uint4(0u, 0u, 0u, 0u);
+        // a part of K: the rows of x lie whole rows apart
+        const int at = KS > 1 && MT > 1 ? task + (task >> 3) / bpr * (bpr_all - bpr) * 8 : task;
+        return __ldcg((const uint4*)xbase + at);
     };
     // PF loads of every thread are in flight at any time: the staging loop costs about one trip to L2 per PF tasks
     constexpr int PF = CPS >= 4 ? 2 : 4;
@@ -478,6 +484,42 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
             if (!mbar_wait(&tbar[rslot], rpar)) {
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 ok = false;
+            } else if (MT > 1 && KS > 1) {
+                // as for one row below, lane l over (activation row, row slot) pairs l, l + 32, ...
+                constexpr int NO = MT > 1 ? MT / 2 : 1;
+                float v[NO];
+#pragma unroll
+                for (int i = 0; i < NO; i++) {
+                    const int o = lane + 32 * i;
+                    v[i] = rb[o];
+                    for (int w = 1; w < NW; w++) v[i] += rb[w * MT * 16 + o];
+                }
+                float* xch = (float*)(smem + xch_off) + titer * (KS - 1) * MT * 16;
+                uint64_t* xb = (uint64_t*)(smem + XBAR_OFF) + titer;
+                if (crank != 0) {
+#pragma unroll
+                    for (int i = 0; i < NO; i++) st_peer_f32(peer_addr(xch + (crank - 1) * MT * 16 + lane + 32 * i, 0), v[i]);
+                    __syncwarp();
+                    if (lane == 0) arrive_peer(peer_addr(xb, 0));
+                } else if (!mbar_wait_cluster(xb, 0)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NO; i++) {
+                        const int o = lane + 32 * i, m = o >> 4, slot = o & 15;
+                        for (int c = 0; c < KS - 1; c++) v[i] += xch[c * MT * 16 + o];
+                        const float up = __shfl_down_sync(0xffffffffu, v[i], 8);
+                        const int row = tile * per_cta + slot;
+                        const float r = gu ? act_gu(v[i], up, p.limit) : v[i];
+                        if (slot < per_cta && row < p.rows && m < p.m) {
+                            if (p.out_f32)
+                                ((float*)ybase)[(size_t)m * p.ldy + row] = r;
+                            else
+                                ((__nv_bfloat16*)ybase)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(r);
+                        }
+                    }
+                }
             } else if (MT == 1 && KS > 1) {
                 // lane l < 16: row slot l of the tile over this CTA's part of K, the eight warps in order
                 float v = 0.0f;
@@ -618,23 +660,30 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // matrix of few, long rows (a tensor-parallel rank's share of a down projection) gets CTAs enough to stream it.
     // Taken when it shortens the longest CTA by a tenth or more and either the machine is not filled otherwise or a CTA's
     // share stays long enough to hide the hand-over (measured on full machines: 235 KB yes, 69 KB no).
+    // Two and more activation rows take it only where the machine is not filled otherwise: 640 x 17408 with 2 / 4 / 8 rows 9.6 / 13.3 /
+    // 26.1 -> 6.8 / 8.1 / 15.1 us, but 5120 x 17408 22.0 / 27.0 / 53.4 -> 29.2 / 32.7 / 59.8 (warp 0 of a cluster's first CTA waits for
+    // the others' sums of every tile, and has four times the sums to add).
     int ksplit = 1;
     size_t xbytes_l = xbytes;
-    if (!routed && mt == 1 && tx == 32) {
-        double best = (double)((ntiles + 148 * cps - 1) / (148 * cps));  // tiles per CTA without a split
+    if (!routed && tx == 32) {
+        double best = (double)((ntiles + 148 * cps - 1) / (148 * cps)) * (mt == 1 ? 1 : cps);  // tiles per CTA (of an SM) without a split
+        if (mt > 1 && cps == 1) best *= 1.5;  // one CTA's eight warps alone do not keep an SM busy
         int best_cps = cps;
         for (int ks = 2; ks <= 4; ks *= 2) {
             if (bpr % (4 * ks) != 0) continue;  // every part starts on a 16-byte boundary of the row
             const int bk = bpr / ks, nchk = (bk + tx - 1) / tx;
-            const long long xk = (long long)bk * XB + (long long)((bk + 3) & ~3) * 4;
-            int ck = 2;
-            if ((227 * 1024) / 3 - 1024 - ((long long)RED_OFF + (long long)((3 + nchk) / nchk + 1) * NW * 64 + xk) >= 3 * (long long)stage_bytes) ck = 3;
+            const long long xk = (long long)mt * bk * XB + (long long)((mt * bk + 3) & ~3) * 4 + (mt > 1 ? (long long)xch_slots(mt) * (ks - 1) * mt * 64 : 0);
+            auto fits = [&](int c) {
+                return (227 * 1024) / c - 1024 - ((long long)RED_OFF + (long long)((3 + nchk) / nchk + 1) * NW * mt * 64 + xk) >= 3 * (long long)stage_bytes;
+            };
+            const int ck = mt == 1 ? (fits(3) ? 3 : 2) : (fits(2) ? 2 : 1);
+            if (mt > 1 && !fits(ck)) continue;
             const int clusters = 148 * ck / ks;
             const int waves = (ntiles + clusters - 1) / clusters;
             const long long share = (long long)waves * ROWS * bk * 36;
             const bool underfilled = (long long)ntiles * ks <= 148LL * ck;
-            if (waves > XCH_SLOTS || share < 32 * 1024 || !(underfilled || share >= 160 * 1024)) continue;
-            const double t = (double)waves / ks;
+            if (waves > xch_slots(mt) || share < 32 * 1024 || !(underfilled || (mt == 1 && share >= 160 * 1024))) continue;
+            const double t = mt == 1 ? (double)waves / ks : (double)waves * ck / ks * (ck == 1 ? 1.5 : 1.0);
             if (t <= 0.9 * best) best = t, ksplit = ks, best_cps = ck, xbytes_l = (size_t)xk;
         }
         if (ksplit > 1) {
@@ -704,6 +753,11 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
             if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2, true>(cfg, p) : launch_m1<32, 3, 1, 2, true>(cfg, p);
             return cps == 2 ? launch_m1<32, 2, 1, 4, true>(cfg, p) : launch_m1<32, 3, 1, 4, true>(cfg, p);
         }
+#define CN_M1_SPLIT(CPSV, MTV, KSV) \
+    if (cps == CPSV && mt == MTV && ksplit == KSV) return launch_m1<32, CPSV, MTV, KSV>(cfg, p);
+        CN_M1_SPLIT(1, 2, 2) CN_M1_SPLIT(1, 2, 4) CN_M1_SPLIT(2, 2, 2) CN_M1_SPLIT(2, 2, 4) CN_M1_SPLIT(1, 4, 2) CN_M1_SPLIT(1, 4, 4)
+        CN_M1_SPLIT(2, 4, 2) CN_M1_SPLIT(2, 4, 4) CN_M1_SPLIT(1, 8, 2) CN_M1_SPLIT(1, 8, 4) CN_M1_SPLIT(2, 8, 2) CN_M1_SPLIT(2, 8, 4)
+#undef CN_M1_SPLIT
         if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2>(cfg, p) : launch_m1<32, 3, 1, 2>(cfg, p);
         return cps == 2 ? launch_m1<32, 2, 1, 4>(cfg, p) : launch_m1<32, 3, 1, 4>(cfg, p);
     }
