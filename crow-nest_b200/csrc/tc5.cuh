@@ -161,10 +161,14 @@ __device__ __forceinline__ void decode64_f16(const uint32_t w[9], uint32_t v[32]
         }
     }
 }
-// bf16: code x scale x 2^-60, exact (six significant bits at most). A code's magnitude x 2^60 comes from two byte-permute
+// bf16: code x scale x 2^-12, exact (six significant bits at most). A code's magnitude x 2^108 comes from two byte-permute
 // tables (high and low byte of the bf16), its sign from the nibble's top bit; a scale byte shifted left by four IS the
 // bf16 of scale x 2^-120, subnormals included. The caller multiplies the sums by BF16_UNSCALE.
-constexpr float BF16_UNSCALE = 1152921504606846976.0f;  // 2^60
+// Why 2^-12: the activations are not scaled per row, so the f32 sums see them as they are. The largest weight becomes 2688 x 2^-12 < 1:
+// no sum of 2^15 products overflows for rows up to 2^113; and rows down to 2^-112 keep 20 bits and more above the last subnormal f32
+// (the tensor core keeps subnormals; measured with 2^-60, where rows of 2^-80 lost a percent and rows below 2^-96 all). Those are
+// the rows that a power of two per row could bring to f16.
+constexpr float BF16_UNSCALE = 4096.0f;  // 2^12
 __device__ __forceinline__ void decode64_bf16(const uint32_t w[9], uint32_t v[32]) {
     const uint32_t sw = scale_bytes_rule(w[0]);
 #pragma unroll
@@ -175,7 +179,7 @@ __device__ __forceinline__ void decode64_bf16(const uint32_t w[9], uint32_t v[32
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const uint32_t sel = h ? mag >> 16 : mag;
-            const uint32_t hi = __byte_perm(0x5D5D5D00u, 0x5E5E5E5Eu, sel);
+            const uint32_t hi = __byte_perm(0x75757500u, 0x76767676u, sel);
             const uint32_t lo = __byte_perm(0xC0800000u, 0xC0804000u, sel);
             const uint32_t sg = __byte_perm(up, cw, h ? 0x7362 : 0x5140);
             const uint32_t hs = hi | (sg & 0x80808080u);

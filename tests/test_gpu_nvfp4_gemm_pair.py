@@ -28,3 +28,21 @@ def test_pair_gemm_matches_the_cpu_reference(rows, k, m):
     scale = np.sqrt(np.mean(ref.astype(np.float64) ** 2, axis=1, keepdims=True))
     assert np.max(np.abs(yf - ref) / scale) <= 1e-4
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("m", [129, 513])
+def test_rows_of_any_magnitude(m):
+    """bf16 rows are not scaled one by one on this path: rows near both ends of what a power of two per row brings into f16 (2^-112 to
+    2^113) come out as well as the others, beside ordinary rows."""
+    rows, k = 512, 2048
+    rng = np.random.default_rng(m)
+    w = ops.Fp4.from_host(synth.nvfp4_matrix(rows, k, rng), rows, k, np.float32(1.0))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda()
+    for i, scale in enumerate([1e-12, 1e-20, 1e-27, 1e-33, 1e12, 1e27, 1e33]):
+        x[5 + 17 * i] *= scale
+    x = x.to(torch.bfloat16)
+    want = x.double() @ ops.dequant(w).double().view(rows, k).t()
+    err = (ops.launch_gemm(w, x).double() - want).norm(dim=1) / want.norm(dim=1)
+    # one rounding of the result to bf16 (2^-9 at most) beside f32 sums
+    assert err.max().item() <= 2.0 ** -9 + 4e-6
+    assert device_status() == 0
