@@ -229,7 +229,8 @@ int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
     RowsParams p = {};
     size_t smem;
     if (a.rows <= 0 || a.k <= 0 || a.k % 256 != 0) CN_FAIL(CN_ERR_SHAPE, "%s: k = %d must be a positive multiple of 256", who, a.k);
-    if ((uintptr_t)a.x & 15) CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
+    if (((uintptr_t)a.w0 | (uintptr_t)a.w1 | (uintptr_t)a.x) & 15)  // bulk copies and 128-bit loads
+        CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
     int cps = 2;
     if (!layout(a, 2, p, smem)) {
         cps = 1;

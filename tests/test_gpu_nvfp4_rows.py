@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from crownest_b200 import device_status, moe, ops, synth
+from crownest_b200 import CrownestError, device_status, moe, ops, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -50,4 +50,28 @@ def test_grouped_experts_against_64_bits(hidden, inter, experts, topk, tokens, s
     # f32 throughout: two long sums of 1.2e-7 each, a dozen f32 roundings; a bf16 result adds its own rounding of at most 2^-9
     bound = 2e-6 if dtype == torch.float32 else 2.0 ** -9 + 2e-6
     assert (y.double() - want).norm() <= bound * want.norm()
+    assert device_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [8, 9, 40])
+@pytest.mark.parametrize("which", [0, 1, 2])
+def test_shared_matrix_off_16_bytes_is_refused(tokens, which):
+    """The refusal is the host's, before the shared expert's first launch, whether its rows go one by one or in groups."""
+    hidden, inter, experts, topk = 256, 256, 4, 2
+    rng = np.random.default_rng(which)
+
+    def matrix(rows, k, off=0):
+        b = synth.nvfp4_matrix(rows, k, rng)
+        buf = torch.zeros(b.size + 16, dtype=torch.uint8, device="cuda")
+        buf[off:off + b.size] = torch.from_numpy(b).cuda()
+        return buf[off:off + b.size]
+
+    sh = [matrix(inter, hidden, 4 if which == i else 0) for i in range(3)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 1.0, 1.0, gate_up=[matrix(2 * inter, hidden)] * experts, down=[matrix(hidden, inter)] * experts, shared=sh,
+                          shared_gs=[1.0] * 3, device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, topk, tokens, shared_inter=inter)
+    x = torch.randn((tokens, hidden), device="cuda").to(torch.bfloat16)
+    with pytest.raises(CrownestError, match="16-byte aligned"):
+        plan.run(w, torch.randn((tokens, experts), device="cuda"), x)
+    torch.cuda.synchronize()
     assert device_status() == 0
