@@ -145,7 +145,7 @@ __global__ void act_cascade_kernel(const void* __restrict__ x, uint8_t* __restri
 }
 
 // The same cascade (LEVELS levels) written as the stage images of the GEMM, and rs[tok] = 2^-k of every row (1 for rows beyond
-// m, which are zero rows). grid (CQ, tokens rounded up to whole token blocks), clusters of CQ along a row, block CTHREADS.
+// m, which are zero rows). grid CQ x tokens rounded up to whole token blocks (on x: y ends at 65,535), clusters of CQ, block CTHREADS.
 // A cluster owns a row: every CTA takes the maximum of its share of the row, the shares meet through distributed shared memory,
 // and four lanes quantise a 16-value sub-block together. What bounds it: the chain of five dependent levels, some 2400
 // instructions when one thread holds a whole sub-block; a quarter of that, and four times the warps to hide it, with four. 64 rows
@@ -159,7 +159,7 @@ __global__ void __cluster_dims__(CQ, 1, 1) __launch_bounds__(CTHREADS) bs_cascad
     __shared__ float shares[CQ];
     pdl_launch_dependents();
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");  // this CTA has started: its shared memory may be written to
-    const int tok = blockIdx.y, tb = tok / TB, tt = tok % TB, rank = blockIdx.x;  // one cluster per row: its rank is blockIdx.x
+    const int tok = blockIdx.x / CQ, tb = tok / TB, tt = tok % TB, rank = blockIdx.x % CQ;  // one cluster per row
     const int kts = k / KT;
     const bool live = tok < m;
     const int ntask = k / 4, share = (ntask / CQ + CTHREADS - 1) / CTHREADS * CTHREADS;  // a task is four values, a quarter of a sub-block
@@ -523,7 +523,7 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
     float* rs = (float*)(xq + (size_t)ntb * kts * B_STAGE);
     float* part = rs + (size_t)ntb * TB + 64;
     if (((uintptr_t)x & 15)) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: x must be 16-byte aligned");
-    const dim3 cgrid(CQ, ntb * TB);
+    const dim3 cgrid((unsigned)CQ * ntb * TB);
     if (dtype == CN_BF16)
         bs_cascade_kernel<1><<<cgrid, CTHREADS, 0, stream>>>(x, xq, rs, k, m);
     else

@@ -72,3 +72,15 @@ def test_fp4_gemm_on_the_batched_benchmark_matrices(rows, k, m):
     ref = cpu_rows(sub, len(pick), k, gs, xf)
     check_close(from_dev_bf16(y)[:, pick], ref, f"fp4 gemm {rows}x{k} m={m} (sample)", ulp_floor=1.0 / 64)
     assert device_status() == 0
+
+
+def test_more_rows_than_a_grid_has_in_y():
+    rows, k, m = 128, 256, 65600
+    rng = np.random.default_rng(8)
+    w = synth.nvfp4_matrix(rows, k, rng)
+    xb, xf = synth.activations(64, k, rng)
+    fw = ops.Fp4Packed(ops.Fp4.from_host(w, rows, k, np.float32(0.37)))
+    y = ops.launch_gemm_fp4(fw, to_dev_bf16(xb).repeat(m // 64, 1))
+    assert torch.equal(y.view(torch.int16), y[:64].view(torch.int16).repeat(m // 64, 1))
+    check_close(from_dev_bf16(y[:64]), cpu_rows(w, rows, k, np.float32(0.37), xf), "first rows", ulp_floor=1.0 / 64)
+    assert device_status() == 0

@@ -56,7 +56,7 @@ def test_grouped_experts_against_64_bits(hidden, inter, experts, topk, tokens, s
 @pytest.mark.parametrize("tokens", [8, 9, 40])
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_shared_matrix_off_16_bytes_is_refused(tokens, which):
-    """The refusal is the host's, before the shared expert's first launch, whether its rows go one by one or in groups."""
+    """The refusal is the host's, whether the shared expert's rows go one by one or in groups."""
     hidden, inter, experts, topk = 256, 256, 4, 2
     rng = np.random.default_rng(which)
 
