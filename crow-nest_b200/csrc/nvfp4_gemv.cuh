@@ -71,7 +71,6 @@ struct GemvParams {
     int experts;  // entries of tab0 / tab1 (0 = unknown); ids outside 0..experts-1 skip the combo
     const unsigned long long* yptrs;  // output row address per combo (null: y + combo * ldy)
     int red_depth;  // multi-row tensor-core kernel: tile-sum slots in flight
-    int ksplit;     // 2: launched as two-CTA clusters, each CTA of a pair over half of K (one activation row only)
     // tensor-parallel line output (see GemvCall): line buffer of every rank (0 = none), first global row, the counter
     unsigned long long yl[8];
     int yl_world, yl_row0;

@@ -10,10 +10,12 @@
 // small shared-memory ring with one mbarrier per slot, so no CTA-wide barrier sits in the loop.
 // With more than one activation row the C columns are packed (four activation rows x the two sub-blocks
 // of a pair: 8 MMAs per group for up to four rows, 16 for eight); row i of an m-row call is summed in
-// exactly the order of a one-row call.
+// exactly the order of a one-row call: k is cut into one, two or four parts by a rule of the matrix alone
+// (one_row_split), and a row's sum is its parts in order, whether the CTAs of a cluster take one each or a CTA
+// several one after another.
 // When the tiles do not fill the last wave and a CTA's share is long enough (the down projection), or the
 // tiles are too few to fill the machine (a tensor-parallel rank's share of it), the launch is made of
-// clusters of two or four CTAs that take a part of K each (see the helpers below).
+// clusters of two or four CTAs that take a part of K each, or with several rows two parts (see the helpers below).
 // The LN variant (one activation row) also stores the output rows as 16-byte lines into the line buffers of
 // the other GPUs of a tensor-parallel group: the exchange that follows the projection starts in its epilogue.
 //
@@ -37,7 +39,7 @@ namespace {
 constexpr int NW = 8;  // consumer warps
 constexpr int NTHREADS = (NW + 1) * 32;
 constexpr int MAX_STAGES = 8;
-constexpr int RED_DEPTH = 10;  // tile sums in flight: a warp runs at most MAX_STAGES chunks ahead of warp 0
+constexpr int RED_DEPTH = 12;  // sums of a tile or part in flight, at most (see red_slots)
 constexpr int XB = 128;        // one 64-value block of f16 activations, 16-byte chunks XOR-swizzled
 // header: mbarriers (full, empty, tile), two 16-byte zero chunks 2048 B apart (the second group of a chunk
 // reads everything 2048 B further on), scale table, tile sums
@@ -51,9 +53,10 @@ constexpr int ROWS = 16;
 // ---- two-CTA cluster helpers (K range of a tile shared between the CTAs of a pair)
 // f32 [8 slots][up to 3 senders][16] sums from the other CTAs of a cluster of two or four, then a barrier per slot
 constexpr int XCH_OFF = 256, XCH_SLOTS = 8, XBAR_OFF = XCH_OFF + XCH_SLOTS * 3 * 64;
-// tiles of a CTA that have a slot of their own (slots are not used twice); with more than one activation row they lie behind the tile sums
-__host__ __device__ constexpr int xch_slots(int mt) { return mt == 1 ? XCH_SLOTS : 16; }
-static_assert(XBAR_OFF + xch_slots(2) * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
+// Tiles of a CTA that have a slot of their own (slots are not used twice). With more than one activation row a cluster has one tile (it
+// is launched only where the machine is not filled otherwise), and its slot - a sum per part of the other CTAs - lies behind the tile sums.
+__host__ __device__ constexpr int xch_slots(int mt) { return mt == 1 ? XCH_SLOTS : 1; }
+static_assert(XBAR_OFF + XCH_SLOTS * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -118,9 +121,11 @@ __device__ __forceinline__ void push_lines(const GemvParams& p, int row0, int nr
 // CPS: CTAs per SM the register allocation must allow; MT: activation rows (1, 2, 4 or 8; p.m of them live)
 // KS: 1, or 2 / 4 = launched as clusters of so many CTAs that share the K range of every tile
 // LN: tensor-parallel line output compiled in (one activation row only); without it the kernel carries none of that code
-template <int TX, int CPS, int MT, int KS = 1, bool LN = false>
+// PP: parts of K that a CTA sums one after another (more than one activation row, and a matrix of KS x PP parts)
+template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1>
 __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const GemvParams p) {
     static_assert(!LN || MT == 1, "line output takes one activation row");
+    static_assert(PP == 1 || MT > 1, "one activation row has a CTA for every part");
     extern __shared__ __align__(128) uint8_t smem[];
     if (threadIdx.x == 0) { CN_STAMP(0); }
     const float gs0_early = __ldg(p.gs0), gs1_early = __ldg(p.gs1);  // tensor scales: asked for first, used late
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     const int RD = p.red_depth;             // tile sums in flight (<= RED_DEPTH)
     // the sums handed over inside a cluster: in the header for one activation row, behind the tile sums for more
     const uint32_t xch_off = MT == 1 ? (uint32_t)XCH_OFF : (uint32_t)(RED_OFF + RD * NW * MT * 64);
-    const uint32_t xs_off = (uint32_t)(RED_OFF + RD * NW * MT * 64) + (KS > 1 && MT > 1 ? (uint32_t)(xch_slots(MT) * (KS - 1) * MT * 64) : 0u);
+    const uint32_t xs_off = (uint32_t)(RED_OFF + RD * NW * MT * 64) + (KS > 1 && MT > 1 ? (uint32_t)(xch_slots(MT) * (KS - 1) * PP * MT * 64) : 0u);
     uint8_t* xs0 = smem + xs_off;           // [MT][bpr][128] f16 activations
     const uint32_t XS = (uint32_t)bpr * XB;  // bytes of one activation row
     float* xinv0 = (float*)(xs0 + (size_t)MT * XS);  // [MT][bpr]
@@ -358,6 +363,26 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
         for (int ps = 0; ps < NP; ps++)
 #pragma unroll
             for (int q = 0; q < 4; q++) pk0[ps][q] = pk1[ps][q] = 0.0f;
+        // PP > 1: which of the eight sums of the part in hand this warp holds, and the group, counted from the chunk in hand, that
+        // ends the part. Groups go to the warps round robin over the whole row, so that the warps stay level; counted from a later
+        // part's start, as where that part has a CTA of its own, they belong to another of the eight sums.
+        [[maybe_unused]] const int gpp = bpr / PP / 2;  // groups of a part
+        [[maybe_unused]] int sum = warp, pend = gpp;
+        [[maybe_unused]] const int rfirst = rslot;
+        [[maybe_unused]] const uint32_t pfirst = rpar;
+        // several rows: this warp's sums, as number `sum` of the eight
+        auto post_rows = [&](float* rb, int sum) {
+#pragma unroll
+            for (int ps = 0; ps < NP; ps++) {
+                const int m = ps * 4 + t;
+                if (m < MT) {
+                    rb[(sum * MT + m) * 16 + g] = (pk0[ps][0] + pk0[ps][1]) + (pk0[ps][2] + pk0[ps][3]);
+                    rb[(sum * MT + m) * 16 + g + 8] = (pk1[ps][0] + pk1[ps][1]) + (pk1[ps][2] + pk1[ps][3]);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tbar[rslot]);
+        };
         for (int c = 0; c < nch; c++) {
             const int ng = min(TX, bpr - c * TX) >> 1;  // groups of two blocks in this chunk
             if (!mbar_wait(&full[s], par)) {
@@ -438,13 +463,35 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                         }
                     }
                 };
-                if (ng == TX / 2) {
+                if (ng == TX / 2 && (PP == 1 || pend > TX / 2)) {
 #pragma unroll
                     for (int j = 0; j < GPW; j++) group(j);
-                } else {
+                    if (PP > 1) pend -= TX / 2;
+                } else if constexpr (PP == 1) {
 #pragma unroll
                     for (int j = 0; j < GPW; j++)
                         if (warp + NW * j < ng) group(j);
+                } else {
+                    // the part ends inside the chunk or with it (every part is longer than a chunk): its groups, then those of the next
+                    for (int lo = 0;;) {
+                        const int hi = min(ng, pend);
+#pragma unroll 1
+                        for (int j = 0; j < GPW; j++)
+                            if (warp + NW * j >= lo && warp + NW * j < hi) group(j);
+                        if (hi == pend) {
+                            post_rows(red + rslot * (NW * MT * 16), sum);
+                            if (++rslot == RD) rslot = 0, rpar ^= 1u;
+#pragma unroll
+                            for (int ps = 0; ps < NP; ps++)
+#pragma unroll
+                                for (int q = 0; q < 4; q++) pk0[ps][q] = pk1[ps][q] = 0.0f;
+                            sum = (sum - gpp) & (NW - 1);
+                            pend += gpp;
+                        }
+                        if (hi == ng) break;
+                        lo = hi;
+                    }
+                    pend -= TX / 2;
                 }
             }
             __syncwarp();
@@ -468,18 +515,65 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                 rb[warp * 16 + g] = a;
                 rb[warp * 16 + g + 8] = b;
             }
-        } else {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tbar[rslot]);
+        } else if constexpr (PP == 1) {
+            post_rows(rb, warp);
+        }
+        if constexpr (PP > 1) {
+            // the parts posted since the tile's start, in order; as for one row below, lane l over (activation row, row slot)
+            // pairs l, l + 32, ...
+            constexpr int NO = MT > 1 ? MT / 2 : 1;
+            float* xch = (float*)(smem + xch_off);
+            uint64_t* xb = (uint64_t*)(smem + XBAR_OFF);
+            float tot[NO];
+            const bool mine = warp == (titer & (NW - 1));  // the warps take turns
 #pragma unroll
-            for (int ps = 0; ps < NP; ps++) {
-                const int m = ps * 4 + t;
-                if (m < MT) {
-                    rb[(warp * MT + m) * 16 + g] = (pk0[ps][0] + pk0[ps][1]) + (pk0[ps][2] + pk0[ps][3]);
-                    rb[(warp * MT + m) * 16 + g + 8] = (pk1[ps][0] + pk1[ps][1]) + (pk1[ps][2] + pk1[ps][3]);
+            for (int pt = 0; pt < PP && mine && ok; pt++) {
+                const int sl = rfirst + pt < RD ? rfirst + pt : rfirst + pt - RD;
+                if (!mbar_wait(&tbar[sl], rfirst + pt < RD ? pfirst : pfirst ^ 1u)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                    break;
+                }
+                const float* q = red + sl * (NW * MT * 16);
+#pragma unroll
+                for (int i = 0; i < NO; i++) {
+                    const int o = lane + 32 * i;
+                    float v = q[o];
+                    for (int w = 1; w < NW; w++) v += q[w * MT * 16 + o];
+                    if (crank != 0)
+                        st_peer_f32(peer_addr(xch + ((crank - 1) * PP + pt) * MT * 16 + o, 0), v);
+                    else
+                        tot[i] = pt == 0 ? v : tot[i] + v;
                 }
             }
+            if (mine && ok && crank != 0) {
+                __syncwarp();
+                if (lane == 0) arrive_peer(peer_addr(xb, 0));
+            } else if (mine && ok) {
+                if (KS > 1 && !mbar_wait_cluster(xb, 0)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NO; i++) {
+                        const int o = lane + 32 * i, m = o >> 4, slot = o & 15;
+                        for (int c = 0; c < (KS - 1) * PP; c++) tot[i] += xch[c * MT * 16 + o];
+                        const float up = __shfl_down_sync(0xffffffffu, tot[i], 8);
+                        const int row = tile * per_cta + slot;
+                        const float r = gu ? act_gu(tot[i], up, p.limit) : tot[i];
+                        if (slot < per_cta && row < p.rows && m < p.m) {
+                            if (p.out_f32)
+                                ((float*)ybase)[(size_t)m * p.ldy + row] = r;
+                            else
+                                ((__nv_bfloat16*)ybase)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(r);
+                        }
+                    }
+                }
+            }
+            continue;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tbar[rslot]);
         if (warp == 0) {
             if (!mbar_wait(&tbar[rslot], rpar)) {
                 cn_dev_fail(CN_DEV_WAIT_FULL);
@@ -494,8 +588,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                     v[i] = rb[o];
                     for (int w = 1; w < NW; w++) v[i] += rb[w * MT * 16 + o];
                 }
-                float* xch = (float*)(smem + xch_off) + titer * (KS - 1) * MT * 16;
-                uint64_t* xb = (uint64_t*)(smem + XBAR_OFF) + titer;
+                float* xch = (float*)(smem + xch_off);
+                uint64_t* xb = (uint64_t*)(smem + XBAR_OFF);
                 if (crank != 0) {
 #pragma unroll
                     for (int i = 0; i < NO; i++) st_peer_f32(peer_addr(xch + (crank - 1) * MT * 16 + lane + 32 * i, 0), v[i]);
@@ -595,11 +689,56 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     if (KS > 1) cluster_sync_all();  // nobody leaves while a CTA of the cluster may still send or receive
 }
 
-template <int TX, int CPS, int MT, int KS = 1, bool LN = false>
+template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1>
 int launch_m1(const cudaLaunchConfig_t& cfg, const GemvParams& p) {
-    CN_ALLOW_SMEM((nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN>), 226 * 1024);
-    CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN>, p));
+    CN_ALLOW_SMEM((nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP>), 226 * 1024);
+    CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP>, p));
     return CN_OK;
+}
+
+// Slots for the sums of a tile's n parts. Warp 0 reads them at the tile's end; another warp is at most `stages` chunks beyond that end
+// then, and the parts that it has posted there end at least `gap` chunks apart: n + stages / gap, and one to spare.
+int red_slots(int stages, int gap, int n) { return n + stages / gap + 1 < RED_DEPTH ? n + stages / gap + 1 : RED_DEPTH; }
+static_assert(4 + MAX_STAGES <= RED_DEPTH, "slots of the tile sums");
+// Shared memory of a CTA in front of its weight ring: header, those sums, the ones handed over inside a cluster, activations.
+long long front_bytes(int stages, int gap, int n, int mt, int bpr, int handed) {
+    return (long long)RED_OFF + (long long)(red_slots(stages, gap, n) * NW + handed) * mt * 64 + (long long)mt * bpr * XB + (long long)((mt * bpr + 3) & ~3) * 4;
+}
+long long sm_share(int cps) { return (227 * 1024) / cps - 1024; }
+long long stage_bytes_of(int tx) { return (long long)ROWS * (tx * 36 + 16); }
+// CTAs per SM for mt rows: as many (up to 4 for one row, 2 for more) as leave every CTA a ring of at least three stages
+int ctas_per_sm(int gap, int n, int mt, int bpr, int tx) {
+    int c = mt == 1 ? 4 : 2;
+    while (c > (mt == 1 ? 2 : 1) && sm_share(c) - front_bytes(3, gap, n, mt, bpr, 0) < 3 * stage_bytes_of(tx)) c--;
+    return c;
+}
+
+// How the one-row call of a matrix is launched: parts of K, which is CTAs per cluster, and CTAs per SM. The parts, a rule of the matrix
+// alone, fix the order of every row's sum whatever the number of activation rows.
+// Clusters of two or four CTAs can share every tile, each CTA over its part of K, the others handing their 16 sums to
+// the first through distributed shared memory: the wave quantum drops from a tile to a half or a quarter, and a
+// matrix of few, long rows (a tensor-parallel rank's share of a down projection) gets CTAs enough to stream it.
+// Taken when it shortens the longest CTA by a tenth or more and either the machine is not filled otherwise or a CTA's
+// share stays long enough to hide the hand-over (measured on full machines: 235 KB yes, 69 KB no).
+struct Split {
+    int parts, cps;
+};
+Split one_row_split(int ntiles, int bpr, int tx) {
+    const int cps = ctas_per_sm((bpr + tx - 1) / tx, 1, 1, bpr, tx);
+    Split r = {1, cps};
+    if (tx != 32) return r;
+    double best = (double)((ntiles + 148 * cps - 1) / (148 * cps));  // tiles per CTA without a split
+    for (int ks = 2; ks <= 4; ks *= 2) {
+        if (bpr % (4 * ks) != 0) continue;  // every part starts on a 16-byte boundary of the row
+        const int bk = bpr / ks, ck = sm_share(3) - front_bytes(3, (bk + tx - 1) / tx, 1, 1, bk, 0) >= 3 * stage_bytes_of(tx) ? 3 : 2;
+        const int clusters = 148 * ck / ks, waves = (ntiles + clusters - 1) / clusters;
+        const long long share = (long long)waves * ROWS * bk * 36;
+        const bool underfilled = (long long)ntiles * ks <= 148LL * ck;
+        if (waves > XCH_SLOTS || share < 32 * 1024 || !(underfilled || share >= 160 * 1024)) continue;
+        const double t = (double)waves / ks;
+        if (t <= 0.9 * best) best = t, r = {ks, ck};
+    }
+    return r;
 }
 
 }  // namespace
@@ -620,23 +759,15 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // blocks per row and stage: the same rule for every row count, so that row i of an m-row call is summed in the
     // order of a one-row call
     const int tx = bpr >= 32 ? 32 : 16;
-    const int pstride = tx * 36 + 16;
-    const size_t stage_bytes = (size_t)ROWS * pstride;
-    const size_t xbytes = (size_t)mt * bpr * XB + (size_t)((mt * bpr + 3) & ~3) * 4;
+    const long long stage_bytes = stage_bytes_of(tx);
     const int per_cta = gu ? ROWS / 2 : ROWS;
     const int ntiles = (rows + per_cta - 1) / per_cta;
-    int nch = (bpr + tx - 1) / tx;
-    // fixed part of a CTA's shared memory for a ring of `st` stages: header, tile-sum slots (a warp runs at most
-    // `st` chunks ahead of warp 0, i.e. st / nch + 1 tiles), activations
-    auto fixed = [&](int st) { return (long long)RED_OFF + (long long)((st + nch) / nch + 1) * NW * mt * 64 + (long long)xbytes; };
-    // CTAs per SM: as many (up to 4 for one row, 2 for more) as leave every CTA a ring of at least three stages
-    int cps = 1;
-    for (int c = mt == 1 ? 4 : 2; c > 1; c--)
-        if ((227 * 1024) / c - 1024 - fixed(3) >= 3 * (long long)stage_bytes) {
-            cps = c;
-            break;
-        }
-    if (mt == 1 && cps < 2) cps = 2;
+    Split one = {1, 0};
+    if (!routed) one = one_row_split(ntiles, bpr, tx);
+    const int parts = one.parts, bpp = bpr / parts;  // parts of K (each longer than a chunk where there are several), blocks of one
+    // chunks from one part's end to the next where a CTA has n of them: a row is cut into whole chunks from its first part's start
+    auto gap = [&](int n) { return n > 1 ? bpp / tx : (bpp + tx - 1) / tx; };
+    int cps = mt == 1 && !routed ? one.cps : ctas_per_sm(gap(parts), parts, mt, bpr, tx);
     // persistent CTAs, each walking its share of the tiles (the routed form keeps one tile per CTA)
     int grid = ntiles;
     if (!routed && grid > 148 * cps) grid = 148 * cps;
@@ -655,54 +786,34 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         }
         grid = (ntiles + ((ntiles + grid - 1) / grid) - 1) / ((ntiles + grid - 1) / grid);  // the same tiles per CTA, fewer CTAs
     }
-    // Clusters of two or four CTAs can share every tile, each CTA over its part of K, the others handing their 16 sums to
-    // the first through distributed shared memory: the wave quantum drops from a tile to a half or a quarter, and a
-    // matrix of few, long rows (a tensor-parallel rank's share of a down projection) gets CTAs enough to stream it.
-    // Taken when it shortens the longest CTA by a tenth or more and either the machine is not filled otherwise or a CTA's
-    // share stays long enough to hide the hand-over (measured on full machines: 235 KB yes, 69 KB no).
-    // Two and more activation rows take it only where the machine is not filled otherwise: 640 x 17408 with 2 / 4 / 8 rows 9.6 / 13.3 /
-    // 26.1 -> 6.8 / 8.1 / 15.1 us, but 5120 x 17408 22.0 / 27.0 / 53.4 -> 29.2 / 32.7 / 59.8 (warp 0 of a cluster's first CTA waits for
-    // the others' sums of every tile, and has four times the sums to add).
-    int ksplit = 1;
-    size_t xbytes_l = xbytes;
-    if (!routed && tx == 32) {
-        double best = (double)((ntiles + 148 * cps - 1) / (148 * cps)) * (mt == 1 ? 1 : cps);  // tiles per CTA (of an SM) without a split
-        if (mt > 1 && cps == 1) best *= 1.5;  // one CTA's eight warps alone do not keep an SM busy
-        int best_cps = cps;
-        for (int ks = 2; ks <= 4; ks *= 2) {
-            if (bpr % (4 * ks) != 0) continue;  // every part starts on a 16-byte boundary of the row
-            const int bk = bpr / ks, nchk = (bk + tx - 1) / tx;
-            const long long xk = (long long)mt * bk * XB + (long long)((mt * bk + 3) & ~3) * 4 + (mt > 1 ? (long long)xch_slots(mt) * (ks - 1) * mt * 64 : 0);
-            auto fits = [&](int c) {
-                return (227 * 1024) / c - 1024 - ((long long)RED_OFF + (long long)((3 + nchk) / nchk + 1) * NW * mt * 64 + xk) >= 3 * (long long)stage_bytes;
-            };
-            const int ck = mt == 1 ? (fits(3) ? 3 : 2) : (fits(2) ? 2 : 1);
-            if (mt > 1 && !fits(ck)) continue;
-            const int clusters = 148 * ck / ks;
-            const int waves = (ntiles + clusters - 1) / clusters;
-            const long long share = (long long)waves * ROWS * bk * 36;
-            const bool underfilled = (long long)ntiles * ks <= 148LL * ck;
-            if (waves > xch_slots(mt) || share < 32 * 1024 || !(underfilled || (mt == 1 && share >= 160 * 1024))) continue;
-            const double t = mt == 1 ? (double)waves / ks : (double)waves * ck / ks * (ck == 1 ? 1.5 : 1.0);
-            if (t <= 0.9 * best) best = t, ksplit = ks, best_cps = ck, xbytes_l = (size_t)xk;
-        }
-        if (ksplit > 1) {
-            cps = best_cps;
-            const int clusters = 148 * cps / ksplit;
-            grid = ksplit * (ntiles < clusters ? ntiles : clusters);
-            nch = (bpr / ksplit + tx - 1) / tx;
+    // CTAs per cluster: one row takes a CTA for every part. Two and more activation rows share a tile only where the machine is not filled
+    // otherwise: 640 x 17408 with 2 / 4 / 8 rows 9.6 / 13.3 / 26.1 -> 6.8 / 8.1 / 15.1 us, but 5120 x 17408 22.0 / 27.0 / 53.4 ->
+    // 29.2 / 32.7 / 59.8 (warp 0 of a cluster's first CTA waits for the others' sums of every tile, and has four times the sums to add). There a
+    // CTA takes the parts one after another.
+    int ksplit = mt == 1 ? parts : 1;
+    if (mt > 1) {
+        double best = (double)((ntiles + 148 * cps - 1) / (148 * cps)) * cps * (cps == 1 ? 1.5 : 1.0);  // tiles of an SM; one CTA's eight warps alone do not keep it busy
+        for (int ks = 2; ks <= parts; ks *= 2) {
+            auto fits = [&](int c) { return sm_share(c) - front_bytes(3, gap(parts / ks), parts / ks, mt, bpr / ks, parts - parts / ks) >= 3 * stage_bytes; };
+            const int ck = fits(2) ? 2 : 1;
+            if (!fits(ck) || (long long)ntiles * ks > 148LL * ck || (long long)ROWS * (bpr / ks) * 36 < 32 * 1024) continue;
+            const double t = (double)ck / ks * (ck == 1 ? 1.5 : 1.0);
+            if (t <= 0.9 * best) best = t, ksplit = ks, cps = ck;
         }
     }
-    auto fixed2 = [&](int st) { return (long long)RED_OFF + (long long)((st + nch) / nch + 1) * NW * mt * 64 + (long long)xbytes_l; };
+    if (ksplit > 1) {
+        const int clusters = 148 * cps / ksplit;
+        grid = ksplit * (ntiles < clusters ? ntiles : clusters);
+    }
+    const int pp = parts / ksplit;  // parts of a CTA
+    auto front = [&](int st) { return front_bytes(st, gap(pp), pp, mt, bpr / ksplit, mt > 1 ? parts - pp : 0); };
     int fit = MAX_STAGES;  // ring depth that fits beside the fixed part
-    while (fit > 1 && fixed2(fit) + (long long)fit * (long long)stage_bytes > (227 * 1024) / cps - 1024) fit--;
+    while (fit > 1 && front(fit) + fit * stage_bytes > sm_share(cps)) fit--;
     int stages = fit;
-    const int total_chunks = nch * ((ntiles + grid / ksplit - 1) / (grid / ksplit));
+    const int total_chunks = ((pp * bpp + tx - 1) / tx) * ((ntiles + grid / ksplit - 1) / (grid / ksplit));
     if (stages > total_chunks) stages = total_chunks;
     if (stages < 1) stages = 1;
-    int red_depth = (stages + nch) / nch + 1;
-    if (red_depth > RED_DEPTH) red_depth = RED_DEPTH;
-    const size_t smem = (size_t)RED_OFF + (size_t)red_depth * NW * mt * 64 + xbytes_l + stages * stage_bytes;
+    const size_t smem = (size_t)(front(stages) + stages * stage_bytes);
     if (smem > 226 * 1024 || fit < 2) {
         // the staged activations of all m rows do not fit beside a ring: two calls over half the rows each
         if (m == 1) CN_FAIL(CN_ERR_LIMIT, "%s: k = %d needs %zu B of shared memory per block", who, k, smem);
@@ -718,8 +829,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = a.x, p.y = a.y;
     p.rows = rows, p.k = k, p.m = m, p.ldy = a.ldy, p.limit = a.limit, p.tx = tx, p.stages = stages, p.out_f32 = a.out_f32;
     p.ids = a.ids, p.order = a.order, p.tab0 = a.tab0, p.tab1 = a.tab1, p.fused_up_rows = a.fused_up_rows, p.x_div = a.x_div;
-    p.red_depth = red_depth;
-    p.ksplit = ksplit;
+    p.red_depth = red_slots(stages, gap(pp), pp);
     p.experts = a.experts, p.yptrs = a.yptrs;
     p.yl_world = 0, p.yl_row0 = 0, p.yl_stride = 0, p.yl_epoch = nullptr, p.yl_tag = 0, p.yl_buf = 0, p.yl_flip = 0;
     for (int d = 0; d < 8; d++) p.yl[d] = 0ull;
@@ -745,6 +855,13 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+#define CN_M1_PARTS(KSV, PPV)                                                                                        \
+    if (mt > 1 && ksplit == KSV && pp == PPV) {                                                                      \
+        if (mt == 2) return cps == 2 ? launch_m1<32, 2, 2, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 2, KSV, false, PPV>(cfg, p); \
+        if (mt == 4) return cps == 2 ? launch_m1<32, 2, 4, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 4, KSV, false, PPV>(cfg, p); \
+        return cps == 2 ? launch_m1<32, 2, 8, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p);              \
+    }
+    CN_M1_PARTS(1, 2) CN_M1_PARTS(1, 4)
     if (ksplit > 1) {
         at[1].id = cudaLaunchAttributeClusterDimension;
         at[1].val.clusterDim.x = (unsigned)ksplit, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
@@ -753,11 +870,8 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
             if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2, true>(cfg, p) : launch_m1<32, 3, 1, 2, true>(cfg, p);
             return cps == 2 ? launch_m1<32, 2, 1, 4, true>(cfg, p) : launch_m1<32, 3, 1, 4, true>(cfg, p);
         }
-#define CN_M1_SPLIT(CPSV, MTV, KSV) \
-    if (cps == CPSV && mt == MTV && ksplit == KSV) return launch_m1<32, CPSV, MTV, KSV>(cfg, p);
-        CN_M1_SPLIT(1, 2, 2) CN_M1_SPLIT(1, 2, 4) CN_M1_SPLIT(2, 2, 2) CN_M1_SPLIT(2, 2, 4) CN_M1_SPLIT(1, 4, 2) CN_M1_SPLIT(1, 4, 4)
-        CN_M1_SPLIT(2, 4, 2) CN_M1_SPLIT(2, 4, 4) CN_M1_SPLIT(1, 8, 2) CN_M1_SPLIT(1, 8, 4) CN_M1_SPLIT(2, 8, 2) CN_M1_SPLIT(2, 8, 4)
-#undef CN_M1_SPLIT
+        CN_M1_PARTS(2, 1) CN_M1_PARTS(2, 2) CN_M1_PARTS(4, 1)
+#undef CN_M1_PARTS
         if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2>(cfg, p) : launch_m1<32, 3, 1, 2>(cfg, p);
         return cps == 2 ? launch_m1<32, 2, 1, 4>(cfg, p) : launch_m1<32, 3, 1, 4>(cfg, p);
     }
