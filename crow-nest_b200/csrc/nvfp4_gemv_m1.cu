@@ -786,19 +786,24 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         }
         grid = (ntiles + ((ntiles + grid - 1) / grid) - 1) / ((ntiles + grid - 1) / grid);  // the same tiles per CTA, fewer CTAs
     }
-    // CTAs per cluster: one row takes a CTA for every part. Two and more activation rows share a tile only where the machine is not filled
-    // otherwise: 640 x 17408 with 2 / 4 / 8 rows 9.6 / 13.3 / 26.1 -> 6.8 / 8.1 / 15.1 us, but 5120 x 17408 22.0 / 27.0 / 53.4 ->
-    // 29.2 / 32.7 / 59.8 (warp 0 of a cluster's first CTA waits for the others' sums of every tile, and has four times the sums to add). There a
-    // CTA takes the parts one after another.
+    // CTAs per cluster: one row takes a CTA for every part. With two and more activation rows the parts of a tile go to the CTAs of a
+    // cluster where the machine is not filled otherwise and that shortens the busiest SM, else to one CTA after another. Its time in
+    // blocks: the tiles or parts that it holds, half as much again where a single CTA's eight warps are all it has (two rows; from
+    // four rows on they nearly keep the issue slots busy: a fifth), and 24 for meeting in the first CTA. Measured, us alone /
+    // shared: 2048 x 8192 with two rows 8.2 / 6.9, with four 7.6 / 8.7; 640 x 17408 with two, four and eight rows 10.8 / 6.8 (four CTAs),
+    // 14.0 / 8.3 (four; 10.5 with two), 27.8 / 15.9 (two); 1000 x 9216 7.0 / 6.0, 8.1 / 7.1, 12.4 / 10.1.
     int ksplit = mt == 1 ? parts : 1;
     if (mt > 1) {
-        double best = (double)((ntiles + 148 * cps - 1) / (148 * cps)) * cps * (cps == 1 ? 1.5 : 1.0);  // tiles of an SM; one CTA's eight warps alone do not keep it busy
+        const double alone = mt == 2 ? 1.5 : 1.2;
+        auto busiest = [&](int ks) {
+            const int n = (int)(((long long)ntiles * ks + 147) / 148);
+            return n * (double)(bpr / ks) * (n == 1 ? alone : 1.0) + (ks > 1 ? 24.0 : 0.0);
+        };
         for (int ks = 2; ks <= parts; ks *= 2) {
             auto fits = [&](int c) { return sm_share(c) - front_bytes(3, gap(parts / ks), parts / ks, mt, bpr / ks, parts - parts / ks) >= 3 * stage_bytes; };
             const int ck = fits(2) ? 2 : 1;
             if (!fits(ck) || (long long)ntiles * ks > 148LL * ck || (long long)ROWS * (bpr / ks) * 36 < 32 * 1024) continue;
-            const double t = (double)ck / ks * (ck == 1 ? 1.5 : 1.0);
-            if (t <= 0.9 * best) best = t, ksplit = ks, cps = ck;
+            if (busiest(ks) <= 0.9 * busiest(ksplit)) ksplit = ks, cps = ck;
         }
     }
     if (ksplit > 1) {
