@@ -128,7 +128,13 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
         int done = 0;
         bool ok = true;
         for (int tile = t0 + warp; tile < t1 && ok; tile += NW) {
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            // bf16 rows: a running sum for each block of a chunk, eight in all. With a single one the rounding of k / 64 additions in a row
+            // made the results of gate / up less exact than one row's of nvfp4_gemv_m1.cu (relative error against 64 bits, k = 2048 / 4096:
+            // 1.5e-7 / 2.1e-7, there 1.3e-7 / 1.4e-7). f32 rows need one: their first plane lies on a grid and its sums hardly round.
+            constexpr int NA = NPL == 1 ? CB : 1;
+            float acc[NA][4];
+#pragma unroll
+            for (int i = 0; i < NA; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
             for (int ch = 0; ch < nch; ch++) {
                 if (!mbar_wait(&full[s], par)) {
                     cn_dev_fail(CN_DEV_WAIT_FULL);
@@ -154,14 +160,17 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
                         mma16816(cc, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
                     }
                     const float2 xi = lds64f(xic + b * 32u);
-                    acc[0] = fmaf(cc[0], xi.x, acc[0]);
-                    acc[1] = fmaf(cc[1], xi.y, acc[1]);
-                    acc[2] = fmaf(cc[2], xi.x, acc[2]);
-                    acc[3] = fmaf(cc[3], xi.y, acc[3]);
+                    float* a = acc[NA > 1 ? b : 0];
+                    a[0] = fmaf(cc[0], xi.x, a[0]);
+                    a[1] = fmaf(cc[1], xi.y, a[1]);
+                    a[2] = fmaf(cc[2], xi.x, a[2]);
+                    a[3] = fmaf(cc[3], xi.y, a[3]);
                 };
                 if (nb == CB) {
 #pragma unroll
                     for (int b = 0; b < CB; b++) block(b);
+                } else if constexpr (NA > 1) {
+                    block(0), block(1), block(2), block(3);  // nb is 4: k is a multiple of 256
                 } else {
                     for (int b = 0; b < nb; b++) block(b);
                 }
@@ -170,18 +179,24 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
                 if (++s == D) s = 0, par ^= 1u;
             }
             if (!ok) break;
+#pragma unroll
+            for (int n = NA / 2; n > 0; n /= 2)
+#pragma unroll
+                for (int i = 0; i < n; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] += acc[i + n][j];
             // lane (g, t): row slots g and g + 8, columns 2 t and 2 t + 1
             float v[2][2];  // [row slot][activation row of this lane]
             int r0;
             if constexpr (NPL == 1) {
-                v[0][0] = acc[0], v[0][1] = acc[1], v[1][0] = acc[2], v[1][1] = acc[3];
+                v[0][0] = acc[0][0], v[0][1] = acc[0][1], v[1][0] = acc[0][2], v[1][1] = acc[0][3];
                 r0 = 2 * t;
             } else {
                 // columns 0-2 are the planes of row 0, 3-5 those of row 1: lane t = 0 ends up with row 0, lane t = 1 with row 1
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    const float na = __shfl_down_sync(0xffffffffu, acc[2 * i], 1), nb = __shfl_down_sync(0xffffffffu, acc[2 * i + 1], 1);
-                    v[i][0] = t == 0 ? fmaf(na, 0x1p-22f, fmaf(acc[2 * i + 1], 0x1p-11f, acc[2 * i])) : fmaf(nb, 0x1p-22f, fmaf(na, 0x1p-11f, acc[2 * i + 1]));
+                    const float na = __shfl_down_sync(0xffffffffu, acc[0][2 * i], 1), nb = __shfl_down_sync(0xffffffffu, acc[0][2 * i + 1], 1);
+                    v[i][0] = t == 0 ? fmaf(na, 0x1p-22f, fmaf(acc[0][2 * i + 1], 0x1p-11f, acc[0][2 * i])) : fmaf(nb, 0x1p-22f, fmaf(na, 0x1p-11f, acc[0][2 * i + 1]));
                 }
                 r0 = t;
             }
