@@ -379,8 +379,12 @@ extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void
         CN_CUDA(cudaGetLastError());
     }
     if (pair) {
+        // results may take the place of the activations: bf16 rows are then read from a copy (every row tile reads them again)
+        const size_t xbytes = (size_t)m * k * 2, ybytes = ((size_t)(m - 1) * ldy + rows) * 2;
+        const bool aside = dtype == CN_BF16 && (uintptr_t)x < (uintptr_t)y + ybytes && (uintptr_t)y < (uintptr_t)x + xbytes;
+        if (aside) CN_CUDA(cudaMemcpyAsync(xh, x, xbytes, cudaMemcpyDeviceToDevice, stream));
         GemmCall c = {};
-        c.w = w, c.gs = gs, c.x_f16 = dtype != CN_BF16, c.x = c.x_f16 ? (const void*)xh : x, c.rs = rs, c.y = y;
+        c.w = w, c.gs = gs, c.x_f16 = dtype != CN_BF16, c.x = c.x_f16 || aside ? (const void*)xh : x, c.rs = rs, c.y = y;
         c.rows = rows, c.k = k, c.m = m, c.ldy = ldy;
         return cn_gemm_pair_launch(c, stream);
     }

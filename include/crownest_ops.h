@@ -207,8 +207,9 @@ int cn_moe_nvfp4_finish(void* plan, const void* shared_gate, const void* shared_
  * cn_nvfp4_gemv streams the weights once and is faster), on tcgen05 tensor cores with the accumulator in
  * tensor memory. Replaces gemm_fp4_dense (engine/src/kernels.rs:533, launched by launch_mma_d,
  * engine/src/gen.rs:2491) and glm5_gemm_fp4_tc (engine/src/kernels_glm5_moe.cu:349), with the latter's
- * arithmetic: weights widened losslessly to f16 (code x block scale), activations as f16 x 2^k per row,
- * exact products, f32 accumulation. w is the container layout, unchanged. The call allocates nothing:
+ * arithmetic: weights widened losslessly (code x block scale), exact products, f32 accumulation. Up to 128 rows, and f32 rows always,
+ * the activations go in as f16 x 2^k per row; more than 128 rows of bf16 as they are, without a pass over them. w is the container
+ * layout, unchanged. y may overlap x (bf16 rows beyond 128 are copied to the workspace first then). The call allocates nothing:
  * `workspace` (device, 256-byte aligned) holds the widened activations and must be at least
  * cn_nvfp4_gemm_workspace_bytes(k, m) bytes; it may be reused by the next call on the same stream. */
 size_t cn_nvfp4_gemm_workspace_bytes(int k, int m);

@@ -46,3 +46,20 @@ def test_rows_of_any_magnitude(m):
     # one rounding of the result to bf16 (2^-9 at most) beside f32 sums
     assert err.max().item() <= 2.0 ** -9 + 4e-6
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,k,at", [(2048, 2048, 4096), (4096, 2048, 1024), (1024, 2048, 7096)])
+def test_results_in_the_place_of_the_activations(rows, k, at, dtype):
+    """More tiles than CTA pairs, so that late tiles read activations after early ones have written; y starts on, before and inside x."""
+    m = 4096
+    rng = np.random.default_rng(rows)
+    w = ops.Fp4.from_host(synth.nvfp4_matrix(rows, k, rng), rows, k, np.float32(1.0))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda().to(dtype)
+    want = ops.launch_gemm(w, x)
+    buf = torch.empty(2 * m * max(rows, k) + 8192, dtype=dtype, device="cuda")
+    xs, ys = buf[4096:4096 + m * k].view(m, k), buf[at:at + m * rows].view(m, rows)
+    xs.copy_(x)
+    ops.launch_gemm(w, xs, ys)
+    assert torch.equal(ys, want)
+    assert device_status() == 0
