@@ -1,4 +1,4 @@
-// NVFP4 GEMM for M >= 9 activation rows (prefill / batched verify): Y[t][n] = gs * sum_k X[t][k] * W[n][k],
+// NVFP4 GEMM for up to 128 activation rows (batched verify, short prompts; more rows: nvfp4_gemm_pair.cu): Y[t][n] = gs * sum_k X[t][k] * W[n][k],
 // on the fifth-generation tensor cores: tcgen05.mma (kind::f16) with the accumulator in tensor memory.
 //
 // Supersedes the reference's prompt GEMMs gemm_fp4_dense (engine/src/kernels.rs:533) and
@@ -12,8 +12,7 @@
 // maximum. Products are exact in the tensor core, accumulation is f32 in tensor memory, the epilogue
 // multiplies by gs * 2^-k once.
 //
-// One CTA = 128 weight rows x TN activation rows (128, or 256 when more than 128 rows are given), K walked
-// 64 at a time through a 3- or 4-stage ring:
+// One CTA = 128 weight rows x TN = 128 activation rows, K walked 64 at a time through a three-stage ring, two CTAs per SM:
 //   warps 0-7   A producers: thread (r, h) owns half of weight row r's 36-byte block per step (prefetched three
 //               steps ahead), cvt.rn.f16x2.e2m1x2 + one HMUL2 per pair, four 16-byte stores into the canonical
 //               K-major 128-byte-swizzle tile (row r at r * 128, chunk c at c ^ (r & 7));
@@ -30,16 +29,14 @@
 
 namespace {
 
-constexpr int TM = 128, TK = 64;
-constexpr int A_BYTES = TM * 128;
+constexpr int TM = 128, TN = 128, TK = 64;
+constexpr int STAGES = 3;
+constexpr int A_BYTES = TM * 128, B_BYTES = TN * 128;
 constexpr int A_WARPS = 8, B_WARPS = 4;  // producers; one more warp issues the MMAs
 constexpr int GEMM_THREADS = (A_WARPS + B_WARPS + 1) * 32;
-// TN activation rows per CTA: 128 (3 stages, two CTAs per SM) or 256 (4 stages, one CTA per SM, half the weight
-// decoding per MMA)
-__host__ __device__ constexpr int stages_of(int tn) { return tn == 256 ? 4 : 3; }
-__host__ __device__ constexpr int smem_of(int tn) { return 2048 + stages_of(tn) * (A_BYTES + tn * 128) + 1024; }  // header (barriers, scale table) + ring + alignment slack
+constexpr int GEMM_SMEM = 2048 + STAGES * (A_BYTES + B_BYTES) + 1024;  // header (barriers, scale table) + ring + alignment slack
 // instruction descriptor, kind::f16: D f32 (bit 4), A and B f16 K-major (0), N >> 3 at bit 17, M >> 4 at bit 24
-__host__ __device__ constexpr uint32_t idesc_of(int tn) { return (1u << 4) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(TM >> 4) << 24); }
+constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -114,16 +111,12 @@ struct GemmParams {
     const float* rs;
     void* y;
     int rows, k, m, ldy, out_bf16;
-    // K shared between `ksplits` CTAs of a tile (blockIdx.y, when m <= 128 and the row tiles alone do not fill the
-    // machine): each writes its raw f32 sums to part[split][m][rows], a second kernel adds them in split order
+    // K shared between `ksplits` CTAs of a tile (blockIdx.y, when the row tiles alone do not fill the machine): each writes its raw f32 sums to part[split][m][rows], a second kernel adds them in split order
     int ksplits;
     float* part;
 };
 
-template <int TN>
-__global__ void __launch_bounds__(GEMM_THREADS, TN == 256 ? 1 : 2) nvfp4_gemm_tc5_kernel(const GemmParams p) {
-    constexpr int STAGES = stages_of(TN), B_BYTES = TN * 128;
-    constexpr uint32_t IDESC = idesc_of(TN);
+__global__ void __launch_bounds__(GEMM_THREADS, 2) nvfp4_gemm_tc5_kernel(const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     // header in the first 1024 bytes as the runtime gives them; the ring starts at the next 1024-byte boundary
     uint64_t* full = (uint64_t*)smem_raw;
@@ -136,8 +129,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, TN == 256 ? 1 : 2) nvfp4_gemm_tc
     uint8_t* ring = smem_raw + (ring_addr - smem_u32(smem_raw));
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int KSP = p.ksplits, ksi = KSP > 1 ? (int)blockIdx.y : 0;
-    const int row0 = blockIdx.x * TM, tok0 = KSP > 1 ? 0 : (int)blockIdx.y * TN;
+    const int KSP = p.ksplits, ksi = (int)blockIdx.y;
+    const int row0 = blockIdx.x * TM;
     const int bpr_all = p.k >> 6;
     const int kbeg = (int)((long long)bpr_all * ksi / KSP), bpr = (int)((long long)bpr_all * (ksi + 1) / KSP) - kbeg;  // this CTA's blocks
     const size_t row_bytes = (size_t)bpr_all * 36;
@@ -249,8 +242,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, TN == 256 ? 1 : 2) nvfp4_gemm_tc
             // eight consecutive lanes copy the eight 16-byte chunks of one activation row: whole 128-byte lines per request
 #pragma unroll
             for (int it = 0; it < TN * 8 / (B_WARPS * 32); it++) {
-                const int idx = it * (B_WARPS * 32) + j, jr = idx >> 3, c = idx & 7, tok = tok0 + jr;
-                uint8_t* dst = ring + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES + (size_t)jr * 128 + ((c ^ (jr & 7)) << 4);
+                const int idx = it * (B_WARPS * 32) + j, tok = idx >> 3, c = idx & 7;
+                uint8_t* dst = ring + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES + (size_t)tok * 128 + ((c ^ (tok & 7)) << 4);
                 if (tok < p.m)
                     cp_async16(smem_u32(dst), (const uint4*)(p.xh + (size_t)tok * p.k) + (size_t)(kbeg + kb) * 8 + c);
                 else
@@ -295,12 +288,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, TN == 256 ? 1 : 2) nvfp4_gemm_tc
             const int row = row0 + 32 * q + lane;
             const float gs = p.gs[0];
             for (int c0 = half * (TN / 2); c0 < (half + 1) * (TN / 2); c0 += 32) {
-                if (tok0 + c0 >= p.m) break;  // uniform
+                if (c0 >= p.m) break;  // uniform
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, v);
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
-                    const int tok = tok0 + c0 + i;
+                    const int tok = c0 + i;
                     if (tok < p.m && row < p.rows) {
                         if (KSP > 1) {
                             p.part[((size_t)ksi * p.m + tok) * p.rows + row] = __uint_as_float(v[i]);
@@ -337,9 +330,8 @@ __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, const 
 
 constexpr int MAX_KSPLITS = 8;
 
-// K splits for m <= 128: enough CTAs for two per SM, at least eight 64-wide steps each
-int gemm_ksplits(int rows, int k, int m) {
-    if (m > 128) return 1;
+// K splits: enough CTAs for two per SM, at least eight 64-wide steps each
+int gemm_ksplits(int rows, int k) {
     const int tiles = (rows + TM - 1) / TM, bpr = k / 64;
     int ks = (2 * 148 + tiles - 1) / tiles;
     if (ks > MAX_KSPLITS) ks = MAX_KSPLITS;
@@ -388,27 +380,16 @@ extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void
         c.rows = rows, c.k = k, c.m = m, c.ldy = ldy;
         return cn_gemm_pair_launch(c, stream);
     }
-    CN_ALLOW_SMEM(nvfp4_gemm_tc5_kernel<128>, (int)smem_of(128));
-    CN_ALLOW_SMEM(nvfp4_gemm_tc5_kernel<256>, (int)smem_of(256));
+    CN_ALLOW_SMEM(nvfp4_gemm_tc5_kernel, GEMM_SMEM);
     GemmParams p;
     p.w = (const uint8_t*)w, p.gs = gs, p.xh = xh, p.rs = rs, p.y = y, p.rows = rows, p.k = k, p.m = m, p.ldy = ldy, p.out_bf16 = dtype == CN_BF16;
-    p.ksplits = 1, p.part = nullptr;
-    if (m > 128) {
-        dim3 grid((unsigned)((rows + TM - 1) / TM), (unsigned)((m + 255) / 256));
-        nvfp4_gemm_tc5_kernel<256><<<grid, GEMM_THREADS, smem_of(256), stream>>>(p);
-    } else {
-        int ks = gemm_ksplits(rows, k, m);
-        if (rows > 32768) ks = 1;  // the workspace holds partial sums for up to 2^15 rows
-        p.ksplits = ks;
-        p.part = (float*)((char*)workspace + (((size_t)m * k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255));
-        dim3 grid((unsigned)((rows + TM - 1) / TM), (unsigned)ks);
-        nvfp4_gemm_tc5_kernel<128><<<grid, GEMM_THREADS, smem_of(128), stream>>>(p);
-        if (ks > 1) {
-            CN_CUDA(cudaGetLastError());
-            gemm_splitk_reduce_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)m), 256, 0, stream>>>(p.part, gs, rs, y, rows, m, ldy, ks,
-                                                                                                         p.out_bf16);
-        }
-    }
+    p.ksplits = rows > 32768 ? 1 : gemm_ksplits(rows, k);  // the workspace holds partial sums for up to 2^15 rows
+    p.part = (float*)((char*)workspace + (((size_t)m * k * 2 + 255) & ~(size_t)255) + (((size_t)m * 4 + 255) & ~(size_t)255));
+    nvfp4_gemm_tc5_kernel<<<dim3((unsigned)((rows + TM - 1) / TM), (unsigned)p.ksplits), GEMM_THREADS, GEMM_SMEM, stream>>>(p);
     CN_CUDA(cudaGetLastError());
+    if (p.ksplits > 1) {
+        gemm_splitk_reduce_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)m), 256, 0, stream>>>(p.part, gs, rs, y, rows, m, ldy, p.ksplits, p.out_bf16);
+        CN_CUDA(cudaGetLastError());
+    }
     return CN_OK;
 }
