@@ -1,5 +1,5 @@
-// NVFP4 GEMM for up to 128 activation rows (batched verify, short prompts; more rows: nvfp4_gemm_pair.cu): Y[t][n] = gs * sum_k X[t][k] * W[n][k],
-// on the fifth-generation tensor cores: tcgen05.mma (kind::f16) with the accumulator in tensor memory.
+// NVFP4 GEMM for up to 128 activation rows (batched verify, short prompts; more rows: nvfp4_gemm_pair.cu):
+// Y[t][n] = gs * sum_k X[t][k] * W[n][k], on the fifth-generation tensor cores: tcgen05.mma (kind::f16) with the accumulator in tensor memory.
 //
 // Supersedes the reference's prompt GEMMs gemm_fp4_dense (engine/src/kernels.rs:533) and
 // glm5_gemm_fp4_tc (engine/src/kernels_glm5_moe.cu:349: "NVFP4 decoded losslessly to f16 in shared
@@ -111,7 +111,8 @@ struct GemmParams {
     const float* rs;
     void* y;
     int rows, k, m, ldy, out_bf16;
-    // K shared between `ksplits` CTAs of a tile (blockIdx.y, when the row tiles alone do not fill the machine): each writes its raw f32 sums to part[split][m][rows], a second kernel adds them in split order
+    // K shared between `ksplits` CTAs of a tile (blockIdx.y, when the row tiles alone do not fill the machine): each writes its raw
+    // f32 sums to part[split][m][rows], a second kernel adds them in split order
     int ksplits;
     float* part;
 };
@@ -129,7 +130,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) nvfp4_gemm_tc5_kernel(const G
     uint8_t* ring = smem_raw + (ring_addr - smem_u32(smem_raw));
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int KSP = p.ksplits, ksi = (int)blockIdx.y;
+    // (the test keeps the kernel within the 72 registers of two CTAs per SM; with plain blockIdx.y it spills, 64 rows 87 -> 105 us)
+    const int KSP = p.ksplits, ksi = KSP > 1 ? (int)blockIdx.y : 0;
     const int row0 = blockIdx.x * TM;
     const int bpr_all = p.k >> 6;
     const int kbeg = (int)((long long)bpr_all * ksi / KSP), bpr = (int)((long long)bpr_all * (ksi + 1) / KSP) - kbeg;  // this CTA's blocks
