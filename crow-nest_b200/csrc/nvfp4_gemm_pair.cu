@@ -18,10 +18,11 @@
 // warps 12-19 write results. Tiles are walked persistently, one pair per two SMs; with up to 192 tokens per tile there
 // are two accumulators and the epilogue of a tile runs under the MMAs of the next.
 // Rings: weights 3 x 18 KB (256 values of K each), activations up to 8 x 16 KB and A slots 4..8 x 32 columns (64 values).
-// Every wait is bounded.
-// Measured: 17408 x 5120 at 512 rows 155 -> 66 us (1.4 PFLOP/s; one CTA per tile with both operands in shared memory
-// before), 5120 x 17408 at 4096 rows 1190 -> 490 us (1.49 PFLOP/s, at the power cap). What got it there beside the
-// layout: MMA issue from a converged warp (elect_lane) and no cluster-scope fences on the rings' barriers (tc5.cuh).
+// Every wait is bounded. The weights are read with L2's ordinary policy: kept as evict-last, for the token tiles that read them again, they
+// gained nothing (512 rows 76.6 and 76.9 us) and stayed behind: a 50 MB matrix read twice after the call took 83 us the second time, 75 now.
+// Measured over the public call with inputs that change from pass to pass: 17408 x 5120 at 512 rows 155 -> 76 us (1.2 PFLOP/s; one CTA
+// per tile with both operands in shared memory before), 5120 x 17408 at 4096 rows 1190 -> 560 us (1.3 PFLOP/s, at the power cap). What
+// got it there beside the layout: MMA issue from a converged warp (elect_lane) and no cluster-scope fences on the rings' barriers (tc5.cuh).
 #include "nvfp4_gemm.cuh"
 #include "tc5.cuh"
 
@@ -131,7 +132,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         // ------------------------------------------------------------ weights and activations in
         if (lane == 0) {
             tma_prefetch_map(&wmap), tma_prefetch_map(&xmap);
-            const uint64_t keep = l2_policy_evict_last();  // every token tile reads the weights again
             int ws = 0, bs = 0;
             uint32_t wp = 1, bp = 1;  // parity of "empty": the first round passes at once
             bool ok = true;
@@ -146,7 +146,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                     }
                     mbar_expect_tx(&wfull[ws], W_STAGE);
                     mbar_arrive(&wfull[ws]);
-                    tma_load_2d(wring + (uint32_t)ws * W_STAGE, &wmap, w * 36, row0, smem_u32(&wfull[ws]), keep);
+                    tma_load_2d(wring + (uint32_t)ws * W_STAGE, &wmap, w * 36, row0, smem_u32(&wfull[ws]));
                     if (++ws == NW_STAGES) ws = 0, wp ^= 1u;
                     for (int q = 0; q < 2; q++) {
                         if (!mbar_wait(&bempty[bs], bp)) {
@@ -286,7 +286,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     if (warp == 2) tc_dealloc<2>(tmem, TMEM_COLS);
 }
 
-// Tokens per tile: the multiple of 16 up to 256 whose tiles fill the pairs' rounds best. A round costs the longer of the
+// Tokens per tile: the multiple of 32 up to 256 whose tiles fill the pairs' rounds best. A round costs the longer of the
 // MMAs (2 cycles per token and 64-value block) and the decode (about 300 cycles per block bf16, 170 f16), plus the
 // epilogue where a single accumulator leaves it exposed.
 int pair_tokens(int rows, int nk, int m, int pairs, bool bf16) {
