@@ -106,3 +106,37 @@ def test_grouped_gate_up_sums_are_as_exact_as_single_rows(hidden):
     # way through the down matrix 6e-8. (A single running sum of k / 64 = 64 terms: 1.4e-7, 2e-7 for gate and up.)
     assert (h - want).norm() <= 1.45e-7 * want.norm()
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("combos,experts", [(20, 12), (47, 6), (60, 100), (200, 6), (64, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_combos_without_a_resident_expert_are_left_out(combos, experts, dtype):
+    """Ids below, at and beyond the tables and null table entries among the rows, one by one (fewer than 48 combos) and in groups of up to
+    eight: their output rows stay as they were, the others are what 64 bits give."""
+    hidden, inter = 512, 768
+    rng = np.random.default_rng(combos + experts)
+    gs_gu, gs_dn = 2.0 ** -4, 0.5
+    gone = {1, experts - 1} if experts > 2 else {1}
+    gu = [None if e in gone else torch.from_numpy(synth.nvfp4_matrix(2 * inter, hidden, rng)).cuda() for e in range(experts)]
+    dn = [None if e in gone else torch.from_numpy(synth.nvfp4_matrix(hidden, inter, rng)).cuda() for e in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, gs_gu, gs_dn, gate_up=gu, down=dn, device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, 1, combos)
+    ids = rng.integers(-2, experts + 2, combos).astype(np.int32)
+    ids[:3] = [-1, experts, 0]
+    x = torch.from_numpy(rng.standard_normal((combos, hidden)).astype(np.float32)).cuda().to(dtype)
+    eo = torch.full((combos, hidden), 7.0, device="cuda")
+    plan.experts_only(w, torch.from_numpy(ids).cuda(), x, eo=eo)
+    want = torch.full((combos, hidden), 7.0, dtype=torch.float64, device="cuda")
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m, torch.tensor([gs], device="cuda"), rows, k)).double().view(rows, k)
+
+    live = [c for c in range(combos) if 0 <= ids[c] < experts and ids[c] not in gone]
+    for c in live:
+        g = deq(gu[ids[c]], 2 * inter, hidden, gs_gu) @ x[c].double()
+        want[c] = deq(dn[ids[c]], hidden, inter, gs_dn) @ (g[:inter] / (1 + torch.exp(-g[:inter])) * g[inter:])
+    out = [c for c in range(combos) if c not in live]
+    assert len(out) >= 3 and torch.equal(eo[out], torch.full((len(out), hidden), 7.0, device="cuda"))
+    err = (eo.double() - want)[live].norm(dim=1) / want[live].norm(dim=1)
+    assert err.max().item() <= 2e-6  # f32 throughout, as above
+    assert device_status() == 0
