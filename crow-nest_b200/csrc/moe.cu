@@ -76,8 +76,8 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 //   ga[] / counts[0]  positions (in order[]) of the one-row groups: an expert's single row, or the one left over after
 //                     its groups of gmax
 //   gb[], gbrows[] / counts[1]  first positions and row counts (2..gmax) of the other groups
-//   gd[], gdrows[] / counts[2]  the same runs cut into groups of one or two rows (for f32 activations, which take two
-//                     of the kernel's four row slots each: a high and a low f16 plane)
+//   gd[], gdrows[] / counts[2]  the same runs cut into groups of one or two rows (for f32 activations, which take three
+//                     of an MMA's eight columns each: three f16 planes)
 // Placement is done by one warp walking the combos in order (match.any finds the lanes of a step that share an expert),
 // so the sort stays stable without ranking every combo against all others.
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,

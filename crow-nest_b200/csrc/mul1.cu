@@ -648,7 +648,7 @@ static int mul1_ffn(Mul1Plan* p, const unsigned long long* ptrs, const void* x, 
                     int out_f32, cudaStream_t st, const int* rowsrc = nullptr, const int* rowdst = nullptr, int live = 0) {
     const Mul1Spec g = spec_of(p, 0), u = spec_of(p, 1), d = spec_of(p, 2);
     // gate and up share each launch: two small grids on two streams cost an event fork and join and ran one after the other
-    // anyway (one token, four experts of 4096 x 1536: 65 -> 55 us with out_block's wide loads; 16 tokens: 298 -> 289)
+    // anyway (one token, four experts of 4096 x 1536: 65 -> 55 us with out_block's wide loads; 16 tokens: 295 us, no difference beyond noise)
     const Mul1Side ga = {p->xh_a, p->xinv_a, p->part_a, g.tr_off, g.suh_off}, up = {p->xh_b, p->xinv_b, p->part_b, u.tr_off, u.suh_off};
     const Mul1Side dn = {p->xh_a, p->xinv_a, p->part_a, d.tr_off, d.suh_off};
     if (int rc = launch_had_in(ptrs, x, ga, &up, g.k, slots, t, x_div, dtype, p->plane, st, rowsrc)) return rc;

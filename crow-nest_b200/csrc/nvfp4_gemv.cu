@@ -511,8 +511,8 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (a.line_bases) CN_FAIL(CN_ERR_SHAPE, "%s: line output takes bf16 activations", who);
     // f32 activations on the tensor cores where a row is long: at k = 2048 (2048 rows) 3.5 us against 4.2 here for one row and
     // 9.2 against 10.2 for eight, at k = 512 2.5 against 2.0 and 7.2 against 5.6 (its sums take one hop more to the output).
-    // The routed form has such short rows, too (64 tokens, 512 experts: 519 us against 451 with this kernel). A rule of k alone: a row's
-    // result does not depend on how many rows the call has.
+    // The routed form stays here at any k (its rows are as short: 64 tokens, 512 experts 519 us against 451 with this kernel); from 16 combos
+    // on nvfp4_rows.cu takes what it can of it (moe.cu). A rule of k alone: a row's result does not depend on how many rows the call has.
     if (!routed && !a.x_f16_ok && k >= 2048) return cn_gemv_col_launch(a, stream, who);
     const bool gu = a.w1 != nullptr || a.tab1 != nullptr || a.fused_up_rows > 0;
     const int bpr = k / 64;

@@ -5,8 +5,8 @@
 // Arithmetic. An E2M1 code times its UE4M3 scale has six significant bits and is exact in f16, so a weight enters the MMA
 // with its scale applied (one HMUL2 per two weights) and a 64-value block needs a single f32 scale step per column. An f32
 // activation is split into three f16 planes over a power-of-two scale per 64-value block: the value on a grid of 2^-10 of
-// the block's largest binade, then what is left rounded to f16, twice (all 24 bits of a value within 2^11 of the block's
-// largest, 22 bits or more of any other). Each plane is a column and the three sums are added at the end. Products are exact,
+// the block's largest binade, then what is left rounded to f16, twice: all 24 bits of a value within 2^11 of the block's largest, 22
+// or more of one within 2^38, and below that (the last plane is a subnormal f16) an error of at most 2^-61 of the largest. Each plane is a column and the three sums are added at the end. Products are exact,
 // accumulation is the tensor core's f32 inside a block and f32 FMAs across blocks; the tensor core cuts every product at
 // 2^-24 of the largest, which the coarse grid keeps the first plane clear of (as a rounded f16 it cost half the accuracy where
 // one value dominates a block). Relative error against 64 bits, k = 4096: 3.6e-8 on N(0,1) rows, 4.5e-8 .. 8e-8 on rows with

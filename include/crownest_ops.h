@@ -163,8 +163,7 @@ int cn_moe_combine(const float* eo, const float* wts, const int32_t* ids, const 
  * allocation; run() allocates nothing and does not synchronise). The plan also owns one side stream
  * and two events: run() enqueues the shared expert there between a fork event recorded on `stream`
  * and a join event `stream` waits for before the combine, so everything is ordered with the caller's
- * stream as if it ran on it (a capture of `stream` takes the side branch in). cn_mul1_ffn and
- * cn_moe_mul1_run do the same with the up projection.
+ * stream as if it ran on it (a capture of `stream` takes the side branch in).
  * Tables are device arrays [experts] of device addresses (0 = expert not resident: its combos are
  * skipped, the contract of engine/src/kernels_mul1.cu:118-119; so are ids outside 0..experts-1). ids, order and the
  * tables must be complete when the call is enqueued or be written by earlier work on `stream`. table_gu = gate [inter][hidden], or
