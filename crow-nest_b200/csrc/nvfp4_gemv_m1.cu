@@ -860,11 +860,15 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-#define CN_M1_PARTS(KSV, PPV)                                                                                        \
-    if (mt > 1 && ksplit == KSV && pp == PPV) {                                                                      \
-        if (mt == 2) return cps == 2 ? launch_m1<32, 2, 2, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 2, KSV, false, PPV>(cfg, p); \
-        if (mt == 4) return cps == 2 ? launch_m1<32, 2, 4, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 4, KSV, false, PPV>(cfg, p); \
-        return cps == 2 ? launch_m1<32, 2, 8, KSV, false, PPV>(cfg, p) : launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p);              \
+    // Parts are 44 blocks and longer, of 132 bytes per activation row: two CTAs per SM hold one part of four rows or two parts of two, and
+    // never eight rows.
+#define CN_M1_PARTS(KSV, PPV)                                                                      \
+    if (mt > 1 && ksplit == KSV && pp == PPV) {                                                    \
+        if (mt == 2 && cps == 2) return launch_m1<32, 2, 2, KSV, false, PPV>(cfg, p);              \
+        if (mt == 2) return launch_m1<32, 1, 2, KSV, false, PPV>(cfg, p);                          \
+        if (mt == 4 && cps == 2) return launch_m1<32, PPV == 1 ? 2 : 1, 4, KSV, false, PPV>(cfg, p); \
+        if (mt == 4) return launch_m1<32, 1, 4, KSV, false, PPV>(cfg, p);                          \
+        return launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p);                                       \
     }
     CN_M1_PARTS(1, 2) CN_M1_PARTS(1, 4)
     if (ksplit > 1) {
