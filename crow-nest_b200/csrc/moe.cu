@@ -308,7 +308,7 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
     const size_t es = dtype == CN_BF16 ? 2 : 4;
     int rc = CN_OK;
     // More rows than a GEMV takes: both projections as one launch each over groups of rows (64 tokens, 512 x 2048: sixteen launches of
-    // 8 us each before, two of 24 and 11 us now; the step with the shared expert 297 -> 246 us).
+    // 8 us each before, two of 24 and 12 us now; the step with the shared expert 297 -> 250 us).
     RowsCall u = {}, d = {};
     u.w0 = shared_gate, u.w1 = shared_up, u.m = tokens, u.gs0 = shared_gs, u.gs1 = shared_gs + 1, u.x = x, u.x_div = 1, u.x_f32 = dtype == CN_F32;
     u.y = p->hs, u.ldy = p->shared_inter, u.rows = p->shared_inter, u.k = p->hidden, u.limit = limit, u.max_groups = (tokens + (u.x_f32 ? 1 : 7)) / (u.x_f32 ? 2 : 8);

@@ -17,7 +17,7 @@
 //   cascade   per (32-token block, 256-column tile): [160 rows x 128 B] the same way, row = level * 32 + token, then the
 //             scale bytes as [4][2][32][16]
 // A CTA owns one 128-row tile and one or two token blocks over a range of column tiles: warp 4 brings the stages in,
-// one lane of warp 5 copies the scale chunks to tensor memory (tcgen05.cp) and issues the MMAs, warps 0-3 read the
+// an elected lane of warp 5 copies the scale chunks to tensor memory (tcgen05.cp) and issues the MMAs, warps 0-3 read the
 // accumulator (tcgen05.ld), add the five levels of every token and store. When the row tiles alone cannot fill the GPU the
 // column range is split over blockIdx.z and a second kernel adds the partial sums in split order.
 #include "tc5.cuh"

@@ -5,8 +5,8 @@
 // Arithmetic. An E2M1 code times its UE4M3 scale has six significant bits and is exact in f16, so a weight enters the MMA
 // with its scale applied (one HMUL2 per two weights) and a 64-value block needs a single f32 scale step per column. An f32
 // activation is split into three f16 planes over a power-of-two scale per 64-value block: the value on a grid of 2^-10 of
-// the block's largest binade, then what is left rounded to f16, twice: all 24 bits of a value within 2^11 of the block's largest, 22
-// or more of one within 2^38, and below that (the last plane is a subnormal f16) an error of at most 2^-61 of the largest. Each plane is a column and the three sums are added at the end. Products are exact,
+// the block's largest binade, then what is left rounded to f16, twice: all 24 bits of a value within 2^10 of the block's largest, 23
+// of one within 2^38, and below that (the last plane is a subnormal f16) an error of at most 2^-60 of the largest. Each plane is a column and the three sums are added at the end. Products are exact,
 // accumulation is the tensor core's f32 inside a block and f32 FMAs across blocks; the tensor core cuts every product at
 // 2^-24 of the largest, which the coarse grid keeps the first plane clear of (as a rounded f16 it cost half the accuracy where
 // one value dominates a block). Relative error against 64 bits, k = 4096: 3.6e-8 on N(0,1) rows, 4.5e-8 .. 8e-8 on rows with
@@ -20,8 +20,8 @@
 // warp idles at a part's ragged end, warp 9 adds the eight sums of a part and stores. Clusters of two or four CTAs share a
 // tile by parts where that fills the machine better; the others hand a part's sums to the first CTA through distributed
 // shared memory.
-// What bounds it: issue slots (about 200 warp instructions per unit whatever the rows, 88 of them the decode and its scaling;
-// 0.63 of the issue slots used). The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
+// What bounds it: issue slots (245 warp instructions per unit of a one-row gate/up in all, 88 of them the decode and its scaling; 0.56 of
+// the slots used there, 0.51 in the down projection). The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
 #include "common.cuh"
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"

@@ -9,8 +9,8 @@
 // by its own bulk copies (16 row pieces of up to eight blocks, two to four chunks ahead), holds all its sums in registers and stores
 // them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
 // columns) share one decode of its weights; a row's sum does not depend on the rows it is grouped with. Bound by issue slots:
-// about 180 warp instructions per 16 x 128 values. Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under the profiler): gate/up
-// 157 -> 129 us, down 203 -> 86 us against one CTA set per combo.
+// some 200 warp instructions per 16 x 128 values in all, 0.59 of the slots. Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
+// the profiler): gate/up 157 -> 133 us, down 203 -> 86 us against one CTA set per combo.
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"
 
