@@ -327,7 +327,7 @@ def moe_measure(kind, tokens, rank, world, local, steps, warmup, cpu=False, e2e=
                "tok_s": tokens * world / (ms * 1e-3), "ms_per_step": ms, "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"],
                "ms_per_step_max": t["ms_per_step_max"], "distinct_experts": distinct, "algorithmic_bytes": nbytes,
                "roofline": {"bound": "hbm", "achieved": gbs / world, "peak": peak, "unit": "GB/s", "frac": gbs / world / peak, "peak_kind": peak_kind,
-                            "scope": "per GPU", "kernel": "nvfp4_gemv_m1_kernel (routed form)" if kind == "moe" else "mul1_gemv_kernel"},
+                            "scope": "per GPU", "kernel": "mul1_gemv_kernel" if kind != "moe" else "nvfp4_rows_kernel" if tokens * wl.topk >= 48 else "nvfp4_gemv_m1_kernel (routed form)"},
                "parallelism": f"ep{world}: all-to-all dispatch / return over peer memory" if world > 1 else "none",
                "launches_per_step": wl.launches_per_step, "device_status": status}
         if e2e_s is not None:
@@ -587,7 +587,7 @@ def gemm_arm(args, rank, world, local):
     yp = torch.empty((m, hidden // world), dtype=torch.bfloat16, device=dev) if world > 1 else y
     y_host = torch.empty((m, hidden), dtype=torch.bfloat16).pin_memory()
     # engine: the block-scaled FP4 MMA (kind::mxf4nvf4 + five-level activation cascade) up to 128 rows, where one pass over
-    # the weights serves every token; beyond that its operand traffic (five cascade columns per token) binds on L2 and the f16
+    # the weights serves every token; beyond that its operand traffic (five cascade columns per token) is what it waits for and the f16
     # MMA on losslessly widened weights is faster (both are tcgen05)
     fp4 = args.engine == "fp4" or (args.engine == "auto" and m <= 128)
     raw_rows = ups[0].w[: 1024 * (hidden // 64 * 36)].cpu().numpy() if world == 1 and not args.no_cpu_baseline else None
@@ -600,6 +600,18 @@ def gemm_arm(args, rank, world, local):
         ws = torch.empty(ops.gemm_workspace_bytes(inter, m), dtype=torch.uint8, device=dev)
         gemm = ops.launch_gemm
     it = [0]
+
+    def launches(rows, k):
+        """Kernels of one GEMM call: activations in (the pair GEMM reads bf16 rows as they are), GEMM, and the sum over a split K range."""
+        if not fp4 and m > 128:
+            return 1
+        tiles = (rows + 127) // 128
+        if fp4:
+            ctas = tiles * (((m + 31) // 32 + 1) // 2)
+            splits = min(148 // ctas, k // 256 // 4) if ctas < 120 else 1
+        else:
+            splits = min((2 * 148 + tiles - 1) // tiles, 8, k // 64 // 8) if rows <= 32768 else 1
+        return 2 + (1 if splits > 1 else 0)
 
     def step():
         i = it[0]
@@ -636,11 +648,12 @@ def gemm_arm(args, rank, world, local):
                            "l2": "three weight copies rotated (300 MB per rank) plus the activations: larger than L2", "launch": "plain launches"},
                 "roofline": {"bound": "tensor", "achieved": tf / world, "peak": peak, "unit": "TFLOP/s", "frac": tf / world / peak, "traffic": None,
                              "peak_kind": kind + " (bf16 GEMM, burst)", "scope": "per GPU",
-                             "kernel": "nvfp4_gemm_bs_kernel (tcgen05 kind::mxf4nvf4)" if fp4 else "nvfp4_gemm_tc5_kernel (tcgen05 kind::f16)", "flops_per_launch": flops / 2 / world, "us_per_launch": ms_step * 1e3 / 2,
+                             "kernel": "nvfp4_gemm_bs_kernel (tcgen05 kind::mxf4nvf4)" if fp4 else f"nvfp4_gemm_{'pair' if m > 128 else 'tc5'}_kernel (tcgen05 kind::f16)", "flops_per_launch": flops / 2 / world, "us_per_launch": ms_step * 1e3 / 2,
                              "hbm_gbs": (2 * hidden * inter // 64 * 36 / world + 2.0 * m * (hidden + inter) * 2) / (ms_step * 1e-3) / 1e9},
                 "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"], "ms_per_step_max": t["ms_per_step_max"],
                 "e2e": {"value": flops / e2e_s / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": x_host.numel() * 2, "d2h_bytes_per_step": y_host.numel() * 2},
-                "gpu_launches": args.steps * t["blocks"] * 4, "clocks": clocks, "device_status": _lib.device_status()}
+                "gpu_launches": args.steps * t["blocks"] * (launches(inter // world, hidden) + launches(hidden // world, inter)), "clocks": clocks,
+                "device_status": _lib.device_status()}
         if world == 1 and not args.no_cpu_baseline:
             import numpy as np
             import oracle
