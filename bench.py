@@ -586,9 +586,7 @@ def gemm_arm(args, rank, world, local):
     hp = torch.empty((m, inter // world), dtype=torch.bfloat16, device=dev) if world > 1 else h
     yp = torch.empty((m, hidden // world), dtype=torch.bfloat16, device=dev) if world > 1 else y
     y_host = torch.empty((m, hidden), dtype=torch.bfloat16).pin_memory()
-    # engine: the block-scaled FP4 MMA (kind::mxf4nvf4 + five-level activation cascade) up to 128 rows, where one pass over
-    # the weights serves every token; beyond that its operand traffic (five cascade columns per token) is what it waits for and the f16
-    # MMA on losslessly widened weights is faster (both are tcgen05)
+    # engine: re-laid weights (cn_nvfp4_bs_gemm) up to 128 rows, container bytes beyond; bf16 rows run on the same kernel from both
     fp4 = args.engine == "fp4" or (args.engine == "auto" and m <= 128)
     raw_rows = ups[0].w[: 1024 * (hidden // 64 * 36)].cpu().numpy() if world == 1 and not args.no_cpu_baseline else None
     if fp4:
@@ -602,16 +600,26 @@ def gemm_arm(args, rank, world, local):
     it = [0]
 
     def launches(rows, k):
-        """Kernels of one GEMM call: activations in (the pair GEMM reads bf16 rows as they are), GEMM, and the sum over a split K range."""
-        if not fp4 and m > 128:
-            return 1
-        tiles = (rows + 127) // 128
-        if fp4:
-            ctas = tiles * (((m + 31) // 32 + 1) // 2)
-            splits = min(148 // ctas, k // 256 // 4) if ctas < 120 else 1
-        else:
-            splits = min((2 * 148 + tiles - 1) // tiles, 8, k // 64 // 8) if rows <= 32768 else 1
-        return 2 + (1 if splits > 1 else 0)
+        """Kernels of one GEMM call: rows into f16 (up to 128 of them), GEMM, and the sum over a split K range (the launcher's choice of tile and
+        split restated: csrc/nvfp4_gemm_pair.cu, pair_shape)."""
+        nw, rt, up = k // 256, (rows + 255) // 256, lambda a, b: (a + b - 1) // b
+        slow = 170.0 if m <= 128 else 300.0
+        most = min(up(m, 32) * 32, 256)
+        room = 8 if (fp4 or m <= 128) and rows <= 32768 else max(1, min(8, 32768 // rows))
+        best, split = 1e30, 1
+        for n in range(up(m, most), up(m, 32) + 1):
+            t = up(up(m, n), 32) * 32
+            for ks in range(1, (room if m <= 512 else 1) + 1):
+                if ks > 1 and ks > nw // 2:
+                    break
+                tail = 2500.0 + 16.0 * t
+                cost = up(rt * up(m, t) * ks, 74) * (4 * up(nw, ks) * max(2.0 * t, slow) + (tail if t > 192 else 400.0)) + (0.0 if t > 192 else tail)
+                cost += 5000.0 + ks * m * rows / 300.0 if ks > 1 else 0.0
+                if cost < best:
+                    best, split = cost, ks
+            if t <= 64:
+                break
+        return (1 if m <= 128 else 0) + 1 + (1 if split > 1 else 0)
 
     def step():
         i = it[0]
@@ -643,12 +651,12 @@ def gemm_arm(args, rank, world, local):
         peak, kind = measured_peak("bf16_tflops", 1590.0)
         line = {"metric": "nvfp4_gemm_tflops", "value": tf, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
                 "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-                "dtype": "e2m1 x e2m1 block-scaled -> f32" if fp4 else "f16 x f16 -> f32", "data": "synthetic",
+                "dtype": "f16 x f16 -> f32" if m <= 128 else "bf16 x bf16 -> f32", "data": "synthetic",
                 "config": {"workload": f"nvfp4 GEMM pair [17408 x 5120] and [5120 x 17408], M={m}", "parallelism": f"tp{world} column split + all-gather" if world > 1 else "none",
                            "l2": "three weight copies rotated (300 MB per rank) plus the activations: larger than L2", "launch": "plain launches"},
                 "roofline": {"bound": "tensor", "achieved": tf / world, "peak": peak, "unit": "TFLOP/s", "frac": tf / world / peak, "traffic": None,
                              "peak_kind": kind + " (bf16 GEMM, burst)", "scope": "per GPU",
-                             "kernel": "nvfp4_gemm_bs_kernel (tcgen05 kind::mxf4nvf4)" if fp4 else f"nvfp4_gemm_{'pair' if m > 128 else 'tc5'}_kernel (tcgen05 kind::f16)", "flops_per_launch": flops / 2 / world, "us_per_launch": ms_step * 1e3 / 2,
+                             "kernel": "nvfp4_gemm_pair_kernel (tcgen05 kind::f16)", "flops_per_launch": flops / 2 / world, "us_per_launch": ms_step * 1e3 / 2,
                              "hbm_gbs": (2 * hidden * inter // 64 * 36 / world + 2.0 * m * (hidden + inter) * 2) / (ms_step * 1e-3) / 1e9},
                 "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"], "ms_per_step_max": t["ms_per_step_max"],
                 "e2e": {"value": flops / e2e_s / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": x_host.numel() * 2, "d2h_bytes_per_step": y_host.numel() * 2},
@@ -745,7 +753,7 @@ def main():
     ap.add_argument("--workload", default="dense", choices=["dense", "gemv", "moe", "mul1", "gemm", "intervals"],
                     help="dense = the headline (layer stack); gemv = one matrix (default 4096 x 4096); moe / mul1 = routed experts; gemm = batched rows")
     ap.add_argument("--tokens", type=int, default=8, help="moe / mul1: token rows per rank")
-    ap.add_argument("--engine", default="auto", choices=["auto", "fp4", "f16"], help="gemm: block-scaled FP4 MMA, f16 MMA on widened weights, or by row count")
+    ap.add_argument("--engine", default="auto", choices=["auto", "fp4", "f16"], help="gemm: re-laid weights (fp4), container bytes (f16), or by row count")
     ap.add_argument("--op", default="gemv", choices=["gemv", "gu", "fp8"], help="gemv workload: plain NVFP4 GEMV, fused gate/up, or the FP8 GEMV")
     ap.add_argument("--rows", type=int, default=4096, help="gemv: output rows")
     ap.add_argument("--cols", type=int, default=4096, help="gemv: k")

@@ -2,6 +2,9 @@
 // per 16 values on both operands, f32 accumulation in tensor memory). Supersedes gemm_fp4_dense / gemm_fp4_dense_b
 // (engine/src/kernels.rs:533, :642; MMA shape :362-372, launched by launch_mma_d, engine/src/gen.rs:2491) and the activation
 // cascade that feeds them (quant_row_prescaled, engine/src/kernels.rs:264-350; host twin act_cascade, :5354-5475).
+// f32 rows only: bf16 rows take the CTA-pair kernel on the same stage images (nvfp4_gemm_pair.cu), which decodes them instead. Measured
+// per call, us, this kernel / that one: 17408 x 5120 at 32 rows 24 / 23, at 64 32 / 21, at 128 55 / 23, at 256 99 / 35; 5120 x 17408 at
+// 16 rows 33 / 26, at 64 45 / 27. f32 rows lose more to f16 (1.4e-4 of a row) than to five levels (5e-6).
 //
 // Both operands of this MMA are FP4, so the activations are re-quantised: every row becomes a per-row power of two times a
 // sum of LEVELS NVFP4 "levels", each level coding what the levels before it left (the reference's cascade, which stops at
@@ -20,6 +23,7 @@
 // an elected lane of warp 5 copies the scale chunks to tensor memory (tcgen05.cp) and issues the MMAs, warps 0-3 read the
 // accumulator (tcgen05.ld), add the five levels of every token and store. When the row tiles alone cannot fill the GPU the
 // column range is split over blockIdx.z and a second kernel adds the partial sums in split order.
+#include "nvfp4_gemm.cuh"
 #include "tc5.cuh"
 
 namespace {
@@ -486,6 +490,13 @@ int ksplits_for(int rows, int k, int m) {
     return ks;
 }
 
+// bf16 rows: the product on CTA pairs that decode the same stage images (nvfp4_gemm_pair.cu)
+bool f16_rows(int m) { return m <= 128; }
+size_t rows_bytes(int k, int m) { return ((size_t)m * k * 2 + 255) & ~(size_t)255; }  // the f16 rows, or a copy of the bf16 ones
+size_t row_factor_bytes(int m) { return ((size_t)m * 4 + 255) & ~(size_t)255; }
+constexpr int MAX_PAIR_SPLITS = 8;
+int pair_splits(int rows, int k, int m) { return m <= 512 ? cn_gemm_pair_splits(rows, k, m, f16_rows(m), MAX_PAIR_SPLITS) : 1; }
+
 }  // namespace
 
 extern "C" size_t cn_nvfp4_bs_packed_bytes(int rows, int k) {
@@ -506,7 +517,10 @@ extern "C" size_t cn_nvfp4_bs_workspace_bytes(int rows, int k, int m) {
     if (rows <= 0 || k <= 0 || k % KT || m <= 0) return 0;
     const size_t ntb = (size_t)(m + TB - 1) / TB;
     const int ks = ksplits_for(rows, k, m);
-    return ntb * (k / KT) * B_STAGE + ntb * TB * 4 + 256 + (ks > 1 ? (size_t)ks * m * rows * 4 : 0);
+    const size_t f32 = ntb * (k / KT) * B_STAGE + ntb * TB * 4 + 256 + (ks > 1 ? (size_t)ks * m * rows * 4 : 0);
+    const int ps = pair_splits(rows, k, m);
+    const size_t bf16 = rows_bytes(k, m) + row_factor_bytes(m) + (ps > 1 ? (size_t)ps * m * rows * 4 : 0);
+    return f32 > bf16 ? f32 : bf16;
 }
 
 extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype,
@@ -518,11 +532,28 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < cn_nvfp4_bs_workspace_bytes(rows, k, m))
         CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_bs_gemm: the workspace must be 256-byte aligned and at least %zu B", cn_nvfp4_bs_workspace_bytes(rows, k, m));
+    if (((uintptr_t)x & 15)) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: x must be 16-byte aligned");
+    if (dtype == CN_BF16) {
+        GemmCall c = {};
+        c.packed = packed, c.gs = gs, c.x = x, c.y = y, c.rows = rows, c.k = k, c.m = m, c.ldy = ldy, c.out_bf16 = 1, c.x_f16 = f16_rows(m);
+        if (c.x_f16) {
+            uint16_t* xh = (uint16_t*)workspace;
+            float* rs = (float*)((char*)workspace + rows_bytes(k, m));
+            if (int rc = cn_gemm_prep_x(x, dtype, xh, rs, k, m, stream)) return rc;
+            c.x = xh, c.rs = rs;
+        } else if ((uintptr_t)x < (uintptr_t)y + ((size_t)(m - 1) * ldy + rows) * 2 && (uintptr_t)y < (uintptr_t)x + (size_t)m * k * 2) {
+            // results may take the place of the activations: every row tile reads these again
+            CN_CUDA(cudaMemcpyAsync(workspace, x, (size_t)m * k * 2, cudaMemcpyDeviceToDevice, stream));
+            c.x = workspace;
+        }
+        c.max_splits = pair_splits(rows, k, m);
+        if (c.max_splits > 1) c.part = (float*)((char*)workspace + rows_bytes(k, m) + row_factor_bytes(m));
+        return cn_gemm_pair_launch(c, stream);
+    }
     const int ntb = (m + TB - 1) / TB, kts = k / KT;
     uint8_t* xq = (uint8_t*)workspace;
     float* rs = (float*)(xq + (size_t)ntb * kts * B_STAGE);
     float* part = rs + (size_t)ntb * TB + 64;
-    if (((uintptr_t)x & 15)) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: x must be 16-byte aligned");
     const dim3 cgrid((unsigned)CQ * ntb * TB);
     if (dtype == CN_BF16)
         bs_cascade_kernel<1><<<cgrid, CTHREADS, 0, stream>>>(x, xq, rs, k, m);

@@ -1,4 +1,5 @@
-// NVFP4 GEMM for more than 128 activation rows (prompt chunks): Y[t][n] = gs * sum_k X[t][k] * W[n][k] on CTA pairs.
+// NVFP4 GEMM on CTA pairs (batched verify, prompts): Y[t][n] = gs * sum_k X[t][k] * W[n][k], weights in the container layout or re-laid
+// (the stage images of nvfp4_gemm_bs.cu).
 //
 // Supersedes the reference's prompt GEMMs gemm_fp4_dense (engine/src/kernels.rs:533) and glm5_gemm_fp4_tc
 // (engine/src/kernels_glm5_moe.cu:349: weights decoded losslessly, f32 accumulate). Same arithmetic here: an E2M1 code
@@ -17,7 +18,12 @@
 // tile's rows), warp 1 of the even CTA issues the MMAs of the pair, two sets of four warps (4-11) decode alternate 64-value blocks,
 // warps 12-19 write results. Tiles are walked persistently, one pair per two SMs; with up to 192 tokens per tile there
 // are two accumulators and the epilogue of a tile runs under the MMAs of the next.
-// Rings: weights 3 x 18 KB (256 values of K each), activations up to 8 x 16 KB and A slots 4..8 x 32 columns (64 values).
+// Rings: weights 3 to 6 x 18 KB (256 values of K each), activations up to 8 x 16 KB and A slots 4..8 x 32 columns (64 values).
+//
+// Up to 128 rows the decode bounds it, not the MMAs: 127 warp instructions per scheduler and 64-value block, most of them at half rate,
+// 255 cycles measured; hence f16 (half the instructions of the decode to bf16), with the rows brought into f16 by a kernel before this one
+// that runs under this one's prologue, all sixteen warps decoding, and K split where row tiles do not fill the pairs. 17408 x 5120 at 64 rows:
+// 80 us (one CTA per tile, widened weights through shared memory) -> 21; 5120 x 17408: 109 -> 27.
 // Every wait is bounded. The weights are read with L2's ordinary policy: kept as evict-last, for the token tiles that read them again, they
 // gained nothing (512 rows 76.6 and 76.9 us) and stayed behind: a 50 MB matrix read twice after the call took 83 us the second time, 75 now.
 // Measured over the public call with inputs that change from pass to pass: 17408 x 5120 at 512 rows 155 -> 76 us (1.2 PFLOP/s; one CTA
@@ -28,7 +34,8 @@
 
 namespace {
 
-constexpr int W_STAGE = 128 * 144, NW_STAGES = 3;
+constexpr int W_STAGE = 128 * 144;  // 256 values of K of 128 rows: container bytes, or the stage image of the re-laid weights
+constexpr int MAX_W_STAGES = 6;
 constexpr int PAIR_THREADS = 640;
 constexpr int HDR = 1024;
 constexpr int SMEM_MAX = 227 * 1024;
@@ -38,39 +45,65 @@ struct PairParams {
     const float* gs;
     const float* rs;  // per activation row (f16 rows)
     void* y;
-    int rows, m, ldy, pair_store;
+    int rows, m, ldy, out_bf16, pair_store;  // pair_store: bf16 results two rows at a time
     int nk;                      // 64-value blocks of K
-    int tn, acc_stride, nacc, na, nb;  // tokens per tile; accumulator columns and count; A and activation ring depths
-    int row_tiles, tiles;
+    int tn, acc_stride, nacc, na, nb, nws;  // tokens per tile; accumulator columns and count; A, activation and weight ring depths
+    int row_tiles, tiles, ksplits;
+    int split_stages, split_more;  // weight stages of a part of K; the first split_more parts have one more
+    const uint8_t* packed;  // re-laid weights (cn_nvfp4_bs_repack), or null: container bytes through wmap
+    int packed_tiles;       // 128-row tiles of them
+    float* part;            // ksplits > 1: raw sums [ksplits][m][rows]
+};
+// A pair's work comes in units, a tile and a part of K (all of it with one split), in the order of the splits. Counted up instead of
+// divided out, so that the compiler sees what the whole warp shares: with a quotient in the MMA warp's loop bounds its operands left the
+// uniform registers (17408 x 5120, 64 rows: 25 -> 29 us; 4096 rows of 5120 x 17408: 585 -> 616).
+struct Unit {
+    int tile, split;
+    __device__ __forceinline__ explicit Unit(int pair, const PairParams& p) : tile(pair), split(0) { wrap(p); }
+    __device__ __forceinline__ void wrap(const PairParams& p) {
+        while (tile >= p.tiles && split < p.ksplits) tile -= p.tiles, split++;
+    }
+    __device__ __forceinline__ bool live(const PairParams& p) const { return split < p.ksplits; }
+    __device__ __forceinline__ void next(int npairs, const PairParams& p) { tile += npairs, wrap(p); }
+    __device__ __forceinline__ int first(const PairParams& p) const { return split * p.split_stages + min(split, p.split_more); }
+    __device__ __forceinline__ int count(const PairParams& p) const { return p.split_stages + (split < p.split_more ? 1 : 0); }
 };
 
-// Blocks SET and SET + 2 of every weight stage, one row per thread: block b is nine words from word 9 b of the row's 144
-// bytes, inside three 16-byte chunks. (Four sets of one block each measured 5 % slower at 200 - 1000 rows.)
-template <bool BF16, int SET>
-__device__ __forceinline__ void decode_set(uint32_t src, uint32_t dst, uint64_t* wfull, uint64_t* wempty, uint64_t* aempty, uint32_t afull_base, int stages,
-                                           int na, int lane) {
-    int ws = 0, as = SET;
-    uint32_t wp = 0, ap = 1;
+// Where a decode warp stands in the rings of weight stages and A slots.
+struct DecodeAt {
+    int ws, as;
+    uint32_t wp, ap;
+};
+// Every SETS-th block of `stages` weight stages from block SET on, one row per thread. Container: block b is nine words from word 9 b of the
+// row's 144 bytes, inside three 16-byte chunks. Re-laid: codes are chunks 2 b and 2 b + 1 of the row's 128 swizzled bytes, the scale word lies
+// in the image's scale part. Two sets of warps where the MMAs or the ALUs bound the loop (four of one block each measured 5 % slower at
+// 200 - 1000 rows of bf16), four where it is the way of a block - load, decode, store to tensor memory, arrival, some 800 cycles - that does.
+template <bool BF16, bool PACKED, int SET, int SETS>
+__device__ __forceinline__ void decode_set(uint32_t src, uint32_t scales, uint32_t dst, uint64_t* wfull, uint64_t* wempty, uint64_t* aempty, uint32_t afull_base,
+                                           int stages, int nws, int na, int lane, DecodeAt& at_) {
+    int ws = at_.ws, as = at_.as;
+    uint32_t wp = at_.wp, ap = at_.ap;
     for (int w = 0; w < stages; w++) {
         if (!mbar_wait(&wfull[ws], wp)) {
             cn_dev_fail(CN_DEV_WAIT_FULL);
             return;
         }
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int b = SET + 2 * h;
+        for (int b = SET; b < 4; b += SETS) {
             uint32_t c[12], v[32];
-            const uint32_t at = src + (uint32_t)ws * W_STAGE + (uint32_t)((9 * b) >> 2) * 16u;
+            const uint32_t at = src + (uint32_t)ws * W_STAGE + (PACKED ? 0u : (uint32_t)((9 * b) >> 2) * 16u);
+            constexpr int C0 = PACKED ? 1 : 0;  // word 0 of a re-laid block is its scale word, from elsewhere
 #pragma unroll
-            for (int i = 0; i < 3; i++)
+            for (int i = 0; i < (PACKED ? 2 : 3); i++)
                 asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(c[4 * i]), "=r"(c[4 * i + 1]), "=r"(c[4 * i + 2]), "=r"(c[4 * i + 3])
-                             : "r"(at + 16u * i));
+                             : "=r"(c[4 * i + C0]), "=r"(c[4 * i + C0 + 1]), "=r"(c[4 * i + C0 + 2]), "=r"(c[4 * i + C0 + 3])
+                             : "r"(PACKED ? at + (uint32_t)(((2 * b + i) ^ (lane & 7)) << 4) : at + 16u * i));
+            if (PACKED) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(c[0]) : "r"(scales + (uint32_t)ws * W_STAGE + 512u * b));
             if (BF16)
-                decode64_bf16(c + b, v);
+                decode64_bf16(c + (PACKED ? 0 : b), v);
             else
-                decode64_f16(c + b, v);
-            if (h == 1) {  // the stage has been read
+                decode64_f16(c + (PACKED ? 0 : b), v);
+            if (b + SETS >= 4) {  // the stage has been read
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&wempty[ws]);
             }
@@ -84,21 +117,24 @@ __device__ __forceinline__ void decode_set(uint32_t src, uint32_t dst, uint64_t*
             tc_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(afull_base + 8u * (uint32_t)as);
-            as += 2;
+            as += SETS;
             if (as >= na) as -= na, ap ^= 1u;
         }
-        if (++ws == NW_STAGES) ws = 0, wp ^= 1u;
+        if (++ws == nws) ws = 0, wp ^= 1u;
     }
+    at_ = {ws, as, wp, ap};
 }
 
-template <bool BF16>
+// SETS = 4 (f16 rows, at most 128 tokens per tile): all sixteen warps decode and write a unit's results when they have decoded it.
+// SPLIT: K may be split; without it the exposed epilogue of a single accumulator carries none of that code (512 rows 77.6 us with, 77.0 without).
+template <bool BF16, bool PACKED, int SETS, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const PairParams p) {
     extern __shared__ uint8_t smem_raw[];
-    // barriers: wfull 3, wempty 3, bfull 8, bempty 8, afull 8, aempty 8, accfull 2, accempty 2
+    // barriers: wfull 6, wempty 6, bfull 8, bempty 8, afull 8, aempty 8, accfull 2, accempty 2
     uint64_t* wfull = (uint64_t*)smem_raw;
-    uint64_t* wempty = wfull + NW_STAGES;
-    uint64_t* bfull = wempty + NW_STAGES;
+    uint64_t* wempty = wfull + MAX_W_STAGES;
+    uint64_t* bfull = wempty + MAX_W_STAGES;
     uint64_t* bempty = bfull + 8;
     uint64_t* afull = bempty + 8;
     uint64_t* aempty = afull + 8;
@@ -115,9 +151,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     const int nw = p.nk >> 2;  // weight stages per tile (k is a multiple of 256)
 
     if (tid == 0) {
-        for (int i = 0; i < NW_STAGES; i++) mbar_init(&wfull[i], 1), mbar_init(&wempty[i], 8);
+        for (int i = 0; i < MAX_W_STAGES; i++) mbar_init(&wfull[i], 1), mbar_init(&wempty[i], 4 * SETS);
         for (int i = 0; i < 8; i++) mbar_init(&bfull[i], 1), mbar_init(&bempty[i], 1), mbar_init(&afull[i], 8), mbar_init(&aempty[i], 1);
-        for (int i = 0; i < 2; i++) mbar_init(&accfull[i], 1), mbar_init(&accempty[i], 16);
+        for (int i = 0; i < 2; i++) mbar_init(&accfull[i], 1), mbar_init(&accempty[i], SETS == 4 ? 32 : 16);
         mbar_fence_init();
     }
     if (warp == 2) tc_alloc<2>(tmem_slot, TMEM_COLS);
@@ -125,20 +161,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     __syncthreads();
     cluster_sync_ctas();  // both CTAs' barriers exist before anything arrives on them
     tc_after();
+    pdl_launch_dependents();
     const uint32_t tmem = warp_uniform(*tmem_slot);
     const uint32_t acol = tmem + (uint32_t)(p.nacc * p.acc_stride);
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ weights and activations in
+    DecodeAt at = {0, (warp - 4) >> 2, 0u, 1u};
+    auto decode = [&](int stages) {
+        const uint32_t src = wring + (uint32_t)(32 * (warp & 3) + lane) * (PACKED ? 128u : 144u);
+        const uint32_t scales = wring + 128u * 128u + (uint32_t)lane * 16u + 4u * (uint32_t)(warp & 3);
+        const uint32_t dst = acol + ((uint32_t)(32 * (warp & 3)) << 16);
+        const uint32_t afull_base = cluster_addr(smem_u32(afull), 0);
+        const int set = (warp - 4) >> 2;
+        if (set == 0) decode_set<BF16, PACKED, 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
+        if (set == 1) decode_set<BF16, PACKED, 1, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
+        if (SETS == 4 && set == 2) decode_set<BF16, PACKED, SETS == 4 ? 2 : 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
+        if (SETS == 4 && set == 3) decode_set<BF16, PACKED, SETS == 4 ? 3 : 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
+    };
+    auto load_w = [&](int ws, int rt, int w) {
+        if (PACKED)  // (the upper half of the last 256-row tile may lie beyond the matrix: it reads the last one, and its results are not stored)
+            bulk_g2s(smem_raw + (wring - smem_u32(smem_raw)) + (uint32_t)ws * W_STAGE, p.packed + ((size_t)min(rt, p.packed_tiles - 1) * nw + w) * W_STAGE,
+                     W_STAGE, &wfull[ws]);
+        else
+            tma_load_2d(wring + (uint32_t)ws * W_STAGE, &wmap, w * 36, rt * 128, smem_u32(&wfull[ws]));
+    };
+    if (BF16 && warp == 0) {
+        // ------------------------------------------------------------ weights and activations in, by one thread: two of them, each as far
+        // ahead as its ring allows, cost 4 - 20 % beyond 128 rows
         if (lane == 0) {
-            tma_prefetch_map(&wmap), tma_prefetch_map(&xmap);
+            if (!PACKED) tma_prefetch_map(&wmap);
+            tma_prefetch_map(&xmap);
             int ws = 0, bs = 0;
             uint32_t wp = 1, bp = 1;  // parity of "empty": the first round passes at once
             bool ok = true;
             const uint32_t bfull0 = smem_u32(bfull) & 0xFEFFFFFFu;  // the even CTA's barriers
-            for (int tile = pair; tile < p.tiles && ok; tile += npairs) {
-                const int row0 = (tile % p.row_tiles) * 256 + (int)rank * 128, tok0 = (tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1);
-                for (int w = 0; w < nw && ok; w++) {
+            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+                const int rt = (u.tile % p.row_tiles) * 2 + (int)rank, tok0 = (u.tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1);
+                const int w0 = u.first(p), w1 = w0 + u.count(p);
+                for (int w = w0; w < w1 && ok; w++) {
                     if (!mbar_wait(&wempty[ws], wp)) {
                         cn_dev_fail(CN_DEV_WAIT_EMPTY);
                         ok = false;
@@ -146,8 +205,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                     }
                     mbar_expect_tx(&wfull[ws], W_STAGE);
                     mbar_arrive(&wfull[ws]);
-                    tma_load_2d(wring + (uint32_t)ws * W_STAGE, &wmap, w * 36, row0, smem_u32(&wfull[ws]));
-                    if (++ws == NW_STAGES) ws = 0, wp ^= 1u;
+                    load_w(ws, rt, w);
+                    if (++ws == p.nws) ws = 0, wp ^= 1u;
                     for (int q = 0; q < 2; q++) {
                         if (!mbar_wait(&bempty[bs], bp)) {
                             cn_dev_fail(CN_DEV_WAIT_EMPTY);
@@ -165,6 +224,56 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                 }
             }
         }
+    } else if (warp == 0) {
+        // ------------------------------------------------------------ f16 rows: weights in. They depend on no earlier kernel, so they start
+        // while the one that prepares the activations still runs.
+        if (lane == 0) {
+            if (!PACKED) tma_prefetch_map(&wmap);
+            int ws = 0;
+            uint32_t wp = 1;  // parity of "empty": the first round passes at once
+            bool ok = true;
+            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+                const int rt = (u.tile % p.row_tiles) * 2 + (int)rank, w0 = u.first(p), w1 = w0 + u.count(p);
+                for (int w = w0; w < w1; w++) {
+                    if (!mbar_wait(&wempty[ws], wp)) {
+                        cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&wfull[ws], W_STAGE);
+                    mbar_arrive(&wfull[ws]);
+                    load_w(ws, rt, w);
+                    if (++ws == p.nws) ws = 0, wp ^= 1u;
+                }
+            }
+        }
+    } else if (!BF16 && warp == 3) {
+        // ------------------------------------------------------------ f16 rows: activations in
+        if (lane == 0) {
+            tma_prefetch_map(&xmap);
+            int bs = 0;
+            uint32_t bp = 1;
+            bool ok = true;
+            const uint32_t bfull0 = smem_u32(bfull) & 0xFEFFFFFFu;  // the even CTA's barriers
+            pdl_wait();  // f16 rows come from the kernel before this one
+            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+                const int tok0 = (u.tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1), w0 = u.first(p), w1 = w0 + u.count(p);
+                for (int q = 2 * w0; q < 2 * w1; q++) {
+                    if (!mbar_wait(&bempty[bs], bp)) {
+                        cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) {  // the even CTA's barrier counts both halves
+                        mbar_expect_tx(&bfull[bs], 2u * bslot);
+                        mbar_arrive(&bfull[bs]);
+                    }
+                    tma_load_2d_pair(ring + (uint32_t)bs * bslot, &xmap, q * 128, tok0, bfull0 + 8u * (uint32_t)bs);
+                    tma_load_2d_pair(ring + (uint32_t)bs * bslot + bbox, &xmap, q * 128 + 64, tok0, bfull0 + 8u * (uint32_t)bs);
+                    if (++bs == p.nb) bs = 0, bp ^= 1u;
+                }
+            }
+        }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issue, even CTA only
         if (rank == 0) {
@@ -173,14 +282,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             int as = 0, bs = 0, ab = 0;
             uint32_t ap = 0, bp = 0, cp = 1;
             bool ok = true;
-            for (int tile = pair; tile < p.tiles && ok; tile += npairs) {
+            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 if (!mbar_wait(&accempty[ab], cp)) {
                     cn_dev_fail(CN_DEV_WAIT_EMPTY);
                     break;
                 }
                 tc_after();
                 const uint32_t d = tmem + (uint32_t)(ab * p.acc_stride);
-                for (int kb = 0; kb < p.nk; kb += 2) {
+                const int nk = 4 * u.count(p);
+                for (int kb = 0; kb < nk; kb += 2) {
                     if (!mbar_wait(&bfull[bs], bp)) {
                         cn_dev_fail(CN_DEV_WAIT_FULL);
                         ok = false;
@@ -214,19 +324,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                 if (++ab == p.nacc) ab = 0, cp ^= 1u;
             }
         }
-    } else if (warp >= 4 && warp < 12) {
+    } else if (SETS == 2 && warp >= 4 && warp < 12) {
         // ------------------------------------------------------------ decode
-        const uint32_t src = wring + (uint32_t)(32 * (warp & 3) + lane) * 144u;
-        const uint32_t dst = acol + ((uint32_t)(32 * (warp & 3)) << 16);
-        const uint32_t afull_base = cluster_addr(smem_u32(afull), 0);
-        const int stages = pair < p.tiles ? nw * ((p.tiles - pair + npairs - 1) / npairs) : 0;
-        if (warp < 8)
-            decode_set<BF16, 0>(src, dst, wfull, wempty, aempty, afull_base, stages, p.na, lane);
-        else
-            decode_set<BF16, 1>(src, dst, wfull, wempty, aempty, afull_base, stages, p.na, lane);
-    } else if (warp >= 12) {
-        // ------------------------------------------------------------ results: lane = weight row, 32 tokens per load, two warps per
+        int stages = 0;
+        for (Unit u(pair, p); u.live(p); u.next(npairs, p)) stages += u.count(p);
+        decode(stages);
+    } else if (warp >= 4) {
+        // ------------------------------------------------------------ results: lane = weight row, 32 tokens per load, the two (four) warps of a
         // quarter of the rows take alternate loads
+        constexpr int FIRST = SETS == 4 ? 4 : 12, STEP = SETS == 4 ? 128 : 64;
         const int quarter = warp & 3;
         const uint32_t lanes = (uint32_t)(32 * quarter) << 16;
         const uint32_t accempty_base = cluster_addr(smem_u32(accempty), 0);
@@ -234,7 +340,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         const int odd = lane & 1;
         int ab = 0;
         uint32_t cp = 0;
-        for (int tile = pair; tile < p.tiles; tile += npairs) {
+        if (SETS == 2) pdl_wait();  // the row factors come from the kernel before this one
+        for (Unit u(pair, p); u.live(p); u.next(npairs, p)) {
+            const int tile = u.tile;
+            float* part = SPLIT && p.ksplits > 1 ? p.part + (size_t)u.split * p.m * p.rows : nullptr;
+            if (SETS == 4) {
+                decode(u.count(p));
+                pdl_wait();
+            }
             if (!mbar_wait(&accfull[ab], cp)) {
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 break;
@@ -242,11 +355,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             tc_after();
             const int rbase = (tile % p.row_tiles) * 256 + (int)rank * 128 + 32 * quarter, row = rbase + lane, tok0 = (tile / p.row_tiles) * p.tn;
             const int live = min(p.tn, p.m - tok0);
-            for (int c0 = 32 * ((warp - 12) >> 2); c0 < live; c0 += 64) {
+            for (int c0 = 32 * ((warp - FIRST) >> 2); c0 < live; c0 += STEP) {
                 uint32_t v[32];
                 tc_ld32(tmem + lanes + (uint32_t)(ab * p.acc_stride + c0), v);
                 tc_wait_ld();
-                if (BF16 && p.pair_store) {
+                if (SPLIT && part) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++)
+                        if (c0 + i < live && row < p.rows) part[(size_t)(tok0 + c0 + i) * p.rows + row] = __uint_as_float(v[i]);
+                } else if (p.pair_store) {
                     // bf16 rows two at a time: lanes l, l + 1 trade so that the even one holds both rows of token c0 + i, the odd one
                     // both of token c0 + i + 1, and a warp's store is 64 contiguous bytes of each
                     __nv_bfloat16* yp = (__nv_bfloat16*)p.y + (size_t)(tok0 + c0 + odd) * p.ldy + (row & ~1);
@@ -254,7 +371,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                     const bool whole = live - c0 >= 32 && rbase + 32 <= p.rows;
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        const float a = __uint_as_float(v[i]) * gs, b = __uint_as_float(v[i + 1]) * gs;
+                        float a = __uint_as_float(v[i]), b = __uint_as_float(v[i + 1]);
+                        if (BF16)
+                            a *= gs, b *= gs;
+                        else
+                            a *= gs * p.rs[min(tok0 + c0 + i, p.m - 1)], b *= gs * p.rs[min(tok0 + c0 + i + 1, p.m - 1)];
                         const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
                         const __nv_bfloat162 o = __floats2bfloat162_rn(odd ? other : a, odd ? b : other);
                         if (whole || (c0 + i + odd < live && row < p.rows)) *(__nv_bfloat162*)yp = o;
@@ -266,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                         const int tok = tok0 + c0 + i;
                         if (c0 + i < live && row < p.rows) {
                             const float r = __uint_as_float(v[i]) * (BF16 ? gs : gs * p.rs[tok]);
-                            if (BF16)
+                            if (p.out_bf16)
                                 ((__nv_bfloat16*)p.y)[(size_t)tok * p.ldy + row] = __float2bfloat16_rn(r);
                             else
                                 ((float*)p.y)[(size_t)tok * p.ldy + row] = r;
@@ -286,51 +407,134 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     if (warp == 2) tc_dealloc<2>(tmem, TMEM_COLS);
 }
 
-// Tokens per tile: the multiple of 32 up to 256 whose tiles fill the pairs' rounds best. A round costs the longer of the
-// MMAs (2 cycles per token and 64-value block) and the decode (about 300 cycles per block bf16, 170 f16), plus the
-// epilogue where a single accumulator leaves it exposed.
-int pair_tokens(int rows, int nk, int m, int pairs, bool bf16) {
-    const int rt = (rows + 255) / 256, most = (m + 31) / 32 * 32 < 256 ? (m + 31) / 32 * 32 : 256;
+// Tokens per tile, and parts of K: the multiple of 32 up to 256 and the split whose units fill the pairs' rounds best. A round costs the
+// longer of the MMAs (2 cycles per token and 64-value block) and the decode (about 300 cycles per block bf16, 170 f16), plus the
+// epilogue where a single accumulator leaves it exposed. A split adds the partial sums' way through L2 and a kernel that adds them.
+struct PairShape {
+    int tn, ksplits;
+};
+PairShape pair_shape(int rows, int nk, int m, int pairs, bool bf16, int max_splits) {
+    const int rt = (rows + 255) / 256, most = (m + 31) / 32 * 32 < 256 ? (m + 31) / 32 * 32 : 256, nw = nk / 4;
     double best = 1e30;
-    int tn = most;
+    PairShape r = {most, 1};
     for (int n = (m + most - 1) / most; n <= (m + 31) / 32; n++) {  // token tiles
         const int t = ((m + n - 1) / n + 31) / 32 * 32;
         const long long tiles = (long long)rt * ((m + t - 1) / t);
-        const long long rounds = (tiles + pairs - 1) / pairs;
         const double step = 2.0 * t > (bf16 ? 300.0 : 170.0) ? 2.0 * t : (bf16 ? 300.0 : 170.0);
         const double tail = 2500.0 + 16.0 * t;
-        const double cost = rounds * (nk * step + (t > 192 ? tail : 400.0)) + (t > 192 ? 0.0 : tail);
-        if (cost < best) best = cost, tn = t;
+        for (int ks = 1; ks <= max_splits && (ks == 1 || ks <= nw / 2); ks++) {
+            const long long rounds = (tiles * ks + pairs - 1) / pairs;
+            const int blocks = 4 * ((nw + ks - 1) / ks);
+            const double add = ks > 1 ? 5000.0 + (double)ks * m * rows / 300.0 : 0.0;
+            const double cost = rounds * (blocks * step + (t > 192 ? tail : 400.0)) + (t > 192 ? 0.0 : tail) + add;
+            if (cost < best) best = cost, r = {t, ks};
+        }
         if (t <= 64) break;
     }
-    return tn;
+    return r;
 }
+
+// y[t][n] = (sum over splits, in order, of part[s][t][n]) * f * gs * rs[t], four outputs per thread where rows and results allow it
+template <int V>
+__global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, const float* __restrict__ gs, const float* __restrict__ rs, float f, void* __restrict__ y,
+                                          int rows, int m, int ldy, int ksplits, int out_bf16) {
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, t = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (n >= rows) return;
+    float v[V];
+    auto load = [&](int s, float* o) {
+        const float* q = part + ((size_t)s * m + t) * rows + n;
+        if constexpr (V == 4)
+            *(float4*)o = __ldcg((const float4*)q);
+        else
+            o[0] = __ldcg(q);
+    };
+    load(0, v);
+    for (int s = 1; s < ksplits; s++) {
+        float a[V];
+        load(s, a);
+#pragma unroll
+        for (int i = 0; i < V; i++) v[i] += a[i];
+    }
+    const float c = gs[0] * f * (rs ? rs[t] : 1.0f);
+#pragma unroll
+    for (int i = 0; i < V; i++) v[i] *= c;
+    if (out_bf16) {
+        __nv_bfloat16* o = (__nv_bfloat16*)y + (size_t)t * ldy + n;
+        if constexpr (V == 4) {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+            *(uint2*)o = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+        } else {
+            *o = __float2bfloat16_rn(v[0]);
+        }
+    } else {
+        float* o = (float*)y + (size_t)t * ldy + n;
+        if constexpr (V == 4)
+            *(float4*)o = *(float4*)v;
+        else
+            *o = v[0];
+    }
+}
+
+template <bool BF16, bool PACKED, int SETS, bool SPLIT>
+int launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, const PairParams& p, int grid, size_t smem, bool after, cudaStream_t stream) {
+    auto kern = nvfp4_gemm_pair_kernel<BF16, PACKED, SETS, SPLIT>;
+    CN_ALLOW_SMEM(kern, SMEM_MAX);
+    if (after)
+        CN_CUDA(cn_launch_pdl(kern, dim3((unsigned)grid), dim3(PAIR_THREADS), smem, stream, wmap, xmap, p));
+    else
+        kern<<<grid, PAIR_THREADS, smem, stream>>>(wmap, xmap, p);
+    CN_CUDA(cudaGetLastError());
+    return CN_OK;
+}
+
+constexpr int PAIRS = 74;
 
 }  // namespace
 
+int cn_gemm_pair_splits(int rows, int k, int m, bool x_f16, int max_splits) { return pair_shape(rows, k / 64, m, PAIRS, !x_f16, max_splits).ksplits; }
+
 int cn_gemm_pair_launch(const GemmCall& c, cudaStream_t stream) {
-    CUtensorMap wmap, xmap;
+    CUtensorMap wmap = {}, xmap;
     const int nk = c.k / 64;
     PairParams p = {};
-    p.gs = c.gs, p.rs = c.x_f16 ? c.rs : nullptr, p.y = c.y, p.rows = c.rows, p.m = c.m, p.ldy = c.ldy, p.nk = nk;
-    p.pair_store = !((c.rows | c.ldy) & 1) && !((uintptr_t)c.y & 3);
-    const int pairs = 74;
-    p.tn = pair_tokens(c.rows, nk, c.m, pairs, !c.x_f16);
+    p.gs = c.gs, p.rs = c.x_f16 ? c.rs : nullptr, p.y = c.y, p.rows = c.rows, p.m = c.m, p.ldy = c.ldy, p.nk = nk, p.out_bf16 = c.out_bf16;
+    p.pair_store = c.out_bf16 && !((c.rows | c.ldy) & 1) && !((uintptr_t)c.y & 3);
+    p.packed = (const uint8_t*)c.packed, p.packed_tiles = (c.rows + 127) / 128, p.part = c.part;
+    const PairShape shape = pair_shape(c.rows, nk, c.m, PAIRS, !c.x_f16, c.part ? c.max_splits : 1);
+    p.tn = shape.tn, p.ksplits = shape.ksplits, p.split_stages = nk / 4 / shape.ksplits, p.split_more = nk / 4 % shape.ksplits;
     p.acc_stride = p.tn;
     p.nacc = p.tn <= 192 ? 2 : 1;
     p.na = (TMEM_COLS - p.nacc * p.acc_stride) / 32;
     p.na = p.na > 8 ? 8 : p.na & ~1;
-    p.nb = (SMEM_MAX - HDR - 1024 - NW_STAGES * W_STAGE) / (p.tn * 128);
+    p.nb = (SMEM_MAX - HDR - 1024 - 3 * W_STAGE) / (p.tn * 128);
     if (p.nb > 8) p.nb = 8;
+    p.nws = (SMEM_MAX - HDR - 1024 - p.nb * p.tn * 128) / W_STAGE;
+    if (p.nws > MAX_W_STAGES) p.nws = MAX_W_STAGES;
     p.row_tiles = (c.rows + 255) / 256;
     p.tiles = p.row_tiles * ((c.m + p.tn - 1) / p.tn);
-    if (int rc = cn_tmap_2d(&wmap, c.w, 4, (unsigned long long)nk * 9, c.rows, (unsigned long long)nk * 36, 36, 128)) return rc;
+    if (!c.packed)
+        if (int rc = cn_tmap_2d(&wmap, c.w, 4, (unsigned long long)nk * 9, c.rows, (unsigned long long)nk * 36, 36, 128)) return rc;
     if (int rc = cn_tmap_2d(&xmap, c.x, c.x_f16 ? 2 : 3, c.k, c.m, (unsigned long long)c.k * 2, 64, p.tn / 2)) return rc;
-    const size_t smem = HDR + 1024 + (size_t)NW_STAGES * W_STAGE + (size_t)p.nb * p.tn * 128;
-    auto kern = c.x_f16 ? nvfp4_gemm_pair_kernel<false> : nvfp4_gemm_pair_kernel<true>;
-    CN_ALLOW_SMEM(kern, SMEM_MAX);
-    const int grid = 2 * (p.tiles < pairs ? p.tiles : pairs);
-    kern<<<grid, PAIR_THREADS, smem, stream>>>(wmap, xmap, p);
-    CN_CUDA(cudaGetLastError());
+    const size_t smem = HDR + 1024 + (size_t)p.nws * W_STAGE + (size_t)p.nb * p.tn * 128;
+    const int units = p.tiles * p.ksplits, grid = 2 * (units < PAIRS ? units : PAIRS);
+    const bool four = c.x_f16 && p.tn <= 128;  // (eight A slots then: every set has its own)
+    int rc = CN_ERR_SHAPE;
+#define CN_PAIR_CASE(BF16V, PACKEDV, SETSV, SPLITV)                                                                                       \
+    if (!c.x_f16 == BF16V && (c.packed != nullptr) == PACKEDV && four == (SETSV == 4) && (c.x_f16 || p.ksplits > 1) == SPLITV)             \
+        rc = launch_pair<BF16V, PACKEDV, SETSV, SPLITV>(wmap, xmap, p, grid, smem, c.x_f16, stream);
+    CN_PAIR_CASE(true, false, 2, false) CN_PAIR_CASE(true, false, 2, true) CN_PAIR_CASE(false, false, 2, true) CN_PAIR_CASE(false, false, 4, true)
+    CN_PAIR_CASE(true, true, 2, false) CN_PAIR_CASE(true, true, 2, true) CN_PAIR_CASE(false, true, 4, true)
+#undef CN_PAIR_CASE
+    if (rc || p.ksplits == 1) return rc;
+    const float f = c.x_f16 ? F16_UNSCALE : BF16_UNSCALE;
+    const bool wide = !((c.rows | c.ldy) & 3) && !((uintptr_t)c.y & 15);
+    if (wide)
+        CN_CUDA(cn_launch_pdl(gemm_splitk_reduce_kernel<4>, dim3((unsigned)((c.rows / 4 + 127) / 128), (unsigned)c.m), dim3(128), 0, stream, p.part, c.gs, p.rs, f, c.y,
+                              c.rows, c.m, c.ldy, p.ksplits, c.out_bf16));
+    else
+        CN_CUDA(cn_launch_pdl(gemm_splitk_reduce_kernel<1>, dim3((unsigned)((c.rows + 127) / 128), (unsigned)c.m), dim3(128), 0, stream, p.part, c.gs, p.rs, f, c.y,
+                              c.rows, c.m, c.ldy, p.ksplits, c.out_bf16));
     return CN_OK;
 }

@@ -97,9 +97,9 @@ class Fp4Packed:
 
 
 def launch_gemm_fp4(w: Fp4Packed, x, y=None, workspace=None):
-    """Y[t][n] = gs * sum_k X[t][k] W[n][k] on the block-scaled FP4 MMA (tcgen05 kind::mxf4nvf4): gemm_fp4_dense
-    (engine/src/kernels.rs:533) with the activations as a five-level NVFP4 cascade (the reference's act_cascade,
-    engine/src/kernels.rs:5354-5475, has three)."""
+    """Y[t][n] = gs * sum_k X[t][k] W[n][k] on the re-laid weights (gemm_fp4_dense, engine/src/kernels.rs:533). bf16 rows are multiplied as they
+    are or as f16, exactly; f32 rows go through the block-scaled FP4 MMA (tcgen05 kind::mxf4nvf4) as a five-level NVFP4 cascade (the
+    reference's act_cascade, engine/src/kernels.rs:5354-5475, has three)."""
     x2 = x.reshape(-1, w.cols)
     m = x2.shape[0]
     if y is None:

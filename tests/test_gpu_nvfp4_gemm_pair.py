@@ -63,3 +63,38 @@ def test_results_in_the_place_of_the_activations(rows, k, at, dtype):
     ops.launch_gemm(w, xs, ys)
     assert torch.equal(ys, want)
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("relaid", [False, True])
+@pytest.mark.parametrize("rows,k,m", [(100, 256, 1), (256, 512, 33), (333, 4096, 9), (600, 4096, 64), (1030, 2048, 65), (5120, 1280, 128), (130, 8192, 129),
+                                      (384, 5120, 300), (512, 1024, 513)])
+def test_few_rows_split_k_and_relaid_weights(rows, k, m, relaid):
+    """Rows at the edges of the f16 path (1, 128, 129 rows), of the split of K (512, 513 rows; one, a few and eight parts) and of the tiles; container
+    bytes and stage images (an odd count of 128-row tiles leaves a CTA of the last pair without one)."""
+    rng = np.random.default_rng(rows + m)
+    w = synth.nvfp4_matrix(rows, k, rng).copy()
+    w.reshape(-1, 36)[::7, 1] = 0x7F
+    w.reshape(-1, 36)[::5, 2] |= 0x80
+    fw = ops.Fp4.from_host(w, rows, k, np.float32(0.37))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda()
+    x[m // 2] *= 1e-6
+    x = x.to(torch.bfloat16)
+    want = x.double() @ ops.dequant(fw, rule=True).double().view(rows, k).t()
+    if relaid:
+        packed = ops.Fp4Packed(fw)
+        run = lambda xs, ys=None: ops.launch_gemm_fp4(packed, xs, ys)
+    else:
+        run = lambda xs, ys=None: ops.launch_gemm(fw, xs, ys)
+    y = run(x)
+    # one rounding of the result to bf16 (half a unit of 2^-7: at most 2^-8 of the value) beside f32 sums (1e-6 of the row's scale, see the other GEMM tests)
+    rms = want.pow(2).mean(dim=1, keepdim=True).sqrt()
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * rms).all()
+    # results over the activations, and in rows further apart than they are long
+    buf = torch.zeros(2 * m * max(rows, k) + 64, dtype=torch.bfloat16, device="cuda")
+    xs, ys = buf[:m * k].view(m, k), buf[16:16 + m * rows].view(m, rows)
+    xs.copy_(x)
+    assert torch.equal(run(xs, ys), y)
+    wide = torch.zeros((m, rows + 6), dtype=torch.bfloat16, device="cuda")
+    run(x, wide[:, :rows])
+    assert torch.equal(wide[:, :rows], y) and not wide[:, rows:].any()
+    assert device_status() == 0
