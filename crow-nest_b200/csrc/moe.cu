@@ -11,6 +11,7 @@
 // step (repeats are L2 hits); gate, up and the activation are one launch; a null table entry
 // skips the combo (the expert lives on another rank).
 #include "common.cuh"
+#include "moe_step.cuh"
 #include "nvfp4_gemv.cuh"
 
 namespace {
@@ -336,17 +337,26 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
     return rc;
 }
 
+// Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
+constexpr int GROUP_COMBOS = 48;
+
+// Routed gate|up of the combos as they come (nearly every CTA of a small step is resident at once and L2 serves an expert's second
+// reader).
+GemvCall routed_gate_up(const MoePlan* p, const unsigned long long* table_gu, const unsigned long long* table_up, const float* gs_gu, const float* gs_up,
+                        const int32_t* ids, const void* x, int combos, int x_div, float limit, int dtype) {
+    GemvCall a = {};
+    a.gs0 = gs_gu, a.gs1 = gs_up ? gs_up : gs_gu, a.x = x, a.y = p->h, a.rows = p->inter, a.k = p->hidden, a.m = 1, a.ldy = p->inter;
+    a.limit = limit, a.dtype = dtype, a.out_f32 = 1, a.ids = ids, a.order = nullptr, a.tab0 = table_gu, a.tab1 = table_up;
+    a.fused_up_rows = table_up ? 0 : p->inter, a.x_div = x_div, a.combos = combos, a.experts = p->experts;
+    return a;
+}
+
 // routed gate|up + activation, then routed down, one launch each over `combos` (token, pick) pairs: combo c reads
 // activation row c / x_div and writes eo row c (or to eo_ptrs[c] when given: a row of another buffer, e.g. in a peer's memory)
 int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigned long long* table_up, const unsigned long long* table_dn,
                    const float* gs_gu, const float* gs_up, const float* gs_dn, const int32_t* ids, const void* x, float* eo,
                    const unsigned long long* eo_ptrs, int combos, int x_div, float limit, int dtype, cudaStream_t stream) {
-    // Routed gate|up of the combos as they come (nearly every CTA of a small step is resident at once and L2 serves an
-    // expert's second reader).
-    GemvCall a = {};
-    a.gs0 = gs_gu, a.gs1 = gs_up ? gs_up : gs_gu, a.x = x, a.y = p->h, a.rows = p->inter, a.k = p->hidden, a.m = 1, a.ldy = p->inter;
-    a.limit = limit, a.dtype = dtype, a.out_f32 = 1, a.ids = ids, a.order = nullptr, a.tab0 = table_gu, a.tab1 = table_up;
-    a.fused_up_rows = table_up ? 0 : p->inter, a.x_div = x_div, a.combos = combos, a.experts = p->experts;
+    const GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, combos, x_div, limit, dtype);
     // From 48 combos on the combos are sorted by expert and cut into groups that share one decode of the expert's weights
     // (nvfp4_rows.cu): the down projection in groups of up to two rows (its rows are f32), gate|up in groups of up to eight bf16 rows
     // where enough of them share an expert (three combo slots for four experts), two f32 rows always. Measured, us per step of
@@ -354,7 +364,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     // experts of 2560 x 1280, top 6: 8 tokens 117 / 106 / 132, 32 tokens 390 / 306 / 267; 288 experts of 4096 x 2048, top 8: 16 tokens
     // 515 / 401 / 440, 32 tokens 956 / 693 / 590; 64 tokens of f32 rows, 512 experts: 614 / 500 / 343. With 40 combos nothing is gained
     // (48 / 48 / 59): the grouping is a launch of its own.
-    if (combos >= 48 && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
+    if (combos >= GROUP_COMBOS && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
         int* ga = p->groups;
         int* gb = ga + combos;
         int* gbrows = gb + combos;
@@ -460,6 +470,20 @@ extern "C" int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, 
     if (dtype == CN_BF16_IN_F32_OUT) dtype = CN_BF16;
     const float* shared = nullptr;
     int rc = CN_OK;
+    if (tokens * p->topk < GROUP_COMBOS) {
+        // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine.
+        MoeDownCall d = {};
+        d.ids = ids, d.wts = wts, d.table = table_dn, d.experts = p->experts, d.topk = p->topk, d.h = p->h, d.gs = gs_dn, d.inter = p->inter;
+        d.shared = shared_gate ? shared_down : nullptr, d.hs = p->hs, d.shared_gs = shared_gs ? shared_gs + 2 : nullptr, d.sgate = sgate;
+        d.shared_inter = p->shared_inter, d.y = y, d.tokens = tokens, d.hidden = p->hidden, d.out_bf16 = ydtype == CN_BF16;
+        if (cn_moe_down_combine_fits(d)) {
+            GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, tokens * p->topk, p->topk, limit, dtype);
+            if (shared_gate)
+                a.side_w0 = shared_gate, a.side_w1 = shared_up, a.side_gs = shared_gs, a.side_y = p->hs, a.side_rows = p->shared_inter, a.side_tokens = tokens;
+            if ((rc = cn_gemv_launch(a, stream, "cn_moe_nvfp4_run (gate/up)"))) return rc;
+            return cn_moe_down_combine_launch(d, stream);
+        }
+    }
     if (shared_gate) {
         rc = shared_branch(p, shared_gate, shared_up, shared_down, shared_gs, x, tokens, limit, dtype, stream);
         shared = p->ys;

@@ -86,19 +86,28 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
     const uint8_t* w1 = p.w1;
     const char* xbase = (const char*)p.x;
     char* ybase = (char*)p.y;
+    int rows = p.rows;
+    const float *gs0 = p.gs0, *gs1 = p.gs1;
     if (p.ids) {
         // ids, order and tables may come from the kernels just before this one, and a CTA whose expert is not resident
         // returns at once: wait for the predecessor grid first, so that even a grid whose CTAs all return early
         // completes only after its predecessor has
         pdl_wait();
-        const int c = p.order ? p.order[blockIdx.y] : (int)blockIdx.y;
-        const int e = p.ids[c];
-        if (e < 0 || (p.experts > 0 && e >= p.experts)) return;  // uniform over the CTA, before any barrier
-        w0 = (const uint8_t*)p.tab0[e];
-        if (!w0) return;  // the expert is not resident here: nothing to read or write
-        w1 = p.tab1 ? (const uint8_t*)p.tab1[e] : (p.fused_up_rows > 0 ? w0 + (size_t)p.fused_up_rows * row_bytes : nullptr);
-        xbase += (size_t)(c / p.x_div) * p.k * (XT == 1 ? 2 : 4);
-        ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * ((XT == 1 && !p.out_f32) ? 2 : 4);
+        if ((int)blockIdx.y >= p.combos) {  // a row of the side pair
+            const int row = (int)blockIdx.y - p.combos;
+            w0 = p.side_w0, w1 = p.side_w1, rows = p.side_rows, gs0 = p.side_gs, gs1 = p.side_gs + 1;
+            xbase += (size_t)row * p.k * (XT == 1 ? 2 : 4);
+            ybase = (char*)(p.side_y + (size_t)row * rows);
+        } else {
+            const int c = p.order ? p.order[blockIdx.y] : (int)blockIdx.y;
+            const int e = p.ids[c];
+            if (e < 0 || (p.experts > 0 && e >= p.experts)) return;  // uniform over the CTA, before any barrier
+            w0 = (const uint8_t*)p.tab0[e];
+            if (!w0) return;  // the expert is not resident here: nothing to read or write
+            w1 = p.tab1 ? (const uint8_t*)p.tab1[e] : (p.fused_up_rows > 0 ? w0 + (size_t)p.fused_up_rows * row_bytes : nullptr);
+            xbase += (size_t)(c / p.x_div) * p.k * (XT == 1 ? 2 : 4);
+            ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * ((XT == 1 && !p.out_f32) ? 2 : 4);
+        }
     }
     const bool gu = w1 != nullptr;
 
@@ -115,6 +124,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
     // output rows of this CTA: plain ROWS consecutive rows; gate/up ROWS/2 consecutive indices
     const int per_cta = gu ? ROWS / 2 : ROWS;
     const int row0 = blockIdx.x * per_cta;
+    if (row0 >= rows) return;  // routed and side matrices of one launch may differ in rows
 
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
@@ -126,7 +136,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
     }
     // scale tables: ue4m3(rule(byte)) * gs, the product the reference tabulates (cpu_nvfp4.rs:98)
     {
-        const float g0 = p.gs0[0], g1 = gu ? p.gs1[0] : g0;
+        const float g0 = gs0[0], g1 = gu ? gs1[0] : g0;
         for (int b = tid; b < 256; b += NTHREADS) {
             const float u = ue4m3_f32((uint32_t)b, true);
             lut[b] = u * g0;
@@ -151,7 +161,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
                 const int j = sl / G, g = sl % G;
                 const int r = gu ? row0 + (j >> 1) * G + g : row0 + sl;
                 const uint8_t* base = (gu && (j & 1)) ? w1 : w0;
-                if (r < p.rows) src[i] = base + (size_t)r * row_bytes;
+                if (r < rows) src[i] = base + (size_t)r * row_bytes;
             }
             total += src[i] ? piece : 0;
         }
@@ -416,7 +426,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
 #pragma unroll
             for (int r = 0; r < RT; r++) {
                 const int row = row0 + r * G + g;
-                if (row < p.rows) {
+                if (row < rows) {
 #pragma unroll
                     for (int m = 0; m < MP; m++)
                         if (m < p.m) {
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
 #pragma unroll
             for (int r = 0; r + 1 < RT; r += 2) {
                 const int row = row0 + (r >> 1) * G + g;
-                if (row < p.rows) {
+                if (row < rows) {
 #pragma unroll
                     for (int m = 0; m < MP; m++)
                         if (m < p.m) {
@@ -502,7 +512,7 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (m < 1 || m > CN_MAX_M) CN_FAIL(CN_ERR_LIMIT, "%s: m = %d, the kernel takes 1..%d activation rows", who, m, CN_MAX_M);
     if (a.ldy < rows) CN_FAIL(CN_ERR_SHAPE, "%s: ldy %d < rows %d", who, a.ldy, rows);
     if (a.dtype != CN_F32 && a.dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "%s: dtype %d is neither CN_F32 nor CN_BF16", who, a.dtype);
-    if (((uintptr_t)a.w0 & 15) || ((uintptr_t)a.w1 & 15) || ((uintptr_t)a.x & 15))
+    if (((uintptr_t)a.w0 & 15) || ((uintptr_t)a.w1 & 15) || ((uintptr_t)a.x & 15) || (((uintptr_t)a.side_w0 | (uintptr_t)a.side_w1) & 15))
         CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
     const bool routed = a.ids != nullptr;
     if (routed && (m != 1 || a.combos < 1 || a.x_div < 1)) CN_FAIL(CN_ERR_SHAPE, "%s: the routed form takes one row per combo", who);
@@ -526,14 +536,14 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (slots / (G * 4) < 2 * 148) rt = 2;
     const int ROWS = G * rt;
     const int per_cta = gu ? ROWS / 2 : ROWS;
-    const int grid = (rows + per_cta - 1) / per_cta;
+    const int grid = ((routed && a.side_tokens > 0 && a.side_rows > rows ? a.side_rows : rows) + per_cta - 1) / per_cta;
     const int xb = (mode == 1 && a.dtype == CN_BF16) ? XB_SWZ : (mode == 1 ? XB_F16 : XB_F32);
     const size_t stage_bytes = (size_t)ROWS * tx * 36;
     const size_t xbytes = (size_t)mp * bpr * xb + (size_t)((mp * bpr + 3) & ~3) * 4;
     const int nchunks = bpr / tx;
     // ring depth: enough bytes in flight per SM to cover the HBM latency (about 96 KB), shared between
     // the CTAs that will be resident together (at most four, fewer when the grid is small)
-    const long long total_ctas = (long long)grid * (routed ? a.combos : 1);
+    const long long total_ctas = (long long)grid * (routed ? a.combos + a.side_tokens : 1);
     int resident = (int)((total_ctas + 147) / 148);
     resident = resident < 1 ? 1 : (resident > 4 ? 4 : resident);
     long long want = (96 * 1024) / resident;                                         // in-flight bytes per CTA
@@ -562,7 +572,9 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.rows = rows, p.k = k, p.m = m, p.ldy = a.ldy, p.limit = a.limit, p.tx = tx, p.stages = stages, p.out_f32 = a.out_f32;
     p.ids = a.ids, p.order = a.order, p.tab0 = a.tab0, p.tab1 = a.tab1, p.fused_up_rows = a.fused_up_rows, p.x_div = a.x_div;
     p.experts = a.experts, p.yptrs = a.yptrs;
-    const int gy = routed ? a.combos : 1;
+    p.combos = a.combos, p.side_w0 = (const uint8_t*)a.side_w0, p.side_w1 = (const uint8_t*)a.side_w1, p.side_gs = a.side_gs, p.side_y = a.side_y;
+    p.side_rows = a.side_rows;
+    const int gy = routed ? a.combos + a.side_tokens : 1;
     if (a.dtype == CN_BF16) return mode == 1 ? launch_m<1, 1>(p, mp, rt, grid, gy, smem, stream) : launch_m<1, 0>(p, mp, rt, grid, gy, smem, stream);
     return mode == 1 ? launch_m<0, 1>(p, mp, rt, grid, gy, smem, stream) : launch_m<0, 0>(p, mp, rt, grid, gy, smem, stream);
 }

@@ -23,6 +23,12 @@ struct GemvCall {
     int fused_up_rows, x_div, combos;
     int experts;  // entries of the tables (0 = unknown: ids are trusted); an id beyond them skips the combo
     const unsigned long long* yptrs;  // routed form: output row address per combo (null: y + combo * ldy); may name peer memory
+    // routed gate/up form: side_tokens > 0 rows more of the same launch, row t of x through the pair side_w0 / side_w1 (side_rows rows, tensor
+    // scales side_gs[0] and [1]) to side_y + t * side_rows: the shared expert beside the routed ones
+    const void *side_w0, *side_w1;
+    const float* side_gs;
+    float* side_y;
+    int side_rows, side_tokens;
     // Tensor-parallel line output (one bf16 activation row, plain or gate/up form): besides y, the output rows go out as
     // 16-byte lines {two rows, number, two rows, number} to the line buffers of the other ranks, where number =
     // *line_epoch * 4096 + line_tag and the buffer used is line_buf ^ (line_flip & *line_epoch & 1).
@@ -70,6 +76,11 @@ struct GemvParams {
     int x_div;
     int experts;  // entries of tab0 / tab1 (0 = unknown); ids outside 0..experts-1 skip the combo
     const unsigned long long* yptrs;  // output row address per combo (null: y + combo * ldy)
+    int combos;                       // routed form: blockIdx.y beyond them is a row of the side pair (see GemvCall)
+    const uint8_t *side_w0, *side_w1;
+    const float* side_gs;
+    float* side_y;
+    int side_rows;
     int red_depth;  // multi-row tensor-core kernel: tile-sum slots in flight
     // tensor-parallel line output (see GemvCall): line buffer of every rank (0 = none), first global row, the counter
     unsigned long long yl[8];

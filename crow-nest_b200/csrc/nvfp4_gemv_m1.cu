@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     static_assert(PP == 1 || MT > 1, "one activation row has a CTA for every part");
     extern __shared__ __align__(128) uint8_t smem[];
     if (threadIdx.x == 0) { CN_STAMP(0); }
-    const float gs0_early = __ldg(p.gs0), gs1_early = __ldg(p.gs1);  // tensor scales: asked for first, used late
+    float gs0_early = __ldg(p.gs0), gs1_early = __ldg(p.gs1);  // tensor scales: asked for first, used late
+    int rows = p.rows;
     constexpr int pstride = TX * 36 + 16;  // padded: the eight rows of a quad column hit distinct banks
     constexpr int stage_bytes = ROWS * pstride;
     constexpr int GPW = TX / 2 / NW > 0 ? TX / 2 / NW : 1;  // groups per warp and full chunk
@@ -150,14 +151,22 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
         // a grid in which every CTA returns early still completes only after its predecessor has, and a later
         // kernel's wait on this grid keeps covering the whole chain.
         pdl_wait();
-        const int c = p.order ? p.order[blockIdx.y] : (int)blockIdx.y;
-        const int e = p.ids[c];
-        if (e < 0 || (p.experts > 0 && e >= p.experts)) return;  // uniform over the CTA, before any barrier
-        w0 = (const uint8_t*)p.tab0[e];
-        if (!w0) return;
-        w1 = p.tab1 ? (const uint8_t*)p.tab1[e] : (p.fused_up_rows > 0 ? w0 + (size_t)p.fused_up_rows * row_bytes : nullptr);
-        xbase += (size_t)(c / p.x_div) * p.k * 2;
-        ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * (p.out_f32 ? 4 : 2);
+        if ((int)blockIdx.y >= p.combos) {  // a row of the side pair
+            const int row = (int)blockIdx.y - p.combos;
+            w0 = p.side_w0, w1 = p.side_w1, rows = p.side_rows;
+            gs0_early = __ldg(p.side_gs), gs1_early = __ldg(p.side_gs + 1);
+            xbase += (size_t)row * p.k * 2;
+            ybase = (char*)(p.side_y + (size_t)row * rows);
+        } else {
+            const int c = p.order ? p.order[blockIdx.y] : (int)blockIdx.y;
+            const int e = p.ids[c];
+            if (e < 0 || (p.experts > 0 && e >= p.experts)) return;  // uniform over the CTA, before any barrier
+            w0 = (const uint8_t*)p.tab0[e];
+            if (!w0) return;
+            w1 = p.tab1 ? (const uint8_t*)p.tab1[e] : (p.fused_up_rows > 0 ? w0 + (size_t)p.fused_up_rows * row_bytes : nullptr);
+            xbase += (size_t)(c / p.x_div) * p.k * 2;
+            ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * (p.out_f32 ? 4 : 2);
+        }
     }
     const bool gu = w1 != nullptr;
 
@@ -177,7 +186,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int per_cta = gu ? ROWS / 2 : ROWS;  // gate/up: 8 indices, row slots 0-7 gate, 8-15 up
-    const int ntiles = (p.rows + per_cta - 1) / per_cta;
+    const int ntiles = (rows + per_cta - 1) / per_cta;
 
     // The producer warp sets up the ring's barriers itself and starts streaming at once (the weights do not
     // depend on the previous kernel); the consumers meet it on named barrier 2 before their first wait.
@@ -209,7 +218,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
             const int row0 = tile * per_cta;
             const int row = gu ? row0 + (lane & 7) : row0 + lane;
             const uint8_t* base = (gu && ((lane >> 3) & 1)) ? w1 : w0;
-            const uint8_t* src = (lane < ROWS && row < p.rows) ? base + (size_t)row * row_bytes : nullptr;
+            const uint8_t* src = (lane < ROWS && row < rows) ? base + (size_t)row * row_bytes : nullptr;
             const uint32_t nvalid = (uint32_t)__popc(__ballot_sync(0xffffffffu, src != nullptr));
             for (int c = 0; c < nch; c++) {
                 const int nblk = min(TX, bpr - c * TX);
@@ -563,7 +572,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                         const float up = __shfl_down_sync(0xffffffffu, tot[i], 8);
                         const int row = tile * per_cta + slot;
                         const float r = gu ? act_gu(tot[i], up, p.limit) : tot[i];
-                        if (slot < per_cta && row < p.rows && m < p.m) {
+                        if (slot < per_cta && row < rows && m < p.m) {
                             if (p.out_f32)
                                 ((float*)ybase)[(size_t)m * p.ldy + row] = r;
                             else
@@ -606,7 +615,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                         const float up = __shfl_down_sync(0xffffffffu, v[i], 8);
                         const int row = tile * per_cta + slot;
                         const float r = gu ? act_gu(v[i], up, p.limit) : v[i];
-                        if (slot < per_cta && row < p.rows && m < p.m) {
+                        if (slot < per_cta && row < rows && m < p.m) {
                             if (p.out_f32)
                                 ((float*)ybase)[(size_t)m * p.ldy + row] = r;
                             else
@@ -638,13 +647,13 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                         const float up = __shfl_down_sync(0xffffffffu, v, 8);
                         const int row = tile * per_cta + lane;
                         const float r = gu ? act_gu(v, up, p.limit) : v;
-                        if (lane < per_cta && row < p.rows) {
+                        if (lane < per_cta && row < rows) {
                             if (p.out_f32)
                                 ((float*)ybase)[row] = r;
                             else
                                 ((__nv_bfloat16*)ybase)[row] = __float2bfloat16_rn(r);
                         }
-                        if (LN) push_lines(p, tile * per_cta, min(per_cta, p.rows - tile * per_cta), r, lane, line_seq, line_buf);
+                        if (LN) push_lines(p, tile * per_cta, min(per_cta, rows - tile * per_cta), r, lane, line_seq, line_buf);
                     }
                 }
             } else if (LN) {
@@ -659,8 +668,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                     }
                 }
                 const float v = gu ? act_gu(v0, v1, p.limit) : v0;
-                if (lane < per_cta && row < p.rows) ((__nv_bfloat16*)ybase)[row] = __float2bfloat16_rn(v);
-                push_lines(p, tile * per_cta, min(per_cta, p.rows - tile * per_cta), v, lane, line_seq, line_buf);
+                if (lane < per_cta && row < rows) ((__nv_bfloat16*)ybase)[row] = __float2bfloat16_rn(v);
+                push_lines(p, tile * per_cta, min(per_cta, rows - tile * per_cta), v, lane, line_seq, line_buf);
             } else if (lane < per_cta) {
                 const int row = tile * per_cta + lane;
 #pragma unroll
@@ -670,7 +679,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                         v0 += rb[(w * MT + m) * 16 + lane];
                         if (gu) v1 += rb[(w * MT + m) * 16 + lane + 8];
                     }
-                    if (row < p.rows && m < p.m) {
+                    if (row < rows && m < p.m) {
                         const float v = gu ? act_gu(v0, v1, p.limit) : v0;
                         if (p.out_f32)
                             ((float*)ybase)[(size_t)m * p.ldy + row] = v;
@@ -761,7 +770,8 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int tx = bpr >= 32 ? 32 : 16;
     const long long stage_bytes = stage_bytes_of(tx);
     const int per_cta = gu ? ROWS / 2 : ROWS;
-    const int ntiles = (rows + per_cta - 1) / per_cta;
+    const int ntiles = ((routed && a.side_tokens > 0 && a.side_rows > rows ? a.side_rows : rows) + per_cta - 1) / per_cta;
+    const int combos = a.combos + (routed ? a.side_tokens : 0);
     Split one = {1, 0};
     if (!routed) one = one_row_split(ntiles, bpr, tx);
     const int parts = one.parts, bpp = bpr / parts;  // parts of K (each longer than a chunk where there are several), blocks of one
@@ -771,15 +781,15 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // persistent CTAs, each walking its share of the tiles (the routed form keeps one tile per CTA)
     int grid = ntiles;
     if (!routed && grid > 148 * cps) grid = 148 * cps;
-    if (routed && (long long)ntiles * a.combos > 3LL * 148 * cps / 2) {
+    if (routed && (long long)ntiles * combos > 3LL * 148 * cps / 2) {
         // many combos: a few persistent CTAs per combo (the activation row is staged once per CTA), about one wave in all
-        grid = 148 * cps / a.combos;
+        grid = 148 * cps / combos;
         if (grid <= 2) {
             // combos near or beyond the CTA slots: 1..6 CTAs per combo, whichever fills the last wave best (fewer on a near tie)
             const double slots = 148.0 * cps;
             double best = 0.0;
             for (int gx = 1; gx <= 6 && gx <= ntiles; gx++) {
-                const double waves = gx * (double)a.combos / slots, eff = waves / (double)(long long)(waves + 0.999999);
+                const double waves = gx * (double)combos / slots, eff = waves / (double)(long long)(waves + 0.999999);
                 if (eff > best + 0.03) best = eff, grid = gx;
             }
             if (grid < 1) grid = 1;
@@ -836,6 +846,8 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.ids = a.ids, p.order = a.order, p.tab0 = a.tab0, p.tab1 = a.tab1, p.fused_up_rows = a.fused_up_rows, p.x_div = a.x_div;
     p.red_depth = red_slots(stages, gap(pp), pp);
     p.experts = a.experts, p.yptrs = a.yptrs;
+    p.combos = a.combos, p.side_w0 = (const uint8_t*)a.side_w0, p.side_w1 = (const uint8_t*)a.side_w1, p.side_gs = a.side_gs, p.side_y = a.side_y;
+    p.side_rows = a.side_rows;
     p.yl_world = 0, p.yl_row0 = 0, p.yl_stride = 0, p.yl_epoch = nullptr, p.yl_tag = 0, p.yl_buf = 0, p.yl_flip = 0;
     for (int d = 0; d < 8; d++) p.yl[d] = 0ull;
     if (a.line_bases) {
@@ -851,7 +863,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.trace = (g_m1_trace && g_m1_trace_i < g_m1_trace_n && !routed) ? g_m1_trace + (size_t)(g_m1_trace_i++) * 512 * 8 : nullptr;
 #endif
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, (unsigned)(routed ? a.combos : 1));
+    cfg.gridDim = dim3((unsigned)grid, (unsigned)(routed ? combos : 1));
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
