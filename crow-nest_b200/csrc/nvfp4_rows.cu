@@ -9,7 +9,7 @@
 // by its own bulk copies (16 row pieces of up to eight blocks, two to four chunks ahead), holds all its sums in registers and stores
 // them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
 // columns) share one decode of its weights; a row's sum does not depend on the rows it is grouped with. Bound by issue slots:
-// some 200 warp instructions per 16 x 128 values in all, 0.59 of the slots. Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
+// some 180 warp instructions per 16 x 128 values in all (200 and 258 us a step with one scale made at a time, 245 now). Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
 // the profiler): gate/up 157 -> 133 us, down 203 -> 86 us against one CTA set per combo.
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"
@@ -48,7 +48,6 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
     const int nch = (bpr + CB - 1) / CB, D = p.depth;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint64_t* full = (uint64_t*)smem + warp * MAX_D;
-    const uint32_t base = smem_u32(smem);
     uint8_t* ring = smem + p.ring_off + (size_t)warp * D * CHUNK;
     const int mytiles = t0 + warp < t1 ? (t1 - t0 - warp + NW - 1) / NW : 0, total = mytiles * nch;
     if (lane == 0) {
@@ -120,11 +119,10 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
 
         const int g = lane >> 2, t = lane & 3;
         const int col = g < ncol ? g : (ncol > 1 ? g & 1 : 0);  // a column beyond the live ones repeats one of them and is not read
-        const uint32_t xa = base + p.x_off + (uint32_t)(col * bpr * 128 + (col & 1) * 64 + t * 16);
-        const uint32_t xflip = (col & 1) ? (uint32_t)-64 : 64u;
-        const uint32_t xi0 = base + p.inv_off + 8u * (uint32_t)t;
-        const uint32_t sel0 = (t >> 1) ? 0x4141u : 0x4040u, sel1 = sel0 + 0x0202u;
-        const uint32_t rbase = smem_u32(ring) + (uint32_t)(g * PITCH + 4 * t);
+        const uint8_t* xa = smem + p.x_off + (size_t)col * bpr * 128 + (col & 1) * 64 + t * 16;
+        const int xflip = (col & 1) ? -64 : 64;
+        const uint8_t* xi0 = smem + p.inv_off + 8 * t;
+        const uint8_t* rbase = ring + g * PITCH + 4 * t;
         int done = 0;
         bool ok = true;
         for (int tile = t0 + warp; tile < t1 && ok; tile += NW) {
@@ -142,29 +140,16 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
                     break;
                 }
                 const int nb = min(CB, bpr - ch * CB);
-                const uint32_t cbase = rbase + (uint32_t)(s * CHUNK), xc = xa + (uint32_t)(ch * CB * 128), xic = xi0 + (uint32_t)(ch * CB * 32);
+                const uint8_t *cbase = rbase + s * CHUNK, *xc = xa + ch * (CB * 128), *xic = xi0 + ch * (CB * 32);
                 auto block = [&](int b) {
-                    const uint32_t pw = cbase + 36u * b, pw8 = pw + 8u * PITCH;
-                    const uint32_t sa = lds32(pw - 4u * t), sb = lds32(pw8 - 4u * t);
-                    float cc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int hf = 0; hf < 2; hf++) {
-                        uint32_t ha[4], hb[4];
-                        e2m1x8_to_f16x2(lds32(pw + 4u + 16u * hf), ha);
-                        e2m1x8_to_f16x2(lds32(pw8 + 4u + 16u * hf), hb);
-                        const uint32_t fa = scale_f16x2(sa, hf ? sel1 : sel0), fb = scale_f16x2(sb, hf ? sel1 : sel0);
-#pragma unroll
-                        for (int i = 0; i < 4; i++) ha[i] = hmul2u(ha[i], fa), hb[i] = hmul2u(hb[i], fb);
-                        const uint4 xv = lds128(xc + b * 128u + (hf ? xflip : 0u));
-                        mma16816(cc, ha[0], hb[0], ha[1], hb[1], xv.x, xv.y);
-                        mma16816(cc, ha[2], hb[2], ha[3], hb[3], xv.z, xv.w);
-                    }
-                    const float2 xi = lds64f(xic + b * 32u);
+                    float cc[1][4];
+                    block_mma<1>(cc, cbase + 36 * b, cbase + 36 * b + 8 * PITCH, t, [&](int, int hf) { return *(const uint4*)(xc + b * 128 + (hf ? xflip : 0)); });
+                    const float2 xi = *(const float2*)(xic + b * 32);
                     float* a = acc[NA > 1 ? b : 0];
-                    a[0] = fmaf(cc[0], xi.x, a[0]);
-                    a[1] = fmaf(cc[1], xi.y, a[1]);
-                    a[2] = fmaf(cc[2], xi.x, a[2]);
-                    a[3] = fmaf(cc[3], xi.y, a[3]);
+                    a[0] = fmaf(cc[0][0], xi.x, a[0]);
+                    a[1] = fmaf(cc[0][1], xi.y, a[1]);
+                    a[2] = fmaf(cc[0][2], xi.x, a[2]);
+                    a[3] = fmaf(cc[0][3], xi.y, a[3]);
                 };
                 if (nb == CB) {
 #pragma unroll
