@@ -16,7 +16,10 @@
 //            one HFMA2 to the codec's f16 weights (bit-exact) and accumulates with f16 x f16 -> f32
 //            mixed FMAs; partial sums of the k-split go to scratch
 //   had_out  y = H128(sum of partials) / 128 * svh
-// The inner loop is instruction-bound, not HBM-bound: about 7 issue slots per 3-bit weight.
+// The first step is part of the GEMV launch for x (every CTA transforms its k-split) and a kernel of its own, with the activation, for h; the
+// last one carries the weighted combine of a routed step. One token, four experts of 4096 x 1536: eight launches 52.5 us, five 43.4.
+// The inner loop is instruction-bound, not HBM-bound: about 7 issue slots per 3-bit weight. A stage is a whole 128-row block of eight tiles: with
+// four the waits and counters of a stage cost 21 of the 70 instructions a tile (16 tokens 280 us a step against 296).
 // Three helpers restate reference text because their operation order defines the bits the parity contract asks for:
 // fwht128 follows mul1_fwht128 (engine/src/kernels_mul1.cu:74-88: the stage order and the a+b / a-b pairing), out_block
 // follows mul1_out_block (:98-110: partial sums left to right, then the transform, 1/128 and the scale), mul1_pair follows
@@ -28,8 +31,8 @@ namespace {
 
 constexpr int MUL1_MAXT = CN_MAX_M;  // activation rows per slot
 constexpr int MUL1_GT = 8;           // most rows of a group when the MoE step bundles the combos of an expert (groups of 4 or 8)
-constexpr int RING = 4;              // stages of the tile ring
-constexpr int UROWS = 4;             // tile rows per stage
+constexpr int RING = 2;              // stages of the tile ring
+constexpr int UROWS = 8;             // tile rows per stage: one 128-row block of the input
 constexpr int XPAD = 8;              // f16 elements added to the pitch of a staged activation row
 
 struct Mul1Spec {
@@ -89,38 +92,38 @@ __device__ __forceinline__ void store_hi_lo(uint16_t* xh, size_t plane, size_t a
     *(uint2*)(xh + plane + at) = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
 }
 
-// xh16[slot][t][k] = the hi / lo planes of H128(x * suh) * mul, xinv[slot][t][k/128] = 1/mul.
-// grid (k/128, matrices, slots), block 32 T (warp t = activation row t). XT: 0 f32, 1 bf16 input. x row of slot: x + (slot / x_div) * T * k.
-// rowsrc (optional): the x row of (slot, t) as an index into x [rows][k], negative = an unused row slot (stored as zeros)
-template <int XT>
-__global__ void mul1_had_in_kernel(const unsigned long long* __restrict__ ptrs, const void* __restrict__ x, Mul1Side sa, Mul1Side sb, int k, int T,
-                                   int x_div, size_t plane, const int* __restrict__ rowsrc) {
-    pdl_launch_dependents();
-    pdl_wait();  // everything below may read what earlier kernels of the stream wrote
-    const int slot = blockIdx.z, t = threadIdx.x >> 5, blk = blockIdx.x, lane = threadIdx.x & 31;  // one warp per activation row
-    if (ptrs[slot] == 0ull) return;  // a null record: nothing to read or write
-    const Mul1Side& sd = blockIdx.y ? sb : sa;
-    uint16_t* xh = sd.xh;
-    float* xinv = sd.xinv;
-    const uint16_t* suh = (const uint16_t*)(ptrs[slot] + (unsigned long long)sd.suh_off);
-    const int src = rowsrc ? rowsrc[slot * T + t] : 0;
-    const size_t xrow = rowsrc ? (size_t)(src < 0 ? 0 : src) * k : ((size_t)(slot / x_div) * T + t) * k, row = ((size_t)slot * T + t) * k;
-    const int c0 = blk * 128 + 4 * lane;
-    float v[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        float xv = XT == 1 ? __bfloat162float(((const __nv_bfloat16*)x)[xrow + c0 + j]) : ((const float*)x)[xrow + c0 + j];
-        if (src < 0) xv = 0.0f;
-        v[j] = __fmul_rn(xv, h2f(suh[c0 + j]));
+// Where the activation rows of a GEMV come from: row t of slot s is row (s / x_div) * T + t of x, or rowsrc[s * T + t] (negative = an
+// unused row of a group: zeros). And where the records come from when the launch is the first of its chain: record s is table[ids[s]],
+// written to ptrs for the kernels behind it (table null: ptrs is filled already).
+struct Mul1In {
+    const void* x;  // null: the side's staged planes are read instead
+    int bf16, x_div;
+    const int* rowsrc;
+    const unsigned long long* table;
+    const int32_t* ids;
+    int experts;
+};
+// elements at .. at + 3 of a row; `wide`: the row's address allows one load
+__device__ __forceinline__ void load_x4(const void* x, int bf16, bool wide, size_t at, float v[4]) {
+    if (bf16) {
+        const uint16_t* p = (const uint16_t*)x + at;
+        uint32_t a, b;
+        if (wide) {
+            const uint2 u = *(const uint2*)p;
+            a = u.x, b = u.y;
+        } else {
+            a = p[0] | ((uint32_t)p[1] << 16), b = p[2] | ((uint32_t)p[3] << 16);
+        }
+        v[0] = __uint_as_float(a << 16), v[1] = __uint_as_float(a & 0xffff0000u), v[2] = __uint_as_float(b << 16), v[3] = __uint_as_float(b & 0xffff0000u);
+    } else {
+        const float* p = (const float*)x + at;
+        if (wide) {
+            const float4 f = *(const float4*)p;
+            v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+        } else {
+            v[0] = p[0], v[1] = p[1], v[2] = p[2], v[3] = p[3];
+        }
     }
-    fwht128(v, lane);
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    float inv;
-    const float mul = block_scale(amax, inv);
-    store_hi_lo(xh, plane, row + c0, v, mul);
-    if (lane == 0) xinv[((size_t)slot * T + t) * (k / 128) + blk] = inv;
 }
 
 // the codec's f16 weights of two states (bit-exact): sum16 = 0x6400 + bytesum(state * 0x83DCD12D) is the
@@ -162,16 +165,26 @@ __device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const
 // y' partials of one k-split. grid (matrices n/128, S, slots), block 288 = 8 decode warps + 1 copy warp.
 // part[slot][sp][t][n]; xh16 [slot][T][k] f16, xinv [slot][T][k/128].
 // MT: activation rows the register allocation is built for (1, 2, 4 or 8; T <= MT of them live)
-template <bool K3, int MT>
-__global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, Mul1Spec sp_,
-                                                        int S, int T, size_t plane, int SPC) {
+// HAD: the input transform is part of the launch: xh = H128(x * suh) per 128-block as hi / lo planes and 1 / scale, one warp per (row, block), straight
+// into shared memory. The CTAs of one k-split repeat it (some 150 instructions a block), which costs less than a launch before this one
+// and the planes' way through memory.
+template <bool K3, int MT, bool HAD>
+__global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, Mul1Spec sp_,
+                                                        int S, int T, size_t plane, int SPC, Mul1In in) {
     pdl_launch_dependents();
     pdl_wait();  // everything below may read what earlier kernels of the stream wrote
     // SPC consecutive k-splits per CTA (blockIdx.y walks groups of SPC): the splits keep their own partial sums, so
     // the arithmetic does not depend on SPC; a CTA that takes several streams them through one ring without a drain
     extern __shared__ __align__(128) uint8_t smem[];
     const int slot = blockIdx.z, sp0 = blockIdx.y * SPC;
-    const unsigned long long rec = ptrs[slot];
+    unsigned long long rec;
+    if (HAD && in.table) {
+        const int e = in.ids[slot];
+        rec = (e < 0 || (in.experts > 0 && e >= in.experts)) ? 0ull : in.table[e];
+        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ptrs[slot] = rec;
+    } else {
+        rec = ptrs[slot];
+    }
     if (rec == 0ull) return;  // uniform, before any barrier
     const int k = sp_.k, n = sp_.n, n32 = sp_.n32;
     const int tiles_n = n >> 4, tps = (k >> 4) / S, kb0 = sp0 * tps, rows = SPC * tps * 16;
@@ -228,16 +241,47 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
         return;
     }
     // the activation rows of this k-split, and their block scales
-    for (int i = threadIdx.x; i < T * rows / 2; i += 256) {
-        const int t = i / (rows / 2), r = i - t * (rows / 2);
-        const size_t at = ((size_t)slot * T + t) * k + (size_t)kb0 * 16;
-        ((uint32_t*)(xs + (size_t)t * pitch))[r] = ((const uint32_t*)(xh + at))[r];
-        ((uint32_t*)(xs + (size_t)(T + t) * pitch))[r] = ((const uint32_t*)(xh + plane + at))[r];
-    }
     const int nblk = rows / 128;
-    for (int i = threadIdx.x; i < T * nblk; i += 256) {
-        const int t = i / nblk, b = i - t * nblk;
-        xi[i] = xinv[((size_t)slot * T + t) * (k / 128) + kb0 / 8 + b];
+    if (HAD) {
+        const uint16_t* suh = (const uint16_t*)(rec + (unsigned long long)sd.suh_off);
+        const bool wide_x = ((uintptr_t)in.x & 15) == 0, wide_s = ((uintptr_t)suh & 7) == 0;
+        for (int i = warp; i < T * nblk; i += 8) {
+            const int t = i / nblk, b = i - t * nblk;
+            const int src = in.rowsrc ? in.rowsrc[slot * T + t] : 0;
+            const size_t xrow = (in.rowsrc ? (size_t)(src < 0 ? 0 : src) : (size_t)(slot / in.x_div) * T + t) * k;
+            const int c0 = kb0 * 16 + b * 128 + 4 * lane;
+            float v[4];
+            load_x4(in.x, in.bf16, wide_x, xrow + c0, v);
+            uint16_t sc[4];
+            if (wide_s) {
+                const uint2 u = *(const uint2*)(suh + c0);
+                sc[0] = (uint16_t)u.x, sc[1] = (uint16_t)(u.x >> 16), sc[2] = (uint16_t)u.y, sc[3] = (uint16_t)(u.y >> 16);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) sc[j] = suh[c0 + j];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = __fmul_rn(src < 0 ? 0.0f : v[j], h2f(sc[j]));
+            fwht128(v, lane);
+            float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            float inv;
+            const float mul = block_scale(amax, inv);
+            store_hi_lo(xs, (size_t)T * pitch, (size_t)t * pitch + b * 128 + 4 * lane, v, mul);
+            if (lane == 0) xi[i] = inv;
+        }
+    } else {
+        for (int i = threadIdx.x; i < T * rows / 2; i += 256) {
+            const int t = i / (rows / 2), r = i - t * (rows / 2);
+            const size_t at = ((size_t)slot * T + t) * k + (size_t)kb0 * 16;
+            ((uint32_t*)(xs + (size_t)t * pitch))[r] = ((const uint32_t*)(xh + at))[r];
+            ((uint32_t*)(xs + (size_t)(T + t) * pitch))[r] = ((const uint32_t*)(xh + plane + at))[r];
+        }
+        for (int i = threadIdx.x; i < T * nblk; i += 256) {
+            const int t = i / nblk, b = i - t * nblk;
+            xi[i] = xinv[((size_t)slot * T + t) * (k / 128) + kb0 / 8 + b];
+        }
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
 
@@ -275,7 +319,7 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
     const int tw = K3 ? TW : n32;
     const int o1 = wi0 + 1 >= tw ? wi0 + 1 - tw : wi0 + 1, o2 = wi0 + 2 >= tw ? wi0 + 2 - tw : wi0 + 2;
     const uint32_t* lane_tile = ring + (size_t)warp * tw;  // this warp's tile of the ring's first tile row
-    int s = 0, cs = 0, spi = 0, blk = 0;
+    int s = 0, cs = 0, spi = 0;
     uint32_t ph = 0;
     for (int c = 0; c < nst; c++) {
         if (!mbar_wait(&full[s], ph)) {
@@ -315,16 +359,13 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(const unsigned long l
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
         if (++s == RING) s = 0, ph ^= 1u;
-        if (cs & 1) {
-            // end of a 128-row block (two stages): hi + lo * 2^-11, then the block's activation scale
+        // the stage was a 128-row block: hi + lo * 2^-11, then the block's activation scale
 #pragma unroll
-            for (int i = 0; i < NM; i++) {
-                const float inv = xil[i][blk];
-                tot0[i] = fmaf(fmaf(acc[i][1], 4.8828125e-4f, acc[i][0]), inv, tot0[i]);
-                tot1[i] = fmaf(fmaf(acc[i][3], 4.8828125e-4f, acc[i][2]), inv, tot1[i]);
-                acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-            }
-            blk++;
+        for (int i = 0; i < NM; i++) {
+            const float inv = xil[i][c];
+            tot0[i] = fmaf(fmaf(acc[i][1], 4.8828125e-4f, acc[i][0]), inv, tot0[i]);
+            tot1[i] = fmaf(fmaf(acc[i][3], 4.8828125e-4f, acc[i][2]), inv, tot1[i]);
+            acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
         }
         if (++cs == nst1) {
             // end of a split: lane (g, t) stores outputs g and g + 8 of its tile column for activation row t (+ 4)
@@ -388,6 +429,41 @@ __global__ void mul1_had_out_kernel(const unsigned long long* __restrict__ ptrs,
             ((__nv_bfloat16*)y)[at + j] = __float2bfloat16_rn(v[j]);
         else
             ((float*)y)[at + j] = v[j];
+    }
+}
+
+// had_out and the weighted combine of the routed step in one launch: y[tok][c] = base + sum_j w_j * had_out(combo tok * K + j)[c], j in pick
+// order, with the arithmetic of moe_combine_kernel; base = shared[tok][c] or 0. grid (n/128, tokens), one warp per pick (K <= 32), which
+// transforms its combo's 128 values into shared memory. place (optional): the (slot * T + t) of a combo, else slot = combo, T = 1.
+template <int YT>
+__global__ void __launch_bounds__(1024) mul1_out_combine_kernel(const unsigned long long* __restrict__ table, const int32_t* __restrict__ ids, const float* __restrict__ wts,
+                                                                const float* __restrict__ part, const float* __restrict__ shared, void* __restrict__ y, int n, int S,
+                                                                int T, int K, int experts, long long svh_off, const int* __restrict__ place) {
+    extern __shared__ float sv[];  // [K][128], then the weights
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tok = blockIdx.y, j = threadIdx.x >> 5, blk = blockIdx.x, lane = threadIdx.x & 31;
+    const int c = tok * K + j, e = ids[c];
+    const unsigned long long rec = (e < 0 || (experts > 0 && e >= experts)) ? 0ull : table[e];
+    float* ws = sv + K * 128;
+    if (lane == 0) ws[j] = wts[c], ws[K + j] = rec ? 1.0f : 0.0f;
+    if (rec) {
+        const int at = place ? place[c] : c, slot = at / T, t = at - slot * T;
+        float v[4];
+        out_block(v, part, (const uint16_t*)(rec + (unsigned long long)svh_off), slot, S, T, t, n, blk, lane);
+        *(float4*)(sv + j * 128 + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 128; i += blockDim.x) {
+        float acc = 0.0f;
+        for (int q = 0; q < K; q++)
+            if (ws[K + q] != 0.0f) acc = __fadd_rn(acc, __fmul_rn(ws[q], sv[q * 128 + i]));
+        const size_t to = (size_t)tok * n + blk * 128 + i;
+        const float r = __fadd_rn(shared ? shared[to] : 0.0f, acc);
+        if (YT == 1)
+            ((__nv_bfloat16*)y)[to] = __float2bfloat16_rn(r);
+        else
+            ((float*)y)[to] = r;
     }
 }
 
@@ -455,15 +531,16 @@ namespace {
 struct Mul1Plan {
     int hidden, inter, bits, half, n32, max_slots, max_t;
     size_t kmax;
-    uint16_t *xh_a, *xh_b;  // [2 planes][slots][T][kmax] f16
+    uint16_t* xh;           // [2 planes][slots][T][kmax] f16: the staged rows of the down projection
     size_t plane;           // elements of one plane
-    float *xinv_a, *xinv_b;  // [slots][T][kmax/128]
+    float* xinv;            // [slots][T][kmax/128]
     float *part_a, *part_b;  // [slots][16][T][kmax]
     unsigned long long* ptrs;  // [slots] gathered record addresses (MoE form)
     int32_t* order;            // [slots] combos sorted by expert (grouped MoE form)
     int* groups;               // [5 * slots + 8] the group lists and counts of cn_moe_group_launch
     int* rowsrc;               // [slots * MUL1_GT] x row of every (group slot, row), -1 = unused
     int* rowdst;               // [slots * MUL1_GT] combo (output row) of every (group slot, row), -1 = unused
+    int* place;                // [slots] (group slot * rows + row) of every combo
     int grp_rows;              // rows the scratch holds per slot: max(max_t, 4)
     float* eo;                 // [slots][T][hidden] expert outputs (MoE form)
 };
@@ -488,21 +565,10 @@ Mul1Spec spec_of(const Mul1Plan* p, int which) {
     return s;
 }
 
-// sb: the second matrix of the launch (up beside gate), or null
-int launch_had_in(const unsigned long long* ptrs, const void* x, const Mul1Side& sa, const Mul1Side* sb, int k, int slots, int T, int x_div, int dtype,
-                  size_t plane, cudaStream_t st, const int* rowsrc = nullptr) {
-    dim3 grid(k / 128, sb ? 2 : 1, slots);
-    if (dtype == CN_BF16)
-        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<1>), grid, dim3(32 * T), 0, st, ptrs, x, sa, sb ? *sb : sa, k, T, x_div, plane, rowsrc));
-    else
-        CN_CUDA(cn_launch_pdl((mul1_had_in_kernel<0>), grid, dim3(32 * T), 0, st, ptrs, x, sa, sb ? *sb : sa, k, T, x_div, plane, rowsrc));
-    CN_CUDA(cudaGetLastError());
-    return CN_OK;
-}
-
 // live: how many of the slots are expected to hold a record (the grouped MoE form launches more slots than it fills)
+// sb: the second matrix of the launch (up beside gate), or null. in: the rows to transform, or null where the side holds them staged
 int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Side* sb, const Mul1Spec& s, int slots, int T, size_t plane,
-                cudaStream_t st, int live = 0) {
+                cudaStream_t st, const Mul1In* in, int live = 0) {
     if (live < 1 || live > slots) live = slots;
     const int mats = sb ? 2 : 1;
     const int S = ksplit(s.k), tps = (s.k / 16) / S;
@@ -525,13 +591,15 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "mul1 gemv: %zu B of shared memory per block", smem);
     const bool k3 = s.bits == 3 && !s.half;
     const int mt = T == 1 ? 1 : (T == 2 ? 2 : (T <= 4 ? 4 : 8));
-#define CN_MUL1_CASE(K3V, MTV)                                                                                                      \
-    if (k3 == K3V && mt == MTV) {                                                                                                   \
-        CN_ALLOW_SMEM((mul1_gemv_kernel<K3V, MTV>), 160 * 1024);                                                                    \
-        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K3V, MTV>), grid, dim3(288), smem, st, ptrs, sa, sb ? *sb : sa, s, S, T, plane, spc));             \
+    const Mul1In none = {};
+#define CN_MUL1_CASE(K3V, MTV, HADV)                                                                                                \
+    if (k3 == K3V && mt == MTV && (in != nullptr) == HADV) {                                                                        \
+        CN_ALLOW_SMEM((mul1_gemv_kernel<K3V, MTV, HADV>), 160 * 1024);                                                              \
+        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K3V, MTV, HADV>), grid, dim3(288), smem, st, const_cast<unsigned long long*>(ptrs), sa, sb ? *sb : sa, s, S, T, plane, spc, in ? *in : none)); \
     }
-    CN_MUL1_CASE(true, 1) CN_MUL1_CASE(true, 2) CN_MUL1_CASE(true, 4) CN_MUL1_CASE(true, 8)
-    CN_MUL1_CASE(false, 1) CN_MUL1_CASE(false, 2) CN_MUL1_CASE(false, 4) CN_MUL1_CASE(false, 8)
+#define CN_MUL1_CASES(K3V, HADV) CN_MUL1_CASE(K3V, 1, HADV) CN_MUL1_CASE(K3V, 2, HADV) CN_MUL1_CASE(K3V, 4, HADV) CN_MUL1_CASE(K3V, 8, HADV)
+    CN_MUL1_CASES(true, true) CN_MUL1_CASES(true, false) CN_MUL1_CASES(false, true) CN_MUL1_CASES(false, false)
+#undef CN_MUL1_CASES
 #undef CN_MUL1_CASE
     CN_CUDA(cudaGetLastError());
     return CN_OK;
@@ -544,20 +612,12 @@ int check_run(const Mul1Plan* p, int slots, int T, const char* who) {
     return CN_OK;
 }
 
-__global__ void mul1_gather_kernel(const unsigned long long* __restrict__ table, const int32_t* __restrict__ ids, unsigned long long* ptrs, int n,
-                                   int experts) {
-    pdl_launch_dependents();
-    pdl_wait();  // everything below may read what earlier kernels of the stream wrote
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < n) ptrs[c] = (ids[c] < 0 || (experts > 0 && ids[c] >= experts)) ? 0ull : table[ids[c]];
-}
-
 // Slot s of the grouped MoE form (gt rows per slot, 4 or 8): the groups of two or more rows first, then the one-row
 // groups, then empty slots (null record). Fills the slot's record address and, per row, where its x row comes from and
 // which combo's output row it is.
 __global__ void mul1_slots_kernel(const unsigned long long* __restrict__ table, const int32_t* __restrict__ ids, const int32_t* __restrict__ order,
                                   const int* __restrict__ ga, const int* __restrict__ gb, const int* __restrict__ gbrows, const int* __restrict__ counts,
-                                  unsigned long long* __restrict__ ptrs, int* __restrict__ rowsrc, int* __restrict__ rowdst, int slots, int x_div, int gt) {
+                                  unsigned long long* __restrict__ ptrs, int* __restrict__ rowsrc, int* __restrict__ rowdst, int* __restrict__ place, int slots, int x_div, int gt) {
     pdl_launch_dependents();
     pdl_wait();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -571,6 +631,7 @@ __global__ void mul1_slots_kernel(const unsigned long long* __restrict__ table, 
         const int c = t < rows ? order[pos + t] : -1;
         rowsrc[s * gt + t] = c < 0 ? -1 : c / x_div;
         rowdst[s * gt + t] = c;
+        if (c >= 0) place[c] = s * gt + t;
     }
 }
 
@@ -594,10 +655,8 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
     // a failure part-way frees what the earlier steps got (the destroy call takes a half-built plan)
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    step(cudaMalloc(&p->xh_a, 2 * p->plane * 2));
-    step(cudaMalloc(&p->xh_b, 2 * p->plane * 2));
-    step(cudaMalloc(&p->xinv_a, rows * (p->kmax / 128) * 4));
-    step(cudaMalloc(&p->xinv_b, rows * (p->kmax / 128) * 4));
+    step(cudaMalloc(&p->xh, 2 * p->plane * 2));
+    step(cudaMalloc(&p->xinv, rows * (p->kmax / 128) * 4));
     step(cudaMalloc(&p->part_a, rows * 16 * p->kmax * 4));
     step(cudaMalloc(&p->part_b, rows * 16 * p->kmax * 4));
     step(cudaMalloc(&p->ptrs, (size_t)max_slots * 8));
@@ -605,6 +664,7 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
     step(cudaMalloc(&p->groups, ((size_t)5 * max_slots + 8) * 4));
     step(cudaMalloc(&p->rowsrc, (size_t)max_slots * MUL1_GT * 4));
     step(cudaMalloc(&p->rowdst, (size_t)max_slots * MUL1_GT * 4));
+    step(cudaMalloc(&p->place, (size_t)max_slots * 4));
     step(cudaMalloc(&p->eo, rows * hidden * 4));
     if (e != cudaSuccess) {
         cn_mul1_plan_destroy(p);
@@ -617,7 +677,7 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
 extern "C" int cn_mul1_plan_destroy(void* plan) {
     Mul1Plan* p = (Mul1Plan*)plan;
     if (!p) return CN_OK;
-    cudaFree(p->xh_a), cudaFree(p->xh_b), cudaFree(p->xinv_a), cudaFree(p->xinv_b), cudaFree(p->part_a), cudaFree(p->part_b), cudaFree(p->ptrs),
+    cudaFree(p->xh), cudaFree(p->xinv), cudaFree(p->place), cudaFree(p->part_a), cudaFree(p->part_b), cudaFree(p->ptrs),
         cudaFree(p->eo), cudaFree(p->order), cudaFree(p->groups), cudaFree(p->rowsrc), cudaFree(p->rowdst);
     delete p;
     return CN_OK;
@@ -631,9 +691,9 @@ extern "C" int cn_mul1_gemv(void* plan, int which, const unsigned long long* ptr
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_mul1_gemv: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     cudaStream_t st = (cudaStream_t)stream;
     const Mul1Spec s = spec_of(p, which);
-    const Mul1Side side = {p->xh_a, p->xinv_a, p->part_a, s.tr_off, s.suh_off};
-    if (int rc = launch_had_in(ptrs, x, side, nullptr, s.k, slots, t, x_div, dtype, p->plane, st)) return rc;
-    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, p->plane, st)) return rc;
+    const Mul1Side side = {nullptr, nullptr, p->part_a, s.tr_off, s.suh_off};
+    const Mul1In in = {x, dtype == CN_BF16, x_div, nullptr, nullptr, nullptr, 0};
+    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, p->plane, st, &in)) return rc;
     dim3 grid(s.n / 128, 1, slots);
     if (dtype == CN_BF16)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, s.n, ksplit(s.k), t, s.svh_off, (const int*)nullptr));
@@ -643,22 +703,26 @@ extern "C" int cn_mul1_gemv(void* plan, int which, const unsigned long long* ptr
     return CN_OK;
 }
 
-// y[slot][t] = down(act(gate x, up x)) as f32 when out_f32, else in `dtype`
-static int mul1_ffn(Mul1Plan* p, const unsigned long long* ptrs, const void* x, void* y, int slots, int t, int x_div, float limit, int dtype,
-                    int out_f32, cudaStream_t st, const int* rowsrc = nullptr, const int* rowdst = nullptr, int live = 0) {
+// The FFN up to the partial sums of the down projection (p->part_a): gate and up with the input transform, the middle, down.
+static int mul1_ffn_parts(Mul1Plan* p, const unsigned long long* ptrs, const Mul1In& in, int slots, int t, float limit, cudaStream_t st, int live = 0) {
     const Mul1Spec g = spec_of(p, 0), u = spec_of(p, 1), d = spec_of(p, 2);
     // gate and up share each launch: two small grids on two streams cost an event fork and join and ran one after the other
     // anyway (one token, four experts of 4096 x 1536: 65 -> 55 us with out_block's wide loads; 16 tokens: 295 us, no difference beyond noise)
-    const Mul1Side ga = {p->xh_a, p->xinv_a, p->part_a, g.tr_off, g.suh_off}, up = {p->xh_b, p->xinv_b, p->part_b, u.tr_off, u.suh_off};
-    const Mul1Side dn = {p->xh_a, p->xinv_a, p->part_a, d.tr_off, d.suh_off};
-    if (int rc = launch_had_in(ptrs, x, ga, &up, g.k, slots, t, x_div, dtype, p->plane, st, rowsrc)) return rc;
-    if (int rc = launch_gemv(ptrs, ga, &up, g, slots, t, p->plane, st, live)) return rc;
-    CN_CUDA(cn_launch_pdl(mul1_act_had_in_kernel, dim3(p->inter / 128, 1, slots), dim3(32 * t), 0, st, ptrs, p->part_a, p->part_b, p->xh_a, p->xinv_a, p->inter, ksplit(p->hidden), t,
+    const Mul1Side ga = {nullptr, nullptr, p->part_a, g.tr_off, g.suh_off}, up = {nullptr, nullptr, p->part_b, u.tr_off, u.suh_off};
+    const Mul1Side dn = {p->xh, p->xinv, p->part_a, d.tr_off, d.suh_off};
+    if (int rc = launch_gemv(ptrs, ga, &up, g, slots, t, p->plane, st, &in, live)) return rc;
+    CN_CUDA(cn_launch_pdl(mul1_act_had_in_kernel, dim3(p->inter / 128, 1, slots), dim3(32 * t), 0, st, ptrs, p->part_a, p->part_b, p->xh, p->xinv, p->inter, ksplit(p->hidden), t,
                                                                          g.svh_off, u.svh_off, d.suh_off, limit, p->plane));
-    CN_CUDA(cudaGetLastError());
-    if (int rc = launch_gemv(ptrs, dn, nullptr, d, slots, t, p->plane, st, live)) return rc;
+    return launch_gemv(ptrs, dn, nullptr, d, slots, t, p->plane, st, nullptr, live);
+}
+
+// y[slot][t] = down(act(gate x, up x)) as f32 when out_f32, else in the type of the rows; rowdst: see mul1_had_out_kernel
+static int mul1_ffn(Mul1Plan* p, const unsigned long long* ptrs, const Mul1In& in, void* y, int slots, int t, float limit, int out_f32, cudaStream_t st,
+                    const int* rowdst = nullptr, int live = 0) {
+    if (int rc = mul1_ffn_parts(p, ptrs, in, slots, t, limit, st, live)) return rc;
+    const Mul1Spec d = spec_of(p, 2);
     dim3 grid(d.n / 128, 1, slots);
-    if (dtype == CN_BF16 && !out_f32)
+    if (in.bf16 && !out_f32)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, d.n, ksplit(d.k), t, d.svh_off, rowdst));
     else
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<0>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, d.n, ksplit(d.k), t, d.svh_off, rowdst));
@@ -672,19 +736,26 @@ extern "C" int cn_mul1_ffn(void* plan, const unsigned long long* ptrs, const voi
     if (int rc = check_run(p, slots, t, "cn_mul1_ffn")) return rc;
     if (x_div < 1) CN_FAIL(CN_ERR_SHAPE, "cn_mul1_ffn: x_div %d", x_div);
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_mul1_ffn: dtype %d is neither CN_F32 nor CN_BF16", dtype);
-    return mul1_ffn(p, ptrs, x, y, slots, t, x_div, limit, dtype, 0, (cudaStream_t)stream);
+    const Mul1In in = {x, dtype == CN_BF16, x_div, nullptr, nullptr, nullptr, 0};
+    return mul1_ffn(p, ptrs, in, y, slots, t, limit, 0, (cudaStream_t)stream);
 }
 
 extern "C" int cn_moe_combine(const float* eo, const float* wts, const int32_t* ids, const unsigned long long* table, const float* shared,
                               const float* sgate, void* y, int tokens, int hidden, int topk, int experts, int dtype, cn_stream_t stream);
 
-extern "C" int cn_moe_mul1_experts(void* plan, const unsigned long long* table, const int32_t* ids, const void* x, float* eo, int combos, int x_div,
-                                   int experts, float limit, int dtype, cn_stream_t stream) {
-    Mul1Plan* p = (Mul1Plan*)plan;
-    if (int rc = check_run(p, combos, 1, "cn_moe_mul1_experts")) return rc;
-    if (x_div < 1 || !eo) CN_FAIL(CN_ERR_SHAPE, "cn_moe_mul1_experts: x_div %d, eo %p", x_div, (void*)eo);
-    if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_moe_mul1_experts: dtype %d is neither CN_F32 nor CN_BF16", dtype);
-    cudaStream_t st = (cudaStream_t)stream;
+namespace {
+
+// How the combos of a routed step run: one slot each, or bundled by expert into slots of T rows (place: see mul1_out_combine_kernel)
+struct Mul1Slots {
+    Mul1In in;
+    int slots, T, live;
+    const int *rowdst, *place;
+};
+
+int mul1_slots(Mul1Plan* p, const unsigned long long* table, const int32_t* ids, const void* x, int combos, int x_div, int experts, int dtype, cudaStream_t st,
+               Mul1Slots& r) {
+    r = {};
+    r.in.x = x, r.in.bf16 = dtype == CN_BF16, r.in.x_div = x_div, r.slots = combos, r.T = 1;
     if (experts > 0 && 2 * combos >= experts) {
         // Enough combos that experts repeat: the combos are sorted by expert and bundled into groups that share one
         // decode of the expert's trellis (a group of up to four rows is one MMA per tile like a single row, eight rows
@@ -704,22 +775,52 @@ extern "C" int cn_moe_mul1_experts(void* plan, const unsigned long long* table, 
             int* counts = gdrows + combos;
             if (int rc = cn_moe_group_launch(ids, table, combos, experts, p->order, ga, gb, gbrows, gd, gdrows, counts, gt, st)) return rc;
             CN_CUDA(cn_launch_pdl(mul1_slots_kernel, dim3(((int)ng + 127) / 128), dim3(128), 0, st, table, ids, p->order, ga, gb, gbrows, counts, p->ptrs,
-                                  p->rowsrc, p->rowdst, (int)ng, x_div, gt));
+                                  p->rowsrc, p->rowdst, p->place, (int)ng, x_div, gt));
             // a slot beyond the groups is a null record, which all kernels skip; a group's unused rows are zero rows
             // (the work per CTA is sized as if a quarter of the launched slots were filled: measured best at 45 of 64 and at 8 of 128)
-            return mul1_ffn(p, p->ptrs, x, eo, (int)ng, gt, 1, limit, dtype, 1, st, p->rowsrc, p->rowdst, (int)((ng + 3) / 4));
+            r.in.rowsrc = p->rowsrc, r.in.x_div = 1, r.slots = (int)ng, r.T = gt, r.live = (int)((ng + 3) / 4), r.rowdst = p->rowdst, r.place = p->place;
+            return CN_OK;
         }
     }
-    CN_CUDA(cn_launch_pdl(mul1_gather_kernel, dim3((combos + 127) / 128), dim3(128), 0, st, table, ids, p->ptrs, combos, experts));
-    CN_CUDA(cudaGetLastError());
-    return mul1_ffn(p, p->ptrs, x, eo, combos, 1, x_div, limit, dtype, 1, st);
+    r.in.table = table, r.in.ids = ids, r.in.experts = experts;
+    return CN_OK;
+}
+
+}  // namespace
+
+extern "C" int cn_moe_mul1_experts(void* plan, const unsigned long long* table, const int32_t* ids, const void* x, float* eo, int combos, int x_div,
+                                   int experts, float limit, int dtype, cn_stream_t stream) {
+    Mul1Plan* p = (Mul1Plan*)plan;
+    if (int rc = check_run(p, combos, 1, "cn_moe_mul1_experts")) return rc;
+    if (x_div < 1 || !eo) CN_FAIL(CN_ERR_SHAPE, "cn_moe_mul1_experts: x_div %d, eo %p", x_div, (void*)eo);
+    if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_moe_mul1_experts: dtype %d is neither CN_F32 nor CN_BF16", dtype);
+    cudaStream_t st = (cudaStream_t)stream;
+    Mul1Slots r;
+    if (int rc = mul1_slots(p, table, ids, x, combos, x_div, experts, dtype, st, r)) return rc;
+    return mul1_ffn(p, p->ptrs, r.in, eo, r.slots, r.T, limit, 1, st, r.rowdst, r.live);
 }
 
 extern "C" int cn_moe_mul1_run(void* plan, const unsigned long long* table, const int32_t* ids, const float* wts, const float* shared, const void* x,
                                void* y, int tokens, int topk, int experts, float limit, int dtype, cn_stream_t stream) {
     Mul1Plan* p = (Mul1Plan*)plan;
-    if (int rc = cn_moe_mul1_experts(plan, table, ids, x, p ? p->eo : nullptr, tokens * topk, topk, experts, limit, dtype, stream)) return rc;
-    return cn_moe_combine(p->eo, wts, ids, table, shared, nullptr, y, tokens, p->hidden, topk, experts, dtype, stream);
+    if (topk > 32 || topk < 1 || tokens < 1 || tokens > 65535) {  // the fused combine takes a warp per pick
+        if (int rc = cn_moe_mul1_experts(plan, table, ids, x, p ? p->eo : nullptr, tokens * topk, topk, experts, limit, dtype, stream)) return rc;
+        return cn_moe_combine(p->eo, wts, ids, table, shared, nullptr, y, tokens, p->hidden, topk, experts, dtype, stream);
+    }
+    if (int rc = check_run(p, tokens * topk, 1, "cn_moe_mul1_run")) return rc;
+    if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_moe_mul1_run: dtype %d is neither CN_F32 nor CN_BF16", dtype);
+    cudaStream_t st = (cudaStream_t)stream;
+    Mul1Slots r;
+    if (int rc = mul1_slots(p, table, ids, x, tokens * topk, topk, experts, dtype, st, r)) return rc;
+    if (int rc = mul1_ffn_parts(p, p->ptrs, r.in, r.slots, r.T, limit, st, r.live)) return rc;
+    const Mul1Spec d = spec_of(p, 2);
+    const dim3 grid(d.n / 128, tokens), block(32 * topk);
+    const size_t smem = (size_t)topk * (128 + 2) * 4;
+    if (dtype == CN_BF16)
+        CN_CUDA(cn_launch_pdl((mul1_out_combine_kernel<1>), grid, block, smem, st, table, ids, wts, p->part_a, shared, y, d.n, ksplit(d.k), r.T, topk, experts, d.svh_off, r.place));
+    else
+        CN_CUDA(cn_launch_pdl((mul1_out_combine_kernel<0>), grid, block, smem, st, table, ids, wts, p->part_a, shared, y, d.n, ksplit(d.k), r.T, topk, experts, d.svh_off, r.place));
+    return CN_OK;
 }
 
 extern "C" int cn_mul1_reconstruct(const void* trellis, void* w_out, int k, int n, int bits, int half, cn_stream_t stream) {
@@ -735,19 +836,15 @@ extern "C" int cn_mul1_reconstruct(const void* trellis, void* w_out, int k, int 
 // For callers that may not allocate device memory at the point of the call - an engine thread that
 // already runs inside a latency-critical decode loop, a plugin host that forbids cudaMalloc after
 // start-up because an allocation synchronises the whole device, or code that holds a memory budget
-// it has fully handed out. The scratch of the GEMV (the transformed activations and the k-split
-// partial sums) lives in a fixed array inside the library image instead of a plan.
+// it has fully handed out. The scratch of the GEMV (the k-split partial sums) lives in a fixed array inside the library image instead of a plan.
 //
 // Limits: slots * t <= CN_MUL1_STATIC_ROWS (8) activation rows per call, hidden and inter <=
-// CN_MUL1_STATIC_DIM (4096). The array is about 2.2 MB and every GPU that loads the library holds
+// CN_MUL1_STATIC_DIM (4096). The array is 2 MB and every GPU that loads the library holds
 // it until the process exits.
 namespace {
 
 constexpr size_t NA_ROWS = 8, NA_DIM = 4096, NA_SPLITS = 16;
-constexpr size_t NA_XH_BYTES = 2 * NA_ROWS * NA_DIM * 2;             // hi and lo f16 planes
-constexpr size_t NA_XINV_BYTES = NA_ROWS * (NA_DIM / 128) * 4;       // one f32 per 128-block
-constexpr size_t NA_PART_BYTES = NA_ROWS * NA_SPLITS * NA_DIM * 4;   // f32 partial sums of the k-split
-constexpr size_t NA_BYTES = NA_XH_BYTES + NA_XINV_BYTES + NA_PART_BYTES;
+constexpr size_t NA_BYTES = NA_ROWS * NA_SPLITS * NA_DIM * 4;  // f32 partial sums of the k-split
 
 // File-scope device array: in host code this name is only a handle for the runtime, never an
 // address a kernel may be given; the device address comes from cudaGetSymbolAddress below.
@@ -790,16 +887,12 @@ extern "C" int cn_mul1_gemv_noalloc(int which, int hidden, int inter, int bits, 
     Mul1Plan view = {};
     view.hidden = hidden, view.inter = inter, view.bits = bits, view.half = half, view.n32 = 8 * bits + (half ? 4 : 0);
     const Mul1Spec s = spec_of(&view, which);
-    uint16_t* xh = (uint16_t*)base;
-    float* xinv = (float*)(base + NA_XH_BYTES);
-    float* part = (float*)(base + NA_XH_BYTES + NA_XINV_BYTES);
-    const size_t plane = NA_ROWS * NA_DIM;  // the lo plane starts one full plane after the hi plane
+    float* part = (float*)base;
     cudaStream_t st = (cudaStream_t)stream;
-    // every region is written before it is read within one call (had_in fills xh / xinv of the live
-    // slots, the GEMV fills every partial that had_out sums), so nothing has to start at zero
-    const Mul1Side side = {xh, xinv, part, s.tr_off, s.suh_off};
-    if (int rc = launch_had_in(ptrs, x, side, nullptr, s.k, slots, t, x_div, dtype, plane, st)) return rc;
-    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, plane, st)) return rc;
+    // the GEMV fills every partial that had_out sums, so nothing has to start at zero
+    const Mul1Side side = {nullptr, nullptr, part, s.tr_off, s.suh_off};
+    const Mul1In in = {x, dtype == CN_BF16, x_div, nullptr, nullptr, nullptr, 0};
+    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, 0, st, &in)) return rc;
     dim3 grid(s.n / 128, 1, slots);
     if (dtype == CN_BF16)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, part, y, s.n, ksplit(s.k), t, s.svh_off, (const int*)nullptr));

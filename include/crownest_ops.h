@@ -275,7 +275,7 @@ int cn_moe_mul1_experts(void* plan, const unsigned long long* table, const int32
 /* The MUL1 GEMV of cn_mul1_gemv without a plan and without any allocation: for a caller that cannot
  * allocate device memory where it makes the call (a decode loop that must not hit the device-wide
  * synchronisation an allocation implies, a host that hands out all device memory at start-up, a
- * plugin sandbox that forbids it). Its scratch is a fixed array of about 2.2 MB inside the library
+ * plugin sandbox that forbids it). Its scratch is a fixed array of 2 MB inside the library
  * image, which every GPU that loads the library keeps until the process exits.
  * This entry point has no counterpart in the reference (there every plan allocates its scratch,
  * engine/src/kernels.rs:6664).
