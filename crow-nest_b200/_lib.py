@@ -19,18 +19,40 @@ class CrownestError(RuntimeError):
     pass
 
 
+HOST_PATH = os.path.join(_HERE, "_host.so")
+
+
+def _build_host(force):
+    """g++ over csrc/host.cpp against torch's headers: the Python extension of the small operators."""
+    src = os.path.join(CSRC, "host.cpp")
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= os.path.getmtime(src):
+        return
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += ["-isystem" + i for i in inc] + [src, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise CrownestError("building _host.so failed:\n" + r.stdout[-2000:] + r.stderr[-4000:])
+
+
 def build(force=False, jobs=8):
-    """nvcc -gencode arch=compute_100a,code=sm_100a over csrc/*.cu (cross-compiles without a GPU)."""
+    """nvcc -gencode arch=compute_100a,code=sm_100a over csrc/*.cu (cross-compiles without a GPU), then the host extension."""
     cmd = ["make", "-C", CSRC, f"-j{jobs}"]
     if force:
         cmd.append("-B")
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise CrownestError("building libcrownest_b200.so failed:\n" + r.stdout[-4000:] + r.stderr[-4000:])
+    _build_host(force)
     return SO_PATH
 
 
 _lib = None
+_host = None
 
 _vp, _i, _f = C.c_void_p, C.c_int, C.c_float
 
@@ -145,6 +167,30 @@ def lib():
 def check(status):
     if status != 0:
         raise CrownestError(lib().cn_last_error_string().decode() or f"status {status}")
+
+
+def _raise_status(status):
+    raise CrownestError(status if isinstance(status, str) else lib().cn_last_error_string().decode() or f"status {status}")
+
+
+def host():
+    """The native host side of the small operators (csrc/host.cpp), bound to the library that lib() loads."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        import torch  # noqa: F401  (its libraries are what the extension links to)
+        if not os.path.exists(HOST_PATH):
+            raise CrownestError(f"{HOST_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
+        L = lib()
+        loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+        loader.exec_module(mod)
+        names = ("cn_nvfp4_gemv", "cn_nvfp4_gemv_gu", "cn_nvfp4_gemm", "cn_nvfp4_gemm_workspace_bytes", "cn_nvfp4_bs_gemm", "cn_nvfp4_bs_workspace_bytes",
+                 "cn_fp8_gemv", "cn_lm_head_argmax", "cn_route_softmax_topk", "cn_route_sigmoid_topk")
+        mod.bind({n: C.cast(getattr(L, n), C.c_void_p).value for n in names}, _raise_status)
+        _host = mod
+    return _host
 
 
 def device_status():

@@ -11,11 +11,11 @@ import numpy as np
 import torch
 
 from . import ops
-from ._lib import CN_BF16, CN_BF16_IN_F32_OUT, CN_F32, CrownestError, check, lib
+from ._lib import CN_BF16, CN_BF16_IN_F32_OUT, CN_F32, CrownestError, check, host, lib
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return host().stream()
 
 
 def _ptr(t):
@@ -24,20 +24,12 @@ def _ptr(t):
 
 def route_softmax_topk(logits, k):
     """ids, wts [T][k] in pick order - router_top10's selection (engine/src/kernels.rs:3109)."""
-    t, e = logits.shape
-    ids = torch.empty((t, k), dtype=torch.int32, device=logits.device)
-    wts = torch.empty((t, k), dtype=torch.float32, device=logits.device)
-    check(lib().cn_route_softmax_topk(logits.data_ptr(), ids.data_ptr(), wts.data_ptr(), t, e, k, _stream()))
-    return ids, wts
+    return host().route_softmax(logits, k)
 
 
 def route_sigmoid_topk(logits, bias, k, scale):
     """glm5_router_sig_topk / route_from_logits (engine/src/glm5_moe.rs:196)."""
-    t, e = logits.shape
-    ids = torch.empty((t, k), dtype=torch.int32, device=logits.device)
-    wts = torch.empty((t, k), dtype=torch.float32, device=logits.device)
-    check(lib().cn_route_sigmoid_topk(logits.data_ptr(), _ptr(bias), ids.data_ptr(), wts.data_ptr(), t, e, k, float(scale), _stream()))
-    return ids, wts
+    return host().route_sigmoid(logits, bias, k, scale)
 
 
 class GpuMoeWeights:

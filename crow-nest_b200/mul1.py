@@ -5,11 +5,11 @@ import ctypes as C
 
 import torch
 
-from ._lib import CN_BF16, CN_F32, CrownestError, check, lib
+from ._lib import CN_BF16, CN_F32, CrownestError, check, host, lib
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return host().stream()
 
 
 def bitrate(k):

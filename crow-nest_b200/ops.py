@@ -10,11 +10,11 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import CN_BF16, CN_F32, CrownestError, check, lib
+from ._lib import CN_BF16, CN_F32, CrownestError, check, host, lib
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return host().stream()
 
 
 def _dtype_code(t):
@@ -52,30 +52,14 @@ class Fp4:
 def launch_gemv(w: Fp4, x, y=None, ldy=None):
     """y[m][r] = sum_k W[r][k] x[m][k] for x [M][k] (M <= 8) - PW::launch_gemv / launch_gemv1,
     Engine::proj_m (engine/src/gen.rs:234-266, :5455). Enqueues and returns ``y``."""
-    x2 = x.reshape(-1, w.cols)
-    m = x2.shape[0]
-    if y is None:
-        y = torch.empty((m, w.rows), dtype=x.dtype, device=x.device)
-    ld = ldy if ldy is not None else (y.stride(0) if y.dim() == 2 else w.rows)
-    check(lib().cn_nvfp4_gemv(w.w.data_ptr(), w.gs.data_ptr(), x2.data_ptr(), y.data_ptr(), w.rows, w.cols, m, ld,
-                              _dtype_code(x), _stream()))
-    return y
+    return host().gemv(w.w, w.gs, w.rows, w.cols, x, y, ldy)
 
 
 def launch_gemm(w: Fp4, x, y=None, workspace=None):
     """Y[t][n] = gs * sum_k X[t][k] W[n][k] for any number of rows t - the prompt GEMM (launch_mma_d,
     engine/src/gen.rs:2491; glm5_gemm_fp4_tc, engine/src/kernels_glm5_moe.cu:349) on tcgen05 tensor cores.
     ``workspace``: a uint8 device tensor of at least ``gemm_workspace_bytes(w.cols, t)`` bytes (allocated when absent)."""
-    x2 = x.reshape(-1, w.cols)
-    m = x2.shape[0]
-    if y is None:
-        y = torch.empty((m, w.rows), dtype=x.dtype, device=x.device)
-    need = gemm_workspace_bytes(w.cols, m)
-    if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-    check(lib().cn_nvfp4_gemm(w.w.data_ptr(), w.gs.data_ptr(), x2.data_ptr(), y.data_ptr(), w.rows, w.cols, m, y.stride(0), _dtype_code(x),
-                              workspace.data_ptr(), workspace.numel(), _stream()))
-    return y
+    return host().gemm(w.w, w.gs, w.rows, w.cols, x, y, workspace)
 
 
 def gemm_workspace_bytes(k, m):
@@ -100,16 +84,7 @@ def launch_gemm_fp4(w: Fp4Packed, x, y=None, workspace=None):
     """Y[t][n] = gs * sum_k X[t][k] W[n][k] on the re-laid weights (gemm_fp4_dense, engine/src/kernels.rs:533). bf16 rows are multiplied as they
     are or as f16, exactly; f32 rows go through the block-scaled FP4 MMA (tcgen05 kind::mxf4nvf4) as a five-level NVFP4 cascade (the
     reference's act_cascade, engine/src/kernels.rs:5354-5475, has three)."""
-    x2 = x.reshape(-1, w.cols)
-    m = x2.shape[0]
-    if y is None:
-        y = torch.empty((m, w.rows), dtype=x.dtype, device=x.device)
-    need = int(lib().cn_nvfp4_bs_workspace_bytes(w.rows, w.cols, m))
-    if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-    check(lib().cn_nvfp4_bs_gemm(w.packed.data_ptr(), w.gs.data_ptr(), x2.data_ptr(), y.data_ptr(), w.rows, w.cols, m, y.stride(0), _dtype_code(x),
-                                 workspace.data_ptr(), workspace.numel(), _stream()))
-    return y
+    return host().bs_gemm(w.packed, w.gs, w.rows, w.cols, x, y, workspace)
 
 
 def act_cascade(x, levels=3):
@@ -146,14 +121,7 @@ def launch_gemv_gu(gate: Fp4, up: Fp4, x, h=None, limit=0.0):
     (engine/src/gen.rs:3974-3981). limit > 0 selects the clamped SwiGLU."""
     if (gate.rows, gate.cols) != (up.rows, up.cols):
         raise CrownestError(f"cpu_nvfp4: expert shapes gate [{gate.rows}, {gate.cols}], up [{up.rows}, {up.cols}] do not fit together")
-    x2 = x.reshape(-1, gate.cols)
-    m = x2.shape[0]
-    if h is None:
-        h = torch.empty((m, gate.rows), dtype=x.dtype, device=x.device)
-    check(lib().cn_nvfp4_gemv_gu(gate.w.data_ptr(), up.w.data_ptr(), gate.gs.data_ptr(), up.gs.data_ptr(), x2.data_ptr(),
-                                 h.data_ptr(), gate.rows, gate.cols, m, h.stride(0) if h.dim() == 2 else gate.rows,
-                                 float(limit), _dtype_code(x), _stream()))
-    return h
+    return host().gemv_gu(gate.w, up.w, gate.gs, up.gs, gate.rows, gate.cols, x, h, limit)
 
 
 def dense_ffn_w(gate: Fp4, up: Fp4, down: Fp4, x, limit=0.0):
@@ -234,14 +202,7 @@ def argmax(logits):
 
 def lm_head_argmax(w: Fp4, x, logits=None):
     """logits = lm_head x and their argmax per row (engine/src/gen.rs:5638-5641): returns (tokens int32 [m], logits [m][vocab])."""
-    x2 = x.reshape(-1, w.cols)
-    m = x2.shape[0]
-    if logits is None:
-        logits = torch.empty((m, w.rows), dtype=x.dtype, device=x.device)
-    tokens = torch.empty(m, dtype=torch.int32, device=x.device)
-    check(lib().cn_lm_head_argmax(w.w.data_ptr(), w.gs.data_ptr(), x2.data_ptr(), logits.data_ptr(), tokens.data_ptr(), w.rows, w.cols, m,
-                                  _dtype_code(x), _stream()))
-    return tokens, logits
+    return host().head(w.w, w.gs, w.rows, w.cols, x, logits)
 
 
 def dequant(w: Fp4, rule=False):
@@ -254,14 +215,4 @@ def dequant(w: Fp4, rule=False):
 def fp8_gemv(w, scale, x, rows, cols, y=None):
     """y[m][r] for E4M3FN weights [rows][cols] (uint8) with f32 scales per 128x128 tile
     (the codec of converter/src/fp8.rs:44-82); x [M][cols], M <= 8."""
-    x2 = x.reshape(-1, cols)
-    m = x2.shape[0]
-    if w.numel() != rows * cols:
-        raise CrownestError(f"fp8: {w.numel()} FP8 bytes for shape [{rows}, {cols}]")
-    sr, sc = -(-rows // 128), -(-cols // 128)
-    if scale.numel() != sr * sc:
-        raise CrownestError(f"fp8: {scale.numel()} scales, the 128x128 grid of [{rows}, {cols}] needs [{sr}, {sc}] = {sr * sc}")
-    if y is None:
-        y = torch.empty((m, rows), dtype=x.dtype, device=x.device)
-    check(lib().cn_fp8_gemv(w.data_ptr(), scale.data_ptr(), x2.data_ptr(), y.data_ptr(), rows, cols, m, y.stride(0), _dtype_code(x), _stream()))
-    return y
+    return host().fp8(w, scale, rows, cols, x, y)
