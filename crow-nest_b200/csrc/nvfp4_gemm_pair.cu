@@ -57,16 +57,17 @@ struct PairParams {
 // A pair's work comes in units, a tile and a part of K (all of it with one split), in the order of the splits. Counted up instead of
 // divided out, so that the compiler sees what the whole warp shares: with a quotient in the MMA warp's loop bounds its operands left the
 // uniform registers (17408 x 5120, 64 rows: 25 -> 29 us; 4096 rows of 5120 x 17408: 585 -> 616).
+template <bool SPLIT>
 struct Unit {
     int tile, split;
     __device__ __forceinline__ explicit Unit(int pair, const PairParams& p) : tile(pair), split(0) { wrap(p); }
     __device__ __forceinline__ void wrap(const PairParams& p) {
-        while (tile >= p.tiles && split < p.ksplits) tile -= p.tiles, split++;
+        while (SPLIT && tile >= p.tiles && split < p.ksplits) tile -= p.tiles, split++;
     }
-    __device__ __forceinline__ bool live(const PairParams& p) const { return split < p.ksplits; }
+    __device__ __forceinline__ bool live(const PairParams& p) const { return SPLIT ? split < p.ksplits : tile < p.tiles; }
     __device__ __forceinline__ void next(int npairs, const PairParams& p) { tile += npairs, wrap(p); }
-    __device__ __forceinline__ int first(const PairParams& p) const { return split * p.split_stages + min(split, p.split_more); }
-    __device__ __forceinline__ int count(const PairParams& p) const { return p.split_stages + (split < p.split_more ? 1 : 0); }
+    __device__ __forceinline__ int first(const PairParams& p) const { return SPLIT ? split * p.split_stages + min(split, p.split_more) : 0; }
+    __device__ __forceinline__ int count(const PairParams& p) const { return SPLIT ? p.split_stages + (split < p.split_more ? 1 : 0) : p.nk >> 2; }
 };
 
 // Where a decode warp stands in the rings of weight stages and A slots.
@@ -194,7 +195,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             uint32_t wp = 1, bp = 1;  // parity of "empty": the first round passes at once
             bool ok = true;
             const uint32_t bfull0 = smem_u32(bfull) & 0xFEFFFFFFu;  // the even CTA's barriers
-            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+            for (Unit<SPLIT> u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 const int rt = (u.tile % p.row_tiles) * 2 + (int)rank, tok0 = (u.tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1);
                 const int w0 = u.first(p), w1 = w0 + u.count(p);
                 for (int w = w0; w < w1 && ok; w++) {
@@ -232,7 +233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             int ws = 0;
             uint32_t wp = 1;  // parity of "empty": the first round passes at once
             bool ok = true;
-            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+            for (Unit<SPLIT> u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 const int rt = (u.tile % p.row_tiles) * 2 + (int)rank, w0 = u.first(p), w1 = w0 + u.count(p);
                 for (int w = w0; w < w1; w++) {
                     if (!mbar_wait(&wempty[ws], wp)) {
@@ -256,7 +257,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             bool ok = true;
             const uint32_t bfull0 = smem_u32(bfull) & 0xFEFFFFFFu;  // the even CTA's barriers
             pdl_wait();  // f16 rows come from the kernel before this one
-            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+            for (Unit<SPLIT> u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 const int tok0 = (u.tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1), w0 = u.first(p), w1 = w0 + u.count(p);
                 for (int q = 2 * w0; q < 2 * w1; q++) {
                     if (!mbar_wait(&bempty[bs], bp)) {
@@ -282,7 +283,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             int as = 0, bs = 0, ab = 0;
             uint32_t ap = 0, bp = 0, cp = 1;
             bool ok = true;
-            for (Unit u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
+            for (Unit<SPLIT> u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 if (!mbar_wait(&accempty[ab], cp)) {
                     cn_dev_fail(CN_DEV_WAIT_EMPTY);
                     break;
@@ -327,7 +328,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     } else if (SETS == 2 && warp >= 4 && warp < 12) {
         // ------------------------------------------------------------ decode
         int stages = 0;
-        for (Unit u(pair, p); u.live(p); u.next(npairs, p)) stages += u.count(p);
+        for (Unit<SPLIT> u(pair, p); u.live(p); u.next(npairs, p)) stages += u.count(p);
         decode(stages);
     } else if (warp >= 4) {
         // ------------------------------------------------------------ results: lane = weight row, 32 tokens per load, the two (four) warps of a
@@ -341,7 +342,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
         int ab = 0;
         uint32_t cp = 0;
         if (SETS == 2) pdl_wait();  // the row factors come from the kernel before this one
-        for (Unit u(pair, p); u.live(p); u.next(npairs, p)) {
+        for (Unit<SPLIT> u(pair, p); u.live(p); u.next(npairs, p)) {
             const int tile = u.tile;
             float* part = SPLIT && p.ksplits > 1 ? p.part + (size_t)u.split * p.m * p.rows : nullptr;
             if (SETS == 4) {
