@@ -81,6 +81,7 @@ struct GemvParams {
     const float* side_gs;
     float* side_y;
     int side_rows;
+    int xch_slots, team_bytes;  // clusters: tiles of one; shared memory of a team in front of the activations
     int red_depth;  // multi-row tensor-core kernel: tile-sum slots in flight
     // tensor-parallel line output (see GemvCall): line buffer of every rank (0 = none), first global row, the counter
     unsigned long long yl[8];

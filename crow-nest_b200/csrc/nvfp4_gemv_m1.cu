@@ -16,6 +16,8 @@
 // When the tiles do not fill the last wave and a CTA's share is long enough (the down projection), or the
 // tiles are too few to fill the machine (a tensor-parallel rank's share of it), the launch is made of
 // clusters of two or four CTAs that take a part of K each, or with several rows two parts (see the helpers below).
+// Where the staged rows of several activation rows leave an SM a single CTA, that CTA holds two teams - nine warps with a ring and tile
+// sums of their own - that share the rows and take tiles like CTAs of their own.
 // The LN variant (one activation row) also stores the output rows as 16-byte lines into the line buffers of
 // the other GPUs of a tensor-parallel group: the exchange that follows the projection starts in its epilogue.
 //
@@ -37,7 +39,7 @@
 namespace {
 
 constexpr int NW = 8;  // consumer warps
-constexpr int NTHREADS = (NW + 1) * 32;
+constexpr int TEAM = (NW + 1) * 32;  // threads of a team: the consumer warps and a producer
 constexpr int MAX_STAGES = 8;
 constexpr int RED_DEPTH = 12;  // sums of a tile or part in flight, at most (see red_slots)
 constexpr int XB = 128;        // one 64-value block of f16 activations, 16-byte chunks XOR-swizzled
@@ -53,10 +55,10 @@ constexpr int ROWS = 16;
 // ---- two-CTA cluster helpers (K range of a tile shared between the CTAs of a pair)
 // f32 [8 slots][up to 3 senders][16] sums from the other CTAs of a cluster of two or four, then a barrier per slot
 constexpr int XCH_OFF = 256, XCH_SLOTS = 8, XBAR_OFF = XCH_OFF + XCH_SLOTS * 3 * 64;
-// Tiles of a CTA that have a slot of their own (slots are not used twice). With more than one activation row a cluster has one tile (it
-// is launched only where the machine is not filled otherwise), and its slot - a sum per part of the other CTAs - lies behind the tile sums.
-__host__ __device__ constexpr int xch_slots(int mt) { return mt == 1 ? XCH_SLOTS : 1; }
-static_assert(XBAR_OFF + XCH_SLOTS * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
+// Tiles of a CTA each have a slot of their own (slots are not used twice). With more than one activation row the slots - a sum per part of
+// the other CTAs - lie behind the tile sums.
+constexpr int MAX_SLOTS = 32;
+static_assert(XBAR_OFF + MAX_SLOTS * 8 <= ZERO2_OFF, "the cluster exchange overlaps the header");
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -122,12 +124,16 @@ __device__ __forceinline__ void push_lines(const GemvParams& p, int row0, int nr
 // KS: 1, or 2 / 4 = launched as clusters of so many CTAs that share the K range of every tile
 // LN: tensor-parallel line output compiled in (one activation row only); without it the kernel carries none of that code
 // PP: parts of K that a CTA sums one after another (more than one activation row, and a matrix of KS x PP parts)
-template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1>
-__global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const GemvParams p) {
+// NT: teams of the CTA
+template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1, int NT = 1>
+__global__ void __launch_bounds__(NT * TEAM, CPS) nvfp4_gemv_m1_kernel(const GemvParams p) {
     static_assert(!LN || MT == 1, "line output takes one activation row");
     static_assert(PP == 1 || MT > 1, "one activation row has a CTA for every part");
+    static_assert(NT == 1 || MT > 1, "one activation row has CTAs enough");
+    constexpr int NTHREADS = NT * TEAM;
     extern __shared__ __align__(128) uint8_t smem[];
     if (threadIdx.x == 0) { CN_STAMP(0); }
+    const int team = NT > 1 ? (int)threadIdx.x / TEAM : 0;
     float gs0_early = __ldg(p.gs0), gs1_early = __ldg(p.gs1);  // tensor scales: asked for first, used late
     int rows = p.rows;
     constexpr int pstride = TX * 36 + 16;  // padded: the eight rows of a quad column hit distinct banks
@@ -135,7 +141,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     constexpr int GPW = TX / 2 / NW > 0 ? TX / 2 / NW : 1;  // groups per warp and full chunk
     // KS > 1: the CTAs of a cluster walk the same tiles, each over its part of K
     const int crank = KS > 1 ? (int)(blockIdx.x % KS) : 0;
-    const int cid = KS > 1 ? (int)(blockIdx.x / KS) : (int)blockIdx.x, ncl = KS > 1 ? (int)(gridDim.x / KS) : (int)gridDim.x;
+    // (the first teams of all CTAs come before the second ones: few tiles spread over the SMs)
+    const int ncta = KS > 1 ? (int)(gridDim.x / KS) : (int)gridDim.x, cid = (KS > 1 ? (int)(blockIdx.x / KS) : (int)blockIdx.x) + team * ncta, ncl = ncta * NT;
     const int bpr_all = p.k >> 6;
     const int bpr = bpr_all / KS, b0 = crank * bpr;  // this CTA's blocks of every row: [b0, b0 + bpr)
     const size_t row_bytes = (size_t)bpr_all * 36;
@@ -170,21 +177,23 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     }
     const bool gu = w1 != nullptr;
 
-    uint64_t* full = (uint64_t*)smem;
+    uint8_t* tm = smem + (NT > 1 ? team * p.team_bytes : 0);  // this team's header, sums and exchange; then come the activations and the rings
+    uint64_t* full = (uint64_t*)tm;
     uint64_t* empty = full + MAX_STAGES;
-    uint64_t* tbar = (uint64_t*)(smem + TBAR_OFF);  // [RED_DEPTH] one per tile-sum buffer
+    uint64_t* tbar = (uint64_t*)(tm + TBAR_OFF);  // [RED_DEPTH] one per tile-sum buffer
     float* lut = (float*)(smem + LUT_OFF);  // [2][256] ue4m3 * gs
-    float* red = (float*)(smem + RED_OFF);  // [red_depth][NW][MT][16] partial sums of a tile
+    float* red = (float*)(tm + RED_OFF);  // [red_depth][NW][MT][16] partial sums of a tile
     const int RD = p.red_depth;             // tile sums in flight (<= RED_DEPTH)
     // the sums handed over inside a cluster: in the header for one activation row, behind the tile sums for more
     const uint32_t xch_off = MT == 1 ? (uint32_t)XCH_OFF : (uint32_t)(RED_OFF + RD * NW * MT * 64);
-    const uint32_t xs_off = (uint32_t)(RED_OFF + RD * NW * MT * 64) + (KS > 1 && MT > 1 ? (uint32_t)(xch_slots(MT) * (KS - 1) * PP * MT * 64) : 0u);
+    const uint32_t xs_off = NT > 1 ? (uint32_t)(NT * p.team_bytes) : (uint32_t)(RED_OFF + RD * NW * MT * 64) + (KS > 1 && MT > 1 ? (uint32_t)(p.xch_slots * (KS - 1) * PP * MT * 64) : 0u);
     uint8_t* xs0 = smem + xs_off;           // [MT][bpr][128] f16 activations
     const uint32_t XS = (uint32_t)bpr * XB;  // bytes of one activation row
     float* xinv0 = (float*)(xs0 + (size_t)MT * XS);  // [MT][bpr]
-    uint8_t* stage0 = (uint8_t*)(xinv0 + ((MT * bpr + 3) & ~3));
+    uint8_t* stage0 = (uint8_t*)(xinv0 + ((MT * bpr + 3) & ~3)) + (NT > 1 ? (size_t)team * S * stage_bytes : 0);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int lane = threadIdx.x & 31, warp = ((int)threadIdx.x - team * TEAM) >> 5;
+    const int tid = NT > 1 ? team * (NW * 32) + (int)threadIdx.x - team * TEAM : (int)threadIdx.x;  // among the consumers
     const int per_cta = gu ? ROWS / 2 : ROWS;  // gate/up: 8 indices, row slots 0-7 gate, 8-15 up
     const int ntiles = (rows + per_cta - 1) / per_cta;
 
@@ -192,11 +201,11 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     // depend on the previous kernel); the consumers meet it on named barrier 2 before their first wait.
     if (warp == NW) {
         // one barrier per lane and round: S full + S empty + RD tile-sum (+ the pair's exchange slots), side by side
-        for (int i = lane; i < 2 * S + RD + (KS > 1 ? xch_slots(MT) : 0); i += 32) {
+        for (int i = lane; i < 2 * S + RD + (KS > 1 ? (MT == 1 ? XCH_SLOTS : p.xch_slots) : 0); i += 32) {
             if (i < S) mbar_init(&full[i], 1);
             else if (i < 2 * S) mbar_init(&empty[i - S], NW);
             else if (i < 2 * S + RD) mbar_init(&tbar[i - 2 * S], NW);
-            else mbar_init((uint64_t*)(smem + XBAR_OFF) + (i - 2 * S - RD), KS - 1);  // one arrival per other CTA of the cluster
+            else mbar_init((uint64_t*)(tm + XBAR_OFF) + (i - 2 * S - RD), KS - 1);  // one arrival per other CTA of the cluster
         }
 #ifdef CN_M1_TRACE
         if (lane == 0) { CN_STAMP(7); }
@@ -276,12 +285,12 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     constexpr int PF = CPS >= 4 ? 2 : 4;
     uint4 pre[PF];
 #pragma unroll
-    for (int i = 0; i < PF; i++) pre[i] = load_x(tid + i * (NW * 32));
+    for (int i = 0; i < PF; i++) pre[i] = load_x(tid + i * (NT * NW * 32));
     if (tid < 4) ((uint32_t*)(smem + ZERO_OFF))[tid] = 0u;
     if (tid >= 4 && tid < 8) ((uint32_t*)(smem + ZERO2_OFF))[tid - 4] = 0u;
     {
         const float g1 = gu ? gs1_early : gs0_early;
-        for (int b = tid; b < 256; b += NW * 32) {
+        for (int b = tid; b < 256; b += NT * NW * 32) {
             const float u = ue4m3_f32((uint32_t)b, true);
             lut[b] = u * gs0_early;
             lut[256 + b] = u * g1;
@@ -290,12 +299,12 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     bool ok = true;
     // bf16 -> f16 * 2^e per 64-value block, chunk i of block b stored at chunk i ^ (b & 7). Eight lanes per block,
     // one 16-byte chunk each, straight from global memory (k % 256 == 0 makes every warp wholly in or out of range).
-    for (int task0 = tid; task0 < ntask; task0 += PF * NW * 32) {
+    for (int task0 = tid; task0 < ntask; task0 += PF * NT * NW * 32) {
 #pragma unroll
       for (int pf = 0; pf < PF; pf++) {
-        const int task = task0 + pf * (NW * 32);
+        const int task = task0 + pf * (NT * NW * 32);
         const uint4 raw = pre[pf];
-        pre[pf] = load_x(task + PF * NW * 32);
+        pre[pf] = load_x(task + PF * NT * NW * 32);
         if (task >= ntask) break;  // uniform over the warp
         const int b = task >> 3, i = task & 7;
         const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -533,8 +542,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
             // the parts posted since the tile's start, in order; as for one row below, lane l over (activation row, row slot)
             // pairs l, l + 32, ...
             constexpr int NO = MT > 1 ? MT / 2 : 1;
-            float* xch = (float*)(smem + xch_off);
-            uint64_t* xb = (uint64_t*)(smem + XBAR_OFF);
+            float* xch = (float*)(tm + xch_off) + titer * ((KS - 1) * PP * MT * 16);
+            uint64_t* xb = (uint64_t*)(tm + XBAR_OFF) + titer;
             float tot[NO];
             const bool mine = warp == (titer & (NW - 1));  // the warps take turns
 #pragma unroll
@@ -597,8 +606,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
                     v[i] = rb[o];
                     for (int w = 1; w < NW; w++) v[i] += rb[w * MT * 16 + o];
                 }
-                float* xch = (float*)(smem + xch_off);
-                uint64_t* xb = (uint64_t*)(smem + XBAR_OFF);
+                float* xch = (float*)(tm + xch_off) + titer * ((KS - 1) * MT * 16);
+                uint64_t* xb = (uint64_t*)(tm + XBAR_OFF) + titer;
                 if (crank != 0) {
 #pragma unroll
                     for (int i = 0; i < NO; i++) st_peer_f32(peer_addr(xch + (crank - 1) * MT * 16 + lane + 32 * i, 0), v[i]);
@@ -698,10 +707,10 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_m1_kernel(const Gemv
     if (KS > 1) cluster_sync_all();  // nobody leaves while a CTA of the cluster may still send or receive
 }
 
-template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1>
+template <int TX, int CPS, int MT, int KS = 1, bool LN = false, int PP = 1, int NT = 1>
 int launch_m1(const cudaLaunchConfig_t& cfg, const GemvParams& p) {
-    CN_ALLOW_SMEM((nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP>), 226 * 1024);
-    CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP>, p));
+    CN_ALLOW_SMEM((nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP, NT>), 226 * 1024);
+    CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_m1_kernel<TX, CPS, MT, KS, LN, PP, NT>, p));
     return CN_OK;
 }
 
@@ -709,9 +718,10 @@ int launch_m1(const cudaLaunchConfig_t& cfg, const GemvParams& p) {
 // then, and the parts that it has posted there end at least `gap` chunks apart: n + stages / gap, and one to spare.
 int red_slots(int stages, int gap, int n) { return n + stages / gap + 1 < RED_DEPTH ? n + stages / gap + 1 : RED_DEPTH; }
 static_assert(4 + MAX_STAGES <= RED_DEPTH, "slots of the tile sums");
-// Shared memory of a CTA in front of its weight ring: header, those sums, the ones handed over inside a cluster, activations.
-long long front_bytes(int stages, int gap, int n, int mt, int bpr, int handed) {
-    return (long long)RED_OFF + (long long)(red_slots(stages, gap, n) * NW + handed) * mt * 64 + (long long)mt * bpr * XB + (long long)((mt * bpr + 3) & ~3) * 4;
+// Shared memory of a CTA in front of its weight rings: for each team header, those sums and the ones handed over inside a cluster; activations.
+long long team_bytes(int stages, int gap, int n, int mt, int handed) { return (long long)RED_OFF + (long long)(red_slots(stages, gap, n) * NW + handed) * mt * 64; }
+long long front_bytes(int stages, int gap, int n, int mt, int bpr, int handed, int teams = 1) {
+    return teams * team_bytes(stages, gap, n, mt, handed) + (long long)mt * bpr * XB + (long long)((mt * bpr + 3) & ~3) * 4;
 }
 long long sm_share(int cps) { return (227 * 1024) / cps - 1024; }
 long long stage_bytes_of(int tx) { return (long long)ROWS * (tx * 36 + 16); }
@@ -796,39 +806,51 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         }
         grid = (ntiles + ((ntiles + grid - 1) / grid) - 1) / ((ntiles + grid - 1) / grid);  // the same tiles per CTA, fewer CTAs
     }
-    // CTAs per cluster: one row takes a CTA for every part. With two and more activation rows the parts of a tile go to the CTAs of a
-    // cluster where the machine is not filled otherwise and that shortens the busiest SM, else to one CTA after another. Its time in
-    // blocks: the tiles or parts that it holds, half as much again where a single CTA's eight warps are all it has (two rows; from
-    // four rows on they nearly keep the issue slots busy: a fifth), and 24 for meeting in the first CTA. Measured, us alone /
-    // shared: 2048 x 8192 with two rows 8.2 / 6.9, with four 7.6 / 8.7; 640 x 17408 with two, four and eight rows 10.8 / 6.8 (four CTAs),
-    // 14.0 / 8.3 (four; 10.5 with two), 27.8 / 15.9 (two); 1000 x 9216 7.0 / 6.0, 8.1 / 7.1, 12.4 / 10.1.
-    int ksplit = mt == 1 ? parts : 1;
-    if (mt > 1) {
-        const double alone = mt == 2 ? 1.5 : 1.2;
-        auto busiest = [&](int ks) {
-            const int n = (int)(((long long)ntiles * ks + 147) / 148);
-            return n * (double)(bpr / ks) * (n == 1 ? alone : 1.0) + (ks > 1 ? 24.0 : 0.0);
-        };
-        for (int ks = 2; ks <= parts; ks *= 2) {
-            auto fits = [&](int c) { return sm_share(c) - front_bytes(3, gap(parts / ks), parts / ks, mt, bpr / ks, parts - parts / ks) >= 3 * stage_bytes; };
-            const int ck = fits(2) ? 2 : 1;
-            if (!fits(ck) || (long long)ntiles * ks > 148LL * ck || (long long)ROWS * (bpr / ks) * 36 < 32 * 1024) continue;
-            if (busiest(ks) <= 0.9 * busiest(ksplit)) ksplit = ks, cps = ck;
+    // CTAs per cluster: one row takes a CTA for every part. With two and more activation rows the parts of a tile go to as many CTAs of a cluster
+    // as make the busiest SM's work shortest, else to one CTA after another. Its time in blocks: the tiles or parts that it holds, the odd one
+    // half as much again (two rows; the more rows, the nearer eight warps come to keeping the issue slots busy), as everything where an SM
+    // has a single team; and 22 for meeting in the first CTA, 44 for four. A CTA of two teams comes before two CTAs (us of the two, two / four rows: 17408 x
+    // 5120 gate / up 27.3 / 30.2 and 27.4 / 31.0, 7168 x 5120 8.5 / 9.8 and 9.3 / 11.1, 3000 x 9216 8.6 / 10.0 and 9.6 / 11.8; eight rows of gate / up
+    // 46.6, one team 59.6), but not in clusters of four, which fill the SMs of a GPC badly with one CTA each (640 x 17408 10.3 / 12.0 and
+    // 6.8 / 8.3), nor where tiles are short (two rows of 20246 x 1536 10.1 and 9.2,
+    // eight of 248000 x 2048 154 and 147). 5120 x 17408, two, four and eight rows:
+    // 18.6 / 21.3 / 34.8 in clusters of two; 22.0 / 26.7 / 53.1 with parts one after another and a single team.
+    int ksplit = mt == 1 ? parts : 1, teams = 1, waves = 1;
+    if (mt > 1 && !routed) {
+        const double alone = mt == 2 ? 1.5 : (mt == 4 ? 1.3 : 1.2);
+        double best = 1e30;
+        for (int ks = 1; ks <= parts; ks *= 2) {
+            if (ks > 1 && (long long)ROWS * (bpr / ks) * 36 < 32 * 1024) continue;
+            const int n = parts / ks;
+            const bool ctas = ks == 4 || (tx == 16 && mt < 8) || (mt == 8 && gap(n) == 1 && ntiles > 8 * 148);
+            for (int f = 0; f < 3; f++) {
+                const int form = !ctas && f < 2 ? 1 - f : f;  // 0: two CTAs per SM, 1: one of two teams, 2: one of one
+                const int c = form == 0 ? 2 : 1, nt = form == 1 ? 2 : 1, per_sm = c * nt, clusters = 148 * c / ks * nt, wv = (ntiles + clusters - 1) / clusters;
+                if (ks > 1 && wv > MAX_SLOTS) continue;
+                const long long room = sm_share(c) - front_bytes(3, gap(n), n, mt, bpr / ks, ks > 1 ? wv * (ks - 1) * n : 0, nt);
+                if (room < (form < 2 ? nt * 3 : 2) * stage_bytes) continue;
+                const long long held = ((long long)ntiles * ks + 147) / 148;
+                const double t = (per_sm < 2 ? held * alone : (double)(held & ~1LL) + (held & 1) * alone) * (bpr / ks) + (ks > 1 ? 11.0 * ks : 0.0);
+                if (t <= (ks == 4 ? 0.91 : 0.9) * best) best = t, ksplit = ks, cps = c, teams = nt, waves = ks > 1 ? wv : 1;
+                break;
+            }
         }
+        grid = ntiles < 148 * cps ? ntiles : 148 * cps;
     }
     if (ksplit > 1) {
         const int clusters = 148 * cps / ksplit;
         grid = ksplit * (ntiles < clusters ? ntiles : clusters);
     }
     const int pp = parts / ksplit;  // parts of a CTA
-    auto front = [&](int st) { return front_bytes(st, gap(pp), pp, mt, bpr / ksplit, mt > 1 ? parts - pp : 0); };
+    const int handed = mt > 1 && ksplit > 1 ? waves * (ksplit - 1) * pp : 0;
+    auto front = [&](int st) { return front_bytes(st, gap(pp), pp, mt, bpr / ksplit, handed, teams); };
     int fit = MAX_STAGES;  // ring depth that fits beside the fixed part
-    while (fit > 1 && front(fit) + fit * stage_bytes > sm_share(cps)) fit--;
+    while (fit > 1 && front(fit) + teams * fit * stage_bytes > sm_share(cps)) fit--;
     int stages = fit;
-    const int total_chunks = ((pp * bpp + tx - 1) / tx) * ((ntiles + grid / ksplit - 1) / (grid / ksplit));
+    const int total_chunks = ((pp * bpp + tx - 1) / tx) * ((ntiles + grid / ksplit * teams - 1) / (grid / ksplit * teams));
     if (stages > total_chunks) stages = total_chunks;
     if (stages < 1) stages = 1;
-    const size_t smem = (size_t)(front(stages) + stages * stage_bytes);
+    const size_t smem = (size_t)(front(stages) + teams * stages * stage_bytes);
     if (smem > 226 * 1024 || fit < 2) {
         // the staged activations of all m rows do not fit beside a ring: two calls over half the rows each
         if (m == 1) CN_FAIL(CN_ERR_LIMIT, "%s: k = %d needs %zu B of shared memory per block", who, k, smem);
@@ -844,7 +866,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = a.x, p.y = a.y;
     p.rows = rows, p.k = k, p.m = m, p.ldy = a.ldy, p.limit = a.limit, p.tx = tx, p.stages = stages, p.out_f32 = a.out_f32;
     p.ids = a.ids, p.order = a.order, p.tab0 = a.tab0, p.tab1 = a.tab1, p.fused_up_rows = a.fused_up_rows, p.x_div = a.x_div;
-    p.red_depth = red_slots(stages, gap(pp), pp);
+    p.red_depth = red_slots(stages, gap(pp), pp), p.xch_slots = waves, p.team_bytes = (int)team_bytes(stages, gap(pp), pp, mt, handed);
     p.experts = a.experts, p.yptrs = a.yptrs;
     p.combos = a.combos, p.side_w0 = (const uint8_t*)a.side_w0, p.side_w1 = (const uint8_t*)a.side_w1, p.side_gs = a.side_gs, p.side_y = a.side_y;
     p.side_rows = a.side_rows;
@@ -864,7 +886,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
 #endif
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, (unsigned)(routed ? combos : 1));
-    cfg.blockDim = dim3(NTHREADS);
+    cfg.blockDim = dim3((unsigned)(teams * TEAM));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute at[2];
@@ -872,27 +894,27 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    // Parts are 44 blocks and longer, of 132 bytes per activation row: two CTAs per SM hold one part of four rows or two parts of two, and
-    // never eight rows.
-#define CN_M1_PARTS(KSV, PPV)                                                                      \
-    if (mt > 1 && ksplit == KSV && pp == PPV) {                                                    \
-        if (mt == 2 && cps == 2) return launch_m1<32, 2, 2, KSV, false, PPV>(cfg, p);              \
-        if (mt == 2) return launch_m1<32, 1, 2, KSV, false, PPV>(cfg, p);                          \
-        if (mt == 4 && cps == 2) return launch_m1<32, PPV == 1 ? 2 : 1, 4, KSV, false, PPV>(cfg, p); \
-        if (mt == 4) return launch_m1<32, 1, 4, KSV, false, PPV>(cfg, p);                          \
-        return launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p);                                       \
-    }
-    CN_M1_PARTS(1, 2) CN_M1_PARTS(1, 4)
     if (ksplit > 1) {
         at[1].id = cudaLaunchAttributeClusterDimension;
         at[1].val.clusterDim.x = (unsigned)ksplit, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
+    }
+    if (mt > 1) {
+#define CN_M1_PARTS(KSV, PPV)                                                                                           \
+    if (ksplit == KSV && pp == PPV) {                                                                                   \
+        if (mt == 2) return teams == 2 ? launch_m1<32, 1, 2, KSV, false, PPV, 2>(cfg, p) : launch_m1<32, 2, 2, KSV, false, PPV>(cfg, p); \
+        if (mt == 4) return teams == 2 ? launch_m1<32, 1, 4, KSV, false, PPV, 2>(cfg, p) : launch_m1<32, 2, 4, KSV, false, PPV>(cfg, p); \
+        return teams == 2 ? launch_m1<32, 1, 8, KSV, false, PPV, 2>(cfg, p) : launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p); \
+    }
+        if (tx == 32 && (parts > 1 || teams > 1)) {
+            CN_M1_PARTS(1, 1) CN_M1_PARTS(1, 2) CN_M1_PARTS(1, 4) CN_M1_PARTS(2, 1) CN_M1_PARTS(2, 2) CN_M1_PARTS(4, 1)
+        }
+#undef CN_M1_PARTS
+    } else if (ksplit > 1) {
         if (p.yl_world > 0) {
             if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2, true>(cfg, p) : launch_m1<32, 3, 1, 2, true>(cfg, p);
             return cps == 2 ? launch_m1<32, 2, 1, 4, true>(cfg, p) : launch_m1<32, 3, 1, 4, true>(cfg, p);
         }
-        CN_M1_PARTS(2, 1) CN_M1_PARTS(2, 2) CN_M1_PARTS(4, 1)
-#undef CN_M1_PARTS
         if (ksplit == 2) return cps == 2 ? launch_m1<32, 2, 1, 2>(cfg, p) : launch_m1<32, 3, 1, 2>(cfg, p);
         return cps == 2 ? launch_m1<32, 2, 1, 4>(cfg, p) : launch_m1<32, 3, 1, 4>(cfg, p);
     }
@@ -904,11 +926,12 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         CN_FAIL(CN_ERR_SHAPE, "%s: line output needs k >= 2048 (k = %d)", who, k);
     }
 #define CN_M1_CASE(TXV, CPSV, MTV) \
-    if (tx == TXV && cps == CPSV && mt == MTV) return launch_m1<TXV, CPSV, MTV>(cfg, p);
+    if (tx == TXV && cps == CPSV && mt == MTV && teams == 1) return launch_m1<TXV, CPSV, MTV>(cfg, p);
     CN_M1_CASE(32, 2, 1) CN_M1_CASE(32, 3, 1) CN_M1_CASE(32, 4, 1) CN_M1_CASE(16, 2, 1) CN_M1_CASE(16, 3, 1) CN_M1_CASE(16, 4, 1)
     CN_M1_CASE(32, 1, 2) CN_M1_CASE(32, 2, 2) CN_M1_CASE(16, 1, 2) CN_M1_CASE(16, 2, 2)
     CN_M1_CASE(32, 1, 4) CN_M1_CASE(32, 2, 4) CN_M1_CASE(16, 1, 4) CN_M1_CASE(16, 2, 4)
     CN_M1_CASE(32, 1, 8) CN_M1_CASE(32, 2, 8) CN_M1_CASE(16, 1, 8) CN_M1_CASE(16, 2, 8)
+    if (tx == 16 && teams == 2 && mt > 1) return mt == 2 ? launch_m1<16, 1, 2, 1, false, 1, 2>(cfg, p) : (mt == 4 ? launch_m1<16, 1, 4, 1, false, 1, 2>(cfg, p) : launch_m1<16, 1, 8, 1, false, 1, 2>(cfg, p));
 #undef CN_M1_CASE
     CN_FAIL(CN_ERR_SHAPE, "%s: no kernel for %d blocks per stage, %d CTAs per SM, %d rows", who, tx, cps, mt);
 }

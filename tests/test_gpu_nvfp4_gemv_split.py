@@ -1,5 +1,5 @@
-"""Several bf16 rows over matrices whose rows are summed in two or four parts of k, by the CTAs of a cluster or by one CTA after another: few
-long rows, a matrix that fills the machine, rows that end inside a tile, activation rows that fill their slots or not. Every row has the
+"""Several bf16 rows over matrices whose rows are summed in one, two or four parts of k, by the CTAs of a cluster or by one CTA after another, with one or
+two teams of warps to a CTA: few long rows, a matrix that fills the machine, rows that end inside a tile, activation rows that fill their slots or not. Every row has the
 bits of a one-row call."""
 import numpy as np
 import pytest
@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,k,gu", [(5120, 17408, False), (5111, 17408, False), (2560, 17408, True), (640, 17408, False), (1280, 17408, False),
-                                       (333, 9216, False), (2048, 8192, False), (2048, 12288, False), (999, 12288, True), (320, 33792, False)])
+                                       (333, 9216, False), (2048, 8192, False), (2048, 12288, False), (999, 12288, True), (320, 33792, False),
+                                       # one part: two teams of a CTA with one tile, with uneven shares, with short rows, with none for the second
+                                       (3000, 5120, True), (7161, 5120, False), (700, 1536, False), (40, 4096, False)])
 @pytest.mark.parametrize("m", [2, 3, 4, 5, 8])
 def test_rows_of_a_shared_tile(rows, k, gu, m):
     rng = np.random.default_rng(rows + k + m)
