@@ -128,3 +128,43 @@ __device__ __forceinline__ float bf16_plane(const uint4& raw, int lane, uint32_t
     }
     return __uint_as_float((e - 6u) << 23);
 }
+
+// ---------------------------------------------------------------- tiles of short rows, by their warp's own asynchronous copies
+// 16 row pieces of eight blocks (288 bytes) -> shared memory, PIECE_PITCH apart: nine 16-byte copies of each lane instead of a bulk copy for every
+// piece, whose number and not size is what the copy engine takes its time for (see nvfp4_rows.cu).
+constexpr int PIECE_PITCH = 8 * 36 + 16, PIECE_TILE = 16 * PIECE_PITCH;
+struct PieceCopy {
+    uint32_t at[9];  // copy i of this lane: row in the lower half, 16-byte part of the piece in the upper
+    __device__ __forceinline__ explicit PieceCopy(int lane) {
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            const uint32_t n = 32u * i + lane, r = n / 18u;
+            at[i] = r | ((n - 18u * r) << 16);
+        }
+    }
+    // rows 0 .. have_lo - 1 of lo and, as rows 8 and on, 0 .. have_hi - 1 of hi; parts of 16 bytes in a piece: 18, or 9 for half of one
+    __device__ __forceinline__ void operator()(uint32_t dst, const uint8_t* lo, const uint8_t* hi, uint32_t row_bytes, uint32_t have_lo, uint32_t have_hi, uint32_t parts,
+                                               uint64_t policy) const {
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            const uint32_t r = at[i] & 0xffffu, part = at[i] >> 16;
+            const bool upper = r >= 8u;
+            if (part < parts && (r & 7u) < (upper ? have_hi : have_lo))
+                asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + r * PIECE_PITCH + part * 16u),
+                             "l"((upper ? hi : lo) + (size_t)((r & 7u) * row_bytes + part * 16u)), "l"(policy)
+                             : "memory");
+        }
+    }
+};
+__device__ __forceinline__ void piece_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the n youngest groups of this thread's copies have landed (n <= 3)
+__device__ __forceinline__ void piece_wait(int n) {
+    if (n <= 0)
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (n == 1)
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (n == 2)
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else
+        asm volatile("cp.async.wait_group 3;" ::: "memory");
+}

@@ -6,7 +6,8 @@
 //
 // An expert's matrices are small (2048 x 512: a row is 288 bytes), so what a GEMV kernel spends per tile - handing sums between
 // warps, staging and scale tables per CTA - outweighs the tile. Here a warp keeps a 16-row tile to itself: it brings the tile in
-// by its own bulk copies (16 row pieces of up to eight blocks, two to four chunks ahead), holds all its sums in registers and stores
+// by its own asynchronous copies (16 row pieces of up to eight blocks, two to four chunks ahead; as a bulk copy each, some 25 cycles of the copy
+// engine whatever their size, they were what the kernel waited for: 64 tokens 244 us a step, 224 with 16-byte copies), holds all its sums in registers and stores
 // them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
 // columns) share one decode of its weights; a row's sum does not depend on the rows it is grouped with. Bound by issue slots:
 // some 180 warp instructions per 16 x 128 values in all (200 and 258 us a step with one scale made at a time, 245 now). Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
@@ -18,10 +19,9 @@ namespace {
 
 constexpr int NW = 8;
 constexpr int CB = 8;  // blocks per row and chunk
-constexpr int PITCH = CB * 36 + 16;
-constexpr int CHUNK = 16 * PITCH;
+constexpr int PITCH = PIECE_PITCH, CHUNK = PIECE_TILE;
 constexpr int MAX_D = 4;
-constexpr int HDR = NW * MAX_D * 8;
+static_assert(PITCH == CB * 36 + 16, "pieces of a chunk");
 
 struct RowsParams {
     RowsCall c;
@@ -47,18 +47,12 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
     const int t0 = (int)((long long)blockIdx.x * T / p.parts), t1 = (int)((long long)(blockIdx.x + 1) * T / p.parts);
     const int nch = (bpr + CB - 1) / CB, D = p.depth;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t* full = (uint64_t*)smem + warp * MAX_D;
     uint8_t* ring = smem + p.ring_off + (size_t)warp * D * CHUNK;
     const int mytiles = t0 + warp < t1 ? (t1 - t0 - warp + NW - 1) / NW : 0, total = mytiles * nch;
-    if (lane == 0) {
-        for (int i = 0; i < D; i++) mbar_init(&full[i], 1);
-        mbar_fence_init();
-    }
-    __syncwarp();
+    const PieceCopy copy(lane);
     const uint64_t pol = l2_policy_evict_first();
     const int n1 = c.count1 ? *c.count1 : 0, ngroups = c.w0 ? (c.m + RG - 1) / RG : (c.order ? n1 + *c.count2 : c.m);
     int s = 0, pstage = 0;  // stage read next, stage filled next: they meet again at the end of every group
-    uint32_t par = 0;
     for (int grp = blockIdx.y; grp < ngroups; grp += gridDim.y) {
         // the group's rows and matrices: one-row groups, larger groups, or (dense form) RG rows after one another
         int pos = grp * RG, nrows = min(RG, c.m - pos);
@@ -75,24 +69,23 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
             if (!w0 || (gu && !w1)) continue;  // this matrix of the expert is not resident
         }
         auto member = [&](int r) { return c.order ? c.order[pos + r] : pos + r; };
-        // chunk i of this warp in turn -> the next stage
-        int ptile = t0 + warp, pch = 0;
+        // chunk i of this warp in turn -> the next stage; a group of copies is closed even when there is no chunk left, so that D - 1 younger
+        // ones stand behind every chunk that is waited for
+        int ptile = t0 + warp, pch = 0, given = 0;
+        const uint32_t ring_at = smem_u32(ring);
         auto issue = [&]() {
-            const int row = gu ? ptile * 8 + (lane & 7) : ptile * 16 + lane;
-            const uint8_t* wb = (gu && ((lane >> 3) & 1)) ? w1 : w0;
-            const bool have = lane < 16 && row < c.rows;
-            const uint32_t piece = (uint32_t)min(CB, bpr - pch * CB) * 36u;
-            const uint32_t n = (uint32_t)__popc(__ballot_sync(0xffffffffu, have));
-            if (lane == 0) {
-                mbar_expect_tx(&full[pstage], n * piece);
-                mbar_arrive(&full[pstage]);
+            if (given++ < total) {
+                const uint32_t parts = (uint32_t)min(CB, bpr - pch * CB) * 9u / 4u;
+                const uint8_t* lo = w0 + (size_t)ptile * per_tile * row_bytes + (size_t)pch * (CB * 36);
+                const uint8_t* hi = gu ? w1 + (lo - w0) : lo + 8 * row_bytes;
+                const int left = c.rows - ptile * per_tile;
+                copy(ring_at + (uint32_t)(pstage * CHUNK), lo, hi, (uint32_t)row_bytes, (uint32_t)min(left, 8), (uint32_t)(gu ? min(left, 8) : max(left - 8, 0)), parts, pol);
+                if (++pch == nch) pch = 0, ptile += NW;
+                if (++pstage == D) pstage = 0;
             }
-            __syncwarp();
-            if (have) bulk_g2s_stream(ring + (size_t)pstage * CHUNK + (size_t)lane * PITCH, wb + (size_t)row * row_bytes + (size_t)pch * (CB * 36), piece, &full[pstage], pol);
-            if (++pch == nch) pch = 0, ptile += NW;
-            if (++pstage == D) pstage = 0;
+            piece_commit();
         };
-        for (int i = 0; i < D && i < total; i++) issue();
+        for (int i = 0; i < D; i++) issue();
 
         // the group's rows: eight lanes per 64-value block; column, block and chunk order as in nvfp4_gemv_col.cu
         const int ncol = NPL * nrows;
@@ -123,9 +116,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
         const int xflip = (col & 1) ? -64 : 64;
         const uint8_t* xi0 = smem + p.inv_off + 8 * t;
         const uint8_t* rbase = ring + g * PITCH + 4 * t;
-        int done = 0;
-        bool ok = true;
-        for (int tile = t0 + warp; tile < t1 && ok; tile += NW) {
+        for (int tile = t0 + warp; tile < t1; tile += NW) {
             // bf16 rows: a running sum for each block of a chunk, eight in all. With a single one the rounding of k / 64 additions in a row
             // made the results of gate / up less exact than one row's of nvfp4_gemv_m1.cu (relative error against 64 bits, k = 2048 / 4096:
             // 1.5e-7 / 2.1e-7, there 1.3e-7 / 1.4e-7). f32 rows need one: their first plane lies on a grid and its sums hardly round.
@@ -134,11 +125,8 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
 #pragma unroll
             for (int i = 0; i < NA; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
             for (int ch = 0; ch < nch; ch++) {
-                if (!mbar_wait(&full[s], par)) {
-                    cn_dev_fail(CN_DEV_WAIT_FULL);
-                    ok = false;
-                    break;
-                }
+                piece_wait(D - 1);
+                __syncwarp();  // the other lanes' copies, too
                 const int nb = min(CB, bpr - ch * CB);
                 const uint8_t *cbase = rbase + s * CHUNK, *xc = xa + ch * (CB * 128), *xic = xi0 + ch * (CB * 32);
                 auto block = [&](int b) {
@@ -160,10 +148,9 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
                     for (int b = 0; b < nb; b++) block(b);
                 }
                 __syncwarp();  // every lane has read the stage
-                if (++done + D <= total) issue();
-                if (++s == D) s = 0, par ^= 1u;
+                issue();
+                if (++s == D) s = 0;
             }
-            if (!ok) break;
 #pragma unroll
             for (int n = NA / 2; n > 0; n /= 2)
 #pragma unroll
@@ -200,13 +187,13 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
                 }
             }
         }
-        if (__syncthreads_or(!ok)) return;  // also: every warp has read this group's rows
+        __syncthreads();  // every warp has read this group's rows
     }
 }
 
 bool layout(const RowsCall& a, int cps, RowsParams& p, size_t& smem) {
     const int bpr = a.k / 64, cols = 8;
-    p.inv_off = HDR;
+    p.inv_off = 0;
     p.x_off = (p.inv_off + (uint32_t)(bpr * 32) + 127u) & ~127u;
     p.ring_off = p.x_off + (uint32_t)((a.x_f32 ? 6 : cols) * bpr * 128);
     const long long room = (227 * 1024) / cps - 1024 - (long long)p.ring_off;
