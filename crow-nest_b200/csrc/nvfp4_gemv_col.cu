@@ -20,8 +20,8 @@
 // warp idles at a part's ragged end, warp 9 adds the eight sums of a part and stores. Clusters of two or four CTAs share a
 // tile by parts where that fills the machine better; the others hand a part's sums to the first CTA through distributed
 // shared memory.
-// What bounds it: issue slots (245 warp instructions per unit of a one-row gate/up in all, 88 of them the decode and its scaling; 0.56 of
-// the slots used there, 0.51 in the down projection). The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
+// What bounds it: the ALU and issue slots (a unit's decode and scaling are 88 warp instructions of half rate), at 0.56 of the slots in gate/up of
+// one row. The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
 #include "common.cuh"
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"
@@ -404,10 +404,15 @@ int cn_gemv_col_launch(const GemvCall& a, cudaStream_t stream, const char* who) 
         const int n = part_start(i + 1, p.lg, bpr) - part_start(i, p.lg, bpr);
         pmax = n > pmax ? n : pmax;
     }
-    const int nch = (pmax + 31) / 32;
-    p.tx = ((pmax + nch - 1) / nch + 3) & ~3;
-    p.pitch = p.tx * 36 + ((p.tx / 4) % 2 == 0 ? 16 : 0);  // an odd number of 16-byte units: the eight rows of a load on distinct banks
-    const long long stage_bytes = (long long)ROWS * p.pitch;
+    // a part in as few equal chunks as have `most` blocks or fewer
+    long long stage_bytes = 0;
+    auto chunks_of = [&](int most) {
+        const int nch = (pmax + most - 1) / most;
+        p.tx = ((pmax + nch - 1) / nch + 3) & ~3;
+        p.pitch = p.tx * 36 + ((p.tx / 4) % 2 == 0 ? 16 : 0);  // an odd number of 16-byte units: the eight rows of a load on distinct banks
+        stage_bytes = (long long)ROWS * p.pitch;
+    };
+    chunks_of(32);
     auto layout = [&](int ks, ColParams& q) {  // returns the shared memory in front of the ring for clusters of ks
         int bmax = 0;
         for (int r = 0; r < ks; r++) {
@@ -448,6 +453,12 @@ int cn_gemv_col_launch(const GemvCall& a, cudaStream_t stream, const char* who) 
         const int rc = cn_gemv_col_launch(lo, stream, who);
         return rc ? rc : cn_gemv_col_launch(hi, stream, who);
     }
+    // Longer chunks, up to a whole part, where three stages of them fit as well: a chunk's wait and release cost every warp some forty
+    // instructions for the one to three units that it has there. FFN 5120 - 17408, one row: 59.1 us with chunks of 20 and 24 blocks, 51.4 of 40
+    // and 36; 162853 x 3584, eight rows: 306 and 251.
+    const int tx32 = p.tx;
+    chunks_of(72);
+    while (p.tx > tx32 && (227 * 1024) / cps - 1024 - layout(ks, p) < 3 * stage_bytes) chunks_of(p.tx - 4);
     p.ks = ks;
     const long long front = layout(ks, p);
     const int clusters = 148 * cps / ks, grid = ks * (ntiles < clusters ? ntiles : clusters);
