@@ -18,20 +18,13 @@ __device__ __forceinline__ float2 lds64f(uint32_t a) {
     asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
     return v;
 }
-// Scale byte i of a word (sel = 0x4i4i) as f16x2 of scale x 2^-8, in both halves: an E4M3 byte shifted left by seven is that
-// f16 as it stands, subnormals included. The engine's reading: bit 7 ignored, 0x7F read as 0x7E.
-__device__ __forceinline__ uint32_t scale_f16x2(uint32_t w, uint32_t sel) {
-    const uint32_t b = __byte_perm(w, 0u, sel) & 0x007f007fu;
-    uint32_t r;
-    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(b), "r"(0x007e007eu));
-    return r << 7;
-}
 __device__ __forceinline__ uint32_t hmul2u(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-// Two scale bytes of a word, `shift` = 8 (t >> 1): bytes t >> 1 and 2 + (t >> 1), as f16x2 of scale x 2^-8 (see scale_f16x2).
+// Two scale bytes of a word, `shift` = 8 (t >> 1): bytes t >> 1 and 2 + (t >> 1), as f16x2 of scale x 2^-8: an E4M3 byte shifted left by
+// seven is that f16 as it stands, subnormals included. The engine's reading: bit 7 ignored, 0x7F read as 0x7E.
 __device__ __forceinline__ __half2 lane_scales(uint32_t w, uint32_t shift) {
     uint32_t r = (w >> shift) & 0x007f007fu;
     asm("min.u16x2 %0, %0, %1;" : "+r"(r) : "r"(0x007e007eu));
@@ -42,8 +35,7 @@ __device__ __forceinline__ __half2 lane_scales(uint32_t w, uint32_t shift) {
 // A and B agree: lane (g, t) takes code words t and t + 4 of rows g (pa, the block's start + 4 t) and g + 8 (pb) - one 32-bit load of
 // eight codes feeds half of two MMAs - and x(ps, half) gives the matching eight activations of column g of group ps. A word's
 // eight values share a scale, so the two words' scales are made in one register (four instructions) and the multiplies take its halves:
-// 184 cycles per 16 x 128 values and scheduler against 218 with one scale at a time (127 and 145 instructions; nvfp4_gemv_col.cu, which
-// something else bounds, gained nothing by it: 59.2 us for an FFN of 5120 - 17408 before, 61.3 with it).
+// 184 cycles per 16 x 128 values and scheduler against 218 with one scale at a time (127 and 145 instructions).
 template <int NP, typename X>
 __device__ __forceinline__ void block_mma(float (&cc)[NP][4], const uint8_t* pa, const uint8_t* pb, int t, X x) {
     const __half2 sa = lane_scales(*(const uint32_t*)(pa - 4 * t), 8u * (t >> 1)), sb = lane_scales(*(const uint32_t*)(pb - 4 * t), 8u * (t >> 1));
@@ -77,7 +69,7 @@ __device__ __forceinline__ float gs_pow2(float gs) {
 // Eight f32 values of a 64-value block, eight consecutive lanes (lane & 24 the same) holding the block: the block's power-of-two
 // scale, and three f16 planes: the value on the block's own grid of 2^5 (values below 2^15 after scaling), then what is left as
 // f16, twice. An infinity or a NaN goes into the first plane and leaves nothing. Returns the inverse scale, times the 2^8 that
-// scale_f16x2 leaves out.
+// lane_scales leaves out.
 __device__ __forceinline__ float f32_planes(const uint4& lo, const uint4& hi, int lane, uint32_t h[3][4]) {
     const uint32_t u[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     uint32_t e = 0;  // largest exponent of the block's finite values

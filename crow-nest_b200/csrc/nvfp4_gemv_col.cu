@@ -211,7 +211,6 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_col_kernel(const Col
             xa[ps] = base + cp.x_off + (uint32_t)(c * nblk * 128 + (c & 1) * 64 + t * 16);
         }
         const uint32_t xi0 = base + cp.inv_off + 8u * (uint32_t)t;
-        const uint32_t sel0 = (t >> 1) ? 0x4141u : 0x4040u, sel1 = sel0 + 0x0202u;
         int s = 0, rs = 0, dealt = 0;
         uint32_t par = 0, rpar = 1;
         bool ok = true;
@@ -237,7 +236,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_col_kernel(const Col
 #pragma unroll
                         for (int bl = 0; bl < 2; bl++) {
                             const uint32_t pw = pa + 36u * bl, pw8 = pw + 8u * (uint32_t)pitch;
-                            const uint32_t sa = lds32(pw - 4u * t), sb = lds32(pw8 - 4u * t);
+                            const __half2 sa = lane_scales(lds32(pw - 4u * t), 8u * (t >> 1)), sb = lane_scales(lds32(pw8 - 4u * t), 8u * (t >> 1));
                             float cc[NP][4];
 #pragma unroll
                             for (int ps = 0; ps < NP; ps++) cc[ps][0] = cc[ps][1] = cc[ps][2] = cc[ps][3] = 0.0f;
@@ -246,7 +245,8 @@ __global__ void __launch_bounds__(NTHREADS, CPS) nvfp4_gemv_col_kernel(const Col
                                 uint32_t ha[4], hb[4];
                                 e2m1x8_to_f16x2(lds32(pw + 4u + 16u * hf), ha);
                                 e2m1x8_to_f16x2(lds32(pw8 + 4u + 16u * hf), hb);
-                                const uint32_t fa = scale_f16x2(sa, hf ? sel1 : sel0), fb = scale_f16x2(sb, hf ? sel1 : sel0);
+                                const __half2 fha = hf ? __high2half2(sa) : __low2half2(sa), fhb = hf ? __high2half2(sb) : __low2half2(sb);
+                                const uint32_t fa = *(const uint32_t*)&fha, fb = *(const uint32_t*)&fhb;
 #pragma unroll
                                 for (int i = 0; i < 4; i++) ha[i] = hmul2u(ha[i], fa), hb[i] = hmul2u(hb[i], fb);
 #pragma unroll
