@@ -17,8 +17,10 @@ constexpr int PREP_THREADS = 256, PREP_KEEP = 4;
 template <int XT>
 __global__ void __launch_bounds__(PREP_THREADS) gemm_prep_x_kernel(const void* __restrict__ x, uint16_t* __restrict__ xh, float* __restrict__ rs, int k) {
     __shared__ float amax_w[PREP_THREADS / 32];
-    pdl_launch_dependents();
     pdl_wait();  // the activations may come from the kernel before this one, and one before it may still read what this one overwrites
+    // Only now: the GEMM reads weights and the tensor scale without waiting for this kernel, so whatever wrote them must be complete by the time
+    // it starts.
+    pdl_launch_dependents();
     const size_t row = blockIdx.x;
     const int n = k >> 3;
     constexpr int NV = XT == 1 ? 1 : 2;

@@ -226,8 +226,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             }
         }
     } else if (warp == 0) {
-        // ------------------------------------------------------------ f16 rows: weights in. They depend on no earlier kernel, so they start
-        // while the one that prepares the activations still runs.
+        // ------------------------------------------------------------ f16 rows: weights in, while the kernel that prepares the activations still
+        // runs. That one has waited for everything before it when it lets this one start, so weights and tensor scale are complete, also where the
+        // kernel in front of the call wrote them.
         if (lane == 0) {
             if (!PACKED) tma_prefetch_map(&wmap);
             int ws = 0;
