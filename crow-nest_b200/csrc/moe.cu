@@ -300,6 +300,13 @@ extern "C" int cn_moe_nvfp4_plan_destroy(void* plan) {
 
 namespace {
 
+// a shared expert takes all of its matrices and scales, and a plan that was made for one; checked before anything is enqueued
+int check_shared(const MoePlan* p, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs, const char* who) {
+    if (!shared_gate || !shared_up || !shared_down || !shared_gs) CN_FAIL(CN_ERR_SHAPE, "%s: null matrix or scales of the shared expert", who);
+    if (p->shared_inter <= 0) CN_FAIL(CN_ERR_SHAPE, "%s: the plan was made without a shared expert", who);
+    return CN_OK;
+}
+
 // the shared expert on every token, up to 8 rows per pass, on the plan's side stream between the fork and join events:
 // whatever happens after the fork, the side stream is joined again (a capture of the caller's stream stays valid)
 int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs, const void* x,
@@ -425,7 +432,8 @@ extern "C" int cn_moe_nvfp4_experts(void* plan, const unsigned long long* table_
 extern "C" int cn_moe_nvfp4_shared_begin(void* plan, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs,
                                          const void* x, int tokens, float limit, int dtype, cn_stream_t stream) {
     MoePlan* p = (MoePlan*)plan;
-    if (!p || !shared_gate || !shared_up || !shared_down || !shared_gs) CN_FAIL(CN_ERR_SHAPE, "cn_moe_nvfp4_shared_begin: null argument");
+    if (!p) CN_FAIL(CN_ERR_SHAPE, "cn_moe_nvfp4_shared_begin: null plan");
+    if (int rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_shared_begin")) return rc;
     if (tokens < 1 || tokens > p->max_tokens) CN_FAIL(CN_ERR_LIMIT, "cn_moe_nvfp4_shared_begin: %d tokens, the plan holds %d", tokens, p->max_tokens);
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_moe_nvfp4_shared_begin: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     const int rc = shared_branch(p, shared_gate, shared_up, shared_down, shared_gs, x, tokens, limit, dtype, (cudaStream_t)stream);
@@ -448,6 +456,7 @@ extern "C" int cn_moe_nvfp4_finish(void* plan, const void* shared_gate, const vo
         CN_CUDA(cudaStreamWaitEvent(stream, p->join, 0));
         shared = p->ys;
     } else if (shared_gate) {
+        if ((rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_finish"))) return rc;
         rc = shared_branch(p, shared_gate, shared_up, shared_down, shared_gs, x, tokens, limit, dtype, stream);
         CN_CUDA(cudaStreamWaitEvent(stream, p->join, 0));
         shared = p->ys;
@@ -470,11 +479,12 @@ extern "C" int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, 
     if (dtype == CN_BF16_IN_F32_OUT) dtype = CN_BF16;
     const float* shared = nullptr;
     int rc = CN_OK;
+    if (shared_gate && (rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_run"))) return rc;
     if (tokens * p->topk < GROUP_COMBOS) {
         // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine.
         MoeDownCall d = {};
         d.ids = ids, d.wts = wts, d.table = table_dn, d.experts = p->experts, d.topk = p->topk, d.h = p->h, d.gs = gs_dn, d.inter = p->inter;
-        d.shared = shared_gate ? shared_down : nullptr, d.hs = p->hs, d.shared_gs = shared_gs ? shared_gs + 2 : nullptr, d.sgate = sgate;
+        d.shared = shared_gate ? shared_down : nullptr, d.hs = p->hs, d.shared_gs = shared_gate ? shared_gs + 2 : nullptr, d.sgate = sgate;
         d.shared_inter = p->shared_inter, d.y = y, d.tokens = tokens, d.hidden = p->hidden, d.out_bf16 = ydtype == CN_BF16;
         if (cn_moe_down_combine_fits(d)) {
             GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, tokens * p->topk, p->topk, limit, dtype);

@@ -163,7 +163,7 @@ int units_of(const MoeDownCall& c) { return c.topk * ((c.inter / 64 + CB - 1) / 
 }  // namespace
 
 bool cn_moe_down_combine_fits(const MoeDownCall& c) {
-    return c.inter % 256 == 0 && (!c.shared || c.shared_inter % 256 == 0) && units_of(c) <= MAX_UNITS && c.topk <= MAX_PICKS && c.tokens <= 65535 &&
+    return c.inter % 256 == 0 && (!c.shared || (c.shared_inter > 0 && c.shared_inter % 256 == 0)) && units_of(c) <= MAX_UNITS && c.topk <= MAX_PICKS && c.tokens <= 65535 &&
            !(((uintptr_t)c.shared | (uintptr_t)c.h | (uintptr_t)c.hs) & 15);
 }
 

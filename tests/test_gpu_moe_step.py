@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from crownest_b200 import device_status, moe, ops, synth
+from crownest_b200 import CrownestError, device_status, moe, ops, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -68,4 +68,35 @@ def test_small_steps_against_64_bits(hidden, inter, topk, tokens, shared, dtype)
     rms = want.pow(2).mean(dim=1, keepdim=True).sqrt()
     assert ((y.double() - want).abs() <= (2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-5 * rms).all()
     assert (y.double() - want).norm() <= (2e-6 if y.dtype == torch.float32 else 2.0 ** -8) * want.norm()
+    assert device_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [1, 64])
+def test_a_shared_expert_that_the_plan_has_no_room_for_is_refused(tokens):
+    """Steps of both sizes: a plan made without a shared expert, and a shared expert without its scales or one of its matrices."""
+    hidden, inter, experts, topk = 256, 256, 8, 4
+    rng = np.random.default_rng(tokens)
+
+    def matrix(rows, k):
+        return torch.from_numpy(synth.nvfp4_matrix(rows, k, rng)).cuda()
+
+    w = moe.GpuMoeWeights(hidden, inter, experts, 1.0, 1.0, gate_up=[matrix(2 * inter, hidden) for _ in range(experts)],
+                          down=[matrix(hidden, inter) for _ in range(experts)], shared=[matrix(inter, hidden), matrix(inter, hidden), matrix(hidden, inter)],
+                          shared_gs=[1.0, 1.0, 1.0], device="cuda")
+    x = torch.zeros((tokens, hidden), device="cuda")
+    ids = torch.arange(topk, device="cuda", dtype=torch.int32).repeat(tokens, 1)
+    wts = torch.ones((tokens, topk), device="cuda")
+    eo = torch.zeros((tokens * topk, hidden), device="cuda")
+    bare = moe.GpuMoePlan(hidden, inter, experts, topk, tokens)
+    for call in (lambda p: p.experts_run(w, ids, wts, x), lambda p: p.shared_begin(w, x), lambda p: p.finish(w, ids, wts, x, eo)):
+        with pytest.raises(CrownestError, match="without a shared expert"):
+            call(bare)
+    whole = moe.GpuMoePlan(hidden, inter, experts, topk, tokens, shared_inter=inter)
+    matrices, scales = w.shared, w.shared_gs
+    for w.shared, w.shared_gs in ((matrices, None), (matrices[:2] + [None], scales), ([matrices[0], None, matrices[2]], scales)):
+        for call in (lambda p: p.experts_run(w, ids, wts, x), lambda p: p.shared_begin(w, x), lambda p: p.finish(w, ids, wts, x, eo)):
+            with pytest.raises(CrownestError, match="null matrix or scales"):
+                call(whole)
+    w.shared, w.shared_gs = matrices, scales
+    assert not whole.experts_run(w, ids, wts, x).any()
     assert device_status() == 0
