@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) fp8_gemv_tc_kernel(const Fp8Par
 #pragma unroll
             for (int u = 0; u < PF; u++) {
                 const int task = t0 + u * NW * 32;
-                if (task >= ntask) break;  // uniform over every 16-lane group: ntask is a multiple of 16
+                if (task >= ntask) break;  // uniform over each half of a warp, not over the warp: ntask is an odd multiple of 16 with an odd number of blocks
                 const int mrow = task / (nkb * 16), rem = task - mrow * nkb * 16;
                 float v[8];
                 if (p.x_bf16) {
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(NTHREADS, CPS) fp8_gemv_tc_kernel(const Fp8Par
 #pragma unroll
                 for (int q = 0; q < 8; q++) amax = fmaxf(amax, fabsf(v[q]));
 #pragma unroll
-                for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffu << (lane & 16), amax, o));
                 uint32_t e = (__float_as_uint(amax) >> 23) & 0xFF;
                 float mul = 1.0f, inv = 1.0f;
                 if (amax > 0.0f && e < 255) {

@@ -30,6 +30,22 @@ def test_fp8_gemv_bf16_matches_the_cpu_reference(rows, cols, m):
     check_close(from_dev_bf16(y), ref, f"fp8 [{rows},{cols}] m={m}", ulp_floor=1.0 / 256)
 
 
+@pytest.mark.parametrize("rows,cols", [(786, 4992), (40, 1152), (129, 17280)])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_odd_numbers_of_column_blocks(rows, cols, m, dtype):
+    """39, 9 and 135 blocks of 128 columns: with an odd number of rows the staging of the activations ends in the middle of a warp."""
+    rng, q, s = make(rows, cols, rows + m)
+    xb, xf = synth.activations(m, cols, rng)
+    ref = oracle.fp8_gemv(q, rows, cols, s, xf)
+    x = to_dev_bf16(xb) if dtype == "bf16" else torch.from_numpy(xf).cuda()
+    y = ops.fp8_gemv(torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda(), x, rows, cols)
+    if dtype == "bf16":
+        check_close(from_dev_bf16(y), ref, f"fp8 [{rows},{cols}] m={m}", ulp_floor=1.0 / 256)
+    else:  # bf16 values in f32 rows are exact in f16: only the order of the f32 sums differs
+        check_close(y.cpu().numpy(), ref, f"fp8 f32 [{rows},{cols}] m={m}", bf16_out=False)
+
+
 def test_fp8_gemv_f32_and_row_invariance():
     rows, cols = 700, 1024
     rng, q, s = make(rows, cols, 3)
