@@ -3,8 +3,9 @@
 //
 // Arithmetic. A = w * s: an E2M1 code times a UE4M3 scale has at most 5 significant bits, so the product is exact in f16 and in bf16.
 // B: bf16 rows as they are beyond 128 of them; else x * 2^k as f16 with one power of two per activation row (row amax brought to
-// [2^13, 2^14)): exact for bf16 input down to 2^-27 of the row maximum. Products are exact in the tensor core, accumulation is f32 in
-// tensor memory, the epilogue multiplies by gs * 2^-k once.
+// [2^13, 2^14) where f32 has that power of two, k <= 127): exact for bf16 input down to 2^-27 of the row maximum. Products are exact in the
+// tensor core, accumulation is f32 in tensor memory, the epilogue multiplies by gs, then by 2^-k (which may be a subnormal f32: the two
+// are not multiplied with one another first).
 #include "common.cuh"
 #include "nvfp4_gemm.cuh"
 
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(PREP_THREADS) gemm_prep_x_kernel(const void* _
         float v[8];
         widen(r, v);
 #pragma unroll
-        for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
+        for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]) < INFINITY ? fabsf(v[j]) : 0.0f);
     };
     uint4 kept[PREP_KEEP][NV];
 #pragma unroll
@@ -65,13 +66,11 @@ __global__ void __launch_bounds__(PREP_THREADS) gemm_prep_x_kernel(const void* _
     amax = 0.0f;
 #pragma unroll
     for (int w = 0; w < PREP_THREADS / 32; w++) amax = fmaxf(amax, amax_w[w]);
-    // amax * mul in [2^13, 2^14): two binades under the largest f16; zero, NaN and infinite rows are left unscaled
-    uint32_t e = (__float_as_uint(amax) >> 23) & 0xFF;
-    float mul = 1.0f, inv = 1.0f;
-    if (amax > 0.0f && e < 255 && e > 14 && e < 240) {
-        mul = __uint_as_float((127u + 13u + 127u - e) << 23);
-        inv = __uint_as_float((e - 13u) << 23);
-    }
+    // The largest finite value * mul in [2^13, 2^14), two binades under the largest f16; rows below 2^-114 get the largest power of two there is,
+    // 2^127, which leaves bf16 values of any size exact (2^-133 * 2^127 = 2^-6). Infinities and NaN stay what they are.
+    const uint32_t e = max((__float_as_uint(amax) >> 23) & 0xFFu, 13u);
+    const float mul = __uint_as_float((127u + 13u + 127u - e) << 23);
+    const float inv = e == 13u ? 0x1p-127f : __uint_as_float((e - 13u) << 23);
     auto store = [&](int i, const uint4 r[NV]) {
         float v[8];
         widen(r, v);

@@ -377,7 +377,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                         if (BF16)
                             a *= gs, b *= gs;
                         else
-                            a *= gs * p.rs[min(tok0 + c0 + i, p.m - 1)], b *= gs * p.rs[min(tok0 + c0 + i + 1, p.m - 1)];
+                            a = a * gs * p.rs[min(tok0 + c0 + i, p.m - 1)], b = b * gs * p.rs[min(tok0 + c0 + i + 1, p.m - 1)];
                         const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
                         const __nv_bfloat162 o = __floats2bfloat162_rn(odd ? other : a, odd ? b : other);
                         if (whole || (c0 + i + odd < live && row < p.rows)) *(__nv_bfloat162*)yp = o;
@@ -388,7 +388,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                     for (int i = 0; i < 32; i++) {
                         const int tok = tok0 + c0 + i;
                         if (c0 + i < live && row < p.rows) {
-                            const float r = __uint_as_float(v[i]) * (BF16 ? gs : gs * p.rs[tok]);
+                            const float r = BF16 ? __uint_as_float(v[i]) * gs : __uint_as_float(v[i]) * gs * p.rs[tok];
                             if (p.out_bf16)
                                 ((__nv_bfloat16*)p.y)[(size_t)tok * p.ldy + row] = __float2bfloat16_rn(r);
                             else
@@ -459,9 +459,9 @@ __global__ void gemm_splitk_reduce_kernel(const float* __restrict__ part, const 
 #pragma unroll
         for (int i = 0; i < V; i++) v[i] += a[i];
     }
-    const float c = gs[0] * f * (rs ? rs[t] : 1.0f);
+    const float c = gs[0] * f, r = rs ? rs[t] : 1.0f;
 #pragma unroll
-    for (int i = 0; i < V; i++) v[i] *= c;
+    for (int i = 0; i < V; i++) v[i] = v[i] * c * r;
     if (out_bf16) {
         __nv_bfloat16* o = (__nv_bfloat16*)y + (size_t)t * ldy + n;
         if constexpr (V == 4) {

@@ -98,3 +98,41 @@ def test_few_rows_split_k_and_relaid_weights(rows, k, m, relaid):
     run(x, wide[:, :rows])
     assert torch.equal(wide[:, :rows], y) and not wide[:, rows:].any()
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 60, 128])
+@pytest.mark.parametrize("form", ["container", "relaid", "f32"])
+@pytest.mark.parametrize("rows", [384, 4000])
+def test_rows_of_any_magnitude_as_f16(m, form, rows):
+    """Rows that are brought into f16 by a power of two each: from subnormal bf16 to the largest finite values, with one part of k and several; an
+    infinity or a NaN reaches the results of its own row and leaves the finite terms beside it alone."""
+    k = 2048
+    rng = np.random.default_rng(m + rows)
+    data, unit = synth.nvfp4_matrix(rows, k, rng), np.clip(rng.standard_normal((m, k)), -3.0, 3.0)
+    for gs, scales in ((2.0 ** 60, [3e-40, 1e-38, 1e-36, 2e-34, 7e-34, 1e-33, 1e-20, 1.0]), (2.0 ** -60, [1.1e38, 1e38, 2e34, 3e30, 1.0])):
+        fw = ops.Fp4.from_host(data, rows, k, np.float32(gs))
+        w = ops.Fp4Packed(fw) if form == "relaid" else fw
+        x = torch.from_numpy(unit * np.array([scales[i % len(scales)] for i in range(m)])[:, None]).cuda().to(torch.float32)
+        x = x if form == "f32" else x.to(torch.bfloat16)
+        y = (ops.launch_gemm_fp4 if form == "relaid" else ops.launch_gemm)(w, x)
+        want = x.double() @ ops.dequant(fw, rule=True).double().view(rows, k).t()
+        err = (y.double() - want).norm(dim=1) / want.norm(dim=1)
+        # bf16: one rounding of the result (2^-9 at most) beside f32 sums; f32 rows: one rounding of every value to f16 (2^-12 in the mean square at most),
+        # the smallest of them to a subnormal f16 (3e-40 becomes 2^-4, which f16 holds in steps of 2^-24)
+        assert err.max().item() <= (2.0 ** -11 if form == "f32" else 2.0 ** -9 + 4e-6)
+    fw = ops.Fp4.from_host(data, rows, k, np.float32(1.0))
+    w = ops.Fp4Packed(fw) if form == "relaid" else fw
+    x = torch.from_numpy(np.abs(unit) * 1e10).cuda().to(torch.float32 if form == "f32" else torch.bfloat16)
+    special = x.clone()
+    special[0, 7], special[m - 1, 9] = float("inf"), float("inf") if m == 1 else float("nan")
+    run = ops.launch_gemm_fp4 if form == "relaid" else ops.launch_gemm
+    y, plain = run(w, special), run(w, x)
+    col = ops.dequant(fw, rule=True).view(rows, k)
+    hit = (torch.where(col[:, 7] != 0, col[:, 7].sign() * float("inf"), float("nan")) if m > 1 else
+           torch.where((col[:, 7] != 0) & (col[:, 9] != 0) & (col[:, 7].sign() == col[:, 9].sign()), col[:, 7].sign() * float("inf"), float("nan")))
+    assert torch.equal(y[0].float().nan_to_num(nan=-7.0), hit.to(y.dtype).float().nan_to_num(nan=-7.0))
+    if m > 1:
+        assert y[m - 1].isnan().all()
+    if m > 2:
+        assert torch.equal(y[1:m - 1], plain[1:m - 1])
+    assert device_status() == 0
