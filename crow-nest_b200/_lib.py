@@ -83,6 +83,7 @@ _SIGS = {
     "cn_ep_return": [C.POINTER(C.c_void_p), _i, _i, _i, _i, C.c_size_t, C.c_size_t, C.c_size_t, C.c_size_t, _vp, _vp, _vp, _vp],
     "cn_nvfp4_gemm": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, C.c_size_t, _vp],
     "cn_nvfp4_gemm_workspace_bytes": [_i, _i],
+    "cn_nvfp4_gemm_workspace_bytes_of": [_i, _i, _i],
     "cn_nvfp4_bs_packed_bytes": [_i, _i],
     "cn_nvfp4_bs_repack": [_vp, _vp, _i, _i, _vp],
     "cn_nvfp4_bs_workspace_bytes": [_i, _i, _i],
@@ -124,7 +125,7 @@ def exported_symbols():
     return sorted(_SIGS)
 
 
-_RESTYPES_INIT = {"cn_nvfp4_gemm_workspace_bytes": C.c_size_t, "cn_ep_flag_bytes": C.c_size_t, "cn_nvfp4_bs_packed_bytes": C.c_size_t,
+_RESTYPES_INIT = {"cn_nvfp4_gemm_workspace_bytes": C.c_size_t, "cn_nvfp4_gemm_workspace_bytes_of": C.c_size_t, "cn_ep_flag_bytes": C.c_size_t, "cn_nvfp4_bs_packed_bytes": C.c_size_t,
                   "cn_nvfp4_bs_workspace_bytes": C.c_size_t}
 
 
@@ -186,7 +187,7 @@ def host():
         loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
         loader.exec_module(mod)
-        names = ("cn_nvfp4_gemv", "cn_nvfp4_gemv_gu", "cn_nvfp4_gemm", "cn_nvfp4_gemm_workspace_bytes", "cn_nvfp4_bs_gemm", "cn_nvfp4_bs_workspace_bytes",
+        names = ("cn_nvfp4_gemv", "cn_nvfp4_gemv_gu", "cn_nvfp4_gemm", "cn_nvfp4_gemm_workspace_bytes_of", "cn_nvfp4_bs_gemm", "cn_nvfp4_bs_workspace_bytes",
                  "cn_fp8_gemv", "cn_lm_head_argmax", "cn_route_softmax_topk", "cn_route_sigmoid_topk")
         mod.bind({n: C.cast(getattr(L, n), C.c_void_p).value for n in names}, _raise_status)
         _host = mod

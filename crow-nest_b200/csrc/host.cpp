@@ -18,7 +18,7 @@ struct Api {
     int (*gemv)(const void*, const void*, const void*, void*, int, int, int, int, int, void*);
     int (*gemv_gu)(const void*, const void*, const void*, const void*, const void*, void*, int, int, int, int, float, int, void*);
     int (*gemm)(const void*, const void*, const void*, void*, int, int, int, int, int, void*, size_t, void*);
-    size_t (*gemm_ws)(int, int);
+    size_t (*gemm_ws)(int, int, int);
     int (*bs_gemm)(const void*, const void*, const void*, void*, int, int, int, int, int, void*, size_t, void*);
     size_t (*bs_ws)(int, int, int);
     int (*fp8)(const void*, const void*, const void*, void*, int, int, int, int, int, void*);
@@ -148,7 +148,7 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const long m = x2.size(0);
         at::Tensor y = a[5] == Py_None ? at::empty({m, rows}, x.options()) : tensor(a[5]);
         at::Tensor ws = a[6] != Py_None ? tensor(a[6])
-                                        : at::empty({(long)(BS ? api.bs_ws(i32(rows), i32(k), i32(m)) : api.gemm_ws(i32(k), i32(m)))}, x.options().dtype(at::kByte));
+                                        : at::empty({(long)(BS ? api.bs_ws : api.gemm_ws)(i32(rows), i32(k), i32(m))}, x.options().dtype(at::kByte));
         const long ld = y.stride(0);
         const int dt = dtype_code(x, a[4]);
         const size_t bytes = (size_t)ws.numel();
@@ -230,7 +230,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     } table[] = {{"cn_nvfp4_gemv", &api.gemv},
                  {"cn_nvfp4_gemv_gu", &api.gemv_gu},
                  {"cn_nvfp4_gemm", &api.gemm},
-                 {"cn_nvfp4_gemm_workspace_bytes", &api.gemm_ws},
+                 {"cn_nvfp4_gemm_workspace_bytes_of", &api.gemm_ws},
                  {"cn_nvfp4_bs_gemm", &api.bs_gemm},
                  {"cn_nvfp4_bs_workspace_bytes", &api.bs_ws},
                  {"cn_fp8_gemv", &api.fp8},

@@ -96,7 +96,21 @@ __global__ void __launch_bounds__(PREP_THREADS) gemm_prep_x_kernel(const void* _
 
 constexpr int MAX_KSPLITS = 8;
 constexpr size_t PART_ROWS = 32768;  // output rows x parts of K that the workspace holds sums of (m <= 128: that many for each of 8 parts)
-constexpr int MAX_SPLIT_M = 512;     // more activation rows fill the machine
+constexpr int MAX_SPLIT_M = 512;     // activation rows up to which K is split
+// f16 activations and row factors, which every call may need
+size_t front_bytes(int k, int m) { return (size_t)m * k * 2 + (((size_t)m * 4 + 255) & ~(size_t)255) + 256; }
+// the raw sums that cn_nvfp4_gemm_workspace_bytes makes room for, whatever the output rows
+size_t sum_bytes(int m) { return m <= 128 ? (size_t)MAX_KSPLITS * m * PART_ROWS * 4 : (m <= MAX_SPLIT_M ? (size_t)m * PART_ROWS * 4 : 0); }
+// More than 128 rows of bf16 go to the tensor cores as they are: their MMAs hide the decode to bf16, which takes twice the instructions
+// of that to f16. Everything else goes as f16 x 2^k per row.
+bool rows_as_f16(int dtype, int m) { return dtype != CN_BF16 || m <= 128; }
+// Parts of K that `bytes` of raw sums allow. Never more than what sum_bytes gives: a larger workspace does not change the order of a sum.
+int splits_allowed(int rows, int m, size_t bytes) {
+    if (m > MAX_SPLIT_M || (size_t)rows > PART_ROWS) return 1;
+    const size_t have = bytes < sum_bytes(m) ? bytes : sum_bytes(m), most = have / ((size_t)m * rows * 4);
+    return most > (size_t)MAX_KSPLITS ? MAX_KSPLITS : (most < 1 ? 1 : (int)most);
+}
+int splits_of(int rows, int k, int m, int dtype, size_t bytes) { return cn_gemm_pair_splits(rows, k, m, rows_as_f16(dtype, m), splits_allowed(rows, m, bytes)); }
 
 }  // namespace
 
@@ -110,9 +124,13 @@ int cn_gemm_prep_x(const void* x, int dtype, uint16_t* xh, float* rs, int k, int
 
 extern "C" size_t cn_nvfp4_gemm_workspace_bytes(int k, int m) {
     if (k <= 0 || m <= 0) return 0;
-    // f16 activations, row factors, and room for the partial sums
-    const size_t part = m <= 128 ? (size_t)MAX_KSPLITS * m * PART_ROWS * 4 : (m <= MAX_SPLIT_M ? (size_t)m * PART_ROWS * 4 : 0);
-    return (size_t)m * k * 2 + (((size_t)m * 4 + 255) & ~(size_t)255) + 256 + part;
+    return front_bytes(k, m) + sum_bytes(m);
+}
+
+extern "C" size_t cn_nvfp4_gemm_workspace_bytes_of(int rows, int k, int m) {
+    if (rows <= 0 || k <= 0 || k % 256 || m <= 0) return 0;
+    const int a = splits_of(rows, k, m, CN_F32, sum_bytes(m)), b = splits_of(rows, k, m, CN_BF16, sum_bytes(m)), s = a > b ? a : b;
+    return front_bytes(k, m) + (s > 1 ? (size_t)s * m * rows * 4 : 0);
 }
 
 extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
@@ -124,21 +142,16 @@ extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_gemm: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     if (((uintptr_t)w & 15) || ((uintptr_t)x & 15) || ((uintptr_t)workspace & 255))
         CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_gemm: weights and activations must be 16-byte aligned, the workspace 256-byte aligned");
-    if (!workspace || workspace_bytes < cn_nvfp4_gemm_workspace_bytes(k, m))
-        CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_gemm: workspace of %zu B, %zu B needed", workspace_bytes, cn_nvfp4_gemm_workspace_bytes(k, m));
+    if (!workspace || workspace_bytes < front_bytes(k, m))
+        CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_gemm: workspace of %zu B, %zu B needed", workspace_bytes, front_bytes(k, m));
     uint16_t* xh = (uint16_t*)workspace;
     float* rs = (float*)((char*)workspace + (((size_t)m * k * 2 + 255) & ~(size_t)255));
     GemmCall c = {};
     c.w = w, c.gs = gs, c.rs = rs, c.y = y, c.rows = rows, c.k = k, c.m = m, c.ldy = ldy, c.out_bf16 = dtype == CN_BF16;
-    // More than 128 rows of bf16 go to the tensor cores as they are: their MMAs hide the decode to bf16, which takes twice the instructions
-    // of that to f16. Everything else goes as f16 x 2^k per row.
-    c.x_f16 = dtype != CN_BF16 || m <= 128;
+    c.x_f16 = rows_as_f16(dtype, m);
     c.x = c.x_f16 ? (const void*)xh : x;
-    if (m <= MAX_SPLIT_M) {
-        c.part = (float*)((char*)rs + (((size_t)m * 4 + 255) & ~(size_t)255));
-        const size_t most = m <= 128 ? (rows <= (int)PART_ROWS ? MAX_KSPLITS : 1) : PART_ROWS / (size_t)rows;
-        c.max_splits = most > (size_t)MAX_KSPLITS ? MAX_KSPLITS : (most < 1 ? 1 : (int)most);
-    }
+    c.max_splits = splits_allowed(rows, m, workspace_bytes - front_bytes(k, m));
+    if (c.max_splits > 1) c.part = (float*)((char*)rs + (((size_t)m * 4 + 255) & ~(size_t)255));
     if (c.x_f16) {
         if (int rc = cn_gemm_prep_x(x, dtype, xh, rs, k, m, stream)) return rc;
     } else {

@@ -494,6 +494,13 @@ int ksplits_for(int rows, int k, int m) {
 bool f16_rows(int m) { return m <= 128; }
 size_t rows_bytes(int k, int m) { return ((size_t)m * k * 2 + 255) & ~(size_t)255; }  // the f16 rows, or a copy of the bf16 ones
 size_t row_factor_bytes(int m) { return ((size_t)m * 4 + 255) & ~(size_t)255; }
+size_t bf16_front_bytes(int k, int m) { return rows_bytes(k, m) + row_factor_bytes(m); }
+// f32 rows: the cascade's images, row factors, and the raw sums of a split K range
+size_t cascade_bytes(int rows, int k, int m) {
+    const size_t ntb = (size_t)(m + TB - 1) / TB;
+    const int ks = ksplits_for(rows, k, m);
+    return ntb * (k / KT) * B_STAGE + ntb * TB * 4 + 256 + (ks > 1 ? (size_t)ks * m * rows * 4 : 0);
+}
 constexpr int MAX_PAIR_SPLITS = 8;
 int pair_splits(int rows, int k, int m) { return m <= 512 ? cn_gemm_pair_splits(rows, k, m, f16_rows(m), MAX_PAIR_SPLITS) : 1; }
 
@@ -515,11 +522,8 @@ extern "C" int cn_nvfp4_bs_repack(const void* w, void* packed, int rows, int k, 
 
 extern "C" size_t cn_nvfp4_bs_workspace_bytes(int rows, int k, int m) {
     if (rows <= 0 || k <= 0 || k % KT || m <= 0) return 0;
-    const size_t ntb = (size_t)(m + TB - 1) / TB;
-    const int ks = ksplits_for(rows, k, m);
-    const size_t f32 = ntb * (k / KT) * B_STAGE + ntb * TB * 4 + 256 + (ks > 1 ? (size_t)ks * m * rows * 4 : 0);
     const int ps = pair_splits(rows, k, m);
-    const size_t bf16 = rows_bytes(k, m) + row_factor_bytes(m) + (ps > 1 ? (size_t)ps * m * rows * 4 : 0);
+    const size_t f32 = cascade_bytes(rows, k, m), bf16 = bf16_front_bytes(k, m) + (ps > 1 ? (size_t)ps * m * rows * 4 : 0);
     return f32 > bf16 ? f32 : bf16;
 }
 
@@ -530,8 +534,9 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
     if (m < 1) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: m = %d", m);
     if (ldy < rows) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: ldy %d < rows %d", ldy, rows);
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: dtype %d is neither CN_F32 nor CN_BF16", dtype);
-    if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < cn_nvfp4_bs_workspace_bytes(rows, k, m))
-        CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_bs_gemm: the workspace must be 256-byte aligned and at least %zu B", cn_nvfp4_bs_workspace_bytes(rows, k, m));
+    const size_t need = dtype == CN_BF16 ? bf16_front_bytes(k, m) : cascade_bytes(rows, k, m);
+    if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < need)
+        CN_FAIL(CN_ERR_LIMIT, "cn_nvfp4_bs_gemm: the workspace must be 256-byte aligned and at least %zu B", need);
     if (((uintptr_t)x & 15)) CN_FAIL(CN_ERR_SHAPE, "cn_nvfp4_bs_gemm: x must be 16-byte aligned");
     if (dtype == CN_BF16) {
         GemmCall c = {};
@@ -546,8 +551,11 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
             CN_CUDA(cudaMemcpyAsync(workspace, x, (size_t)m * k * 2, cudaMemcpyDeviceToDevice, stream));
             c.x = workspace;
         }
-        c.max_splits = pair_splits(rows, k, m);
-        if (c.max_splits > 1) c.part = (float*)((char*)workspace + rows_bytes(k, m) + row_factor_bytes(m));
+        // as many parts of K as the workspace has room for sums of
+        const int most = pair_splits(rows, k, m);
+        const size_t room = (workspace_bytes - need) / ((size_t)m * rows * 4);
+        c.max_splits = room < (size_t)most ? (int)room : most;
+        if (c.max_splits > 1) c.part = (float*)((char*)workspace + need);
         return cn_gemm_pair_launch(c, stream);
     }
     const int ntb = (m + TB - 1) / TB, kts = k / KT;

@@ -58,12 +58,14 @@ def launch_gemv(w: Fp4, x, y=None, ldy=None):
 def launch_gemm(w: Fp4, x, y=None, workspace=None):
     """Y[t][n] = gs * sum_k X[t][k] W[n][k] for any number of rows t - the prompt GEMM (launch_mma_d,
     engine/src/gen.rs:2491; glm5_gemm_fp4_tc, engine/src/kernels_glm5_moe.cu:349) on tcgen05 tensor cores.
-    ``workspace``: a uint8 device tensor of at least ``gemm_workspace_bytes(w.cols, t)`` bytes (allocated when absent)."""
+    ``workspace``: a uint8 device tensor of ``gemm_workspace_bytes(w.cols, t)`` bytes, or ``gemm_workspace_bytes(w.cols, t, w.rows)`` for this
+    matrix alone (allocated when absent)."""
     return host().gemm(w.w, w.gs, w.rows, w.cols, x, y, workspace)
 
 
-def gemm_workspace_bytes(k, m):
-    return int(lib().cn_nvfp4_gemm_workspace_bytes(k, m))
+def gemm_workspace_bytes(k, m, rows=None):
+    """Workspace of `launch_gemm` for m rows: enough for any matrix of k columns, or what a matrix of `rows` rows takes."""
+    return int(lib().cn_nvfp4_gemm_workspace_bytes(k, m) if rows is None else lib().cn_nvfp4_gemm_workspace_bytes_of(rows, k, m))
 
 
 class Fp4Packed:

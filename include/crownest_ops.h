@@ -209,9 +209,13 @@ int cn_moe_nvfp4_finish(void* plan, const void* shared_gate, const void* shared_
  * arithmetic: weights widened losslessly (code x block scale), exact products, f32 accumulation. Up to 128 rows, and f32 rows always,
  * the activations go in as f16 x 2^k per row; more than 128 rows of bf16 as they are, without a pass over them. w is the container
  * layout, unchanged. y may overlap x (bf16 rows beyond 128 are copied to the workspace first then). The call allocates nothing:
- * `workspace` (device, 256-byte aligned) holds the widened activations and must be at least
- * cn_nvfp4_gemm_workspace_bytes(k, m) bytes; it may be reused by the next call on the same stream. */
+ * `workspace` (device, 256-byte aligned) holds the f16 activations and, where k is split over the machine (up to 512 rows), the partial
+ * sums of its parts; it may be reused by the next call on the same stream. cn_nvfp4_gemm_workspace_bytes gives what is enough for any
+ * number of output rows, cn_nvfp4_gemm_workspace_bytes_of what a matrix of `rows` rows takes; both give the same results. Less is
+ * accepted, down to the activations and their factors (m * k * 2 + m * 4 rounded up to 256 + 256 bytes): k is then split into as many
+ * parts as there is room for. */
 size_t cn_nvfp4_gemm_workspace_bytes(int k, int m);
+size_t cn_nvfp4_gemm_workspace_bytes_of(int rows, int k, int m);
 int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
                   size_t workspace_bytes, cn_stream_t stream);
 

@@ -8,7 +8,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import oracle
-from crownest_b200 import device_status, ops, synth
+from crownest_b200 import CrownestError, device_status, ops, synth
 from test_gpu_nvfp4_gemv import check_close, from_dev_bf16, to_dev_bf16
 
 
@@ -135,4 +135,44 @@ def test_rows_of_any_magnitude_as_f16(m, form, rows):
         assert y[m - 1].isnan().all()
     if m > 2:
         assert torch.equal(y[1:m - 1], plain[1:m - 1])
+    assert device_status() == 0
+
+
+def rows_as_stored(k, m):
+    """Bytes of the activations and their factors, without room for partial sums."""
+    return m * k * 2 + (m * 4 + 255) // 256 * 256 + 256
+
+
+@pytest.mark.parametrize("rows,k,m", [(600, 4096, 64), (1024, 10240, 200), (2048, 8192, 512), (600, 4096, 513), (17408, 512, 300), (40000, 512, 20)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_workspaces_of_every_accepted_size(rows, k, m, dtype):
+    """No room for partial sums, room for two or three parts of k, what the matrix takes, what any matrix takes, and more than that: the last three
+    give the same bits, all of them the product; below the first the call is refused."""
+    rng = np.random.default_rng(rows + m)
+    w = ops.Fp4.from_host(synth.nvfp4_matrix(rows, k, rng), rows, k, np.float32(0.37))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda().to(torch.bfloat16).to(dtype)
+    want = x.double() @ ops.dequant(w, rule=True).double().view(rows, k).t()
+    rms = want.pow(2).mean(dim=1, keepdim=True).sqrt()
+    # bf16: one rounding of the result, at most 2^-8 of the value. The sum in tensor memory: each of the k / 16 steps may cut the running sum by 2^-23 of
+    # itself, which no output's running sum takes beyond six times the row's scale.
+    most = (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + k / 16 * 2.0 ** -23 * 6 * rms
+    least, own, whole = rows_as_stored(k, m), ops.gemm_workspace_bytes(k, m, rows), ops.gemm_workspace_bytes(k, m)
+    assert least <= own <= whole
+    ys = {}
+    for n in (least, least + 4 * m * rows * 2, least + 4 * m * rows * 3 + 60, own, whole, whole + 4 * m * rows * 4):
+        ws = torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda")
+        y = ys[n] = ops.launch_gemm(w, x, workspace=ws)
+        assert ((y.double() - want).abs() <= most).all()
+    assert torch.equal(ys[own], ys[whole]) and torch.equal(ys[whole + 4 * m * rows * 4], ys[whole]) and torch.equal(ops.launch_gemm(w, x), ys[whole])
+    with pytest.raises(CrownestError, match="needed"):
+        ops.launch_gemm(w, x, workspace=torch.empty(least - 1, dtype=torch.uint8, device="cuda"))
+    packed = ops.Fp4Packed(w)
+    full = ops.launch_gemm_fp4(packed, x)
+    if dtype == torch.bfloat16:
+        for n in (least, least + 4 * m * rows * 2):
+            y = ops.launch_gemm_fp4(packed, x, workspace=torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda"))
+            assert ((y.double() - want).abs() <= most).all()
+        assert ((full.double() - want).abs() <= most).all()
+    else:  # five cascade levels: the bound of the block-scaled GEMM's own test
+        assert ((full.double() - want).abs() <= 1e-4 * rms).all()
     assert device_status() == 0
