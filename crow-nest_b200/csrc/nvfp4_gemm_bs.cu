@@ -156,8 +156,7 @@ __global__ void act_cascade_kernel(const void* __restrict__ x, uint8_t* __restri
 // of 5120: 10.5 us under the profiler against 13.1 (row factors, one 2-byte load per value) + 9.2 as two kernels; the GEMM is
 // launched so that its prologue and first weights overlap it (17408 x 5120 at 64 rows: 47 -> 32 us per call).
 constexpr int CQ = 4, CTHREADS = 256;
-template <int XT>
-__global__ void __cluster_dims__(CQ, 1, 1) __launch_bounds__(CTHREADS) bs_cascade_kernel(const void* __restrict__ x, uint8_t* __restrict__ ws,
+__global__ void __cluster_dims__(CQ, 1, 1) __launch_bounds__(CTHREADS) bs_cascade_kernel(const float* __restrict__ x, uint8_t* __restrict__ ws,
                                                                                         float* __restrict__ rs, int k, int m) {
     __shared__ float amax_w[32];
     __shared__ float shares[CQ];
@@ -168,13 +167,7 @@ __global__ void __cluster_dims__(CQ, 1, 1) __launch_bounds__(CTHREADS) bs_cascad
     const bool live = tok < m;
     const int ntask = k / 4, share = (ntask / CQ + CTHREADS - 1) / CTHREADS * CTHREADS;  // a task is four values, a quarter of a sub-block
     const int t0 = rank * share, t1 = min(t0 + share, ntask);
-    auto load4 = [&](int task) -> float4 {
-        if (XT == 1) {
-            const uint2 a = *(const uint2*)((const char*)x + ((size_t)tok * k + (size_t)task * 4) * 2);
-            return make_float4(__uint_as_float(a.x << 16), __uint_as_float(a.x & 0xffff0000u), __uint_as_float(a.y << 16), __uint_as_float(a.y & 0xffff0000u));
-        }
-        return *(const float4*)((const char*)x + ((size_t)tok * k + (size_t)task * 4) * 4);
-    };
+    auto load4 = [&](int task) -> float4 { return *(const float4*)(x + (size_t)tok * k + (size_t)task * 4); };
     float amax = 0.0f;
     if (live) {
         for (int task = t0 + (int)threadIdx.x; task < t1; task += CTHREADS) {
@@ -303,9 +296,9 @@ struct BsParams {
     const uint8_t* xq;  // cascade images
     const float* gs;
     const float* rs;    // [token blocks * TB] the rows' 2^-k
-    void* y;
+    float* y;
     float* part;        // [ksplits][m][rows] raw sums when ksplits > 1
-    int rows, k, m, ldy, out_bf16, ksplits;
+    int rows, k, m, ldy, ksplits;
 };
 
 // grid (row tiles, token blocks / NB, ksplits)
@@ -445,15 +438,10 @@ __global__ void __launch_bounds__(BS_THREADS, 1) nvfp4_gemm_bs_kernel(const BsPa
                 for (int i = 0; i < TB; i++) {
                     const int tok = (tb0 + nb) * TB + i;
                     if (tok < p.m && row < p.rows) {
-                        if (p.ksplits > 1) {
+                        if (p.ksplits > 1)
                             p.part[((size_t)ksi * p.m + tok) * p.rows + row] = acc[i];
-                        } else {
-                            const float r = acc[i] * (gs * p.rs[tok]);
-                            if (p.out_bf16)
-                                ((__nv_bfloat16*)p.y)[(size_t)tok * p.ldy + row] = __float2bfloat16_rn(r);
-                            else
-                                ((float*)p.y)[(size_t)tok * p.ldy + row] = r;
-                        }
+                        else
+                            p.y[(size_t)tok * p.ldy + row] = acc[i] * (gs * p.rs[tok]);
                     }
                 }
             }
@@ -466,16 +454,12 @@ __global__ void __launch_bounds__(BS_THREADS, 1) nvfp4_gemm_bs_kernel(const BsPa
 
 // y[t][n] = (sum over splits, in order, of part[s][t][n]) * gs * rs[t]
 __global__ void bs_splitk_reduce_kernel(const float* __restrict__ part, const float* __restrict__ gs, const float* __restrict__ rs,
-                                        void* __restrict__ y, int rows, int m, int ldy, int ksplits, int out_bf16) {
+                                        float* __restrict__ y, int rows, int m, int ldy, int ksplits) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
     if (n >= rows) return;
     float v = part[(size_t)t * rows + n];
     for (int s = 1; s < ksplits; s++) v += part[((size_t)s * m + t) * rows + n];
-    v *= gs[0] * rs[t];
-    if (out_bf16)
-        ((__nv_bfloat16*)y)[(size_t)t * ldy + n] = __float2bfloat16_rn(v);
-    else
-        ((float*)y)[(size_t)t * ldy + n] = v;
+    y[(size_t)t * ldy + n] = v * (gs[0] * rs[t]);
 }
 
 int ksplits_for(int rows, int k, int m) {
@@ -562,14 +546,10 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
     uint8_t* xq = (uint8_t*)workspace;
     float* rs = (float*)(xq + (size_t)ntb * kts * B_STAGE);
     float* part = rs + (size_t)ntb * TB + 64;
-    const dim3 cgrid((unsigned)CQ * ntb * TB);
-    if (dtype == CN_BF16)
-        bs_cascade_kernel<1><<<cgrid, CTHREADS, 0, stream>>>(x, xq, rs, k, m);
-    else
-        bs_cascade_kernel<0><<<cgrid, CTHREADS, 0, stream>>>(x, xq, rs, k, m);
+    bs_cascade_kernel<<<(unsigned)CQ * ntb * TB, CTHREADS, 0, stream>>>((const float*)x, xq, rs, k, m);
     CN_CUDA(cudaGetLastError());
     BsParams p;
-    p.wp = (const uint8_t*)packed, p.xq = xq, p.gs = gs, p.rs = rs, p.y = y, p.rows = rows, p.k = k, p.m = m, p.ldy = ldy, p.out_bf16 = dtype == CN_BF16;
+    p.wp = (const uint8_t*)packed, p.xq = xq, p.gs = gs, p.rs = rs, p.y = (float*)y, p.rows = rows, p.k = k, p.m = m, p.ldy = ldy;
     p.ksplits = ksplits_for(rows, k, m), p.part = p.ksplits > 1 ? part : nullptr;
     const int rts = (rows + 127) / 128;
     if (ntb >= 2) {
@@ -581,7 +561,7 @@ extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void*
     }
     CN_CUDA(cudaGetLastError());
     if (p.ksplits > 1) {
-        bs_splitk_reduce_kernel<<<dim3((rows + 255) / 256, m), 256, 0, stream>>>(part, gs, rs, y, rows, m, ldy, p.ksplits, p.out_bf16);
+        bs_splitk_reduce_kernel<<<dim3((rows + 255) / 256, m), 256, 0, stream>>>(part, gs, rs, p.y, rows, m, ldy, p.ksplits);
         CN_CUDA(cudaGetLastError());
     }
     return CN_OK;
