@@ -346,6 +346,11 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
 
 // Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
 constexpr int GROUP_COMBOS = 48;
+// ... and from which the ungrouped down projection keeps a warp to a tile (measured: see routed_experts).
+constexpr int ROWS_COMBOS = 16;
+// Units of work (16 result rows of a token x eight 64-value blocks of an expert) up to which a step of that many combos runs in two launches
+// (measured: see cn_moe_nvfp4_run).
+constexpr long long STEP_UNITS = 8192;
 
 // Routed gate|up of the combos as they come (nearly every CTA of a small step is resident at once and L2 serves an expert's second
 // reader).
@@ -407,7 +412,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     RowsCall one = {};
     one.ids = ids, one.m = combos, one.tab0 = table_dn, one.gs0 = gs_dn, one.x = p->h, one.x_div = 1, one.x_f32 = 1, one.y = eo, one.yptrs = eo_ptrs;
     one.ldy = p->hidden, one.rows = p->hidden, one.k = p->inter, one.max_groups = combos, one.experts = p->experts;
-    if (combos >= 16 && cn_rows_fits(one)) return cn_rows_launch(one, stream, "cn_moe_nvfp4 (down)");
+    if (combos >= ROWS_COMBOS && cn_rows_fits(one)) return cn_rows_launch(one, stream, "cn_moe_nvfp4 (down)");
     GemvCall d = {};
     d.gs0 = gs_dn, d.x = p->h, d.y = eo, d.yptrs = eo_ptrs, d.rows = p->hidden, d.k = p->inter, d.m = 1, d.ldy = p->hidden, d.dtype = CN_F32, d.out_f32 = 1;
     d.x_f16_ok = 0, d.ids = ids, d.order = nullptr, d.tab0 = table_dn, d.x_div = 1, d.combos = combos, d.experts = p->experts;
@@ -481,12 +486,17 @@ extern "C" int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, 
     int rc = CN_OK;
     if (shared_gate && (rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_run"))) return rc;
     if (tokens * p->topk < GROUP_COMBOS) {
-        // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine.
+        // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine. A warp
+        // of the second waits for each of its units by itself, so from 16 combos on - where the routed kernel below has a warp per tile with two to
+        // four chunks in flight - it is only taken for few units of work. us per step in two launches / with the other kernels (a side stream for
+        // the shared expert), units: 512 experts of 2048 x 512, top 10, 4 tokens 37 / 43 (5.6 k); 64 of 2048 x 1280, top 10, 2 tokens 41 / 45 (7.9 k), 4 tokens
+        // 71 / 65 (15.9 k); 128 of 2560 x 1280, top 6, 3 tokens 49.5 / 48.5 (9.1 k), 4 tokens 64 / 53 (12.2 k); 128 of 1024 x 1280, top 8, 5 tokens 48.9 / 47.1
+        // (7.7 k); 288 of 4096 x 2048, top 8, 2 tokens 84 / 71 (18.4 k), 5 tokens 186 / 151; 1 token 48.5, 54.8 with the kernels for fewer than 16 combos.
         MoeDownCall d = {};
         d.ids = ids, d.wts = wts, d.table = table_dn, d.experts = p->experts, d.topk = p->topk, d.h = p->h, d.gs = gs_dn, d.inter = p->inter;
         d.shared = shared_gate ? shared_down : nullptr, d.hs = p->hs, d.shared_gs = shared_gate ? shared_gs + 2 : nullptr, d.sgate = sgate;
         d.shared_inter = p->shared_inter, d.y = y, d.tokens = tokens, d.hidden = p->hidden, d.out_bf16 = ydtype == CN_BF16;
-        if (cn_moe_down_combine_fits(d)) {
+        if (cn_moe_down_combine_fits(d) && (tokens * p->topk < ROWS_COMBOS || cn_moe_down_combine_units(d) <= STEP_UNITS)) {
             GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, tokens * p->topk, p->topk, limit, dtype);
             if (shared_gate)
                 a.side_w0 = shared_gate, a.side_w1 = shared_up, a.side_gs = shared_gs, a.side_y = p->hs, a.side_rows = p->shared_inter, a.side_tokens = tokens;

@@ -167,6 +167,8 @@ bool cn_moe_down_combine_fits(const MoeDownCall& c) {
            !(((uintptr_t)c.shared | (uintptr_t)c.h | (uintptr_t)c.hs) & 15);
 }
 
+long long cn_moe_down_combine_units(const MoeDownCall& c) { return (long long)((c.hidden + 15) / 16) * c.tokens * units_of(c); }
+
 int cn_moe_down_combine_launch(const MoeDownCall& c, cudaStream_t stream) {
     if (!cn_moe_down_combine_fits(c)) CN_FAIL(CN_ERR_SHAPE, "moe down projections: inter %d, shared inter %d, %d picks", c.inter, c.shared_inter, c.topk);
     const int units = units_of(c);

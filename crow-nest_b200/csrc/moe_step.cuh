@@ -22,4 +22,6 @@ struct MoeDownCall {
     int tokens, hidden, out_bf16;
 };
 bool cn_moe_down_combine_fits(const MoeDownCall& c);
+// 16 result rows of a token x eight 64-value blocks of one of its experts, over the whole call
+long long cn_moe_down_combine_units(const MoeDownCall& c);
 int cn_moe_down_combine_launch(const MoeDownCall& c, cudaStream_t stream);

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("hidden,inter,topk,tokens,shared", [(256, 256, 1, 1, 0), (512, 768, 11, 4, 256), (256, 512, 1, 47, 1024), (1024, 2048, 8, 5, 2048),
-                                                           (768, 1280, 6, 7, 512), (256, 256, 40, 1, 256)])
+                                                           (768, 1280, 6, 7, 512), (256, 256, 40, 1, 256),
+                                                           # long k below 16 combos; 44 combos on both sides of the units that two launches take
+                                                           (1024, 2048, 8, 1, 2048), (512, 2048, 4, 11, 1024), (768, 2048, 4, 11, 1024)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, "partial"])
 def test_small_steps_against_64_bits(hidden, inter, topk, tokens, shared, dtype):
     rng = np.random.default_rng(hidden + inter + tokens)
