@@ -16,10 +16,11 @@
 //            one HFMA2 to the codec's f16 weights (bit-exact) and accumulates with f16 x f16 -> f32
 //            mixed FMAs; partial sums of the k-split go to scratch
 //   had_out  y = H128(sum of partials) / 128 * svh
-// The first step is part of the GEMV launch for x (every CTA transforms its k-split) and a kernel of its own, with the activation, for h; the
-// last one carries the weighted combine of a routed step. One token, four experts of 4096 x 1536: eight launches 52.5 us, five 43.4.
+// The first step is part of the GEMV launch for x where there are few rows (every CTA transforms its k-split) and a launch of its own for more
+// (staged_rows), and a kernel of its own, with the activation, for h; the last one carries the weighted combine of a routed step. One token, four experts
+// of 4096 x 1536: eight launches 52.5 us, five 43.4.
 // The inner loop is instruction-bound, not HBM-bound: about 7 issue slots per 3-bit weight. A stage is a whole 128-row block of eight tiles: with
-// four the waits and counters of a stage cost 21 of the 70 instructions a tile (16 tokens 280 us a step against 296).
+// four the waits and counters of a stage took a step of 16 tokens from 280 to 296 us.
 // Three helpers restate reference text because their operation order defines the bits the parity contract asks for:
 // fwht128 follows mul1_fwht128 (engine/src/kernels_mul1.cu:74-88: the stage order and the a+b / a-b pairing), out_block
 // follows mul1_out_block (:98-110: partial sums left to right, then the transform, 1/128 and the scale), mul1_pair follows
@@ -126,6 +127,60 @@ __device__ __forceinline__ void load_x4(const void* x, int bf16, bool wide, size
     }
 }
 
+// The input transform of 128 values of row t of a slot, by one warp: v = H128(x * suh), four values a lane; returns the power of two that
+// brings them into f16 and, in inv, its inverse.
+struct Mul1Block {
+    const Mul1In& in;
+    const uint16_t* suh;
+    bool wide_x, wide_s;
+    __device__ __forceinline__ Mul1Block(const Mul1In& in_, unsigned long long rec, long long suh_off)
+        : in(in_), suh((const uint16_t*)(rec + (unsigned long long)suh_off)), wide_x(((uintptr_t)in_.x & 15) == 0), wide_s(((uintptr_t)suh & 7) == 0) {}
+    __device__ __forceinline__ float operator()(int slot, int t, int T, int k, int c0, int lane, float v[4], float& inv) const {
+        const int src = in.rowsrc ? in.rowsrc[slot * T + t] : 0;
+        const size_t xrow = (in.rowsrc ? (size_t)(src < 0 ? 0 : src) : (size_t)(slot / in.x_div) * T + t) * k;
+        load_x4(in.x, in.bf16, wide_x, xrow + c0, v);
+        uint16_t sc[4];
+        if (wide_s) {
+            const uint2 u = *(const uint2*)(suh + c0);
+            sc[0] = (uint16_t)u.x, sc[1] = (uint16_t)(u.x >> 16), sc[2] = (uint16_t)u.y, sc[3] = (uint16_t)(u.y >> 16);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) sc[j] = suh[c0 + j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = __fmul_rn(src < 0 ? 0.0f : v[j], h2f(sc[j]));
+        fwht128(v, lane);
+        float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        return block_scale(amax, inv);
+    }
+};
+// the record of a slot: of the combo's expert where the launch is the first of its chain
+__device__ __forceinline__ unsigned long long slot_record(const unsigned long long* ptrs, const Mul1In& in, int slot) {
+    if (!in.table) return ptrs[slot];
+    const int e = in.ids[slot];
+    return (e < 0 || (in.experts > 0 && e >= in.experts)) ? 0ull : in.table[e];
+}
+
+// The input transform as a launch of its own: xh = the hi / lo planes, xinv = the inverse scales. grid (k/128, matrices, slots), block 32 T (warp t =
+// activation row t). Taken where the CTAs of the GEMV would repeat it too often (see staged_rows).
+__global__ void mul1_had_in_kernel(unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, int k, int T, size_t plane, Mul1In in) {
+    pdl_launch_dependents();
+    pdl_wait();  // everything below may read what earlier kernels of the stream wrote
+    const int slot = blockIdx.z, t = threadIdx.x >> 5, blk = blockIdx.x, lane = threadIdx.x & 31;
+    const unsigned long long rec = slot_record(ptrs, in, slot);
+    if (in.table && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ptrs[slot] = rec;
+    if (rec == 0ull) return;  // a null record: nothing to read or write
+    const Mul1Side& sd = blockIdx.y ? side_b : side_a;
+    const size_t row = (size_t)slot * T + t;
+    const int c0 = blk * 128 + 4 * lane;
+    float v[4], inv;
+    const float mul = Mul1Block(in, rec, sd.suh_off)(slot, t, T, k, c0, lane, v, inv);
+    store_hi_lo(sd.xh, plane, row * k + c0, v, mul);
+    if (lane == 0) sd.xinv[row * (k / 128) + blk] = inv;
+}
+
 // the codec's f16 weights of two states (bit-exact): sum16 = 0x6400 + bytesum(state * 0x83DCD12D) is the
 // f16 pattern of 1024 + s; w = fma(sum16, 0x1eee, 0xc931) in f16 with one rounding (converter/src/mul1.rs:135-143)
 __device__ __forceinline__ uint32_t mul1_pair(uint32_t s0, uint32_t s1) {
@@ -177,14 +232,8 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
     // the arithmetic does not depend on SPC; a CTA that takes several streams them through one ring without a drain
     extern __shared__ __align__(128) uint8_t smem[];
     const int slot = blockIdx.z, sp0 = blockIdx.y * SPC;
-    unsigned long long rec;
-    if (HAD && in.table) {
-        const int e = in.ids[slot];
-        rec = (e < 0 || (in.experts > 0 && e >= in.experts)) ? 0ull : in.table[e];
-        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ptrs[slot] = rec;
-    } else {
-        rec = ptrs[slot];
-    }
+    const unsigned long long rec = HAD ? slot_record(ptrs, in, slot) : ptrs[slot];
+    if (HAD && in.table && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ptrs[slot] = rec;
     if (rec == 0ull) return;  // uniform, before any barrier
     const int k = sp_.k, n = sp_.n, n32 = sp_.n32;
     const int tiles_n = n >> 4, tps = (k >> 4) / S, kb0 = sp0 * tps, rows = SPC * tps * 16;
@@ -243,31 +292,11 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
     // the activation rows of this k-split, and their block scales
     const int nblk = rows / 128;
     if (HAD) {
-        const uint16_t* suh = (const uint16_t*)(rec + (unsigned long long)sd.suh_off);
-        const bool wide_x = ((uintptr_t)in.x & 15) == 0, wide_s = ((uintptr_t)suh & 7) == 0;
+        const Mul1Block block(in, rec, sd.suh_off);
         for (int i = warp; i < T * nblk; i += 8) {
             const int t = i / nblk, b = i - t * nblk;
-            const int src = in.rowsrc ? in.rowsrc[slot * T + t] : 0;
-            const size_t xrow = (in.rowsrc ? (size_t)(src < 0 ? 0 : src) : (size_t)(slot / in.x_div) * T + t) * k;
-            const int c0 = kb0 * 16 + b * 128 + 4 * lane;
-            float v[4];
-            load_x4(in.x, in.bf16, wide_x, xrow + c0, v);
-            uint16_t sc[4];
-            if (wide_s) {
-                const uint2 u = *(const uint2*)(suh + c0);
-                sc[0] = (uint16_t)u.x, sc[1] = (uint16_t)(u.x >> 16), sc[2] = (uint16_t)u.y, sc[3] = (uint16_t)(u.y >> 16);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) sc[j] = suh[c0 + j];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) v[j] = __fmul_rn(src < 0 ? 0.0f : v[j], h2f(sc[j]));
-            fwht128(v, lane);
-            float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            float inv;
-            const float mul = block_scale(amax, inv);
+            float v[4], inv;
+            const float mul = block(slot, t, T, k, kb0 * 16 + b * 128 + 4 * lane, lane, v, inv);
             store_hi_lo(xs, (size_t)T * pitch, (size_t)t * pitch + b * 128 + 4 * lane, v, mul);
             if (lane == 0) xi[i] = inv;
         }
@@ -531,9 +560,9 @@ namespace {
 struct Mul1Plan {
     int hidden, inter, bits, half, n32, max_slots, max_t;
     size_t kmax;
-    uint16_t* xh;           // [2 planes][slots][T][kmax] f16: the staged rows of the down projection
+    uint16_t *xh, *xh_up;   // [2 planes][slots][T][kmax] f16: staged rows (of the down projection; of gate and of up where they are staged)
     size_t plane;           // elements of one plane
-    float* xinv;            // [slots][T][kmax/128]
+    float *xinv, *xinv_up;  // [slots][T][kmax/128]
     float *part_a, *part_b;  // [slots][16][T][kmax]
     unsigned long long* ptrs;  // [slots] gathered record addresses (MoE form)
     int32_t* order;            // [slots] combos sorted by expert (grouped MoE form)
@@ -605,6 +634,19 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     return CN_OK;
 }
 
+// Whether the rows are transformed by a launch of their own. Inside the GEMV every CTA of a k-split repeats the transform of its part: (n / 128) x (k / 128)
+// block transforms for a row and matrix, against a launch more. us per call inside / apart, hidden 4096, inter 1536, one matrix (384 transforms a row) or
+// gate and up (768) and the whole FFN: gate of 4 slots, 1 row each 16.4 / 18.4 (1.5 k), 4 rows 16.4 / 18.4 (6.1 k), 8 rows 20.5 / 20.5 (12.3 k); 16 slots, 2 rows
+// 42.6 / 42.5 (12.3 k), 8 rows 57.4 / 52.8; 48 slots, 8 rows 166 / 135; FFN of 4 slots, 1 row 41.0 / 43.0 (3.1 k), 4 rows 45.1 / 45.1 (12.3 k); 16 slots, 8 rows
+// 170 / 149; a routed step of 16 tokens 268 / 256, of 64 tokens 575 / 516.
+bool staged_rows(const Mul1Spec& s, int matrices, int slots, int T) { return (long long)matrices * slots * T * (s.n / 128) * (s.k / 128) > 12288; }
+
+// sb: the second matrix of the launch (up beside gate), or null
+int launch_had_in(unsigned long long* ptrs, const Mul1In& in, const Mul1Side& sa, const Mul1Side* sb, int k, int slots, int T, size_t plane, cudaStream_t st) {
+    CN_CUDA(cn_launch_pdl(mul1_had_in_kernel, dim3(k / 128, sb ? 2 : 1, slots), dim3(32 * T), 0, st, ptrs, sa, sb ? *sb : sa, k, T, plane, in));
+    return CN_OK;
+}
+
 int check_run(const Mul1Plan* p, int slots, int T, const char* who) {
     if (!p) CN_FAIL(CN_ERR_SHAPE, "%s: null plan", who);
     if (slots < 1 || slots > p->max_slots || T < 1 || T > p->max_t)
@@ -656,7 +698,9 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     step(cudaMalloc(&p->xh, 2 * p->plane * 2));
+    step(cudaMalloc(&p->xh_up, 2 * p->plane * 2));
     step(cudaMalloc(&p->xinv, rows * (p->kmax / 128) * 4));
+    step(cudaMalloc(&p->xinv_up, rows * (p->kmax / 128) * 4));
     step(cudaMalloc(&p->part_a, rows * 16 * p->kmax * 4));
     step(cudaMalloc(&p->part_b, rows * 16 * p->kmax * 4));
     step(cudaMalloc(&p->ptrs, (size_t)max_slots * 8));
@@ -677,7 +721,7 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
 extern "C" int cn_mul1_plan_destroy(void* plan) {
     Mul1Plan* p = (Mul1Plan*)plan;
     if (!p) return CN_OK;
-    cudaFree(p->xh), cudaFree(p->xinv), cudaFree(p->place), cudaFree(p->part_a), cudaFree(p->part_b), cudaFree(p->ptrs),
+    cudaFree(p->xh), cudaFree(p->xh_up), cudaFree(p->xinv), cudaFree(p->xinv_up), cudaFree(p->place), cudaFree(p->part_a), cudaFree(p->part_b), cudaFree(p->ptrs),
         cudaFree(p->eo), cudaFree(p->order), cudaFree(p->groups), cudaFree(p->rowsrc), cudaFree(p->rowdst);
     delete p;
     return CN_OK;
@@ -691,9 +735,12 @@ extern "C" int cn_mul1_gemv(void* plan, int which, const unsigned long long* ptr
     if (dtype != CN_F32 && dtype != CN_BF16) CN_FAIL(CN_ERR_SHAPE, "cn_mul1_gemv: dtype %d is neither CN_F32 nor CN_BF16", dtype);
     cudaStream_t st = (cudaStream_t)stream;
     const Mul1Spec s = spec_of(p, which);
-    const Mul1Side side = {nullptr, nullptr, p->part_a, s.tr_off, s.suh_off};
+    const Mul1Side side = {p->xh, p->xinv, p->part_a, s.tr_off, s.suh_off};
     const Mul1In in = {x, dtype == CN_BF16, x_div, nullptr, nullptr, nullptr, 0};
-    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, p->plane, st, &in)) return rc;
+    const bool staged = staged_rows(s, 1, slots, t);
+    if (staged)
+        if (int rc = launch_had_in(const_cast<unsigned long long*>(ptrs), in, side, nullptr, s.k, slots, t, p->plane, st)) return rc;  // (table null: ptrs is read)
+    if (int rc = launch_gemv(ptrs, side, nullptr, s, slots, t, p->plane, st, staged ? nullptr : &in)) return rc;
     dim3 grid(s.n / 128, 1, slots);
     if (dtype == CN_BF16)
         CN_CUDA(cn_launch_pdl((mul1_had_out_kernel<1>), dim3(grid), dim3(32 * t), 0, st, ptrs, p->part_a, y, s.n, ksplit(s.k), t, s.svh_off, (const int*)nullptr));
@@ -708,9 +755,12 @@ static int mul1_ffn_parts(Mul1Plan* p, const unsigned long long* ptrs, const Mul
     const Mul1Spec g = spec_of(p, 0), u = spec_of(p, 1), d = spec_of(p, 2);
     // gate and up share each launch: two small grids on two streams cost an event fork and join and ran one after the other
     // anyway (one token, four experts of 4096 x 1536: 65 -> 55 us with out_block's wide loads; 16 tokens: 295 us, no difference beyond noise)
-    const Mul1Side ga = {nullptr, nullptr, p->part_a, g.tr_off, g.suh_off}, up = {nullptr, nullptr, p->part_b, u.tr_off, u.suh_off};
+    const Mul1Side ga = {p->xh, p->xinv, p->part_a, g.tr_off, g.suh_off}, up = {p->xh_up, p->xinv_up, p->part_b, u.tr_off, u.suh_off};
     const Mul1Side dn = {p->xh, p->xinv, p->part_a, d.tr_off, d.suh_off};
-    if (int rc = launch_gemv(ptrs, ga, &up, g, slots, t, p->plane, st, &in, live)) return rc;
+    const bool staged = staged_rows(g, 2, slots, t);
+    if (staged)
+        if (int rc = launch_had_in(const_cast<unsigned long long*>(ptrs), in, ga, &up, g.k, slots, t, p->plane, st)) return rc;
+    if (int rc = launch_gemv(ptrs, ga, &up, g, slots, t, p->plane, st, staged ? nullptr : &in, live)) return rc;
     CN_CUDA(cn_launch_pdl(mul1_act_had_in_kernel, dim3(p->inter / 128, 1, slots), dim3(32 * t), 0, st, ptrs, p->part_a, p->part_b, p->xh, p->xinv, p->inter, ksplit(p->hidden), t,
                                                                          g.svh_off, u.svh_off, d.suh_off, limit, p->plane));
     return launch_gemv(ptrs, dn, nullptr, d, slots, t, p->plane, st, nullptr, live);

@@ -158,3 +158,61 @@ def test_moe_step_with_bundled_rows_matches_the_cpu_reference(tokens, experts, t
     y2 = plan.moe(table, ids, wts, dev(x), limit=10.0)
     assert torch.equal(y.view(torch.int32), y2.view(torch.int32))
     plan.free()
+
+
+def records(n, hidden, inter, K, seed):
+    """Codes uniform, scales small with random signs; in one allocation, as addresses."""
+    rng = np.random.default_rng(seed)
+    size = mul1.record_bytes(hidden, inter, K)
+    rec = rng.integers(0, 256, (n, size), dtype=np.uint8)
+    at = int(3 * (hidden // 16) * (inter // 16) * 32 * K)
+    v = (np.abs(rng.standard_normal((n, 3 * (hidden + inter)))) * 0.02 + 1e-3) * rng.choice([-1.0, 1.0], (n, 3 * (hidden + inter)))
+    rec[:, at:at + 6 * (hidden + inter)] = v.astype(np.float16).view(np.uint8)
+    rec[:, at + 6 * (hidden + inter):] = 0
+    d = dev(rec)
+    return d, torch.tensor([r.data_ptr() for r in d.unbind(0)], dtype=torch.int64, device="cuda")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("K", [3.0, 3.5])
+@pytest.mark.parametrize("t,x_div", [(1, 1), (3, 1), (8, 1), (8, 4)])
+def test_rows_transformed_in_a_launch_of_their_own_have_the_same_bits(dtype, K, t, x_div):
+    """Many slots take a launch for the input transform, few have it inside the GEMV: slot by slot the same results, also off 16 bytes and beside null records."""
+    hidden, inter, slots = 512, 384, 12288 // (4 * 3 * t) // 4 * 4 + 8
+    rec, ptrs = records(5, hidden, inter, K, t)
+    ptrs = ptrs.repeat(-(-slots // 5))[:slots].clone()
+    ptrs[3::7] = 0
+    gen = torch.Generator(device="cuda").manual_seed(t)
+    whole, one = mul1.Mul1Plan(hidden, inter, K, slots=slots, tokens=t), mul1.Mul1Plan(hidden, inter, K, slots=4, tokens=t)
+    for which, k in ((0, hidden), (2, inter)):
+        n = slots // x_div * t * k
+        x = (torch.randn(n + 1, device="cuda", generator=gen) * 0.25).to(dtype)[1:].view(slots // x_div, t, k)  # off 16 bytes
+        y = whole.run_slots(which, ptrs, x, x_div=x_div)
+        for s in list(range(0, 16, 4)) + [slots - 4]:
+            assert torch.equal(one.run_slots(which, ptrs[s:s + 4], x[s // x_div:(s + 4) // x_div], x_div=x_div), y[s:s + 4]), (which, s)
+    x = (torch.randn((slots // x_div, t, hidden), device="cuda", generator=gen) * 0.25).to(dtype)
+    y = whole.ffn(ptrs, x, x_div=x_div, limit=5.0)
+    assert y.isfinite().all() and y[0].any() and not y[3].any()
+    for s in list(range(0, 16, 4)) + [slots - 4]:
+        assert torch.equal(one.ffn(ptrs[s:s + 4], x[s // x_div:(s + 4) // x_div], x_div=x_div, limit=5.0), y[s:s + 4]), s
+
+
+@pytest.mark.parametrize("tokens,experts", [(150, 1500), (150, 40), (40, 40)])
+def test_routed_steps_of_many_combos_match_one_token_steps(tokens, experts):
+    """Combos that keep a slot each (few of them for the experts there are) and combos in groups of four and eight rows, with their rows transformed in a
+    launch of their own: ids outside the table, experts that are not resident; against steps of one token, which have the transform inside the GEMV."""
+    hidden, inter, topk, K = 512, 384, 4, 3.0
+    rec, ptrs = records(8, hidden, inter, K, 3)
+    table = ptrs.repeat(-(-experts // 8))[:experts].clone()
+    table[5::11] = 0
+    rng = np.random.default_rng(tokens + experts)
+    ids = np.stack([rng.permutation(experts)[:topk] for _ in range(tokens)]).astype(np.int32)
+    ids[::9, 1], ids[::13, 2] = -1, experts
+    d_ids = dev(ids)
+    wts = torch.from_numpy(rng.uniform(0.1, 1.0, (tokens, topk)).astype(np.float32)).cuda()
+    x = torch.from_numpy((rng.standard_normal((tokens, hidden)) * 0.25).astype(np.float32)).cuda()
+    whole, one = mul1.Mul1Plan(hidden, inter, K, slots=tokens * topk), mul1.Mul1Plan(hidden, inter, K, slots=topk)
+    y = whole.moe(table, d_ids, wts, x, limit=5.0)
+    assert y.isfinite().all()
+    for i in range(0, tokens, 7):
+        assert torch.equal(one.moe(table, d_ids[i:i + 1], wts[i:i + 1], x[i:i + 1], limit=5.0), y[i:i + 1]), i
