@@ -600,26 +600,7 @@ def gemm_arm(args, rank, world, local):
     it = [0]
 
     def launches(rows, k):
-        """Kernels of one GEMM call: rows into f16 (up to 128 of them), GEMM, and the sum over a split K range (the launcher's choice of tile and
-        split restated: csrc/nvfp4_gemm_pair.cu, pair_shape)."""
-        nw, rt, up = k // 256, (rows + 255) // 256, lambda a, b: (a + b - 1) // b
-        slow = 170.0 if m <= 128 else 300.0
-        most = min(up(m, 32) * 32, 256)
-        room = 8 if (fp4 or m <= 128) and rows <= 32768 else max(1, min(8, 32768 // rows))
-        best, split = 1e30, 1
-        for n in range(up(m, most), up(m, 32) + 1):
-            t = up(up(m, n), 32) * 32
-            for ks in range(1, (room if m <= 512 else 1) + 1):
-                if ks > 1 and ks > nw // 2:
-                    break
-                tail = 2500.0 + 16.0 * t
-                cost = up(rt * up(m, t) * ks, 74) * (4 * up(nw, ks) * max(2.0 * t, slow) + (tail if t > 192 else 400.0)) + (0.0 if t > 192 else tail)
-                cost += 5000.0 + ks * m * rows / 300.0 if ks > 1 else 0.0
-                if cost < best:
-                    best, split = cost, ks
-            if t <= 64:
-                break
-        return (1 if m <= 128 else 0) + 1 + (1 if split > 1 else 0)
+        return (_lib.lib().cn_nvfp4_bs_launches if fp4 else _lib.lib().cn_nvfp4_gemm_launches)(rows, k, m, _lib.CN_BF16)
 
     def step():
         i = it[0]

@@ -84,6 +84,8 @@ _SIGS = {
     "cn_nvfp4_gemm": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, C.c_size_t, _vp],
     "cn_nvfp4_gemm_workspace_bytes": [_i, _i],
     "cn_nvfp4_gemm_workspace_bytes_of": [_i, _i, _i],
+    "cn_nvfp4_gemm_launches": [_i, _i, _i, _i],
+    "cn_nvfp4_bs_launches": [_i, _i, _i, _i],
     "cn_nvfp4_bs_packed_bytes": [_i, _i],
     "cn_nvfp4_bs_repack": [_vp, _vp, _i, _i, _vp],
     "cn_nvfp4_bs_workspace_bytes": [_i, _i, _i],

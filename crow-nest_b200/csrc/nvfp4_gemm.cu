@@ -133,6 +133,11 @@ extern "C" size_t cn_nvfp4_gemm_workspace_bytes_of(int rows, int k, int m) {
     return front_bytes(k, m) + (s > 1 ? (size_t)s * m * rows * 4 : 0);
 }
 
+extern "C" int cn_nvfp4_gemm_launches(int rows, int k, int m, int dtype) {
+    if (rows <= 0 || k <= 0 || k % 256 || m <= 0) return 0;
+    return (rows_as_f16(dtype, m) ? 1 : 0) + 1 + (splits_of(rows, k, m, dtype, sum_bytes(m)) > 1 ? 1 : 0);
+}
+
 extern "C" int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
                              size_t workspace_bytes, cn_stream_t stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;

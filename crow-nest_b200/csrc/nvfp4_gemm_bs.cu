@@ -511,6 +511,12 @@ extern "C" size_t cn_nvfp4_bs_workspace_bytes(int rows, int k, int m) {
     return f32 > bf16 ? f32 : bf16;
 }
 
+extern "C" int cn_nvfp4_bs_launches(int rows, int k, int m, int dtype) {
+    if (rows <= 0 || k <= 0 || k % KT || m <= 0) return 0;
+    if (dtype == CN_BF16) return (f16_rows(m) ? 1 : 0) + 1 + (pair_splits(rows, k, m) > 1 ? 1 : 0);
+    return 2 + (ksplits_for(rows, k, m) > 1 ? 1 : 0);
+}
+
 extern "C" int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype,
                                 void* workspace, size_t workspace_bytes, cn_stream_t stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;

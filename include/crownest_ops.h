@@ -216,6 +216,8 @@ int cn_moe_nvfp4_finish(void* plan, const void* shared_gate, const void* shared_
  * parts as there is room for. */
 size_t cn_nvfp4_gemm_workspace_bytes(int k, int m);
 size_t cn_nvfp4_gemm_workspace_bytes_of(int rows, int k, int m);
+/* kernels that one call launches (with a workspace of one of these sizes; 0 for a shape that is refused) */
+int cn_nvfp4_gemm_launches(int rows, int k, int m, int dtype);
 int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
                   size_t workspace_bytes, cn_stream_t stream);
 
@@ -236,6 +238,7 @@ int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int ro
 size_t cn_nvfp4_bs_packed_bytes(int rows, int k);
 int cn_nvfp4_bs_repack(const void* w, void* packed, int rows, int k, cn_stream_t stream);
 size_t cn_nvfp4_bs_workspace_bytes(int rows, int k, int m);
+int cn_nvfp4_bs_launches(int rows, int k, int m, int dtype); /* kernels of one call, as cn_nvfp4_gemm_launches */
 int cn_nvfp4_bs_gemm(const void* packed, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
                      size_t workspace_bytes, cn_stream_t stream);
 int cn_nvfp4_act_cascade(const void* x, void* out, int rows, int k, int levels, int dtype, cn_stream_t stream);
