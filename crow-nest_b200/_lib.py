@@ -19,13 +19,23 @@ class CrownestError(RuntimeError):
     pass
 
 
-HOST_PATH = os.path.join(_HERE, "_host.so")
+def _torch_tag():
+    """Python's and torch's version: the host extension is bound to the C++ interface of both."""
+    import re
+    import sys
+    import torch
+    return re.sub(r"[^0-9A-Za-z.-]", "_", f"py{sys.version_info[0]}.{sys.version_info[1]}-torch{torch.__version__}")
+
+
+def host_path():
+    """The host extension's file. Its name holds the versions it was built for: one built for another torch is not loaded but missing."""
+    return os.path.join(_HERE, f"_host-{_torch_tag()}.so")
 
 
 def _build_host(force):
     """g++ over csrc/host.cpp against torch's headers: the Python extension of the small operators."""
-    src = os.path.join(CSRC, "host.cpp")
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= os.path.getmtime(src):
+    src, out = os.path.join(CSRC, "host.cpp"), host_path()
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(src):
         return
     import sysconfig
     import torch
@@ -33,10 +43,10 @@ def _build_host(force):
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
            os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
     cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    cmd += ["-isystem" + i for i in inc] + [src, "-o", HOST_PATH, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    cmd += ["-isystem" + i for i in inc] + [src, "-o", out, "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise CrownestError("building _host.so failed:\n" + r.stdout[-2000:] + r.stderr[-4000:])
+        raise CrownestError("building the host extension failed:\n" + r.stdout[-2000:] + r.stderr[-4000:])
 
 
 def build(force=False, jobs=8):
@@ -183,10 +193,11 @@ def host():
         import importlib.machinery
         import importlib.util
         import torch  # noqa: F401  (its libraries are what the extension links to)
-        if not os.path.exists(HOST_PATH):
-            raise CrownestError(f"{HOST_PATH} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
+        path = host_path()
+        if not os.path.exists(path):
+            raise CrownestError(f"{path} is missing: run `python -c 'import __graft_entry__ as g; g.build()'`")
         L = lib()
-        loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+        loader = importlib.machinery.ExtensionFileLoader("_host", path)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
         loader.exec_module(mod)
         names = ("cn_nvfp4_gemv", "cn_nvfp4_gemv_gu", "cn_nvfp4_gemm", "cn_nvfp4_gemm_workspace_bytes_of", "cn_nvfp4_bs_gemm", "cn_nvfp4_bs_workspace_bytes",
