@@ -11,8 +11,8 @@
 // side stream and back.
 //
 // What bounds it: latency. The ids are older than the kernel before this one (which waits for whatever wrote them before it lets this one
-// start), so the first weights are on their way while gate / up still runs; after it there is one trip to L2 for h, some 900
-// instructions a unit, and a barrier.
+// start), so the first weights are on their way while gate / up still runs; after it there is one trip to L2 for h, the
+// unit itself (some 1450 warp instructions with its loads and planes), and a barrier.
 #include "moe_step.cuh"
 #include "nvfp4_col.cuh"
 

@@ -20,9 +20,9 @@
 // are two accumulators and the epilogue of a tile runs under the MMAs of the next.
 // Rings: weights 3 to 6 x 18 KB (256 values of K each), activations up to 8 x 16 KB and A slots 4..8 x 32 columns (64 values).
 //
-// Up to 128 rows the decode bounds it, not the MMAs: 127 warp instructions per scheduler and 64-value block, most of them at half rate,
-// 255 cycles measured; hence f16 (half the instructions of the decode to bf16), with the rows brought into f16 by a kernel before this one
-// that runs under this one's prologue, all sixteen warps decoding, and K split where row tiles do not fill the pairs. 17408 x 5120 at 64 rows:
+// Up to 128 rows the decode bounds it, not the MMAs: the way of a block through a warp (172 warp instructions per scheduler and 64-value block in all, no
+// unit near its rate) and the start and end of a launch; hence f16 (half the instructions of the decode to bf16), with the rows brought into f16 by a
+// kernel before this one that runs under this one's prologue, all sixteen warps decoding, and K split where row tiles do not fill the pairs. 17408 x 5120 at 64 rows:
 // 80 us (one CTA per tile, widened weights through shared memory) -> 21; 5120 x 17408: 109 -> 27.
 // Every wait is bounded. The weights are read with L2's ordinary policy: kept as evict-last, for the token tiles that read them again, they
 // gained nothing (512 rows 76.6 and 76.9 us) and stayed behind: a 50 MB matrix read twice after the call took 83 us the second time, 75 now.
@@ -78,7 +78,7 @@ struct DecodeAt {
 // Every SETS-th block of `stages` weight stages from block SET on, one row per thread. Container: block b is nine words from word 9 b of the
 // row's 144 bytes, inside three 16-byte chunks. Re-laid: codes are chunks 2 b and 2 b + 1 of the row's 128 swizzled bytes, the scale word lies
 // in the image's scale part. Two sets of warps where the MMAs or the ALUs bound the loop (four of one block each measured 5 % slower at
-// 200 - 1000 rows of bf16), four where it is the way of a block - load, decode, store to tensor memory, arrival, some 800 cycles - that does.
+// 200 - 1000 rows of bf16), four where it is the way of a block - load, decode, store to tensor memory, arrival - that does.
 template <bool BF16, bool PACKED, int SET, int SETS>
 __device__ __forceinline__ void decode_set(uint32_t src, uint32_t scales, uint32_t dst, uint64_t* wfull, uint64_t* wempty, uint64_t* aempty, uint32_t afull_base,
                                            int stages, int nws, int na, int lane, DecodeAt& at_) {

@@ -20,8 +20,8 @@
 // warp idles at a part's ragged end, warp 9 adds the eight sums of a part and stores. Clusters of two or four CTAs share a
 // tile by parts where that fills the machine better; the others hand a part's sums to the first CTA through distributed
 // shared memory.
-// What bounds it: the ALU and issue slots (a unit's decode and scaling are 88 warp instructions of half rate), at 0.56 of the slots in gate/up of
-// one row. The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
+// What bounds it: issue slots, at 0.63 of them in gate/up of one row (206 warp instructions a unit in all; 5120 x 17408 in clusters of two 0.47 and
+// 250). The FMA kernel that it replaces for k >= 2048 spends 3.2 slots per weight AND row.
 #include "common.cuh"
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"

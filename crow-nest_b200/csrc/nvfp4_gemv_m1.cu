@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(NT * TEAM, CPS) nvfp4_gemv_m1_kernel(const Gem
         }
         if (!ok) break;
         // the four lanes of a quad hold two columns each; then the eight warps' K ranges meet in shared memory:
-        // every warp posts its sums and arrives on the slot's barrier, warp 0 alone waits for all eight
+        // every warp posts its sums and arrives on the slot's barrier; the one that adds them (see red_slots) waits for all eight
         float* rb = red + rslot * (NW * MT * 16);
         if constexpr (MT == 1) {
             float a = acc0[0], b = acc1[0];
@@ -714,8 +714,9 @@ int launch_m1(const cudaLaunchConfig_t& cfg, const GemvParams& p) {
     return CN_OK;
 }
 
-// Slots for the sums of a tile's n parts. Warp 0 reads them at the tile's end; another warp is at most `stages` chunks beyond that end
-// then, and the parts that it has posted there end at least `gap` chunks apart: n + stages / gap, and one to spare.
+// Slots for the sums of a tile's n parts. One warp reads them at the tile's end (warp 0, or the warps by turns, tile by tile) and releases no stage
+// beyond that end before it has; another warp is then at most `stages` chunks beyond it, and the parts that it has posted there end at
+// least `gap` chunks apart: n + stages / gap, and one to spare.
 int red_slots(int stages, int gap, int n) { return n + stages / gap + 1 < RED_DEPTH ? n + stages / gap + 1 : RED_DEPTH; }
 static_assert(4 + MAX_STAGES <= RED_DEPTH, "slots of the tile sums");
 // Shared memory of a CTA in front of its weight rings: for each team header, those sums and the ones handed over inside a cluster; activations.
@@ -813,8 +814,9 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // 5120 gate / up 27.3 / 30.2 and 27.4 / 31.0, 7168 x 5120 8.5 / 9.8 and 9.3 / 11.1, 3000 x 9216 8.6 / 10.0 and 9.6 / 11.8; eight rows of gate / up
     // 46.6, one team 59.6), but not in clusters of four, which fill the SMs of a GPC badly with one CTA each (640 x 17408 10.3 / 12.0 and
     // 6.8 / 8.3), nor where tiles are short (two rows of 20246 x 1536 10.1 and 9.2,
-    // eight of 248000 x 2048 154 and 147). 5120 x 17408, two, four and eight rows:
-    // 18.6 / 21.3 / 34.8 in clusters of two; 22.0 / 26.7 / 53.1 with parts one after another and a single team.
+    // eight of 248000 x 2048 154 and 147). Eight rows in two teams spill 20 to 44 bytes a thread (18 warps leave each 96 registers); the figure
+    // for eight rows above has that in it. 5120 x 17408, two, four and eight rows: 18.6 / 21.3 / 34.8 in clusters of two; 22.0 / 26.7 / 53.1 with
+    // parts one after another and a single team.
     int ksplit = mt == 1 ? parts : 1, teams = 1, waves = 1;
     if (mt > 1 && !routed) {
         const double alone = mt == 2 ? 1.5 : (mt == 4 ? 1.3 : 1.2);

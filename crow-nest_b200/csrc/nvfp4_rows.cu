@@ -6,12 +6,11 @@
 //
 // An expert's matrices are small (2048 x 512: a row is 288 bytes), so what a GEMV kernel spends per tile - handing sums between
 // warps, staging and scale tables per CTA - outweighs the tile. Here a warp keeps a 16-row tile to itself: it brings the tile in
-// by its own asynchronous copies (16 row pieces of up to eight blocks, two to four chunks ahead; as a bulk copy each, some 25 cycles of the copy
-// engine whatever their size, they were what the kernel waited for: 64 tokens 244 us a step, 224 with 16-byte copies), holds all its sums in registers and stores
-// them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
+// by its own asynchronous copies (16 row pieces of up to eight blocks, two to four chunks ahead; as a bulk copy for every piece they were what the
+// kernel waited for: 64 tokens 244 us a step, 224 with 16-byte copies), holds all its sums in registers and stores them; warps meet only once, when the group's rows have been staged. Up to eight bf16 rows or two f32 rows of an expert (six
 // columns) share one decode of its weights; a row's sum does not depend on the rows it is grouped with. Bound by issue slots:
-// some 180 warp instructions per 16 x 128 values in all (200 and 258 us a step with one scale made at a time, 245 now). Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
-// the profiler): gate/up 157 -> 133 us, down 203 -> 86 us against one CTA set per combo.
+// some 175 warp instructions per 16 x 128 values in all (200 with one scale made at a time: 258 us a step against 245). Measured at 64 tokens, 512 experts of 2048 x 512, top 10 (under
+// the profiler): gate/up 157 -> 114 us, down 203 -> 77 us against one CTA set per combo.
 #include "nvfp4_col.cuh"
 #include "nvfp4_gemv.cuh"
 
@@ -216,7 +215,7 @@ int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
     RowsParams p = {};
     size_t smem;
     if (a.rows <= 0 || a.k <= 0 || a.k % 256 != 0) CN_FAIL(CN_ERR_SHAPE, "%s: k = %d must be a positive multiple of 256", who, a.k);
-    if (((uintptr_t)a.w0 | (uintptr_t)a.w1 | (uintptr_t)a.x) & 15)  // bulk copies and 128-bit loads
+    if (((uintptr_t)a.w0 | (uintptr_t)a.w1 | (uintptr_t)a.x) & 15)  // 16-byte asynchronous copies and 128-bit loads
         CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
     int cps = 2;
     if (!layout(a, 2, p, smem)) {

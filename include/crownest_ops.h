@@ -9,6 +9,12 @@
  *   - work is enqueued on the caller's stream and the call returns at once: no allocation, no
  *     synchronisation, no host access to the buffers (so calls can be captured in a CUDA graph);
  *   - outputs are assigned, never accumulated into, unless stated.
+ *   - weights of the GEMV calls (cn_nvfp4_gemv, _gu, _lines, cn_lm_head_argmax, cn_nvfp4_seq_run, cn_fp8_gemv) are constant while
+ *     work is queued: these kernels ask for weights and tensor scales before the kernel directly in front of them on the
+ *     stream has ended (programmatic dependent launch), and wait for it only before they touch activations and results.
+ *     A kernel that writes weights or scales is followed by an event wait, a copy or any plainly launched kernel before such
+ *     a call. All other calls (routed experts, MUL1, batched GEMMs, repack) read nothing before what is in front has ended,
+ *     but for the tensor scales of routed gate / up.
  * Differences: shapes are plain ints instead of device int buffers, kernels are compiled ahead of
  * time for sm_100a, and errors come back as a status code (0 = ok) with a message in
  * cn_last_error_string() instead of a panic.
@@ -161,9 +167,10 @@ int cn_moe_combine(const float* eo, const float* wts, const int32_t* ids, const 
 /* The routed-expert decode step, GpuMoePlan-shaped (engine/src/glm5_moe.rs:518-793; Flash-Next call
  * site Engine::moe_run, engine/src/gen.rs:4168-4532). The plan owns the scratch (the only
  * allocation; run() allocates nothing and does not synchronise). The plan also owns one side stream
- * and two events: run() enqueues the shared expert there between a fork event recorded on `stream`
- * and a join event `stream` waits for before the combine, so everything is ordered with the caller's
- * stream as if it ran on it (a capture of `stream` takes the side branch in).
+ * and two events: run() enqueues the shared expert of all but small steps there between a fork event
+ * recorded on `stream` and a join event `stream` waits for before the combine, so everything is ordered
+ * with the caller's stream as if it ran on it (a capture of `stream` takes the side branch in). A shared
+ * expert takes all of its pointers and a plan with shared_inter > 0; anything else is refused.
  * Tables are device arrays [experts] of device addresses (0 = expert not resident: its combos are
  * skipped, the contract of engine/src/kernels_mul1.cu:118-119; so are ids outside 0..experts-1). ids, order and the
  * tables must be complete when the call is enqueued or be written by earlier work on `stream`. table_gu = gate [inter][hidden], or
@@ -207,7 +214,8 @@ int cn_moe_nvfp4_finish(void* plan, const void* shared_gate, const void* shared_
  * tensor memory. Replaces gemm_fp4_dense (engine/src/kernels.rs:533, launched by launch_mma_d,
  * engine/src/gen.rs:2491) and glm5_gemm_fp4_tc (engine/src/kernels_glm5_moe.cu:349), with the latter's
  * arithmetic: weights widened losslessly (code x block scale), exact products, f32 accumulation. Up to 128 rows, and f32 rows always,
- * the activations go in as f16 x 2^k per row; more than 128 rows of bf16 as they are, without a pass over them. w is the container
+ * the activations go in as f16 x 2^k per row (one power of two for a row's largest finite value, subnormal to largest: bf16 values are
+ * exact down to 2^-27 of it, f32 values rounded to f16); more than 128 rows of bf16 as they are, without a pass over them. w is the container
  * layout, unchanged. y may overlap x (bf16 rows beyond 128 are copied to the workspace first then). The call allocates nothing:
  * `workspace` (device, 256-byte aligned) holds the f16 activations and, where k is split over the machine (up to 512 rows), the partial
  * sums of its parts; it may be reused by the next call on the same stream. cn_nvfp4_gemm_workspace_bytes gives what is enough for any
@@ -221,18 +229,20 @@ int cn_nvfp4_gemm_launches(int rows, int k, int m, int dtype);
 int cn_nvfp4_gemm(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype, void* workspace,
                   size_t workspace_bytes, cn_stream_t stream);
 
-/* The same product on the block-scaled FP4 tensor-core path: tcgen05.mma kind::mxf4nvf4 (both operands E2M1 with one
- * UE4M3 scale per 16 values, f32 accumulation in tensor memory). Replaces gemm_fp4_dense / gemm_fp4_dense_b
+/* The same product on weights that are re-laid for it. Replaces gemm_fp4_dense / gemm_fp4_dense_b
  * (engine/src/kernels.rs:533, :642) and quant_x_fp4 / quant_row_prescaled (:264-351, host twin act_cascade :5354-5475).
  * The weights are re-laid once at load (cn_nvfp4_bs_repack into cn_nvfp4_bs_packed_bytes bytes, 16-byte aligned: tiles of
  * 128 rows x 256 columns in the tensor core's shared-memory layout, scale byte 0x7F -> 0x7E and bit 7 cleared as the
- * reference does at load, engine/src/residency.rs:119-137). The activations of every call go through the reference's
- * cascade - a per-row power of two times a sum of NVFP4 levels, each coding the residual of the ones before - with five
- * levels instead of the reference's three (three leave 8e-4 relative L2, inside 1e-3 but tens of bf16 ulp on small outputs;
- * each level buys a factor of about 16). The levels of a token ride as columns of the MMA and are added in the epilogue.
- * k a multiple of 256; workspace (256-byte aligned, cn_nvfp4_bs_workspace_bytes) holds the cascade and, for few rows, the
- * partial sums of a split K range. Meant for 16 < m <= a few hundred rows, where it streams the weights near HBM speed;
- * for thousands of rows cn_nvfp4_gemm is as fast. cn_nvfp4_act_cascade exposes the cascade alone in the reference's byte
+ * reference does at load, engine/src/residency.rs:119-137).
+ * bf16 rows: the arithmetic and the kernel of cn_nvfp4_gemm, which decodes the stage images instead of container bytes.
+ * f32 rows: the block-scaled FP4 tensor-core path, tcgen05.mma kind::mxf4nvf4 (both operands E2M1 with one UE4M3 scale per
+ * 16 values, f32 accumulation in tensor memory). The activations go through the reference's cascade - a per-row power of two
+ * (between 2^-64 and 2^64) times a sum of NVFP4 levels, each coding the residual of the ones before - with five levels
+ * instead of the reference's three: 1.1e-5 relative L2 on f32 values where three leave 8e-4; each level buys a factor of
+ * about 16. The levels of a token ride as columns of the MMA and are added in the epilogue.
+ * k a multiple of 256; workspace (256-byte aligned, cn_nvfp4_bs_workspace_bytes for both types) holds the f16 rows or the
+ * cascade and, for few rows, the partial sums of a split K range; with bf16 rows less is accepted as in cn_nvfp4_gemm.
+ * cn_nvfp4_act_cascade exposes the cascade alone in the reference's byte
  * layout ([rows][levels * k/64 * 36 + 4]; level L at L * k/64 * 36, then the f32 factor 2^-k), bit-identical to the
  * reference's host twin; levels 1..8. */
 size_t cn_nvfp4_bs_packed_bytes(int rows, int k);
