@@ -785,6 +785,15 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int combos = a.combos + (routed ? a.side_tokens : 0);
     Split one = {1, 0};
     if (!routed) one = one_row_split(ntiles, bpr, tx);
+    // Larger matrices go to the fifth-generation tensor cores, whatever the number of rows (a rule of the matrix alone: a row's bits are those of a one-row
+    // call). us a call in a stream of dependent ones, there / here, for one and four rows: gate / up of 17408 x 5120 18.7 / 20.7 and 23.4 / 30.1, 5120 x 17408 12.4 /
+    // 15.4 and 15.0 / 21.1, 4096 x 4096 4.5 / 4.6 and 5.7 / 5.5, 20000 x 1536 5.8 / 7.4 and 7.3 / 9.5, 2048 x 4096 3.4 / 4.1 and 3.9 / 4.5; below, its longer way
+    // from the activations to the first product shows: 2048 x 2048 3.2 / 2.9 and 3.4 / 3.6, 512 x 2048 2.9 / 2.1 and 3.1 / 2.9. Few long rows stay too: its clusters end at
+    // eight CTAs a tile of 128 rows (640 x 17408 6.3 / 5.8, 512 x 16384 5.9 / 4.9, 2048 x 16384 7.7 / 8.1). A row that does not fit here is refused as it was.
+    if (!routed && (long long)rows * k * (gu ? 2 : 1) >= 8000000 && !(rows * (gu ? 2 : 1) <= 1280 && k > 14336)) {
+        const int bp = bpr / one.parts;
+        if (front_bytes(2, (bp + tx - 1) / tx, 1, 1, bp, 0) + 2 * stage_bytes <= sm_share(one.cps)) return cn_gemv_tc_launch(a, stream, who);
+    }
     const int parts = one.parts, bpp = bpr / parts;  // parts of K (each longer than a chunk where there are several), blocks of one
     // chunks from one part's end to the next where a CTA has n of them: a row is cut into whole chunks from its first part's start
     auto gap = [&](int n) { return n > 1 ? bpp / tx : (bpp + tx - 1) / tx; };

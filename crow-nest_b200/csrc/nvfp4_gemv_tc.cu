@@ -1,0 +1,660 @@
+// NVFP4 GEMV for 1..8 bf16 activation rows on the fifth-generation tensor cores (tcgen05.mma kind::mxf4nvf4, block scale): plain and gate / up form,
+// with or without the tensor-parallel line output. Supersedes gemv_nvfp4_w / _gu / _wm / _gum (engine/src/kernels_p2.rs:355-530).
+//
+// The weights are the A operand as they are: E2M1 codes with one UE4M3 scale per 16 values is what this MMA multiplies, so nothing is decoded. A bf16
+// row is the B operand as eight columns of signed octal digits: per 16 values a power of two and a number of 23 bits, digit j of a value being one
+// of -4..3, all of them E2M1 values (a bf16 value is exact unless it is below 2^-14 of its block's largest, and then off by 2^-22 of that at most).
+// Products, scales and digits are exact; a column's sum over 256 values is the tensor core's, which is the f32 nearest to it or the one beside (k = 256:
+// 2.5e-8 of a row against 64 bits, as much as the last rounding alone); the columns are added from the smallest up, and the chunks of 256 in f32 in order
+// (k = 4096: 6.2e-8, 17408: 8.6e-8). The columns of one row do not depend on those of another: a row of an m-row call has the bits of a one-row call,
+// and eight rows (64 columns) take the tensor core no longer than one, which is bound by reading A.
+//
+// A block of 16 whose largest value is below 2^-17 of its chunk's largest or below 2^-105, or that holds an infinity or NaN, takes no part in this: the
+// threads that add the chunk multiply it out from global memory in f32 (slow_block).
+//
+// A CTA owns 128 rows (64 of gate and 64 of up) over a part of k; a cluster of C CTAs shares the tile, part by part, and every CTA adds and stores
+// 128 / C of its rows, the parts in order. Warps: 0-3 add up and store (a thread is a row), 4-7 move container blocks (36 bytes) into the operand's
+// layout, 8-11 turn activations into digits, 12 loads (TMA, boxes of 128 rows x 144 bytes of container), 13 issues the MMAs. Loads and the move do
+// not wait for the kernel in front: when the activations come, five chunks of weights a CTA lie ready or nearly so.
+//
+// What bounds it, one row: HBM for large matrices (gate / up of 17408 x 5120: 100 MB in 18.6 us, of which 2.6 until the first product; the CTAs then take 6.1 TB/s);
+// for small ones the chain from one call to the next, some 3 us: end of the grid in front 0.8, activations 0.4, digits 0.35, first sum 0.4, adding up in
+// the cluster 0.4, output and end of the grid 0.6. From four rows on also the digits (one warp and row: 0.35 us a chunk). In a stream of dependent calls, us
+// here / mma.sync kernel (nvfp4_gemv_m1.cu): gate / up of 17408 x 5120 18.6 / 20.7, two rows 19.4 / 27.2, four 23.4 / 30.1, eight 31.4 / 46.6; 5120 x 17408
+// 12.4 / 15.4, 13.0 / 18.4, 15.1 / 21.1, 19.7 / 34.7; 25000 x 8192 21.8 / 28.1, four rows 27.5 / 32.1.
+// Measured and not kept: tiles of fewer rows so that every SM has the same bytes (the CTAs more hold up the next kernel: 5120 x 5120 5.9 -> 6.9); two teams of
+// warps for the move (18.6 -> 20.0, gate / up); L2 prefetches beyond the stages (18.6 -> 19.3 and more); a third operand stage in a container stage's place (20.6).
+#include "nvfp4_gemv.cuh"
+#include "tc5.cuh"
+
+#include <atomic>
+
+namespace {
+
+constexpr int CH = 256;                                       // values of k in a chunk: four MMAs
+constexpr int RAW_STAGE = 128 * 144;                          // container bytes of a chunk
+constexpr int A_CODES = 128 * 128, A_STAGE = A_CODES + 4 * 512;  // the same as operand: 128-byte swizzled rows, then the scales of the four MMAs
+constexpr int NX = 16;      // chunk factors in flight (a warp is at most a few chunks ahead of another)
+constexpr int NDONE = 4;    // barriers of finished chunks
+constexpr int MAX_RAW = 4;  // container stages
+constexpr int NA = 2;       // chunks laid out for the tensor core
+constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 4;
+constexpr int EPI_WARPS = 4, LOADER = 12, ISSUER = 13;  // warps 0-3 sums and output, 4-7 weights, 8-11 activations
+constexpr int THREADS = 448;
+constexpr int LV = 8;       // digits of a value
+constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, slow blocks}; [NX][4] scale bytes of 0xFF seen
+__host__ __device__ constexpr int ncol(int mt) { return mt * LV < 16 ? 16 : mt * LV; }      // columns of the MMA
+__host__ __device__ constexpr int b_codes(int mt) { return ncol(mt) * 128; }
+__host__ __device__ constexpr int b_stage(int mt) { return b_codes(mt) + 4 * 512; }
+__host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                 // chunks of digits
+__host__ __device__ constexpr int ex_slot(int mt) { return 168 * mt * 4; }                  // sums of a tile handed over: 128 rows, shares rounded up to 4
+__host__ __device__ constexpr int tmem_cols(int mt) { return mt <= 4 ? 128 : 256; }
+__host__ __device__ constexpr int smem_of(int mt, int raw) {
+    return HEADER + 1024 + NA * A_STAGE + nb_of(mt) * b_stage(mt) + raw * RAW_STAGE + 2 * ex_slot(mt);
+}
+
+struct TcParams {
+    const uint8_t* w0;
+    const uint8_t* w1;  // gate / up: up
+    const float* gs0;
+    const float* gs1;
+    const __nv_bfloat16* x;
+    void* y;
+    int rows, k, m, ldy, out_f32;
+    float limit;
+    uint32_t qinv;                 // 2^20 / share, rounded up: idx / share for idx < 1024
+    int csize, tiles, raw, share;  // CTAs per cluster, row tiles, container stages, rows (or pairs) of a tile that a CTA stores
+    unsigned long long yl[8];
+    int yl_world, yl_row0;
+    unsigned long long yl_stride;
+    const unsigned int* yl_epoch;
+    int yl_tag, yl_buf, yl_flip;
+};
+
+// ---------------------------------------------------------------- tcgen05
+__device__ __forceinline__ uint64_t desc_sf(uint32_t smem_addr) {  // a scale chunk: 32 rows of 16 bytes, no swizzle, 8-row groups 128 B apart
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(128 >> 4) << 32) | ((uint64_t)1 << 46);
+}
+// kind::mxf4nvf4: A and B E2M1 (format 1) K-major, UE4M3 scales (0), N >> 3 at bit 17, M >> 4 at bit 24
+__host__ __device__ constexpr uint32_t idesc_bs(int n) { return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24); }
+__device__ __forceinline__ void cp_sf(uint32_t taddr, uint64_t sdesc) {
+    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+__device__ __forceinline__ void umma_bs(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
+        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst), "l"(m),
+        "r"(x), "r"(y), "r"(bar), "l"(policy)
+        : "memory");
+}
+// a value into another CTA's shared memory, counted there on a barrier of the same CTA
+__device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {  // bounded, with cluster-scope acquire
+    const long long t0 = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (clock64() - t0 > 2000000000LL) return false;
+    }
+}
+
+// ---------------------------------------------------------------- 256 values of an activation row as digits (a warp; a lane holds eight values)
+// codes: the row's eight lines of the B tile (line j = digit j), 1024 bytes; sf: the scales of the four MMAs, n0 the row's first column.
+// With E the exponent of the block's largest value, a value is q x 2^(E - 21), |q| <= 2^22: its digits are the octal digits of q + 44444444 (octal), less
+// four each. The scale byte is 2^(8 - (Emax - E)), Emax that of the chunk.
+__device__ __forceinline__ void to_digits(uint4 raw, int lane, uint8_t* codes, uint8_t* sf, int n0, float2* fs) {
+    uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+    uint32_t top = __vmaxu2(__vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu));
+    top = max(top >> 16, top & 0xffffu);
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));  // two lanes hold a block of 16
+    uint32_t e = top >> 7;
+    const bool odd = top != 0u && (e < 22u || e == 255u);  // below 2^-105 (a scale of its digits would be no number), infinity, NaN
+    const uint32_t emax = max(__reduce_max_sync(0xffffffffu, odd ? 0u : e), 22u);
+    const bool slow = odd || (top != 0u && emax - e > 17u);
+    const uint32_t slow_lanes = __ballot_sync(0xffffffffu, slow);
+    if (slow || top == 0u) {
+        e = emax;
+        u[0] = u[1] = u[2] = u[3] = 0u;
+    }
+    const float scale = __uint_as_float((275u - e) << 23);  // 2^(21 - (e - 127))
+    uint32_t lo[4], hi[4];  // value pair p: byte j = digits j (hi: 4 + j) of both
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        uint32_t sel[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float v = __uint_as_float(h ? u[p] & 0xffff0000u : u[p] << 16);
+            uint32_t q = __float_as_uint(fmaf(v, scale, 12582912.0f)) + (044444444u - 0x4b400000u);  // (q + 2^22 is the sum's mantissa: rounded to nearest even)
+            q += (q & 0x00fff000u) * 15u;  // octal digits apart: four to sixteen bits, two to eight, one to four
+            q += (q & 0x0fc00fc0u) * 3u;
+            q += q & 0x38383838u;
+            sel[h] = q;
+        }
+        // digit d - 4 as E2M1: -4 .. 3 = E D C A 0 2 4 5; the even value's in the low nibble
+        lo[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0]) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1]);
+        hi[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0] >> 16) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1] >> 16);
+    }
+    const uint32_t at = (uint32_t)(lane >> 2), in = (uint32_t)(lane & 3) * 4u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t* s = h ? hi : lo;
+        const uint32_t a = __byte_perm(s[0], s[1], 0x5140), b = __byte_perm(s[2], s[3], 0x5140);
+        const uint32_t c = __byte_perm(s[0], s[1], 0x7362), d = __byte_perm(s[2], s[3], 0x7362);
+        const uint32_t w[4] = {__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(c, d, 0x5410), __byte_perm(c, d, 0x7632)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) *(uint32_t*)(codes + (4 * h + j) * 128 + ((at ^ (uint32_t)(4 * h + j)) << 4) + in) = w[j];
+    }
+    const uint32_t under = emax - e;  // 0..17: 2^8 .. 2^-9, the last three subnormal
+    uint32_t sw = (under <= 14u ? (15u - under) << 3 : 32u >> (under - 12u)) << (8 * ((lane >> 1) & 3));
+    sw |= __shfl_xor_sync(0xffffffffu, sw, 2);
+    sw |= __shfl_xor_sync(0xffffffffu, sw, 4);
+    const int n = n0 + (lane & 7);
+    *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
+    if (lane == 0) *fs = make_float2(__uint_as_float((emax - 8u) << 23), __uint_as_float(slow_lanes));  // 2^(Emax - 8)
+}
+
+// one block of 16 values from global memory: sum of code x activation, times the block's scale
+__device__ __noinline__ float slow_block(const uint8_t* wblk, int sub, const __nv_bfloat16* x) {
+    float sum = 0.0f;
+    for (int i = 0; i < 16; i++) {
+        const uint32_t b = wblk[4 + sub * 8 + (i >> 1)], n = (i & 1) ? b >> 4 : b & 15u, c = n & 7u;
+        const float v = c < 2u ? 0.5f * (float)c : __uint_as_float(((126u + (c >> 1)) << 23) | ((c & 1u) << 22));
+        const uint32_t xb = __ldcg((const unsigned short*)x + i);
+        sum = fmaf((n & 8u) ? -v : v, __uint_as_float(xb << 16), sum);
+    }
+    return sum * ue4m3_f32(wblk[sub], true);
+}
+
+template <int MT>
+__global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
+                                                                   const TcParams p) {
+    constexpr int N = ncol(MT), NB = nb_of(MT), B_STAGE = b_stage(MT);
+    constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = 2 * N, SFB_COL = 2 * N + 32;
+    static_assert(2 * N + 64 <= tmem_cols(MT), "tensor memory columns");
+    extern __shared__ uint8_t smem[];
+    uint64_t* raw_full = (uint64_t*)smem;
+    uint64_t* raw_empty = raw_full + MAX_RAW;
+    uint64_t* a_full = raw_empty + MAX_RAW;   // [NA]
+    uint64_t* xbar = a_full + NA;            // [NX] digits of a chunk
+    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk
+    uint64_t* d_empty = done + NDONE;         // [2] accumulators
+    uint64_t* exbar = d_empty + 2;            // [2] sums handed over
+    uint32_t* tmem_slot = (uint32_t*)(exbar + 2);
+    float2* fs = (float2*)(smem + FS_OFF);    // [NX][8]
+    uint32_t* wf = (uint32_t*)(smem + WF_OFF);  // [NX][4]
+    const uint32_t base = (smem_u32(smem) + HEADER + 1023u) & ~1023u;
+    uint8_t* a0 = smem + (base - smem_u32(smem));
+    uint8_t* b0 = a0 + NA * A_STAGE;
+    uint8_t* r0 = b0 + NB * B_STAGE;
+    const int R = p.raw;
+    float* ex = (float*)(r0 + (size_t)R * RAW_STAGE);
+    const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
+    const int C = p.csize, rank = C > 1 ? (int)cluster_rank() : 0;
+    const int cid = (int)blockIdx.x / C, ncl = (int)gridDim.x / C;
+    const int nk = p.k / CH, ck0 = rank * nk / C, nc = (rank + 1) * nk / C - ck0;
+    const int ntl = (p.tiles - cid + ncl - 1) / ncl, total = ntl * nc;
+    const bool gu = p.w1 != nullptr;
+    const int per_tile = gu ? 64 : 128;
+
+    auto load = [&](int s, int tile, int chunk, uint64_t pol) {
+        mbar_expect_tx(&raw_full[s], RAW_STAGE);
+        mbar_arrive(&raw_full[s]);
+        const uint32_t dst = smem_u32(r0) + (uint32_t)(s * RAW_STAGE), bar = smem_u32(&raw_full[s]);
+        tma_load_2d_hint(dst, &map0, chunk * 36, tile * per_tile, bar, pol);
+        if (gu) tma_load_2d_hint(dst + RAW_STAGE / 2, &map1, chunk * 36, tile * per_tile, bar, pol);
+    };
+    if (warp == LOADER) {
+        // a barrier a lane: container stages, operand stages, digits, finished chunks, accumulators, sums handed over
+        for (int i = lane; i < NBAR; i += 32)
+            mbar_init(raw_full + i, i < MAX_RAW ? 1 : i < 2 * MAX_RAW + NA ? 4 : i < 2 * MAX_RAW + NA + NX ? (MT < 4 ? MT : 4) : i < NBAR - 4 ? 1 : i < NBAR - 2 ? EPI_WARPS : 1);
+        mbar_fence_init();
+        __syncwarp();
+        if (lane == 0) {
+            // the weights do not depend on the kernel in front: the first stages are asked for at once
+            const uint64_t pol = l2_policy_evict_first();
+            for (int i = 0, tile = cid, c = 0; i < R && i < total; i++) {
+                load(i, tile, ck0 + c, pol);
+                if (++c == nc) c = 0, tile += ncl;
+            }
+        }
+        __syncwarp();
+    } else if (warp == ISSUER) {
+        tc_alloc<1>(tmem_slot, tmem_cols(MT));
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = warp_uniform(*tmem_slot);
+    if (C > 1) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+
+    if (warp == LOADER) {
+        // ------------------------------------------------------------ loads
+        if (lane == 0) {
+            const uint64_t pol = l2_policy_evict_first();
+            int s = 0, tile = cid, c = 0;
+            uint32_t par = 1;
+            for (int i = 0; i < total; i++) {
+                if (i >= R) {
+                    if (!mbar_wait(&raw_empty[s], par)) {
+                        cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                        for (int j = 0; j < R; j++) mbar_wait(&raw_full[j], ((uint32_t)((i - 1 - j) / R)) & 1u);  // copies in flight
+                        break;
+                    }
+                    load(s, tile, ck0 + c, pol);
+                }
+                // The next kernel may start when only three loads of this one are left: its weights then stream while this one drains. Earlier, its first
+                // loads would hold up the last ones here (16384 x 2048: 6.9 us a call, 5.6 so; 4096 x 8192 7.5 and 6.3; behind the last load 6.1 and 6.4).
+                // (Behind the allocation in any case: a kernel that starts early finds this one's tensor memory taken.)
+                if (i == max(total - 3, 0)) pdl_launch_dependents();
+                if (++c == nc) c = 0, tile += ncl;
+                if (++s == R) s = 0, par ^= 1u;
+            }
+        }
+        __syncwarp();
+    } else if (warp == ISSUER) {
+        // ------------------------------------------------------------ scale copies and MMAs
+        const uint32_t a_u = warp_uniform(smem_u32(a0)), b_u = warp_uniform(smem_u32(b0));
+        for (int i = 0; i < total; i++) {
+            const int a = i & 1, b = i % NB;
+            if (!mbar_wait(&a_full[a], (i >> 1) & 1)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            tc_after();
+            const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * A_STAGE)), db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
+            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_STAGE + A_CODES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + b_codes(MT)));
+            const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
+            if (elect_lane()) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) cp_sf(ta + 4 * j, sa + 32 * j);
+            }
+            __syncwarp();
+            if (!mbar_wait(&xbar[i % NX], (i / NX) & 1) || (i >= 2 && !mbar_wait(&d_empty[a], ((i >> 1) - 1) & 1))) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            tc_after();
+            if (elect_lane()) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) cp_sf(tb + 4 * j, sb + 32 * j);
+#pragma unroll
+                for (int j = 0; j < 4; j++) umma_bs(td, da + 2 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
+                tc_commit<1>(&done[i % NDONE]);
+            }
+            __syncwarp();
+        }
+    } else if (warp >= 8) {
+        // ------------------------------------------------------------ activations -> digits: a warp takes whole rows of a chunk
+        constexpr int CPR = MT < 4 ? 4 / MT : 1;  // chunks side by side in the four warps
+        constexpr int TPW = MT > 4 ? MT / 4 : 1;  // rows of a warp
+        const int w = warp - 8, myrow = MT < 4 ? w % MT : w, mychunk = MT < 4 ? w / MT : 0;
+        pdl_wait();  // the activations may come from the kernel before this one
+        uint4 nx[TPW];
+        int c = mychunk % nc;
+        auto fetch = [&]() {
+#pragma unroll
+            for (int t = 0; t < TPW; t++) {
+                const int row = myrow + 4 * t;
+                nx[t] = make_uint4(0u, 0u, 0u, 0u);
+                if (row < p.m) nx[t] = __ldcg((const uint4*)(p.x + (size_t)row * p.k + (size_t)(ck0 + c) * CH) + lane);
+            }
+            c += CPR;
+            while (c >= nc) c -= nc;
+        };
+        fetch();
+        for (int i = mychunk; i < total; i += CPR) {
+            uint4 now[TPW];
+#pragma unroll
+            for (int t = 0; t < TPW; t++) now[t] = nx[t];
+            fetch();
+            if (i >= NB && !mbar_wait(&done[(i - NB) % NDONE], ((i - NB) / NDONE) & 1)) {
+                cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                break;
+            }
+            uint8_t* bs = b0 + (i % NB) * B_STAGE;
+#pragma unroll
+            for (int t = 0; t < TPW; t++) {
+                const int row = myrow + 4 * t;  // (beyond p.m: zeros, in columns that nothing reads)
+                to_digits(now[t], lane, bs + row * 1024, bs + b_codes(MT), row * LV, &fs[(i % NX) * 8 + row]);
+            }
+            fence_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&xbar[i % NX]);
+        }
+    } else if (warp >= EPI_WARPS) {
+        // ------------------------------------------------------------ container blocks -> operand layout: a warp takes 32 rows, a lane the four
+        // blocks of a row (144 bytes: no bank twice among eight lanes, nor in the swizzled lines)
+        const int w = warp - 4;
+        int s = 0;
+        uint32_t par = 0;
+        for (int i = 0; i < total; i++) {
+            if (!mbar_wait(&raw_full[s], par)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + (w * 32 + lane) * 9;
+            uint32_t v[36];
+#pragma unroll
+            for (int j = 0; j < 9; j++) {
+                const uint4 q = src[j];
+                v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
+            }
+            uint32_t odd = 0u;
+#pragma unroll
+            for (int b = 0; b < 4; b++) odd |= v[9 * b] & ((v[9 * b] & 0x7f7f7f7fu) + 0x01010101u);
+            odd = __any_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const uint32_t sc = v[9 * b];
+                v[9 * b] = scale_bytes_rule(sc);
+                if (odd) {  // 0xFF stands for 480, which the tensor core does not know: nothing here, and the block is multiplied out below
+                    const uint32_t ff = sc & ((sc & 0x7f7f7f7fu) + 0x01010101u) & 0x80808080u;
+                    v[9 * b] &= ~(ff - (ff >> 7));
+                }
+            }
+            if (i >= NA && !mbar_wait(&done[(i - NA) % NDONE], ((i - NA) / NDONE) & 1)) {
+                cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                break;
+            }
+            uint8_t* dst = a0 + (i & 1) * A_STAGE;
+            uint8_t* line = dst + (w * 32 + lane) * 128;
+            const uint32_t sw = (uint32_t)(lane & 7);
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
+                *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
+                *(uint32_t*)(dst + A_CODES + b * 512 + lane * 16 + w * 4) = v[9 * b];
+            }
+            if (lane == 0) wf[(i % NX) * 4 + w] = odd;
+            fence_async();
+            __syncwarp();
+            // (the stage is given back here and not behind the loads: an arrival can overtake loads whose values nothing has used yet)
+            if (lane < 2) mbar_arrive(lane == 0 ? &a_full[i & 1] : &raw_empty[s]);
+            if (++s == R) s = 0, par ^= 1u;
+        }
+    } else {
+        // ------------------------------------------------------------ sums and output
+        pdl_wait();
+        const float gs = *(gu && warp >= 2 ? p.gs1 : p.gs0);
+        const unsigned int epoch = p.yl_world > 0 ? *(volatile const unsigned int*)p.yl_epoch : 0u;
+        const int r = warp * 32 + lane;  // this thread's row of the tile
+        float acc[MT];
+#pragma unroll
+        for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+        bool met = C == 1;
+        int c = 0, tile = cid, nt = 0;
+        for (int i = 0; i < total; i++) {
+            if (!mbar_wait(&done[i % NDONE], (i / NDONE) & 1) || !mbar_wait(&xbar[i % NX], (i / NX) & 1)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            tc_after();
+            const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i & 1));
+            const uint32_t odd = wf[(i % NX) * 4 + warp];
+            uint32_t slow = odd;
+            constexpr int G = MT < 4 ? MT : 4;  // rows at a time
+#pragma unroll
+            for (int m0 = 0; m0 < MT; m0 += G) {
+                uint32_t d[G * LV];
+#pragma unroll
+                for (int m = 0; m < G; m++) tc_ld8(td + LV * (m0 + m), d + LV * m);
+                tc_wait_ld();
+                if (m0 + G == MT) {
+                    tc_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&d_empty[i & 1]);
+                }
+#pragma unroll
+                for (int m = 0; m < G; m++) {
+                    float s = __uint_as_float(d[LV * m]);
+#pragma unroll
+                    for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                    const float2 f = fs[(i % NX) * 8 + m0 + m];
+                    acc[m0 + m] = fmaf(s * gs, f.x, acc[m0 + m]);
+                    slow |= __float_as_uint(f.y);
+                }
+            }
+            if (slow) {
+                const int row = tile * per_tile + (gu ? r & 63 : r);
+                if (row < p.rows) {
+                    const uint8_t* wr = (gu && r >= 64 ? p.w1 : p.w0) + ((size_t)row * nk + ck0 + c) * 144;
+#pragma unroll
+                    for (int m = 0; m < MT; m++) {
+                        if (m >= p.m) continue;
+                        const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
+                        for (int b = 0; b < 16; b++)
+                            if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
+                                acc[m] += slow_block(wr + (b >> 2) * 36, b & 3, p.x + (size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * gs;
+                    }
+                }
+            }
+            if (++c < nc) continue;
+            // the tile's last chunk of this part
+            if (C == 1 && !gu && p.yl_world == 0) {
+                const int row = tile * 128 + r;
+#pragma unroll
+                for (int m = 0; m < MT; m++)
+                    if (row < p.rows && m < p.m) {
+                        if (p.out_f32)
+                            ((float*)p.y)[(size_t)m * p.ldy + row] = acc[m];
+                        else
+                            ((__nv_bfloat16*)p.y)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(acc[m]);
+                    }
+            } else {
+                // CTA o of the cluster adds and stores the rows (pairs) [o, o + 1) x share of the tile. Two slots in turn: whoever sends a tile's sums has
+                // all of the tile before, whose senders had read the one before that.
+                const int q = p.share, half = gu ? r >> 6 : 0, at = gu ? r & 63 : r, o = at / q, halves = gu ? 2 : 1;
+                float* slot = ex + (nt & 1) * (ex_slot(MT) / 4);
+                float* mine = slot + (size_t)((rank * halves + half) * MT) * q + (at - o * q);
+                if (C == 1) {
+#pragma unroll
+                    for (int m = 0; m < MT; m++) mine[m * q] = acc[m];
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                } else {
+                    if (!met) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // every CTA of the cluster has its barriers
+                    met = true;
+                    const uint32_t there = cluster_addr(smem_u32(mine), (uint32_t)o), bar = cluster_addr(smem_u32(&exbar[nt & 1]), (uint32_t)o);
+#pragma unroll
+                    for (int m = 0; m < MT; m++)
+                        if (m < p.m) st_async_f32(there + (uint32_t)(m * q * 4), acc[m], bar);
+                    if (r == 0) {
+                        mbar_expect_tx(&exbar[nt & 1], (uint32_t)(C * halves * p.m * 4 * max(0, min(q, per_tile - rank * q))));
+                        mbar_arrive(&exbar[nt & 1]);
+                    }
+                    if (!wait_cluster(&exbar[nt & 1], (nt >> 1) & 1)) {
+                        cn_dev_fail(CN_DEV_WAIT_FULL);
+                        break;
+                    }
+                }
+                const int first = rank * q, have = min(q, per_tile - first);
+                for (int idx0 = 0; idx0 < q * p.m; idx0 += 128) {
+                    const int idx = idx0 + r, m = MT == 1 ? 0 : (int)(((uint32_t)idx * p.qinv) >> 20), lp = idx - m * q, row = tile * per_tile + first + lp;
+                    const bool live = m < p.m && lp < have && row < p.rows;
+                    float v = 0.0f;
+                    if (live) {
+                        float v1 = 0.0f;
+                        const float* from = slot + m * q + lp;
+                        const int step = halves * MT * q;
+                        float part[8];
+#pragma unroll
+                        for (int src = 0; src < 8; src++) part[src] = src < C ? from[src * step] : 0.0f;
+                        v = part[0];
+#pragma unroll
+                        for (int src = 1; src < 8; src++)
+                            if (src < C) v += part[src];
+                        if (gu) {
+#pragma unroll
+                            for (int src = 0; src < 8; src++) part[src] = src < C ? from[src * step + MT * q] : 0.0f;
+                            v1 = part[0];
+#pragma unroll
+                            for (int src = 1; src < 8; src++)
+                                if (src < C) v1 += part[src];
+                        }
+                        if (gu) v = act_gu(v, v1, p.limit);
+                        if (p.out_f32)
+                            ((float*)p.y)[(size_t)m * p.ldy + row] = v;
+                        else
+                            ((__nv_bfloat16*)p.y)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(v);
+                    }
+                    if (MT == 1 && p.yl_world > 0) {
+                        // four rows are one 16-byte line {rows 0-1, number, rows 2-3, number} in every peer's line buffer: plain stores, the receiver polls the number
+                        const uint32_t bits = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
+                        const uint32_t pair = bits | (__shfl_down_sync(0xffffffffu, bits, 1) << 16), next = __shfl_down_sync(0xffffffffu, pair, 2);
+                        const unsigned int seq = epoch * 4096u + (unsigned int)p.yl_tag, buf = (unsigned int)p.yl_buf ^ ((unsigned int)p.yl_flip & epoch & 1u);
+                        if (live && (lane & 3) == 0)
+                            for (int dst = 0; dst < p.yl_world; dst++)
+                                if (p.yl[dst] != 0ull) {
+                                    uint4* line = (uint4*)(uintptr_t)(p.yl[dst] + (unsigned long long)buf * p.yl_stride) + ((p.yl_row0 + row) >> 2);
+                                    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(line), "r"(pair), "r"(seq), "r"(next), "r"(seq) : "memory");
+                                }
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+            c = 0, tile += ncl, nt++;
+        }
+        tc_before();
+        if (C > 1) {
+            // A CTA that has had every sum sent to it may leave: nothing more comes. One that gave up waits for the others.
+            if (!met) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+            if (nt < ntl) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        }
+    }
+    if (C > 1 && warp >= EPI_WARPS) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    }
+    __syncthreads();
+    if (warp == ISSUER) tc_dealloc<1>(tmem, tmem_cols(MT));
+}
+
+// ---------------------------------------------------------------- launch
+const void* kernel_of(int mt) {
+    return mt == 1 ? (const void*)nvfp4_gemv_tc_kernel<1> : mt == 2 ? (const void*)nvfp4_gemv_tc_kernel<2> : mt == 4 ? (const void*)nvfp4_gemv_tc_kernel<4> : (const void*)nvfp4_gemv_tc_kernel<8>;
+}
+constexpr int SM_SHARE = (227 * 1024) / 2 - 1024;  // two CTAs per SM
+// (asked of a kernel of the same size without tensor memory: for one with it the runtime answers one CTA per SM, whatever its size)
+__global__ void __launch_bounds__(THREADS, 2) occupancy_kernel(int* out) {
+    extern __shared__ uint8_t smem[];
+    if (out) out[0] = smem[threadIdx.x];
+}
+
+// clusters of c CTAs that the current device holds at a time, two CTAs per SM: asked once per device (0: an error)
+int clusters_of(int c) {
+    static std::atomic<int> known[64][9];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    int n = dev < 64 ? known[dev][c].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        if (cn_allow_smem((const void*)occupancy_kernel, SM_SHARE) != cudaSuccess) return 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(c * 512)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SM_SHARE;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)c, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
+        cfg.attrs = at, cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, occupancy_kernel, &cfg) != cudaSuccess || n < 1) return 0;
+        if (dev < 64) known[dev][c].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// CTAs per cluster, a rule of the matrix alone, since it fixes the order of a row's sum: the least estimate of the time. A chunk takes a CTA 0.42 us, 0.62
+// from the ninth on (three stages of container bytes in flight), more where all CTAs together reach the memory's rate; the chunks are between those of
+// the busiest CTA and the mean; 0.3 for adding up a tile in a cluster, 0.3 where a second CTA per SM keeps the next kernel out. Measured, us with 1 / 2 / 4 /
+// 6 / 8 CTAs: 16384 x 2048 5.7 / 6.5 / 7.1 / 8.6 / 8.2, 8192 x 4096 9.5 / 6.2 / 6.5 / 7.2 / 7.4, 4096 x 8192 17.2 / 10.1 / 6.3 / 6.9 / 6.9, 7168 x 5120 11.5
+// / 7.2 / 6.9 / 7.7 / 8.0, 5120 x 17408 48 / 24 / 14.6 / 12.3 / 16.4, gate / up of 17408 x 5120 18.5 / 19.6 / 20.9 / 25 / 36. 3, 5 and 7 never were the fastest.
+int cut_of(int tiles, int nk) {
+    int best_c = 0;
+    double best = 1e30;
+    for (int c = 1; c <= 8 && c <= nk; c += c == 1 ? 1 : 2) {
+        const int n = clusters_of(c);
+        if (n < 1) return 0;
+        const int used = tiles < n ? tiles : n, ctas = used * c, waves = (tiles + n - 1) / n, part = (nk + c - 1) / c;
+        const double chunks = 0.5 * (waves * part + (double)tiles * nk / ctas), share = 0.0033 * ctas;
+        const double fast = share > 0.42 ? share : 0.42, slow = share > 0.62 ? share : 0.62;
+        const double t = fast * (chunks < 8 ? chunks : 8) + (chunks > 8 ? (chunks - 8) * slow : 0.0) + (c > 1 ? 0.3 * waves : 0.0) + (ctas > 148 ? 0.3 : 0.0);
+        if (t < best) best = t, best_c = c;
+    }
+    return best_c;
+}
+
+}  // namespace
+
+int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
+    const bool gu = a.w1 != nullptr;
+    const int m = a.m, mt = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
+    const int per_tile = gu ? 64 : 128, tiles = (a.rows + per_tile - 1) / per_tile, nk = a.k / CH;
+    const int c = cut_of(tiles, nk), ncl = clusters_of(c);
+    if (c < 1 || ncl < 1) CN_FAIL(CN_ERR_CUDA, "%s: the device does not say how many clusters it holds", who);
+    const int clusters = tiles < ncl ? tiles : ncl;
+    TcParams p = {};
+    p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = (const __nv_bfloat16*)a.x, p.y = a.y;
+    p.rows = a.rows, p.k = a.k, p.m = m, p.ldy = a.ldy, p.out_f32 = a.out_f32, p.limit = a.limit, p.csize = c, p.tiles = tiles;
+    p.share = ((per_tile + c - 1) / c + 3) & ~3;
+    p.qinv = ((1u << 20) + (uint32_t)p.share - 1u) / (uint32_t)p.share;
+    int raw = MAX_RAW;
+    while (smem_of(mt, raw) > SM_SHARE) raw--;
+    p.raw = raw;
+    if (a.line_bases) {
+        if (m != 1 || a.out_f32 || a.line_world < 2 || a.line_world > 8 || (a.rows & 3) || (a.line_row0 & 3) || !a.line_epoch || a.line_tag < 1 ||
+            a.line_tag > 4095 || (a.line_buf & ~1))
+            CN_FAIL(CN_ERR_SHAPE, "%s: line output needs one bf16 row, 2..8 ranks and row counts in multiples of 4 (rows %d, first row %d, ranks %d)", who,
+                    a.rows, a.line_row0, a.line_world);
+        p.yl_world = a.line_world, p.yl_row0 = a.line_row0, p.yl_stride = (unsigned long long)a.line_stride, p.yl_epoch = a.line_epoch;
+        p.yl_tag = a.line_tag, p.yl_buf = a.line_buf, p.yl_flip = a.line_flip ? 1 : 0;
+        for (int d = 0; d < a.line_world; d++) p.yl[d] = a.line_bases[d];
+    }
+    CUtensorMap map0, map1;
+    const unsigned long long row_bytes = (unsigned long long)nk * 144;
+    if (int rc = cn_tmap_2d(&map0, a.w0, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, (unsigned)per_tile)) return rc;
+    if (!gu)
+        map1 = map0;
+    else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
+        return rc;
+    // a CTA asks for no smaller a share of shared memory than of tensor memory: whatever fits an SM beside it finds tensor memory too
+    int smem = smem_of(mt, raw);
+    const int floor_bytes = mt == 8 ? SM_SHARE : (227 * 1024) / 4;
+    if (smem < floor_bytes) smem = floor_bytes;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * c)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = (size_t)smem, cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = 1;
+    if (c > 1) {
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = (unsigned)c, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
+    CN_ALLOW_SMEM(kernel_of(mt), SM_SHARE);
+    if (mt == 1) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<1>, map0, map1, p));
+    if (mt == 2) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<2>, map0, map1, p));
+    if (mt == 4) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<4>, map0, map1, p));
+    if (mt == 8) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<8>, map0, map1, p));
+    return CN_OK;
+}
