@@ -1,4 +1,4 @@
-// Device helpers of the kernels whose activation rows are MMA columns (nvfp4_gemv_col.cu, nvfp4_rows.cu): weights with their scale
+// Device helpers of the kernels whose activation rows are MMA columns (nvfp4_rows.cu, moe_step.cu): weights with their scale
 // applied in f16 (exact), f32 activations as three f16 planes.
 #pragma once
 #include "common.cuh"

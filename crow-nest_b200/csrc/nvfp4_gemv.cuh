@@ -106,11 +106,8 @@ __device__ __forceinline__ float act_gu(float g, float u, float limit) {
 // bf16 activation rows (1..8): persistent CTAs, tensor-core inner loop in word form (nvfp4_gemv_m1.cu)
 int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
-// bf16 activation rows (1..8) of a plain or gate / up call: tcgen05, block scale (nvfp4_gemv_tc.cu)
+// bf16 or f32 activation rows (1..8) of a plain or gate / up call: tcgen05, block scale (nvfp4_gemv_tc.cu)
 int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who);
-
-// f32 activation rows (1..8) as columns of the tensor-core tile, three f16 planes each (nvfp4_gemv_col.cu)
-int cn_gemv_col_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
 // Rows of activations in groups that share a matrix (nvfp4_rows.cu). Routed form: the *count1 one-row groups at pos1 (none when
 // count1 is null), then *count2 groups at pos2 of rows2 rows (up to eight bf16 or two f32 rows of one expert); positions are into

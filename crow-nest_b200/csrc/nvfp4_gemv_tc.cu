@@ -28,6 +28,7 @@
 #include "tc5.cuh"
 
 #include <atomic>
+#include <type_traits>
 
 namespace {
 
@@ -41,28 +42,26 @@ constexpr int NA = 2;       // chunks laid out for the tensor core
 constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 4;
 constexpr int EPI_WARPS = 4, LOADER = 12, ISSUER = 13;  // warps 0-3 sums and output, 4-7 weights, 8-11 activations
 constexpr int THREADS = 448;
-constexpr int LV = 8;       // digits of a value
 constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, slow blocks}; [NX][4] scale bytes of 0xFF seen
-__host__ __device__ constexpr int ncol(int mt) { return mt * LV < 16 ? 16 : mt * LV; }      // columns of the MMA
-__host__ __device__ constexpr int b_codes(int mt) { return ncol(mt) * 128; }
-__host__ __device__ constexpr int b_stage(int mt) { return b_codes(mt) + 4 * 512; }
-__host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                 // chunks of digits
-__host__ __device__ constexpr int ex_slot(int mt) { return 168 * mt * 4; }                  // sums of a tile handed over: 128 rows, shares rounded up to 4
-__host__ __device__ constexpr int tmem_cols(int mt) { return mt <= 4 ? 128 : 256; }
-__host__ __device__ constexpr int smem_of(int mt, int raw) {
-    return HEADER + 1024 + NA * A_STAGE + nb_of(mt) * b_stage(mt) + raw * RAW_STAGE + 2 * ex_slot(mt);
-}
+__host__ __device__ constexpr int digits_of(bool f32) { return f32 ? 10 : 8; }
+__host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_of(f32) + 15) / 16 * 16; }  // columns of the MMA
+__host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
+__host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
+__host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                                // chunks of digits
+__host__ __device__ constexpr int tmem_cols(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 <= 128 ? 128 : 256; }
+__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * A_STAGE + nb_of(mt) * b_stage(mt, f32); }
 
 struct TcParams {
     const uint8_t* w0;
     const uint8_t* w1;  // gate / up: up
     const float* gs0;
     const float* gs1;
-    const __nv_bfloat16* x;
+    const void* x;
     void* y;
     int rows, k, m, ldy, out_f32;
     float limit;
     uint32_t qinv;                 // 2^20 / share, rounded up: idx / share for idx < 1024
+    int ex_bytes;                  // a slot of sums handed over
     int csize, tiles, raw, share;  // CTAs per cluster, row tiles, container stages, rows (or pairs) of a tile that a CTA stores
     unsigned long long yl[8];
     int yl_world, yl_row0;
@@ -93,6 +92,9 @@ __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* v) {
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tc_ld2(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar, uint64_t policy) {
     asm volatile(
@@ -103,6 +105,10 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
 // a value into another CTA's shared memory, counted there on a barrier of the same CTA
 __device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t bar) { st_async_f32(addr, v, bar); }
+__device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(__double_as_longlong(v)), "r"(bar) : "memory");
 }
 __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {  // bounded, with cluster-scope acquire
     const long long t0 = clock64();
@@ -121,32 +127,52 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity) {  
 }
 
 // ---------------------------------------------------------------- 256 values of an activation row as digits (a warp; a lane holds eight values)
-// codes: the row's eight lines of the B tile (line j = digit j), 1024 bytes; sf: the scales of the four MMAs, n0 the row's first column.
-// With E the exponent of the block's largest value, a value is q x 2^(E - 21), |q| <= 2^22: its digits are the octal digits of q + 44444444 (octal), less
-// four each. The scale byte is 2^(8 - (Emax - E)), Emax that of the chunk.
-__device__ __forceinline__ void to_digits(uint4 raw, int lane, uint8_t* codes, uint8_t* sf, int n0, float2* fs) {
-    uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-    uint32_t top = __vmaxu2(__vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu));
-    top = max(top >> 16, top & 0xffffu);
+// bs: the B tile; the row's lines are `row` x the digits of a value + j for digit j. With E the exponent of a block's largest value, a value is
+// q x 2^(E - 21), |q| <= 2^22 (f32: q x 2^(E - 27), |q| <= 2^28): its digits are the octal digits of q + 44444444 (octal; f32: ten fours), less four
+// each. The scale byte is 2^(8 - (Emax - E)), Emax that of the chunk.
+template <bool F32>
+__device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* bs, uint8_t* sf, int row, float2* fs) {
+    constexpr int LV = digits_of(F32);
+    constexpr uint32_t LEAST = F32 ? 28u : 22u;  // biased exponent below which the scale of a block would be no number
+    uint32_t u[F32 ? 8 : 4], top;
+    u[0] = raw[0].x, u[1] = raw[0].y, u[2] = raw[0].z, u[3] = raw[0].w;
+    if constexpr (F32) {
+        u[4] = raw[1].x, u[5] = raw[1].y, u[6] = raw[1].z, u[7] = raw[1].w;
+        top = u[0] & 0x7fffffffu;
+#pragma unroll
+        for (int i = 1; i < 8; i++) top = max(top, u[i] & 0x7fffffffu);
+    } else {
+        top = __vmaxu2(__vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu));
+        top = max(top >> 16, top & 0xffffu);
+    }
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));  // two lanes hold a block of 16
-    uint32_t e = top >> 7;
-    const bool odd = top != 0u && (e < 22u || e == 255u);  // below 2^-105 (a scale of its digits would be no number), infinity, NaN
-    const uint32_t emax = max(__reduce_max_sync(0xffffffffu, odd ? 0u : e), 22u);
+    uint32_t e = top >> (F32 ? 23 : 7);
+    const bool odd = top != 0u && (e < LEAST || e == 255u);  // too small, infinity, NaN
+    const uint32_t emax = max(__reduce_max_sync(0xffffffffu, odd ? 0u : e), LEAST);
     const bool slow = odd || (top != 0u && emax - e > 17u);
     const uint32_t slow_lanes = __ballot_sync(0xffffffffu, slow);
     if (slow || top == 0u) {
         e = emax;
-        u[0] = u[1] = u[2] = u[3] = 0u;
+#pragma unroll
+        for (int i = 0; i < (F32 ? 8 : 4); i++) u[i] = 0u;
     }
-    const float scale = __uint_as_float((275u - e) << 23);  // 2^(21 - (e - 127))
-    uint32_t lo[4], hi[4];  // value pair p: byte j = digits j (hi: 4 + j) of both
+    const float scale = __uint_as_float(((F32 ? 281u : 275u) - e) << 23);  // 2^(21 - (e - 127)), f32: 27
+    uint32_t lo[4], hi[4], over[4];  // value pair p: byte j = digits j (hi: 4 + j; over: 8 + j) of both
 #pragma unroll
     for (int p = 0; p < 4; p++) {
-        uint32_t sel[2];
+        uint32_t sel[2], up[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const float v = __uint_as_float(h ? u[p] & 0xffff0000u : u[p] << 16);
-            uint32_t q = __float_as_uint(fmaf(v, scale, 12582912.0f)) + (044444444u - 0x4b400000u);  // (q + 2^22 is the sum's mantissa: rounded to nearest even)
+            uint32_t q;
+            if constexpr (F32) {
+                q = (uint32_t)(__float2int_rn(__uint_as_float(u[2 * p + h]) * scale) + 04444444444);
+                up[h] = q >> 24;
+                up[h] += up[h] & 0x38u;
+                q &= 0x00ffffffu;
+            } else {
+                const float v = __uint_as_float(h ? u[p] & 0xffff0000u : u[p] << 16);
+                q = __float_as_uint(fmaf(v, scale, 12582912.0f)) + (044444444u - 0x4b400000u);  // (q + 2^22 is the sum's mantissa: rounded to nearest even)
+            }
             q += (q & 0x00fff000u) * 15u;  // octal digits apart: four to sixteen bits, two to eight, one to four
             q += (q & 0x0fc00fc0u) * 3u;
             q += q & 0x38383838u;
@@ -155,44 +181,69 @@ __device__ __forceinline__ void to_digits(uint4 raw, int lane, uint8_t* codes, u
         // digit d - 4 as E2M1: -4 .. 3 = E D C A 0 2 4 5; the even value's in the low nibble
         lo[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0]) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1]);
         hi[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0] >> 16) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1] >> 16);
+        if constexpr (F32) {
+            const uint32_t c = __byte_perm(0x0A0C0D0Eu, 0x05040200u, up[0] | (up[1] << 8));  // even 8, even 9, odd 8, odd 9
+            over[p] = c | (c >> 12);
+        }
     }
     const uint32_t at = (uint32_t)(lane >> 2), in = (uint32_t)(lane & 3) * 4u;
+    auto put = [&](int j, uint32_t w) {
+        if constexpr (F32) {
+            const uint32_t n = (uint32_t)(row * LV + j), r = n & 7u;
+            *(uint32_t*)(bs + n * 128u + ((at ^ r) << 4) + in) = w;
+        } else {
+            *(uint32_t*)(bs + row * 1024 + j * 128 + ((at ^ (uint32_t)j) << 4) + in) = w;
+        }
+    };
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const uint32_t* s = h ? hi : lo;
         const uint32_t a = __byte_perm(s[0], s[1], 0x5140), b = __byte_perm(s[2], s[3], 0x5140);
         const uint32_t c = __byte_perm(s[0], s[1], 0x7362), d = __byte_perm(s[2], s[3], 0x7362);
-        const uint32_t w[4] = {__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(c, d, 0x5410), __byte_perm(c, d, 0x7632)};
-#pragma unroll
-        for (int j = 0; j < 4; j++) *(uint32_t*)(codes + (4 * h + j) * 128 + ((at ^ (uint32_t)(4 * h + j)) << 4) + in) = w[j];
+        put(4 * h, __byte_perm(a, b, 0x5410));
+        put(4 * h + 1, __byte_perm(a, b, 0x7632));
+        put(4 * h + 2, __byte_perm(c, d, 0x5410));
+        put(4 * h + 3, __byte_perm(c, d, 0x7632));
+    }
+    if constexpr (F32) {
+        const uint32_t a = __byte_perm(over[0], over[1], 0x5140), b = __byte_perm(over[2], over[3], 0x5140);
+        put(8, __byte_perm(a, b, 0x5410));
+        put(9, __byte_perm(a, b, 0x7632));
     }
     const uint32_t under = emax - e;  // 0..17: 2^8 .. 2^-9, the last three subnormal
     uint32_t sw = (under <= 14u ? (15u - under) << 3 : 32u >> (under - 12u)) << (8 * ((lane >> 1) & 3));
     sw |= __shfl_xor_sync(0xffffffffu, sw, 2);
     sw |= __shfl_xor_sync(0xffffffffu, sw, 4);
-    const int n = n0 + (lane & 7);
+    int n = row * LV + (lane & 7);
     *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
+    if (F32 && (lane & 7) < LV - 8) {
+        n += 8;
+        *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
+    }
     if (lane == 0) *fs = make_float2(__uint_as_float((emax - 8u) << 23), __uint_as_float(slow_lanes));  // 2^(Emax - 8)
 }
 
 // one block of 16 values from global memory: sum of code x activation, times the block's scale
-__device__ __noinline__ float slow_block(const uint8_t* wblk, int sub, const __nv_bfloat16* x) {
+template <bool F32>
+__device__ __noinline__ float slow_block(const uint8_t* wblk, int sub, const void* x) {
     float sum = 0.0f;
     for (int i = 0; i < 16; i++) {
         const uint32_t b = wblk[4 + sub * 8 + (i >> 1)], n = (i & 1) ? b >> 4 : b & 15u, c = n & 7u;
         const float v = c < 2u ? 0.5f * (float)c : __uint_as_float(((126u + (c >> 1)) << 23) | ((c & 1u) << 22));
-        const uint32_t xb = __ldcg((const unsigned short*)x + i);
-        sum = fmaf((n & 8u) ? -v : v, __uint_as_float(xb << 16), sum);
+        const float xv = F32 ? __ldcg((const float*)x + i) : __uint_as_float((uint32_t)__ldcg((const unsigned short*)x + i) << 16);
+        sum = fmaf((n & 8u) ? -v : v, xv, sum);
     }
     return sum * ue4m3_f32(wblk[sub], true);
 }
 
-template <int MT>
+template <int MT, bool F32>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                                                                    const TcParams p) {
-    constexpr int N = ncol(MT), NB = nb_of(MT), B_STAGE = b_stage(MT);
+    constexpr int LV = digits_of(F32), ES = F32 ? 4 : 2;
+    constexpr int N = ncol(MT, F32), NB = nb_of(MT), B_STAGE = b_stage(MT, F32), B_CODES = b_codes(MT, F32);
+    using Acc = typename std::conditional<F32, double, float>::type;
     constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = 2 * N, SFB_COL = 2 * N + 32;
-    static_assert(2 * N + 64 <= tmem_cols(MT), "tensor memory columns");
+    static_assert(2 * N + 64 <= tmem_cols(MT, F32), "tensor memory columns");
     extern __shared__ uint8_t smem[];
     uint64_t* raw_full = (uint64_t*)smem;
     uint64_t* raw_empty = raw_full + MAX_RAW;
@@ -209,7 +260,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint8_t* b0 = a0 + NA * A_STAGE;
     uint8_t* r0 = b0 + NB * B_STAGE;
     const int R = p.raw;
-    float* ex = (float*)(r0 + (size_t)R * RAW_STAGE);
+    uint8_t* ex = r0 + (size_t)R * RAW_STAGE;
     const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
     const int C = p.csize, rank = C > 1 ? (int)cluster_rank() : 0;
     const int cid = (int)blockIdx.x / C, ncl = (int)gridDim.x / C;
@@ -241,7 +292,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
         __syncwarp();
     } else if (warp == ISSUER) {
-        tc_alloc<1>(tmem_slot, tmem_cols(MT));
+        tc_alloc<1>(tmem_slot, tmem_cols(MT, F32));
     }
     tc_before();
     __syncthreads();
@@ -284,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             }
             tc_after();
             const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * A_STAGE)), db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
-            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_STAGE + A_CODES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + b_codes(MT)));
+            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_STAGE + A_CODES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
             const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
             if (elect_lane()) {
 #pragma unroll
@@ -311,23 +362,29 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         constexpr int TPW = MT > 4 ? MT / 4 : 1;  // rows of a warp
         const int w = warp - 8, myrow = MT < 4 ? w % MT : w, mychunk = MT < 4 ? w / MT : 0;
         pdl_wait();  // the activations may come from the kernel before this one
-        uint4 nx[TPW];
+        constexpr int XR = F32 ? 2 : 1;           // 16-byte pieces of a lane's eight values
+        uint4 nx[TPW][XR];
         int c = mychunk % nc;
         auto fetch = [&]() {
 #pragma unroll
             for (int t = 0; t < TPW; t++) {
                 const int row = myrow + 4 * t;
-                nx[t] = make_uint4(0u, 0u, 0u, 0u);
-                if (row < p.m) nx[t] = __ldcg((const uint4*)(p.x + (size_t)row * p.k + (size_t)(ck0 + c) * CH) + lane);
+#pragma unroll
+                for (int q = 0; q < XR; q++) {
+                    nx[t][q] = make_uint4(0u, 0u, 0u, 0u);
+                    if (row < p.m) nx[t][q] = __ldcg((const uint4*)((const char*)p.x + ((size_t)row * p.k + (size_t)(ck0 + c) * CH) * ES) + lane * XR + q);
+                }
             }
             c += CPR;
             while (c >= nc) c -= nc;
         };
         fetch();
         for (int i = mychunk; i < total; i += CPR) {
-            uint4 now[TPW];
+            uint4 now[TPW][XR];
 #pragma unroll
-            for (int t = 0; t < TPW; t++) now[t] = nx[t];
+            for (int t = 0; t < TPW; t++)
+#pragma unroll
+                for (int q = 0; q < XR; q++) now[t][q] = nx[t][q];
             fetch();
             if (i >= NB && !mbar_wait(&done[(i - NB) % NDONE], ((i - NB) / NDONE) & 1)) {
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
@@ -337,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
             for (int t = 0; t < TPW; t++) {
                 const int row = myrow + 4 * t;  // (beyond p.m: zeros, in columns that nothing reads)
-                to_digits(now[t], lane, bs + row * 1024, bs + b_codes(MT), row * LV, &fs[(i % NX) * 8 + row]);
+                to_digits<F32>(now[t], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
             }
             fence_async();
             __syncwarp();
@@ -397,12 +454,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     } else {
         // ------------------------------------------------------------ sums and output
         pdl_wait();
-        const float gs = *(gu && warp >= 2 ? p.gs1 : p.gs0);
+        const float gs0 = *p.gs0, gs1 = gu ? *p.gs1 : 0.0f, gs = gu && warp >= 2 ? gs1 : gs0;
         const unsigned int epoch = p.yl_world > 0 ? *(volatile const unsigned int*)p.yl_epoch : 0u;
         const int r = warp * 32 + lane;  // this thread's row of the tile
-        float acc[MT];
+        Acc acc[MT];  // f32 rows: without the tensor scale
 #pragma unroll
-        for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+        for (int m = 0; m < MT; m++) acc[m] = 0;
         bool met = C == 1;
         int c = 0, tile = cid, nt = 0;
         for (int i = 0; i < total; i++) {
@@ -414,12 +471,15 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i & 1));
             const uint32_t odd = wf[(i % NX) * 4 + warp];
             uint32_t slow = odd;
-            constexpr int G = MT < 4 ? MT : 4;  // rows at a time
+            constexpr int G = F32 ? (MT < 2 ? MT : 2) : (MT < 4 ? MT : 4);  // rows at a time
 #pragma unroll
             for (int m0 = 0; m0 < MT; m0 += G) {
                 uint32_t d[G * LV];
 #pragma unroll
-                for (int m = 0; m < G; m++) tc_ld8(td + LV * (m0 + m), d + LV * m);
+                for (int m = 0; m < G; m++) {
+                    tc_ld8(td + LV * (m0 + m), d + LV * m);
+                    if (F32) tc_ld2(td + LV * (m0 + m) + 8, d + LV * m + 8);
+                }
                 tc_wait_ld();
                 if (m0 + G == MT) {
                     tc_before();
@@ -428,11 +488,26 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 }
 #pragma unroll
                 for (int m = 0; m < G; m++) {
-                    float s = __uint_as_float(d[LV * m]);
-#pragma unroll
-                    for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
                     const float2 f = fs[(i % NX) * 8 + m0 + m];
-                    acc[m0 + m] = fmaf(s * gs, f.x, acc[m0 + m]);
+                    float s = __uint_as_float(d[LV * m]);
+                    if constexpr (F32) {
+                        // what the last three additions round off is kept; the chunks are added in 64 bits
+                        float rest = 0.0f;
+#pragma unroll
+                        for (int j = 1; j < LV - 3; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+#pragma unroll
+                        for (int j = LV - 3; j < LV; j++) {
+                            const float a = s * 0.125f, b = __uint_as_float(d[LV * m + j]);
+                            s = a + b;
+                            const float bb = s - a;
+                            rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
+                        }
+                        acc[m0 + m] += ((double)s + (double)rest) * (double)f.x;
+                    } else {
+#pragma unroll
+                        for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                        acc[m0 + m] = fmaf(s * gs, f.x, acc[m0 + m]);
+                    }
                     slow |= __float_as_uint(f.y);
                 }
             }
@@ -446,7 +521,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                         const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
                         for (int b = 0; b < 16; b++)
                             if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
-                                acc[m] += slow_block(wr + (b >> 2) * 36, b & 3, p.x + (size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * gs;
+                                acc[m] += slow_block<F32>(wr + (b >> 2) * 36, b & 3, (const char*)p.x + ((size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * ES) * (F32 ? 1.0f : gs);
                     }
                 }
             }
@@ -457,7 +532,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
                 for (int m = 0; m < MT; m++)
                     if (row < p.rows && m < p.m) {
-                        if (p.out_f32)
+                        if (F32)
+                            ((float*)p.y)[(size_t)m * p.ldy + row] = (float)(acc[m] * gs);
+                        else if (p.out_f32)
                             ((float*)p.y)[(size_t)m * p.ldy + row] = acc[m];
                         else
                             ((__nv_bfloat16*)p.y)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(acc[m]);
@@ -466,8 +543,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 // CTA o of the cluster adds and stores the rows (pairs) [o, o + 1) x share of the tile. Two slots in turn: whoever sends a tile's sums has
                 // all of the tile before, whose senders had read the one before that.
                 const int q = p.share, half = gu ? r >> 6 : 0, at = gu ? r & 63 : r, o = at / q, halves = gu ? 2 : 1;
-                float* slot = ex + (nt & 1) * (ex_slot(MT) / 4);
-                float* mine = slot + (size_t)((rank * halves + half) * MT) * q + (at - o * q);
+                Acc* slot = (Acc*)(ex + (nt & 1) * p.ex_bytes);
+                Acc* mine = slot + (size_t)((rank * halves + half) * MT) * q + (at - o * q);
                 if (C == 1) {
 #pragma unroll
                     for (int m = 0; m < MT; m++) mine[m * q] = acc[m];
@@ -478,9 +555,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                     const uint32_t there = cluster_addr(smem_u32(mine), (uint32_t)o), bar = cluster_addr(smem_u32(&exbar[nt & 1]), (uint32_t)o);
 #pragma unroll
                     for (int m = 0; m < MT; m++)
-                        if (m < p.m) st_async_f32(there + (uint32_t)(m * q * 4), acc[m], bar);
+                        if (m < p.m) st_async(there + (uint32_t)(m * q * (int)sizeof(Acc)), acc[m], bar);
                     if (r == 0) {
-                        mbar_expect_tx(&exbar[nt & 1], (uint32_t)(C * halves * p.m * 4 * max(0, min(q, per_tile - rank * q))));
+                        mbar_expect_tx(&exbar[nt & 1], (uint32_t)(C * halves * p.m * (int)sizeof(Acc) * max(0, min(q, per_tile - rank * q))));
                         mbar_arrive(&exbar[nt & 1]);
                     }
                     if (!wait_cluster(&exbar[nt & 1], (nt >> 1) & 1)) {
@@ -494,31 +571,27 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                     const bool live = m < p.m && lp < have && row < p.rows;
                     float v = 0.0f;
                     if (live) {
-                        float v1 = 0.0f;
-                        const float* from = slot + m * q + lp;
+                        const Acc* from = slot + m * q + lp;
                         const int step = halves * MT * q;
-                        float part[8];
+                        auto add_up = [&](const Acc* at0, float scale) -> float {
+                            Acc part[8];
 #pragma unroll
-                        for (int src = 0; src < 8; src++) part[src] = src < C ? from[src * step] : 0.0f;
-                        v = part[0];
-#pragma unroll
-                        for (int src = 1; src < 8; src++)
-                            if (src < C) v += part[src];
-                        if (gu) {
-#pragma unroll
-                            for (int src = 0; src < 8; src++) part[src] = src < C ? from[src * step + MT * q] : 0.0f;
-                            v1 = part[0];
+                            for (int src = 0; src < 8; src++) part[src] = src < C ? at0[src * step] : (Acc)0;
+                            Acc sum = part[0];
 #pragma unroll
                             for (int src = 1; src < 8; src++)
-                                if (src < C) v1 += part[src];
-                        }
+                                if (src < C) sum += part[src];
+                            return F32 ? (float)(sum * scale) : (float)sum;
+                        };
+                        v = add_up(from, gs0);
+                        const float v1 = gu ? add_up(from + MT * q, gs1) : 0.0f;
                         if (gu) v = act_gu(v, v1, p.limit);
-                        if (p.out_f32)
+                        if (F32 || p.out_f32)
                             ((float*)p.y)[(size_t)m * p.ldy + row] = v;
                         else
                             ((__nv_bfloat16*)p.y)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(v);
                     }
-                    if (MT == 1 && p.yl_world > 0) {
+                    if (MT == 1 && !F32 && p.yl_world > 0) {
                         // four rows are one 16-byte line {rows 0-1, number, rows 2-3, number} in every peer's line buffer: plain stores, the receiver polls the number
                         const uint32_t bits = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
                         const uint32_t pair = bits | (__shfl_down_sync(0xffffffffu, bits, 1) << 16), next = __shfl_down_sync(0xffffffffu, pair, 2);
@@ -533,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 }
             }
 #pragma unroll
-            for (int m = 0; m < MT; m++) acc[m] = 0.0f;
+            for (int m = 0; m < MT; m++) acc[m] = 0;
             c = 0, tile += ncl, nt++;
         }
         tc_before();
@@ -549,13 +622,10 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     }
     __syncthreads();
-    if (warp == ISSUER) tc_dealloc<1>(tmem, tmem_cols(MT));
+    if (warp == ISSUER) tc_dealloc<1>(tmem, tmem_cols(MT, F32));
 }
 
 // ---------------------------------------------------------------- launch
-const void* kernel_of(int mt) {
-    return mt == 1 ? (const void*)nvfp4_gemv_tc_kernel<1> : mt == 2 ? (const void*)nvfp4_gemv_tc_kernel<2> : mt == 4 ? (const void*)nvfp4_gemv_tc_kernel<4> : (const void*)nvfp4_gemv_tc_kernel<8>;
-}
 constexpr int SM_SHARE = (227 * 1024) / 2 - 1024;  // two CTAs per SM
 // (asked of a kernel of the same size without tensor memory: for one with it the runtime answers one CTA per SM, whatever its size)
 __global__ void __launch_bounds__(THREADS, 2) occupancy_kernel(int* out) {
@@ -603,25 +673,35 @@ int cut_of(int tiles, int nk) {
     return best_c;
 }
 
+template <int MT, bool F32>
+int launch_tc(const cudaLaunchConfig_t& cfg, const CUtensorMap& map0, const CUtensorMap& map1, const TcParams& p) {
+    CN_ALLOW_SMEM((nvfp4_gemv_tc_kernel<MT, F32>), SM_SHARE);
+    CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<MT, F32>, map0, map1, p));
+    return CN_OK;
+}
+
 }  // namespace
 
 int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
-    const bool gu = a.w1 != nullptr;
+    const bool gu = a.w1 != nullptr, f32 = a.dtype == CN_F32;
     const int m = a.m, mt = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
     const int per_tile = gu ? 64 : 128, tiles = (a.rows + per_tile - 1) / per_tile, nk = a.k / CH;
     const int c = cut_of(tiles, nk), ncl = clusters_of(c);
     if (c < 1 || ncl < 1) CN_FAIL(CN_ERR_CUDA, "%s: the device does not say how many clusters it holds", who);
     const int clusters = tiles < ncl ? tiles : ncl;
     TcParams p = {};
-    p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = (const __nv_bfloat16*)a.x, p.y = a.y;
+    p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = a.x, p.y = a.y;
     p.rows = a.rows, p.k = a.k, p.m = m, p.ldy = a.ldy, p.out_f32 = a.out_f32, p.limit = a.limit, p.csize = c, p.tiles = tiles;
     p.share = ((per_tile + c - 1) / c + 3) & ~3;
     p.qinv = ((1u << 20) + (uint32_t)p.share - 1u) / (uint32_t)p.share;
-    int raw = MAX_RAW;
-    while (smem_of(mt, raw) > SM_SHARE) raw--;
-    p.raw = raw;
+    // sums handed over: a slot per tile in flight, two where a CTA has several tiles
+    p.ex_bytes = c > 1 || gu || a.line_bases ? c * (gu ? 2 : 1) * p.share * mt * (f32 ? 8 : 4) : 0;
+    const int front = fixed_smem(mt, f32) + (tiles > clusters ? 2 : 1) * p.ex_bytes;
+    p.raw = (SM_SHARE - front) / RAW_STAGE;
+    if (p.raw > MAX_RAW) p.raw = MAX_RAW;
+    if (p.raw < 1) CN_FAIL(CN_ERR_LIMIT, "%s: %d rows in clusters of %d leave no room for weights", who, m, c);
     if (a.line_bases) {
-        if (m != 1 || a.out_f32 || a.line_world < 2 || a.line_world > 8 || (a.rows & 3) || (a.line_row0 & 3) || !a.line_epoch || a.line_tag < 1 ||
+        if (m != 1 || f32 || a.out_f32 || a.line_world < 2 || a.line_world > 8 || (a.rows & 3) || (a.line_row0 & 3) || !a.line_epoch || a.line_tag < 1 ||
             a.line_tag > 4095 || (a.line_buf & ~1))
             CN_FAIL(CN_ERR_SHAPE, "%s: line output needs one bf16 row, 2..8 ranks and row counts in multiples of 4 (rows %d, first row %d, ranks %d)", who,
                     a.rows, a.line_row0, a.line_world);
@@ -637,8 +717,8 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
         return rc;
     // a CTA asks for no smaller a share of shared memory than of tensor memory: whatever fits an SM beside it finds tensor memory too
-    int smem = smem_of(mt, raw);
-    const int floor_bytes = mt == 8 ? SM_SHARE : (227 * 1024) / 4;
+    int smem = front + p.raw * RAW_STAGE;
+    const int floor_bytes = tmem_cols(mt, f32) == 256 ? SM_SHARE : (227 * 1024) / 4;
     if (smem < floor_bytes) smem = floor_bytes;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * c)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = (size_t)smem, cfg.stream = stream;
@@ -651,10 +731,6 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         at[1].val.clusterDim.x = (unsigned)c, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
     }
-    CN_ALLOW_SMEM(kernel_of(mt), SM_SHARE);
-    if (mt == 1) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<1>, map0, map1, p));
-    if (mt == 2) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<2>, map0, map1, p));
-    if (mt == 4) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<4>, map0, map1, p));
-    if (mt == 8) CN_CUDA(cudaLaunchKernelEx(&cfg, nvfp4_gemv_tc_kernel<8>, map0, map1, p));
-    return CN_OK;
+    if (f32) return mt == 1 ? launch_tc<1, true>(cfg, map0, map1, p) : mt == 2 ? launch_tc<2, true>(cfg, map0, map1, p) : mt == 4 ? launch_tc<4, true>(cfg, map0, map1, p) : launch_tc<8, true>(cfg, map0, map1, p);
+    return mt == 1 ? launch_tc<1, false>(cfg, map0, map1, p) : mt == 2 ? launch_tc<2, false>(cfg, map0, map1, p) : mt == 4 ? launch_tc<4, false>(cfg, map0, map1, p) : launch_tc<8, false>(cfg, map0, map1, p);
 }

@@ -1,8 +1,8 @@
 // Routed-expert NVFP4 rows: groups of activation rows of one expert as the columns of the tensor-core tile, one warp per tile.
 //
 // Supersedes gemv_fp4_ptrb over the pointer tables (engine/src/kernels.rs:195-233) together with the grouping idea of the
-// reference's prefill path (moe_count / moe_plan / moe_scatter, engine/src/kernels.rs:3334-3420). Arithmetic as in
-// nvfp4_gemv_col.cu: weights with their scale in f16 (exact), f32 rows as three f16 planes, f32 sums.
+// reference's prefill path (moe_count / moe_plan / moe_scatter, engine/src/kernels.rs:3334-3420). Arithmetic: weights
+// with their scale in f16 (exact), f32 rows as three f16 planes, f32 sums.
 //
 // An expert's matrices are small (2048 x 512: a row is 288 bytes), so what a GEMV kernel spends per tile - handing sums between
 // warps, staging and scale tables per CTA - outweighs the tile. Here a warp keeps a 16-row tile to itself: it brings the tile in
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) nvfp4_rows_kernel(const RowsPara
         };
         for (int i = 0; i < D; i++) issue();
 
-        // the group's rows: eight lanes per 64-value block; column, block and chunk order as in nvfp4_gemv_col.cu
+        // the group's rows: eight lanes per 64-value block; column, block and chunk order as nvfp4_col.cuh reads them
         const int ncol = NPL * nrows;
         for (int r = 0; r < nrows; r++) {
             const int combo = member(r);

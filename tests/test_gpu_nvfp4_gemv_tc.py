@@ -1,4 +1,4 @@
-"""The GEMV on the fifth-generation tensor cores (matrices of eight million weights and more), against 64 bits: clusters of one to eight CTAs, one tile of 128
+"""The GEMV on the fifth-generation tensor cores (bf16 rows: matrices of eight million weights and more), against 64 bits: clusters of one to eight CTAs, one tile of 128
 rows to a CTA and several, parts of unequal length, rows that end inside a tile, every number of activation rows; activations of any magnitude, not finite
 ones, and scale bytes that the tensor core reads differently. Every row has the bits of a one-row call."""
 import numpy as np
@@ -41,6 +41,53 @@ def test_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
     for i in range(m):
         assert torch.equal(call(x[i:i + 1]).view(torch.int16)[0], y.view(torch.int16)[i]), i
     assert device_status() == 0
+
+
+# f32: any number of rows from k = 2048 on, six million weights and more below; a CTA with one container stage (8200 x 4096: two tiles in clusters, eight rows)
+@pytest.mark.parametrize("rows,k,gu", [(64, 2048, False), (130, 4608, False), (1100, 8192, False), (12300, 512, False), (40000, 256, False), (20000, 4096, False), (5120, 17408, False),
+                                       (3000, 1024, True), (1000, 2304, True)])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8])
+def test_f32_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
+    rng, g, g64 = _make(rows, k, rows + k, 2.0 ** -10)  # (a power of two: the weights themselves are exact in f32)
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda()
+    want, call = x.double() @ g64.t(), lambda v: ops.launch_gemv(g, v)
+    # one rounding to f32 (2^-24 of each result at most) and digits that end at 2^-28 of their block's largest value, the largest of sixteen being some two
+    # times their root mean square; an activation behind it adds a handful of f32 roundings (expf two ulp, divide, two products)
+    bound = 2.0 ** -24 + 2.0 ** -27
+    if gu:
+        _, u, u64 = _make(rows, k, rows + k + 1, 2.0 ** -10)
+        want, call, bound = want / (1 + torch.exp(-want)) * (x.double() @ u64.t()), lambda v: ops.launch_gemv_gu(g, u, v), 8 * 2.0 ** -23
+    y = call(x)
+    assert (y.double() - want).norm() <= bound * want.norm()
+    for i in range(m):
+        assert torch.equal(call(x[i:i + 1]).view(torch.int32)[0], y.view(torch.int32)[i]), i
+    assert device_status() == 0
+
+
+def test_f32_rows_of_any_magnitude():
+    rng, w, w64 = _make(300, 4096, 8, 1.0)
+    x = rng.standard_normal((8, 4096)).astype(np.float32)
+    x[0] *= 2.0 ** -90
+    x[1] *= 2.0 ** 90
+    x[2, ::16] *= 1e4
+    x[3] *= np.exp2(rng.integers(-60, 60, 256).repeat(16)).astype(np.float32)
+    x[4] *= np.exp2(rng.integers(-20, 1, 4096)).astype(np.float32)
+    x[5, 300:] = 0.0
+    x[6] *= 2.0 ** -118
+    x[7, 9], x[7, 4000] = np.inf, np.nan
+    xd = torch.from_numpy(x).cuda()
+    y, want = ops.launch_gemv(w, xd), xd.double() @ w64.t()
+    for i in range(7):
+        # blocks multiplied out on their own are sums of 16 f32 products
+        assert (y[i].double() - want[i]).norm() <= (2.0 ** -23 if i in (3, 6) else 2.0 ** -24 + 2.0 ** -26) * want[i].norm(), i
+    assert y[7].isnan().all() and device_status() == 0
+
+
+def test_a_row_too_long_is_refused():
+    from crownest_b200 import CrownestError
+    w = ops.Fp4(torch.zeros(108800 // 64 * 36, dtype=torch.uint8, device="cuda"), torch.ones(1, device="cuda"), 1, 108800)
+    with pytest.raises(CrownestError, match="108544"):
+        ops.launch_gemv(w, torch.zeros((1, 108800), device="cuda"))
 
 
 def test_rows_of_any_magnitude():
@@ -90,7 +137,7 @@ def test_scale_bytes_that_the_tensor_core_reads_differently():
     s = w.w.view(8192 * 16, 36)[:, :4]
     pick = torch.from_numpy(rng.integers(0, 50, (8192 * 16, 4))).cuda()
     s[pick == 0], s[pick == 1], s[pick == 2] = 0x7F, 0xFF, 0xB5
-    w64 = ops.dequant(w).double().view(8192, 1024)
+    w64 = ops.dequant(w, rule=True).double().view(8192, 1024)
     assert float(w64.abs().max()) == pytest.approx(6 * 480e-3)
     x = torch.from_numpy(rng.standard_normal((5, 1024)).astype(np.float32)).cuda().to(torch.bfloat16)
     _near(ops.launch_gemv(w, x), x.double() @ w64.t())
