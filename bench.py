@@ -327,7 +327,7 @@ def moe_measure(kind, tokens, rank, world, local, steps, warmup, cpu=False, e2e=
                "tok_s": tokens * world / (ms * 1e-3), "ms_per_step": ms, "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"],
                "ms_per_step_max": t["ms_per_step_max"], "distinct_experts": distinct, "algorithmic_bytes": nbytes,
                "roofline": {"bound": "hbm", "achieved": gbs / world, "peak": peak, "unit": "GB/s", "frac": gbs / world / peak, "peak_kind": peak_kind,
-                            "scope": "per GPU", "kernel": "mul1_gemv_kernel" if kind != "moe" else "nvfp4_rows_kernel" if tokens * wl.topk >= 48 else "nvfp4_gemv_m1_kernel (routed form)"},
+                            "scope": "per GPU", "kernel": "mul1_gemv_kernel" if kind != "moe" else "nvfp4_rows_tc_kernel" if tokens * wl.topk >= 48 else "nvfp4_gemv_m1_kernel (routed form)"},
                "parallelism": f"ep{world}: all-to-all dispatch / return over peer memory" if world > 1 else "none",
                "launches_per_step": wl.launches_per_step, "device_status": status}
         if e2e_s is not None:

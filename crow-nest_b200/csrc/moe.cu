@@ -77,20 +77,17 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 //   ga[] / counts[0]  positions (in order[]) of the one-row groups: an expert's single row, or the one left over after
 //                     its groups of gmax
 //   gb[], gbrows[] / counts[1]  first positions and row counts (2..gmax) of the other groups
-//   gd[], gdrows[] / counts[2]  the same runs cut into groups of one or two rows (for f32 activations, which take three
-//                     of an MMA's eight columns each: three f16 planes)
 // Placement is done by one warp walking the combos in order (match.any finds the lanes of a step that share an expert),
 // so the sort stays stable without ranking every combo against all others.
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,
                                                          int32_t* __restrict__ order, int* __restrict__ ga, int* __restrict__ gb,
-                                                         int* __restrict__ gbrows, int* __restrict__ gd, int* __restrict__ gdrows,
-                                                         int* __restrict__ counts, int gmax) {
+                                                         int* __restrict__ gbrows, int* __restrict__ counts, int gmax) {
     extern __shared__ int sm[];  // [E + 1] counts, [E + 1] starts, [E + 1] running, [n] bins
     int* cnt = sm;
     int* start = sm + (E + 1);
     int* run = sm + 2 * (E + 1);
     int* bin = sm + 3 * (E + 1);
-    __shared__ int wsa[32], wsb[32], wsd[32];
+    __shared__ int wsa[32], wsb[32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int i = tid; i <= E; i += blockDim.x) cnt[i] = 0;
@@ -105,36 +102,34 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     // per expert: one-row groups and larger groups, then three exclusive prefix sums over the experts (rows, a, b)
     const int per = (E + 1 + (int)blockDim.x - 1) / (int)blockDim.x;
     const int i0 = min(tid * per, E + 1), i1 = min(i0 + per, E + 1);
-    int rows = 0, na = 0, nb = 0, nd = 0;
+    int rows = 0, na = 0, nb = 0;
     for (int i = i0; i < i1; i++) {
         const int k = cnt[i];
         rows += k;
-        if (i < E) na += (k % gmax) == 1, nb += k / gmax + ((k % gmax) >= 2), nd += (k + 1) >> 1;
+        if (i < E) na += (k % gmax) == 1, nb += k / gmax + ((k % gmax) >= 2);
     }
-    int ir = rows, ia = na, ib = nb, id = nd;
+    int ir = rows, ia = na, ib = nb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int vr = __shfl_up_sync(0xffffffffu, ir, o), va = __shfl_up_sync(0xffffffffu, ia, o), vb = __shfl_up_sync(0xffffffffu, ib, o);
-        const int vd = __shfl_up_sync(0xffffffffu, id, o);
-        if (lane >= o) ir += vr, ia += va, ib += vb, id += vd;
+        if (lane >= o) ir += vr, ia += va, ib += vb;
     }
     __shared__ int wsr[32];
-    if (lane == 31) wsr[wid] = ir, wsa[wid] = ia, wsb[wid] = ib, wsd[wid] = id;
+    if (lane == 31) wsr[wid] = ir, wsa[wid] = ia, wsb[wid] = ib;
     __syncthreads();
     if (wid == 0) {
-        int r = wsr[lane], a = wsa[lane], b = wsb[lane], d = wsd[lane];
-        const int r0 = r, a0 = a, b0 = b, d0 = d;
+        int r = wsr[lane], a = wsa[lane], b = wsb[lane];
+        const int r0 = r, a0 = a, b0 = b;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int vr = __shfl_up_sync(0xffffffffu, r, o), va = __shfl_up_sync(0xffffffffu, a, o), vb = __shfl_up_sync(0xffffffffu, b, o);
-            const int vd = __shfl_up_sync(0xffffffffu, d, o);
-            if (lane >= o) r += vr, a += va, b += vb, d += vd;
+            if (lane >= o) r += vr, a += va, b += vb;
         }
-        wsr[lane] = r - r0, wsa[lane] = a - a0, wsb[lane] = b - b0, wsd[lane] = d - d0;
-        if (lane == 31) counts[0] = a, counts[1] = b, counts[2] = d;
+        wsr[lane] = r - r0, wsa[lane] = a - a0, wsb[lane] = b - b0;
+        if (lane == 31) counts[0] = a, counts[1] = b;
     }
     __syncthreads();
-    int pr = wsr[wid] + ir - rows, pa = wsa[wid] + ia - na, pb = wsb[wid] + ib - nb, pd = wsd[wid] + id - nd;
+    int pr = wsr[wid] + ir - rows, pa = wsa[wid] + ia - na, pb = wsb[wid] + ib - nb;
     for (int i = i0; i < i1; i++) {
         const int k = cnt[i];
         start[i] = pr;
@@ -144,7 +139,6 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
             const int rem = k % gmax, at = pr + k - rem;
             if (rem == 1) ga[pa++] = at;
             if (rem >= 2) gb[pb] = at, gbrows[pb] = rem, pb++;
-            for (int q = 0; q < k; q += 2) gd[pd] = pr + q, gdrows[pd] = k - q >= 2 ? 2 : 1, pd++;
         }
         pr += k;
     }
@@ -214,7 +208,7 @@ struct MoePlan {
     float* hs;       // [max_tokens][shared inter <= inter_s]
     float* ys;       // [max_tokens][hidden]
     int32_t* order;  // [max_tokens * topk]
-    int* groups;     // [5 * max_tokens * topk + 8]: the group lists of moe_group_kernel and their three counts
+    int* groups;     // [3 * max_tokens * topk + 8]: the group lists of moe_group_kernel and their two counts
     int shared_inter;
     // the shared expert does not depend on the routed experts until the combine: it is enqueued on a side stream
     // between two events (fork after the caller's earlier work, join before the combine), also under stream capture
@@ -225,14 +219,14 @@ struct MoePlan {
 
 }  // namespace
 
-// the grouping step for other operators of the library (declared in nvfp4_gemv.cuh): lists of `combos` ints each, counts of 3
+// the grouping step for other operators of the library (declared in nvfp4_gemv.cuh): lists of `combos` ints each, counts of 2
 int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int combos, int experts, int32_t* order, int* ga, int* gb, int* gbrows,
-                        int* gd, int* gdrows, int* counts, int gmax, cudaStream_t stream) {
+                        int* counts, int gmax, cudaStream_t stream) {
     if (gmax != 4 && gmax != 8) CN_FAIL(CN_ERR_SHAPE, "grouping: groups of %d rows (4 or 8)", gmax);
     const size_t smem = (size_t)(3 * (experts + 1) + combos) * sizeof(int);
     if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "grouping %d combos over %d experts needs %zu B of shared memory", combos, experts, smem);
     CN_ALLOW_SMEM(moe_group_kernel, 160 * 1024);
-    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1), dim3(1024), smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, gd, gdrows, counts, gmax));
+    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1), dim3(1024), smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax));
     return CN_OK;
 }
 
@@ -275,7 +269,7 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
     step(cudaMalloc(&p->hs, (size_t)max_tokens * (shared_inter > 0 ? shared_inter : 1) * sizeof(float)));
     step(cudaMalloc(&p->ys, (size_t)max_tokens * hidden * sizeof(float)));
     step(cudaMalloc(&p->order, combos * sizeof(int32_t)));
-    step(cudaMalloc(&p->groups, (5 * combos + 8) * sizeof(int)));
+    step(cudaMalloc(&p->groups, (3 * combos + 8) * sizeof(int)));
     step(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
     step(cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming));
     step(cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming));
@@ -307,6 +301,8 @@ int check_shared(const MoePlan* p, const void* shared_gate, const void* shared_u
     return CN_OK;
 }
 
+constexpr int MAX_ROW = 32768;  // values of a row in the kernel for groups of rows; longer ones are left to the GEMVs, which know their limits
+
 // the shared expert on every token, up to 8 rows per pass, on the plan's side stream between the fork and join events:
 // whatever happens after the fork, the side stream is joined again (a capture of the caller's stream stays valid)
 int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs, const void* x,
@@ -315,15 +311,15 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
     CN_CUDA(cudaStreamWaitEvent(p->side, p->fork, 0));
     const size_t es = dtype == CN_BF16 ? 2 : 4;
     int rc = CN_OK;
-    // More rows than a GEMV takes: both projections as one launch each over groups of rows (64 tokens, 512 x 2048: sixteen launches of
-    // 8 us each before, two of 24 and 12 us now; the step with the shared expert 297 -> 250 us).
-    RowsCall u = {}, d = {};
-    u.w0 = shared_gate, u.w1 = shared_up, u.m = tokens, u.gs0 = shared_gs, u.gs1 = shared_gs + 1, u.x = x, u.x_div = 1, u.x_f32 = dtype == CN_F32;
-    u.y = p->hs, u.ldy = p->shared_inter, u.rows = p->shared_inter, u.k = p->hidden, u.limit = limit, u.max_groups = (tokens + (u.x_f32 ? 1 : 7)) / (u.x_f32 ? 2 : 8);
-    d.w0 = shared_down, d.m = tokens, d.gs0 = shared_gs + 2, d.x = p->hs, d.x_div = 1, d.x_f32 = 1, d.y = p->ys, d.ldy = p->hidden, d.rows = p->hidden;
-    d.k = p->shared_inter, d.max_groups = (tokens + 1) / 2;
-    const bool grouped = tokens > CN_MAX_M && cn_rows_fits(u) && cn_rows_fits(d);
+    // More rows than a GEMV takes: both projections as one launch each over groups of eight rows (64 tokens, 512 x 2048: 22 and 11 us with the mma.sync kernel that
+    // took groups of eight bf16 or two f32 rows; the step 204 -> 199).
+    const bool grouped = tokens > CN_MAX_M && p->hidden <= MAX_ROW && p->shared_inter <= MAX_ROW;
     if (grouped) {
+        RowsCall u = {}, d = {};
+        u.w0 = shared_gate, u.w1 = shared_up, u.m = tokens, u.gs0 = shared_gs, u.gs1 = shared_gs + 1, u.x = x, u.x_div = 1, u.x_f32 = dtype == CN_F32;
+        u.y = p->hs, u.ldy = p->shared_inter, u.rows = p->shared_inter, u.k = p->hidden, u.limit = limit, u.max_groups = (tokens + 7) / 8;
+        d.w0 = shared_down, d.m = tokens, d.gs0 = shared_gs + 2, d.x = p->hs, d.x_div = 1, d.x_f32 = 1, d.y = p->ys, d.ldy = p->hidden, d.rows = p->hidden;
+        d.k = p->shared_inter, d.max_groups = (tokens + 7) / 8;
         rc = cn_rows_launch(u, p->side, "cn_moe_nvfp4_run (shared gate/up)");
         if (rc == CN_OK) rc = cn_rows_launch(d, p->side, "cn_moe_nvfp4_run (shared down)");
     }
@@ -346,7 +342,7 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
 
 // Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
 constexpr int GROUP_COMBOS = 48;
-// ... and from which the ungrouped down projection keeps a warp to a tile (measured: see routed_experts).
+// ... and from which the ungrouped down projection runs on the tensor cores (measured: see routed_experts).
 constexpr int ROWS_COMBOS = 16;
 // Units of work (16 result rows of a token x eight 64-value blocks of an expert) up to which a step of that many combos runs in two launches
 // (measured: see cn_moe_nvfp4_run).
@@ -369,50 +365,37 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
                    const float* gs_gu, const float* gs_up, const float* gs_dn, const int32_t* ids, const void* x, float* eo,
                    const unsigned long long* eo_ptrs, int combos, int x_div, float limit, int dtype, cudaStream_t stream) {
     const GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, combos, x_div, limit, dtype);
-    // From 48 combos on the combos are sorted by expert and cut into groups that share one decode of the expert's weights
-    // (nvfp4_rows.cu): the down projection in groups of up to two rows (its rows are f32), gate|up in groups of up to eight bf16 rows
-    // where enough of them share an expert (three combo slots for four experts), two f32 rows always. Measured, us per step of
-    // ungrouped / down grouped / both: 512 experts of 2048 x 512, top 10: 16 tokens 122 / 113 / 120, 64 tokens 444 / 325 / 297; 128
-    // experts of 2560 x 1280, top 6: 8 tokens 117 / 106 / 132, 32 tokens 390 / 306 / 267; 288 experts of 4096 x 2048, top 8: 16 tokens
-    // 515 / 401 / 440, 32 tokens 956 / 693 / 590; 64 tokens of f32 rows, 512 experts: 614 / 500 / 343. With 40 combos nothing is gained
-    // (48 / 48 / 59): the grouping is a launch of its own.
-    if (combos >= GROUP_COMBOS && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
+    const bool short_rows = p->hidden <= MAX_ROW && p->inter <= MAX_ROW;
+    // From 48 combos on the combos are sorted by expert and cut into groups of up to eight rows that share one pass over the expert's weights (nvfp4_rows_tc.cu).
+    // us per step (64 tokens, 512 experts of 2048 x 512, top 10, unless said otherwise) now / with mma.sync kernels that decoded the weights to f16 for eight bf16
+    // or two f32 rows: 199 / 213, 128 tokens 292 / 322, 16 tokens 95 / 110, f32 rows 207 / 232; 64 experts of 1024 x 1280, top 8, 108 tokens 156 / 190; 128 experts, f32,
+    // 100 tokens 218 / 291; 288 experts of 4096 x 2048, top 8, 10 tokens 198 / 239. With 40 combos nothing was gained (48 / 48 us): the grouping is a launch of its own.
+    if (combos >= GROUP_COMBOS && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
         int* ga = p->groups;
         int* gb = ga + combos;
         int* gbrows = gb + combos;
-        int* gd = gbrows + combos;
-        int* gdrows = gd + combos;
-        int* counts = gdrows + combos;
-        auto bound = [&](int rows) { return combos < p->experts + combos / rows ? combos : p->experts + combos / rows; };  // an expert ends in one short group
+        int* counts = gbrows + combos;
         RowsCall u = {};
         u.ids = ids, u.order = p->order, u.tab0 = table_gu, u.tab1 = table_up, u.fused_up_rows = a.fused_up_rows, u.gs0 = a.gs0, u.gs1 = a.gs1;
         u.x = x, u.x_div = x_div, u.x_f32 = dtype == CN_F32, u.y = p->h, u.ldy = p->inter, u.rows = p->inter, u.k = p->hidden, u.limit = limit;
-        u.max_groups = bound(u.x_f32 ? 2 : 8);
-        if (u.x_f32)
-            u.count2 = counts + 2, u.pos2 = gd, u.rows2 = gdrows;
-        else
-            u.count1 = counts, u.pos1 = ga, u.count2 = counts + 1, u.pos2 = gb, u.rows2 = gbrows;
+        u.max_groups = combos < p->experts + combos / 8 ? combos : p->experts + combos / 8;  // an expert ends in one short group
+        u.count1 = counts, u.pos1 = ga, u.count2 = counts + 1, u.pos2 = gb, u.rows2 = gbrows;
         RowsCall d = {};
         d.ids = ids, d.order = p->order, d.tab0 = table_dn, d.gs0 = gs_dn, d.x = p->h, d.x_div = 1, d.x_f32 = 1, d.y = eo, d.yptrs = eo_ptrs, d.ldy = p->hidden;
-        d.rows = p->hidden, d.k = p->inter, d.count2 = counts + 2, d.pos2 = gd, d.rows2 = gdrows, d.max_groups = bound(2);
-        if (cn_rows_fits(d)) {
-            if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, gd, gdrows, counts, 8, stream)) return rc;
-            if ((u.x_f32 || 4LL * combos >= 3LL * p->experts) && cn_rows_fits(u)) {
-                if (int rc = cn_rows_launch(u, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
-            } else if (int rc = cn_gemv_launch(a, stream, "cn_moe_nvfp4 (gate/up)")) {
-                return rc;
-            }
-            return cn_rows_launch(d, stream, "cn_moe_nvfp4 (down, grouped)");
-        }
+        d.rows = p->hidden, d.k = p->inter, d.max_groups = u.max_groups;
+        d.count1 = counts, d.pos1 = ga, d.count2 = counts + 1, d.pos2 = gb, d.rows2 = gbrows;
+        if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, counts, 8, stream)) return rc;
+        if (int rc = cn_rows_launch(u, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
+        return cn_rows_launch(d, stream, "cn_moe_nvfp4 (down, grouped)");
     }
     if (int rc = cn_gemv_launch(a, stream, "cn_moe_nvfp4 (gate/up)")) return rc;
-    // The down projection of 16 combos and more: the combos one by one, a warp per tile with f32 rows as f16 planes instead of FMAs.
-    // Measured, us per step with / without: 128 experts of 2560 x 1280, top 6, 4 tokens 60 / 76; 288 experts of 4096 x 2048, top 8, 5 tokens
-    // 158 / 171, 1 token 62 / 56; 64 experts of 2048 x 512, top 8, 4 tokens 38 / 42, 1 token 32 / 28.
+    // The down projection of 16 combos and more: the combos one by one, on the tensor cores instead of FMAs. us per step now / with the mma.sync kernel that kept a warp
+    // to a tile: 288 experts of 4096 x 2048, top 8, 5 tokens 136 / 142, 3 tokens 87 / 90; 64 experts of 2048 x 1280, top 8, 4 tokens 51.5 / 53.3. With FMAs (171 for the
+    // first) only fewer are faster: 1 token 56 / 62 with that kernel.
     RowsCall one = {};
     one.ids = ids, one.m = combos, one.tab0 = table_dn, one.gs0 = gs_dn, one.x = p->h, one.x_div = 1, one.x_f32 = 1, one.y = eo, one.yptrs = eo_ptrs;
     one.ldy = p->hidden, one.rows = p->hidden, one.k = p->inter, one.max_groups = combos, one.experts = p->experts;
-    if (combos >= ROWS_COMBOS && cn_rows_fits(one)) return cn_rows_launch(one, stream, "cn_moe_nvfp4 (down)");
+    if (combos >= ROWS_COMBOS && short_rows) return cn_rows_launch(one, stream, "cn_moe_nvfp4 (down)");
     GemvCall d = {};
     d.gs0 = gs_dn, d.x = p->h, d.y = eo, d.yptrs = eo_ptrs, d.rows = p->hidden, d.k = p->inter, d.m = 1, d.ldy = p->hidden, d.dtype = CN_F32, d.out_f32 = 1;
     d.x_f16_ok = 0, d.ids = ids, d.order = nullptr, d.tab0 = table_dn, d.x_div = 1, d.combos = combos, d.experts = p->experts;

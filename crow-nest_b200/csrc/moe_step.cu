@@ -1,6 +1,6 @@
 // The second half of a small routed-expert step in one launch: down projections of a token's experts and of the shared expert, and the
 // weighted combine. Supersedes gemv_fp4_ptrb over the down table, acc_combo and gate_shared (engine/src/kernels.rs:195-233, :1583-1599)
-// for steps of few combos; many share experts and run in groups instead (nvfp4_rows.cu).
+// for steps of few combos; many share experts and run in groups instead (nvfp4_rows_tc.cu).
 //
 // A CTA owns 16 rows of one token's result. Its work is cut into units - an expert's down matrix, eight 64-value blocks of k - and every
 // warp keeps its units to itself: it brings 16 row pieces in by its own bulk copies, cuts 512 values of h into f16 planes (three columns of

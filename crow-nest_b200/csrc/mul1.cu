@@ -566,7 +566,7 @@ struct Mul1Plan {
     float *part_a, *part_b;  // [slots][16][T][kmax]
     unsigned long long* ptrs;  // [slots] gathered record addresses (MoE form)
     int32_t* order;            // [slots] combos sorted by expert (grouped MoE form)
-    int* groups;               // [5 * slots + 8] the group lists and counts of cn_moe_group_launch
+    int* groups;               // [3 * slots + 8] the group lists and counts of cn_moe_group_launch
     int* rowsrc;               // [slots * MUL1_GT] x row of every (group slot, row), -1 = unused
     int* rowdst;               // [slots * MUL1_GT] combo (output row) of every (group slot, row), -1 = unused
     int* place;                // [slots] (group slot * rows + row) of every combo
@@ -705,7 +705,7 @@ extern "C" int cn_mul1_plan_create(void** plan_out, int hidden, int inter, int b
     step(cudaMalloc(&p->part_b, rows * 16 * p->kmax * 4));
     step(cudaMalloc(&p->ptrs, (size_t)max_slots * 8));
     step(cudaMalloc(&p->order, (size_t)max_slots * 4));
-    step(cudaMalloc(&p->groups, ((size_t)5 * max_slots + 8) * 4));
+    step(cudaMalloc(&p->groups, ((size_t)3 * max_slots + 8) * 4));
     step(cudaMalloc(&p->rowsrc, (size_t)max_slots * MUL1_GT * 4));
     step(cudaMalloc(&p->rowdst, (size_t)max_slots * MUL1_GT * 4));
     step(cudaMalloc(&p->place, (size_t)max_slots * 4));
@@ -820,10 +820,8 @@ int mul1_slots(Mul1Plan* p, const unsigned long long* table, const int32_t* ids,
             int* ga = p->groups;
             int* gb = ga + combos;
             int* gbrows = gb + combos;
-            int* gd = gbrows + combos;
-            int* gdrows = gd + combos;
-            int* counts = gdrows + combos;
-            if (int rc = cn_moe_group_launch(ids, table, combos, experts, p->order, ga, gb, gbrows, gd, gdrows, counts, gt, st)) return rc;
+            int* counts = gbrows + combos;
+            if (int rc = cn_moe_group_launch(ids, table, combos, experts, p->order, ga, gb, gbrows, counts, gt, st)) return rc;
             CN_CUDA(cn_launch_pdl(mul1_slots_kernel, dim3(((int)ng + 127) / 128), dim3(128), 0, st, table, ids, p->order, ga, gb, gbrows, counts, p->ptrs,
                                   p->rowsrc, p->rowdst, p->place, (int)ng, x_div, gt));
             // a slot beyond the groups is a null record, which all kernels skip; a group's unused rows are zero rows

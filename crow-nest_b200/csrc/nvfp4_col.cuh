@@ -1,4 +1,4 @@
-// Device helpers of the kernels whose activation rows are MMA columns (nvfp4_rows.cu, moe_step.cu): weights with their scale
+// Device helpers of the kernels whose activation rows are MMA columns (moe_step.cu): weights with their scale
 // applied in f16 (exact), f32 activations as three f16 planes.
 #pragma once
 #include "common.cuh"
@@ -35,7 +35,7 @@ __device__ __forceinline__ __half2 lane_scales(uint32_t w, uint32_t shift) {
 // A and B agree: lane (g, t) takes code words t and t + 4 of rows g (pa, the block's start + 4 t) and g + 8 (pb) - one 32-bit load of
 // eight codes feeds half of two MMAs - and x(ps, half) gives the matching eight activations of column g of group ps. A word's
 // eight values share a scale, so the two words' scales are made in one register (four instructions) and the multiplies take its halves
-// (a step of 64 tokens in nvfp4_rows.cu 258 us with one scale at a time, 245 with two).
+// (measured in a kernel for groups of rows: a step of 64 tokens 258 us with one scale at a time, 245 with two).
 template <int NP, typename X>
 __device__ __forceinline__ void block_mma(float (&cc)[NP][4], const uint8_t* pa, const uint8_t* pb, int t, X x) {
     const __half2 sa = lane_scales(*(const uint32_t*)(pa - 4 * t), 8u * (t >> 1)), sb = lane_scales(*(const uint32_t*)(pb - 4 * t), 8u * (t >> 1));
@@ -123,7 +123,7 @@ __device__ __forceinline__ float bf16_plane(const uint4& raw, int lane, uint32_t
 
 // ---------------------------------------------------------------- tiles of short rows, by their warp's own asynchronous copies
 // 16 row pieces of eight blocks (288 bytes) -> shared memory, PIECE_PITCH apart: nine 16-byte copies of each lane instead of a bulk copy for every
-// piece, whose number and not size is what the copy engine takes its time for (see nvfp4_rows.cu).
+// piece, whose number and not size is what the copy engine takes its time for.
 constexpr int PIECE_PITCH = 8 * 36 + 16, PIECE_TILE = 16 * PIECE_PITCH;
 struct PieceCopy {
     uint32_t at[9];  // copy i of this lane: row in the lower half, 16-byte part of the piece in the upper

@@ -44,10 +44,9 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
 // Sort combos by expert and cut every expert's run into groups (moe.cu): order [combos]; ga = positions (in order) of the
 // one-row groups, counts[0] of them; gb / gbrows = positions and row counts (2..gmax, gmax 4 or 8) of the larger groups,
-// counts[1]; gd / gdrows = the same runs cut into groups of one or two rows, counts[2]. Combos without a resident expert
-// are in no group.
+// counts[1]. Combos without a resident expert are in no group.
 int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int combos, int experts, int32_t* order, int* ga, int* gb, int* gbrows,
-                        int* gd, int* gdrows, int* counts, int gmax, cudaStream_t stream);
+                        int* counts, int gmax, cudaStream_t stream);
 
 // Kernel-side parameters shared by the CUDA-core and the tensor-core GEMV kernels.
 struct GemvParams {
@@ -109,8 +108,8 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 // bf16 or f32 activation rows (1..8) of a plain or gate / up call: tcgen05, block scale (nvfp4_gemv_tc.cu)
 int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
-// Rows of activations in groups that share a matrix (nvfp4_rows.cu). Routed form: the *count1 one-row groups at pos1 (none when
-// count1 is null), then *count2 groups at pos2 of rows2 rows (up to eight bf16 or two f32 rows of one expert); positions are into
+// Rows of activations in groups that share a matrix (nvfp4_rows_tc.cu). Routed form: the *count1 one-row groups at pos1 (none when
+// count1 is null), then *count2 groups at pos2 of rows2 rows (up to eight rows of one expert); positions are into
 // `order`; without `order`, m combos one by one. Dense form (w0 set): m rows of one matrix, or of a gate / up pair.
 struct RowsCall {
     const void *w0, *w1;
@@ -132,5 +131,4 @@ struct RowsCall {
     int max_groups;  // bound of the groups
     int experts;     // entries of the tables (0 = unknown: ids are trusted); an id beyond them skips the combo
 };
-bool cn_rows_fits(const RowsCall& a);
 int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who);

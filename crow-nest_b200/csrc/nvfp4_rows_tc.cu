@@ -1,0 +1,446 @@
+// NVFP4 matrices times groups of up to eight activation rows on tcgen05.mma kind::mxf4nvf4: the routed experts of a step (groups of rows of one expert) and the
+// shared expert of more rows than a GEMV takes. Supersedes gemv_fp4_ptrb over the pointer tables (engine/src/kernels.rs:195-233) together with the grouping
+// of the reference's prefill path (moe_count / moe_plan / moe_scatter, engine/src/kernels.rs:3334-3420). Arithmetic as in nvfp4_gemv_tc.cu: weights as they
+// are, rows as octal digits, chunks of 256 values of k added in order (f32, for f32 rows f64).
+//
+// Persistent CTAs, two per SM, walk units of (group, 128-row tile; 64 gate and 64 up rows). The matrices come from device tables, so there is no tensor map:
+// a scout warp looks up 32 units at a time (positions, combos, expert, addresses) and hands them to the other warps through a ring, and the warps that lay
+// the weights out for the tensor core bring them in themselves, by 16-byte asynchronous copies, past the ends of units. Warps: 0-3 add up and store,
+// 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form a warp's rows are 16 of gate and the same 16 of up.
+//
+// What bounds it: the way of the weights through a warp (gate / up of 64 tokens, 512 experts of 2048 x 512, top 10: 2150 cycles a chunk of 18 KB and CTA, 470 of
+// them loads, 500 stores and their fence, 580 the copies of a later chunk), 4.1 TB/s; us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16
+// or two f32 rows: gate / up 105 / 114, down 70 / 77. Tried: the same with a bulk copy for each row piece of 144 bytes 166 and 93; copies asked for
+// before the stores of the chunk in hand, one chunk less ahead, 109 and 79.
+#include "nvfp4_digits.cuh"
+#include "nvfp4_gemv.cuh"
+
+#include <type_traits>
+
+namespace {
+
+constexpr int RG = 8;        // most rows of a group
+constexpr int CH = 256;      // values of k in a chunk
+constexpr int A_CODES = 128 * 128, A_STAGE = A_CODES + 4 * 512;
+constexpr int PIECE = 32 * 144;  // container bytes of a warp's 32 rows and a chunk
+__host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 2 : 3; }  // chunks in flight, as many as fit
+constexpr int NA = 2, NB = 2, NX = 16, NDONE = 4, NU = 8;  // operand stages, chunks of digits, chunk factors, finished chunks, units in the ring
+constexpr int NBAR = NA + NX + NDONE + 2 + 2 * NU;
+constexpr int SCOUT = 12, ISSUER = 13, THREADS = 448;
+constexpr int FS_OFF = 512, WF_OFF = 1536, UNIT_OFF = 1792, HEADER = 2560;
+__host__ __device__ constexpr int ncol(bool f32) { return RG * digits_of(f32); }
+__host__ __device__ constexpr int b_stage(bool f32) { return ncol(f32) * 128 + 4 * 512; }
+__host__ __device__ constexpr int smem_of(bool f32) { return NA * A_STAGE + NB * b_stage(f32) + 4 * depth_of(f32) * PIECE + HEADER; }
+constexpr int SM_SHARE = (227 * 1024) / 2 - 1024;
+static_assert(smem_of(true) <= SM_SHARE && smem_of(false) <= SM_SHARE, "shared memory");
+
+struct Unit {
+    unsigned long long w0, w1;
+    int tile, nrows;  // nrows < 0: the end
+    int combo[RG];
+    int pad[2];
+};
+static_assert(sizeof(Unit) == 64 && UNIT_OFF + NU * 64 <= HEADER && NBAR * 8 + 8 <= FS_OFF, "header");
+
+template <bool F32>
+__global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCall c) {
+    constexpr int D = depth_of(F32), LV = digits_of(F32), ES = F32 ? 4 : 2, N = ncol(F32), B_CODES = N * 128, B_STAGE = b_stage(F32);
+    constexpr uint32_t SFA_COL = 2 * N, SFB_COL = 2 * N + 32, TMEM = 256;
+    static_assert(2 * N + 64 <= (int)TMEM, "tensor memory columns");
+    using Acc = typename std::conditional<F32, double, float>::type;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t *a0 = smem, *b0 = a0 + NA * A_STAGE, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;
+    uint64_t* a_full = (uint64_t*)head;       // [NA]
+    uint64_t* xbar = a_full + NA;             // [NX] digits of a chunk
+    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk
+    uint64_t* d_empty = done + NDONE;         // [2] accumulators
+    uint64_t* unit_full = d_empty + 2;        // [NU]
+    uint64_t* unit_empty = unit_full + NU;    // [NU]
+    uint32_t* tmem_slot = (uint32_t*)(unit_empty + NU);
+    float2* fs = (float2*)(head + FS_OFF);      // [NX][8] {factor, slow blocks}
+    uint32_t* wf = (uint32_t*)(head + WF_OFF);  // [NX][4] scale bytes of 0xFF seen
+    Unit* units = (Unit*)(head + UNIT_OFF);     // [NU]
+    const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
+    const bool gu = c.tab1 || c.w1 || c.fused_up_rows > 0;
+    const int nk = c.k / CH, per_tile = gu ? 64 : 128, T = (c.rows + per_tile - 1) / per_tile;
+    const size_t row_bytes = (size_t)nk * 144;
+
+    if (warp == SCOUT) {
+        // a barrier a lane and round: operand stages, digits, finished chunks, accumulators, units full and empty (four + four + four + one warps read them)
+        for (int i = lane; i < NBAR; i += 32)
+            mbar_init(a_full + i, i < NA + NX ? 4 : i < NA + NX + NDONE ? 1 : i < NA + NX + NDONE + 2 ? 4 : i < NBAR - NU ? 1 : 13);
+        mbar_fence_init();
+        __syncwarp();
+    } else if (warp == ISSUER) {
+        tc_alloc<1>(tmem_slot, TMEM);
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = warp_uniform(*tmem_slot);
+    pdl_launch_dependents();  // (behind the allocation of tensor memory)
+    pdl_wait();               // groups, ids and activations come from the kernels before this one
+
+    if (warp == SCOUT) {
+        // ------------------------------------------------------------ units: a lane looks one up, lane after lane hands them on
+        const int n1 = c.count1 ? *c.count1 : 0, ngroups = c.w0 ? (c.m + RG - 1) / RG : (c.order ? n1 + *c.count2 : c.m);
+        const long long total = (long long)ngroups * T;
+        int q = 0;
+        bool ok = true;
+        auto room = [&]() {  // the ring has a place for unit q
+            if (q >= NU && !mbar_wait(&unit_empty[q % NU], (uint32_t)(q / NU - 1) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                ok = false;
+            }
+            return ok;
+        };
+        for (long long u0 = blockIdx.x; u0 < total && ok; u0 += 32LL * gridDim.x) {
+            const long long u = u0 + (long long)lane * gridDim.x;
+            Unit mine = {};
+            bool valid = u < total;
+            if (valid) {
+                const int grp = (int)(u / T);
+                mine.tile = (int)(u - (long long)grp * T);
+                int pos = grp * RG;
+                mine.nrows = min(RG, c.m - pos), mine.w0 = (unsigned long long)c.w0, mine.w1 = (unsigned long long)c.w1;
+                if (!c.w0) {
+                    if (c.order)
+                        pos = grp < n1 ? c.pos1[grp] : c.pos2[grp - n1], mine.nrows = grp < n1 ? 1 : c.rows2[grp - n1];
+                    else
+                        pos = grp, mine.nrows = 1;  // the combos as they come
+                }
+#pragma unroll
+                for (int r = 0; r < RG; r++) mine.combo[r] = r < mine.nrows ? (c.order ? c.order[pos + r] : pos + r) : 0;
+                if (!c.w0) {
+                    const int e = c.ids[mine.combo[0]];
+                    valid = e >= 0 && !(c.experts > 0 && e >= c.experts);
+                    if (valid) {
+                        mine.w0 = c.tab0[e];
+                        mine.w1 = c.tab1 ? c.tab1[e] : (c.fused_up_rows > 0 && mine.w0 ? mine.w0 + (unsigned long long)c.fused_up_rows * row_bytes : 0ull);
+                        valid = mine.w0 && (!gu || mine.w1);  // (a matrix that is not resident: nothing to do)
+                    }
+                }
+            }
+            for (uint32_t left = __ballot_sync(0xffffffffu, valid); left && room(); left &= left - 1, q++) {
+                const int j = __ffs(left) - 1;
+                if (lane == j) {
+                    units[q % NU] = mine;
+                    mbar_arrive(&unit_full[q % NU]);
+                }
+                __syncwarp();
+            }
+        }
+        if (ok && room() && lane == 0) {
+            units[q % NU].nrows = -1;
+            mbar_arrive(&unit_full[q % NU]);
+        }
+        __syncwarp();
+    } else if (warp == ISSUER) {
+        // ------------------------------------------------------------ scale copies and MMAs
+        const uint32_t a_u = warp_uniform(smem_u32(a0)), b_u = warp_uniform(smem_u32(b0));
+        bool ok = true;
+        for (int q = 0, i = 0; ok; q++) {
+            if (!mbar_wait(&unit_full[q % NU], (uint32_t)(q / NU) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            const int nrows = (int)warp_uniform((uint32_t)units[q % NU].nrows);
+            if (nrows < 0) break;
+            const uint32_t idesc = idesc_bs((nrows * LV + 15) & ~15);
+            for (int ch = 0; ch < nk; ch++, i++) {
+                const int a = i & 1;
+                if (!mbar_wait(&a_full[a], (uint32_t)(i >> 1) & 1u) || !mbar_wait(&xbar[i % NX], (uint32_t)(i / NX) & 1u) ||
+                    (i >= 2 && !mbar_wait(&d_empty[a], (uint32_t)((i >> 1) - 1) & 1u))) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                    break;
+                }
+                tc_after();
+                const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * A_STAGE)), db = tc_desc_sw128(b_u + (uint32_t)(a * B_STAGE));
+                const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_STAGE + A_CODES)), sb = desc_sf(b_u + (uint32_t)(a * B_STAGE + B_CODES));
+                const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
+                if (elect_lane()) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        cp_sf(ta + 4 * j, sa + 32 * j);
+                        cp_sf(tb + 4 * j, sb + 32 * j);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; j++) umma_bs(td, da + 2 * j, db + 2 * j, idesc, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
+                    tc_commit<1>(&done[i % NDONE]);
+                }
+                __syncwarp();
+            }
+            if (lane == 0) mbar_arrive(&unit_empty[q % NU]);
+        }
+    } else if (warp >= 8) {
+        // ------------------------------------------------------------ activations -> digits: rows of a chunk and the next chunk's go round the four warps
+        constexpr int XR = F32 ? 2 : 1;
+        const int w = warp - 8;
+        int q = 0, ch = 0, nrows = 0;
+        uint4 nx[2][XR];
+        bool ok = true;
+        auto unit = [&](int n) -> int {  // rows of unit n
+            if (!mbar_wait(&unit_full[n % NU], (uint32_t)(n / NU) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                ok = false;
+                return -1;
+            }
+            return units[n % NU].nrows;
+        };
+        auto fetch = [&](int n, int rows, int chunk, int i) {
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const int row = ((w - i) & 3) + 4 * t;
+                if (row < rows) {
+                    const uint4* x = (const uint4*)((const char*)c.x + ((size_t)(units[n % NU].combo[row] / c.x_div) * c.k + (size_t)chunk * CH) * ES) + lane * XR;
+#pragma unroll
+                    for (int j = 0; j < XR; j++) nx[t][j] = __ldcg(x + j);
+                }
+            }
+        };
+        nrows = unit(0);
+        if (nrows >= 0) fetch(0, nrows, 0, 0);
+        for (int i = 0; nrows >= 0; i++) {
+            uint4 now[2][XR];
+#pragma unroll
+            for (int t = 0; t < 2; t++)
+#pragma unroll
+                for (int j = 0; j < XR; j++) now[t][j] = nx[t][j];
+            const int at = q;
+            int next_rows = nrows;
+            if (++ch == nk) ch = 0, q++, next_rows = unit(q);
+            if (next_rows >= 0) fetch(q, next_rows, ch, i + 1);
+            if (!ok) break;
+            if (i >= NB && !mbar_wait(&done[(i - NB) % NDONE], (uint32_t)((i - NB) / NDONE) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                break;
+            }
+            uint8_t* bs = b0 + (i % NB) * B_STAGE;
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const int row = ((w - i) & 3) + 4 * t;
+                if (row < nrows) to_digits<F32>(now[t], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
+            }
+            fence_async();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&xbar[i % NX]);
+                if (q != at) mbar_arrive(&unit_empty[at % NU]);
+            }
+            nrows = next_rows;
+        }
+    } else if (warp >= 4) {
+        // ------------------------------------------------------------ weights: 32 rows of the tile to a warp, copied in ahead and laid out as the A operand
+        const int w = warp - 4;
+        const uint32_t ring = smem_u32(r0) + (uint32_t)(w * D * PIECE);
+        const uint64_t pol = l2_policy_evict_first();
+        // sixteen-byte pieces, nine to a row and chunk, side by side in the stage; in the gate / up form rows 16-31 of a warp are the up rows of its gate rows
+        uint32_t off[9];
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            const int id = lane + 32 * j, row = id / 9;
+            off[j] = (uint32_t)(gu ? row & 15 : row) * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u;
+        }
+        int iq = 0, ic = 0, is = 0, have = 0;  // what is asked for next: unit, chunk, stage; rows there are
+        const uint8_t *from = nullptr, *from1 = nullptr;
+        bool more = true, ok = true;
+        auto issue = [&]() {
+            if (more && ic == 0) {
+                if (!mbar_wait(&unit_full[iq % NU], (uint32_t)(iq / NU) & 1u)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    more = ok = false;
+                } else {
+                    const Unit& u = units[iq % NU];
+                    more = u.nrows >= 0;
+                    const int first = u.tile * per_tile + w * (gu ? 16 : 32);
+                    from = (const uint8_t*)u.w0 + (size_t)first * row_bytes, from1 = (const uint8_t*)u.w1 + (size_t)first * row_bytes;
+                    have = min(max(c.rows - first, 0), gu ? 16 : 32);
+                }
+            }
+            if (more) {
+                const uint32_t dst = ring + (uint32_t)(is * PIECE + lane * 16);
+#pragma unroll
+                for (int j = 0; j < 9; j++) {
+                    const int row = (lane + 32 * j) / 9;
+                    const uint8_t* src = (gu && row >= 16 ? from1 : from) + off[j] + (uint32_t)(ic * 144);
+                    if ((gu ? row & 15 : row) < have)
+                        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"(src), "l"(pol) : "memory");
+                }
+                if (++is == D) is = 0;
+                if (++ic == nk) ic = 0, iq++;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll 1
+        for (int i = 0; i < D; i++) issue();
+        for (int q = 0, i = 0, s = 0; ok; q++) {
+            if (!mbar_wait(&unit_full[q % NU], (uint32_t)(q / NU) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            if (units[q % NU].nrows < 0) break;
+            for (int ch = 0; ch < nk; ch++, i++) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+                __syncwarp();  // the other lanes' copies, too
+                const uint4* src = (const uint4*)(r0 + (size_t)(w * D + s) * PIECE) + lane * 9;
+                uint32_t v[36];
+#pragma unroll
+                for (int j = 0; j < 9; j++) {
+                    const uint4 x = src[j];
+                    v[4 * j] = x.x, v[4 * j + 1] = x.y, v[4 * j + 2] = x.z, v[4 * j + 3] = x.w;
+                }
+                uint32_t odd = 0u;
+#pragma unroll
+                for (int b = 0; b < 4; b++) odd |= v[9 * b] & ((v[9 * b] & 0x7f7f7f7fu) + 0x01010101u);
+                odd = __any_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    const uint32_t sc = v[9 * b];
+                    v[9 * b] = scale_bytes_rule(sc);
+                    if (odd) {  // 0xFF stands for 480, which the tensor core does not know: nothing here, and the block is multiplied out below
+                        const uint32_t ff = sc & ((sc & 0x7f7f7f7fu) + 0x01010101u) & 0x80808080u;
+                        v[9 * b] &= ~(ff - (ff >> 7));
+                    }
+                }
+                if (i >= NA && !mbar_wait(&done[(i - NA) % NDONE], (uint32_t)((i - NA) / NDONE) & 1u)) {
+                    cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                    ok = false;
+                    break;
+                }
+                uint8_t* dst = a0 + (i & 1) * A_STAGE;
+                uint8_t* line = dst + (w * 32 + lane) * 128;
+                const uint32_t sw = (uint32_t)(lane & 7);
+#pragma unroll
+                for (int b = 0; b < 4; b++) {
+                    *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
+                    *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
+                    *(uint32_t*)(dst + A_CODES + b * 512 + lane * 16 + w * 4) = v[9 * b];
+                }
+                if (lane == 0) wf[(i % NX) * 4 + w] = odd;
+                fence_async();
+                __syncwarp();  // every lane has read the stage
+                if (lane == 0) mbar_arrive(&a_full[i & 1]);
+                issue();
+                if (++s == D) s = 0;
+            }
+            if (ok && lane == 0) mbar_arrive(&unit_empty[q % NU]);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        // ------------------------------------------------------------ sums and output: a thread is a row of the tile
+        const float gs0 = __ldg(c.gs0), gs1 = gu ? __ldg(c.gs1) : 0.0f, gs = gu && lane >= 16 ? gs1 : gs0;
+        bool ok = true;
+        for (int q = 0, i = 0; ok; q++) {
+            if (!mbar_wait(&unit_full[q % NU], (uint32_t)(q / NU) & 1u)) {
+                cn_dev_fail(CN_DEV_WAIT_FULL);
+                break;
+            }
+            const Unit& u = units[q % NU];
+            const int nrows = (int)warp_uniform((uint32_t)u.nrows), row = u.tile * per_tile + (gu ? warp * 16 + (lane & 15) : warp * 32 + lane);
+            if (nrows < 0) break;
+            Acc acc[RG];  // f32 rows: without the tensor scale
+#pragma unroll
+            for (int m = 0; m < RG; m++) acc[m] = 0;
+            for (int ch = 0; ch < nk; ch++, i++) {
+                if (!mbar_wait(&done[i % NDONE], (uint32_t)(i / NDONE) & 1u) || !mbar_wait(&xbar[i % NX], (uint32_t)(i / NX) & 1u)) {
+                    cn_dev_fail(CN_DEV_WAIT_FULL);
+                    ok = false;
+                    break;
+                }
+                tc_after();
+                const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i & 1));
+                const uint32_t odd = wf[(i % NX) * 4 + warp];
+                uint32_t slow = odd;
+#pragma unroll
+                for (int m0 = 0; m0 < RG; m0 += 2) {
+                    if (m0 >= nrows) break;
+                    uint32_t d[2 * LV];
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        tc_ld8(td + LV * (m0 + m), d + LV * m);
+                        if (F32) tc_ld2(td + LV * (m0 + m) + 8, d + LV * m + 8);
+                    }
+                    tc_wait_ld();
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        if (m0 + m >= nrows) break;
+                        const float2 f = fs[(i % NX) * 8 + m0 + m];
+                        float s = __uint_as_float(d[LV * m]);
+                        if constexpr (F32) {
+                            float rest = 0.0f;  // what the last three additions round off
+#pragma unroll
+                            for (int j = 1; j < LV - 3; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+#pragma unroll
+                            for (int j = LV - 3; j < LV; j++) {
+                                const float a = s * 0.125f, b = __uint_as_float(d[LV * m + j]);
+                                s = a + b;
+                                const float bb = s - a;
+                                rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
+                            }
+                            acc[m0 + m] += ((double)s + (double)rest) * (double)f.x;
+                        } else {
+#pragma unroll
+                            for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                            acc[m0 + m] = fmaf(s * gs, f.x, acc[m0 + m]);
+                        }
+                        slow |= __float_as_uint(f.y);
+                    }
+                }
+                tc_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&d_empty[i & 1]);
+                if (slow && row < c.rows) {
+                    const uint8_t* wr = (const uint8_t*)(gu && lane >= 16 ? u.w1 : u.w0) + ((size_t)row * nk + ch) * 144;
+#pragma unroll
+                    for (int m = 0; m < RG; m++) {
+                        if (m >= nrows) continue;
+                        const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
+                        for (int b = 0; b < 16; b++)
+                            if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
+                                acc[m] += slow_block<F32>(wr + (b >> 2) * 36, b & 3,
+                                                          (const char*)c.x + ((size_t)(u.combo[m] / c.x_div) * c.k + (size_t)ch * CH + b * 16) * ES) * (F32 ? 1.0f : gs);
+                    }
+                }
+            }
+            if (!ok) break;
+#pragma unroll
+            for (int m = 0; m < RG; m++) {
+                if (m >= nrows) break;
+                float v = F32 ? (float)(acc[m] * gs) : (float)acc[m];
+                if (gu) v = act_gu(v, __shfl_down_sync(0xffffffffu, v, 16), c.limit);
+                if (row >= c.rows || (gu && lane >= 16)) continue;
+                const int combo = u.combo[m];
+                float* y = c.yptrs ? (float*)c.yptrs[combo] : c.y + (size_t)combo * c.ldy;
+                y[row] = v;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&unit_empty[q % NU]);
+        }
+        tc_before();
+    }
+    __syncthreads();
+    if (warp == ISSUER) tc_dealloc<1>(tmem, TMEM);
+}
+
+}  // namespace
+
+int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
+    if (a.rows <= 0 || a.k <= 0 || a.k % 256 != 0) CN_FAIL(CN_ERR_SHAPE, "%s: k = %d must be a positive multiple of 256", who, a.k);
+    if (((uintptr_t)a.w0 | (uintptr_t)a.w1 | (uintptr_t)a.x) & 15)  // 16-byte asynchronous copies and 128-bit loads
+        CN_FAIL(CN_ERR_SHAPE, "%s: weight and activation pointers must be 16-byte aligned", who);
+    RowsCall p = a;
+    if (!p.gs1) p.gs1 = a.gs0;
+    const bool gu = a.tab1 || a.w1 || a.fused_up_rows > 0, f32 = a.x_f32 != 0;
+    const long long units = (long long)a.max_groups * ((a.rows + (gu ? 63 : 127)) / (gu ? 64 : 128));
+    const dim3 grid((unsigned)(units < 2 * 148 ? units : 2 * 148));
+    // (all of an SM's half, so that two CTAs and no more share its tensor memory)
+    if (f32) {
+        CN_ALLOW_SMEM(nvfp4_rows_tc_kernel<true>, SM_SHARE);
+        CN_CUDA(cn_launch_pdl(nvfp4_rows_tc_kernel<true>, grid, dim3(THREADS), SM_SHARE, stream, p));
+    } else {
+        CN_ALLOW_SMEM(nvfp4_rows_tc_kernel<false>, SM_SHARE);
+        CN_CUDA(cn_launch_pdl(nvfp4_rows_tc_kernel<false>, grid, dim3(THREADS), SM_SHARE, stream, p));
+    }
+    return CN_OK;
+}

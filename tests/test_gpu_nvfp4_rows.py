@@ -140,3 +140,39 @@ def test_combos_without_a_resident_expert_are_left_out(combos, experts, dtype):
     err = (eo.double() - want)[live].norm(dim=1) / want[live].norm(dim=1)
     assert err.max().item() <= 2e-6  # f32 throughout, as above
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("hidden,inter,tokens,experts", [(256, 256, 50, 2), (512, 256, 100, 3), (768, 1280, 49, 40)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_odd_scales_and_rows_that_are_not_finite(hidden, inter, tokens, experts, dtype):
+    """Scale bytes 0x7F and 0xFF, and an infinity and a NaN among the rows of a group: every other row of it is what 64 bits give."""
+    rng = np.random.default_rng(hidden + inter)
+
+    def matrix(rows, k):
+        m = torch.from_numpy(synth.nvfp4_matrix(rows, k, rng)).cuda()
+        s = m.view(-1, 36)[:, :4]
+        s[:] = torch.from_numpy(rng.integers(0x70, 0x7F, tuple(s.shape)).astype(np.uint8)).cuda()  # (all of a size: no sums that cancel)
+        pick = torch.from_numpy(rng.integers(0, 50, tuple(s.shape))).cuda()
+        s[pick == 0], s[pick == 1] = 0x7F, 0xFF
+        return m
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(experts)], [matrix(hidden, inter) for _ in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 2.0 ** -13, 2.0 ** -10, gate_up=gu, down=dn, device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, 1, tokens)
+    x = torch.from_numpy(rng.standard_normal((tokens, hidden)).astype(np.float32)).cuda().to(dtype)
+    x[3, 7], x[5, 100] = float("inf"), float("nan")
+    ids = torch.from_numpy(rng.integers(0, experts, tokens).astype(np.int32)).cuda()
+    eo = torch.empty((tokens, hidden), device="cuda")
+    plan.experts_only(w, ids, x, eo=eo)
+    assert not eo[5].isfinite().any() and not eo[3].isfinite().all()
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m, torch.tensor([gs], device="cuda"), rows, k), rule=True).double().view(rows, k)
+
+    for c in range(tokens):
+        if c in (3, 5):
+            continue
+        g = deq(gu[ids[c]], 2 * inter, hidden, 2.0 ** -13) @ x[c].double()
+        want = deq(dn[ids[c]], hidden, inter, 2.0 ** -10) @ (g[:inter] / (1 + torch.exp(-g[:inter])) * g[inter:])
+        assert (eo[c].double() - want).norm() <= 2e-6 * want.norm(), c  # f32 throughout, as above
+    assert device_status() == 0
