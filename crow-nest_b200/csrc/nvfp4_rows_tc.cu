@@ -260,12 +260,20 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             }
             if (more) {
                 const uint32_t dst = ring + (uint32_t)(is * PIECE + lane * 16);
+                // piece 32 j + lane: of row 16 and on from piece 144
+                const uint8_t *lo = from + (uint32_t)(ic * 144), *hi = gu ? from1 + (uint32_t)(ic * 144) : lo, *mid = lane < 16 ? lo : hi;
+                auto copy = [&](int j, uint32_t at) {
+                    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"((j < 4 ? lo : j == 4 ? mid : hi) + at), "l"(pol) : "memory");
+                };
+                if (have == (gu ? 16 : 32)) {
 #pragma unroll
-                for (int j = 0; j < 9; j++) {
-                    const int row = (lane + 32 * j) / 9;
-                    const uint8_t* src = (gu && row >= 16 ? from1 : from) + off[j] + (uint32_t)(ic * 144);
-                    if ((gu ? row & 15 : row) < have)
-                        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"(src), "l"(pol) : "memory");
+                    for (int j = 0; j < 9; j++) copy(j, off[j]);
+                } else {  // the matrix ends inside these rows
+#pragma unroll 1
+                    for (int j = 0; j < 9; j++) {
+                        const int id = lane + 32 * j, row = id / 9, r = gu ? row & 15 : row;
+                        if (r < have) copy(j, (uint32_t)r * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u);
+                    }
                 }
                 if (++is == D) is = 0;
                 if (++ic == nk) ic = 0, iq++;
