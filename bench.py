@@ -27,9 +27,9 @@ sys.path.insert(0, ROOT)
 METRIC = "nvfp4_gemv_hbm_gbs"
 UNIT = "GB/s"
 # DRAM bytes moved per algorithmic byte by the M = 1 kernel: dram__bytes_read.sum + dram__bytes_write.sum of one
-# captured gate/up launch (100.3 MB read + 4.6 MB written = 104.9 MB) over its algorithmic bytes (100.3 MB); the capture is
-# summarised in profiles/nvfp4_gemv_m1_kernel_gateup_17408x5120.md
-TRAFFIC_RATIO = 1.046
+# captured gate/up launch (103.1 MB read + 3.6 MB written = 106.7 MB) over its algorithmic bytes (100.3 MB); the capture is
+# summarised in profiles/nvfp4_gemv_tc_kernel_gateup_17408x5120.md
+TRAFFIC_RATIO = 1.063
 MIN_TIMED_S = 0.5
 
 
@@ -443,7 +443,7 @@ def gemv_arm(args, rank, world, local):
                        "l2": f"{copies} distinct weight copies ({copies * nb / 2 ** 20:.0f} MiB) rotated launch by launch: larger than L2",
                        "launch": f"CUDA graph replay of {per_graph} launches"},
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None, "peak_kind": peak_kind,
-                         "kernel": "fp8_gemv_tc_kernel" if op == "fp8" else "nvfp4_gemv_m1_kernel", "bytes_per_launch": bytes_launch, "us_per_launch": us},
+                         "kernel": "fp8_gemv_tc_kernel" if op == "fp8" else "nvfp4_gemv_tc_kernel" if nb >= 4.5e6 else "nvfp4_gemv_m1_kernel", "bytes_per_launch": bytes_launch, "us_per_launch": us},
             "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"], "ms_per_step_max": t["ms_per_step_max"],
             "e2e": {"value": bytes_launch / e2e_s / 1e9, "unit": UNIT, "h2d_bytes_per_step": x_host.numel() * 2, "d2h_bytes_per_step": y_host.numel() * 2,
                     "note": "one launch per host call"},
@@ -466,7 +466,7 @@ def gemv_arm(args, rank, world, local):
 # ---------------------------------------------------------------------------------------------- interval table
 def intervals_arm(args, rank=0, world=1, local=0):
     """`--workload intervals`: where the time of a projection goes inside the dense stack. Needs the diagnostic build of the
-    library (`make -C crow-nest_b200/csrc trace`), whose one-row GEMV kernel stamps %globaltimer per CTA at entry, after the
+    library (`make -C crow-nest_b200/csrc trace`), whose GEMV kernels stamp %globaltimer per CTA at entry, after the
     wait on the predecessor grid, after the activations are staged, when its first stage has landed, at its end, and in the
     producer warp at its first and after its last bulk copy; under torchrun the exchange kernel of the tensor-parallel stack
     stamps its own steps too. Prints markdown tables (ns after the previous launch's last CTA ended; medians over the CTAs
@@ -806,7 +806,7 @@ def main():
                 "roofline": {"bound": "hbm", "achieved": per_gpu, "peak": peak, "unit": "GB/s", "frac": per_gpu / peak, "scope": "per GPU",
                              "traffic": TRAFFIC_RATIO * bytes_step / world / (4 * stack.layers) if m == 1 else None,
                              "traffic_note": "dram read+write bytes of one ncu capture of the gate/up launch (profiles/), scaled to the average projection by bytes",
-                             "peak_kind": peak_kind, "kernel": "nvfp4_gemv_seq_kernel" if fused else "nvfp4_gemv_m1_kernel", "bytes_per_launch": bytes_step / world / (4 * stack.layers),
+                             "peak_kind": peak_kind, "kernel": "nvfp4_gemv_seq_kernel" if fused else "nvfp4_gemv_tc_kernel", "bytes_per_launch": bytes_step / world / (4 * stack.layers),
                              "us_per_launch": ms_step * 1e3 / (4 * stack.layers)},
                 "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"], "ms_per_step_max": t["ms_per_step_max"],
                 "e2e": {"value": bytes_step / e2e_s / 1e9, "unit": UNIT, "h2d_bytes_per_step": x_host.numel() * 2,

@@ -41,6 +41,9 @@ struct GemvCall {
 };
 
 int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who);
+#ifdef CN_M1_TRACE
+unsigned long long* cn_trace_slot();  // diagnostic build: where the next launch stamps (nvfp4_gemv_m1.cu), or null
+#endif
 
 // Sort combos by expert and cut every expert's run into groups (moe.cu): order [combos]; ga = positions (in order) of the
 // one-row groups, counts[0] of them; gb / gbrows = positions and row counts (2..gmax, gmax 4 or 8) of the larger groups,

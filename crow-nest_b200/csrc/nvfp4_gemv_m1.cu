@@ -1,5 +1,5 @@
-// NVFP4 GEMV for 1..8 bf16 activation rows (decode, MTP verify, and every combo of the routed-expert
-// step): persistent CTAs, tensor-core inner loop in "word" form. Supersedes gemv_nvfp4_w / _gu / _wm /
+// NVFP4 GEMV for 1..8 bf16 activation rows of smaller matrices (larger ones: nvfp4_gemv_tc.cu) and for every combo of the routed-expert
+// step: persistent CTAs, tensor-core inner loop in "word" form. Supersedes gemv_nvfp4_w / _gu / _wm /
 // _gum (engine/src/kernels_p2.rs:355-530) and the routed record kernels gemv_fp4(_b), gemv_fp4_ptrb
 // (engine/src/kernels.rs:118-195) for bf16 activations.
 //
@@ -768,6 +768,7 @@ Split one_row_split(int ntiles, int bpr, int tx) {
 static unsigned long long* g_m1_trace = nullptr;
 static int g_m1_trace_n = 0, g_m1_trace_i = 0;
 extern "C" void cn_m1_trace(unsigned long long* buf, int launches) { g_m1_trace = buf, g_m1_trace_n = launches, g_m1_trace_i = 0; }
+unsigned long long* cn_trace_slot() { return g_m1_trace && g_m1_trace_i < g_m1_trace_n ? g_m1_trace + (size_t)(g_m1_trace_i++) * 512 * 8 : nullptr; }
 #endif
 
 int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
@@ -893,7 +894,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         for (int d = 0; d < a.line_world; d++) p.yl[d] = a.line_bases[d];
     }
 #ifdef CN_M1_TRACE
-    p.trace = (g_m1_trace && g_m1_trace_i < g_m1_trace_n && !routed) ? g_m1_trace + (size_t)(g_m1_trace_i++) * 512 * 8 : nullptr;
+    p.trace = routed ? nullptr : cn_trace_slot();
 #endif
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, (unsigned)(routed ? combos : 1));
@@ -918,7 +919,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         return teams == 2 ? launch_m1<32, 1, 8, KSV, false, PPV, 2>(cfg, p) : launch_m1<32, 1, 8, KSV, false, PPV>(cfg, p); \
     }
         if (tx == 32 && (parts > 1 || teams > 1)) {
-            CN_M1_PARTS(1, 1) CN_M1_PARTS(1, 2) CN_M1_PARTS(1, 4) CN_M1_PARTS(2, 1) CN_M1_PARTS(2, 2) CN_M1_PARTS(4, 1)
+            CN_M1_PARTS(1, 1) CN_M1_PARTS(2, 1) CN_M1_PARTS(2, 2) CN_M1_PARTS(4, 1)
         }
 #undef CN_M1_PARTS
     } else if (ksplit > 1) {
@@ -933,16 +934,14 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         // line output: the shapes of a tensor-parallel rank (32 blocks per stage)
         if (tx == 32 && cps == 2) return launch_m1<32, 2, 1, 1, true>(cfg, p);
         if (tx == 32 && cps == 3) return launch_m1<32, 3, 1, 1, true>(cfg, p);
-        if (tx == 32 && cps == 4) return launch_m1<32, 4, 1, 1, true>(cfg, p);
         CN_FAIL(CN_ERR_SHAPE, "%s: line output needs k >= 2048 (k = %d)", who, k);
     }
 #define CN_M1_CASE(TXV, CPSV, MTV) \
     if (tx == TXV && cps == CPSV && mt == MTV && teams == 1) return launch_m1<TXV, CPSV, MTV>(cfg, p);
-    CN_M1_CASE(32, 2, 1) CN_M1_CASE(32, 3, 1) CN_M1_CASE(32, 4, 1) CN_M1_CASE(16, 2, 1) CN_M1_CASE(16, 3, 1) CN_M1_CASE(16, 4, 1)
-    CN_M1_CASE(32, 1, 2) CN_M1_CASE(32, 2, 2) CN_M1_CASE(16, 1, 2) CN_M1_CASE(16, 2, 2)
-    CN_M1_CASE(32, 1, 4) CN_M1_CASE(32, 2, 4) CN_M1_CASE(16, 1, 4) CN_M1_CASE(16, 2, 4)
-    CN_M1_CASE(32, 1, 8) CN_M1_CASE(32, 2, 8) CN_M1_CASE(16, 1, 8) CN_M1_CASE(16, 2, 8)
-    if (tx == 16 && teams == 2 && mt > 1) return mt == 2 ? launch_m1<16, 1, 2, 1, false, 1, 2>(cfg, p) : (mt == 4 ? launch_m1<16, 1, 4, 1, false, 1, 2>(cfg, p) : launch_m1<16, 1, 8, 1, false, 1, 2>(cfg, p));
+    CN_M1_CASE(32, 2, 1) CN_M1_CASE(32, 3, 1) CN_M1_CASE(16, 4, 1)
+    CN_M1_CASE(32, 1, 2) CN_M1_CASE(32, 1, 4) CN_M1_CASE(32, 1, 8)
+    CN_M1_CASE(16, 2, 2) CN_M1_CASE(16, 2, 4) CN_M1_CASE(16, 2, 8)
+    if (tx == 16 && teams == 2 && mt == 8) return launch_m1<16, 1, 8, 1, false, 1, 2>(cfg, p);
 #undef CN_M1_CASE
     CN_FAIL(CN_ERR_SHAPE, "%s: no kernel for %d blocks per stage, %d CTAs per SM, %d rows", who, tx, cps, mt);
 }

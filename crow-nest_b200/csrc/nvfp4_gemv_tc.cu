@@ -67,7 +67,24 @@ struct TcParams {
     unsigned long long yl_stride;
     const unsigned int* yl_epoch;
     int yl_tag, yl_buf, yl_flip;
+#ifdef CN_M1_TRACE
+    unsigned long long* trace;  // [8] globaltimer stamps per CTA of this launch, or null
+#endif
 };
+
+// Diagnostic build (-DCN_M1_TRACE): the stamps of nvfp4_gemv_m1.cu, by a lane each: entry (0), wait on the predecessor over (1), first digits (2), first chunk laid
+// out (3), sums stored (4), first (5) and last (6) load asked for.
+#ifdef CN_M1_TRACE
+__device__ __forceinline__ unsigned long long gtime() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+#define CN_STAMP(i) \
+    if (p.trace && lane == 0) p.trace[(size_t)blockIdx.x * 8 + (i)] = gtime()
+#else
+#define CN_STAMP(i)
+#endif
 
 __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar, uint64_t policy) {
     asm volatile(
@@ -140,6 +157,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         tma_load_2d_hint(dst, &map0, chunk * 36, tile * per_tile, bar, pol);
         if (gu) tma_load_2d_hint(dst + RAW_STAGE / 2, &map1, chunk * 36, tile * per_tile, bar, pol);
     };
+    if (warp == 0) { CN_STAMP(0); }
     if (warp == LOADER) {
         // a barrier a lane: container stages, operand stages, digits, finished chunks, accumulators, sums handed over
         for (int i = lane; i < NBAR; i += 32)
@@ -149,6 +167,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         if (lane == 0) {
             // the weights do not depend on the kernel in front: the first stages are asked for at once
             const uint64_t pol = l2_policy_evict_first();
+            CN_STAMP(5);
             for (int i = 0, tile = cid, c = 0; i < R && i < total; i++) {
                 load(i, tile, ck0 + c, pol);
                 if (++c == nc) c = 0, tile += ncl;
@@ -186,6 +205,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 if (++c == nc) c = 0, tile += ncl;
                 if (++s == R) s = 0, par ^= 1u;
             }
+            CN_STAMP(6);
         }
         __syncwarp();
     } else if (warp == ISSUER) {
@@ -226,6 +246,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         constexpr int TPW = MT > 4 ? MT / 4 : 1;  // rows of a warp
         const int w = warp - 8, myrow = MT < 4 ? w % MT : w, mychunk = MT < 4 ? w / MT : 0;
         pdl_wait();  // the activations may come from the kernel before this one
+        if (w == 0) { CN_STAMP(1); }
         constexpr int XR = F32 ? 2 : 1;           // 16-byte pieces of a lane's eight values
         uint4 nx[TPW][XR];
         int c = mychunk % nc;
@@ -263,6 +284,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             fence_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&xbar[i % NX]);
+            if (i == 0) { CN_STAMP(2); }
         }
     } else if (warp >= EPI_WARPS) {
         // ------------------------------------------------------------ container blocks -> operand layout: a warp takes 32 rows, a lane the four
@@ -313,6 +335,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             __syncwarp();
             // (the stage is given back here and not behind the loads: an arrival can overtake loads whose values nothing has used yet)
             if (lane < 2) mbar_arrive(lane == 0 ? &a_full[i & 1] : &raw_empty[s]);
+            if (w == 0 && i == 0) { CN_STAMP(3); }
             if (++s == R) s = 0, par ^= 1u;
         }
     } else {
@@ -479,6 +502,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             c = 0, tile += ncl, nt++;
         }
         tc_before();
+        if (warp == 0) { CN_STAMP(4); }
         if (C > 1) {
             // A CTA that has had every sum sent to it may leave: nothing more comes. One that gave up waits for the others.
             if (!met) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
@@ -578,6 +602,9 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         p.yl_tag = a.line_tag, p.yl_buf = a.line_buf, p.yl_flip = a.line_flip ? 1 : 0;
         for (int d = 0; d < a.line_world; d++) p.yl[d] = a.line_bases[d];
     }
+#ifdef CN_M1_TRACE
+    p.trace = cn_trace_slot();
+#endif
     CUtensorMap map0, map1;
     const unsigned long long row_bytes = (unsigned long long)nk * 144;
     if (int rc = cn_tmap_2d(&map0, a.w0, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, (unsigned)per_tile)) return rc;
