@@ -1,4 +1,4 @@
-// NVFP4 GEMV for 1..8 bf16 activation rows of smaller matrices (larger ones: nvfp4_gemv_tc.cu) and for every combo of the routed-expert
+// NVFP4 GEMV for 1..8 bf16 activation rows of smaller matrices (larger ones: nvfp4_gemv_tc.cu; the rule is in cn_gemv_m1_launch) and for every combo of the routed-expert
 // step: persistent CTAs, tensor-core inner loop in "word" form. Supersedes gemv_nvfp4_w / _gu / _wm /
 // _gum (engine/src/kernels_p2.rs:355-530) and the routed record kernels gemv_fp4(_b), gemv_fp4_ptrb
 // (engine/src/kernels.rs:118-195) for bf16 activations.
@@ -788,10 +788,15 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (!routed) one = one_row_split(ntiles, bpr, tx);
     // Larger matrices go to the fifth-generation tensor cores, whatever the number of rows (a rule of the matrix alone: a row's bits are those of a one-row
     // call). us a call in a stream of dependent ones, there / here, for one and four rows: gate / up of 17408 x 5120 18.7 / 20.7 and 23.4 / 30.1, 5120 x 17408 12.4 /
-    // 15.4 and 15.0 / 21.1, 4096 x 4096 4.5 / 4.6 and 5.7 / 5.5, 20000 x 1536 5.8 / 7.4 and 7.3 / 9.5, 2048 x 4096 3.4 / 4.1 and 3.9 / 4.5; below, its longer way
-    // from the activations to the first product shows: 2048 x 2048 3.2 / 2.9 and 3.4 / 3.6, 512 x 2048 2.9 / 2.1 and 3.1 / 2.9. Few long rows stay too: its clusters end at
+    // 15.4 and 15.0 / 21.1, 4096 x 4096 4.4 / 4.6 and 5.6 / 5.5, 2048 x 4096 3.5 / 4.1 and 3.9 / 4.6; below eight million weights its longer way
+    // from the activations to the first product shows: 2048 x 2048 3.2 / 2.9 and 3.4 / 3.6, 512 x 2048 2.9 / 2.1 and 3.1 / 2.9. So it does with shorter rows than 4096
+    // values, where the kernel here has parts of K to share only late, until there are rows for all SMs: 3328 x 3584 4.4 / 3.5 and 5.4 / 5.0, 5632 x 1536 4.5 / 3.9 and
+    // 4.7 / 4.8, 8192 x 3072 5.9 / 5.3 and 7.6 / 7.1, gate / up of 3584 x 3328 6.7 / 5.7 and 8.6 / 7.7; but 10000 x 1536 4.5 / 4.9 and 5.2 / 6.4, 12288 x 2560 6.1 / 6.6 and 7.4 /
+    // 8.5, 25949 x 1024 5.1 / 6.6 and 5.9 / 9.5, gate / up of 6144 x 2560 6.2 / 6.5 and 7.4 / 9.3. (One row of a few gate / up matrices of 4096 to 4608 values is slower there: 3072 x 4352
+    // 6.4 / 5.9, four 7.5 / 8.6.) Few long rows stay too: its clusters end at
     // eight CTAs a tile of 128 rows (640 x 17408 6.3 / 5.8, 512 x 16384 5.9 / 4.9, 2048 x 16384 7.7 / 8.1). A row that does not fit here is refused as it was.
-    if (!routed && (long long)rows * k * (gu ? 2 : 1) >= 8000000 && !(rows * (gu ? 2 : 1) <= 1280 && k > 14336)) {
+    const long long all_rows = (long long)rows * (gu ? 2 : 1);
+    if (!routed && all_rows * k >= 8000000 && (k >= 4096 || all_rows >= 10000) && !(all_rows <= 1280 && k > 14336)) {
         const int bp = bpr / one.parts;
         if (front_bytes(2, (bp + tx - 1) / tx, 1, 1, bp, 0) + 2 * stage_bytes <= sm_share(one.cps)) return cn_gemv_tc_launch(a, stream, who);
     }
