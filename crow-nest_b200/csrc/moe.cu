@@ -89,7 +89,10 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     int* bin = sm + 3 * (E + 1);
     __shared__ int wsa[32], wsb[32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The kernels that take the lists wait before they read them; their launch, barriers and tensor memory go on meanwhile: 64 tokens, top 10 of 512 experts
+    // 207.1 -> 197.5 us a step, MUL1 with 16 tokens 266.4 -> 264.3.
+    pdl_launch_dependents();
+    pdl_wait();
     for (int i = tid; i <= E; i += blockDim.x) cnt[i] = 0;
     __syncthreads();
     for (int c = tid; c < n; c += blockDim.x) {
