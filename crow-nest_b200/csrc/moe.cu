@@ -73,20 +73,23 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 
 // Sort the combos by expert and cut every expert's run into groups of up to gmax rows, gmax 4 or 8 (one CTA of 1024 threads):
 //   order[]           the combos sorted by expert, stable; combos without a resident expert (id outside 0..E-1, or a
-//                     null entry of `tab`) last and in no group
+//                     null entry of `tab`) last, in any order, and in no group
 //   ga[] / counts[0]  positions (in order[]) of the one-row groups: an expert's single row, or the one left over after
 //                     its groups of gmax
 //   gb[], gbrows[] / counts[1]  first positions and row counts (2..gmax) of the other groups
-// Placement is done by one warp walking the combos in order (match.any finds the lanes of a step that share an expert),
-// so the sort stays stable without ranking every combo against all others.
+// Placement: every combo counts the earlier ones among its expert's (the list in shared memory, in the order of the counting atomics), which keeps the sort
+// stable; where an expert has more than LONG_RUN rows, or the list does not fit (listed = 0), one warp walks the combos in order instead (match.any finds the lanes of a
+// step that share an expert; 20 dependent steps for 640 combos). A step of 64 tokens, top 10 of 512 experts: 203.0 -> 199.9 us, replayed 199.5 -> 198.8.
+constexpr int LONG_RUN = 64;
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,
                                                          int32_t* __restrict__ order, int* __restrict__ ga, int* __restrict__ gb,
-                                                         int* __restrict__ gbrows, int* __restrict__ counts, int gmax) {
-    extern __shared__ int sm[];  // [E + 1] counts, [E + 1] starts, [E + 1] running, [n] bins
+                                                         int* __restrict__ gbrows, int* __restrict__ counts, int gmax, int listed) {
+    extern __shared__ int sm[];  // [E + 1] counts, [E + 1] starts, [E + 1] running, [n] bins, [n] the experts' combos (listed)
     int* cnt = sm;
     int* start = sm + (E + 1);
     int* run = sm + 2 * (E + 1);
-    int* bin = sm + 3 * (E + 1);
+    int* bin = sm + 3 * (E + 1);  // expert in the low 14 bits (as many fit beside each other), place among the expert's combos above
+    int* list = bin + n;
     __shared__ int wsa[32], wsb[32];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     // The kernels that take the lists wait before they read them; their launch, barriers and tensor memory go on meanwhile: 64 tokens, top 10 of 512 experts
@@ -98,8 +101,7 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     for (int c = tid; c < n; c += blockDim.x) {
         const int e = ids[c];
         const int b = (e < 0 || e >= E || (tab && tab[e] == 0ull)) ? E : e;
-        bin[c] = b;
-        atomicAdd(&cnt[b], 1);
+        bin[c] = b | atomicAdd(&cnt[b], 1) << 14;
     }
     __syncthreads();
     // per expert: one-row groups and larger groups, then three exclusive prefix sums over the experts (rows, a, b)
@@ -133,8 +135,10 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     }
     __syncthreads();
     int pr = wsr[wid] + ir - rows, pa = wsa[wid] + ia - na, pb = wsb[wid] + ib - nb;
+    bool walk = !listed;
     for (int i = i0; i < i1; i++) {
         const int k = cnt[i];
+        walk |= k > LONG_RUN && i < E;
         start[i] = pr;
         run[i] = pr;
         if (i < E) {
@@ -145,11 +149,21 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
         }
         pr += k;
     }
-    __syncthreads();
+    if (!__syncthreads_or(walk)) {
+        for (int c = tid; c < n; c += blockDim.x) list[start[bin[c] & 0x3fff] + (bin[c] >> 14)] = c;
+        __syncthreads();
+        for (int c = tid; c < n; c += blockDim.x) {
+            const int b = bin[c] & 0x3fff, at = start[b], k = b < E ? cnt[b] : 0;
+            int before = b < E ? 0 : bin[c] >> 14;  // (nothing reads the order of those without an expert)
+            for (int i = 0; i < k; i++) before += list[at + i] < c;
+            order[at + before] = c;
+        }
+        return;
+    }
     if (wid == 0) {
         for (int c0 = 0; c0 < n; c0 += 32) {
             const int c = c0 + lane;
-            const int b = c < n ? bin[c] : -1 - lane;  // lanes beyond the end match nobody
+            const int b = c < n ? bin[c] & 0x3fff : -1 - lane;  // lanes beyond the end match nobody
             const unsigned same = __match_any_sync(0xffffffffu, b);
             if (c < n) {
                 const int base = run[b];
@@ -229,7 +243,9 @@ int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int c
     const size_t smem = (size_t)(3 * (experts + 1) + combos) * sizeof(int);
     if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "grouping %d combos over %d experts needs %zu B of shared memory", combos, experts, smem);
     CN_ALLOW_SMEM(moe_group_kernel, 160 * 1024);
-    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1), dim3(1024), smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax));
+    const size_t listed = smem + (size_t)combos * sizeof(int);
+    const bool fits = listed <= 160 * 1024;
+    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1), dim3(1024), fits ? listed : smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax, (int)fits));
     return CN_OK;
 }
 

@@ -142,6 +142,28 @@ def test_combos_without_a_resident_expert_are_left_out(combos, experts, dtype):
     assert device_status() == 0
 
 
+@pytest.mark.parametrize("run", [8, 64, 65, 200])
+def test_groups_of_long_runs(run):
+    """An expert with up to 64 rows and with more beside others and rows without an expert (placed by two ways of the grouping): every row is that of a step with
+    few rows, to f32 sums of another order."""
+    hidden, inter, experts = 256, 256, 5
+    rng = np.random.default_rng(run)
+    gu = [torch.from_numpy(synth.nvfp4_matrix(2 * inter, hidden, rng)).cuda() for _ in range(experts)]
+    dn = [torch.from_numpy(synth.nvfp4_matrix(hidden, inter, rng)).cuda() for _ in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 2.0 ** -4, 0.5, gate_up=gu, down=dn, device="cuda")
+    ids = rng.permutation(np.concatenate([np.full(run, 3), np.full(70, -1), np.repeat([0, 1, 4], [1, 9, 17])])).astype(np.int32)
+    n = len(ids)
+    x = torch.from_numpy(rng.standard_normal((n, hidden)).astype(np.float32)).cuda()
+    idd, eo = torch.from_numpy(ids).cuda(), torch.full((n, hidden), 7.0, device="cuda")
+    moe.GpuMoePlan(hidden, inter, experts, 1, n).experts_only(w, idd, x, eo=eo)
+    few, want = moe.GpuMoePlan(hidden, inter, experts, 1, 8), torch.full((n, hidden), 7.0, device="cuda")
+    for c in range(0, n, 8):
+        few.experts_only(w, idd[c:c + 8], x[c:c + 8], eo=want[c:c + 8])
+    assert torch.equal(eo[idd < 0], want[idd < 0])
+    assert ((eo - want).norm(dim=1) <= 4e-6 * want.norm(dim=1)).all()  # 2e-6 of either, as above
+    assert device_status() == 0
+
+
 @pytest.mark.parametrize("hidden,inter,tokens,experts", [(256, 256, 50, 2), (512, 256, 100, 3), (768, 1280, 49, 40)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_odd_scales_and_rows_that_are_not_finite(hidden, inter, tokens, experts, dtype):
