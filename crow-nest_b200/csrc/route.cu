@@ -94,7 +94,10 @@ __global__ void route_softmax_kernel(const float* __restrict__ logits, int32_t* 
     uint32_t* keys = (uint32_t*)(s_w + K);  // [P]
     __shared__ float bmax[32];
     __shared__ float s_den;
-    pdl_launch_dependents();  // (a later kernel waits for this one before it touches anything; its launch need not)
+    // In this order: kernels behind this one read what is older than it (tensor scales) before they wait. The launch itself goes on under the kernel in front: a MUL1 step of
+    // one token 44.2 -> 42.0 us, 64 tokens of the NVFP4 step 198 -> 193.
+    pdl_wait();
+    pdl_launch_dependents();
     const int P = blockDim.x, e = threadIdx.x, t = blockIdx.x;
     const bool in = e < E;
     const float l = in ? logits[(size_t)t * E + e] : -INFINITY;
@@ -120,6 +123,7 @@ __global__ void route_sigmoid_kernel(const float* __restrict__ logits, const flo
     float* vals = sm;
     float* s_w = sm + blockDim.x;
     uint32_t* keys = (uint32_t*)(s_w + K);
+    pdl_wait();  // (as above)
     pdl_launch_dependents();
     const int P = blockDim.x, e = threadIdx.x, t = blockIdx.x;
     float s = 0.0f;
@@ -159,8 +163,7 @@ int check(int tokens, int experts, int k, const char* who) {
 extern "C" int cn_route_softmax_topk(const float* logits, int32_t* ids, float* wts, int tokens, int experts, int k, cn_stream_t stream) {
     if (int rc = check(tokens, experts, k, "cn_route_softmax_topk")) return rc;
     const int P = pow2_at_least(experts);
-    route_softmax_kernel<<<tokens, P, (2 * P + k) * sizeof(float), (cudaStream_t)stream>>>(logits, ids, wts, experts, k);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(route_softmax_kernel, dim3(tokens), dim3(P), (2 * P + k) * sizeof(float), (cudaStream_t)stream, logits, ids, wts, experts, k));
     return CN_OK;
 }
 
@@ -168,7 +171,6 @@ extern "C" int cn_route_sigmoid_topk(const float* logits, const float* bias, int
                                      float scale, cn_stream_t stream) {
     if (int rc = check(tokens, experts, k, "cn_route_sigmoid_topk")) return rc;
     const int P = pow2_at_least(experts);
-    route_sigmoid_kernel<<<tokens, P, (2 * P + k) * sizeof(float), (cudaStream_t)stream>>>(logits, bias, ids, wts, experts, k, scale);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(route_sigmoid_kernel, dim3(tokens), dim3(P), (2 * P + k) * sizeof(float), (cudaStream_t)stream, logits, bias, ids, wts, experts, k, scale));
     return CN_OK;
 }
