@@ -39,7 +39,8 @@ constexpr int NX = 16;      // chunk factors in flight (a warp is at most a few 
 constexpr int NDONE = 4;    // barriers of finished chunks
 constexpr int MAX_RAW = 4;  // container stages
 constexpr int NA = 2;       // chunks laid out for the tensor core
-constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 5;
+constexpr int NSLOT = 3;    // tiles whose sums are on their way in a cluster
+constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 2 + NSLOT + 2;
 constexpr int EPI_WARPS = 4, LOADER = 12, ISSUER = 13;  // warps 0-3 sums and output, 4-7 weights, 8-11 activations
 constexpr int THREADS = 448;
 constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, slow blocks}; [NX][4] scale bytes of 0xFF seen
@@ -131,9 +132,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint64_t* xbar = a_full + NA;            // [NX] digits of a chunk
     uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk
     uint64_t* d_empty = done + NDONE;         // [2] accumulators
-    uint64_t* exbar = d_empty + 2;            // [2] sums handed over
-    uint64_t* meet = exbar + 2;               // the four adding warps
-    uint32_t* tmem_slot = (uint32_t*)(meet + 1);
+    uint64_t* exbar = d_empty + 2;            // [NSLOT] sums handed over
+    uint64_t* meet = exbar + NSLOT;           // [2] the four adding warps, tile by tile: its sums are in the slot (one CTA), have been read from it (cluster)
+    uint32_t* tmem_slot = (uint32_t*)(meet + 2);
     float2* fs = (float2*)(smem + FS_OFF);    // [NX][8]
     uint32_t* wf = (uint32_t*)(smem + WF_OFF);  // [NX][4]
     const uint32_t base = (smem_u32(smem) + HEADER + 1023u) & ~1023u;
@@ -161,7 +162,13 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     if (warp == LOADER) {
         // a barrier a lane: container stages, operand stages, digits, finished chunks, accumulators, sums handed over
         for (int i = lane; i < NBAR; i += 32)
-            mbar_init(raw_full + i, i < MAX_RAW ? 1 : i < 2 * MAX_RAW + NA ? 4 : i < 2 * MAX_RAW + NA + NX ? (MT < 4 ? MT : 4) : i < NBAR - 5 ? 1 : i < NBAR - 3 ? EPI_WARPS : i < NBAR - 1 ? 1 : EPI_WARPS);
+            mbar_init(raw_full + i, i < MAX_RAW                         ? 1
+                                    : i < 2 * MAX_RAW + NA              ? 4
+                                    : i < 2 * MAX_RAW + NA + NX         ? (MT < 4 ? MT : 4)
+                                    : i < 2 * MAX_RAW + NA + NX + NDONE ? 1
+                                    : i < NBAR - NSLOT - 2              ? EPI_WARPS
+                                    : i < NBAR - 2                      ? 1
+                                                                        : EPI_WARPS);
         mbar_fence_init();
         __syncwarp();
         if (lane == 0) {
@@ -402,13 +409,18 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 const int row = tile * per_tile + (gu ? r & 63 : r);
                 if (row < p.rows) {
                     const uint8_t* wr = (gu && r >= 64 ? p.w1 : p.w0) + ((size_t)row * nk + ck0 + c) * 144;
-#pragma unroll
-                    for (int m = 0; m < MT; m++) {
-                        if (m >= p.m) continue;
+#pragma unroll 1
+                    for (int m = 0; m < p.m; m++) {
                         const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
+                        Acc v = 0;
+#pragma unroll 1
                         for (int b = 0; b < 16; b++)
                             if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
-                                acc[m] += slow_block<F32>(wr + (b >> 2) * 36, b & 3, (const char*)p.x + ((size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * ES) * (F32 ? 1.0f : gs);
+                                v += slow_block<F32>(wr + (b >> 2) * 36, b & 3, (const char*)p.x + ((size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * ES);
+                        if (!F32) v *= gs;
+#pragma unroll
+                        for (int j = 0; j < MT; j++)
+                            if (j == m) acc[j] += v;
                     }
                 }
             }
@@ -427,32 +439,38 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                             ((__nv_bfloat16*)p.y)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(acc[m]);
                     }
             } else {
-                // CTA o of the cluster adds and stores the rows (pairs) [o, o + 1) x share of the tile. Two slots in turn: whoever sends a tile's sums has
-                // all of the tile before, whose senders had read the one before that.
+                // CTA o of the cluster adds and stores the rows (pairs) [o, o + 1) x share of the tile. Three slots in turn. Whoever sends tile n has all of tile n - 1; every CTA owns
+                // rows, so a part of that came from every CTA, and from a warp that sent it only when all four adding warps of its CTA had read tile n - 3 (`meet`),
+                // which had the slot before.
                 const int q = p.share, half = gu ? r >> 6 : 0, at = gu ? r & 63 : r, o = at / q, halves = gu ? 2 : 1;
-                Acc* slot = (Acc*)(ex + (nt & 1) * p.ex_bytes);
+                const int turn = nt % NSLOT;
+                Acc* slot = (Acc*)(ex + turn * p.ex_bytes);
                 Acc* mine = slot + (size_t)((rank * halves + half) * MT) * q + (at - o * q);
                 if (C == 1) {
 #pragma unroll
                     for (int m = 0; m < MT; m++) mine[m * q] = acc[m];
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(meet);
-                    if (!mbar_wait(meet, nt & 1)) {
+                    if (lane == 0) mbar_arrive(&meet[nt & 1]);
+                    if (!mbar_wait(&meet[nt & 1], (nt >> 1) & 1)) {
                         cn_dev_fail(CN_DEV_WAIT_FULL);
                         break;
                     }
                 } else {
                     if (!met) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // every CTA of the cluster has its barriers
                     met = true;
-                    const uint32_t there = cluster_addr(smem_u32(mine), (uint32_t)o), bar = cluster_addr(smem_u32(&exbar[nt & 1]), (uint32_t)o);
+                    if (nt > 1 && ntl > NSLOT && !mbar_wait(&meet[nt & 1], ((nt - 2) >> 1) & 1)) {
+                        cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                        break;
+                    }
+                    const uint32_t there = cluster_addr(smem_u32(mine), (uint32_t)o), bar = cluster_addr(smem_u32(&exbar[turn]), (uint32_t)o);
 #pragma unroll
                     for (int m = 0; m < MT; m++)
                         if (m < p.m) st_async(there + (uint32_t)(m * q * (int)sizeof(Acc)), acc[m], bar);
                     if (r == 0) {
-                        mbar_expect_tx(&exbar[nt & 1], (uint32_t)(C * halves * p.m * (int)sizeof(Acc) * max(0, min(q, per_tile - rank * q))));
-                        mbar_arrive(&exbar[nt & 1]);
+                        mbar_expect_tx(&exbar[turn], (uint32_t)(C * halves * p.m * (int)sizeof(Acc) * max(0, min(q, per_tile - rank * q))));
+                        mbar_arrive(&exbar[turn]);
                     }
-                    if (!wait_cluster(&exbar[nt & 1], (nt >> 1) & 1)) {
+                    if (!wait_cluster(&exbar[turn], (uint32_t)(nt / NSLOT) & 1u)) {
                         cn_dev_fail(CN_DEV_WAIT_FULL);
                         break;
                     }
@@ -495,6 +513,10 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                                     asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(line), "r"(pair), "r"(seq), "r"(next), "r"(seq) : "memory");
                                 }
                     }
+                }
+                if (C > 1 && ntl > NSLOT) {
+                    __syncwarp();  // every lane has read the slot
+                    if (lane == 0) mbar_arrive(&meet[nt & 1]);
                 }
             }
 #pragma unroll
@@ -587,9 +609,9 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.rows = a.rows, p.k = a.k, p.m = m, p.ldy = a.ldy, p.out_f32 = a.out_f32, p.limit = a.limit, p.csize = c, p.tiles = tiles;
     p.share = ((per_tile + c - 1) / c + 3) & ~3;
     p.qinv = ((1u << 20) + (uint32_t)p.share - 1u) / (uint32_t)p.share;
-    // sums handed over: a slot per tile in flight, two where a CTA has several tiles
+    // sums handed over: a slot per tile in flight, up to NSLOT
     p.ex_bytes = c > 1 || gu || a.line_bases ? c * (gu ? 2 : 1) * p.share * mt * (f32 ? 8 : 4) : 0;
-    const int front = fixed_smem(mt, f32) + (tiles > clusters ? 2 : 1) * p.ex_bytes;
+    const int per_cluster = (tiles + clusters - 1) / clusters, front = fixed_smem(mt, f32) + (per_cluster < NSLOT ? per_cluster : NSLOT) * p.ex_bytes;
     p.raw = (SM_SHARE - front) / RAW_STAGE;
     if (p.raw > MAX_RAW) p.raw = MAX_RAW;
     if (p.raw < 1) CN_FAIL(CN_ERR_LIMIT, "%s: %d rows in clusters of %d leave no room for weights", who, m, c);

@@ -185,3 +185,25 @@ def test_a_chain_of_calls_in_a_graph():
         torch.cuda.synchronize()
         assert torch.equal(bufs[1].view(torch.int16), ref.view(torch.int16))
     assert device_status() == 0
+
+
+# clusters of two, four and six CTAs with one or two chunks of k to each, three and more tiles to some of them: sums of a tile must not reach a slot that another warp still reads
+@pytest.mark.parametrize("rows,k,gu", [(40960, 1024, False), (38400, 1792, False), (38400, 2048, False), (38400, 4352, False), (20000, 1024, True)])
+@pytest.mark.parametrize("m,dtype", [(1, torch.bfloat16), (8, torch.bfloat16), (1, torch.float32), (8, torch.float32)])
+def test_many_tiles_of_few_chunks_repeat_exactly(rows, k, gu, m, dtype):
+    """Rows 32 to 63 of every tile hold scale bytes of 0xFF, whose blocks are multiplied out one by one: that warp reads its sums behind the others."""
+    rng, g, _ = _make(64, k, rows + k)
+    g.w, g.rows = g.w.view(64, -1).repeat(-(-rows // 64), 1)[:rows].reshape(-1).contiguous(), rows
+    g.w.view(rows, k // 64, 36)[:, :, 2][torch.arange(rows, device="cuda") % 128 // 32 == 1] = 0xFF
+    want = ops.dequant(g, rule=True).view(rows, k)
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda().to(dtype)
+    want = x.double() @ want.double().t()
+    if gu:
+        want, call = want / (1 + torch.exp(-want)) * want, lambda: ops.launch_gemv_gu(g, g, x)
+    else:
+        call = lambda: ops.launch_gemv(g, x)  # noqa: E731
+    y = call()
+    assert (y.double() - want).norm() <= (2.0 ** -9 + 1e-6 if dtype == torch.bfloat16 else 2.0 ** -20) * want.norm()
+    bits = torch.int16 if dtype == torch.bfloat16 else torch.int32
+    assert all(torch.equal(call().view(bits), y.view(bits)) for _ in range(200))
+    assert device_status() == 0
