@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint64_t* raw_empty = raw_full + MAX_RAW;
     uint64_t* a_full = raw_empty + MAX_RAW;   // [NA]
     uint64_t* xbar = a_full + NA;            // [NX] digits of a chunk
-    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk
+    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
     uint64_t* d_empty = done + NDONE;         // [2] accumulators
     uint64_t* exbar = d_empty + 2;            // [NSLOT] sums handed over
     uint64_t* meet = exbar + NSLOT;           // [2] the four adding warps, tile by tile: its sums are in the slot (one CTA), have been read from it (cluster)
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             mbar_init(raw_full + i, i < MAX_RAW                         ? 1
                                     : i < 2 * MAX_RAW + NA              ? 4
                                     : i < 2 * MAX_RAW + NA + NX         ? (MT < 4 ? MT : 4)
-                                    : i < 2 * MAX_RAW + NA + NX + NDONE ? 1
+                                    : i < 2 * MAX_RAW + NA + NX + NDONE ? 2
                                     : i < NBAR - NSLOT - 2              ? EPI_WARPS
                                     : i < NBAR - 2                      ? 1
                                                                         : EPI_WARPS);
@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
                 for (int j = 0; j < 4; j++) umma_bs(td, da + 2 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
                 tc_commit<1>(&done[i % NDONE]);
+                mbar_arrive(&done[i % NDONE]);
             }
             __syncwarp();
         }
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         bool met = C == 1;
         int c = 0, tile = cid, nt = 0;
         for (int i = 0; i < total; i++) {
-            if (!mbar_wait(&done[i % NDONE], (i / NDONE) & 1) || !mbar_wait(&xbar[i % NX], (i / NX) & 1)) {
+            if (!mbar_wait(&done[i % NDONE], (i / NDONE) & 1)) {
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 break;
             }

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     uint8_t *a0 = smem, *b0 = a0 + NA * A_STAGE, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;
     uint64_t* a_full = (uint64_t*)head;       // [NA]
     uint64_t* xbar = a_full + NA;             // [NX] digits of a chunk
-    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk
+    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
     uint64_t* d_empty = done + NDONE;         // [2] accumulators
     uint64_t* unit_full = d_empty + 2;        // [NU]
     uint64_t* unit_empty = unit_full + NU;    // [NU]
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     if (warp == SCOUT) {
         // a barrier a lane and round: operand stages, digits, finished chunks, accumulators, units full and empty (four + four + four + one warps read them)
         for (int i = lane; i < NBAR; i += 32)
-            mbar_init(a_full + i, i < NA + NX ? 4 : i < NA + NX + NDONE ? 1 : i < NA + NX + NDONE + 2 ? 4 : i < NBAR - NU ? 1 : 13);
+            mbar_init(a_full + i, i < NA + NX ? 4 : i < NA + NX + NDONE ? 2 : i < NA + NX + NDONE + 2 ? 4 : i < NBAR - NU ? 1 : 13);
         mbar_fence_init();
         __syncwarp();
     } else if (warp == ISSUER) {
@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
 #pragma unroll
                     for (int j = 0; j < 4; j++) umma_bs(td, da + 2 * j, db + 2 * j, idesc, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
                     tc_commit<1>(&done[i % NDONE]);
+                    mbar_arrive(&done[i % NDONE]);
                 }
                 __syncwarp();
             }
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
 #pragma unroll
             for (int m = 0; m < RG; m++) acc[m] = 0;
             for (int ch = 0; ch < nk; ch++, i++) {
-                if (!mbar_wait(&done[i % NDONE], (uint32_t)(i / NDONE) & 1u) || !mbar_wait(&xbar[i % NX], (uint32_t)(i / NX) & 1u)) {
+                if (!mbar_wait(&done[i % NDONE], (uint32_t)(i / NDONE) & 1u)) {
                     cn_dev_fail(CN_DEV_WAIT_FULL);
                     ok = false;
                     break;
