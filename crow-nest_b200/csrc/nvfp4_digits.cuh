@@ -1,9 +1,11 @@
 // Shared by the kernels that multiply NVFP4 weights as they are on tcgen05.mma kind::mxf4nvf4 (nvfp4_gemv_tc.cu, nvfp4_rows_tc.cu): PTX wrappers, 256 values
-// of an activation row as octal digits, and a block of 16 multiplied out in f32.
+// of an activation row as octal digits, and blocks of 16 multiplied out.
 #pragma once
 #include "tc5.cuh"
 
-__host__ __device__ constexpr int digits_of(bool f32) { return f32 ? 10 : 8; }
+#include <type_traits>
+
+__host__ __device__ constexpr int digits_of(bool f32) { return f32 ? 12 : 8; }
 
 // ---------------------------------------------------------------- tcgen05
 __device__ __forceinline__ uint64_t desc_sf(uint32_t smem_addr) {  // a scale chunk: 32 rows of 16 bytes, no swizzle, 8-row groups 128 B apart
@@ -27,57 +29,85 @@ __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* v) {
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tc_ld2(uint32_t taddr, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr) : "memory");
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// a row's digits of one chunk
+template <bool F32>
+__device__ __forceinline__ void tc_ld_digits(uint32_t taddr, uint32_t* v) {
+    tc_ld8(taddr, v);
+    if (F32) tc_ld4(taddr + 8, v + 8);
+}
+
 // ---------------------------------------------------------------- 256 values of an activation row as digits (a warp; a lane holds eight values)
-// bs: the B tile; the row's lines are `row` x the digits of a value + j for digit j. With E the exponent of a block's largest value, a value is
-// q x 2^(E - 21), |q| <= 2^22 (f32: q x 2^(E - 27), |q| <= 2^28): its digits are the octal digits of q + 44444444 (octal; f32: ten fours), less four
-// each. The scale byte is 2^(8 - (Emax - E)), Emax that of the chunk.
+// bs: the B tile; the row's lines are `row` x the digits of a value + j for digit j. With E the exponent of a block's largest value, a value is q x 2^(E - 21), |q| <= 2^22
+// (f32: q x 2^(E - 33), |q| <= 2^34): its digits are the octal digits of q + 44444444 (octal; f32: twelve fours), less four each. The scale byte is 2^(8 - (Emax - E)), Emax
+// that of the chunk.
+//
+// A bf16 value is whole in its digits from 2^-14 of 2^E on, an f32 value from 2^-10 on; smaller ones are off by 2^-22 (f32: 2^-34) of 2^E at most. That is nothing beside the
+// large values of a block, but much where one or two stand alone and meet small weights. So a block of which fewer than three values reach 2^-8 of the
+// largest has no digits: the threads that add the chunk multiply it out (`whole_blocks`). Rows of 1e4 beside values of size 1, one to a block, weights zero there: f32 2.6e-8 off, with ten digits and
+// no such rule 1.6e-5; such a block is one in 1e5 of an FFN's hidden rows (SiLU of deviation 7 times its like), none of normally distributed ones. The same goes for blocks below
+// 2^-17 of their chunk's largest value or below 2^-99, and for those with an infinity or NaN.
+// fs[row]: 2^(Emax - 8) and the blocks without digits (block b: bit 2 b).
+constexpr float TO_INT = 12582912.0f;  // 3 x 2^22: a sum with it has the nearest whole number in its mantissa (ties to even)
+
 template <bool F32>
 __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* bs, uint8_t* sf, int row, float2* fs) {
     constexpr int LV = digits_of(F32);
-    constexpr uint32_t LEAST = F32 ? 28u : 22u;  // biased exponent below which the scale of a block would be no number
-    uint32_t u[F32 ? 8 : 4], top;
+    constexpr uint32_t LEAST = 28u, EXP = F32 ? 23u : 7u;  // least biased E: all scales are numbers
+    uint32_t u[F32 ? 8 : 4], pair[4], top;  // largest values of four pairs, and of the block
     u[0] = raw[0].x, u[1] = raw[0].y, u[2] = raw[0].z, u[3] = raw[0].w;
     if constexpr (F32) {
         u[4] = raw[1].x, u[5] = raw[1].y, u[6] = raw[1].z, u[7] = raw[1].w;
-        top = u[0] & 0x7fffffffu;
 #pragma unroll
-        for (int i = 1; i < 8; i++) top = max(top, u[i] & 0x7fffffffu);
+        for (int i = 0; i < 4; i++) pair[i] = max(u[2 * i] & 0x7fffffffu, u[2 * i + 1] & 0x7fffffffu);
     } else {
-        top = __vmaxu2(__vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu));
-        top = max(top >> 16, top & 0xffffu);
+        const uint32_t a = __vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), b = __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu);
+        pair[0] = a & 0xffffu, pair[1] = a >> 16, pair[2] = b & 0xffffu, pair[3] = b >> 16;
     }
+    top = max(max(pair[0], pair[1]), max(pair[2], pair[3]));
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));  // two lanes hold a block of 16
-    uint32_t e = top >> (F32 ? 23 : 7);
-    const bool odd = top != 0u && (e < LEAST || e == 255u);  // too small, infinity, NaN
-    const uint32_t emax = max(__reduce_max_sync(0xffffffffu, odd ? 0u : e), LEAST);
-    const bool slow = odd || (top != 0u && emax - e > 17u);
-    const uint32_t slow_lanes = __ballot_sync(0xffffffffu, slow);
-    if (slow || top == 0u) {
-        e = emax;
+    uint32_t e = top >> EXP;
+    bool none = e == 255u;  // infinity, NaN
+    const uint32_t emax = max(__reduce_max_sync(0xffffffffu, none ? 0u : e), LEAST);
+    const uint32_t limit = (max(e, 9u) - 8u) << EXP;
+    none |= top != 0u && (e + 17u < emax || e < LEAST);
+    int large = (pair[0] >= limit) + (pair[1] >= limit) + (pair[2] >= limit) + (pair[3] >= limit);
+    large += __shfl_xor_sync(0xffffffffu, large, 1);
+    uint32_t blocks = 0u;
+    if (__any_sync(0xffffffffu, none || (top != 0u && large < 3))) {
+        large = 0;
 #pragma unroll
-        for (int i = 0; i < (F32 ? 8 : 4); i++) u[i] = 0u;
+        for (int i = 0; i < 8; i++) large += (F32 ? u[i] & 0x7fffffffu : (u[i >> 1] >> (16 * (i & 1))) & 0x7fffu) >= limit;
+        large += __shfl_xor_sync(0xffffffffu, large, 1);
+        none |= top != 0u && large < 3;
+        blocks = __ballot_sync(0xffffffffu, none) & 0x55555555u;
+#pragma unroll
+        for (int i = 0; i < (F32 ? 8 : 4); i++) u[i] = none ? 0u : u[i];
     }
-    const float scale = __uint_as_float(((F32 ? 281u : 275u) - e) << 23);  // 2^(21 - (e - 127)), f32: 27
+    if (none || top == 0u) e = emax;
+    const float scale = __uint_as_float(((F32 ? 269u : 275u) - e) << 23);  // 2^(21 - (e - 127)), f32: 15
     uint32_t lo[4], hi[4], over[4];  // value pair p: byte j = digits j (hi: 4 + j; over: 8 + j) of both
 #pragma unroll
     for (int p = 0; p < 4; p++) {
         uint32_t sel[2], up[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
+            const float v = __uint_as_float(F32 ? u[F32 ? 2 * p + h : p] : h ? u[p] & 0xffff0000u : u[p] << 16);
             uint32_t q;
             if constexpr (F32) {
-                q = (uint32_t)(__float2int_rn(__uint_as_float(u[2 * p + h]) * scale) + 04444444444);
-                up[h] = q >> 24;
-                up[h] += up[h] & 0x38u;
-                q &= 0x00ffffffu;
+                // six digits of the value in units of 2^(E - 15), six of what is left, which may reach beyond them by one
+                const float t = fmaf(v, scale, TO_INT), w = fmaf(fmaf(v, scale, TO_INT - t), 262144.0f, TO_INT);
+                const uint32_t lq = __float_as_uint(w) + (0444444u - 0x4b400000u), hq = __float_as_uint(t) + (0444444u - 0x4b400000u) + (lq >> 18);
+                q = (lq & 0x3ffffu) | ((hq & 0x3fu) << 18);
+                uint32_t x = hq >> 6;
+                x += (x & 0xfc0u) * 3u;
+                up[h] = x + (x & 0x3838u);
             } else {
-                const float v = __uint_as_float(h ? u[p] & 0xffff0000u : u[p] << 16);
-                q = __float_as_uint(fmaf(v, scale, 12582912.0f)) + (044444444u - 0x4b400000u);  // (q + 2^22 is the sum's mantissa: rounded to nearest even)
+                q = __float_as_uint(fmaf(v, scale, TO_INT)) + (044444444u - 0x4b400000u);
             }
             q += (q & 0x00fff000u) * 15u;  // octal digits apart: four to sixteen bits, two to eight, one to four
             q += (q & 0x0fc00fc0u) * 3u;
@@ -87,23 +117,16 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
         // digit d - 4 as E2M1: -4 .. 3 = E D C A 0 2 4 5; the even value's in the low nibble
         lo[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0]) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1]);
         hi[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, sel[0] >> 16) | __byte_perm(0xA0C0D0E0u, 0x50402000u, sel[1] >> 16);
-        if constexpr (F32) {
-            const uint32_t c = __byte_perm(0x0A0C0D0Eu, 0x05040200u, up[0] | (up[1] << 8));  // even 8, even 9, odd 8, odd 9
-            over[p] = c | (c >> 12);
-        }
+        if constexpr (F32) over[p] = __byte_perm(0x0A0C0D0Eu, 0x05040200u, up[0]) | __byte_perm(0xA0C0D0E0u, 0x50402000u, up[1]);
     }
     const uint32_t at = (uint32_t)(lane >> 2), in = (uint32_t)(lane & 3) * 4u;
     auto put = [&](int j, uint32_t w) {
-        if constexpr (F32) {
-            const uint32_t n = (uint32_t)(row * LV + j), r = n & 7u;
-            *(uint32_t*)(bs + n * 128u + ((at ^ r) << 4) + in) = w;
-        } else {
-            *(uint32_t*)(bs + row * 1024 + j * 128 + ((at ^ (uint32_t)j) << 4) + in) = w;
-        }
+        const uint32_t n = (uint32_t)(row * LV + j);
+        *(uint32_t*)(bs + n * 128u + ((at ^ (F32 ? n & 7u : (uint32_t)j)) << 4) + in) = w;
     };
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const uint32_t* s = h ? hi : lo;
+    for (int h = 0; h < LV / 4; h++) {
+        const uint32_t* s = h == 0 ? lo : h == 1 ? hi : over;
         const uint32_t a = __byte_perm(s[0], s[1], 0x5140), b = __byte_perm(s[2], s[3], 0x5140);
         const uint32_t c = __byte_perm(s[0], s[1], 0x7362), d = __byte_perm(s[2], s[3], 0x7362);
         put(4 * h, __byte_perm(a, b, 0x5410));
@@ -111,34 +134,72 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
         put(4 * h + 2, __byte_perm(c, d, 0x5410));
         put(4 * h + 3, __byte_perm(c, d, 0x7632));
     }
-    if constexpr (F32) {
-        const uint32_t a = __byte_perm(over[0], over[1], 0x5140), b = __byte_perm(over[2], over[3], 0x5140);
-        put(8, __byte_perm(a, b, 0x5410));
-        put(9, __byte_perm(a, b, 0x7632));
-    }
     const uint32_t under = emax - e;  // 0..17: 2^8 .. 2^-9, the last three subnormal
     uint32_t sw = (under <= 14u ? (15u - under) << 3 : 32u >> (under - 12u)) << (8 * ((lane >> 1) & 3));
     sw |= __shfl_xor_sync(0xffffffffu, sw, 2);
     sw |= __shfl_xor_sync(0xffffffffu, sw, 4);
     int n = row * LV + (lane & 7);
     *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
-    if (F32 && (lane & 7) < LV - 8) {
+    if ((lane & 7) < LV - 8) {
         n += 8;
         *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
     }
-    if (lane == 0) *fs = make_float2(__uint_as_float((emax - 8u) << 23), __uint_as_float(slow_lanes));  // 2^(Emax - 8)
+    if (lane == 0) *fs = make_float2(__uint_as_float((emax - 8u) << 23), __uint_as_float(blocks));
 }
 
-// one block of 16 values from global memory: sum of code x activation, times the block's scale
+// a chunk's factor in 64 bits (a normal power of two)
+__device__ __forceinline__ double power_of_two(float f) { return __hiloint2double((int)((__float_as_uint(f) >> 3) + (896u << 20)), 0); }
+
+// Blocks of 16 without digits (`blocks`, bit 2 b) and, where `odd`, those whose scale byte is 0xFF (480, which the tensor core does not know and is given as nothing), from global memory: the
+// row's 144 container bytes at wr times 256 values at x. All that a block (bf16: two blocks) needs is
+// asked for at once: what it costs is the way to memory. f32: products and sums in 64 bits. One row of gate / up 17408 x 5120 with a NaN 21.9 -> 22.6 us, 4096 x 4096 4.7 -> 6.3;
+// eight rows with a value of 1e4 in the same place 37 -> 49 us.
 template <bool F32>
-static __device__ __noinline__ float slow_block(const uint8_t* wblk, int sub, const void* x) {
-    float sum = 0.0f;
-    for (int i = 0; i < 16; i++) {
-        const uint32_t b = wblk[4 + sub * 8 + (i >> 1)], n = (i & 1) ? b >> 4 : b & 15u, c = n & 7u;
-        const float v = c < 2u ? 0.5f * (float)c : __uint_as_float(((126u + (c >> 1)) << 23) | ((c & 1u) << 22));
-        const float xv = F32 ? __ldcg((const float*)x + i) : __uint_as_float((uint32_t)__ldcg((const unsigned short*)x + i) << 16);
-        sum = fmaf((n & 8u) ? -v : v, xv, sum);
+static __device__ __noinline__ typename std::conditional<F32, double, float>::type whole_blocks(const uint8_t* wr, uint32_t blocks, bool odd, const void* x) {
+    using Acc = typename std::conditional<F32, double, float>::type;
+    constexpr int XR = F32 ? 4 : 2, NB = F32 ? 1 : 2;
+    if (odd) {
+        uint32_t s[4];
+#pragma unroll
+        for (int g = 0; g < 4; g++) s[g] = __ldcg((const uint32_t*)(wr + 36 * g));
+#pragma unroll
+        for (int b = 0; b < 16; b++) blocks |= ((s[b >> 2] >> (8 * (b & 3))) & 0xffu) == 0xffu ? 1u << (2 * b) : 0u;
     }
-    return sum * ue4m3_f32(wblk[sub], true);
+    Acc sum = 0;
+    while (blocks) {
+        uint32_t scale[NB], code[NB][2];
+        uint4 v[NB][XR];
+#pragma unroll
+        for (int h = 0; h < NB; h++) {
+            const int b = blocks ? (__ffs(blocks) - 1) >> 1 : -1;
+            blocks &= blocks - 1u;
+            if (b >= 0) {
+                const uint8_t* blk = wr + 36 * (b >> 2);
+                scale[h] = __ldcg((const uint32_t*)blk) >> (8 * (b & 3)) & 0xffu;
+                code[h][0] = __ldcg((const uint32_t*)(blk + 4) + 2 * (b & 3)), code[h][1] = __ldcg((const uint32_t*)(blk + 4) + 2 * (b & 3) + 1);
+#pragma unroll
+                for (int i = 0; i < XR; i++) v[h][i] = __ldcg((const uint4*)x + b * XR + i);
+            } else {
+                scale[h] = code[h][0] = code[h][1] = 0u;
+#pragma unroll
+                for (int i = 0; i < XR; i++) v[h][i] = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < NB; h++) {
+            Acc t = 0;
+            uint32_t w[8];
+            e2m1x8_to_f16x2(code[h][0], w), e2m1x8_to_f16x2(code[h][1], w + 4);
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const uint4 q = v[h][i / (F32 ? 4 : 8)];
+                const int wd = F32 ? i & 3 : (i >> 1) & 3;
+                const uint32_t bits = wd == 0 ? q.x : wd == 1 ? q.y : wd == 2 ? q.z : q.w;
+                const float xv = __uint_as_float(F32 ? bits : (i & 1) ? bits & 0xffff0000u : bits << 16);
+                t += (Acc)((i & 1) ? f16hi_to_f32(w[i >> 1]) : f16lo_to_f32(w[i >> 1])) * (Acc)xv;
+            }
+            sum += t * (Acc)ue4m3_f32(scale[h], true);
+        }
+    }
+    return sum;
 }
-

@@ -1,16 +1,14 @@
-// NVFP4 GEMV for 1..8 bf16 activation rows on the fifth-generation tensor cores (tcgen05.mma kind::mxf4nvf4, block scale): plain and gate / up form,
-// with or without the tensor-parallel line output. Supersedes gemv_nvfp4_w / _gu / _wm / _gum (engine/src/kernels_p2.rs:355-530).
+// NVFP4 GEMV for 1..8 bf16 or f32 activation rows on the fifth-generation tensor cores (tcgen05.mma kind::mxf4nvf4, block scale): plain and gate / up form, with or without
+// the tensor-parallel line output (bf16). Supersedes gemv_nvfp4_w / _gu / _wm / _gum (engine/src/kernels_p2.rs:355-530).
 //
 // The weights are the A operand as they are: E2M1 codes with one UE4M3 scale per 16 values is what this MMA multiplies, so nothing is decoded. A bf16
-// row is the B operand as eight columns of signed octal digits: per 16 values a power of two and a number of 23 bits, digit j of a value being one
-// of -4..3, all of them E2M1 values (a bf16 value is exact unless it is below 2^-14 of its block's largest, and then off by 2^-22 of that at most).
+// row is the B operand as eight columns of signed octal digits, an f32 row as twelve: per 16 values a power of two and a number of 23 (35) bits, digit j of a value being one
+// of -4..3, all of them E2M1 values (what they hold of a value: nvfp4_digits.cuh).
 // Products, scales and digits are exact; a column's sum over 256 values is the tensor core's, which is the f32 nearest to it or the one beside (k = 256:
-// 2.5e-8 of a row against 64 bits, as much as the last rounding alone); the columns are added from the smallest up, and the chunks of 256 in f32 in order
-// (k = 4096: 6.2e-8, 17408: 8.6e-8). The columns of one row do not depend on those of another: a row of an m-row call has the bits of a one-row call,
-// and eight rows (64 columns) take the tensor core no longer than one, which is bound by reading A.
-//
-// A block of 16 whose largest value is below 2^-17 of its chunk's largest or below 2^-105, or that holds an infinity or NaN, takes no part in this: the
-// threads that add the chunk multiply it out from global memory in f32 (slow_block).
+// 2.5e-8 of a row against 64 bits, as much as the last rounding alone). The columns are added from the smallest up and the chunks of 256 in order; bf16 rows in f32
+// (k = 4096: 6.2e-8, 17408: 8.6e-8), f32 rows with what the last two additions round off kept, chunks in 64 bits (2.5e-8: the result's own rounding). The columns of one row do not
+// depend on those of another: a row of an m-row call has the bits of a one-row call, and eight rows (64 or 96 columns) take the tensor core little longer than one, which is bound by
+// reading A.
 //
 // A CTA owns 128 rows (64 of gate and 64 of up) over a part of k; a cluster of C CTAs shares the tile, part by part, and every CTA adds and stores
 // 128 / C of its rows, the parts in order. Warps: 0-3 add up and store (a thread is a row), 4-7 move container blocks (36 bytes) into the operand's
@@ -371,10 +369,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             for (int m0 = 0; m0 < MT; m0 += G) {
                 uint32_t d[G * LV];
 #pragma unroll
-                for (int m = 0; m < G; m++) {
-                    tc_ld8(td + LV * (m0 + m), d + LV * m);
-                    if (F32) tc_ld2(td + LV * (m0 + m) + 8, d + LV * m + 8);
-                }
+                for (int m = 0; m < G; m++) tc_ld_digits<F32>(td + LV * (m0 + m), d + LV * m);
                 tc_wait_ld();
                 if (m0 + G == MT) {
                     tc_before();
@@ -386,18 +381,18 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                     const float2 f = fs[(i % NX) * 8 + m0 + m];
                     float s = __uint_as_float(d[LV * m]);
                     if constexpr (F32) {
-                        // what the last three additions round off is kept; the chunks are added in 64 bits
+                        // what the last two additions round off is kept; the chunks are added in 64 bits
                         float rest = 0.0f;
 #pragma unroll
-                        for (int j = 1; j < LV - 3; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                        for (int j = 1; j < LV - 2; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
 #pragma unroll
-                        for (int j = LV - 3; j < LV; j++) {
+                        for (int j = LV - 2; j < LV; j++) {
                             const float a = s * 0.125f, b = __uint_as_float(d[LV * m + j]);
                             s = a + b;
                             const float bb = s - a;
                             rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
                         }
-                        acc[m0 + m] += ((double)s + (double)rest) * (double)f.x;
+                        acc[m0 + m] += ((double)s + (double)rest) * power_of_two(f.x);
                     } else {
 #pragma unroll
                         for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
@@ -412,12 +407,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                     const uint8_t* wr = (gu && r >= 64 ? p.w1 : p.w0) + ((size_t)row * nk + ck0 + c) * 144;
 #pragma unroll 1
                     for (int m = 0; m < p.m; m++) {
-                        const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
-                        Acc v = 0;
-#pragma unroll 1
-                        for (int b = 0; b < 16; b++)
-                            if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
-                                v += slow_block<F32>(wr + (b >> 2) * 36, b & 3, (const char*)p.x + ((size_t)m * p.k + (size_t)(ck0 + c) * CH + b * 16) * ES);
+                        const uint32_t blocks = __float_as_uint(fs[(i % NX) * 8 + m].y);
+                        if (!(blocks | odd)) continue;
+                        Acc v = whole_blocks<F32>(wr, blocks, odd != 0u, (const char*)p.x + ((size_t)m * p.k + (size_t)(ck0 + c) * CH) * ES);
                         if (!F32) v *= gs;
 #pragma unroll
                         for (int j = 0; j < MT; j++)

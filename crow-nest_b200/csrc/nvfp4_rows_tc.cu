@@ -366,10 +366,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                     if (m0 >= nrows) break;
                     uint32_t d[2 * LV];
 #pragma unroll
-                    for (int m = 0; m < 2; m++) {
-                        tc_ld8(td + LV * (m0 + m), d + LV * m);
-                        if (F32) tc_ld2(td + LV * (m0 + m) + 8, d + LV * m + 8);
-                    }
+                    for (int m = 0; m < 2; m++) tc_ld_digits<F32>(td + LV * (m0 + m), d + LV * m);
                     tc_wait_ld();
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
@@ -377,17 +374,17 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                         const float2 f = fs[(i % NX) * 8 + m0 + m];
                         float s = __uint_as_float(d[LV * m]);
                         if constexpr (F32) {
-                            float rest = 0.0f;  // what the last three additions round off
+                            float rest = 0.0f;  // what the last two additions round off
 #pragma unroll
-                            for (int j = 1; j < LV - 3; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                            for (int j = 1; j < LV - 2; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
 #pragma unroll
-                            for (int j = LV - 3; j < LV; j++) {
+                            for (int j = LV - 2; j < LV; j++) {
                                 const float a = s * 0.125f, b = __uint_as_float(d[LV * m + j]);
                                 s = a + b;
                                 const float bb = s - a;
                                 rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
                             }
-                            acc[m0 + m] += ((double)s + (double)rest) * (double)f.x;
+                            acc[m0 + m] += ((double)s + (double)rest) * power_of_two(f.x);
                         } else {
 #pragma unroll
                             for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
@@ -401,14 +398,15 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 if (lane == 0) mbar_arrive(&d_empty[i & 1]);
                 if (slow && row < c.rows) {
                     const uint8_t* wr = (const uint8_t*)(gu && lane >= 16 ? u.w1 : u.w0) + ((size_t)row * nk + ch) * 144;
+#pragma unroll 1
+                    for (int m = 0; m < nrows; m++) {
+                        const uint32_t blocks = __float_as_uint(fs[(i % NX) * 8 + m].y);
+                        if (!(blocks | odd)) continue;
+                        Acc v = whole_blocks<F32>(wr, blocks, odd != 0u, (const char*)c.x + ((size_t)(u.combo[m] / c.x_div) * c.k + (size_t)ch * CH) * ES);
+                        if (!F32) v *= gs;
 #pragma unroll
-                    for (int m = 0; m < RG; m++) {
-                        if (m >= nrows) continue;
-                        const uint32_t mask = __float_as_uint(fs[(i % NX) * 8 + m].y);
-                        for (int b = 0; b < 16; b++)
-                            if (((mask >> (2 * b)) & 1u) || (odd && wr[(b >> 2) * 36 + (b & 3)] == 0xFFu))
-                                acc[m] += slow_block<F32>(wr + (b >> 2) * 36, b & 3,
-                                                          (const char*)c.x + ((size_t)(u.combo[m] / c.x_div) * c.k + (size_t)ch * CH + b * 16) * ES) * (F32 ? 1.0f : gs);
+                        for (int j = 0; j < RG; j++)
+                            if (j == m) acc[j] += v;
                     }
                 }
             }

@@ -207,3 +207,65 @@ def test_many_tiles_of_few_chunks_repeat_exactly(rows, k, gu, m, dtype):
     bits = torch.int16 if dtype == torch.bfloat16 else torch.int32
     assert all(torch.equal(call().view(bits), y.view(bits)) for _ in range(200))
     assert device_status() == 0
+
+
+def _zero_columns(w, rows, every):
+    """Weights of columns 0, every, 2 every, ... are zero (every: 2, 16 or 256): those are low nibbles."""
+    codes = w.w.view(rows, -1, 36)[:, :, 4:]
+    if every == 256:
+        codes[:, ::4, 0] &= 0xF0
+    else:
+        codes[:, :, ::every // 2] &= 0xF0
+
+
+# one value of 1e3 to 1e7 beside others of size 1 in every block of 16, or one of up to 2^30 a chunk of 256: such blocks are multiplied out. Every other value so: digits
+# that end at 2^-34 (bf16: 2^-22) of a block's largest value, rounded
+@pytest.mark.parametrize("every,size", [(16, 1e4), (16, 1e3), (16, 100.0), (16, 1e7), (256, 2.0 ** 20), (256, 2.0 ** 30), (256, 1e5), (2, 1e4), (2, 1e7)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_small_values_count_where_the_large_ones_beside_them_meet_zero_weights(every, size, dtype):
+    rows, k, m = 2048, 4096, 3
+    rng, w, _ = _make(rows, k, every + int(size) % 97, 1.0)
+    _zero_columns(w, rows, every)
+    w64 = ops.dequant(w).double().view(rows, k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[:, ::every] *= np.float32(size)
+    xd = torch.from_numpy(x).cuda().to(dtype)
+    y, want, total = ops.launch_gemv(w, xd).double(), xd.double() @ w64.t(), xd.double().abs() @ w64.abs().t()
+    # the result's rounding (half a unit in the last place); sums of exact products in f32: a column of digits is the nearest f32 or the one beside it, so are the sums of
+    # columns and chunks
+    bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24) * want.abs() + 2.0 ** -22 * total
+    # digits end at 2^-22 (f32: 2^-34) of a block's largest value, unless fewer than three of its values reach 2^-8 of that
+    blocks = xd.double().abs().view(m, -1, 16)
+    largest, third = blocks.amax(2, keepdim=True), blocks.topk(3, dim=2).values[:, :, 2:]
+    largest = torch.where(third < largest * 2.0 ** -9, 0.0, largest).expand(-1, -1, 16).reshape(m, k)
+    bound += (2.0 ** -23 if dtype == torch.bfloat16 else 2.0 ** -35) * (2 * largest @ w64.abs().t())
+    if every != 2 and dtype == torch.float32:
+        assert (y - want).norm() <= 1e-7 * want.norm()
+    assert ((y - want).abs() <= bound).all(), ((y - want).abs() / total).max()
+    for i in range(m):
+        assert torch.equal(ops.launch_gemv(w, xd[i:i + 1])[0].double(), y[i]), i
+    assert device_status() == 0
+
+
+def test_values_at_the_ends_of_the_range():
+    """Subnormal values beside normal ones, a chunk below what digits are made of, the largest values there are; bf16 and f32 rows of several calls have the bits of a one-row call."""
+    rows, k = 2048, 4096
+    rng, w, _ = _make(rows, k, 77, 2.0 ** -20)
+    _zero_columns(w, rows, 16)
+    w64 = ops.dequant(w).double().view(rows, k)
+    for dtype, tiny in ((torch.bfloat16, 2.0 ** -133), (torch.float32, 2.0 ** -149)):
+        x = torch.from_numpy(rng.standard_normal((5, k)).astype(np.float32)).cuda().to(dtype)
+        x[0, 256:] = 0.0
+        x[0, :256] = tiny * torch.arange(256, device="cuda").to(dtype)
+        x[1, 1::16] = tiny
+        x[2] *= 2.0 ** -116
+        x[3, ::16] = torch.finfo(dtype).max
+        x[4, ::2] *= 2.0 ** -60
+        y = ops.launch_gemv(w, x)
+        for i in range(5):
+            assert torch.equal(ops.launch_gemv(w, x[i:i + 1])[0], y[i]), i
+            want, total = x[i].double() @ w64.t(), x[i].double().abs() @ w64.abs().t()
+            # (results below the least normal number lose bits of their own)
+            bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24) * want.abs() + 2.0 ** -22 * total + 2.0 ** (-133 if dtype == torch.bfloat16 else -146)
+            assert ((y[i].double() - want).abs() <= bound).all(), i
+    assert device_status() == 0

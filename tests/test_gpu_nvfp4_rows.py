@@ -198,3 +198,37 @@ def test_odd_scales_and_rows_that_are_not_finite(hidden, inter, tokens, experts,
         want = deq(dn[ids[c]], hidden, inter, 2.0 ** -10) @ (g[:inter] / (1 + torch.exp(-g[:inter])) * g[inter:])
         assert (eo[c].double() - want).norm() <= 2e-6 * want.norm(), c  # f32 throughout, as above
     assert device_status() == 0
+
+
+@pytest.mark.parametrize("size", [1e3, 1e4, 1e7])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_small_values_of_grouped_rows_beside_large_ones(size, dtype):
+    """One value in sixteen of a row is large and meets zero weights: gate and up are what the small ones give."""
+    hidden, inter, experts, tokens = 512, 512, 3, 60
+    rng = np.random.default_rng(int(size))
+
+    def matrix(rows, k):
+        m = torch.from_numpy(synth.nvfp4_matrix(rows, k, rng)).cuda()
+        if rows == 2 * inter:
+            m.view(-1, 36)[:, 4::8] &= 0xF0  # the low half of a code byte: columns 0, 16, ..
+        return m
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m, torch.tensor([gs], device="cuda"), rows, k), rule=True).double().view(rows, k)
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(experts)], [matrix(hidden, inter) for _ in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 2.0 ** -3, 2.0 ** -3, gate_up=gu, down=dn, device="cuda")
+    x = torch.from_numpy(rng.standard_normal((tokens, hidden)).astype(np.float32)).cuda()
+    x[:, ::16] *= size
+    for m in gu:
+        assert not deq(m, 2 * inter, hidden, 1.0)[:, ::16].any()
+    x = x.to(dtype)
+    ids = torch.from_numpy(rng.integers(0, experts, tokens).astype(np.int32)).cuda()
+    eo = torch.empty((tokens, hidden), device="cuda")
+    moe.GpuMoePlan(hidden, inter, experts, 1, tokens).experts_only(w, ids, x, eo=eo)
+    for c in range(tokens):
+        g = deq(gu[ids[c]], 2 * inter, hidden, 2.0 ** -3) @ x[c].double()
+        want = deq(dn[ids[c]], hidden, inter, 2.0 ** -3) @ (g[:inter] / (1 + torch.exp(-g[:inter])) * g[inter:])
+        # f32 throughout, as above; bf16 rows: digits of a block that is not multiplied out end at 2^-22 of its largest value, which is 2^8 of the third largest at most
+        assert (eo[c].double() - want).norm() <= (2e-6 if dtype == torch.float32 else 2.0 ** -15) * want.norm(), c
+    assert device_status() == 0
