@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 2) occupancy_kernel(int* out) {
     if (out) out[0] = smem[threadIdx.x];
 }
 
-// clusters of c CTAs that the current device holds at a time, two CTAs per SM: asked once per device (0: an error)
+// clusters of c CTAs that the current device holds at a time, two CTAs per SM: asked once per device (0: an error). How many are launched, and nothing else.
 int clusters_of(int c) {
     static std::atomic<int> known[64][9];
     int dev = 0;
@@ -561,17 +561,19 @@ int clusters_of(int c) {
     return n;
 }
 
-// CTAs per cluster, a rule of the matrix alone, since it fixes the order of a row's sum: the least estimate of the time. A chunk takes a CTA 0.42 us, 0.62
+// CTAs per cluster, a rule of the matrix alone, since it fixes the order of a row's sum: the least estimate of the time. Neither the device nor the number of rows has a part in it: the
+// clusters that are there at a time are what any B200 holds (parts differ by a few with the way their SMs lie in GPCs; one with more starts more, one with fewer takes a round more).
+// A chunk takes a CTA 0.42 us, 0.62
 // from the ninth on (three stages of container bytes in flight), more where all CTAs together reach the memory's rate; the chunks are between those of
 // the busiest CTA and the mean; 0.3 for adding up a tile in a cluster, 0.3 where a second CTA per SM keeps the next kernel out. Measured, us with 1 / 2 / 4 /
 // 6 / 8 CTAs: 16384 x 2048 5.7 / 6.5 / 7.1 / 8.6 / 8.2, 8192 x 4096 9.5 / 6.2 / 6.5 / 7.2 / 7.4, 4096 x 8192 17.2 / 10.1 / 6.3 / 6.9 / 6.9, 7168 x 5120 11.5
 // / 7.2 / 6.9 / 7.7 / 8.0, 5120 x 17408 48 / 24 / 14.6 / 12.3 / 16.4, gate / up of 17408 x 5120 18.5 / 19.6 / 20.9 / 25 / 36. 3, 5 and 7 never were the fastest.
 int cut_of(int tiles, int nk) {
-    int best_c = 0;
+    constexpr int AT_ONCE[9] = {0, 296, 148, 0, 70, 0, 46, 0, 32};
+    int best_c = 1;
     double best = 1e30;
     for (int c = 1; c <= 8 && c <= nk; c += c == 1 ? 1 : 2) {
-        const int n = clusters_of(c);
-        if (n < 1) return 0;
+        const int n = AT_ONCE[c];
         const int used = tiles < n ? tiles : n, ctas = used * c, waves = (tiles + n - 1) / n, part = (nk + c - 1) / c;
         const double chunks = 0.5 * (waves * part + (double)tiles * nk / ctas), share = 0.0033 * ctas;
         const double fast = share > 0.42 ? share : 0.42, slow = share > 0.62 ? share : 0.62;
@@ -590,12 +592,14 @@ int launch_tc(const cudaLaunchConfig_t& cfg, const CUtensorMap& map0, const CUte
 
 }  // namespace
 
+extern "C" int cn_nvfp4_gemv_cut(int rows, int k, int gate_up) { return rows < 1 || k < CH ? 0 : cut_of(gate_up ? (rows + 63) / 64 : (rows + 127) / 128, k / CH); }
+
 int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const bool gu = a.w1 != nullptr, f32 = a.dtype == CN_F32;
     const int m = a.m, mt = m == 1 ? 1 : m == 2 ? 2 : m <= 4 ? 4 : 8;
     const int per_tile = gu ? 64 : 128, tiles = (a.rows + per_tile - 1) / per_tile, nk = a.k / CH;
     const int c = cut_of(tiles, nk), ncl = clusters_of(c);
-    if (c < 1 || ncl < 1) CN_FAIL(CN_ERR_CUDA, "%s: the device does not say how many clusters it holds", who);
+    if (ncl < 1) CN_FAIL(CN_ERR_CUDA, "%s: the device does not say how many clusters it holds", who);
     const int clusters = tiles < ncl ? tiles : ncl;
     TcParams p = {};
     p.w0 = (const uint8_t*)a.w0, p.w1 = (const uint8_t*)a.w1, p.gs0 = a.gs0, p.gs1 = a.gs1 ? a.gs1 : a.gs0, p.x = a.x, p.y = a.y;

@@ -68,6 +68,10 @@ int cn_device_status(int* code_out);
  * (kernel, device) has not been allowed `bytes` yet (recorded when commit != 0), else 0. Makes no CUDA call; exported so
  * that the per-device rule can be checked without a GPU. */
 int cn_smem_book(const void* kernel, int device, int bytes, int commit);
+/* Into how many parts of k the tensor-core GEMV cuts the rows of a larger matrix (1, 2, 4, 6 or 8 CTAs of a cluster): the order of a row's sum. A rule of
+ * the matrix alone - rows, values of a row, gate / up or plain - whatever the device and the number of activation rows. Makes no CUDA call; exported so that it
+ * can be checked without a GPU. */
+int cn_nvfp4_gemv_cut(int rows, int k, int gate_up);
 
 /* ---------------------------------------------------------------- NVFP4 GEMV, M = 1..8
  * y[m][r] = sum_k W[r][k] * x[m][k], m < M.

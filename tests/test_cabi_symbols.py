@@ -44,3 +44,16 @@ def test_shared_memory_attribute_is_booked_per_kernel_and_device():
     assert L.cn_smem_book(k1, 1, 100 * 1024, 1) == 1  # another device: its own call
     assert L.cn_smem_book(k2, 0, 100 * 1024, 1) == 1  # another kernel: its own call
     assert L.cn_smem_book(k1, 1, 100 * 1024, 1) == 0
+
+
+def test_the_cut_of_a_row_needs_no_device():
+    """Into how many parts a row is cut fixes the order of its sum: a rule of the matrix alone, the same on every GPU and on none."""
+    cut = _lib.lib().cn_nvfp4_gemv_cut
+    for rows in (1, 128, 2048, 4096, 5120, 9728, 17408, 40960, 248320):
+        for k in (256, 512, 1024, 4096, 5376, 17408):
+            for gu in (0, 1):
+                c = cut(rows, k, gu)
+                assert c in (1, 2, 4, 6, 8) and c <= k // 256, (rows, k, gu, c)
+    # a few that were timed
+    assert [cut(*m) for m in ((4096, 4096, 0), (5120, 5120, 0), (7168, 5120, 0), (5120, 17408, 0), (17408, 5120, 1), (16384, 2048, 0))] == [4, 4, 4, 6, 1, 1]
+    assert cut(0, 4096, 0) == 0 and cut(4096, 128, 0) == 0
