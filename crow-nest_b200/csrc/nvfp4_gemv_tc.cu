@@ -563,21 +563,25 @@ int clusters_of(int c) {
 
 // CTAs per cluster, a rule of the matrix alone, since it fixes the order of a row's sum: the least estimate of the time. Neither the device nor the number of rows has a part in it: the
 // clusters that are there at a time are what any B200 holds (parts differ by a few with the way their SMs lie in GPCs; one with more starts more, one with fewer takes a round more).
-// A chunk takes a CTA 0.42 us, 0.62
-// from the ninth on (three stages of container bytes in flight), more where all CTAs together reach the memory's rate; the chunks are between those of
-// the busiest CTA and the mean; 0.3 for adding up a tile in a cluster, 0.3 where a second CTA per SM keeps the next kernel out. Measured, us with 1 / 2 / 4 /
-// 6 / 8 CTAs: 16384 x 2048 5.7 / 6.5 / 7.1 / 8.6 / 8.2, 8192 x 4096 9.5 / 6.2 / 6.5 / 7.2 / 7.4, 4096 x 8192 17.2 / 10.1 / 6.3 / 6.9 / 6.9, 7168 x 5120 11.5
-// / 7.2 / 6.9 / 7.7 / 8.0, 5120 x 17408 48 / 24 / 14.6 / 12.3 / 16.4, gate / up of 17408 x 5120 18.5 / 19.6 / 20.9 / 25 / 36. 3, 5 and 7 never were the fastest.
+// A chunk takes a CTA 0.41 us, 0.68 from the tenth on (what lies ready when the activations come is gone by then), more where all CTAs together reach the memory's rate: 0.0032
+// for each of them, and 0.92 late in a launch of two to an SM. Without clusters an SM with two CTAs needs 0.86 for a chunk of either however many other SMs have one, and the last
+// round counts in full and more. The chunks are otherwise nearer to the mean than to those of the busiest CTA; 0.62 for adding up a tile in a cluster and 0.026 for each of its CTAs. The figures are those that
+// made the picks for 130 matrices, each timed with every cut, lose least (1 percent on average; 22 for the estimate that stood here before, which had a matrix of 152 tiles as 152 CTAs on 148 SMs).
+// Measured, us with 1 / 2 / 4 / 6 / 8 CTAs: 16384 x 2048 5.7 / 6.5 / 7.1 / 8.6 / 8.2, 8192 x 4096 9.5 / 6.2 / 6.5 / 7.2 / 7.4, 4096 x 8192 17.2 / 10.1 / 6.3 / 6.9 / 6.9, 7168 x 5120 11.5
+// / 7.2 / 6.9 / 7.7 / 8.0, 5120 x 17408 48 / 24 / 14.6 / 12.3 / 16.4, gate / up of 17408 x 5120 18.5 / 19.6 / 20.9 / 25 / 36, of 9728 x 5120 18.1 / 16.3 / 13.8 / 15.6 / 17.2, of
+// 12288 x 4096 15.2 / 14.0 / 14.0 / 15.7 / 16.2, of 20480 x 2048 13.0 / 11.7 / 14.2. 3, 5 and 7 never were the fastest.
 int cut_of(int tiles, int nk) {
     constexpr int AT_ONCE[9] = {0, 296, 148, 0, 70, 0, 46, 0, 32};
     int best_c = 1;
     double best = 1e30;
     for (int c = 1; c <= 8 && c <= nk; c += c == 1 ? 1 : 2) {
-        const int n = AT_ONCE[c];
-        const int used = tiles < n ? tiles : n, ctas = used * c, waves = (tiles + n - 1) / n, part = (nk + c - 1) / c;
-        const double chunks = 0.5 * (waves * part + (double)tiles * nk / ctas), share = 0.0033 * ctas;
-        const double fast = share > 0.42 ? share : 0.42, slow = share > 0.62 ? share : 0.62;
-        const double t = fast * (chunks < 8 ? chunks : 8) + (chunks > 8 ? (chunks - 8) * slow : 0.0) + (c > 1 ? 0.3 * waves : 0.0) + (ctas > 148 ? 0.3 : 0.0);
+        const int n = AT_ONCE[c], used = tiles < n ? tiles : n, ctas = used * c, waves = (tiles + n - 1) / n;
+        const double busiest = (double)waves * ((nk + c - 1) / c), mean = (double)tiles * nk / ctas, share = 0.0032 * ctas;
+        const double chunks = mean + (c == 1 ? 1.6 : 0.21) * (busiest - mean);
+        double early = share > 0.41 ? share : 0.41, late = ctas > 148 ? 0.92 : 0.68;
+        if (late < share) late = share;
+        if (c == 1 && ctas > 148) early = late = 0.86;
+        const double t = early * (chunks < 9.3 ? chunks : 9.3) + (chunks > 9.3 ? (chunks - 9.3) * late : 0.0) + (c > 1 ? 0.62 * waves + 0.026 * c : 0.0);
         if (t < best) best = t, best_c = c;
     }
     return best_c;

@@ -56,4 +56,6 @@ def test_the_cut_of_a_row_needs_no_device():
                 assert c in (1, 2, 4, 6, 8) and c <= k // 256, (rows, k, gu, c)
     # a few that were timed
     assert [cut(*m) for m in ((4096, 4096, 0), (5120, 5120, 0), (7168, 5120, 0), (5120, 17408, 0), (17408, 5120, 1), (16384, 2048, 0))] == [4, 4, 4, 6, 1, 1]
+    # 152 to 192 and 313 tiles, which leave most SMs one CTA or a short second round without a cluster
+    assert [cut(*m) for m in ((9728, 5120, 1), (12288, 4096, 1), (20000, 2048, 1), (20224, 4096, 0))] == [4, 4, 2, 4]
     assert cut(0, 4096, 0) == 0 and cut(4096, 128, 0) == 0
