@@ -47,9 +47,9 @@ __device__ __forceinline__ void tc_ld_digits(uint32_t taddr, uint32_t* v) {
 // that of the chunk.
 //
 // A bf16 value is whole in its digits from 2^-14 of 2^E on, an f32 value from 2^-10 on; smaller ones are off by 2^-22 (f32: 2^-34) of 2^E at most. That is nothing beside the
-// large values of a block, but much where one or two stand alone and meet small weights. So a block of which fewer than three values reach 2^-8 of the
-// largest has no digits: the threads that add the chunk multiply it out (`whole_blocks`). Rows of 1e4 beside values of size 1, one to a block, weights zero there: f32 2.6e-8 off, with ten digits and
-// no such rule 1.6e-5; such a block is one in 1e5 of an FFN's hidden rows (SiLU of deviation 7 times its like), none of normally distributed ones. The same goes for blocks below
+// large values of a block, but much where one or two stand alone and meet small weights. So a block of which one half (eight values) has none that reaches 2^-8 of the
+// largest and the other fewer than three has no digits: the threads that add the chunk multiply it out (`whole_blocks`). Rows of 1e4 beside values of size 1, one to a block, weights zero there: f32 2.6e-8 off, with ten digits and
+// no such rule 1.6e-5; such a block is less than one in 1e5 of an FFN's hidden rows (SiLU of deviation 7 times its like; the look at its values one in 300), none of normally distributed ones. The same goes for blocks below
 // 2^-17 of their chunk's largest value or below 2^-99, and for those with an infinity or NaN.
 // fs[row]: 2^(Emax - 8) and the blocks without digits (block b: bit 2 b).
 constexpr float TO_INT = 12582912.0f;  // 3 x 2^22: a sum with it has the nearest whole number in its mantissa (ties to even)
@@ -58,32 +58,30 @@ template <bool F32>
 __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* bs, uint8_t* sf, int row, float2* fs) {
     constexpr int LV = digits_of(F32);
     constexpr uint32_t LEAST = 28u, EXP = F32 ? 23u : 7u;  // least biased E: all scales are numbers
-    uint32_t u[F32 ? 8 : 4], pair[4], top;  // largest values of four pairs, and of the block
+    uint32_t u[F32 ? 8 : 4], mine;  // the lane's largest value
     u[0] = raw[0].x, u[1] = raw[0].y, u[2] = raw[0].z, u[3] = raw[0].w;
     if constexpr (F32) {
         u[4] = raw[1].x, u[5] = raw[1].y, u[6] = raw[1].z, u[7] = raw[1].w;
+        mine = u[0] & 0x7fffffffu;
 #pragma unroll
-        for (int i = 0; i < 4; i++) pair[i] = max(u[2 * i] & 0x7fffffffu, u[2 * i + 1] & 0x7fffffffu);
+        for (int i = 1; i < 8; i++) mine = max(mine, u[i] & 0x7fffffffu);
     } else {
-        const uint32_t a = __vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), b = __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu);
-        pair[0] = a & 0xffffu, pair[1] = a >> 16, pair[2] = b & 0xffffu, pair[3] = b >> 16;
+        mine = __vmaxu2(__vmaxu2(u[0] & 0x7fff7fffu, u[1] & 0x7fff7fffu), __vmaxu2(u[2] & 0x7fff7fffu, u[3] & 0x7fff7fffu));
+        mine = max(mine >> 16, mine & 0xffffu);
     }
-    top = max(max(pair[0], pair[1]), max(pair[2], pair[3]));
-    top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));  // two lanes hold a block of 16
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 1), top = max(mine, other);  // two lanes hold a block of 16
     uint32_t e = top >> EXP;
     bool none = e == 255u;  // infinity, NaN
     const uint32_t emax = max(__reduce_max_sync(0xffffffffu, none ? 0u : e), LEAST);
     const uint32_t limit = (max(e, 9u) - 8u) << EXP;
     none |= top != 0u && (e + 17u < emax || e < LEAST);
-    int large = (pair[0] >= limit) + (pair[1] >= limit) + (pair[2] >= limit) + (pair[3] >= limit);
-    large += __shfl_xor_sync(0xffffffffu, large, 1);
     uint32_t blocks = 0u;
-    if (__any_sync(0xffffffffu, none || (top != 0u && large < 3))) {
-        large = 0;
+    if (__any_sync(0xffffffffu, none || (top != 0u && min(mine, other) < limit))) {
+        int large = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) large += (F32 ? u[i] & 0x7fffffffu : (u[i >> 1] >> (16 * (i & 1))) & 0x7fffu) >= limit;
         large += __shfl_xor_sync(0xffffffffu, large, 1);
-        none |= top != 0u && large < 3;
+        none |= top != 0u && min(mine, other) < limit && large < 3;
         blocks = __ballot_sync(0xffffffffu, none) & 0x55555555u;
 #pragma unroll
         for (int i = 0; i < (F32 ? 8 : 4); i++) u[i] = none ? 0u : u[i];

@@ -234,10 +234,11 @@ def test_small_values_count_where_the_large_ones_beside_them_meet_zero_weights(e
     # the result's rounding (half a unit in the last place); sums of exact products in f32: a column of digits is the nearest f32 or the one beside it, so are the sums of
     # columns and chunks
     bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24) * want.abs() + 2.0 ** -22 * total
-    # digits end at 2^-22 (f32: 2^-34) of a block's largest value, unless fewer than three of its values reach 2^-8 of that
+    # digits end at 2^-22 (f32: 2^-34) of a block's largest value, unless one half of the block has none that reaches 2^-8 of that and the other fewer than three
     blocks = xd.double().abs().view(m, -1, 16)
     largest, third = blocks.amax(2, keepdim=True), blocks.topk(3, dim=2).values[:, :, 2:]
-    largest = torch.where(third < largest * 2.0 ** -9, 0.0, largest).expand(-1, -1, 16).reshape(m, k)
+    half = blocks.view(m, -1, 2, 8).amax(3).amin(2)[:, :, None]
+    largest = torch.where(torch.maximum(third, half) < largest * 2.0 ** -9, 0.0, largest).expand(-1, -1, 16).reshape(m, k)
     bound += (2.0 ** -23 if dtype == torch.bfloat16 else 2.0 ** -35) * (2 * largest @ w64.abs().t())
     if every != 2 and dtype == torch.float32:
         assert (y - want).norm() <= 1e-7 * want.norm()
