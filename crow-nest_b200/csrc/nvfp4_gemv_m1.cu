@@ -794,9 +794,10 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // 4.7 / 4.8, 8192 x 3072 5.9 / 5.3 and 7.6 / 7.1, gate / up of 3584 x 3328 6.7 / 5.7 and 8.6 / 7.7; but 10000 x 1536 4.5 / 4.9 and 5.2 / 6.4, 12288 x 2560 6.1 / 6.6 and 7.4 /
     // 8.5, 25949 x 1024 5.1 / 6.6 and 5.9 / 9.5, gate / up of 6144 x 2560 6.2 / 6.5 and 7.4 / 9.3. (One row of a few gate / up matrices of 4096 to 4608 values is slower there: 3072 x 4352
     // 6.4 / 5.9, four 7.5 / 8.6.) Few long rows stay too: its clusters end at
-    // eight CTAs a tile of 128 rows (640 x 17408 6.3 / 5.8, 512 x 16384 5.9 / 4.9, 2048 x 16384 7.7 / 8.1). A row that does not fit here is refused as it was.
+    // eight CTAs a tile of 128 rows (640 x 17408 6.3 / 5.8, 512 x 16384 5.9 / 4.9, 2048 x 16384 7.7 / 8.1). A row that does not fit here is refused as it was, and so are lines
+    // of rows shorter than 2048 values, below.
     const long long all_rows = (long long)rows * (gu ? 2 : 1);
-    if (!routed && all_rows * k >= 8000000 && (k >= 4096 || all_rows >= 10000) && !(all_rows <= 1280 && k > 14336)) {
+    if (!routed && all_rows * k >= 8000000 && (k >= 4096 || all_rows >= 10000) && !(all_rows <= 1280 && k > 14336) && !(a.line_bases && tx != 32)) {
         const int bp = bpr / one.parts;
         if (front_bytes(2, (bp + tx - 1) / tx, 1, 1, bp, 0) + 2 * stage_bytes <= sm_share(one.cps)) return cn_gemv_tc_launch(a, stream, who);
     }

@@ -158,6 +158,18 @@ def test_lines_of_a_larger_slice():
     assert np.array_equal(got[1, 800:], dense.pack_lines(bits, dense.line_number(5, 9))) and not got[0].any() and not got[1, :800].any()
 
 
+def test_lines_of_short_rows_are_refused():
+    import ctypes as C
+    from crownest_b200 import CrownestError
+    w = ops.Fp4(torch.zeros(12288 * 16 * 36, dtype=torch.uint8, device="cuda"), torch.ones(1, device="cuda"), 12288, 1024)
+    x, y = torch.zeros((1, 1024), dtype=torch.bfloat16, device="cuda"), torch.zeros((1, 12288), dtype=torch.bfloat16, device="cuda")
+    peer, epoch = torch.zeros((2, 3072 * 2, 4), dtype=torch.int32, device="cuda"), torch.zeros(16, dtype=torch.int32, device="cuda")
+    with pytest.raises(CrownestError, match="k >= 2048"):
+        ops.launch_gemv_lines(w, x, y, ((C.c_ulonglong * 2)(peer.data_ptr(), 0), 2, 0, 2 * 3072 * 16, epoch.data_ptr(), 9, 1, 0))
+    torch.cuda.synchronize()
+    assert not peer.any() and not y.any()
+
+
 def test_a_chain_of_calls_in_a_graph():
     """Kernels of a stream start before the one in front has ended: 40 dependent calls, replayed, give the bits of calls one by one."""
     _, w, _ = _make(4096, 4096, 6, 0.02)
