@@ -443,7 +443,7 @@ def gemv_arm(args, rank, world, local):
                        "l2": f"{copies} distinct weight copies ({copies * nb / 2 ** 20:.0f} MiB) rotated launch by launch: larger than L2",
                        "launch": f"CUDA graph replay of {per_graph} launches"},
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None, "peak_kind": peak_kind,
-                         "kernel": "fp8_gemv_tc_kernel" if op == "fp8" else "nvfp4_gemv_tc_kernel" if nb >= 4.5e6 and (k >= 4096 or nb / k >= 5625) else "nvfp4_gemv_m1_kernel", "bytes_per_launch": bytes_launch, "us_per_launch": us},
+                         "kernel": "fp8_gemv_tc_kernel" if op == "fp8" else "nvfp4_gemv_tc_kernel" if nb >= 4.5e6 and (k >= 4096 or nb / k >= 5625) and not (nb / k <= 720 and k > 14336) else "nvfp4_gemv_m1_kernel", "bytes_per_launch": bytes_launch, "us_per_launch": us},
             "blocks": t["blocks"], "ms_per_step_min": t["ms_per_step_min"], "ms_per_step_max": t["ms_per_step_max"],
             "e2e": {"value": bytes_launch / e2e_s / 1e9, "unit": UNIT, "h2d_bytes_per_step": x_host.numel() * 2, "d2h_bytes_per_step": y_host.numel() * 2,
                     "note": "one launch per host call"},
