@@ -352,7 +352,7 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
         if (rc != CN_OK) break;
         GemvCall s = {};
         s.w0 = shared_down, s.gs0 = shared_gs + 2, s.x = p->hs + (size_t)t0 * p->shared_inter, s.y = p->ys + (size_t)t0 * p->hidden;
-        s.rows = p->hidden, s.k = p->shared_inter, s.m = m, s.ldy = p->hidden, s.dtype = CN_F32, s.out_f32 = 1, s.x_f16_ok = 0;
+        s.rows = p->hidden, s.k = p->shared_inter, s.m = m, s.ldy = p->hidden, s.dtype = CN_F32, s.out_f32 = 1;
         rc = cn_gemv_launch(s, p->side, "cn_moe_nvfp4_run (shared down)");
     }
     CN_CUDA(cudaEventRecord(p->join, p->side));
@@ -417,7 +417,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     if (combos >= ROWS_COMBOS && short_rows) return cn_rows_launch(one, stream, "cn_moe_nvfp4 (down)");
     GemvCall d = {};
     d.gs0 = gs_dn, d.x = p->h, d.y = eo, d.yptrs = eo_ptrs, d.rows = p->hidden, d.k = p->inter, d.m = 1, d.ldy = p->hidden, d.dtype = CN_F32, d.out_f32 = 1;
-    d.x_f16_ok = 0, d.ids = ids, d.order = nullptr, d.tab0 = table_dn, d.x_div = 1, d.combos = combos, d.experts = p->experts;
+    d.ids = ids, d.order = nullptr, d.tab0 = table_dn, d.x_div = 1, d.combos = combos, d.experts = p->experts;
     return cn_gemv_launch(d, stream, "cn_moe_nvfp4 (down)");
 }
 

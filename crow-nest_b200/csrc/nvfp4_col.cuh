@@ -3,26 +3,6 @@
 #pragma once
 #include "common.cuh"
 
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float2 lds64f(uint32_t a) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t hmul2u(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
 // Two scale bytes of a word, `shift` = 8 (t >> 1): bytes t >> 1 and 2 + (t >> 1), as f16x2 of scale x 2^-8: an E4M3 byte shifted left by
 // seven is that f16 as it stands, subnormals included. The engine's reading: bit 7 ignored, 0x7F read as 0x7E.
 __device__ __forceinline__ __half2 lane_scales(uint32_t w, uint32_t shift) {
@@ -97,66 +77,4 @@ __device__ __forceinline__ float f32_planes(const uint4& lo, const uint4& hi, in
         h[0][q] = *(const uint32_t*)&h0, h[1][q] = *(const uint32_t*)&h1, h[2][q] = *(const uint32_t*)&h2;
     }
     return __uint_as_float((e - 6u) << 23);
-}
-// The same for eight bf16 values: one plane, exact.
-__device__ __forceinline__ float bf16_plane(const uint4& raw, int lane, uint32_t h[1][4]) {
-    const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
-    uint32_t e = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint32_t ea = (u[q] >> 7) & 0xFF, eb = (u[q] >> 23) & 0xFF;
-        e = max(e, max(ea == 255u ? 0u : ea, eb == 255u ? 0u : eb));
-    }
-    const uint32_t gm = 0xffu << (lane & 24);
-    e = max(e, __shfl_xor_sync(gm, e, 1));
-    e = max(e, __shfl_xor_sync(gm, e, 2));
-    e = max(e, __shfl_xor_sync(gm, e, 4));
-    e = e < 15 ? 15 : e;
-    const float mul = __uint_as_float((268u - e) << 23);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const __half2 hh = __floats2half2_rn(__uint_as_float(u[q] << 16) * mul, __uint_as_float(u[q] & 0xffff0000u) * mul);
-        h[0][q] = *(const uint32_t*)&hh;
-    }
-    return __uint_as_float((e - 6u) << 23);
-}
-
-// ---------------------------------------------------------------- tiles of short rows, by their warp's own asynchronous copies
-// 16 row pieces of eight blocks (288 bytes) -> shared memory, PIECE_PITCH apart: nine 16-byte copies of each lane instead of a bulk copy for every
-// piece, whose number and not size is what the copy engine takes its time for.
-constexpr int PIECE_PITCH = 8 * 36 + 16, PIECE_TILE = 16 * PIECE_PITCH;
-struct PieceCopy {
-    uint32_t at[9];  // copy i of this lane: row in the lower half, 16-byte part of the piece in the upper
-    __device__ __forceinline__ explicit PieceCopy(int lane) {
-#pragma unroll
-        for (int i = 0; i < 9; i++) {
-            const uint32_t n = 32u * i + lane, r = n / 18u;
-            at[i] = r | ((n - 18u * r) << 16);
-        }
-    }
-    // rows 0 .. have_lo - 1 of lo and, as rows 8 and on, 0 .. have_hi - 1 of hi; parts of 16 bytes in a piece: 18, or 9 for half of one
-    __device__ __forceinline__ void operator()(uint32_t dst, const uint8_t* lo, const uint8_t* hi, uint32_t row_bytes, uint32_t have_lo, uint32_t have_hi, uint32_t parts,
-                                               uint64_t policy) const {
-#pragma unroll
-        for (int i = 0; i < 9; i++) {
-            const uint32_t r = at[i] & 0xffffu, part = at[i] >> 16;
-            const bool upper = r >= 8u;
-            if (part < parts && (r & 7u) < (upper ? have_hi : have_lo))
-                asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + r * PIECE_PITCH + part * 16u),
-                             "l"((upper ? hi : lo) + (size_t)((r & 7u) * row_bytes + part * 16u)), "l"(policy)
-                             : "memory");
-        }
-    }
-};
-__device__ __forceinline__ void piece_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// all but the n youngest groups of this thread's copies have landed (n <= 3)
-__device__ __forceinline__ void piece_wait(int n) {
-    if (n <= 0)
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    else if (n == 1)
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else if (n == 2)
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-    else
-        asm volatile("cp.async.wait_group 3;" ::: "memory");
 }

@@ -148,6 +148,63 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
 // a chunk's factor in 64 bits (a normal power of two)
 __device__ __forceinline__ double power_of_two(float f) { return __hiloint2double((int)((__float_as_uint(f) >> 3) + (896u << 20)), 0); }
 
+// ---------------------------------------------------------------- container blocks -> operand layout (a lane: the four blocks of a row)
+constexpr int A_CODES = 128 * 128, A_STAGE = A_CODES + 4 * 512;  // a chunk of 128 rows as operand A: 128-byte swizzled rows, then the scales of the four MMAs
+
+// A row's 144 bytes at src into registers, scale bytes as the tensor core is to read them; whether any row of the warp has one of 0xFF: that stands for 480, which it does not know, and is
+// nothing here (`whole_blocks` multiplies the block out).
+__device__ __forceinline__ uint32_t load_row(const uint4* src, uint32_t (&v)[36]) {
+#pragma unroll
+    for (int j = 0; j < 9; j++) {
+        const uint4 q = src[j];
+        v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
+    }
+    uint32_t odd = 0u;
+#pragma unroll
+    for (int b = 0; b < 4; b++) odd |= v[9 * b] & ((v[9 * b] & 0x7f7f7f7fu) + 0x01010101u);
+    odd = __any_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        const uint32_t sc = v[9 * b];
+        v[9 * b] = scale_bytes_rule(sc);
+        if (odd) {
+            const uint32_t ff = sc & ((sc & 0x7f7f7f7fu) + 0x01010101u) & 0x80808080u;
+            v[9 * b] &= ~(ff - (ff >> 7));
+        }
+    }
+    return odd;
+}
+// row 32 w + lane of the operand stage at dst
+__device__ __forceinline__ void store_row(uint8_t* dst, int w, int lane, const uint32_t (&v)[36]) {
+    uint8_t* line = dst + (w * 32 + lane) * 128;
+    const uint32_t sw = (uint32_t)(lane & 7);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
+        *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
+        *(uint32_t*)(dst + A_CODES + b * 512 + lane * 16 + w * 4) = v[9 * b];
+    }
+}
+
+// ---------------------------------------------------------------- sums
+// A row's columns of digits into its sum over the chunk, in units of the highest digit: from the smallest up; f32: what the last two additions round off into `rest`.
+template <bool F32>
+__device__ __forceinline__ float sum_digits(const uint32_t* d, float& rest) {
+    constexpr int LV = digits_of(F32), PLAIN = F32 ? LV - 2 : LV;
+    float s = __uint_as_float(d[0]);
+    rest = 0.0f;
+#pragma unroll
+    for (int j = 1; j < PLAIN; j++) s = fmaf(s, 0.125f, __uint_as_float(d[j]));
+#pragma unroll
+    for (int j = PLAIN; j < LV; j++) {
+        const float a = s * 0.125f, b = __uint_as_float(d[j]);
+        s = a + b;
+        const float bb = s - a;
+        rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
+    }
+    return s;
+}
+
 // Blocks of 16 without digits (`blocks`, bit 2 b) and, where `odd`, those whose scale byte is 0xFF (480, which the tensor core does not know and is given as nothing), from global memory: the
 // row's 144 container bytes at wr times 256 values at x. All that a block (bf16: two blocks) needs is
 // asked for at once: what it costs is the way to memory. f32: products and sums in 64 bits. One row of gate / up 17408 x 5120 with a NaN 21.9 -> 22.6 us, 4096 x 4096 4.7 -> 6.3;

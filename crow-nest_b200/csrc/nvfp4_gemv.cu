@@ -1,5 +1,5 @@
-// NVFP4 GEMV for M = 1..8 activation rows on sm_100a: the decode projection of the dense family
-// and its small-M (speculative verify) form, plain or with the fused gate/up activation.
+// NVFP4 GEMV for M = 1..8 f32 activation rows of smaller matrices and for the f32 rows of single routed experts (bf16 rows: nvfp4_gemv_m1.cu; larger matrices of either type:
+// nvfp4_gemv_tc.cu; the rules are in cn_gemv_launch and cn_gemv_m1_launch), plain or with the fused gate/up activation.
 //
 // Supersedes gemv_nvfp4_w / _gu / _wm / _gum (engine/src/kernels_p2.rs:355-530) and the record
 // kernels gemv_fp4(_b) (engine/src/kernels.rs:118-189), glm5_gemv_fp4 (engine/src/kernels_glm5_moe.cu:284).
@@ -9,14 +9,10 @@
 //     through a ring of shared-memory stages with 1-D bulk copies (TMA, completion counted on an
 //     mbarrier), one piece of TX 36-byte blocks per row and stage; it never waits for anything
 //     but a free stage, so the weight stream runs ahead of the arithmetic;
-//   - a second helper warp stages the matching slice of the M activation rows, converted once
-//     per CTA: bf16 -> f16 with a power-of-two scale per 64-value block (exact; the inverse is
-//     applied with the block's partial sum), or f32 kept as f32;
+//   - the activation rows are staged once per CTA, as they are;
 //   - consumer warps: lane (ry, tx) owns k-block tx of the stage for RT rows; the nine words of a
 //     block are read with conflict-free 4-byte loads (36-byte stride), codes are decoded in
-//     registers (cvt.rn.f16x2.e2m1x2: every E2M1 value is exact in f16) and multiplied with
-//     fma.rn.f32.f16 (f16 x f16 product exact, f32 accumulate; measured at the FFMA rate on
-//     B200), each 16-value sub-block's partial sum is multiplied by its UE4M3 scale * tensor
+//     registers (cvt.rn.f16x2.e2m1x2: every E2M1 value is exact in f16) and multiplied in f32, each 16-value sub-block's partial sum is multiplied by its UE4M3 scale * tensor
 //     scale (a 256-entry table, the reference's scale_lut) and accumulated in f32; the K split
 //     over the TX lanes is reduced with xor shuffles in a fixed order.
 // Each (row, m) pair runs the same instruction sequence whatever M is, so row m of an M-row call
@@ -32,48 +28,13 @@ namespace {
 constexpr int NW = 4;  // consumer warps
 constexpr int NTHREADS = (NW + 1) * 32;
 constexpr int MAX_STAGES = 8;
-constexpr int XB_F16 = 144;  // bytes of one k-block's 64 activations as f16, padded: conflict-free 16-byte loads
-constexpr int XB_F32 = 272;  // the same as f32
-constexpr int XB_SWZ = 128;  // bf16 rows staged by TMA, converted in place: 16-byte chunks XOR-swizzled instead of padded
+constexpr int XB = 272;  // bytes of one k-block's 64 activations, padded: conflict-free 16-byte loads
 constexpr int HDR_BYTES = 256 + 2048;  // barriers, two scale tables
 
-// one load group of eight activation values: raw words in flight, widened exactly to f32 on use
-template <int XT>
-struct XRaw {
-    uint4 a;
-    uint4 b;  // f32 input only
-};
-template <int XT>
-__device__ __forceinline__ void load_x8(const void* x, size_t at, XRaw<XT>& r) {
-    if (XT == 1) {
-        r.a = *(const uint4*)((const __nv_bfloat16*)x + at);
-    } else {
-        r.a = *(const uint4*)((const float*)x + at);
-        r.b = *(const uint4*)((const float*)x + at + 4);
-    }
-}
-template <int XT>
-__device__ __forceinline__ void widen_x8(const XRaw<XT>& r, float v[8]) {
-    if (XT == 1) {
-        const uint32_t u[4] = {r.a.x, r.a.y, r.a.z, r.a.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            v[2 * i] = __uint_as_float(u[i] << 16);
-            v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-        }
-    } else {
-        v[0] = __uint_as_float(r.a.x), v[1] = __uint_as_float(r.a.y), v[2] = __uint_as_float(r.a.z), v[3] = __uint_as_float(r.a.w);
-        v[4] = __uint_as_float(r.b.x), v[5] = __uint_as_float(r.b.y), v[6] = __uint_as_float(r.b.z), v[7] = __uint_as_float(r.b.w);
-    }
-}
-
-// XT: 0 = f32 activations/outputs, 1 = bf16. MP: activation rows compiled in (1, 2, 4, 8).
-// RT: rows per consumer thread. MODE: 0 = f32 FMA, 1 = f16 x f16 + f32 mixed FMA (bf16 input only).
-template <int XT, int MP, int RT, int MODE>
+// MP: activation rows compiled in (1, 2, 4, 8). RT: rows per consumer thread.
+template <int MP, int RT>
 __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr bool SWZ = XT == 1 && MODE == 1;
-    constexpr int XB = SWZ ? XB_SWZ : (MODE == 1 ? XB_F16 : XB_F32);
     const int TX = p.tx;
     const int G = NW * (32 / TX);  // row groups per CTA
     const int ROWS = G * RT;       // row slots per stage
@@ -96,7 +57,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
         if ((int)blockIdx.y >= p.combos) {  // a row of the side pair
             const int row = (int)blockIdx.y - p.combos;
             w0 = p.side_w0, w1 = p.side_w1, rows = p.side_rows, gs0 = p.side_gs, gs1 = p.side_gs + 1;
-            xbase += (size_t)row * p.k * (XT == 1 ? 2 : 4);
+            xbase += (size_t)row * p.k * 4;
             ybase = (char*)(p.side_y + (size_t)row * rows);
         } else {
             const int c = p.order ? p.order[blockIdx.y] : (int)blockIdx.y;
@@ -105,19 +66,17 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
             w0 = (const uint8_t*)p.tab0[e];
             if (!w0) return;  // the expert is not resident here: nothing to read or write
             w1 = p.tab1 ? (const uint8_t*)p.tab1[e] : (p.fused_up_rows > 0 ? w0 + (size_t)p.fused_up_rows * row_bytes : nullptr);
-            xbase += (size_t)(c / p.x_div) * p.k * (XT == 1 ? 2 : 4);
-            ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * ((XT == 1 && !p.out_f32) ? 2 : 4);
+            xbase += (size_t)(c / p.x_div) * p.k * 4;
+            ybase = p.yptrs ? (char*)p.yptrs[c] : ybase + (size_t)c * p.ldy * 4;
         }
     }
     const bool gu = w1 != nullptr;
 
     uint64_t* full = (uint64_t*)smem;
     uint64_t* empty = full + MAX_STAGES;
-    uint64_t* xbar = empty + MAX_STAGES;  // the activation rows have landed
     float* lut = (float*)(smem + 256);    // [2][256]
     uint8_t* xs0 = smem + HDR_BYTES;                              // [MP][bpr][XB] staged activations
-    float* xinv0 = (float*)(xs0 + (size_t)MP * bpr * XB);         // [MP][bpr] inverse block scales
-    uint8_t* stage0 = (uint8_t*)(xinv0 + ((MP * bpr + 3) & ~3));  // the weight ring
+    uint8_t* stage0 = xs0 + (size_t)MP * bpr * XB;                // the weight ring
     const int stage_bytes = ROWS * piece;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -131,7 +90,6 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
             mbar_init(&full[s], 1);  // the producer's expect_tx arrive; the copies count bytes
             mbar_init(&empty[s], NW);
         }
-        mbar_init(xbar, 1);
         mbar_fence_init();
     }
     // scale tables: ue4m3(rule(byte)) * gs, the product the reference tabulates (cpu_nvfp4.rs:98)
@@ -191,115 +149,33 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
     // the weight ring. Groups of 8 values; lane & 7 = position in the 64-value block, so the 8
     // lanes of a block sit side by side. All loads of a batch are in flight before the first
     // conversion (one L2 round trip per batch, not per group).
-    if (SWZ) {
-        // bf16 rows: one bulk copy per row into shared memory, then an in-place conversion to f16 with a
-        // power-of-two scale per 64-value block. A thread owns whole 128-byte blocks (no exchange) and
-        // writes the eight 16-byte chunks of block b at chunk index i ^ (b & 7): conflict-free 16-byte
-        // loads for eight lanes reading eight consecutive blocks, without padding.
-        if (tid == 0) {
-            pdl_wait();  // activations may come from the previous kernel of the stream
-            mbar_expect_tx(xbar, (uint32_t)p.m * (uint32_t)p.k * 2u);
-            mbar_arrive(xbar);
-            for (int m = 0; m < p.m; m++) bulk_g2s(xs0 + (size_t)m * bpr * XB, xbase + (size_t)m * p.k * 2, (uint32_t)p.k * 2u, xbar);
-        }
-        if (!mbar_wait(xbar, 0)) {
-            cn_dev_fail(CN_DEV_WAIT_FULL);
-            return;
-        }
-        for (int b = tid; b < MP * bpr; b += NW * 32) {
-            const int m = b / bpr;
-            uint4* blkp = (uint4*)(xs0 + (size_t)b * XB);
-            uint4 raw[8];
+    pdl_wait();  // activations may come from the previous kernel of the stream
+    constexpr int BATCH = 4;
+    const int groups = MP * bpr * 8;
+    for (int g0 = 0; g0 < groups; g0 += BATCH * NW * 32) {
+        uint4 raw[BATCH][2];
 #pragma unroll
-            for (int i = 0; i < 8; i++) raw[i] = m < p.m ? blkp[i] : make_uint4(0, 0, 0, 0);
-            float amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t u[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    amax = fmaxf(amax, fabsf(__uint_as_float(u[q] << 16)));
-                    amax = fmaxf(amax, fabsf(__uint_as_float(u[q] & 0xffff0000u)));
-                }
-            }
-            uint32_t e = (__float_as_uint(amax) >> 23) & 0xFF;
-            float mul = 1.0f, inv = 1.0f;
-            if (amax > 0.0f && e < 255) {
-                e = e < 15 ? 15 : e;
-                mul = __uint_as_float((268u - e) << 23);
-                inv = __uint_as_float((e - 14u) << 23);
-            }
-            const int sw = (b % bpr) & 7;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const uint32_t u[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-                uint32_t h[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const __half2 hh = __floats2half2_rn(__uint_as_float(u[q] << 16) * mul, __uint_as_float(u[q] & 0xffff0000u) * mul);
-                    h[q] = *(const uint32_t*)&hh;
-                }
-                blkp[i ^ sw] = make_uint4(h[0], h[1], h[2], h[3]);
-            }
-            xinv0[b] = inv;
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
-    } else {
-        pdl_wait();  // activations may come from the previous kernel of the stream
-        constexpr int BATCH = 4;
-        const int groups = MP * bpr * 8;
-        for (int g0 = 0; g0 < groups; g0 += BATCH * NW * 32) {
-            XRaw<XT> raw[BATCH];
-#pragma unroll
-            for (int b = 0; b < BATCH; b++) {
-                const int gq = g0 + b * NW * 32 + tid;
-                const int m = gq / (bpr * 8), gi = gq % (bpr * 8);
-                raw[b].a = make_uint4(0, 0, 0, 0);
-                raw[b].b = make_uint4(0, 0, 0, 0);
-                if (gq < groups && m < p.m) load_x8<XT>(xbase, (size_t)m * p.k + (size_t)gi * 8, raw[b]);
-            }
-#pragma unroll
-            for (int b = 0; b < BATCH; b++) {
-                const int gq = g0 + b * NW * 32 + tid;
-                const int m = gq / (bpr * 8), gi = gq % (bpr * 8), kb = gi >> 3, wi = gi & 7;
-                const bool live = gq < groups;  // uniform over each aligned group of 8 lanes
-                uint8_t* dst = xs0 + (size_t)(m * bpr + kb) * XB;
-                float vv[8];
-                widen_x8<XT>(raw[b], vv);
-                if (MODE == 1) {
-                    // power-of-two scale per 64-value block: |x| * mul < 2^15, exact in f16
-                    float amax = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(vv[i]));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                    uint32_t e = (__float_as_uint(amax) >> 23) & 0xFF;
-                    float mul = 1.0f, inv = 1.0f;
-                    if (amax > 0.0f && e < 255) {
-                        e = e < 15 ? 15 : e;
-                        mul = __uint_as_float((268u - e) << 23);
-                        inv = __uint_as_float((e - 14u) << 23);
-                    }
-                    if (live) {
-                        uint32_t h[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const __half2 hh = __floats2half2_rn(vv[2 * i] * mul, vv[2 * i + 1] * mul);
-                            h[i] = *(const uint32_t*)&hh;
-                        }
-                        *(uint4*)(dst + wi * 16) = make_uint4(h[0], h[1], h[2], h[3]);
-                        if (wi == 0) xinv0[m * bpr + kb] = inv;
-                    }
-                } else if (live) {
-                    *(float4*)(dst + wi * 32) = make_float4(vv[0], vv[1], vv[2], vv[3]);
-                    *(float4*)(dst + wi * 32 + 16) = make_float4(vv[4], vv[5], vv[6], vv[7]);
-                }
+        for (int b = 0; b < BATCH; b++) {
+            const int gq = g0 + b * NW * 32 + tid;
+            const int m = gq / (bpr * 8), gi = gq % (bpr * 8);
+            raw[b][0] = raw[b][1] = make_uint4(0, 0, 0, 0);
+            if (gq < groups && m < p.m) {
+                const uint4* x = (const uint4*)((const float*)xbase + (size_t)m * p.k + (size_t)gi * 8);
+                raw[b][0] = x[0], raw[b][1] = x[1];
             }
         }
-        // the consumer warps only (the producer warp is streaming): named barrier 1
-        asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) {
+            const int gq = g0 + b * NW * 32 + tid;
+            const int m = gq / (bpr * 8), gi = gq % (bpr * 8), kb = gi >> 3, wi = gi & 7;
+            if (gq < groups) {
+                uint4* dst = (uint4*)(xs0 + (size_t)(m * bpr + kb) * XB + wi * 32);
+                dst[0] = raw[b][0], dst[1] = raw[b][1];
+            }
+        }
     }
+    // the consumer warps only (the producer warp is streaming): named barrier 1
+    asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
     const int txi = lane % TX, ry = lane / TX;
     const int g = warp * (32 / TX) + ry;
     float acc[RT][MP];
@@ -330,84 +206,43 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
             for (int m = 0; m < MP; m++) blk[r][m] = 0.0f;
 #pragma unroll
         for (int sb = 0; sb < 4; sb++) {
-            if (MODE == 1) {
-                uint4 xa[MP], xb[MP];
-#pragma unroll
-                for (int m = 0; m < MP; m++) {
-                    const uint4* xp = (const uint4*)(xs + (size_t)m * bpr * XB);
-                    if (SWZ) {
-                        const int sw = (c * TX + txi) & 7;
-                        xa[m] = xp[(2 * sb) ^ sw];
-                        xb[m] = xp[(2 * sb + 1) ^ sw];
-                    } else {
-                        xa[m] = xp[2 * sb];
-                        xb[m] = xp[2 * sb + 1];
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < RT; r++) {
-                    const float sc = lut[((gu && (r & 1)) ? 256 : 0) + ((wv[r][0] >> (8 * sb)) & 0xFF)];
-                    const uint32_t c0 = wv[r][1 + 2 * sb], c1 = wv[r][2 + 2 * sb];
-                    uint32_t h[8];
-                    e2m1x8_to_f16x2(c0, h);
-                    e2m1x8_to_f16x2(c1, h + 4);
-#pragma unroll
-                    for (int m = 0; m < MP; m++) {
-                        const uint32_t xv[8] = {xa[m].x, xa[m].y, xa[m].z, xa[m].w, xb[m].x, xb[m].y, xb[m].z, xb[m].w};
-                        float p0 = 0.0f, p1 = 0.0f;  // even / odd values: two independent chains
-#pragma unroll
-                        for (int i = 0; i < 8; i++) fma2_f16_f32(p0, p1, h[i], xv[i]);
-                        blk[r][m] = fmaf(p0 + p1, sc, blk[r][m]);
-                    }
-                }
-            } else {
-                float xv[MP][16];
-#pragma unroll
-                for (int m = 0; m < MP; m++) {
-                    const float4* xp = (const float4*)(xs + (size_t)m * bpr * XB + sb * 64);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const float4 t = xp[i];
-                        xv[m][4 * i] = t.x, xv[m][4 * i + 1] = t.y, xv[m][4 * i + 2] = t.z, xv[m][4 * i + 3] = t.w;
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < RT; r++) {
-                    const float sc = lut[((gu && (r & 1)) ? 256 : 0) + ((wv[r][0] >> (8 * sb)) & 0xFF)];
-                    const uint32_t c0 = wv[r][1 + 2 * sb], c1 = wv[r][2 + 2 * sb];
-                    float wf[16];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const uint32_t h0 = e2m1x2_to_f16x2((c0 >> (8 * i)) & 0xFF), h1 = e2m1x2_to_f16x2((c1 >> (8 * i)) & 0xFF);
-                        wf[2 * i] = f16lo_to_f32(h0), wf[2 * i + 1] = f16hi_to_f32(h0);
-                        wf[8 + 2 * i] = f16lo_to_f32(h1), wf[8 + 2 * i + 1] = f16hi_to_f32(h1);
-                    }
-#pragma unroll
-                    for (int m = 0; m < MP; m++) {
-                        float p0 = 0.0f, p1 = 0.0f;
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            p0 = fmaf(wf[2 * i], xv[m][2 * i], p0);
-                            p1 = fmaf(wf[2 * i + 1], xv[m][2 * i + 1], p1);
-                        }
-                        blk[r][m] = fmaf(p0 + p1, sc, blk[r][m]);
-                    }
-                }
-            }
-        }
-        if (MODE == 1) {
+            float xv[MP][16];
 #pragma unroll
             for (int m = 0; m < MP; m++) {
-                const float inv = xinv0[m * bpr + c * TX + txi];
+                const float4* xp = (const float4*)(xs + (size_t)m * bpr * XB + sb * 64);
 #pragma unroll
-                for (int r = 0; r < RT; r++) acc[r][m] = fmaf(blk[r][m], inv, acc[r][m]);
+                for (int i = 0; i < 4; i++) {
+                    const float4 t = xp[i];
+                    xv[m][4 * i] = t.x, xv[m][4 * i + 1] = t.y, xv[m][4 * i + 2] = t.z, xv[m][4 * i + 3] = t.w;
+                }
             }
-        } else {
 #pragma unroll
-            for (int r = 0; r < RT; r++)
+            for (int r = 0; r < RT; r++) {
+                const float sc = lut[((gu && (r & 1)) ? 256 : 0) + ((wv[r][0] >> (8 * sb)) & 0xFF)];
+                const uint32_t c0 = wv[r][1 + 2 * sb], c1 = wv[r][2 + 2 * sb];
+                float wf[16];
 #pragma unroll
-                for (int m = 0; m < MP; m++) acc[r][m] += blk[r][m];
+                for (int i = 0; i < 4; i++) {
+                    const uint32_t h0 = e2m1x2_to_f16x2((c0 >> (8 * i)) & 0xFF), h1 = e2m1x2_to_f16x2((c1 >> (8 * i)) & 0xFF);
+                    wf[2 * i] = f16lo_to_f32(h0), wf[2 * i + 1] = f16hi_to_f32(h0);
+                    wf[8 + 2 * i] = f16lo_to_f32(h1), wf[8 + 2 * i + 1] = f16hi_to_f32(h1);
+                }
+#pragma unroll
+                for (int m = 0; m < MP; m++) {
+                    float p0 = 0.0f, p1 = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        p0 = fmaf(wf[2 * i], xv[m][2 * i], p0);
+                        p1 = fmaf(wf[2 * i + 1], xv[m][2 * i + 1], p1);
+                    }
+                    blk[r][m] = fmaf(p0 + p1, sc, blk[r][m]);
+                }
+            }
         }
+#pragma unroll
+        for (int r = 0; r < RT; r++)
+#pragma unroll
+            for (int m = 0; m < MP; m++) acc[r][m] += blk[r][m];
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
@@ -429,12 +264,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
                 if (row < rows) {
 #pragma unroll
                     for (int m = 0; m < MP; m++)
-                        if (m < p.m) {
-                            if (XT == 1 && !p.out_f32)
-                                ((__nv_bfloat16*)ybase)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(acc[r][m]);
-                            else
-                                ((float*)ybase)[(size_t)m * p.ldy + row] = acc[r][m];
-                        }
+                        if (m < p.m) ((float*)ybase)[(size_t)m * p.ldy + row] = acc[r][m];
                 }
             }
         } else {
@@ -444,13 +274,7 @@ __global__ void __launch_bounds__(NTHREADS, (MP <= 2 ? 4 : 1)) nvfp4_gemv_kernel
                 if (row < rows) {
 #pragma unroll
                     for (int m = 0; m < MP; m++)
-                        if (m < p.m) {
-                            const float h = act_gu(acc[r][m], acc[r + 1][m], p.limit);
-                            if (XT == 1 && !p.out_f32)
-                                ((__nv_bfloat16*)ybase)[(size_t)m * p.ldy + row] = __float2bfloat16_rn(h);
-                            else
-                                ((float*)ybase)[(size_t)m * p.ldy + row] = h;
-                        }
+                        if (m < p.m) ((float*)ybase)[(size_t)m * p.ldy + row] = act_gu(acc[r][m], acc[r + 1][m], p.limit);
                 }
             }
         }
@@ -476,9 +300,9 @@ __global__ void nvfp4_dequant_kernel(const uint8_t* __restrict__ w, const float*
     }
 }
 
-template <int XT, int MP, int RT, int MODE>
+template <int MP, int RT>
 int launch_one(const GemvParams& p, int grid, int gy, size_t smem, cudaStream_t stream) {
-    auto kern = nvfp4_gemv_kernel<XT, MP, RT, MODE>;
+    auto kern = nvfp4_gemv_kernel<MP, RT>;
     CN_ALLOW_SMEM(kern, 200 * 1024);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, (unsigned)gy);
@@ -494,12 +318,15 @@ int launch_one(const GemvParams& p, int grid, int gy, size_t smem, cudaStream_t 
     return CN_OK;
 }
 
-template <int XT, int MODE>
+// Four rows per thread only for the many tiles of a routed call, which has one row: a plain call that large (9472 rows of 1024 values) is the tcgen05 kernel's.
 int launch_m(const GemvParams& p, int mp, int rt, int grid, int gy, size_t smem, cudaStream_t stream) {
-#define CN_CASE(MPV, RTV) \
-    if (mp == MPV && rt == RTV) return launch_one<XT, MPV, RTV, MODE>(p, grid, gy, smem, stream);
-    CN_CASE(1, 2) CN_CASE(1, 4) CN_CASE(2, 2) CN_CASE(2, 4) CN_CASE(4, 2) CN_CASE(4, 4) CN_CASE(8, 2) CN_CASE(8, 4)
-#undef CN_CASE
+    if (mp == 1 && rt == 4) return launch_one<1, 4>(p, grid, gy, smem, stream);
+    if (rt == 2) {
+        if (mp == 1) return launch_one<1, 2>(p, grid, gy, smem, stream);
+        if (mp == 2) return launch_one<2, 2>(p, grid, gy, smem, stream);
+        if (mp == 4) return launch_one<4, 2>(p, grid, gy, smem, stream);
+        if (mp == 8) return launch_one<8, 2>(p, grid, gy, smem, stream);
+    }
     CN_FAIL(CN_ERR_SHAPE, "nvfp4 gemv: no kernel for m %d, rows per thread %d", mp, rt);
 }
 
@@ -524,16 +351,15 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // k = 2048 the mma.sync kernel with three f16 planes that was there before took 3.2 and 8.1 for 2048 rows (3.5 and 5.4 now), at 17408 x 5120, gate / up, 26.6 and 84.6
     // (19.4 and 45.6). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
     // A rule of the matrix alone: a row's result does not depend on how many rows the call has.
-    if (!routed && !a.x_f16_ok && (k >= 2048 || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
-        if (k > 108544) CN_FAIL(CN_ERR_LIMIT, "%s: k = %d, f32 rows have up to 108544 values", who, k);
+    if (!routed && (k >= 2048 || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
+        if (k > 108544) CN_FAIL(CN_ERR_LIMIT,  // (the library's limit for f32 rows, as it was; this kernel has none)
+                                 "%s: k = %d, f32 rows have up to 108544 values", who, k);
         return cn_gemv_tc_launch(a, stream, who);
     }
     const bool gu = a.w1 != nullptr || a.tab1 != nullptr || a.fused_up_rows > 0;
     const int bpr = k / 64;
     const int tx = bpr % 16 == 0 ? 16 : (bpr % 8 == 0 ? 8 : 4);
     const int mp = m == 1 ? 1 : (m == 2 ? 2 : (m <= 4 ? 4 : 8));
-    // f32 activations keep exact f32 arithmetic unless the caller allows rounding them to f16 at staging
-    const int mode = (a.dtype == CN_BF16 || a.x_f16_ok) ? 1 : 0;
     const int G = NW * (32 / tx);
     int rt = 4;
     const long long slots = (long long)rows * (gu ? 2 : 1) * (routed ? a.combos : 1);
@@ -541,9 +367,8 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int ROWS = G * rt;
     const int per_cta = gu ? ROWS / 2 : ROWS;
     const int grid = ((routed && a.side_tokens > 0 && a.side_rows > rows ? a.side_rows : rows) + per_cta - 1) / per_cta;
-    const int xb = (mode == 1 && a.dtype == CN_BF16) ? XB_SWZ : (mode == 1 ? XB_F16 : XB_F32);
     const size_t stage_bytes = (size_t)ROWS * tx * 36;
-    const size_t xbytes = (size_t)mp * bpr * xb + (size_t)((mp * bpr + 3) & ~3) * 4;
+    const size_t xbytes = (size_t)mp * bpr * XB;
     const int nchunks = bpr / tx;
     // ring depth: enough bytes in flight per SM to cover the HBM latency (about 96 KB), shared between
     // the CTAs that will be resident together (at most four, fewer when the grid is small)
@@ -557,17 +382,16 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     stages = stages < 2 ? 2 : (stages > MAX_STAGES ? MAX_STAGES : stages);
     if (stages > nchunks) stages = nchunks < 1 ? 1 : nchunks;
     const size_t smem = HDR_BYTES + xbytes + stages * stage_bytes;
-    if (smem > 200 * 1024) {
+    if (smem + (size_t)mp * bpr * 4 > 200 * 1024) {  // (four bytes a block to spare: the limits are those of a layout that had a scale beside each)
         // the staged activations of all m rows do not fit one CTA: two calls over half the rows each
         // (each row's arithmetic is the same whatever the split, so results do not change)
         if (m == 1) CN_FAIL(CN_ERR_LIMIT, "%s: k = %d needs %zu B of shared memory per block", who, k, smem);
         const int m0 = m / 2;
-        const size_t es = a.dtype == CN_BF16 ? 2 : 4, eso = (a.dtype == CN_BF16 && !a.out_f32) ? 2 : 4;
         GemvCall lo = a, hi = a;
         lo.m = m0;
         hi.m = m - m0;
-        hi.x = (const char*)a.x + (size_t)m0 * k * es;
-        hi.y = (char*)a.y + (size_t)m0 * a.ldy * eso;
+        hi.x = (const float*)a.x + (size_t)m0 * k;
+        hi.y = (float*)a.y + (size_t)m0 * a.ldy;
         int rc = cn_gemv_launch(lo, stream, who);
         return rc ? rc : cn_gemv_launch(hi, stream, who);
     }
@@ -579,8 +403,7 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     p.combos = a.combos, p.side_w0 = (const uint8_t*)a.side_w0, p.side_w1 = (const uint8_t*)a.side_w1, p.side_gs = a.side_gs, p.side_y = a.side_y;
     p.side_rows = a.side_rows;
     const int gy = routed ? a.combos + a.side_tokens : 1;
-    if (a.dtype == CN_BF16) return mode == 1 ? launch_m<1, 1>(p, mp, rt, grid, gy, smem, stream) : launch_m<1, 0>(p, mp, rt, grid, gy, smem, stream);
-    return mode == 1 ? launch_m<0, 1>(p, mp, rt, grid, gy, smem, stream) : launch_m<0, 0>(p, mp, rt, grid, gy, smem, stream);
+    return launch_m(p, mp, rt, grid, gy, smem, stream);
 }
 
 extern "C" int cn_nvfp4_gemv(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype,

@@ -14,7 +14,6 @@ struct GemvCall {
     float limit;   // > 0: clamped SwiGLU in the gate/up form
     int dtype;     // CN_F32 or CN_BF16 activations
     int out_f32;   // store f32 whatever the activation type
-    int x_f16_ok;  // f32 activations may be rounded to f16 (11 bits) at staging: the fast arithmetic path
     // routed-expert form: one launch over `combos` (token, rank) pairs, matrices from device pointer tables
     const int32_t* ids;
     const int32_t* order;

@@ -32,7 +32,6 @@ namespace {
 
 constexpr int CH = 256;                                       // values of k in a chunk: four MMAs
 constexpr int RAW_STAGE = 128 * 144;                          // container bytes of a chunk
-constexpr int A_CODES = 128 * 128, A_STAGE = A_CODES + 4 * 512;  // the same as operand: 128-byte swizzled rows, then the scales of the four MMAs
 constexpr int NX = 16;      // chunk factors in flight (a warp is at most a few chunks ahead of another)
 constexpr int NDONE = 4;    // barriers of finished chunks
 constexpr int MAX_RAW = 4;  // container stages
@@ -305,37 +304,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             }
             const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + (w * 32 + lane) * 9;
             uint32_t v[36];
-#pragma unroll
-            for (int j = 0; j < 9; j++) {
-                const uint4 q = src[j];
-                v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
-            }
-            uint32_t odd = 0u;
-#pragma unroll
-            for (int b = 0; b < 4; b++) odd |= v[9 * b] & ((v[9 * b] & 0x7f7f7f7fu) + 0x01010101u);
-            odd = __any_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                const uint32_t sc = v[9 * b];
-                v[9 * b] = scale_bytes_rule(sc);
-                if (odd) {  // 0xFF stands for 480, which the tensor core does not know: nothing here, and the block is multiplied out below
-                    const uint32_t ff = sc & ((sc & 0x7f7f7f7fu) + 0x01010101u) & 0x80808080u;
-                    v[9 * b] &= ~(ff - (ff >> 7));
-                }
-            }
+            const uint32_t odd = load_row(src, v);
             if (i >= NA && !mbar_wait(&done[(i - NA) % NDONE], ((i - NA) / NDONE) & 1)) {
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            uint8_t* dst = a0 + (i & 1) * A_STAGE;
-            uint8_t* line = dst + (w * 32 + lane) * 128;
-            const uint32_t sw = (uint32_t)(lane & 7);
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
-                *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
-                *(uint32_t*)(dst + A_CODES + b * 512 + lane * 16 + w * 4) = v[9 * b];
-            }
+            store_row(a0 + (i & 1) * A_STAGE, w, lane, v);
             if (lane == 0) wf[(i % NX) * 4 + w] = odd;
             fence_async();
             __syncwarp();
@@ -379,25 +353,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
                 for (int m = 0; m < G; m++) {
                     const float2 f = fs[(i % NX) * 8 + m0 + m];
-                    float s = __uint_as_float(d[LV * m]);
-                    if constexpr (F32) {
-                        // what the last two additions round off is kept; the chunks are added in 64 bits
-                        float rest = 0.0f;
-#pragma unroll
-                        for (int j = 1; j < LV - 2; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
-#pragma unroll
-                        for (int j = LV - 2; j < LV; j++) {
-                            const float a = s * 0.125f, b = __uint_as_float(d[LV * m + j]);
-                            s = a + b;
-                            const float bb = s - a;
-                            rest = rest * 0.125f + ((a - (s - bb)) + (b - bb));
-                        }
-                        acc[m0 + m] += ((double)s + (double)rest) * power_of_two(f.x);
-                    } else {
-#pragma unroll
-                        for (int j = 1; j < LV; j++) s = fmaf(s, 0.125f, __uint_as_float(d[LV * m + j]));
+                    float rest;
+                    const float s = sum_digits<F32>(d + LV * m, rest);
+                    if constexpr (F32)
+                        acc[m0 + m] += ((double)s + (double)rest) * power_of_two(f.x);  // the chunks are added in 64 bits
+                    else
                         acc[m0 + m] = fmaf(s * gs, f.x, acc[m0 + m]);
-                    }
                     slow |= __float_as_uint(f.y);
                 }
             }
