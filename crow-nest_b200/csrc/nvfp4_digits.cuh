@@ -5,7 +5,7 @@
 
 #include <type_traits>
 
-__host__ __device__ constexpr int digits_of(bool f32) { return f32 ? 12 : 8; }
+__host__ __device__ constexpr int digits_of(bool f32) { return f32 ? 11 : 8; }
 
 // ---------------------------------------------------------------- tcgen05
 __device__ __forceinline__ uint64_t desc_sf(uint32_t smem_addr) {  // a scale chunk: 32 rows of 16 bytes, no swizzle, 8-row groups 128 B apart
@@ -29,27 +29,28 @@ __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* v) {
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
+__device__ __forceinline__ void tc_ld2(uint32_t taddr, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tc_ld1(uint32_t taddr, uint32_t* v) { asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v[0]) : "r"(taddr) : "memory"); }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // a row's digits of one chunk
 template <bool F32>
 __device__ __forceinline__ void tc_ld_digits(uint32_t taddr, uint32_t* v) {
     tc_ld8(taddr, v);
-    if (F32) tc_ld4(taddr + 8, v + 8);
+    if (F32) tc_ld2(taddr + 8, v + 8), tc_ld1(taddr + 10, v + 10);
 }
 
 // ---------------------------------------------------------------- 256 values of an activation row as digits (a warp; a lane holds eight values)
 // bs: the B tile; the row's lines are `row` x the digits of a value + j for digit j. With E the exponent of a block's largest value, a value is q x 2^(E - 21), |q| <= 2^22
-// (f32: q x 2^(E - 33), |q| <= 2^34): its digits are the octal digits of q + 44444444 (octal; f32: twelve fours), less four each. The scale byte is 2^(8 - (Emax - E)), Emax
+// (f32: q x 2^(E - 30), |q| <= 2^31): its digits are the octal digits of q + 44444444 (octal; f32: eleven fours), less four each. The scale byte is 2^(8 - (Emax - E)), Emax
 // that of the chunk.
 //
-// A bf16 value is whole in its digits from 2^-14 of 2^E on, an f32 value from 2^-10 on; smaller ones are off by 2^-22 (f32: 2^-34) of 2^E at most. That is nothing beside the
+// A bf16 value is whole in its digits from 2^-14 of 2^E on, an f32 value from 2^-7 on; smaller ones are off by 2^-22 (f32: 2^-31) of 2^E at most. That is nothing beside the
 // large values of a block, but much where one or two stand alone and meet small weights. So a block of which one half (eight values) has none that reaches 2^-8 of the
-// largest and the other fewer than three has no digits: the threads that add the chunk multiply it out (`whole_blocks`). Rows of 1e4 beside values of size 1, one to a block, weights zero there: f32 2.6e-8 off, with ten digits and
-// no such rule 1.6e-5; such a block is less than one in 1e5 of an FFN's hidden rows (SiLU of deviation 7 times its like; the look at its values one in 300), none of normally distributed ones. The same goes for blocks below
+// largest and the other fewer than three has no digits: the threads that add the chunk multiply it out (`whole_blocks`). So f32 values are off by 2^-24 of the third largest (or of the largest of a half) at most, bf16 ones by 2^-15.
+// Rows of 1e4 beside values of size 1, one to a block, weights zero there: f32 3.4e-8 off, with ten digits and no such rule 1.6e-5; such a block is less than one in 1e5 of an FFN's hidden rows (SiLU of deviation 7 times its like; the look at its values one in 300), none of normally distributed ones. The same goes for blocks below
 // 2^-17 of their chunk's largest value or below 2^-99, and for those with an infinity or NaN.
 // fs[row]: 2^(Emax - 8) and the blocks without digits (block b: bit 2 b).
 constexpr float TO_INT = 12582912.0f;  // 3 x 2^22: a sum with it has the nearest whole number in its mantissa (ties to even)
@@ -87,7 +88,7 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
         for (int i = 0; i < (F32 ? 8 : 4); i++) u[i] = none ? 0u : u[i];
     }
     if (none || top == 0u) e = emax;
-    const float scale = __uint_as_float(((F32 ? 269u : 275u) - e) << 23);  // 2^(21 - (e - 127)), f32: 15
+    const float scale = __uint_as_float(((F32 ? 266u : 275u) - e) << 23);  // 2^(21 - (e - 127)), f32: 12
     uint32_t lo[4], hi[4], over[4];  // value pair p: byte j = digits j (hi: 4 + j; over: 8 + j) of both
 #pragma unroll
     for (int p = 0; p < 4; p++) {
@@ -97,9 +98,9 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
             const float v = __uint_as_float(F32 ? u[F32 ? 2 * p + h : p] : h ? u[p] & 0xffff0000u : u[p] << 16);
             uint32_t q;
             if constexpr (F32) {
-                // six digits of the value in units of 2^(E - 15), six of what is left, which may reach beyond them by one
+                // five digits of the value in units of 2^(E - 12), six of what is left, which may reach beyond them by one
                 const float t = fmaf(v, scale, TO_INT), w = fmaf(fmaf(v, scale, TO_INT - t), 262144.0f, TO_INT);
-                const uint32_t lq = __float_as_uint(w) + (0444444u - 0x4b400000u), hq = __float_as_uint(t) + (0444444u - 0x4b400000u) + (lq >> 18);
+                const uint32_t lq = __float_as_uint(w) + (0444444u - 0x4b400000u), hq = __float_as_uint(t) + (044444u - 0x4b400000u) + (lq >> 18);
                 q = (lq & 0x3ffffu) | ((hq & 0x3fu) << 18);
                 uint32_t x = hq >> 6;
                 x += (x & 0xfc0u) * 3u;
@@ -123,14 +124,14 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
         *(uint32_t*)(bs + n * 128u + ((at ^ (F32 ? n & 7u : (uint32_t)j)) << 4) + in) = w;
     };
 #pragma unroll
-    for (int h = 0; h < LV / 4; h++) {
+    for (int h = 0; h < (F32 ? 3 : 2); h++) {
         const uint32_t* s = h == 0 ? lo : h == 1 ? hi : over;
         const uint32_t a = __byte_perm(s[0], s[1], 0x5140), b = __byte_perm(s[2], s[3], 0x5140);
         const uint32_t c = __byte_perm(s[0], s[1], 0x7362), d = __byte_perm(s[2], s[3], 0x7362);
         put(4 * h, __byte_perm(a, b, 0x5410));
         put(4 * h + 1, __byte_perm(a, b, 0x7632));
         put(4 * h + 2, __byte_perm(c, d, 0x5410));
-        put(4 * h + 3, __byte_perm(c, d, 0x7632));
+        if (4 * h + 3 < LV) put(4 * h + 3, __byte_perm(c, d, 0x7632));
     }
     const uint32_t under = emax - e;  // 0..17: 2^8 .. 2^-9, the last three subnormal
     uint32_t sw = (under <= 14u ? (15u - under) << 3 : 32u >> (under - 12u)) << (8 * ((lane >> 1) & 3));

@@ -2,7 +2,7 @@
 // the tensor-parallel line output (bf16). Supersedes gemv_nvfp4_w / _gu / _wm / _gum (engine/src/kernels_p2.rs:355-530).
 //
 // The weights are the A operand as they are: E2M1 codes with one UE4M3 scale per 16 values is what this MMA multiplies, so nothing is decoded. A bf16
-// row is the B operand as eight columns of signed octal digits, an f32 row as twelve: per 16 values a power of two and a number of 23 (35) bits, digit j of a value being one
+// row is the B operand as eight columns of signed octal digits, an f32 row as eleven: per 16 values a power of two and a number of 23 (32) bits, digit j of a value being one
 // of -4..3, all of them E2M1 values (what they hold of a value: nvfp4_digits.cuh).
 // Products, scales and digits are exact; a column's sum over 256 values is the tensor core's, which is the f32 nearest to it or the one beside (k = 256:
 // 2.5e-8 of a row against 64 bits, as much as the last rounding alone). The columns are added from the smallest up and the chunks of 256 in order; bf16 rows in f32
