@@ -387,8 +387,8 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     const bool short_rows = p->hidden <= MAX_ROW && p->inter <= MAX_ROW;
     // From 48 combos on the combos are sorted by expert and cut into groups of up to eight rows that share one pass over the expert's weights (nvfp4_rows_tc.cu).
     // us per step (64 tokens, 512 experts of 2048 x 512, top 10, unless said otherwise) now / with mma.sync kernels that decoded the weights to f16 for eight bf16
-    // or two f32 rows: 199 / 213, 128 tokens 292 / 322, 16 tokens 95 / 110, f32 rows 207 / 232; 64 experts of 1024 x 1280, top 8, 108 tokens 156 / 190; 128 experts, f32,
-    // 100 tokens 218 / 291; 288 experts of 4096 x 2048, top 8, 10 tokens 198 / 239. With 40 combos nothing was gained (48 / 48 us): the grouping is a launch of its own.
+    // or two f32 rows: 192 / 213, 128 tokens 293 / 323, 16 tokens 86 / 109, f32 rows 208 / 234; 64 experts of 1024 x 1280, top 8, 108 tokens 178 / 198; 128 experts, f32,
+    // 100 tokens 216 / 291; 288 experts of 4096 x 2048, top 8, 10 tokens 198 / 239. With 40 combos nothing was gained (48 / 48 us): the grouping is a launch of its own.
     if (combos >= GROUP_COMBOS && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
         int* ga = p->groups;
         int* gb = ga + combos;

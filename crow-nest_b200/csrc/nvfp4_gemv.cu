@@ -347,9 +347,9 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (a.dtype == CN_BF16) return cn_gemv_m1_launch(a, stream, who);
     if (a.line_bases) CN_FAIL(CN_ERR_SHAPE, "%s: line output takes bf16 activations", who);
     // f32 activations on the fifth-generation tensor cores where a row is long or a matrix large. us a call in a stream of dependent ones, there / here for one
-    // and eight rows: 16384 x 512 3.2 / 3.7 and 5.5 / 13, 20000 x 1536 6.1 / 11.1 and 13.2 / 49, 8192 x 512 3.5 / 3.3 and 5.8 / 6.5, 2048 x 1024 3.3 / 2.3 and 5.1 / 6.8. At
-    // k = 2048 the mma.sync kernel with three f16 planes that was there before took 3.2 and 8.1 for 2048 rows (3.5 and 5.4 now), at 17408 x 5120, gate / up, 26.6 and 84.6
-    // (19.4 and 45.6). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
+    // and eight rows: 16384 x 512 3.2 / 3.7 and 5.9 / 13, 20000 x 1536 6.8 / 11.1 and 13.2 / 49, 8192 x 512 2.9 / 3.2 and 5.5 / 6.4, 2048 x 1024 3.5 / 2.2 and 5.3 / 6.8. At
+    // k = 2048 the mma.sync kernel with three f16 planes that was there before took 3.3 and 8.1 for 2048 rows (3.8 and 5.7 now), at 17408 x 5120, gate / up, 26.7 and 84.8
+    // (19.6 and 52). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
     // A rule of the matrix alone: a row's result does not depend on how many rows the call has.
     if (!routed && (k >= 2048 || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
         if (k > 108544) CN_FAIL(CN_ERR_LIMIT,  // (the library's limit for f32 rows, as it was; this kernel has none)

@@ -787,14 +787,14 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     Split one = {1, 0};
     if (!routed) one = one_row_split(ntiles, bpr, tx);
     // Larger matrices go to the fifth-generation tensor cores, whatever the number of rows (a rule of the matrix alone: a row's bits are those of a one-row
-    // call). us a call in a stream of dependent ones, there / here, for one and four rows: gate / up of 17408 x 5120 18.7 / 20.7 and 23.4 / 30.1, 5120 x 17408 12.4 /
-    // 15.4 and 15.0 / 21.1, 4096 x 4096 4.4 / 4.6 and 5.6 / 5.5, 2048 x 4096 3.5 / 4.1 and 3.9 / 4.6; below eight million weights its longer way
-    // from the activations to the first product shows: 2048 x 2048 3.2 / 2.9 and 3.4 / 3.6, 512 x 2048 2.9 / 2.1 and 3.1 / 2.9. So it does with shorter rows than 4096
-    // values, where the kernel here has parts of K to share only late, until there are rows for all SMs: 3328 x 3584 4.4 / 3.5 and 5.4 / 5.0, 5632 x 1536 4.5 / 3.9 and
-    // 4.7 / 4.8, 8192 x 3072 5.9 / 5.3 and 7.6 / 7.1, gate / up of 3584 x 3328 6.7 / 5.7 and 8.6 / 7.7; but 10000 x 1536 4.5 / 4.9 and 5.2 / 6.4, 12288 x 2560 6.1 / 6.6 and 7.4 /
-    // 8.5, 25949 x 1024 5.1 / 6.6 and 5.9 / 9.5, gate / up of 6144 x 2560 6.2 / 6.5 and 7.4 / 9.3. (One row of a few gate / up matrices of 4096 to 4608 values is slower there: 3072 x 4352
-    // 6.4 / 5.9, four 7.5 / 8.6.) Few long rows stay too: its clusters end at
-    // eight CTAs a tile of 128 rows (640 x 17408 6.3 / 5.8, 512 x 16384 5.9 / 4.9, 2048 x 16384 7.7 / 8.1). A row that does not fit here is refused as it was, and so are lines
+    // call). us a call in a stream of dependent ones, there / here, for one and four rows: gate / up of 17408 x 5120 18.8 / 20.7 and 23.8 / 30.1, 5120 x 17408 12.4 /
+    // 15.5 and 15.3 / 21.1, 4096 x 4096 4.5 / 4.6 and 5.7 / 5.5, 2048 x 4096 3.6 / 4.3 and 3.9 / 4.6; below eight million weights its longer way
+    // from the activations to the first product shows: 2048 x 2048 3.4 / 2.9 and 3.5 / 3.4, 512 x 2048 3.0 / 2.1 and 3.1 / 2.9. So it does with shorter rows than 4096
+    // values, where the kernel here has parts of K to share only late, until there are rows for all SMs: 3328 x 3584 4.5 / 3.5 and 5.2 / 5.0, 5632 x 1536 4.5 / 3.9 and
+    // 4.7 / 4.9, 8192 x 3072 5.8 / 5.4 and 7.7 / 7.0, gate / up of 3584 x 3328 6.1 / 5.5 and 7.2 / 7.6; but 10000 x 1536 4.4 / 4.9 and 5.3 / 6.4, 12288 x 2560 6.0 / 6.5 and 7.6 /
+    // 8.5, 25949 x 1024 5.0 / 6.5 and 5.9 / 9.5, gate / up of 6144 x 2560 6.2 / 6.5 and 7.5 / 9.2. (One row of a few matrices of 4096 to 4608 values is slower there: gate / up of 3072 x 4352
+    // 6.3 / 5.8, four 7.5 / 8.5; 3328 x 4608 4.6 / 4.3, 5.3 / 6.0.) Few long rows stay too: its clusters end at
+    // eight CTAs a tile of 128 rows (640 x 17408 6.4 / 5.9, 512 x 16384 6.0 / 5.0, 2048 x 16384 7.3 / 8.1). A row that does not fit here is refused as it was, and so are lines
     // of rows shorter than 2048 values, below.
     const long long all_rows = (long long)rows * (gu ? 2 : 1);
     if (!routed && all_rows * k >= 8000000 && (k >= 4096 || all_rows >= 10000) && !(all_rows <= 1280 && k > 14336) && !(a.line_bases && tx != 32)) {

@@ -3,7 +3,7 @@
 //
 // The weights are the A operand as they are: E2M1 codes with one UE4M3 scale per 16 values is what this MMA multiplies, so nothing is decoded. A bf16
 // row is the B operand as eight columns of signed octal digits, an f32 row as eleven: per 16 values a power of two and a number of 23 (32) bits, digit j of a value being one
-// of -4..3, all of them E2M1 values (what they hold of a value: nvfp4_digits.cuh).
+// of -4..3, all of them E2M1 values (what they hold of a value, and the blocks that are multiplied out instead: nvfp4_digits.cuh).
 // Products, scales and digits are exact; a column's sum over 256 values is the tensor core's, which is the f32 nearest to it or the one beside (k = 256:
 // 2.5e-8 of a row against 64 bits, as much as the last rounding alone). The columns are added from the smallest up and the chunks of 256 in order; bf16 rows in f32
 // (k = 4096: 6.2e-8, 17408: 8.6e-8), f32 rows with what the last two additions round off kept, chunks in 64 bits (2.5e-8: the result's own rounding). The columns of one row do not
@@ -15,11 +15,13 @@
 // layout, 8-11 turn activations into digits, 12 loads (TMA, boxes of 128 rows x 144 bytes of container), 13 issues the MMAs. Loads and the move do
 // not wait for the kernel in front: when the activations come, five chunks of weights a CTA lie ready or nearly so.
 //
-// What bounds it, one row: HBM for large matrices (gate / up of 17408 x 5120: 100 MB in 18.6 us, of which 2.6 until the first product; the CTAs then take 6.1 TB/s);
+// What bounds it, one row: HBM for large matrices (gate / up of 17408 x 5120: 100 MB in 18.8 us, of which 2.6 until the first product; the CTAs then take 6.1 TB/s);
 // for small ones the chain from one call to the next, some 3 us: end of the grid in front 0.8, activations 0.4, digits 0.35, first sum 0.4, adding up in
 // the cluster 0.4, output and end of the grid 0.6. From four rows on also the digits (one warp and row: 0.35 us a chunk). In a stream of dependent calls, us
-// here / mma.sync kernel (nvfp4_gemv_m1.cu): gate / up of 17408 x 5120 18.6 / 20.7, two rows 19.4 / 27.2, four 23.4 / 30.1, eight 31.4 / 46.6; 5120 x 17408
-// 12.4 / 15.4, 13.0 / 18.4, 15.1 / 21.1, 19.7 / 34.7; 25000 x 8192 21.8 / 28.1, four rows 27.5 / 32.1.
+// here / mma.sync kernel (nvfp4_gemv_m1.cu): gate / up of 17408 x 5120 18.8 / 20.7, two rows 19.4 / 27.3, four 23.8 / 30.1, eight 33.1 / 46.5; 5120 x 17408
+// 12.4 / 15.5, 12.8 / 18.5, 15.3 / 21.1, 20.7 / 34.7; 25000 x 8192 22.0 / 28.2, four rows 28.0 / 32.0. f32 rows, here / mma.sync with three f16 planes a row: gate / up of
+// 17408 x 5120 19.6 / 26.7, 22.7 / 39.8, 29.3 / 41.2, 52 / 85; 5120 x 17408 12.7 / 22.1, 14.5 / 38, 18.4 / 62, 30 / 122.
+// The loads and stores of a container row stand in functions that nvfp4_rows_tc.cu shares; written out here they take four bf16 rows of that gate / up 1 us less, one and eight 0.4 and 0.8 more.
 // Measured and not kept: tiles of fewer rows so that every SM has the same bytes (the CTAs more hold up the next kernel: 5120 x 5120 5.9 -> 6.9); two teams of
 // warps for the move (18.6 -> 20.0, gate / up); L2 prefetches beyond the stages (18.6 -> 19.3 and more); a third operand stage in a container stage's place (20.6).
 #include "nvfp4_digits.cuh"
@@ -40,7 +42,7 @@ constexpr int NSLOT = 3;    // tiles whose sums are on their way in a cluster
 constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 2 + NSLOT + 2;
 constexpr int EPI_WARPS = 4, LOADER = 12, ISSUER = 13;  // warps 0-3 sums and output, 4-7 weights, 8-11 activations
 constexpr int THREADS = 448;
-constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, slow blocks}; [NX][4] scale bytes of 0xFF seen
+constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, blocks without digits}; [NX][4] scale bytes of 0xFF seen
 __host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_of(f32) + 15) / 16 * 16; }  // columns of the MMA
 __host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
 __host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
@@ -596,7 +598,8 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         map1 = map0;
     else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
         return rc;
-    // a CTA asks for no smaller a share of shared memory than of tensor memory: whatever fits an SM beside it finds tensor memory too
+    // A CTA asks for no smaller a share of shared memory than of tensor memory: as many of these kernels (or of nvfp4_rows_tc.cu's) as fit an SM find tensor memory there. The pair
+    // GEMM, which takes all of it, stands apart by its registers: 640 threads of 72 leave no room for 448 of 72.
     int smem = front + p.raw * RAW_STAGE;
     const int floor_bytes = tmem_cols(mt, f32) == 256 ? SM_SHARE : (227 * 1024) / 4;
     if (smem < floor_bytes) smem = floor_bytes;

@@ -1,7 +1,7 @@
 // NVFP4 matrices times groups of up to eight activation rows on tcgen05.mma kind::mxf4nvf4: the routed experts of a step (groups of rows of one expert) and the
 // shared expert of more rows than a GEMV takes. Supersedes gemv_fp4_ptrb over the pointer tables (engine/src/kernels.rs:195-233) together with the grouping
 // of the reference's prefill path (moe_count / moe_plan / moe_scatter, engine/src/kernels.rs:3334-3420). Arithmetic as in nvfp4_gemv_tc.cu: weights as they
-// are, rows as octal digits, chunks of 256 values of k added in order (f32, for f32 rows f64).
+// are, rows as octal digits (blocks that these do not hold well multiplied out), chunks of 256 values of k added in order (f32, for f32 rows 64 bits).
 //
 // Persistent CTAs, two per SM, walk units of (group, 128-row tile; 64 gate and 64 up rows). The matrices come from device tables, so there is no tensor map:
 // a scout warp looks up 32 units at a time (positions, combos, expert, addresses) and hands them to the other warps through a ring, and the warps that lay
@@ -10,7 +10,7 @@
 //
 // What bounds it: the way of the weights through a warp (gate / up of 64 tokens, 512 experts of 2048 x 512, top 10: 2150 cycles a chunk of 18 KB and CTA, 470 of
 // them loads, 500 stores and their fence, 580 the copies of a later chunk), 4.1 TB/s; us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16
-// or two f32 rows: gate / up 105 / 114, down 70 / 77. Tried: the same with a bulk copy for each row piece of 144 bytes 166 and 93; copies asked for
+// or two f32 rows: gate / up 103 / 114, down 72 / 77. Tried: the same with a bulk copy for each row piece of 144 bytes 166 and 93; copies asked for
 // before the stores of the chunk in hand, one chunk less ahead, 109 and 79.
 #include "nvfp4_digits.cuh"
 #include "nvfp4_gemv.cuh"
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     uint64_t* unit_full = d_empty + 2;        // [NU]
     uint64_t* unit_empty = unit_full + NU;    // [NU]
     uint32_t* tmem_slot = (uint32_t*)(unit_empty + NU);
-    float2* fs = (float2*)(head + FS_OFF);      // [NX][8] {factor, slow blocks}
+    float2* fs = (float2*)(head + FS_OFF);      // [NX][8] {factor, blocks without digits}
     uint32_t* wf = (uint32_t*)(head + WF_OFF);  // [NX][4] scale bytes of 0xFF seen
     Unit* units = (Unit*)(head + UNIT_OFF);     // [NU]
     const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
