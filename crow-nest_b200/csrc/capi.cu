@@ -42,8 +42,8 @@ cudaError_t cn_allow_smem(const void* kernel, int bytes) {
     return e;
 }
 
-int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
-               unsigned box_cols, unsigned box_rows) {
+static int encode_map(CUtensorMap* map, CUtensorMapDataType type, unsigned rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                      CUtensorMapSwizzle swizzle) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static Encode encode = nullptr;
@@ -54,14 +54,26 @@ int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long 
         if (!fn) CN_FAIL(CN_ERR_CUDA, "cuTensorMapEncodeTiled is not in this driver");
         encode = (Encode)fn;
     }
+    const cuuint32_t es[3] = {1, 1, 1};
+    const CUresult r = encode(map, type, rank, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) CN_FAIL(CN_ERR_CUDA, "tensor map of [%llu x %llu]: driver error %d", (unsigned long long)dims[1], (unsigned long long)dims[0], (int)r);
+    return CN_OK;
+}
+
+int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
+               unsigned box_cols, unsigned box_rows) {
     const CUtensorMapDataType type = elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : elem == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const cuuint64_t dims[2] = {cols, rows}, strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_cols, box_rows}, es[2] = {1, 1};
-    const CUresult r = encode(map, type, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              elem == 4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) CN_FAIL(CN_ERR_CUDA, "tensor map of [%llu x %llu]: driver error %d", rows, cols, (int)r);
-    return CN_OK;
+    const cuuint32_t box[2] = {box_cols, box_rows};
+    return encode_map(map, type, 2, base, dims, strides, box, elem == 4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int cn_tmap_blocks(CUtensorMap* map, const void* base, int elem, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
+                   unsigned box_blocks) {
+    const cuuint64_t dims[3] = {64, rows, blocks}, strides[2] = {row_bytes, 128};
+    const cuuint32_t box[3] = {64, box_rows, box_blocks};
+    return encode_map(map, elem == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 extern "C" const char* cn_last_error_string(void) { return t_err; }

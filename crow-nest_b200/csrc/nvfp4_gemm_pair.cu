@@ -18,12 +18,14 @@
 // tile's rows), warp 1 of the even CTA issues the MMAs of the pair, two sets of four warps (4-11) decode alternate 64-value blocks,
 // warps 12-19 write results. Tiles are walked persistently, one pair per two SMs; with up to 192 tokens per tile there
 // are two accumulators and the epilogue of a tile runs under the MMAs of the next.
-// Rings: weights 3 to 6 x 18 KB (256 values of K each), activations up to 8 x 16 KB and A slots 4..8 x 32 columns (64 values).
+// Rings: weights 3 to 6 x 18 KB (256 values of K each); beyond 128 rows activations in slots of 128 values (up to 8) and A slots of 64 (4 to 8, 32 columns each), up to 128 rows both in slots
+// of 256 (four and three): every slot costs the thread that asks for it some 300 cycles and the one that issues its MMAs 100, whatever it holds.
 //
-// Up to 128 rows the decode bounds it, not the MMAs: the way of a block through a warp (172 warp instructions per scheduler and 64-value block in all, no
-// unit near its rate) and the start and end of a launch; hence f16 (half the instructions of the decode to bf16), with the rows brought into f16 by a
-// kernel before this one that runs under this one's prologue, all sixteen warps decoding, and K split where row tiles do not fill the pairs. 17408 x 5120 at 64 rows:
-// 80 us (one CTA per tile, widened weights through shared memory) -> 21; 5120 x 17408: 109 -> 27.
+// Up to 128 rows the way of a block through a decode warp bounds it (650 cycles of 1000 a stage), up to some 90 rows, then the MMAs, and the start and end of a launch (8 us of a call: the
+// kernel that prepares the rows, this one, and the one that adds the parts wait for one another); hence f16 (half the instructions of the decode to bf16), with the rows brought into f16 by a
+// kernel before this one that runs under this one's prologue, all sixteen warps decoding, and K split where row tiles do not fill the pairs. 17408 x 5120 at 64 rows, us in a graph of
+// calls: 80 (one CTA per tile, widened weights through shared memory), 20.6 (rings of 64 and 128 values, two boxes for each activation slot: 303 cycles a block, the rate
+// of the thread that asked for the boxes, at 16 rows as at 64), 17.1; container bytes 20.9 -> 18.2; 5120 x 17408 26.1 -> 21.5, 8192 x 5120 at 128 rows 20.2 -> 16.7.
 // Every wait is bounded. The weights are read with L2's ordinary policy: kept as evict-last, for the token tiles that read them again, they
 // gained nothing (512 rows 76.6 and 76.9 us) and stayed behind: a 50 MB matrix read twice after the call took 83 us the second time, 75 now.
 // Measured over the public call with inputs that change from pass to pass: 17408 x 5120 at 512 rows 155 -> 76 us (1.2 PFLOP/s; one CTA
@@ -36,6 +38,8 @@ namespace {
 
 constexpr int W_STAGE = 128 * 144;  // 256 values of K of 128 rows: container bytes, or the stage image of the re-laid weights
 constexpr int MAX_W_STAGES = 6;
+__host__ __device__ constexpr int slot_blocks(int sets) { return sets == 4 ? 4 : 1; }  // 64-value blocks of an A slot
+__host__ __device__ constexpr int box_blocks(int sets) { return sets == 4 ? 4 : 2; }   // and of an activation slot
 constexpr int PAIR_THREADS = 640;
 constexpr int HDR = 1024;
 constexpr int SMEM_MAX = 227 * 1024;
@@ -47,7 +51,7 @@ struct PairParams {
     void* y;
     int rows, m, ldy, out_bf16, pair_store;  // pair_store: bf16 results two rows at a time
     int nk;                      // 64-value blocks of K
-    int tn, acc_stride, nacc, na, nb, nws;  // tokens per tile; accumulator columns and count; A, activation and weight ring depths
+    int tn, acc_stride, nacc, na, nb, nws;  // tokens per tile; accumulator columns and count; A, activation and weight ring depths (slots)
     int row_tiles, tiles, ksplits;
     int split_stages, split_more;  // weight stages of a part of K; the first split_more parts have one more
     const uint8_t* packed;  // re-laid weights (cn_nvfp4_bs_repack), or null: container bytes through wmap
@@ -75,36 +79,61 @@ struct DecodeAt {
     int ws, as;
     uint32_t wp, ap;
 };
-// Every SETS-th block of `stages` weight stages from block SET on, one row per thread. Container: block b is nine words from word 9 b of the
-// row's 144 bytes, inside three 16-byte chunks. Re-laid: codes are chunks 2 b and 2 b + 1 of the row's 128 swizzled bytes, the scale word lies
-// in the image's scale part. Two sets of warps where the MMAs or the ALUs bound the loop (four of one block each measured 5 % slower at
-// 200 - 1000 rows of bf16), four where it is the way of a block - load, decode, store to tensor memory, arrival - that does.
-template <bool BF16, bool PACKED, int SET, int SETS>
+// Block b of the stage's row at `at` (its scale word at `scale` where the weights are re-laid): scale word and eight code words. Container: nine words from word 9 b of the row's 144 bytes,
+// inside three 16-byte chunks. Re-laid: codes are chunks 2 b and 2 b + 1 of the row's 128 swizzled bytes, the scale word lies in the image's scale part.
+__device__ __forceinline__ void lds128(uint32_t* v, uint32_t at) {
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at));
+}
+template <int B>
+__device__ __forceinline__ void load_container(uint32_t (&c)[9], uint32_t at) {
+    uint32_t t[12];
+#pragma unroll
+    for (int i = 0; i < 3; i++) lds128(t + 4 * i, at + (uint32_t)(((9 * B) >> 2) + i) * 16u);
+#pragma unroll
+    for (int i = 0; i < 9; i++) c[i] = t[B + i];
+}
+template <bool PACKED>
+__device__ __forceinline__ void load_block(uint32_t (&c)[9], uint32_t at, uint32_t scale, int b, int lane) {
+    if (PACKED) {
+        lds128(c + 1, at + (uint32_t)(((2 * b) ^ (lane & 7)) << 4));
+        lds128(c + 5, at + (uint32_t)(((2 * b + 1) ^ (lane & 7)) << 4));
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(c[0]) : "r"(scale + 512u * b));
+    } else if (b == 0) {
+        load_container<0>(c, at);
+    } else if (b == 1) {
+        load_container<1>(c, at);
+    } else if (b == 2) {
+        load_container<2>(c, at);
+    } else {
+        load_container<3>(c, at);
+    }
+}
+// Every SETS-th block of `stages` weight stages from block `set` on, one row per thread. Two sets of warps where the MMAs or the ALUs bound the loop (four of one block each measured 5 %
+// slower at 200 - 1000 rows of bf16), four where it is the way of a block - load, decode, store to tensor memory, arrival - that does. Four sets run one copy of the code (SET = -1): with
+// one for each, instructions come late (17408 x 5120, 64 rows: 18.0 us a call on re-laid weights, 17.1 so). Two have one each, SET = 0 and 1, whose blocks the compiler knows
+// (5120 x 17408 at 512 rows: 72 us, 77 with one copy).
+template <bool BF16, bool PACKED, int SETS, int SET>
 __device__ __forceinline__ void decode_set(uint32_t src, uint32_t scales, uint32_t dst, uint64_t* wfull, uint64_t* wempty, uint64_t* aempty, uint32_t afull_base,
-                                           int stages, int nws, int na, int lane, DecodeAt& at_) {
+                                           int stages, int nws, int na, int lane, int which, DecodeAt& at_) {
+    constexpr int G = slot_blocks(SETS);
+    const int set = SET < 0 ? which : SET;
     int ws = at_.ws, as = at_.as;
     uint32_t wp = at_.wp, ap = at_.ap;
+    const uint32_t col = dst + 32u * (uint32_t)(set % G);
     for (int w = 0; w < stages; w++) {
         if (!mbar_wait(&wfull[ws], wp)) {
             cn_dev_fail(CN_DEV_WAIT_FULL);
             return;
         }
 #pragma unroll
-        for (int b = SET; b < 4; b += SETS) {
-            uint32_t c[12], v[32];
-            const uint32_t at = src + (uint32_t)ws * W_STAGE + (PACKED ? 0u : (uint32_t)((9 * b) >> 2) * 16u);
-            constexpr int C0 = PACKED ? 1 : 0;  // word 0 of a re-laid block is its scale word, from elsewhere
-#pragma unroll
-            for (int i = 0; i < (PACKED ? 2 : 3); i++)
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(c[4 * i + C0]), "=r"(c[4 * i + C0 + 1]), "=r"(c[4 * i + C0 + 2]), "=r"(c[4 * i + C0 + 3])
-                             : "r"(PACKED ? at + (uint32_t)(((2 * b + i) ^ (lane & 7)) << 4) : at + 16u * i));
-            if (PACKED) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(c[0]) : "r"(scales + (uint32_t)ws * W_STAGE + 512u * b));
+        for (int j = 0; j < 4 / SETS; j++) {
+            uint32_t c[9], v[32];
+            load_block<PACKED>(c, src + (uint32_t)ws * W_STAGE, scales + (uint32_t)ws * W_STAGE, set + SETS * j, lane);
             if (BF16)
-                decode64_bf16(c + (PACKED ? 0 : b), v);
+                decode64_bf16(c, v);
             else
-                decode64_f16(c + (PACKED ? 0 : b), v);
-            if (b + SETS >= 4) {  // the stage has been read
+                decode64_f16(c, v);
+            if (j == 4 / SETS - 1) {  // the stage has been read
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&wempty[ws]);
             }
@@ -113,12 +142,12 @@ __device__ __forceinline__ void decode_set(uint32_t src, uint32_t scales, uint32
                 return;
             }
             tc_after();
-            tc_st32(dst + (uint32_t)as * 32u, v);
+            tc_st32(col + (uint32_t)as * (32u * G), v);
             tc_wait_st();
             tc_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(afull_base + 8u * (uint32_t)as);
-            as += SETS;
+            as += SETS / G;
             if (as >= na) as -= na, ap ^= 1u;
         }
         if (++ws == nws) ws = 0, wp ^= 1u;
@@ -131,6 +160,7 @@ __device__ __forceinline__ void decode_set(uint32_t src, uint32_t scales, uint32
 template <bool BF16, bool PACKED, int SETS, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const PairParams p) {
+    constexpr int G = slot_blocks(SETS), KB = box_blocks(SETS);
     extern __shared__ uint8_t smem_raw[];
     // barriers: wfull 6, wempty 6, bfull 8, bempty 8, afull 8, aempty 8, accfull 2, accempty 2
     uint64_t* wfull = (uint64_t*)smem_raw;
@@ -143,7 +173,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     uint64_t* accempty = accfull + 2;
     uint32_t* tmem_slot = (uint32_t*)(accempty + 2);
     const uint32_t ring = (smem_u32(smem_raw) + HDR + 1023u) & ~1023u;
-    const uint32_t bbox = (uint32_t)p.tn * 64u, bslot = 2u * bbox;  // tn / 2 rows of 128 bytes, twice
+    const uint32_t bbox = (uint32_t)p.tn * 64u, bslot = KB * bbox;  // tn / 2 rows of 128 bytes, for every block of a slot
     const uint32_t wring = ring + (uint32_t)p.nb * bslot;
 
     const int tid = threadIdx.x, warp = (int)warp_uniform((uint32_t)tid >> 5), lane = tid & 31;
@@ -153,7 +183,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 
     if (tid == 0) {
         for (int i = 0; i < MAX_W_STAGES; i++) mbar_init(&wfull[i], 1), mbar_init(&wempty[i], 4 * SETS);
-        for (int i = 0; i < 8; i++) mbar_init(&bfull[i], 1), mbar_init(&bempty[i], 1), mbar_init(&afull[i], 8), mbar_init(&aempty[i], 1);
+        for (int i = 0; i < 8; i++) mbar_init(&bfull[i], 1), mbar_init(&bempty[i], 1), mbar_init(&afull[i], 8 * G), mbar_init(&aempty[i], 1);
         for (int i = 0; i < 2; i++) mbar_init(&accfull[i], 1), mbar_init(&accempty[i], SETS == 4 ? 32 : 16);
         mbar_fence_init();
     }
@@ -166,17 +196,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
     const uint32_t tmem = warp_uniform(*tmem_slot);
     const uint32_t acol = tmem + (uint32_t)(p.nacc * p.acc_stride);
 
-    DecodeAt at = {0, (warp - 4) >> 2, 0u, 1u};
+    DecodeAt at = {0, ((warp - 4) >> 2) / G, 0u, 1u};
     auto decode = [&](int stages) {
         const uint32_t src = wring + (uint32_t)(32 * (warp & 3) + lane) * (PACKED ? 128u : 144u);
         const uint32_t scales = wring + 128u * 128u + (uint32_t)lane * 16u + 4u * (uint32_t)(warp & 3);
         const uint32_t dst = acol + ((uint32_t)(32 * (warp & 3)) << 16);
         const uint32_t afull_base = cluster_addr(smem_u32(afull), 0);
         const int set = (warp - 4) >> 2;
-        if (set == 0) decode_set<BF16, PACKED, 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
-        if (set == 1) decode_set<BF16, PACKED, 1, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
-        if (SETS == 4 && set == 2) decode_set<BF16, PACKED, SETS == 4 ? 2 : 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
-        if (SETS == 4 && set == 3) decode_set<BF16, PACKED, SETS == 4 ? 3 : 0, SETS>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, at);
+        if (SETS == 4) decode_set<BF16, PACKED, SETS, -1>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, set, at);
+        if (SETS == 2 && set == 0) decode_set<BF16, PACKED, SETS, 0>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, set, at);
+        if (SETS == 2 && set == 1) decode_set<BF16, PACKED, SETS, 1>(src, scales, dst, wfull, wempty, aempty, afull_base, stages, p.nws, p.na, lane, set, at);
     };
     auto load_w = [&](int ws, int rt, int w) {
         if (PACKED)  // (the upper half of the last 256-row tile may lie beyond the matrix: it reads the last one, and its results are not stored)
@@ -208,7 +237,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                     mbar_arrive(&wfull[ws]);
                     load_w(ws, rt, w);
                     if (++ws == p.nws) ws = 0, wp ^= 1u;
-                    for (int q = 0; q < 2; q++) {
+                    for (int q = 0; q < 4 / KB; q++) {
                         if (!mbar_wait(&bempty[bs], bp)) {
                             cn_dev_fail(CN_DEV_WAIT_EMPTY);
                             ok = false;
@@ -218,8 +247,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                             mbar_expect_tx(&bfull[bs], 2u * bslot);
                             mbar_arrive(&bfull[bs]);
                         }
-                        tma_load_2d_pair(ring + (uint32_t)bs * bslot, &xmap, (w * 4 + 2 * q) * 64, tok0, bfull0 + 8u * (uint32_t)bs);
-                        tma_load_2d_pair(ring + (uint32_t)bs * bslot + bbox, &xmap, (w * 4 + 2 * q + 1) * 64, tok0, bfull0 + 8u * (uint32_t)bs);
+                        tma_load_3d_pair(ring + (uint32_t)bs * bslot, &xmap, 0, tok0, w * 4 + KB * q, bfull0 + 8u * (uint32_t)bs);
                         if (++bs == p.nb) bs = 0, bp ^= 1u;
                     }
                 }
@@ -260,7 +288,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             pdl_wait();  // f16 rows come from the kernel before this one
             for (Unit<SPLIT> u(pair, p); u.live(p) && ok; u.next(npairs, p)) {
                 const int tok0 = (u.tile / p.row_tiles) * p.tn + (int)rank * (p.tn >> 1), w0 = u.first(p), w1 = w0 + u.count(p);
-                for (int q = 2 * w0; q < 2 * w1; q++) {
+                for (int q = w0 * (4 / KB); q < w1 * (4 / KB); q++) {
                     if (!mbar_wait(&bempty[bs], bp)) {
                         cn_dev_fail(CN_DEV_WAIT_EMPTY);
                         ok = false;
@@ -270,8 +298,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                         mbar_expect_tx(&bfull[bs], 2u * bslot);
                         mbar_arrive(&bfull[bs]);
                     }
-                    tma_load_2d_pair(ring + (uint32_t)bs * bslot, &xmap, q * 128, tok0, bfull0 + 8u * (uint32_t)bs);
-                    tma_load_2d_pair(ring + (uint32_t)bs * bslot + bbox, &xmap, q * 128 + 64, tok0, bfull0 + 8u * (uint32_t)bs);
+                    tma_load_3d_pair(ring + (uint32_t)bs * bslot, &xmap, 0, tok0, KB * q, bfull0 + 8u * (uint32_t)bs);
                     if (++bs == p.nb) bs = 0, bp ^= 1u;
                 }
             }
@@ -292,27 +319,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
                 tc_after();
                 const uint32_t d = tmem + (uint32_t)(ab * p.acc_stride);
                 const int nk = 4 * u.count(p);
-                for (int kb = 0; kb < nk; kb += 2) {
+                for (int kb = 0; kb < nk; kb += KB) {
                     if (!mbar_wait(&bfull[bs], bp)) {
                         cn_dev_fail(CN_DEV_WAIT_FULL);
                         ok = false;
                         break;
                     }
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (!mbar_wait(&afull[as], ap)) ok = false;
-                        tc_after();
-                        const uint32_t a = acol + (uint32_t)as * 32u;
+                    for (int h = 0; h < KB; h++) {
+                        if (h % G == 0) {
+                            if (!mbar_wait(&afull[as], ap)) ok = false;
+                            tc_after();
+                        }
+                        const uint32_t a = acol + (uint32_t)as * (32u * G) + 32u * (h % G);
                         const uint64_t b = bdesc0 + (((uint32_t)bs * bslot + (uint32_t)h * bbox) >> 4);
                         if (elect_lane()) {
 #pragma unroll
                             for (int kk = 0; kk < 4; kk++)  // 16 values: 8 columns of A, 32 bytes of B inside the swizzled row
                                 tc_mma_ts<2>(d, a + 8u * kk, b + 2u * kk, idesc, (kb > 0 || h > 0 || kk > 0) ? 1u : 0u);
-                            tc_commit<2>(&aempty[as]);
-                            if (h == 1) tc_commit<2>(&bempty[bs]);
+                            if (h % G == G - 1) tc_commit<2>(&aempty[as]);
+                            if (h == KB - 1) tc_commit<2>(&bempty[bs]);
                         }
                         __syncwarp();
-                        if (++as == p.na) as = 0, ap ^= 1u;
+                        if (h % G == G - 1 && ++as == p.na) as = 0, ap ^= 1u;
                     }
                     if (!ok) {
                         cn_dev_fail(CN_DEV_WAIT_FULL);
@@ -506,22 +535,24 @@ int cn_gemm_pair_launch(const GemmCall& c, cudaStream_t stream) {
     p.packed = (const uint8_t*)c.packed, p.packed_tiles = (c.rows + 127) / 128, p.part = c.part;
     const PairShape shape = pair_shape(c.rows, nk, c.m, PAIRS, !c.x_f16, c.part ? c.max_splits : 1);
     p.tn = shape.tn, p.ksplits = shape.ksplits, p.split_stages = nk / 4 / shape.ksplits, p.split_more = nk / 4 % shape.ksplits;
+    const bool four = c.x_f16 && p.tn <= 128;
+    const int slot = slot_blocks(four ? 4 : 2), box = box_blocks(four ? 4 : 2);
     p.acc_stride = p.tn;
-    p.nacc = p.tn <= 192 ? 2 : 1;
-    p.na = (TMEM_COLS - p.nacc * p.acc_stride) / 32;
-    p.na = p.na > 8 ? 8 : p.na & ~1;
-    p.nb = (SMEM_MAX - HDR - 1024 - 3 * W_STAGE) / (p.tn * 128);
-    if (p.nb > 8) p.nb = 8;
-    p.nws = (SMEM_MAX - HDR - 1024 - p.nb * p.tn * 128) / W_STAGE;
+    p.nacc = p.tn <= 192 && !four ? 2 : 1;  // (the warps that decode write the results too: a second accumulator would have no one to fill its A slots meanwhile)
+    p.na = (TMEM_COLS - p.nacc * p.acc_stride) / (32 * slot);
+    p.na = p.na > 8 ? 8 : four ? p.na : p.na & ~1;
+    const int bslot = p.tn * 64 * box;
+    p.nb = (SMEM_MAX - HDR - 1024 - 3 * W_STAGE) / bslot;
+    if (p.nb > 16 / box) p.nb = 16 / box;
+    p.nws = (SMEM_MAX - HDR - 1024 - p.nb * bslot) / W_STAGE;
     if (p.nws > MAX_W_STAGES) p.nws = MAX_W_STAGES;
     p.row_tiles = (c.rows + 255) / 256;
     p.tiles = p.row_tiles * ((c.m + p.tn - 1) / p.tn);
     if (!c.packed)
         if (int rc = cn_tmap_2d(&wmap, c.w, 4, (unsigned long long)nk * 9, c.rows, (unsigned long long)nk * 36, 36, 128)) return rc;
-    if (int rc = cn_tmap_2d(&xmap, c.x, c.x_f16 ? 2 : 3, c.k, c.m, (unsigned long long)c.k * 2, 64, p.tn / 2)) return rc;
-    const size_t smem = HDR + 1024 + (size_t)p.nws * W_STAGE + (size_t)p.nb * p.tn * 128;
+    if (int rc = cn_tmap_blocks(&xmap, c.x, c.x_f16 ? 2 : 3, nk, c.m, (unsigned long long)c.k * 2, p.tn / 2, box)) return rc;
+    const size_t smem = HDR + 1024 + (size_t)p.nws * W_STAGE + (size_t)p.nb * bslot;
     const int units = p.tiles * p.ksplits, grid = 2 * (units < PAIRS ? units : PAIRS);
-    const bool four = c.x_f16 && p.tn <= 128;  // (eight A slots then: every set has its own)
     int rc = CN_ERR_SHAPE;
 #define CN_PAIR_CASE(BF16V, PACKEDV, SETSV, SPLITV)                                                                                       \
     if (!c.x_f16 == BF16V && (c.packed != nullptr) == PACKEDV && four == (SETSV == 4) && (c.x_f16 || p.ksplits > 1) == SPLITV)             \

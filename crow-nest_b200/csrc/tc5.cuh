@@ -11,6 +11,10 @@
 // 4 = 32-bit, no swizzle (NVFP4 container bytes).
 int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
                unsigned box_cols, unsigned box_rows);
+// A row-major matrix of 16-bit values (elem 2 or 3) as blocks of 64 columns: coordinates (column of a block, row, block), boxes of box_rows rows and box_blocks blocks, each block
+// the operand tile that a 2-D box of it would be.
+int cn_tmap_blocks(CUtensorMap* map, const void* base, int elem, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
+                   unsigned box_blocks);
 
 // ---------------------------------------------------------------- device: TMA and clusters
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* m) { asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory"); }
@@ -19,11 +23,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* m, 
                  "r"(y), "r"(bar)
                  : "memory");
 }
-// the same from either CTA of a pair; `bar` may name the even CTA's barrier (peer bit cleared)
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) {
+// from either CTA of a pair; `bar` may name the even CTA's barrier (peer bit cleared)
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* m, int x, int y, int z, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(m), "r"(x),
-        "r"(y), "r"(bar)
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst), "l"(m), "r"(x),
+        "r"(y), "r"(z), "r"(bar)
         : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {

@@ -100,6 +100,22 @@ def test_few_rows_split_k_and_relaid_weights(rows, k, m, relaid):
     assert device_status() == 0
 
 
+@pytest.mark.parametrize("relaid", [False, True])
+@pytest.mark.parametrize("rows,k,m", [(19200, 256, 33), (300, 768, 65), (520, 1280, 97), (18950, 1024, 128), (256, 2304, 32)])
+def test_slots_of_a_whole_weight_stage(rows, k, m, relaid):
+    """Up to 128 rows a stage of 256 values of k is one slot of each ring: fewer stages than slots, one more than the A slots, every width of the token tile (32 to 128), and more
+    tiles than CTA pairs, whose second round finds the rings wherever the first one left them. Every output."""
+    rng = np.random.default_rng(rows + m)
+    fw = ops.Fp4.from_host(synth.nvfp4_matrix(rows, k, rng), rows, k, np.float32(0.37))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda().to(torch.bfloat16)
+    want = x.double() @ ops.dequant(fw, rule=True).double().view(rows, k).t()
+    y = ops.launch_gemm_fp4(ops.Fp4Packed(fw), x) if relaid else ops.launch_gemm(fw, x)
+    rms = want.pow(2).mean(dim=1, keepdim=True).sqrt()
+    # as above: one rounding of the result to bf16 beside f32 sums
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * rms).all()
+    assert device_status() == 0
+
+
 @pytest.mark.parametrize("m", [1, 60, 128])
 @pytest.mark.parametrize("form", ["container", "relaid", "f32"])
 @pytest.mark.parametrize("rows", [384, 4000])
