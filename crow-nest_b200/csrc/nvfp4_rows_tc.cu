@@ -27,7 +27,8 @@ constexpr int NA = 2, NB = 2, NX = 16, NDONE = 4, NU = 8;  // operand stages, ch
 constexpr int NBAR = NA + NX + NDONE + 2 + 2 * NU;
 constexpr int SCOUT = 12, ISSUER = 13, THREADS = 448;
 constexpr int FS_OFF = 512, WF_OFF = 1536, UNIT_OFF = 1792, HEADER = 2560;
-__host__ __device__ constexpr int ncol(bool f32) { return RG * digits_of(f32); }
+// columns of the widest MMA, whose N is a multiple of 16: the accumulators lie this far apart in tensor memory (eight f32 rows are 88 columns, and 96 are written)
+__host__ __device__ constexpr int ncol(bool f32) { return (RG * digits_of(f32) + 15) / 16 * 16; }
 __host__ __device__ constexpr int b_stage(bool f32) { return ncol(f32) * 128 + 4 * 512; }
 __host__ __device__ constexpr int smem_of(bool f32) { return NA * A_STAGE + NB * b_stage(f32) + 4 * depth_of(f32) * PIECE + HEADER; }
 constexpr int SM_SHARE = (227 * 1024) / 2 - 1024;
@@ -45,7 +46,7 @@ template <bool F32>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCall c) {
     constexpr int D = depth_of(F32), LV = digits_of(F32), ES = F32 ? 4 : 2, N = ncol(F32), B_CODES = N * 128, B_STAGE = b_stage(F32);
     constexpr uint32_t SFA_COL = 2 * N, SFB_COL = 2 * N + 32, TMEM = 256;
-    static_assert(2 * N + 64 <= (int)TMEM, "tensor memory columns");
+    static_assert(2 * N + 64 <= (int)TMEM && N % 16 == 0, "tensor memory columns");
     using Acc = typename std::conditional<F32, double, float>::type;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *a0 = smem, *b0 = a0 + NA * A_STAGE, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;

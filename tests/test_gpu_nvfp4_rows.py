@@ -53,6 +53,43 @@ def test_grouped_experts_against_64_bits(hidden, inter, experts, topk, tokens, s
     assert device_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [56, 64, 125])
+def test_full_groups_repeat_bit_for_bit(tokens, dtype):
+    """Every expert has all tokens: groups of eight rows (and of seven or five at the end), one chunk right behind the other. The accumulators of two chunks in flight lie side by side in
+    tensor memory; eight f32 rows fill theirs (the down projection's rows are f32 whatever x is). Every run has the same bits and the right ones."""
+    hidden, inter, experts = 768, 1280, 4
+    rng = np.random.default_rng(tokens)
+
+    def matrix(rows, k):
+        return torch.from_numpy(synth.nvfp4_matrix(rows, k, rng)).cuda()
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(experts)], [matrix(hidden, inter) for _ in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 0.03, 0.7, gate_up=gu, down=dn, device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, experts, tokens)
+    x = torch.from_numpy(rng.standard_normal((tokens, hidden)).astype(np.float32)).cuda().to(dtype)
+    logits = torch.from_numpy(rng.standard_normal((tokens, experts)).astype(np.float32)).cuda()
+    runs = [torch.empty_like(x) for _ in range(40)]
+    for y in runs:
+        plan.run(w, logits, x, y, router="softmax")
+    assert all(torch.equal(y, runs[0]) for y in runs)
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m.view(-1), torch.tensor([gs], dtype=torch.float32, device="cuda"), rows, k)).double().view(rows, k)
+
+    ids, wts = plan.ids.view(tokens, experts), plan.wts.view(tokens, experts).double()
+    x64, want = x.double(), torch.zeros((tokens, hidden), dtype=torch.float64, device="cuda")
+    for e in range(experts):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        full = deq(gu[e], 2 * inter, hidden, 0.03)
+        a = x64[t] @ full[:inter].t()
+        want.index_add_(0, t, wts[t, j, None] * ((a / (1 + torch.exp(-a)) * (x64[t] @ full[inter:].t())) @ deq(dn[e], hidden, inter, 0.7).t()))
+    bound = 2e-6 if dtype == torch.float32 else 2.0 ** -9 + 2e-6  # as above
+    assert (runs[0].double() - want).norm() <= bound * want.norm()
+    assert device_status() == 0
+
+
+
 @pytest.mark.parametrize("tokens", [8, 9, 40])
 @pytest.mark.parametrize("which", [0, 1, 2])
 def test_shared_matrix_off_16_bytes_is_refused(tokens, which):
