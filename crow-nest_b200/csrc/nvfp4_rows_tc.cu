@@ -218,10 +218,13 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 break;
             }
             uint8_t* bs = b0 + (i % NB) * B_STAGE;
+            // one copy of the code for both rows of a warp: with two, instructions come late (the roles of a CTA share the instruction cache): us per step with / without, 64 tokens
+            // of 512 experts 195.6 / 190.9, 128 tokens 291 / 272, of 64 experts (groups of eight) 148 / 134, f32 rows 171 / 151
+#pragma unroll 1
+            for (int row = (w - i) & 3; row < nrows; row += 4) {
+                to_digits<F32>(now[0], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
 #pragma unroll
-            for (int t = 0; t < 2; t++) {
-                const int row = ((w - i) & 3) + 4 * t;
-                if (row < nrows) to_digits<F32>(now[t], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
+                for (int j = 0; j < XR; j++) now[0][j] = now[1][j];
             }
             fence_async();
             __syncwarp();
