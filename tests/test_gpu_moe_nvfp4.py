@@ -35,6 +35,34 @@ def test_sigmoid_router_indices_are_bit_exact(tokens, experts, k, scale):
     assert np.max(np.abs(w.cpu().numpy() - rw)) <= 1e-6
 
 
+@pytest.mark.parametrize("experts,k", [(225, 8), (256, 8), (257, 9), (512, 10), (512, 16), (513, 17), (1000, 32), (1024, 10), (33, 2)])
+def test_router_picks_by_rank_are_those_of_the_rounds(experts, k):
+    """Rows whose best experts are spread over the warps of a block, sit in one of them, tie by the dozen (more than a warp can rank), or are fewer than k; warps enough for the picks and
+    one too few. Both routers, picks as the oracle's."""
+    rng = np.random.default_rng(experts + k)
+    spread = rng.standard_normal((6, experts)).astype(np.float32)
+    rising = np.sort(rng.standard_normal((2, experts)).astype(np.float32), axis=1)
+    tied = np.round(rng.standard_normal((6, experts)) * 2).astype(np.float32)
+    some = np.full((2, experts), -np.inf, np.float32)  # every probability but these is zero, and ties
+    some[:, rng.permutation(experts)[:k - 1]] = 1.0
+    flat = np.zeros((1, experts), np.float32)
+    logits = np.concatenate([spread, rising, rising[:, ::-1], tied, some, flat]).copy()
+    ids, w = moe.route_softmax_topk(torch.from_numpy(logits).cuda(), k)
+    rids, rw = oracle.route_softmax_topk(logits, k)
+    assert np.array_equal(ids.cpu().numpy(), rids)
+    assert np.max(np.abs(w.cpu().numpy() - rw)) <= 1e-6
+    bias = np.round(rng.uniform(-1, 1, size=experts), 1).astype(np.float32)
+    for b in (None, bias):
+        sids, sw = moe.route_sigmoid_topk(torch.from_numpy(logits).cuda(), None if b is None else torch.from_numpy(b).cuda(), k, 2.5)
+        rids, rw = oracle.route_sigmoid_topk(logits, np.zeros(experts, np.float32) if b is None else b, k, 2.5)
+        assert np.array_equal(sids.cpu().numpy(), rids)
+        assert np.max(np.abs(sw.cpu().numpy() - rw)) <= 1e-6
+    odd = torch.from_numpy(spread).cuda()
+    odd[0, 3], odd[1, :] = float("nan"), float("nan")  # a NaN takes the row's sum, and every probability with it: expert 0 k times
+    ids, _ = moe.route_softmax_topk(odd, k)
+    assert not ids[:2].any() and torch.equal(ids[2:].cpu(), torch.from_numpy(oracle.route_softmax_topk(spread[2:], k)[0]))
+
+
 def test_sigmoid_router_ties_and_nan():
     l = torch.tensor([[0.0, 1.0, 1.0, float("nan"), 1.0, -1.0, 1.0], [float("nan")] * 7], device="cuda")
     ids, _ = moe.route_sigmoid_topk(l, None, 3, 1.0)
