@@ -11,7 +11,7 @@
 //   gemv     y' = xh W_hat over a k-split: each CTA owns 8 adjacent tile columns (128 outputs) and
 //            k/(16 S) tile rows; the 768-byte run of 8 tiles per tile row arrives by 1-D bulk copy
 //            (TMA) into a shared-memory ring; warp w decodes tile column w: lane g extracts its 8
-//            states from a 64-bit window (compile-time shifts at K = 3), multiplies by 0x83DCD12D,
+//            states from two 32-bit windows (compile-time shifts at K = 2, 3, 3.5, 4), multiplies by 0x83DCD12D,
 //            sums the bytes with dp4a (+0x6400 = the f16 pattern of 1024 + s), maps pairs through
 //            one HFMA2 to the codec's f16 weights (bit-exact) and accumulates with f16 x f16 -> f32
 //            mixed FMAs; partial sums of the k-split go to scratch
@@ -19,7 +19,10 @@
 // The first step is part of the GEMV launch for x where there are few rows (every CTA transforms its k-split) and a launch of its own for more
 // (staged_rows), and a kernel of its own, with the activation, for h; the last one carries the weighted combine of a routed step. One token, four experts
 // of 4096 x 1536: eight launches 52.5 us, five 43.4.
-// The inner loop is instruction-bound, not HBM-bound: about 7 issue slots per 3-bit weight. A stage is a whole 128-row block of eight tiles: with
+// The inner loop is instruction-bound, not HBM-bound: about 6 issue slots per weight. us per step of 16 tokens, 64 experts of 4096 x 1536, top 4: K = 3 257.7 with three words a lane and two loads a
+// B operand, 249.7 with two and one; K = 3.5 480 with the words of every state looked up on their own, 290 with two windows; K = 4 439 / 256; one token at K = 2 61.9 / 41.4. Measured and not kept: pairs
+// of sums put together by a multiplication in place of a byte permute (260.1 at K = 3), shifts by multiplications (270 and more): IMAD and dp4a share a pipe that is as full as the one
+// of shifts and masks. A stage is a whole 128-row block of eight tiles: with
 // four the waits and counters of a stage took a step of 16 tokens from 280 to 296 us.
 // Three helpers restate reference text because their operation order defines the bits the parity contract asks for:
 // fwht128 follows mul1_fwht128 (engine/src/kernels_mul1.cu:74-88: the stage order and the a+b / a-b pairing), out_block
@@ -34,7 +37,8 @@ constexpr int MUL1_MAXT = CN_MAX_M;  // activation rows per slot
 constexpr int MUL1_GT = 8;           // most rows of a group when the MoE step bundles the combos of an expert (groups of 4 or 8)
 constexpr int RING = 2;              // stages of the tile ring
 constexpr int UROWS = 8;             // tile rows per stage: one 128-row block of the input
-constexpr int XPAD = 8;              // f16 elements added to the pitch of a staged activation row
+constexpr int XPAD = 16;             // f16 elements added to the pitch of a staged activation row
+constexpr int SMEM_MOST = 160 * 1024, PAD_MORE = 16;  // shared memory of a GEMV call with a pad of eight; bytes of a pad beyond that
 
 struct Mul1Spec {
     int k, n;        // in, out
@@ -91,6 +95,25 @@ __device__ __forceinline__ void store_hi_lo(uint16_t* xh, size_t plane, size_t a
     }
     *(uint2*)(xh + at) = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
     *(uint2*)(xh + plane + at) = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
+}
+
+// where word i of a staged row lies: see mul1_gemv_kernel
+__device__ __forceinline__ int word_at(int i) { return (i & ~7) | ((i & 3) << 1) | ((i >> 2) & 1); }
+// the same planes for four values (4 lane .. 4 lane + 3) of a 128-block in shared memory
+__device__ __forceinline__ void store_planes(uint16_t* blk, int plane, int lane, const float v[4], float mul) {
+    uint32_t* w = (uint32_t*)blk;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        uint16_t hi[2], lo[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const float s = v[2 * j + q] * mul;
+            const __half h = __float2half_rn(s);
+            hi[q] = __half_as_ushort(h), lo[q] = __half_as_ushort(__float2half_rn((s - __half2float(h)) * 2048.0f));
+        }
+        const int at = word_at(2 * lane + j);
+        w[at] = hi[0] | ((uint32_t)hi[1] << 16), w[plane / 2 + at] = lo[0] | ((uint32_t)lo[1] << 16);
+    }
 }
 
 // Where the activation rows of a GEMV come from: row t of slot s is row (s / x_div) * T + t of x, or rowsrc[s * T + t] (negative = an
@@ -191,29 +214,42 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t s0, uint32_t s1) {
     return w;
 }
 
-// Lane g's eight 16-bit states of one tile. K3: bits = 3, whole bitrate, every shift a constant after the
-// window is aligned to the lane's first bit. Otherwise the general circular extraction.
-template <bool K3>
-__device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const int lo[8], int wi0, int sh0, uint32_t st[8]) {
-    if (K3) {
-        // words wi0, wi0+1, wi0+2 (circular) hold bits [24g - 13, 24g + 24); align the window to bit 0
-        const uint32_t w0 = tile[wi0], w1 = tile[wi0 + 1 >= n32 ? wi0 + 1 - n32 : wi0 + 1], w2 = tile[wi0 + 2 >= n32 ? wi0 + 2 - n32 : wi0 + 2];
-        const uint32_t hi = __funnelshift_l(w1, w0, sh0), lw = __funnelshift_l(w2, w1, sh0);
-        // state j = bits [3j, 3j + 16) of the 64-bit window hi:lw (MSB first)
-        st[0] = hi >> 16;
-        st[1] = (hi >> 13) & 0xffffu;
-        st[2] = (hi >> 10) & 0xffffu;
-        st[3] = (hi >> 7) & 0xffffu;
-        st[4] = (hi >> 4) & 0xffffu;
-        st[5] = (hi >> 1) & 0xffffu;
-        st[6] = __funnelshift_l(lw, hi, 18) >> 16;
-        st[7] = __funnelshift_l(lw, hi, 21) >> 16;
-    } else {
+// A lane's eight states at a bitrate of K2 / 2 that is known at compile time. They lie in 16 + off(7) bits of the tile, which start at one of a few bits of a word: those that end within
+// the first 32 of them are cut out of the window `hi` of these, the others out of the last 32, `lw`. Where no lane starts so late that the second window goes beyond the next word (ALONE), both
+// come from the same two words; else the second has two of its own.
+template <int K2>
+struct Rate {
+    static constexpr int words = 4 * K2;  // of a tile
+    __host__ __device__ static constexpr int off(int j) { return K2 % 2 == 0 ? K2 / 2 * j : j / 2 * K2 + (j & 1 ? K2 / 2 + 1 : 0); }
+    static constexpr int second = off(7) > 16 ? off(7) - 16 : 0;  // first bit of `lw`
+    __host__ __device__ static constexpr bool alone() {
+        for (int g = 0; g < 32; g++)
+            if (((4 * K2 * g + K2 / 2 - 16) & 31) + second > 32) return false;
+        return true;
+    }
+    __host__ __device__ static constexpr bool fits() {
+        for (int j = 0; j < 8; j++)
+            if (off(j) > 16 && off(j) < second) return false;
+        return true;
+    }
+};
+// 16 bits of x from bit `at` on, the most significant bit being 0
+template <int AT>
+__device__ __forceinline__ uint32_t field(uint32_t x) {
+    return AT == 0 ? x >> 16 : (x >> (16 - AT)) & 0xffffu;
+}
+template <int K2, int J>
+__device__ __forceinline__ uint32_t state(uint32_t hi, uint32_t lw) {
+    using R = Rate<K2>;
+    constexpr bool first = R::off(J) <= 16;
+    return field<first ? R::off(J) : R::off(J) - R::second>(first ? hi : lw);
+}
+// The same at any bitrate.
+__device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const int lo[8], uint32_t st[8]) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int i = lo[j] >> 5, o = lo[j] & 31, i1 = i + 1 == n32 ? 0 : i + 1;
-            st[j] = __funnelshift_l(tile[i1], tile[i], o) >> 16;
-        }
+    for (int j = 0; j < 8; j++) {
+        const int i = lo[j] >> 5, o = lo[j] & 31, i1 = i + 1 == n32 ? 0 : i + 1;
+        st[j] = __funnelshift_l(tile[i1], tile[i], o) >> 16;
     }
 }
 
@@ -223,7 +259,8 @@ __device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const
 // HAD: the input transform is part of the launch: xh = H128(x * suh) per 128-block as hi / lo planes and 1 / scale, one warp per (row, block), straight
 // into shared memory. The CTAs of one k-split repeat it (some 150 instructions a block), which costs less than a launch before this one
 // and the planes' way through memory.
-template <bool K3, int MT, bool HAD>
+// K2: twice the bitrate where the kernel is built for it, 0: any
+template <int K2, int MT, bool HAD>
 __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, Mul1Spec sp_,
                                                         int S, int T, size_t plane, int SPC, Mul1In in) {
     pdl_launch_dependents();
@@ -248,8 +285,8 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
     uint64_t* full = (uint64_t*)smem;
     uint64_t* empty = full + RING;
     uint32_t* ring = (uint32_t*)(smem + 128);                                   // [RING][UROWS][8][n32]
-    // [2][T][pitch] f16: hi plane, lo plane; a row pitch of 16 bytes more than a multiple of 256 keeps the eight rows
-    // the lanes of a warp read at once on distinct banks
+    // [T][2][pitch] f16, hi and lo plane of a row beside each other, the words of every 16 values in the order 0 4 1 5 2 6 3 7: a lane's two words of a B operand are one 64-bit load. A pitch of
+    // 32 bytes more than a multiple of 256 keeps the four columns that half a warp reads at once on distinct banks
     const int pitch = rows + XPAD;
     uint16_t* xs = (uint16_t*)(smem + 128 + (size_t)RING * UROWS * run_bytes);
     float* xi = (float*)(xs + (size_t)2 * T * pitch);  // [T][rows/128]
@@ -297,15 +334,15 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
             const int t = i / nblk, b = i - t * nblk;
             float v[4], inv;
             const float mul = block(slot, t, T, k, kb0 * 16 + b * 128 + 4 * lane, lane, v, inv);
-            store_hi_lo(xs, (size_t)T * pitch, (size_t)t * pitch + b * 128 + 4 * lane, v, mul);
+            store_planes(xs + (size_t)2 * t * pitch + b * 128, pitch, lane, v, mul);
             if (lane == 0) xi[i] = inv;
         }
     } else {
         for (int i = threadIdx.x; i < T * rows / 2; i += 256) {
             const int t = i / (rows / 2), r = i - t * (rows / 2);
             const size_t at = ((size_t)slot * T + t) * k + (size_t)kb0 * 16;
-            ((uint32_t*)(xs + (size_t)t * pitch))[r] = ((const uint32_t*)(xh + at))[r];
-            ((uint32_t*)(xs + (size_t)(T + t) * pitch))[r] = ((const uint32_t*)(xh + plane + at))[r];
+            ((uint32_t*)(xs + (size_t)2 * t * pitch))[word_at(r)] = ((const uint32_t*)(xh + at))[r];
+            ((uint32_t*)(xs + (size_t)(2 * t + 1) * pitch))[word_at(r)] = ((const uint32_t*)(xh + plane + at))[r];
         }
         for (int i = threadIdx.x; i < T * nblk; i += 256) {
             const int t = i / nblk, b = i - t * nblk;
@@ -335,18 +372,21 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
 #pragma unroll
     for (int i = 0; i < NM; i++) {
         const int rb = min(4 * i + (g >> 1), T - 1), rc = min(4 * i + t4, T - 1);
-        xb[i] = xs + ((size_t)(g & 1) * T + rb) * pitch + 2 * t4;
+        xb[i] = xs + (size_t)(2 * rb + (g & 1)) * pitch + 4 * t4;
         xil[i] = xi + rc * nblk;
     }
     float acc[NM][4], tot0[NM], tot1[NM];
 #pragma unroll
     for (int i = 0; i < NM; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = tot0[i] = tot1[i] = 0.0f;
-    // Everything a tile needs beyond its own words is a constant offset from pointers that move once per stage: at
-    // K = 3 a tile is 24 words, and a split is a whole number of stages and of 128-row blocks (tps % 8 == 0, which
+    // Everything a tile needs beyond its own words is a constant offset from pointers that move once per stage: where the bitrate
+    // is known a tile's words are (24 at K = 3), and a split is a whole number of stages and of 128-row blocks (tps % 8 == 0, which
     // the launcher guarantees), so the loop carries no division, no bounds test and no address arithmetic per tile.
-    constexpr int TW = K3 ? 24 : 0;  // words of a tile when known at compile time
-    const int tw = K3 ? TW : n32;
-    const int o1 = wi0 + 1 >= tw ? wi0 + 1 - tw : wi0 + 1, o2 = wi0 + 2 >= tw ? wi0 + 2 - tw : wi0 + 2;
+    using R = Rate<K2 ? K2 : 6>;
+    static_assert(R::fits(), "states that lie in neither window");
+    constexpr int TW = K2 ? R::words : 0;  // words of a tile when known at compile time
+    constexpr bool ALONE = R::alone();
+    const int tw = K2 ? TW : n32;
+    const int o1 = wi0 + 1 == tw ? 0 : wi0 + 1, wi1 = (wi0 + ((sh0 + R::second) >> 5)) % tw, o2 = wi1 + 1 == tw ? 0 : wi1 + 1, sh1 = ALONE ? sh0 + R::second : (sh0 + R::second) & 31;
     const uint32_t* lane_tile = ring + (size_t)warp * tw;  // this warp's tile of the ring's first tile row
     int s = 0, cs = 0, spi = 0;
     uint32_t ph = 0;
@@ -360,29 +400,22 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
 #pragma unroll
         for (int u = 0; u < UROWS; u++) {
             uint32_t st[8];
-            if (K3) {
-                // words wi0, wi0 + 1, wi0 + 2 (circular) hold bits [24 g - 13, 24 g + 24) of the tile; the window is
-                // aligned to the lane's first bit and state j = bits [3 j, 3 j + 16) of it, most significant bit first
+            if (K2) {
                 const uint32_t* tl = tb + u * 8 * TW;
-                const uint32_t w0 = tl[wi0], w1 = tl[o1], w2 = tl[o2];
-                const uint32_t hi = __funnelshift_l(w1, w0, sh0), lw = __funnelshift_l(w2, w1, sh0);
-                st[0] = hi >> 16;
-                st[1] = (hi >> 13) & 0xffffu;
-                st[2] = (hi >> 10) & 0xffffu;
-                st[3] = (hi >> 7) & 0xffffu;
-                st[4] = (hi >> 4) & 0xffffu;
-                st[5] = (hi >> 1) & 0xffffu;
-                st[6] = __funnelshift_l(lw, hi, 18) >> 16;
-                st[7] = __funnelshift_l(lw, hi, 21) >> 16;
+                const uint32_t w0 = tl[wi0], w1 = tl[o1];
+                // (a shift of 32 is the second word itself)
+                const uint32_t hi = __funnelshift_l(w1, w0, sh0), lw = R::second == 0 ? hi : ALONE ? __funnelshift_lc(w1, w0, sh1) : __funnelshift_l(tl[o2], tl[wi1], sh1);
+                st[0] = state<R::words / 4, 0>(hi, lw), st[1] = state<R::words / 4, 1>(hi, lw), st[2] = state<R::words / 4, 2>(hi, lw), st[3] = state<R::words / 4, 3>(hi, lw);
+                st[4] = state<R::words / 4, 4>(hi, lw), st[5] = state<R::words / 4, 5>(hi, lw), st[6] = state<R::words / 4, 6>(hi, lw), st[7] = state<R::words / 4, 7>(hi, lw);
             } else {
-                lane_states<false>(tb + (size_t)u * 8 * tw, n32, lo, wi0, sh0, st);
+                lane_states(tb + (size_t)u * 8 * tw, n32, lo, st);
             }
             const uint32_t w01 = mul1_pair(st[0], st[1]), w23 = mul1_pair(st[2], st[3]);
             const uint32_t w45 = mul1_pair(st[4], st[5]), w67 = mul1_pair(st[6], st[7]);
 #pragma unroll
             for (int i = 0; i < NM; i++) {
-                const uint32_t* xr = (const uint32_t*)(xb[i] + kx + u * 16);
-                mma16816(acc[i], w01, w45, w23, w67, xr[0], xr[4]);
+                const uint2 xr = *(const uint2*)(xb[i] + kx + u * 16);
+                mma16816(acc[i], w01, w45, w23, w67, xr.x, xr.y);
             }
         }
         __syncwarp();
@@ -605,11 +638,12 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     // k-splits per CTA: as many as still leave about four CTAs per SM (the splits keep separate partial sums, so
     // this only moves work between CTAs) and fit the staged activations
     int spc = 1;
+    const size_t most = SMEM_MOST + (size_t)2 * T * PAD_MORE;  // (a limit of the calls, which has no part of the pad in it that a row got later)
     for (int c = S; c > 1; c--) {
         if (S % c) continue;
         const long long ctas = (long long)mats * (s.n / 128) * (S / c) * live;
         const size_t need = 128 + (size_t)RING * UROWS * 32 * s.n32 + (size_t)2 * T * (c * tps * 16 + XPAD) * 2 + 8 + (size_t)T * (c * tps / 8) * 4;
-        if (ctas >= 592 && need <= 160 * 1024) {
+        if (ctas >= 592 && need <= most) {
             spc = c;
             break;
         }
@@ -617,17 +651,18 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     const int rows = spc * tps * 16;
     const size_t smem = 128 + (size_t)RING * UROWS * 32 * s.n32 + (size_t)2 * T * (rows + XPAD) * 2 + 8 + (size_t)T * (rows / 128) * 4;
     dim3 grid(mats * (s.n / 128), S / spc, slots);
-    if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "mul1 gemv: %zu B of shared memory per block", smem);
-    const bool k3 = s.bits == 3 && !s.half;
+    if (smem > most) CN_FAIL(CN_ERR_LIMIT, "mul1 gemv: %zu B of shared memory per block", smem);
+    const int rate = 2 * s.bits + (s.half ? 1 : 0), k2 = rate == 4 || rate == 6 || rate == 7 || rate == 8 ? rate : 0;
     const int mt = T == 1 ? 1 : (T == 2 ? 2 : (T <= 4 ? 4 : 8));
     const Mul1In none = {};
-#define CN_MUL1_CASE(K3V, MTV, HADV)                                                                                                \
-    if (k3 == K3V && mt == MTV && (in != nullptr) == HADV) {                                                                        \
-        CN_ALLOW_SMEM((mul1_gemv_kernel<K3V, MTV, HADV>), 160 * 1024);                                                              \
-        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K3V, MTV, HADV>), grid, dim3(288), smem, st, const_cast<unsigned long long*>(ptrs), sa, sb ? *sb : sa, s, S, T, plane, spc, in ? *in : none)); \
+#define CN_MUL1_CASE(K2V, MTV, HADV)                                                                                                \
+    if (k2 == K2V && mt == MTV && (in != nullptr) == HADV) {                                                                        \
+        CN_ALLOW_SMEM((mul1_gemv_kernel<K2V, MTV, HADV>), SMEM_MOST + 2 * MUL1_MAXT * PAD_MORE);                                    \
+        CN_CUDA(cn_launch_pdl((mul1_gemv_kernel<K2V, MTV, HADV>), grid, dim3(288), smem, st, const_cast<unsigned long long*>(ptrs), sa, sb ? *sb : sa, s, S, T, plane, spc, in ? *in : none)); \
     }
-#define CN_MUL1_CASES(K3V, HADV) CN_MUL1_CASE(K3V, 1, HADV) CN_MUL1_CASE(K3V, 2, HADV) CN_MUL1_CASE(K3V, 4, HADV) CN_MUL1_CASE(K3V, 8, HADV)
-    CN_MUL1_CASES(true, true) CN_MUL1_CASES(true, false) CN_MUL1_CASES(false, true) CN_MUL1_CASES(false, false)
+#define CN_MUL1_CASES(K2V) CN_MUL1_CASE(K2V, 1, true) CN_MUL1_CASE(K2V, 2, true) CN_MUL1_CASE(K2V, 4, true) CN_MUL1_CASE(K2V, 8, true) \
+    CN_MUL1_CASE(K2V, 1, false) CN_MUL1_CASE(K2V, 2, false) CN_MUL1_CASE(K2V, 4, false) CN_MUL1_CASE(K2V, 8, false)
+    CN_MUL1_CASES(0) CN_MUL1_CASES(4) CN_MUL1_CASES(6) CN_MUL1_CASES(7) CN_MUL1_CASES(8)
 #undef CN_MUL1_CASES
 #undef CN_MUL1_CASE
     CN_CUDA(cudaGetLastError());

@@ -69,6 +69,29 @@ def test_gemv_matches_the_cpu_reference(K, hidden, inter, t):
     plan.free()
 
 
+@pytest.mark.parametrize("K", [1.0, 1.5, 2.0, 2.5, 3.0, 3.5, 4.0, 5.0, 8.0])
+@pytest.mark.parametrize("t", [1, 2, 4, 7])
+@pytest.mark.parametrize("slots", [1, 520])
+def test_every_bitrate_at_every_row_count(K, t, slots):
+    """Rates whose states come out of windows known at compile time (2, 3, 3.5, 4) and the others, each with its words of a tile and the lane whose window goes round the tile's end; rows
+    transformed inside the GEMV (few slots) and staged by a launch of their own (many; the rows of the last slots are looked at). The other records are null."""
+    hidden, inter = 768, 512
+    rec = tk.mul1_record(int(2 * K) + t, hidden, inter, K)
+    tb, (gs, gv, us, uv, ds, dv) = expert_parts(rec, hidden, inter, K)
+    d_rec = dev(rec)
+    ptrs = torch.zeros(slots, dtype=torch.int64, device="cuda")
+    ptrs[-1] = d_rec.data_ptr()
+    plan = mul1.Mul1Plan(hidden, inter, K, slots=slots, tokens=t)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    for which, (k, n, tro, su, sv) in enumerate([(hidden, inter, 0, gs, gv), (hidden, inter, tb, us, uv), (inter, hidden, 2 * tb, ds, dv)]):
+        x = torch.rand((slots, t, k), device="cuda", generator=gen) * 4 - 2
+        y = plan.run_slots(which, ptrs, x)[-1].cpu().numpy().astype(np.float64)
+        ref = oracle.mul1_gemv(rec[tro:tro + tb], su, sv, k, n, K, x[-1].cpu().numpy(), threads=8).astype(np.float64)
+        # two transforms of seven f32 additions and a sum of k products of 22-bit activations, against the same in another order: some 30 roundings of 6e-8
+        assert np.linalg.norm(y - ref) <= 4e-6 * np.linalg.norm(ref)
+    plan.free()
+
+
 def test_null_slots_are_skipped_and_rows_are_batch_invariant():
     hidden, inter, K = 512, 256, 3.0
     rec = dev(tk.mul1_record(3, hidden, inter, K))
