@@ -39,7 +39,7 @@ constexpr int NDONE = 4;    // barriers of finished chunks
 constexpr int MAX_RAW = 4;  // container stages
 constexpr int NA = 2;       // chunks laid out for the tensor core
 constexpr int NSLOT = 3;    // tiles whose sums are on their way in a cluster
-constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + 2 + NSLOT + 2;
+constexpr int NBAR = 2 * MAX_RAW + NA + NX + NDONE + NSLOT + 2;
 constexpr int EPI_WARPS = 4, LOADER = 12, ISSUER = 13;  // warps 0-3 sums and output, 4-7 weights, 8-11 activations
 constexpr int THREADS = 448;
 constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk factors [NX][8] {factor, blocks without digits}; [NX][4] scale bytes of 0xFF seen
@@ -128,10 +128,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint64_t* raw_full = (uint64_t*)smem;
     uint64_t* raw_empty = raw_full + MAX_RAW;
     uint64_t* a_full = raw_empty + MAX_RAW;   // [NA]
-    uint64_t* xbar = a_full + NA;            // [NX] digits of a chunk
+    uint64_t* xbar = a_full + NA;            // [NX] digits of a chunk, and its accumulators (those of two chunks before) have been read
     uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
-    uint64_t* d_empty = done + NDONE;         // [2] accumulators
-    uint64_t* exbar = d_empty + 2;            // [NSLOT] sums handed over
+    uint64_t* exbar = done + NDONE;           // [NSLOT] sums handed over
     uint64_t* meet = exbar + NSLOT;           // [2] the four adding warps, tile by tile: its sums are in the slot (one CTA), have been read from it (cluster)
     uint32_t* tmem_slot = (uint32_t*)(meet + 2);
     float2* fs = (float2*)(smem + FS_OFF);    // [NX][8]
@@ -159,13 +158,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     };
     if (warp == 0) { CN_STAMP(0); }
     if (warp == LOADER) {
-        // a barrier a lane: container stages, operand stages, digits, finished chunks, accumulators, sums handed over
+        // a barrier a lane: container stages, operand stages, digits and accumulators, finished chunks, sums handed over
         for (int i = lane; i < NBAR; i += 32)
             mbar_init(raw_full + i, i < MAX_RAW                         ? 1
                                     : i < 2 * MAX_RAW + NA              ? 4
-                                    : i < 2 * MAX_RAW + NA + NX         ? (MT < 4 ? MT : 4)
+                                    : i < 2 * MAX_RAW + NA + NX         ? (MT < 4 ? MT : 4) + EPI_WARPS
                                     : i < 2 * MAX_RAW + NA + NX + NDONE ? 2
-                                    : i < NBAR - NSLOT - 2              ? EPI_WARPS
                                     : i < NBAR - 2                      ? 1
                                                                         : EPI_WARPS);
         mbar_fence_init();
@@ -232,7 +230,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 for (int j = 0; j < 4; j++) cp_sf(ta + 4 * j, sa + 32 * j);
             }
             __syncwarp();
-            if (!mbar_wait(&xbar[i % NX], (i / NX) & 1) || (i >= 2 && !mbar_wait(&d_empty[a], ((i >> 1) - 1) & 1))) {
+            if (!mbar_wait(&xbar[i % NX], (i / NX) & 1)) {  // (one wait for both: each costs the issuer some 75 cycles, passed or not)
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 break;
             }
@@ -322,6 +320,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
     } else {
         // ------------------------------------------------------------ sums and output
+        if (lane < 2) mbar_arrive(&xbar[lane]);  // the accumulators of the first two chunks
         pdl_wait();
         const float gs0 = *p.gs0, gs1 = gu ? *p.gs1 : 0.0f, gs = gu && warp >= 2 ? gs1 : gs0;
         const unsigned int epoch = p.yl_world > 0 ? *(volatile const unsigned int*)p.yl_epoch : 0u;
@@ -350,7 +349,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 if (m0 + G == MT) {
                     tc_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&d_empty[i & 1]);
+                    if (lane == 0) mbar_arrive(&xbar[(i + 2) % NX]);
                 }
 #pragma unroll
                 for (int m = 0; m < G; m++) {

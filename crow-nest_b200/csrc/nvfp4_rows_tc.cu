@@ -24,7 +24,7 @@ constexpr int CH = 256;      // values of k in a chunk
 constexpr int PIECE = 32 * 144;  // container bytes of a warp's 32 rows and a chunk
 __host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 2 : 3; }  // chunks in flight, as many as fit
 constexpr int NA = 2, NB = 2, NX = 16, NDONE = 4, NU = 8;  // operand stages, chunks of digits, chunk factors, finished chunks, units in the ring
-constexpr int NBAR = NA + NX + NDONE + 2 + 2 * NU;
+constexpr int NBAR = NX + NDONE + 2 * NU;
 constexpr int SCOUT = 12, ISSUER = 13, THREADS = 448;
 constexpr int FS_OFF = 512, WF_OFF = 1536, UNIT_OFF = 1792, HEADER = 2560;
 // columns of the widest MMA, whose N is a multiple of 16: the accumulators lie this far apart in tensor memory (eight f32 rows are 88 columns, and 96 are written)
@@ -50,11 +50,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     using Acc = typename std::conditional<F32, double, float>::type;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *a0 = smem, *b0 = a0 + NA * A_STAGE, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;
-    uint64_t* a_full = (uint64_t*)head;       // [NA]
-    uint64_t* xbar = a_full + NA;             // [NX] digits of a chunk
-    uint64_t* done = xbar + NX;               // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
-    uint64_t* d_empty = done + NDONE;         // [2] accumulators
-    uint64_t* unit_full = d_empty + 2;        // [NU]
+    uint64_t* ready = (uint64_t*)head;        // [NX] weights and digits of a chunk, and its accumulators (those of two chunks before) have been read
+    uint64_t* done = ready + NX;              // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
+    uint64_t* unit_full = done + NDONE;       // [NU]
     uint64_t* unit_empty = unit_full + NU;    // [NU]
     uint32_t* tmem_slot = (uint32_t*)(unit_empty + NU);
     float2* fs = (float2*)(head + FS_OFF);      // [NX][8] {factor, blocks without digits}
@@ -66,9 +64,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     const size_t row_bytes = (size_t)nk * 144;
 
     if (warp == SCOUT) {
-        // a barrier a lane and round: operand stages, digits, finished chunks, accumulators, units full and empty (four + four + four + one warps read them)
-        for (int i = lane; i < NBAR; i += 32)
-            mbar_init(a_full + i, i < NA + NX ? 4 : i < NA + NX + NDONE ? 2 : i < NA + NX + NDONE + 2 ? 4 : i < NBAR - NU ? 1 : 13);
+        // a barrier a lane and round: chunks (four warps each that bring weights, digits and empty accumulators), finished chunks, units full and empty (four + four + four + one warps read them)
+        for (int i = lane; i < NBAR; i += 32) mbar_init(ready + i, i < NX ? 12 : i < NX + NDONE ? 2 : i < NBAR - NU ? 1 : 13);
         mbar_fence_init();
         __syncwarp();
     } else if (warp == ISSUER) {
@@ -149,8 +146,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             const uint32_t idesc = idesc_bs((nrows * LV + 15) & ~15);
             for (int ch = 0; ch < nk; ch++, i++) {
                 const int a = i & 1;
-                if (!mbar_wait(&a_full[a], (uint32_t)(i >> 1) & 1u) || !mbar_wait(&xbar[i % NX], (uint32_t)(i / NX) & 1u) ||
-                    (i >= 2 && !mbar_wait(&d_empty[a], (uint32_t)((i >> 1) - 1) & 1u))) {
+                if (!mbar_wait(&ready[i % NX], (uint32_t)(i / NX) & 1u)) {  // (one wait for all three: each costs some 75 cycles, passed or not)
                     cn_dev_fail(CN_DEV_WAIT_FULL);
                     ok = false;
                     break;
@@ -229,7 +225,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             fence_async();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&xbar[i % NX]);
+                mbar_arrive(&ready[i % NX]);
                 if (q != at) mbar_arrive(&unit_empty[at % NU]);
             }
             nrows = next_rows;
@@ -307,7 +303,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 if (lane == 0) wf[(i % NX) * 4 + w] = odd;
                 fence_async();
                 __syncwarp();  // every lane has read the stage
-                if (lane == 0) mbar_arrive(&a_full[i & 1]);
+                if (lane == 0) mbar_arrive(&ready[i % NX]);
                 issue();
                 if (++s == D) s = 0;
             }
@@ -316,6 +312,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ------------------------------------------------------------ sums and output: a thread is a row of the tile
+        if (lane < 2) mbar_arrive(&ready[lane]);  // the accumulators of the first two chunks
         const float gs0 = __ldg(c.gs0), gs1 = gu ? __ldg(c.gs1) : 0.0f, gs = gu && lane >= 16 ? gs1 : gs0;
         bool ok = true;
         for (int q = 0, i = 0; ok; q++) {
@@ -361,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 }
                 tc_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&d_empty[i & 1]);
+                if (lane == 0) mbar_arrive(&ready[(i + 2) % NX]);
                 if (slow && row < c.rows) {
                     const uint8_t* wr = (const uint8_t*)(gu && lane >= 16 ? u.w1 : u.w0) + ((size_t)row * nk + ch) * 144;
 #pragma unroll 1
