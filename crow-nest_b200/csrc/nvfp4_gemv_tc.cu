@@ -293,8 +293,11 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
     } else if (warp >= EPI_WARPS) {
         // ------------------------------------------------------------ container blocks -> operand layout: a warp takes 32 rows, a lane the four
-        // blocks of a row (144 bytes: no bank twice among eight lanes, nor in the swizzled lines)
+        // blocks of a row (144 bytes: no bank twice among eight lanes of neighbouring rows, nor in the swizzled lines)
         const int w = warp - 4;
+        // eight f32 rows: rows in order, the other order needs registers that there are not (4096 x 4096 10.95 us so, 11.1; gate / up of 17408 x 5120 51.4 / 52.2)
+        constexpr bool IN_ORDER = MT == 8 && F32;
+        const int row = IN_ORDER ? 32 * w + lane : operand_row(w, lane);
         int s = 0;
         uint32_t par = 0;
         for (int i = 0; i < total; i++) {
@@ -302,15 +305,18 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 break;
             }
-            const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + (w * 32 + lane) * 9;
+            const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + row * 9;
             uint32_t v[36];
             const uint32_t odd = load_row(src, v);
             if (i >= NA && !mbar_wait(&done[(i - NA) % NDONE], ((i - NA) / NDONE) & 1)) {
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            store_row(a0 + (i & 1) * A_STAGE, w, lane, v);
-            if (lane == 0) wf[(i % NX) * 4 + w] = odd;
+            store_row(a0 + (i & 1) * A_STAGE, row, v);
+            if (!IN_ORDER)
+                put_odd(wf + (i % NX) * 4, w, lane, odd);
+            else if (lane == 0)
+                wf[(i % NX) * 4 + w] = odd;
             fence_async();
             __syncwarp();
             // (the stage is given back here and not behind the loads: an arrival can overtake loads whose values nothing has used yet)

@@ -6,7 +6,8 @@
 // Persistent CTAs, two per SM, walk units of (group, 128-row tile; 64 gate and 64 up rows). The matrices come from device tables, so there is no tensor map:
 // a scout warp looks up 32 units at a time (positions, combos, expert, addresses) and hands them to the other warps through a ring, and the warps that lay
 // the weights out for the tensor core bring them in themselves, by 16-byte asynchronous copies, past the ends of units. Warps: 0-3 add up and store,
-// 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form a warp's rows are 16 of gate and the same 16 of up.
+// 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form an adding warp's rows are 16 of gate and the same 16 of up; a weights warp's eight rows of each
+// adding warp's, so two of them bring gate and two up.
 //
 // What bounds it: the way of the weights through a warp (gate / up of 64 tokens, 512 experts of 2048 x 512, top 10: 2150 cycles a chunk of 18 KB and CTA, 470 of
 // them loads, 500 stores and their fence, 580 the copies of a later chunk), 4.1 TB/s; us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16
@@ -237,15 +238,16 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         const int w = warp - 4;
         const uint32_t ring = smem_u32(r0) + (uint32_t)(w * D * PIECE);
         const uint64_t pol = l2_policy_evict_first();
-        // sixteen-byte pieces, nine to a row and chunk, side by side in the stage; in the gate / up form rows 16-31 of a warp are the up rows of its gate rows
+        // sixteen-byte pieces, nine to a row and chunk, side by side in the stage, which has the rows by lanes
+        auto tile_row = [&](int row) { return (row >> 3) * (gu ? 16 : 32) + (row & 7); };  // from the warp's first on
         uint32_t off[9];
 #pragma unroll
         for (int j = 0; j < 9; j++) {
             const int id = lane + 32 * j, row = id / 9;
-            off[j] = (uint32_t)(gu ? row & 15 : row) * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u;
+            off[j] = (uint32_t)tile_row(row) * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u;
         }
         int iq = 0, ic = 0, is = 0, have = 0, asked = 0;  // what is asked for next: unit, chunk, stage; rows there are; chunks so far
-        const uint8_t *from = nullptr, *from1 = nullptr;
+        const uint8_t* from = nullptr;
         bool more = true, ok = true;
         auto issue = [&]() {
             if (more && ic == 0) {
@@ -255,27 +257,26 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 } else {
                     const Unit& u = units[iq % NU];
                     more = u.nrows >= 0;
-                    const int first = u.tile * per_tile + w * (gu ? 16 : 32);
-                    from = (const uint8_t*)u.w0 + (size_t)first * row_bytes, from1 = (const uint8_t*)u.w1 + (size_t)first * row_bytes;
-                    have = min(max(c.rows - first, 0), gu ? 16 : 32);
+                    const int first = u.tile * per_tile + 8 * (gu ? w & 1 : w);
+                    from = (const uint8_t*)(gu && w >= 2 ? u.w1 : u.w0) + (size_t)first * row_bytes;
+                    have = c.rows - first;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&unit_empty[iq % NU]);  // (nothing else of the unit is wanted here)
                 }
             }
             if (more) {
                 const uint32_t dst = ring + (uint32_t)(is * PIECE + lane * 16);
-                // piece 32 j + lane: of row 16 and on from piece 144
-                const uint8_t *lo = from + (uint32_t)(ic * 144), *hi = gu ? from1 + (uint32_t)(ic * 144) : lo, *mid = lane < 16 ? lo : hi;
+                const uint8_t* chunk = from + (uint32_t)(ic * 144);
                 auto copy = [&](int j, uint32_t at) {
-                    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"((j < 4 ? lo : j == 4 ? mid : hi) + at), "l"(pol) : "memory");
+                    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"(chunk + at), "l"(pol) : "memory");
                 };
-                if (have == (gu ? 16 : 32)) {
+                if (have > tile_row(31)) {
 #pragma unroll
                     for (int j = 0; j < 9; j++) copy(j, off[j]);
                 } else {  // the matrix ends inside these rows
 #pragma unroll 1
                     for (int j = 0; j < 9; j++) {
-                        const int id = lane + 32 * j, row = id / 9, r = gu ? row & 15 : row;
+                        const int id = lane + 32 * j, row = id / 9, r = tile_row(row);
                         if (r < have) copy(j, (uint32_t)r * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u);
                     }
                 }
@@ -299,8 +300,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            store_row(a0 + (i & 1) * A_STAGE, w, lane, v);
-            if (lane == 0) wf[(i % NX) * 4 + w] = odd;
+            store_row(a0 + (i & 1) * A_STAGE, operand_row(w, lane), v);
+            put_odd(wf + (i % NX) * 4, w, lane, odd);
             fence_async();
             __syncwarp();  // every lane has read the stage
             if (lane == 0) mbar_arrive(&ready[i % NX]);
