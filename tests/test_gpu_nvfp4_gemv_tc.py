@@ -152,6 +152,28 @@ def test_scale_bytes_that_the_tensor_core_reads_differently():
     _near(ops.launch_gemv(w, x), x.double() @ w64.t())
 
 
+@pytest.mark.parametrize("gu", [False, True])
+@pytest.mark.parametrize("m,dtype", [(1, torch.bfloat16), (8, torch.bfloat16), (4, torch.float32), (8, torch.float32)])
+def test_one_row_of_a_tile_with_such_scale_bytes(gu, m, dtype):
+    """Row t of tile t alone has 0xFF: the lane that meets it and the thread that sums the row are in different warps."""
+    per = 64 if gu else 128
+    rng, g, _ = _make(per * per, 1024, 11)
+    sel = torch.arange(per, device="cuda") * (per + 1)
+    g.w.view(per * per, 16, 36)[:, :, :4][sel] = 0xFF
+    w64 = ops.dequant(g, rule=True).double().view(per * per, 1024)
+    x = torch.from_numpy(rng.standard_normal((m, 1024)).astype(np.float32)).cuda().to(dtype)
+    want = x.double() @ w64.t()
+    if gu:  # (up of the same rows)
+        want, y = want / (1 + torch.exp(-want)) * want, ops.launch_gemv_gu(g, g, x)
+    else:
+        y = ops.launch_gemv(g, x)
+    bound = 2.0 ** -8 + 1e-6 if dtype == torch.bfloat16 else 2.0 ** -20  # half a step of a bf16 value is 2^-8 of it at most; f32: products of a block in 64 bits, rows as digits
+    for part in (sel, torch.arange(per * per, device="cuda")):
+        off = (y.double() - want)[:, part]
+        assert off.norm() <= bound * want[:, part].norm()
+    assert device_status() == 0
+
+
 def test_lines_of_a_larger_slice():
     import ctypes as C
     from crownest_b200 import dense
