@@ -212,21 +212,25 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             if (++ch == nk) ch = 0, q++, next_rows = unit(q);
             if (next_rows >= 0) fetch(q, next_rows, ch, i + 1);
             if (!ok) break;
-            if (i >= NB && !mbar_wait(&done[(i - NB) % NDONE], (uint32_t)((i - NB) / NDONE) & 1u)) {
-                cn_dev_fail(CN_DEV_WAIT_EMPTY);
-                break;
-            }
-            uint8_t* bs = b0 + (i % NB) * B_STAGE;
-            // one copy of the code for both rows of a warp: with two, instructions come late (the roles of a CTA share the instruction cache): us per step with / without, 64 tokens
-            // of 512 experts 195.6 / 190.9, 128 tokens 291 / 272, of 64 experts (groups of eight) 148 / 134, f32 rows 171 / 151
+            // a warp without a row in this chunk only counts itself (64 tokens of 512 experts 176.4 -> 174.0 us). It has one every four chunks at least, so it is no more than six chunks
+            // ahead of the MMAs, and there are NX slots.
+            if (((w - i) & 3) < nrows) {
+                if (i >= NB && !mbar_wait(&done[(i - NB) % NDONE], (uint32_t)((i - NB) / NDONE) & 1u)) {
+                    cn_dev_fail(CN_DEV_WAIT_EMPTY);
+                    break;
+                }
+                uint8_t* bs = b0 + (i % NB) * B_STAGE;
+                // one copy of the code for both rows of a warp: with two, instructions come late (the roles of a CTA share the instruction cache): us per step with / without, 64 tokens
+                // of 512 experts 195.6 / 190.9, 128 tokens 291 / 272, of 64 experts (groups of eight) 148 / 134, f32 rows 171 / 151
 #pragma unroll 1
-            for (int row = (w - i) & 3; row < nrows; row += 4) {
-                to_digits<F32>(now[0], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
+                for (int row = (w - i) & 3; row < nrows; row += 4) {
+                    to_digits<F32>(now[0], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
 #pragma unroll
-                for (int j = 0; j < XR; j++) now[0][j] = now[1][j];
+                    for (int j = 0; j < XR; j++) now[0][j] = now[1][j];
+                }
+                fence_async();
+                __syncwarp();
             }
-            fence_async();
-            __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&ready[i % NX]);
                 if (q != at) mbar_arrive(&unit_empty[at % NU]);
