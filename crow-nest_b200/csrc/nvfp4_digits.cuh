@@ -23,6 +23,14 @@ __device__ __forceinline__ void umma_bs(uint32_t tmem_d, uint64_t da, uint64_t d
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
         : "memory");
 }
+// the same with A in tensor memory: a row's 64 values in eight columns of its lane
+__device__ __forceinline__ void umma_bs_ta(uint32_t tmem_d, uint32_t ta, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], [%1], %2, %3, [%4], [%5], p;\n\t}"
+        ::"r"(tmem_d), "r"(ta), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -150,7 +158,8 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
 __device__ __forceinline__ double power_of_two(float f) { return __hiloint2double((int)((__float_as_uint(f) >> 3) + (896u << 20)), 0); }
 
 // ---------------------------------------------------------------- container blocks -> operand layout (a lane: the four blocks of a row)
-constexpr int A_CODES = 128 * 128, A_STAGE = A_CODES + 4 * 512;  // a chunk of 128 rows as operand A: 128-byte swizzled rows, then the scales of the four MMAs
+constexpr int A_CODES = 128 * 128, A_SCALES = 4 * 512, A_STAGE = A_CODES + A_SCALES;  // a chunk of 128 rows as operand A: 128-byte swizzled rows, then the scales of the four MMAs
+constexpr int A_COLS = 32;  // the codes of a chunk in tensor memory: columns
 
 // The operand row that lane `lane` of weights warp w lays out: eight rows of each of the four groups of 32 whose scales lie side by side in 16 bytes. So the scale bytes of a warp fill
 // 128 bytes (those of 32 rows in a row would lie 16 bytes apart, four ways into the same banks). us, rows in order / so: one row of gate / up 17408 x 5120 19.1 / 18.7, four 24.0 / 23.0,
@@ -183,6 +192,10 @@ __device__ __forceinline__ uint32_t load_row(const uint4* src, uint32_t (&v)[36]
     }
     return odd;
 }
+__device__ __forceinline__ void store_scales(uint8_t* dst, int row, const uint32_t (&v)[36]) {
+#pragma unroll
+    for (int b = 0; b < 4; b++) *(uint32_t*)(dst + b * 512 + (row & 31) * 16 + (row >> 5) * 4) = v[9 * b];
+}
 // row `row` of the operand stage at dst
 __device__ __forceinline__ void store_row(uint8_t* dst, int row, const uint32_t (&v)[36]) {
     uint8_t* line = dst + row * 128;
@@ -191,8 +204,19 @@ __device__ __forceinline__ void store_row(uint8_t* dst, int row, const uint32_t 
     for (int b = 0; b < 4; b++) {
         *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
         *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
-        *(uint32_t*)(dst + A_CODES + b * 512 + (row & 31) * 16 + (row >> 5) * 4) = v[9 * b];
     }
+    store_scales(dst + A_CODES, row, v);
+}
+// ... and with the codes in tensor memory, where a warp reaches 32 lanes: row 32 w + lane
+__device__ __forceinline__ void store_row_ta(uint32_t taddr, uint8_t* scales, int w, int lane, const uint32_t (&v)[36]) {
+    uint32_t codes[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) codes[i] = v[9 * (i >> 3) + 1 + (i & 7)];
+    tc_after();  // (the MMAs that read these columns are done)
+    tc_st32(taddr + ((uint32_t)(w * 32) << 16), codes);
+    store_scales(scales, 32 * w + lane, v);
+    tc_wait_st();
+    tc_before();
 }
 
 // ---------------------------------------------------------------- sums

@@ -47,8 +47,11 @@ __host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_o
 __host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
 __host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
 __host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                                // chunks of digits
-__host__ __device__ constexpr int tmem_cols(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 <= 128 ? 128 : 256; }
-__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * A_STAGE + nb_of(mt) * b_stage(mt, f32); }
+// codes of weights in tensor memory: where two stages fit beside two chunks' accumulators and scales (all but eight f32 rows)
+__host__ __device__ constexpr bool a_in_tmem(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 + NA * A_COLS <= 256; }
+__host__ __device__ constexpr int a_stage(int mt, bool f32) { return a_in_tmem(mt, f32) ? A_SCALES : A_STAGE; }
+__host__ __device__ constexpr int tmem_cols(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 + (a_in_tmem(mt, f32) ? NA * A_COLS : 0) <= 128 ? 128 : 256; }
+__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * a_stage(mt, f32) + nb_of(mt) * b_stage(mt, f32); }
 
 struct TcParams {
     const uint8_t* w0;
@@ -122,8 +125,10 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     constexpr int LV = digits_of(F32), ES = F32 ? 4 : 2;
     constexpr int N = ncol(MT, F32), NB = nb_of(MT), B_STAGE = b_stage(MT, F32), B_CODES = b_codes(MT, F32);
     using Acc = typename std::conditional<F32, double, float>::type;
-    constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = 2 * N, SFB_COL = 2 * N + 32;
-    static_assert(2 * N + 64 <= tmem_cols(MT, F32), "tensor memory columns");
+    constexpr bool TA = a_in_tmem(MT, F32);
+    constexpr int AS = a_stage(MT, F32);
+    constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = 2 * N, SFB_COL = 2 * N + 32, A_COL = 2 * N + 64;
+    static_assert(2 * N + 64 + (TA ? NA * A_COLS : 0) <= tmem_cols(MT, F32), "tensor memory columns");
     extern __shared__ uint8_t smem[];
     uint64_t* raw_full = (uint64_t*)smem;
     uint64_t* raw_empty = raw_full + MAX_RAW;
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint32_t* wf = (uint32_t*)(smem + WF_OFF);  // [NX][4]
     const uint32_t base = (smem_u32(smem) + HEADER + 1023u) & ~1023u;
     uint8_t* a0 = smem + (base - smem_u32(smem));
-    uint8_t* b0 = a0 + NA * A_STAGE;
+    uint8_t* b0 = a0 + NA * AS;
     uint8_t* r0 = b0 + NB * B_STAGE;
     const int R = p.raw;
     uint8_t* ex = r0 + (size_t)R * RAW_STAGE;
@@ -222,8 +227,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 break;
             }
             tc_after();
-            const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * A_STAGE)), db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
-            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_STAGE + A_CODES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
+            const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * AS)), db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
+            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * AS + (TA ? 0 : A_CODES))), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
             const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
             if (elect_lane()) {
 #pragma unroll
@@ -239,7 +244,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
                 for (int j = 0; j < 4; j++) cp_sf(tb + 4 * j, sb + 32 * j);
 #pragma unroll
-                for (int j = 0; j < 4; j++) umma_bs(td, da + 2 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
+                for (int j = 0; j < 4; j++) {
+                    if constexpr (TA)
+                        umma_bs_ta(td, tmem + A_COL + A_COLS * a + 8 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
+                    else
+                        umma_bs(td, da + 2 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
+                }
                 tc_commit<1>(&done[i % NDONE]);
                 mbar_arrive(&done[i % NDONE]);
             }
@@ -295,9 +305,6 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         // ------------------------------------------------------------ container blocks -> operand layout: a warp takes 32 rows, a lane the four
         // blocks of a row (144 bytes: no bank twice among eight lanes of neighbouring rows, nor in the swizzled lines)
         const int w = warp - 4;
-        // eight f32 rows: rows in order, the other order needs registers that there are not (4096 x 4096 10.95 us so, 11.1; gate / up of 17408 x 5120 51.4 / 52.2)
-        constexpr bool IN_ORDER = MT == 8 && F32;
-        const int row = IN_ORDER ? 32 * w + lane : operand_row(w, lane);
         int s = 0;
         uint32_t par = 0;
         for (int i = 0; i < total; i++) {
@@ -305,18 +312,18 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 cn_dev_fail(CN_DEV_WAIT_FULL);
                 break;
             }
-            const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + row * 9;
+            const uint4* src = (const uint4*)(r0 + (size_t)s * RAW_STAGE) + (w * 32 + lane) * 9;
             uint32_t v[36];
             const uint32_t odd = load_row(src, v);
             if (i >= NA && !mbar_wait(&done[(i - NA) % NDONE], ((i - NA) / NDONE) & 1)) {
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            store_row(a0 + (i & 1) * A_STAGE, row, v);
-            if (!IN_ORDER)
-                put_odd(wf + (i % NX) * 4, w, lane, odd);
-            else if (lane == 0)
-                wf[(i % NX) * 4 + w] = odd;
+            if constexpr (TA)
+                store_row_ta(tmem + A_COL + A_COLS * (i & 1), a0 + (i & 1) * AS, w, lane, v);
+            else
+                store_row(a0 + (i & 1) * AS, 32 * w + lane, v);
+            if (lane == 0) wf[(i % NX) * 4 + w] = odd;
             fence_async();
             __syncwarp();
             // (the stage is given back here and not behind the loads: an arrival can overtake loads whose values nothing has used yet)
