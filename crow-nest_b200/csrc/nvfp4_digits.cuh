@@ -16,15 +16,8 @@ __host__ __device__ constexpr uint32_t idesc_bs(int n) { return (1u << 7) | (1u 
 __device__ __forceinline__ void cp_sf(uint32_t taddr, uint64_t sdesc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
-__device__ __forceinline__ void umma_bs(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
-        : "memory");
-}
-// the same with A in tensor memory: a row's 64 values in eight columns of its lane
-__device__ __forceinline__ void umma_bs_ta(uint32_t tmem_d, uint32_t ta, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
+// A in tensor memory: a row's 64 values in eight columns of its lane
+__device__ __forceinline__ void umma_bs(uint32_t tmem_d, uint32_t ta, uint64_t db, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], [%1], %2, %3, [%4], [%5], p;\n\t}"
@@ -158,17 +151,8 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
 __device__ __forceinline__ double power_of_two(float f) { return __hiloint2double((int)((__float_as_uint(f) >> 3) + (896u << 20)), 0); }
 
 // ---------------------------------------------------------------- container blocks -> operand layout (a lane: the four blocks of a row)
-constexpr int A_CODES = 128 * 128, A_SCALES = 4 * 512, A_STAGE = A_CODES + A_SCALES;  // a chunk of 128 rows as operand A: 128-byte swizzled rows, then the scales of the four MMAs
-constexpr int A_COLS = 32;  // the codes of a chunk in tensor memory: columns
+constexpr int A_COLS = 32, A_SCALES = 4 * 512;  // a chunk of 128 rows as operand A: columns of tensor memory with its codes, bytes of the four MMAs' scales
 
-// The operand row that lane `lane` of weights warp w lays out: eight rows of each of the four groups of 32 whose scales lie side by side in 16 bytes. So the scale bytes of a warp fill
-// 128 bytes (those of 32 rows in a row would lie 16 bytes apart, four ways into the same banks). us, rows in order / so: one row of gate / up 17408 x 5120 19.1 / 18.7, four 24.0 / 23.0,
-// a step of 64 layers of 5120 x 17408 2785 / 2730, 64 tokens of 512 experts 178.6 / 176.4.
-__device__ __forceinline__ int operand_row(int w, int lane) { return 32 * (lane >> 3) + 8 * w + (lane & 7); }
-// What lanes of weights warp w have a row with a scale byte of 0xFF (`odd`), for the warps that sum these rows: a byte of the word of each.
-__device__ __forceinline__ void put_odd(uint32_t* words, int w, int lane, uint32_t odd) {
-    if (lane < 4) ((uint8_t*)words)[4 * lane + w] = (uint8_t)(odd >> (8 * lane));
-}
 // A row's 144 bytes at src into registers, scale bytes as the tensor core is to read them; which lanes' rows have one of 0xFF: that stands for 480, which it does not know, and is
 // nothing here (`whole_blocks` multiplies the block out).
 __device__ __forceinline__ uint32_t load_row(const uint4* src, uint32_t (&v)[36]) {
@@ -196,19 +180,10 @@ __device__ __forceinline__ void store_scales(uint8_t* dst, int row, const uint32
 #pragma unroll
     for (int b = 0; b < 4; b++) *(uint32_t*)(dst + b * 512 + (row & 31) * 16 + (row >> 5) * 4) = v[9 * b];
 }
-// row `row` of the operand stage at dst
-__device__ __forceinline__ void store_row(uint8_t* dst, int row, const uint32_t (&v)[36]) {
-    uint8_t* line = dst + row * 128;
-    const uint32_t sw = (uint32_t)(row & 7);
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-        *(uint4*)(line + (((2u * b) ^ sw) << 4)) = make_uint4(v[9 * b + 1], v[9 * b + 2], v[9 * b + 3], v[9 * b + 4]);
-        *(uint4*)(line + (((2u * b + 1u) ^ sw) << 4)) = make_uint4(v[9 * b + 5], v[9 * b + 6], v[9 * b + 7], v[9 * b + 8]);
-    }
-    store_scales(dst + A_CODES, row, v);
-}
-// ... and with the codes in tensor memory, where a warp reaches 32 lanes: row 32 w + lane
-__device__ __forceinline__ void store_row_ta(uint32_t taddr, uint8_t* scales, int w, int lane, const uint32_t (&v)[36]) {
+// Row 32 w + lane of the operand: its codes into A_COLS columns of tensor memory, of which a warp reaches 32 lanes, its scales into shared memory, from where the issuing thread has them copied.
+// Laid out in shared memory, as operand A by descriptor, the codes went through it twice more (stored, read by the MMA), and it was what a chunk used most: us, so / now, one row of gate / up of
+// 17408 x 5120 19.1 / 17.6, four rows 23.9 / 22.1; 4096 x 4096 4.6 / 4.2; 64 layers of 5120 x 17408 2811 / 2488.
+__device__ __forceinline__ void store_row(uint32_t taddr, uint8_t* scales, int w, int lane, const uint32_t (&v)[36]) {
     uint32_t codes[32];
 #pragma unroll
     for (int i = 0; i < 32; i++) codes[i] = v[9 * (i >> 3) + 1 + (i & 7)];

@@ -47,11 +47,10 @@ __host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_o
 __host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
 __host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
 __host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                                // chunks of digits
-// codes of weights in tensor memory: where two stages fit beside two chunks' accumulators and scales (all but eight f32 rows)
-__host__ __device__ constexpr bool a_in_tmem(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 + NA * A_COLS <= 256; }
-__host__ __device__ constexpr int a_stage(int mt, bool f32) { return a_in_tmem(mt, f32) ? A_SCALES : A_STAGE; }
-__host__ __device__ constexpr int tmem_cols(int mt, bool f32) { return 2 * ncol(mt, f32) + 64 + (a_in_tmem(mt, f32) ? NA * A_COLS : 0) <= 128 ? 128 : 256; }
-__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * a_stage(mt, f32) + nb_of(mt) * b_stage(mt, f32); }
+// accumulators, in half of an SM's tensor memory beside the codes of two chunks and the scales: those of two chunks where they fit (all but eight f32 rows)
+constexpr int TMEM = 256, TM_FIXED = NA * A_COLS + 64;
+__host__ __device__ constexpr int nacc(int mt, bool f32) { return 2 * ncol(mt, f32) + TM_FIXED <= TMEM ? 2 : 1; }
+__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * A_SCALES + nb_of(mt) * b_stage(mt, f32); }
 
 struct TcParams {
     const uint8_t* w0;
@@ -125,10 +124,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     constexpr int LV = digits_of(F32), ES = F32 ? 4 : 2;
     constexpr int N = ncol(MT, F32), NB = nb_of(MT), B_STAGE = b_stage(MT, F32), B_CODES = b_codes(MT, F32);
     using Acc = typename std::conditional<F32, double, float>::type;
-    constexpr bool TA = a_in_tmem(MT, F32);
-    constexpr int AS = a_stage(MT, F32);
-    constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = 2 * N, SFB_COL = 2 * N + 32, A_COL = 2 * N + 64;
-    static_assert(2 * N + 64 + (TA ? NA * A_COLS : 0) <= tmem_cols(MT, F32), "tensor memory columns");
+    constexpr int NACC = nacc(MT, F32);
+    constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = NACC * N, SFB_COL = NACC * N + 32, A_COL = NACC * N + 64;
+    static_assert(NACC * N + TM_FIXED <= TMEM, "tensor memory columns");
     extern __shared__ uint8_t smem[];
     uint64_t* raw_full = (uint64_t*)smem;
     uint64_t* raw_empty = raw_full + MAX_RAW;
@@ -142,7 +140,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
     uint32_t* wf = (uint32_t*)(smem + WF_OFF);  // [NX][4]
     const uint32_t base = (smem_u32(smem) + HEADER + 1023u) & ~1023u;
     uint8_t* a0 = smem + (base - smem_u32(smem));
-    uint8_t* b0 = a0 + NA * AS;
+    uint8_t* b0 = a0 + NA * A_SCALES;
     uint8_t* r0 = b0 + NB * B_STAGE;
     const int R = p.raw;
     uint8_t* ex = r0 + (size_t)R * RAW_STAGE;
@@ -184,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
         __syncwarp();
     } else if (warp == ISSUER) {
-        tc_alloc<1>(tmem_slot, tmem_cols(MT, F32));
+        tc_alloc<1>(tmem_slot, TMEM);
     }
     tc_before();
     __syncthreads();
@@ -227,9 +225,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 break;
             }
             tc_after();
-            const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * AS)), db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
-            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * AS + (TA ? 0 : A_CODES))), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
-            const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
+            const uint64_t db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
+            const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_SCALES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
+            const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * (i % NACC);
             if (elect_lane()) {
 #pragma unroll
                 for (int j = 0; j < 4; j++) cp_sf(ta + 4 * j, sa + 32 * j);
@@ -244,12 +242,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
 #pragma unroll
                 for (int j = 0; j < 4; j++) cp_sf(tb + 4 * j, sb + 32 * j);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if constexpr (TA)
-                        umma_bs_ta(td, tmem + A_COL + A_COLS * a + 8 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
-                    else
-                        umma_bs(td, da + 2 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
-                }
+                for (int j = 0; j < 4; j++) umma_bs(td, tmem + A_COL + A_COLS * a + 8 * j, db + 2 * j, IDESC, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
                 tc_commit<1>(&done[i % NDONE]);
                 mbar_arrive(&done[i % NDONE]);
             }
@@ -303,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
     } else if (warp >= EPI_WARPS) {
         // ------------------------------------------------------------ container blocks -> operand layout: a warp takes 32 rows, a lane the four
-        // blocks of a row (144 bytes: no bank twice among eight lanes of neighbouring rows, nor in the swizzled lines)
+        // blocks of a row (144 bytes: no bank twice among eight lanes)
         const int w = warp - 4;
         int s = 0;
         uint32_t par = 0;
@@ -319,10 +312,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            if constexpr (TA)
-                store_row_ta(tmem + A_COL + A_COLS * (i & 1), a0 + (i & 1) * AS, w, lane, v);
-            else
-                store_row(a0 + (i & 1) * AS, 32 * w + lane, v);
+            store_row(tmem + A_COL + A_COLS * (i & 1), a0 + (i & 1) * A_SCALES, w, lane, v);
             if (lane == 0) wf[(i % NX) * 4 + w] = odd;
             fence_async();
             __syncwarp();
@@ -333,7 +323,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         }
     } else {
         // ------------------------------------------------------------ sums and output
-        if (lane < 2) mbar_arrive(&xbar[lane]);  // the accumulators of the first two chunks
+        if (lane < NACC) mbar_arrive(&xbar[lane]);  // the accumulators of the first two chunks
         pdl_wait();
         const float gs0 = *p.gs0, gs1 = gu ? *p.gs1 : 0.0f, gs = gu && warp >= 2 ? gs1 : gs0;
         const unsigned int epoch = p.yl_world > 0 ? *(volatile const unsigned int*)p.yl_epoch : 0u;
@@ -349,7 +339,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 break;
             }
             tc_after();
-            const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i & 1));
+            const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i % NACC));
             const uint32_t odd = wf[(i % NX) * 4 + warp];
             uint32_t slow = odd;
             constexpr int G = F32 ? (MT < 2 ? MT : 2) : (MT < 4 ? MT : 4);  // rows at a time
@@ -362,7 +352,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
                 if (m0 + G == MT) {
                     tc_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&xbar[(i + 2) % NX]);
+                    if (lane == 0) mbar_arrive(&xbar[(i + NACC) % NX]);
                 }
 #pragma unroll
                 for (int m = 0; m < G; m++) {
@@ -505,7 +495,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
         asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     }
     __syncthreads();
-    if (warp == ISSUER) tc_dealloc<1>(tmem, tmem_cols(MT, F32));
+    if (warp == ISSUER) tc_dealloc<1>(tmem, TMEM);
 }
 
 // ---------------------------------------------------------------- launch
@@ -610,13 +600,10 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         map1 = map0;
     else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
         return rc;
-    // A CTA asks for no smaller a share of shared memory than of tensor memory: as many of these kernels (or of nvfp4_rows_tc.cu's) as fit an SM find tensor memory there. The pair
+    // A CTA asks for half of an SM's shared memory, as of its tensor memory: as many of these kernels (or of nvfp4_rows_tc.cu's) as fit an SM find tensor memory there. The pair
     // GEMM, which takes all of it, stands apart by its registers: 640 threads of 72 leave no room for 448 of 72.
-    int smem = front + p.raw * RAW_STAGE;
-    const int floor_bytes = tmem_cols(mt, f32) == 256 ? SM_SHARE : (227 * 1024) / 4;
-    if (smem < floor_bytes) smem = floor_bytes;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(clusters * c)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = (size_t)smem, cfg.stream = stream;
+    cfg.gridDim = dim3((unsigned)(clusters * c)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SM_SHARE, cfg.stream = stream;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;

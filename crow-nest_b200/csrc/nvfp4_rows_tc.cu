@@ -6,8 +6,7 @@
 // Persistent CTAs, two per SM, walk units of (group, 128-row tile; 64 gate and 64 up rows). The matrices come from device tables, so there is no tensor map:
 // a scout warp looks up 32 units at a time (positions, combos, expert, addresses) and hands them to the other warps through a ring, and the warps that lay
 // the weights out for the tensor core bring them in themselves, by 16-byte asynchronous copies, past the ends of units. Warps: 0-3 add up and store,
-// 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form an adding warp's rows are 16 of gate and the same 16 of up; a weights warp's eight rows of each
-// adding warp's, so two of them bring gate and two up.
+// 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form a warp's rows are 16 of gate and the same 16 of up.
 //
 // What bounds it: the way of the weights through a warp (gate / up of 64 tokens, 512 experts of 2048 x 512, top 10: 2150 cycles a chunk of 18 KB and CTA, 470 of
 // them loads, 500 stores and their fence, 580 the copies of a later chunk), 4.1 TB/s; us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16
@@ -23,7 +22,7 @@ namespace {
 constexpr int RG = 8;        // most rows of a group
 constexpr int CH = 256;      // values of k in a chunk
 constexpr int PIECE = 32 * 144;  // container bytes of a warp's 32 rows and a chunk
-__host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 2 : 4; }  // chunks in flight, as many as fit
+__host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 3 : 4; }  // chunks in flight, as many as fit
 constexpr int NA = 2, NB = 2, NX = 16, NDONE = 4, NU = 8;  // operand stages, chunks of digits, chunk factors, finished chunks, units in the ring
 constexpr int NBAR = NX + NDONE + 2 * NU;
 constexpr int SCOUT = 12, ISSUER = 13, THREADS = 448;
@@ -31,10 +30,10 @@ constexpr int FS_OFF = 512, WF_OFF = 1536, UNIT_OFF = 1792, HEADER = 2560;
 // columns of the widest MMA, whose N is a multiple of 16: the accumulators lie this far apart in tensor memory (eight f32 rows are 88 columns, and 96 are written)
 __host__ __device__ constexpr int ncol(bool f32) { return (RG * digits_of(f32) + 15) / 16 * 16; }
 __host__ __device__ constexpr int b_stage(bool f32) { return ncol(f32) * 128 + 4 * 512; }
-// codes of weights in tensor memory: where two stages fit beside two chunks' accumulators and scales
-__host__ __device__ constexpr bool a_in_tmem(bool f32) { return 2 * ncol(f32) + 64 + NA * A_COLS <= 256; }
-__host__ __device__ constexpr int a_stage(bool f32) { return a_in_tmem(f32) ? A_SCALES : A_STAGE; }
-__host__ __device__ constexpr int smem_of(bool f32) { return NA * a_stage(f32) + NB * b_stage(f32) + 4 * depth_of(f32) * PIECE + HEADER; }
+// accumulators, in half of an SM's tensor memory beside the codes of two chunks and the scales: those of two chunks where they fit
+constexpr int TMEM = 256, TM_FIXED = NA * A_COLS + 64;
+__host__ __device__ constexpr int nacc(bool f32) { return 2 * ncol(f32) + TM_FIXED <= TMEM ? 2 : 1; }
+__host__ __device__ constexpr int smem_of(bool f32) { return NA * A_SCALES + NB * b_stage(f32) + 4 * depth_of(f32) * PIECE + HEADER; }
 constexpr int SM_SHARE = (227 * 1024) / 2 - 1024;
 static_assert(smem_of(true) <= SM_SHARE && smem_of(false) <= SM_SHARE, "shared memory");
 
@@ -48,13 +47,12 @@ static_assert(UNIT_OFF + NU * sizeof(Unit) <= HEADER && NBAR * 8 + 8 <= FS_OFF, 
 template <bool F32>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCall c) {
     constexpr int D = depth_of(F32), LV = digits_of(F32), ES = F32 ? 4 : 2, N = ncol(F32), B_CODES = N * 128, B_STAGE = b_stage(F32);
-    constexpr bool TA = a_in_tmem(F32);
-    constexpr int AS = a_stage(F32);
-    constexpr uint32_t SFA_COL = 2 * N, SFB_COL = 2 * N + 32, A_COL = 2 * N + 64, TMEM = 256;
-    static_assert(2 * N + 64 + (TA ? NA * A_COLS : 0) <= (int)TMEM && N % 16 == 0, "tensor memory columns");
+    constexpr int NACC = nacc(F32);
+    constexpr uint32_t SFA_COL = NACC * N, SFB_COL = NACC * N + 32, A_COL = NACC * N + 64;
+    static_assert(NACC * N + TM_FIXED <= TMEM && N % 16 == 0, "tensor memory columns");
     using Acc = typename std::conditional<F32, double, float>::type;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *a0 = smem, *b0 = a0 + NA * AS, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;
+    uint8_t *a0 = smem, *b0 = a0 + NA * A_SCALES, *r0 = b0 + NB * B_STAGE, *head = r0 + (size_t)4 * D * PIECE;
     uint64_t* ready = (uint64_t*)head;        // [NX] weights and digits of a chunk, and its accumulators (those of two chunks before) have been read
     uint64_t* done = ready + NX;              // [NDONE] MMAs of a chunk; the issuer arrives too, and hands on what weight and activation warps wrote beside the operands
     uint64_t* unit_full = done + NDONE;       // [NU]
@@ -160,9 +158,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                     break;
                 }
                 tc_after();
-                const uint64_t da = tc_desc_sw128(a_u + (uint32_t)(a * AS)), db = tc_desc_sw128(b_u + (uint32_t)(a * B_STAGE));
-                const uint64_t sa = desc_sf(a_u + (uint32_t)(a * AS + (TA ? 0 : A_CODES))), sb = desc_sf(b_u + (uint32_t)(a * B_STAGE + B_CODES));
-                const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * a;
+                const uint64_t db = tc_desc_sw128(b_u + (uint32_t)(a * B_STAGE));
+                const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_SCALES)), sb = desc_sf(b_u + (uint32_t)(a * B_STAGE + B_CODES));
+                const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * (i % NACC);
                 if (elect_lane()) {
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
@@ -170,12 +168,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                         cp_sf(tb + 4 * j, sb + 32 * j);
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if constexpr (TA)
-                            umma_bs_ta(td, tmem + A_COL + A_COLS * a + 8 * j, db + 2 * j, idesc, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
-                        else
-                            umma_bs(td, da + 2 * j, db + 2 * j, idesc, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
-                    }
+                    for (int j = 0; j < 4; j++) umma_bs(td, tmem + A_COL + A_COLS * a + 8 * j, db + 2 * j, idesc, ta + 4 * j, tb + 4 * j, j > 0 ? 1u : 0u);
                     tc_commit<1>(&done[i % NDONE]);
                     mbar_arrive(&done[i % NDONE]);
                 }
@@ -252,13 +245,12 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         const int w = warp - 4;
         const uint32_t ring = smem_u32(r0) + (uint32_t)(w * D * PIECE);
         const uint64_t pol = l2_policy_evict_first();
-        // sixteen-byte pieces, nine to a row and chunk, side by side in the stage, which has the rows by lanes
-        auto tile_row = [&](int row) { return TA ? (gu ? row & 15 : row) : (row >> 3) * (gu ? 16 : 32) + (row & 7); };  // from the warp's first on
+        // sixteen-byte pieces, nine to a row and chunk, side by side in the stage; in the gate / up form rows 16-31 of a warp are the up rows of its gate rows
         uint32_t off[9];
 #pragma unroll
         for (int j = 0; j < 9; j++) {
             const int id = lane + 32 * j, row = id / 9;
-            off[j] = (uint32_t)tile_row(row) * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u;
+            off[j] = (uint32_t)(gu ? row & 15 : row) * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u;
         }
         int iq = 0, ic = 0, is = 0, have = 0, asked = 0;  // what is asked for next: unit, chunk, stage; rows there are; chunks so far
         const uint8_t *from = nullptr, *from1 = nullptr;
@@ -271,9 +263,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 } else {
                     const Unit& u = units[iq % NU];
                     more = u.nrows >= 0;
-                    const int first = u.tile * per_tile + (TA ? w * (gu ? 16 : 32) : 8 * (gu ? w & 1 : w));
-                    from = (const uint8_t*)(!TA && gu && w >= 2 ? u.w1 : u.w0) + (size_t)first * row_bytes;
-                    if (TA && gu) from1 = (const uint8_t*)u.w1 + (size_t)first * row_bytes;
+                    const int first = u.tile * per_tile + w * (gu ? 16 : 32);
+                    from = (const uint8_t*)u.w0 + (size_t)first * row_bytes, from1 = (const uint8_t*)u.w1 + (size_t)first * row_bytes;
                     have = c.rows - first;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&unit_empty[iq % NU]);  // (nothing else of the unit is wanted here)
@@ -281,18 +272,18 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             }
             if (more) {
                 const uint32_t dst = ring + (uint32_t)(is * PIECE + lane * 16);
-                // (codes in tensor memory, gate / up: piece 32 j + lane is of an up row from 144 on)
-                const uint8_t *chunk = from + (uint32_t)(ic * 144), *hi = TA && gu ? from1 + (uint32_t)(ic * 144) : chunk, *mid = lane < 16 ? chunk : hi;
+                // piece 32 j + lane: of row 16 and on from piece 144
+                const uint8_t *lo = from + (uint32_t)(ic * 144), *hi = gu ? from1 + (uint32_t)(ic * 144) : lo, *mid = lane < 16 ? lo : hi;
                 auto copy = [&](int j, uint32_t at) {
-                    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"((!TA || j < 4 ? chunk : j == 4 ? mid : hi) + at), "l"(pol) : "memory");
+                    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst + 512u * j), "l"((j < 4 ? lo : j == 4 ? mid : hi) + at), "l"(pol) : "memory");
                 };
-                if (have > (TA && gu ? 15 : tile_row(31))) {
+                if (have >= (gu ? 16 : 32)) {
 #pragma unroll
                     for (int j = 0; j < 9; j++) copy(j, off[j]);
                 } else {  // the matrix ends inside these rows
 #pragma unroll 1
                     for (int j = 0; j < 9; j++) {
-                        const int id = lane + 32 * j, row = id / 9, r = tile_row(row);
+                        const int id = lane + 32 * j, row = id / 9, r = gu ? row & 15 : row;
                         if (r < have) copy(j, (uint32_t)r * (uint32_t)row_bytes + (uint32_t)(id - 9 * row) * 16u);
                     }
                 }
@@ -316,13 +307,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 cn_dev_fail(CN_DEV_WAIT_EMPTY);
                 break;
             }
-            if constexpr (TA) {
-                store_row_ta(tmem + A_COL + A_COLS * (i & 1), a0 + (i & 1) * AS, w, lane, v);
-                if (lane == 0) wf[(i % NX) * 4 + w] = odd;
-            } else {
-                store_row(a0 + (i & 1) * AS, operand_row(w, lane), v);
-                put_odd(wf + (i % NX) * 4, w, lane, odd);
-            }
+            store_row(tmem + A_COL + A_COLS * (i & 1), a0 + (i & 1) * A_SCALES, w, lane, v);
+            if (lane == 0) wf[(i % NX) * 4 + w] = odd;
             fence_async();
             __syncwarp();  // every lane has read the stage
             if (lane == 0) mbar_arrive(&ready[i % NX]);
@@ -332,7 +318,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ------------------------------------------------------------ sums and output: a thread is a row of the tile
-        if (lane < 2) mbar_arrive(&ready[lane]);  // the accumulators of the first two chunks
+        if (lane < NACC) mbar_arrive(&ready[lane]);  // the accumulators of the first two chunks
         const float gs0 = __ldg(c.gs0), gs1 = gu ? __ldg(c.gs1) : 0.0f, gs = gu && lane >= 16 ? gs1 : gs0;
         bool ok = true;
         for (int q = 0, i = 0; ok; q++) {
@@ -353,7 +339,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                     break;
                 }
                 tc_after();
-                const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i & 1));
+                const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i % NACC));
                 const uint32_t odd = wf[(i % NX) * 4 + warp];
                 uint32_t slow = odd;
 #pragma unroll
@@ -378,7 +364,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 }
                 tc_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&ready[(i + 2) % NX]);
+                if (lane == 0) mbar_arrive(&ready[(i + NACC) % NX]);
                 if (slow && row < c.rows) {
                     const uint8_t* wr = (const uint8_t*)(gu && lane >= 16 ? u.w1 : u.w0) + ((size_t)row * nk + ch) * 144;
 #pragma unroll 1
