@@ -12,6 +12,7 @@
 // skips the combo (the expert lives on another rank).
 #include "common.cuh"
 #include "moe_step.cuh"
+#include "nvfp4_digits.cuh"
 #include "nvfp4_gemv.cuh"
 
 namespace {
@@ -83,7 +84,7 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 constexpr int LONG_RUN = 64;
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,
                                                          int32_t* __restrict__ order, int* __restrict__ ga, int* __restrict__ gb,
-                                                         int* __restrict__ gbrows, int* __restrict__ counts, int gmax, int listed) {
+                                                         int* __restrict__ gbrows, int* __restrict__ counts, int gmax, int listed, const DigitsCall dc) {
     extern __shared__ int sm[];  // [E + 1] counts, [E + 1] starts, [E + 1] running, [n] bins, [n] the experts' combos (listed)
     int* cnt = sm;
     int* start = sm + (E + 1);
@@ -96,6 +97,16 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     // 207.1 -> 197.5 us a step, MUL1 with 16 tokens 266.4 -> 264.3.
     pdl_launch_dependents();
     pdl_wait();
+    if (blockIdx.x > 0) {  // not the grouping: a warp a chunk of activations
+        const int i = ((int)blockIdx.x - 1) * 32 + wid;
+        if (i < dc.chunks) {
+            if (dc.f32)
+                put_record<true>((const float*)dc.x + (size_t)i * 256, lane, dc.out + (size_t)i * digit_record(true));
+            else
+                put_record<false>((const __nv_bfloat16*)dc.x + (size_t)i * 256, lane, dc.out + (size_t)i * digit_record(false));
+        }
+        return;
+    }
     for (int i = tid; i <= E; i += blockDim.x) cnt[i] = 0;
     __syncthreads();
     for (int c = tid; c < n; c += blockDim.x) {
@@ -218,6 +229,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ eo, const float* __
         ((float*)y)[(size_t)t * H + c] = v;
 }
 
+// Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
+constexpr int GROUP_COMBOS = 48;
+// Bytes of a plan's store of digits at most.
+constexpr size_t DIGITS_MOST = (size_t)64 << 20;
+
 struct MoePlan {
     int hidden, inter, experts, topk, max_tokens, device;
     float* h;        // [max_tokens * topk][inter]
@@ -226,6 +242,8 @@ struct MoePlan {
     float* ys;       // [max_tokens][hidden]
     int32_t* order;  // [max_tokens * topk]
     int* groups;     // [3 * max_tokens * topk + 8]: the group lists of moe_group_kernel and their two counts
+    uint8_t* xd;     // records of the digits of x; null where there is no room for them
+    size_t xd_bytes;
     int shared_inter;
     // the shared expert does not depend on the routed experts until the combine: it is enqueued on a side stream
     // between two events (fork after the caller's earlier work, join before the combine), also under stream capture
@@ -238,14 +256,14 @@ struct MoePlan {
 
 // the grouping step for other operators of the library (declared in nvfp4_gemv.cuh): lists of `combos` ints each, counts of 2
 int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int combos, int experts, int32_t* order, int* ga, int* gb, int* gbrows,
-                        int* counts, int gmax, cudaStream_t stream) {
+                        int* counts, int gmax, cudaStream_t stream, const DigitsCall& digits) {
     if (gmax != 4 && gmax != 8) CN_FAIL(CN_ERR_SHAPE, "grouping: groups of %d rows (4 or 8)", gmax);
     const size_t smem = (size_t)(3 * (experts + 1) + combos) * sizeof(int);
     if (smem > 160 * 1024) CN_FAIL(CN_ERR_LIMIT, "grouping %d combos over %d experts needs %zu B of shared memory", combos, experts, smem);
     CN_ALLOW_SMEM(moe_group_kernel, 160 * 1024);
     const size_t listed = smem + (size_t)combos * sizeof(int);
     const bool fits = listed <= 160 * 1024;
-    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1), dim3(1024), fits ? listed : smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax, (int)fits));
+    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1u + (unsigned)((digits.chunks + 31) / 32)), dim3(1024), fits ? listed : smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax, (int)fits, digits));
     return CN_OK;
 }
 
@@ -296,6 +314,15 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
         cn_moe_nvfp4_plan_destroy(p);
         CN_FAIL(CN_ERR_CUDA, "cn_moe_nvfp4_plan_create: %s", cudaGetErrorString(e));
     }
+    // Records of the digits of x for the grouped step, bounded; without them (and for more rows than they hold) the digits are made where they are used, which has the same bits.
+    if (combos >= GROUP_COMBOS) {
+        p->xd_bytes = (size_t)max_tokens * (hidden / 256) * digit_record(true);
+        if (p->xd_bytes > DIGITS_MOST) p->xd_bytes = DIGITS_MOST;
+        if (cudaMalloc(&p->xd, p->xd_bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            p->xd = nullptr, p->xd_bytes = 0;
+        }
+    }
     *plan_out = p;
     return CN_OK;
 }
@@ -303,7 +330,7 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
 extern "C" int cn_moe_nvfp4_plan_destroy(void* plan) {
     MoePlan* p = (MoePlan*)plan;
     if (!p) return CN_OK;
-    cudaFree(p->h), cudaFree(p->eo), cudaFree(p->hs), cudaFree(p->ys), cudaFree(p->order), cudaFree(p->groups);
+    cudaFree(p->h), cudaFree(p->eo), cudaFree(p->hs), cudaFree(p->ys), cudaFree(p->order), cudaFree(p->groups), cudaFree(p->xd);
     if (p->side) cudaStreamDestroy(p->side);
     if (p->fork) cudaEventDestroy(p->fork);
     if (p->join) cudaEventDestroy(p->join);
@@ -359,8 +386,6 @@ int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, co
     return rc;
 }
 
-// Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
-constexpr int GROUP_COMBOS = 48;
 // ... and from which the ungrouped down projection runs on the tensor cores (measured: see routed_experts).
 constexpr int ROWS_COMBOS = 16;
 // Units of work (16 result rows of a token x eight 64-value blocks of an expert) up to which a step of that many combos runs in two launches
@@ -403,7 +428,17 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
         d.ids = ids, d.order = p->order, d.tab0 = table_dn, d.gs0 = gs_dn, d.x = p->h, d.x_div = 1, d.x_f32 = 1, d.y = eo, d.yptrs = eo_ptrs, d.ldy = p->hidden;
         d.rows = p->hidden, d.k = p->inter, d.max_groups = u.max_groups;
         d.count1 = counts, d.pos1 = ga, d.count2 = counts + 1, d.pos2 = gb, d.rows2 = gbrows;
-        if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, counts, 8, stream)) return rc;
+        const bool f32 = dtype == CN_F32;
+        const long long x_chunks = (long long)((combos + x_div - 1) / x_div) * (p->hidden / 256);
+        // The digits of x are made once, beside the grouping, and not by every tile of gate / up: us per step, in each tile / so: 64 tokens 169 / 167, 128 tokens 247 / 234, 64 tokens of f32
+        // 187 / 179, 288 experts of 4096 x 2048, 32 tokens 369 / 339, 10 tokens 180 / 176, 64 experts of 1024 x 1280, 108 tokens 140 / 129; 16 and 24 tokens of 512 experts the same. Those of h,
+        // a launch of their own in front of the down projection: 64 tokens 167 / 175, 108 tokens 129 / 122, 128 tokens 234 / 232.
+        DigitsCall dx = {};
+        if (!((uintptr_t)x & 15) && x_chunks * digit_record(f32) <= (long long)p->xd_bytes) {
+            dx.x = x, dx.chunks = (int)x_chunks, dx.f32 = f32, dx.out = p->xd;
+            u.digits = p->xd;
+        }
+        if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, counts, 8, stream, dx)) return rc;
         if (int rc = cn_rows_launch(u, stream, "cn_moe_nvfp4 (gate/up, grouped)")) return rc;
         return cn_rows_launch(d, stream, "cn_moe_nvfp4 (down, grouped)");
     }

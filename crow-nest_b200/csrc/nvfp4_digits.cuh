@@ -56,7 +56,7 @@ __device__ __forceinline__ void tc_ld_digits(uint32_t taddr, uint32_t* v) {
 // fs[row]: 2^(Emax - 8) and the blocks without digits (block b: bit 2 b).
 constexpr float TO_INT = 12582912.0f;  // 3 x 2^22: a sum with it has the nearest whole number in its mantissa (ties to even)
 
-template <bool F32>
+template <bool F32, bool RECORD = false>
 __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* bs, uint8_t* sf, int row, float2* fs) {
     constexpr int LV = digits_of(F32);
     constexpr uint32_t LEAST = 28u, EXP = F32 ? 23u : 7u;  // least biased E: all scales are numbers
@@ -138,14 +138,58 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
     uint32_t sw = (under <= 14u ? (15u - under) << 3 : 32u >> (under - 12u)) << (8 * ((lane >> 1) & 3));
     sw |= __shfl_xor_sync(0xffffffffu, sw, 2);
     sw |= __shfl_xor_sync(0xffffffffu, sw, 4);
-    int n = row * LV + (lane & 7);
-    *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
-    if ((lane & 7) < LV - 8) {
-        n += 8;
+    if constexpr (RECORD) {
+        if ((lane & 7) == 0) ((uint32_t*)sf)[lane >> 3] = sw;
+    } else {
+        int n = row * LV + (lane & 7);
         *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
+        if ((lane & 7) < LV - 8) {
+            n += 8;
+            *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = sw;
+        }
     }
     if (lane == 0) *fs = make_float2(__uint_as_float((emax - 8u) << 23), __uint_as_float(blocks));
 }
+
+// The same kept in global memory, for matrices of many tiles, which would each make the digits of their rows: the lines as of row 0, four words of scales, factor and blocks without digits.
+__host__ __device__ constexpr int digit_record(bool f32) { return digits_of(f32) * 128 + 32; }
+template <bool F32>
+__device__ __forceinline__ void put_record(const void* x, int lane, uint8_t* rec) {  // x: the chunk's 256 values
+    constexpr int XR = F32 ? 2 : 1;
+    uint4 raw[XR];
+#pragma unroll
+    for (int j = 0; j < XR; j++) raw[j] = __ldcg((const uint4*)x + lane * XR + j);
+    to_digits<F32, true>(raw, lane, rec, rec + digits_of(F32) * 128, 0, (float2*)(rec + digits_of(F32) * 128 + 16));
+}
+template <bool F32>
+struct DigitRecord {  // a lane's part of one
+    static constexpr int PIECES = digits_of(F32) * 8, PER = (PIECES + 31) / 32;
+    uint4 code[PER];
+    uint32_t scales;
+    float2 f;
+    __device__ __forceinline__ void load(const uint8_t* rec, int lane) {
+#pragma unroll
+        for (int p = 0; p < PER; p++)
+            if (lane + 32 * p < PIECES) code[p] = __ldcg((const uint4*)rec + lane + 32 * p);
+        scales = __ldcg((const uint32_t*)(rec + PIECES * 16) + (lane >> 3));
+        f = __ldcg((const float2*)(rec + PIECES * 16 + 16));
+    }
+    __device__ __forceinline__ void store(int lane, uint8_t* bs, uint8_t* sf, int row, float2* fs) const {
+        constexpr int LV = digits_of(F32);
+#pragma unroll
+        for (int p = 0; p < PER; p++) {
+            const int id = lane + 32 * p, j = id >> 3, n = row * LV + j;
+            if (id < PIECES) *(uint4*)(bs + n * 128 + ((((id & 7) ^ j ^ n) & 7) << 4)) = code[p];
+        }
+        int n = row * LV + (lane & 7);
+        *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = scales;
+        if ((lane & 7) < LV - 8) {
+            n += 8;
+            *(uint32_t*)(sf + (lane >> 3) * 512 + (n & 31) * 16 + (n >> 5) * 4) = scales;
+        }
+        if (lane == 0) *fs = f;
+    }
+};
 
 // a chunk's factor in 64 bits (a normal power of two)
 __device__ __forceinline__ double power_of_two(float f) { return __hiloint2double((int)((__float_as_uint(f) >> 3) + (896u << 20)), 0); }

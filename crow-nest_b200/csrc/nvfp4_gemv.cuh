@@ -46,9 +46,14 @@ unsigned long long* cn_trace_slot();  // diagnostic build: where the next launch
 
 // Sort combos by expert and cut every expert's run into groups (moe.cu): order [combos]; ga = positions (in order) of the
 // one-row groups, counts[0] of them; gb / gbrows = positions and row counts (2..gmax, gmax 4 or 8) of the larger groups,
-// counts[1]. Combos without a resident expert are in no group.
+// counts[1]. Combos without a resident expert are in no group. Beside it, where given, chunks of activations into records of digits (nvfp4_digits.cuh).
+struct DigitsCall {
+    const void* x;  // rows one after another
+    int chunks, f32;
+    uint8_t* out;
+};
 int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int combos, int experts, int32_t* order, int* ga, int* gb, int* gbrows,
-                        int* counts, int gmax, cudaStream_t stream);
+                        int* counts, int gmax, cudaStream_t stream, const DigitsCall& digits = {});
 
 // Kernel-side parameters shared by the CUDA-core and the tensor-core GEMV kernels.
 struct GemvParams {
@@ -125,6 +130,7 @@ struct RowsCall {
     const float* gs0;
     const float* gs1;
     const void* x;  // activation row of combo c: row c / x_div, bf16 (or f32 when x_f32)
+    const uint8_t* digits;  // records of its chunks (nvfp4_digits.cuh), or null: made where they are used
     int x_div, x_f32;
     float* y;  // f32 row of combo c at y + c * ldy, or at yptrs[c]
     const unsigned long long* yptrs;

@@ -44,7 +44,16 @@ struct Unit {
 };
 static_assert(UNIT_OFF + NU * sizeof(Unit) <= HEADER && NBAR * 8 + 8 <= FS_OFF, "header");
 
-template <bool F32>
+template <int XR>
+struct Values {  // a lane's eight values of a chunk
+    uint4 v[XR];
+    __device__ __forceinline__ void load(const void* x, int lane) {
+#pragma unroll
+        for (int j = 0; j < XR; j++) v[j] = __ldcg((const uint4*)x + lane * XR + j);
+    }
+};
+
+template <bool F32, bool KEPT>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCall c) {
     constexpr int D = depth_of(F32), LV = digits_of(F32), ES = F32 ? 4 : 2, N = ncol(F32), B_CODES = N * 128, B_STAGE = b_stage(F32);
     constexpr int NACC = nacc(F32);
@@ -181,7 +190,8 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         constexpr int XR = F32 ? 2 : 1;
         const int w = warp - 8;
         int q = 0, ch = 0, nrows = 0;
-        uint4 nx[2][XR];
+        using Held = typename std::conditional<KEPT, DigitRecord<F32>, Values<XR>>::type;
+        Held nx[2];
         bool ok = true;
         auto unit = [&](int n) -> int {  // rows of unit n
             if (!mbar_wait(&unit_full[n % NU], (uint32_t)(n / NU) & 1u)) {
@@ -196,20 +206,17 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             for (int t = 0; t < 2; t++) {
                 const int row = ((w - i) & 3) + 4 * t;
                 if (row < rows) {
-                    const uint4* x = (const uint4*)((const char*)c.x + ((size_t)units[n % NU].xrow[row] * c.k + (size_t)chunk * CH) * ES) + lane * XR;
-#pragma unroll
-                    for (int j = 0; j < XR; j++) nx[t][j] = __ldcg(x + j);
+                    if constexpr (KEPT)
+                        nx[t].load(c.digits + ((size_t)units[n % NU].xrow[row] * nk + chunk) * digit_record(F32), lane);
+                    else
+                        nx[t].load((const char*)c.x + ((size_t)units[n % NU].xrow[row] * c.k + (size_t)chunk * CH) * ES, lane);
                 }
             }
         };
         nrows = unit(0);
         if (nrows >= 0) fetch(0, nrows, 0, 0);
         for (int i = 0; nrows >= 0; i++) {
-            uint4 now[2][XR];
-#pragma unroll
-            for (int t = 0; t < 2; t++)
-#pragma unroll
-                for (int j = 0; j < XR; j++) now[t][j] = nx[t][j];
+            Held now[2] = {nx[0], nx[1]};
             const int at = q;
             int next_rows = nrows;
             if (++ch == nk) ch = 0, q++, next_rows = unit(q);
@@ -227,9 +234,11 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
                 // of 512 experts 195.6 / 190.9, 128 tokens 291 / 272, of 64 experts (groups of eight) 148 / 134, f32 rows 171 / 151
 #pragma unroll 1
                 for (int row = (w - i) & 3; row < nrows; row += 4) {
-                    to_digits<F32>(now[0], lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
-#pragma unroll
-                    for (int j = 0; j < XR; j++) now[0][j] = now[1][j];
+                    if constexpr (KEPT)
+                        now[0].store(lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
+                    else
+                        to_digits<F32>(now[0].v, lane, bs, bs + B_CODES, row, &fs[(i % NX) * 8 + row]);
+                    now[0] = now[1];
                 }
                 fence_async();
                 __syncwarp();
@@ -399,6 +408,13 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
     if (warp == ISSUER) tc_dealloc<1>(tmem, TMEM);
 }
 
+template <bool F32, bool KEPT>
+int launch(const RowsCall& p, dim3 grid, cudaStream_t stream) {
+    CN_ALLOW_SMEM((nvfp4_rows_tc_kernel<F32, KEPT>), SM_SHARE);
+    CN_CUDA(cn_launch_pdl(nvfp4_rows_tc_kernel<F32, KEPT>, grid, dim3(THREADS), SM_SHARE, stream, p));
+    return CN_OK;
+}
+
 }  // namespace
 
 int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
@@ -411,12 +427,5 @@ int cn_rows_launch(const RowsCall& a, cudaStream_t stream, const char* who) {
     const long long units = (long long)a.max_groups * ((a.rows + (gu ? 63 : 127)) / (gu ? 64 : 128));
     const dim3 grid((unsigned)(units < 2 * 148 ? units : 2 * 148));
     // (all of an SM's half, so that two CTAs and no more share its tensor memory)
-    if (f32) {
-        CN_ALLOW_SMEM(nvfp4_rows_tc_kernel<true>, SM_SHARE);
-        CN_CUDA(cn_launch_pdl(nvfp4_rows_tc_kernel<true>, grid, dim3(THREADS), SM_SHARE, stream, p));
-    } else {
-        CN_ALLOW_SMEM(nvfp4_rows_tc_kernel<false>, SM_SHARE);
-        CN_CUDA(cn_launch_pdl(nvfp4_rows_tc_kernel<false>, grid, dim3(THREADS), SM_SHARE, stream, p));
-    }
-    return CN_OK;
+    return f32 ? (p.digits ? launch<true, true>(p, grid, stream) : launch<true, false>(p, grid, stream)) : p.digits ? launch<false, true>(p, grid, stream) : launch<false, false>(p, grid, stream);
 }

@@ -237,6 +237,29 @@ def test_odd_scales_and_rows_that_are_not_finite(hidden, inter, tokens, experts,
     assert device_status() == 0
 
 
+@pytest.mark.parametrize("hidden,inter,rows", [(256, 256, 49), (768, 512, 130), (2048, 256, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_digits_made_once_are_those_made_in_each_tile(hidden, inter, rows, dtype):
+    """A plan holds the digits of as many rows as it has tokens; a step over more (one for each pick) makes them in each tile. Same bits, with values that have no digits among them."""
+    rng = np.random.default_rng(rows)
+
+    def matrix(n, k):
+        return torch.from_numpy(synth.nvfp4_matrix(n, k, rng)).cuda()
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(5)], [matrix(hidden, inter) for _ in range(5)]
+    w = moe.GpuMoeWeights(hidden, inter, 5, 0.03, 0.7, gate_up=gu, down=dn, device="cuda")
+    x = torch.from_numpy((rng.standard_normal((rows, hidden)) * np.where(rng.random((rows, hidden)) < 0.01, 1e4, 1.0)).astype(np.float32)).cuda().to(dtype)
+    x[3, 7] = float("inf")
+    ids = torch.from_numpy(rng.integers(0, 5, rows).astype(np.int32)).cuda()
+    out = []
+    for plan in (moe.GpuMoePlan(hidden, inter, 5, 1, rows), moe.GpuMoePlan(hidden, inter, 5, 5, -(-rows // 5))):
+        eo = torch.zeros((rows, hidden), device="cuda")
+        plan.experts_only(w, ids, x, eo=eo)
+        out.append(eo.view(torch.int32).clone())
+    assert torch.equal(*out)
+    assert device_status() == 0
+
+
 @pytest.mark.parametrize("size", [1e3, 1e4, 1e7])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_small_values_of_grouped_rows_beside_large_ones(size, dtype):
