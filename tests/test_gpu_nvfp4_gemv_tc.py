@@ -1,4 +1,4 @@
-"""The GEMV on the fifth-generation tensor cores (bf16 rows: matrices of eight million weights and more, with rows of 4096 values or 10000 rows), against 64 bits: clusters of one to eight CTAs, one tile of 128
+"""The GEMV on the fifth-generation tensor cores (bf16 rows: matrices of long rows, or of enough tiles, cn_gemv_m1_launch), against 64 bits: clusters of one to eight CTAs, one tile of 128
 rows to a CTA and several, parts of unequal length, rows that end inside a tile, every number of activation rows; activations of any magnitude, not finite
 ones, and scale bytes that the tensor core reads differently. Every row has the bits of a one-row call."""
 import numpy as np
@@ -47,6 +47,26 @@ def test_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
     _rounded(y, want, 2e-3 if gu else 3e-4)
     for _ in range(3):
         assert torch.equal(y.view(torch.int16), call(x).view(torch.int16))
+    for i in range(m):
+        assert torch.equal(call(x[i:i + 1]).view(torch.int16)[0], y.view(torch.int16)[i]), i
+    assert device_status() == 0
+
+
+# the smallest matrices that come here: 74 tiles, 64 of few chunks, 40 of two chunks, long rows (gate / up: pairs of rows count twice)
+@pytest.mark.parametrize("rows,k,gu", [(9345, 512, False), (8065, 1024, False), (4993, 512, False), (1400, 5120, False), (520, 8192, False), (4673, 512, True), (4065, 1024, True),
+                                       (260, 8192, True)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_smallest_matrices_of_the_rule(rows, k, gu, m):
+    rng, g, g64 = _make(rows, k, rows + k)
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda().to(torch.bfloat16)
+    want, call = x.double() @ g64.t(), lambda v: ops.launch_gemv(g, v)
+    if gu:
+        _, u, u64 = _make(rows, k, rows + k + 1)
+        want, call = want / (1 + torch.exp(-want)) * (x.double() @ u64.t()), lambda v: ops.launch_gemv_gu(g, u, v)
+    y = call(x)
+    # shares as above, with few values: that many expected, and four deviations of their number
+    few = (2e-3 if gu else 3e-4) * y.numel()
+    _rounded(y, want, (few + 4 * few ** 0.5) / y.numel())
     for i in range(m):
         assert torch.equal(call(x[i:i + 1]).view(torch.int16)[0], y.view(torch.int16)[i]), i
     assert device_status() == 0
