@@ -346,12 +346,13 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // bf16 activations: the tensor-core kernel
     if (a.dtype == CN_BF16) return cn_gemv_m1_launch(a, stream, who);
     if (a.line_bases) CN_FAIL(CN_ERR_SHAPE, "%s: line output takes bf16 activations", who);
-    // f32 activations on the fifth-generation tensor cores where a row is long or a matrix large. us a call in a stream of dependent ones, there / here for one
-    // and eight rows: 16384 x 512 3.2 / 3.7 and 5.9 / 13, 20000 x 1536 6.8 / 11.1 and 13.2 / 49, 8192 x 512 2.9 / 3.2 and 5.5 / 6.4, 2048 x 1024 3.5 / 2.2 and 5.3 / 6.8. At
-    // k = 2048 the mma.sync kernel with three f16 planes that was there before took 3.3 and 8.1 for 2048 rows (3.8 and 5.7 now), at 17408 x 5120, gate / up, 26.7 and 84.8
-    // (19.6 and 52). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
+    // f32 activations on the fifth-generation tensor cores where a row is long, a matrix large, or a row no whole number of this kernel's steps of 512 values. us a call in a stream of
+    // dependent ones, there / here for one and eight rows: 12288 x 512 3.0 / 3.4 and 5.7 / 12.6, 8192 x 512 2.9 / 3.1 and 5.4 / 6.4, 4096 x 512 2.8 / 2.3 and 5.0 / 6.0, 2048 x 1024 3.4 / 2.4 and 5.3 / 6.8,
+    // 256 x 1792 3.2 / 5.3 and 5.4 / 14.7, 256 x 1280 3.2 / 4.1 and 5.5 / 11.4, 256 x 768 3.0 / 3.0 and 5.6 / 8.1; gate / up of 256 x 1280 3.5 / 4.2 and 5.6 / 12.2, of 256 x 768 3.5 / 3.1 and
+    // 7.4 / 8.8. The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
     // A rule of the matrix alone: a row's result does not depend on how many rows the call has.
-    if (!routed && (k >= 2048 || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
+    const bool odd_steps = k % 512 != 0 && (k >= 1280 || (k >= 768 && rows >= 64 && !a.w1));
+    if (!routed && (k >= 2048 || odd_steps || (k >= 512 && rows >= 8192 && !a.w1) || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
         if (k > 108544) CN_FAIL(CN_ERR_LIMIT,  // (the library's limit for f32 rows, as it was; this kernel has none)
                                  "%s: k = %d, f32 rows have up to 108544 values", who, k);
         return cn_gemv_tc_launch(a, stream, who);

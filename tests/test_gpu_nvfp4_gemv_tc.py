@@ -52,7 +52,7 @@ def test_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
     assert device_status() == 0
 
 
-# the smallest matrices that come here: 74 tiles, 64 of few chunks, 40 of two chunks, long rows (gate / up: pairs of rows count twice)
+# bf16: the smallest matrices that come here: 74 tiles, 64 of few chunks, 40 of two chunks, long rows (gate / up: pairs of rows count twice)
 @pytest.mark.parametrize("rows,k,gu", [(9345, 512, False), (8065, 1024, False), (4993, 512, False), (1400, 5120, False), (520, 8192, False), (4673, 512, True), (4065, 1024, True),
                                        (260, 8192, True)])
 @pytest.mark.parametrize("m", [1, 3, 8])
@@ -91,6 +91,13 @@ def test_f32_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
     for i in range(m):
         assert torch.equal(call(x[i:i + 1]).view(torch.int32)[0], y.view(torch.int32)[i]), i
     assert device_status() == 0
+
+
+# rows of no whole number of 512-value steps, and many rows of few chunks
+@pytest.mark.parametrize("rows,k,gu", [(64, 768, False), (130, 1280, False), (16, 1792, False), (8192, 512, False), (9000, 1024, False), (16, 1280, True), (200, 1792, True)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_f32_rows_of_short_matrices(rows, k, gu, m):
+    test_f32_rows_against_64_bits_and_one_row_calls(rows, k, gu, m)
 
 
 def test_f32_rows_of_any_magnitude():
