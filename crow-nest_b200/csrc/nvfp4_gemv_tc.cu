@@ -46,11 +46,12 @@ constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk fa
 __host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_of(f32) + 15) / 16 * 16; }  // columns of the MMA
 __host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
 __host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
-__host__ __device__ constexpr int nb_of(int mt) { return mt <= 2 ? 4 : 2; }                                // chunks of digits
+// chunks of digits (us with two / four: four rows of gate / up 17408 x 5120 22.0 / 21.6, eight 31.6 / 30.7; where they fit beside three container stages)
+__host__ __device__ constexpr int nb_of(int mt, bool f32) { return mt == 8 && f32 ? 2 : 4; }
 // accumulators, in half of an SM's tensor memory beside the codes of two chunks and the scales: those of two chunks where they fit (all but eight f32 rows)
 constexpr int TMEM = 256, TM_FIXED = NA * A_COLS + 64;
 __host__ __device__ constexpr int nacc(int mt, bool f32) { return 2 * ncol(mt, f32) + TM_FIXED <= TMEM ? 2 : 1; }
-__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * A_SCALES + nb_of(mt) * b_stage(mt, f32); }
+__host__ __device__ constexpr int fixed_smem(int mt, bool f32) { return HEADER + 1024 + NA * A_SCALES + nb_of(mt, f32) * b_stage(mt, f32); }
 
 struct TcParams {
     const uint8_t* w0;
@@ -122,7 +123,7 @@ template <int MT, bool F32>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                                                                    const TcParams p) {
     constexpr int LV = digits_of(F32), ES = F32 ? 4 : 2;
-    constexpr int N = ncol(MT, F32), NB = nb_of(MT), B_STAGE = b_stage(MT, F32), B_CODES = b_codes(MT, F32);
+    constexpr int N = ncol(MT, F32), NB = nb_of(MT, F32), B_STAGE = b_stage(MT, F32), B_CODES = b_codes(MT, F32);
     using Acc = typename std::conditional<F32, double, float>::type;
     constexpr int NACC = nacc(MT, F32);
     constexpr uint32_t IDESC = idesc_bs(N), SFA_COL = NACC * N, SFB_COL = NACC * N + 32, A_COL = NACC * N + 64;
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_gemv_tc_kernel(const __grid_
             const uint32_t td = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(N * (i % NACC));
             const uint32_t odd = wf[(i % NX) * 4 + warp];
             uint32_t slow = odd;
-            constexpr int G = F32 ? (MT < 2 ? MT : 2) : (MT < 4 ? MT : 4);  // rows at a time
+            constexpr int G = MT < 4 ? MT : F32 && MT == 4 ? 2 : 1;  // rows at a time (eight bf16 rows of gate / up 17408 x 5120: four 32.7 us, two 32.4, one 31.6; four rows: four 21.6, one 21.5)
 #pragma unroll
             for (int m0 = 0; m0 < MT; m0 += G) {
                 uint32_t d[G * LV];
