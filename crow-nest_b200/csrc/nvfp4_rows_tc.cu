@@ -22,8 +22,8 @@ namespace {
 constexpr int RG = 8;        // most rows of a group
 constexpr int CH = 256;      // values of k in a chunk
 constexpr int PIECE = 32 * 144;  // container bytes of a warp's 32 rows and a chunk
-__host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 3 : 4; }  // chunks in flight, as many as fit
-constexpr int NA = 2, NB = 2, NX = 16, NDONE = 4, NU = 8;  // operand stages, chunks of digits, chunk factors, finished chunks, units in the ring
+__host__ __device__ constexpr int depth_of(bool f32) { return f32 ? 2 : 3; }  // chunks in flight, as many as fit beside four chunks of digits (two and one chunk more in flight: 64 tokens of f32 179 / 177 us, 288 experts 338 / 331)
+constexpr int NA = 2, NB = 4, NX = 16, NDONE = 4, NU = 8;  // operand stages, chunks of digits, chunk factors, finished chunks, units in the ring
 constexpr int NBAR = NX + NDONE + 2 * NU;
 constexpr int SCOUT = 12, ISSUER = 13, THREADS = 448;
 constexpr int FS_OFF = 512, WF_OFF = 1536, UNIT_OFF = 1792, HEADER = 2560;
@@ -160,15 +160,15 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
             if (nrows < 0) break;
             const uint32_t idesc = idesc_bs((nrows * LV + 15) & ~15);
             for (int ch = 0; ch < nk; ch++, i++) {
-                const int a = i & 1;
+                const int a = i & 1, b = i % NB;
                 if (!mbar_wait(&ready[i % NX], (uint32_t)(i / NX) & 1u)) {  // (one wait for all three: each costs some 75 cycles, passed or not)
                     cn_dev_fail(CN_DEV_WAIT_FULL);
                     ok = false;
                     break;
                 }
                 tc_after();
-                const uint64_t db = tc_desc_sw128(b_u + (uint32_t)(a * B_STAGE));
-                const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_SCALES)), sb = desc_sf(b_u + (uint32_t)(a * B_STAGE + B_CODES));
+                const uint64_t db = tc_desc_sw128(b_u + (uint32_t)(b * B_STAGE));
+                const uint64_t sa = desc_sf(a_u + (uint32_t)(a * A_SCALES)), sb = desc_sf(b_u + (uint32_t)(b * B_STAGE + B_CODES));
                 const uint32_t ta = tmem + SFA_COL + 16 * a, tb = tmem + SFB_COL + 16 * a, td = tmem + N * (i % NACC);
                 if (elect_lane()) {
 #pragma unroll
