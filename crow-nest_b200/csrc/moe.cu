@@ -229,8 +229,14 @@ __global__ void moe_combine_kernel(const float* __restrict__ eo, const float* __
         ((float*)y)[(size_t)t * H + c] = v;
 }
 
-// Combos from which the routed step groups the rows of an expert (measured: see routed_experts).
-constexpr int GROUP_COMBOS = 48;
+// Combos from which the routed step groups the rows of an expert (measured: see routed_experts), and fewer of larger experts: one by one, each combo streams its expert, and f32 rows take CUDA
+// cores. us per step one by one / grouped: 288 experts of 4096 x 2048, top 8, 3 tokens 93.5 / 87, 5 tokens 136 / 114, f32 2 tokens 93 / 75, 5 tokens 191 / 120; 128 of 2560 x 1280, top 6,
+// 4 tokens 55.7 / 55.7, 7 tokens 81 / 73, f32 3 tokens 66 / 53, 7 tokens 106 / 75; 512 of 2048 x 768, top 10, 4 tokens 51 / 54, f32 3 tokens 53.6 / 50.9; 64 of 1024 x 1280, top 8, f32 5 tokens
+// 59 / 41.5; 512 of 2048 x 512, top 10, 4 tokens 35.5 / 49, f32 45 / 50.
+constexpr int GROUP_COMBOS = 48, GROUP_LEAST = 16;
+bool groups_rows(int combos, int hidden, int inter, bool f32) {
+    return combos >= GROUP_COMBOS || (combos >= (f32 ? GROUP_LEAST : 24) && (long long)combos * hidden * inter >= (f32 ? 47000000 : 80000000));
+}
 // Bytes of a plan's store of digits at most.
 constexpr size_t DIGITS_MOST = (size_t)64 << 20;
 
@@ -315,7 +321,7 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
         CN_FAIL(CN_ERR_CUDA, "cn_moe_nvfp4_plan_create: %s", cudaGetErrorString(e));
     }
     // Records of the digits of x for the grouped step, bounded; without them (and for more rows than they hold) the digits are made where they are used, which has the same bits.
-    if (combos >= GROUP_COMBOS) {
+    if (combos >= GROUP_LEAST) {
         p->xd_bytes = (size_t)max_tokens * (hidden / 256) * digit_record(true);
         if (p->xd_bytes > DIGITS_MOST) p->xd_bytes = DIGITS_MOST;
         if (cudaMalloc(&p->xd, p->xd_bytes) != cudaSuccess) {
@@ -414,7 +420,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     // us per step (64 tokens, 512 experts of 2048 x 512, top 10, unless said otherwise) now / with mma.sync kernels that decoded the weights to f16 for eight bf16
     // or two f32 rows: 192 / 213, 128 tokens 293 / 323, 16 tokens 86 / 109, f32 rows 208 / 234; 64 experts of 1024 x 1280, top 8, 108 tokens 178 / 198; 128 experts, f32,
     // 100 tokens 216 / 291; 288 experts of 4096 x 2048, top 8, 10 tokens 198 / 239. With 40 combos nothing was gained (48 / 48 us): the grouping is a launch of its own.
-    if (combos >= GROUP_COMBOS && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
+    if (groups_rows(combos, p->hidden, p->inter, dtype == CN_F32) && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
         int* ga = p->groups;
         int* gb = ga + combos;
         int* gbrows = gb + combos;
@@ -522,7 +528,7 @@ extern "C" int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, 
     const float* shared = nullptr;
     int rc = CN_OK;
     if (shared_gate && (rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_run"))) return rc;
-    if (tokens * p->topk < GROUP_COMBOS) {
+    if (!groups_rows(tokens * p->topk, p->hidden, p->inter, dtype == CN_F32)) {
         // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine. A warp
         // of the second waits for each of its units by itself, so from 16 combos on - where the routed kernel below has a warp per tile with two to
         // four chunks in flight - it is only taken for few units of work. us per step in two launches / with the other kernels (a side stream for

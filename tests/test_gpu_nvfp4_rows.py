@@ -53,6 +53,13 @@ def test_grouped_experts_against_64_bits(hidden, inter, experts, topk, tokens, s
     assert device_status() == 0
 
 
+# large experts are grouped with fewer combos (either side of the rule: 16 and more of f32 rows, 24 and more of bf16 rows)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [7, 8, 11, 12])
+def test_fewer_combos_of_large_experts_against_64_bits(tokens, dtype):
+    test_grouped_experts_against_64_bits(4096, 2048, 3, 2, tokens, 256, dtype)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [56, 64, 125])
 def test_full_groups_repeat_bit_for_bit(tokens, dtype):
