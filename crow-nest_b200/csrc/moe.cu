@@ -246,7 +246,7 @@ struct MoePlan {
     float* eo;       // [max_tokens * topk][hidden]
     float* hs;       // [max_tokens][shared inter <= inter_s]
     float* ys;       // [max_tokens][hidden]
-    int32_t* order;  // [max_tokens * topk]
+    int32_t* order;  // [max_tokens * topk]; groups and xd lie behind it
     int* groups;     // [3 * max_tokens * topk + 8]: the group lists of moe_group_kernel and their two counts
     uint8_t* xd;     // records of the digits of x; null where there is no room for them
     size_t xd_bytes;
@@ -311,23 +311,23 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
     step(cudaMalloc(&p->eo, combos * hidden * sizeof(float)));
     step(cudaMalloc(&p->hs, (size_t)max_tokens * (shared_inter > 0 ? shared_inter : 1) * sizeof(float)));
     step(cudaMalloc(&p->ys, (size_t)max_tokens * hidden * sizeof(float)));
-    step(cudaMalloc(&p->order, combos * sizeof(int32_t)));
-    step(cudaMalloc(&p->groups, (3 * combos + 8) * sizeof(int)));
+    // lists, and behind them records of the digits of x for the grouped step, bounded; without them (and for more rows than they hold) the digits are made where they are used, which has the same bits
+    const size_t order_bytes = (combos * sizeof(int32_t) + 255) / 256 * 256, group_bytes = ((3 * combos + 8) * sizeof(int) + 255) / 256 * 256;
+    p->xd_bytes = combos < GROUP_LEAST ? 0 : (size_t)max_tokens * (hidden / 256) * digit_record(true);
+    if (p->xd_bytes > DIGITS_MOST) p->xd_bytes = DIGITS_MOST;
+    uint8_t* lists = nullptr;
+    if (e == cudaSuccess && p->xd_bytes && cudaMalloc(&lists, order_bytes + group_bytes + p->xd_bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        lists = nullptr, p->xd_bytes = 0;
+    }
+    if (!lists) step(cudaMalloc(&lists, order_bytes + group_bytes));
+    if (lists) p->order = (int32_t*)lists, p->groups = (int*)(lists + order_bytes), p->xd = p->xd_bytes ? lists + order_bytes + group_bytes : nullptr;
     step(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
     step(cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming));
     step(cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming));
     if (e != cudaSuccess) {
         cn_moe_nvfp4_plan_destroy(p);
         CN_FAIL(CN_ERR_CUDA, "cn_moe_nvfp4_plan_create: %s", cudaGetErrorString(e));
-    }
-    // Records of the digits of x for the grouped step, bounded; without them (and for more rows than they hold) the digits are made where they are used, which has the same bits.
-    if (combos >= GROUP_LEAST) {
-        p->xd_bytes = (size_t)max_tokens * (hidden / 256) * digit_record(true);
-        if (p->xd_bytes > DIGITS_MOST) p->xd_bytes = DIGITS_MOST;
-        if (cudaMalloc(&p->xd, p->xd_bytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            p->xd = nullptr, p->xd_bytes = 0;
-        }
     }
     *plan_out = p;
     return CN_OK;
@@ -336,7 +336,7 @@ extern "C" int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, 
 extern "C" int cn_moe_nvfp4_plan_destroy(void* plan) {
     MoePlan* p = (MoePlan*)plan;
     if (!p) return CN_OK;
-    cudaFree(p->h), cudaFree(p->eo), cudaFree(p->hs), cudaFree(p->ys), cudaFree(p->order), cudaFree(p->groups), cudaFree(p->xd);
+    cudaFree(p->h), cudaFree(p->eo), cudaFree(p->hs), cudaFree(p->ys), cudaFree(p->order);
     if (p->side) cudaStreamDestroy(p->side);
     if (p->fork) cudaEventDestroy(p->fork);
     if (p->join) cudaEventDestroy(p->join);
@@ -416,10 +416,10 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
                    const unsigned long long* eo_ptrs, int combos, int x_div, float limit, int dtype, cudaStream_t stream) {
     const GemvCall a = routed_gate_up(p, table_gu, table_up, gs_gu, gs_up, ids, x, combos, x_div, limit, dtype);
     const bool short_rows = p->hidden <= MAX_ROW && p->inter <= MAX_ROW;
-    // From 48 combos on the combos are sorted by expert and cut into groups of up to eight rows that share one pass over the expert's weights (nvfp4_rows_tc.cu).
+    // From 48 combos on (and fewer of large experts) the combos are sorted by expert and cut into groups of up to eight rows that share one pass over the expert's weights (nvfp4_rows_tc.cu).
     // us per step (64 tokens, 512 experts of 2048 x 512, top 10, unless said otherwise) now / with mma.sync kernels that decoded the weights to f16 for eight bf16
-    // or two f32 rows: 192 / 213, 128 tokens 293 / 323, 16 tokens 86 / 109, f32 rows 208 / 234; 64 experts of 1024 x 1280, top 8, 108 tokens 178 / 198; 128 experts, f32,
-    // 100 tokens 216 / 291; 288 experts of 4096 x 2048, top 8, 10 tokens 198 / 239. With 40 combos nothing was gained (48 / 48 us): the grouping is a launch of its own.
+    // or two f32 rows: 163 / 213, 128 tokens 230 / 323, 16 tokens 82 / 109, f32 rows 177 / 234; 64 experts of 1024 x 1280, top 8, 108 tokens 129 / 198;
+    // 288 experts of 4096 x 2048, top 8, 10 tokens 175 / 239. Fewer combos: see `groups_rows`.
     if (groups_rows(combos, p->hidden, p->inter, dtype == CN_F32) && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
         int* ga = p->groups;
         int* gb = ga + combos;
