@@ -11,18 +11,17 @@
 // reading A.
 //
 // A CTA owns 128 rows (64 of gate and 64 of up) over a part of k; a cluster of C CTAs shares the tile, part by part, and every CTA adds and stores
-// 128 / C of its rows, the parts in order. Warps: 0-3 add up and store (a thread is a row), 4-7 move container blocks (36 bytes) into the operand's
-// layout, 8-11 turn activations into digits, 12 loads (TMA, boxes of 128 rows x 144 bytes of container), 13 issues the MMAs. Loads and the move do
-// not wait for the kernel in front: when the activations come, five chunks of weights a CTA lie ready or nearly so.
+// 128 / C of its rows, the parts in order. Warps: 0-3 add up and store (a thread is a row), 4-7 move container blocks (36 bytes): codes into
+// tensor memory, scales into the chunks that are copied there; 8-11 turn activations into digits, 12 loads (TMA, boxes of 128 rows x 144 bytes of container), 13 issues the MMAs. Loads and the move do
+// not wait for the kernel in front: when the activations come, six chunks of weights a CTA lie ready or nearly so.
 //
-// What bounds it, one row: HBM for large matrices (gate / up of 17408 x 5120: 100 MB in 18.8 us, of which 2.6 until the first product; the CTAs then take 6.1 TB/s);
+// What bounds it, one row: HBM for large matrices (gate / up of 17408 x 5120: 100 MB in 17.4 us, of which 2.6 until the first product);
 // for small ones the chain from one call to the next, some 3 us: end of the grid in front 0.8, activations 0.4, digits 0.35, first sum 0.4, adding up in
 // the cluster 0.4, output and end of the grid 0.6. From four rows on also the digits (one warp and row: 0.35 us a chunk). In a stream of dependent calls, us
-// here / mma.sync kernel (nvfp4_gemv_m1.cu): gate / up of 17408 x 5120 18.8 / 20.7, two rows 19.4 / 27.3, four 23.8 / 30.1, eight 33.1 / 46.5; 5120 x 17408
-// 12.4 / 15.5, 12.8 / 18.5, 15.3 / 21.1, 20.7 / 34.7; 25000 x 8192 22.0 / 28.2, four rows 28.0 / 32.0. f32 rows, here / mma.sync with three f16 planes a row: gate / up of
-// 17408 x 5120 19.6 / 26.7, 22.7 / 39.8, 29.3 / 41.2, 52 / 85; 5120 x 17408 12.7 / 22.1, 14.5 / 38, 18.4 / 62, 30 / 122.
-// The loads and stores of a container row stand in functions that nvfp4_rows_tc.cu shares; written out here they take four bf16 rows of that gate / up 1 us less, one and eight 0.4 and 0.8 more.
-// Measured and not kept: tiles of fewer rows so that every SM has the same bytes (the CTAs more hold up the next kernel: 5120 x 5120 5.9 -> 6.9); two teams of
+// here / mma.sync kernel (nvfp4_gemv_m1.cu): gate / up of 17408 x 5120 17.4 / 20.7, two rows 17.7 / 27.3, four 21.5 / 30.1, eight 30.7 / 46.5; 5120 x 17408
+// 10.7 / 15.5, 11.4 / 18.5, 14.0 / 21.1, 19.2 / 34.7; 25000 x 8192 19.5 / 28.2, four rows 25.0 / 32.0. f32 rows, here / mma.sync with three f16 planes a row: gate / up of
+// 17408 x 5120 17.7 / 26.7, 19.0 / 39.8, 29.0 / 41.2, 49.3 / 85; 5120 x 17408 11.1 / 22.1, 12.7 / 38, 18.2 / 62, 29.2 / 122.
+// Measured and not kept: a fifth container stage (the same); weight and activation warps on schedulers of their own (4096 x 4096 4.7 -> 4.9); and, while the operand lay in shared memory: tiles of fewer rows so that every SM has the same bytes (the CTAs more hold up the next kernel: 5120 x 5120 5.9 -> 6.9); two teams of
 // warps for the move (18.6 -> 20.0, gate / up); L2 prefetches beyond the stages (18.6 -> 19.3 and more); a third operand stage in a container stage's place (20.6).
 #include "nvfp4_digits.cuh"
 #include "nvfp4_gemv.cuh"
@@ -533,9 +532,10 @@ int clusters_of(int c) {
 // for each of them, and 0.92 late in a launch of two to an SM. Without clusters an SM with two CTAs needs 0.86 for a chunk of either however many other SMs have one, and the last
 // round counts in full and more. The chunks are otherwise nearer to the mean than to those of the busiest CTA; 0.62 for adding up a tile in a cluster and 0.026 for each of its CTAs. The figures are those that
 // made the picks for 130 matrices, each timed with every cut, lose least (1 percent on average; 22 for the estimate that stood here before, which had a matrix of 152 tiles as 152 CTAs on 148 SMs).
-// Measured, us with 1 / 2 / 4 / 6 / 8 CTAs: 16384 x 2048 5.7 / 6.5 / 7.1 / 8.6 / 8.2, 8192 x 4096 9.5 / 6.2 / 6.5 / 7.2 / 7.4, 4096 x 8192 17.2 / 10.1 / 6.3 / 6.9 / 6.9, 7168 x 5120 11.5
-// / 7.2 / 6.9 / 7.7 / 8.0, 5120 x 17408 48 / 24 / 14.6 / 12.3 / 16.4, gate / up of 17408 x 5120 18.5 / 19.6 / 20.9 / 25 / 36, of 9728 x 5120 18.1 / 16.3 / 13.8 / 15.6 / 17.2, of
-// 12288 x 4096 15.2 / 14.0 / 14.0 / 15.7 / 16.2, of 20480 x 2048 13.0 / 11.7 / 14.2. 3, 5 and 7 never were the fastest.
+// They were taken while the operand
+// lay in shared memory; with the codes in tensor memory the picks lose 1.6 percent on average over 33 matrices and one, two and four rows (most: 10240 x 8192 10, one row of 4096 x 14336 9), and stay, since they are
+// the order of sums. Measured, us of one row with 1 / 2 / 4 / 6 / 8 CTAs: 16384 x 2048 5.1 / 6.0 / 6.6 / 8.0 / 8.3, 7168 x 5120 9.4 / 6.4 / 6.6 / 7.2 / 7.7, 5120 x 17408 27.7 / 15.6 / 11.7 / 10.8 / 11.3, gate / up of
+// 17408 x 5120 17.6 / 17.4 / 17.7 / 19.9 / 22.4, of 9728 x 5120 13.0 / 13.0 / 11.5 / 13.2 / 15.0, of 12288 x 4096 11.6 / 11.8 / 11.8 / 13.8 / 14.4, of 20480 x 2048 10.6 / 10.3 / 12.3. 3, 5 and 7 never were the fastest.
 int cut_of(int tiles, int nk) {
     constexpr int AT_ONCE[9] = {0, 296, 148, 0, 70, 0, 46, 0, 32};
     int best_c = 1;

@@ -8,10 +8,12 @@
 // the weights out for the tensor core bring them in themselves, by 16-byte asynchronous copies, past the ends of units. Warps: 0-3 add up and store,
 // 4-7 weights, 8-11 activations, 12 scout, 13 issues the MMAs. In the gate / up form a warp's rows are 16 of gate and the same 16 of up.
 //
-// What bounds it: the way of the weights through a warp (gate / up of 64 tokens, 512 experts of 2048 x 512, top 10: 2150 cycles a chunk of 18 KB and CTA, 470 of
-// them loads, 500 stores and their fence, 580 the copies of a later chunk), 4.1 TB/s; us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16
-// or two f32 rows: gate / up 103 / 114, down 72 / 77. Tried: the same with a bulk copy for each row piece of 144 bytes 166 and 93; copies asked for
-// before the stores of the chunk in hand, one chunk less ahead, 109 and 79.
+// What bounds it: no unit of the chip but the roles' own loops and hand-overs. A step of 64 tokens, 512 experts of 2048 x 512, top 10, took 165 us; with all copies, stores, digits and sums left
+// out 89, with the copies alone left out 139, the stores 167, the digits 148, the sums 158. (With operand A in shared memory that was the nearest bound, 1740 of 2390 cycles of a chunk in both CTAs.)
+// us under the profiler, here / mma.sync kernel that decoded to f16 for eight bf16 or two f32 rows: gate / up 85 / 114 (5.0 TB/s), down 63 / 77.
+// Tried: a bulk copy for each row piece of 144 bytes (gate / up 105 -> 166 us); copies asked for before the stores of the chunk in hand, one chunk less ahead (109); three or four chunks of
+// accumulators and operands in flight (the same); two teams of weight warps, and weight and activation warps on schedulers of their own (slower); digits that stay in their stages while tiles of
+// one group follow each other (the same); the operand's bytes taken as they lie in the container (an illegal instruction, whose cause was not found).
 #include "nvfp4_digits.cuh"
 #include "nvfp4_gemv.cuh"
 
