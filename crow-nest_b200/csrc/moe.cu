@@ -355,6 +355,11 @@ int check_shared(const MoePlan* p, const void* shared_gate, const void* shared_u
 
 constexpr int MAX_ROW = 32768;  // values of a row in the kernel for groups of rows; longer ones are left to the GEMVs, which know their limits
 
+// whether these combos run in groups: by the rule, where the rows and the grouping's shared memory allow it
+bool grouped(const MoePlan* p, int combos, bool f32) {
+    return groups_rows(combos, p->hidden, p->inter, f32) && p->hidden <= MAX_ROW && p->inter <= MAX_ROW && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024;
+}
+
 // the shared expert on every token, up to 8 rows per pass, on the plan's side stream between the fork and join events:
 // whatever happens after the fork, the side stream is joined again (a capture of the caller's stream stays valid)
 int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs, const void* x,
@@ -420,7 +425,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
     // us per step (64 tokens, 512 experts of 2048 x 512, top 10, unless said otherwise) now / with mma.sync kernels that decoded the weights to f16 for eight bf16
     // or two f32 rows: 163 / 213, 128 tokens 230 / 323, 16 tokens 82 / 109, f32 rows 177 / 234; 64 experts of 1024 x 1280, top 8, 108 tokens 129 / 198;
     // 288 experts of 4096 x 2048, top 8, 10 tokens 175 / 239. Fewer combos: see `groups_rows`.
-    if (groups_rows(combos, p->hidden, p->inter, dtype == CN_F32) && short_rows && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024) {
+    if (grouped(p, combos, dtype == CN_F32)) {
         int* ga = p->groups;
         int* gb = ga + combos;
         int* gbrows = gb + combos;
@@ -528,7 +533,7 @@ extern "C" int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, 
     const float* shared = nullptr;
     int rc = CN_OK;
     if (shared_gate && (rc = check_shared(p, shared_gate, shared_up, shared_down, shared_gs, "cn_moe_nvfp4_run"))) return rc;
-    if (!groups_rows(tokens * p->topk, p->hidden, p->inter, dtype == CN_F32)) {
+    if (tokens * p->topk < GROUP_COMBOS && !grouped(p, tokens * p->topk, dtype == CN_F32)) {
         // A small step in two launches: gate / up of the combos and of the shared expert, then their down projections with the combine. A warp
         // of the second waits for each of its units by itself, so from 16 combos on - where the routed kernel below has a warp per tile with two to
         // four chunks in flight - it is only taken for few units of work. us per step in two launches / with the other kernels (a side stream for

@@ -602,7 +602,7 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
         return rc;
     // A CTA asks for half of an SM's shared memory, as of its tensor memory: as many of these kernels (or of nvfp4_rows_tc.cu's) as fit an SM find tensor memory there. The pair
-    // GEMM, which takes all of it, stands apart by its registers: 640 threads of 72 leave no room for 448 of 72.
+    // GEMM, which takes all of it, stands apart by its registers: 640 threads of 72 leave no room for 448 of 64.
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * c)), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SM_SHARE, cfg.stream = stream;
     cudaLaunchAttribute at[2];
