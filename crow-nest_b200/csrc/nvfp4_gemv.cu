@@ -349,7 +349,7 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // f32 activations on the fifth-generation tensor cores where a row is long, a matrix large, or a row no whole number of this kernel's steps of 512 values. us a call in a stream of
     // dependent ones, there / here for one and eight rows: 12288 x 512 3.0 / 3.4 and 5.7 / 12.6, 8192 x 512 2.9 / 3.1 and 5.4 / 6.4, 4096 x 512 2.8 / 2.3 and 5.0 / 6.0, 2048 x 1024 3.4 / 2.4 and 5.3 / 6.8,
     // 256 x 1792 3.2 / 5.3 and 5.4 / 14.7, 256 x 1280 3.2 / 4.1 and 5.5 / 11.4, 256 x 768 3.0 / 3.0 and 5.6 / 8.1; gate / up of 256 x 1280 3.5 / 4.2 and 5.6 / 12.2, of 256 x 768 3.5 / 3.1 and
-    // 7.4 / 8.8. The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
+    // 7.4 / 8.8. Against 64 bits a row is 2.7e-8 off there, 1.0e-7 here (normally distributed rows, SiLU rows, cubes). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
     // A rule of the matrix alone: a row's result does not depend on how many rows the call has.
     const bool odd_steps = k % 512 != 0 && (k >= 1280 || (k >= 768 && rows >= 64 && !a.w1));
     if (!routed && (k >= 2048 || odd_steps || (k >= 512 && rows >= 8192 && !a.w1) || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
