@@ -83,6 +83,7 @@ _SIGS = {
     "cn_moe_combine": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "cn_moe_nvfp4_plan_create": [C.POINTER(C.c_void_p), _i, _i, _i, _i, _i, _i],
     "cn_moe_nvfp4_plan_destroy": [_vp],
+    "cn_moe_nvfp4_plan_digits": [_vp, C.POINTER(C.c_void_p), C.POINTER(C.c_size_t)],
     "cn_moe_nvfp4_run": [_vp] * 16 + [_i, _f, _i, _vp],
     "cn_moe_nvfp4_experts": [_vp] * 11 + [_i, _i, _f, _i, _vp],
     "cn_moe_nvfp4_finish": [_vp] * 12 + [_i, _f, _i, _vp],

@@ -82,6 +82,38 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 // stable; where an expert has more than LONG_RUN rows, or the list does not fit (listed = 0), one warp walks the combos in order instead (match.any finds the lanes of a
 // step that share an expert; 20 dependent steps for 640 combos). A step of 64 tokens, top 10 of 512 experts: 203.0 -> 199.9 us, replayed 199.5 -> 198.8.
 constexpr int LONG_RUN = 64;
+__device__ __forceinline__ bool resident(int e, const unsigned long long* __restrict__ tab, int E) { return e >= 0 && e < E && !(tab && tab[e] == 0ull); }
+// Records of the chunks of activations, by warp `w` of `warps`. Rows none of whose combos has a resident expert are left out, since nothing reads them and most inbox slots of an
+// expert-parallel rank are such rows: one rank of eight, 512 experts of 2048 x 512, top 10, 64 tokens a rank (620 of 5120 slots in use), routed experts 88.7 -> 78.4 us. A lane looks one of the
+// warp's chunks up, the ids and then the entries of eight combos at a time. The first chunk of a warp is made without a look: up to a chunk for every warp they are made beside
+// the grouping on SMs that have nothing else to do, and two more trips to memory in front of them show (160 slots 23.0 -> 23.3 us).
+template <bool F32>
+__device__ __forceinline__ void put_records(const DigitsCall& dc, const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E, int w, int warps, int lane) {
+    const char* x = (const char*)dc.x;
+    constexpr size_t BYTES = 256 * (F32 ? 4 : 2);
+    for (int i0 = w; i0 < dc.chunks; i0 += 32 * warps) {
+        ChunkValues<F32> v;
+        v.load(x + i0 * BYTES, lane);
+        const int at = i0 + lane * warps;
+        bool read = at == w;
+        if (!read && at < dc.chunks) {
+            const int c0 = at / dc.row_chunks * dc.x_div, c1 = min(c0 + dc.x_div, n);
+            for (int c = c0; c < c1 && !read; c += 8) {
+                int e[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) e[j] = c + j < c1 ? ids[c + j] : -1;
+#pragma unroll
+                for (int j = 0; j < 8; j++) read |= resident(e[j], tab, E);
+            }
+        }
+        for (uint32_t todo = __ballot_sync(0xffffffffu, read); todo; todo &= todo - 1u) {
+            const int j = __ffs(todo) - 1;
+            const size_t i = (size_t)(i0 + j * warps);
+            if (j > 0) v.load(x + i * BYTES, lane);
+            put_record<F32>(v, lane, dc.out + i * digit_record(F32));
+        }
+    }
+}
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,
                                                          int32_t* __restrict__ order, int* __restrict__ ga, int* __restrict__ gb,
                                                          int* __restrict__ gbrows, int* __restrict__ counts, int gmax, int listed, const DigitsCall dc) {
@@ -97,21 +129,19 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     // 207.1 -> 197.5 us a step, MUL1 with 16 tokens 266.4 -> 264.3.
     pdl_launch_dependents();
     pdl_wait();
-    if (blockIdx.x > 0) {  // not the grouping: a warp a chunk of activations
-        const int i = ((int)blockIdx.x - 1) * 32 + wid;
-        if (i < dc.chunks) {
-            if (dc.f32)
-                put_record<true>((const float*)dc.x + (size_t)i * 256, lane, dc.out + (size_t)i * digit_record(true));
-            else
-                put_record<false>((const __nv_bfloat16*)dc.x + (size_t)i * 256, lane, dc.out + (size_t)i * digit_record(false));
-        }
+    if (blockIdx.x > 0) {  // not the grouping
+        const int w = ((int)blockIdx.x - 1) * 32 + wid, warps = ((int)gridDim.x - 1) * 32;
+        if (dc.f32)
+            put_records<true>(dc, ids, tab, n, E, w, warps, lane);
+        else
+            put_records<false>(dc, ids, tab, n, E, w, warps, lane);
         return;
     }
     for (int i = tid; i <= E; i += blockDim.x) cnt[i] = 0;
     __syncthreads();
     for (int c = tid; c < n; c += blockDim.x) {
         const int e = ids[c];
-        const int b = (e < 0 || e >= E || (tab && tab[e] == 0ull)) ? E : e;
+        const int b = resident(e, tab, E) ? e : E;
         bin[c] = b | atomicAdd(&cnt[b], 1) << 14;
     }
     __syncthreads();
@@ -237,6 +267,8 @@ constexpr int GROUP_COMBOS = 48, GROUP_LEAST = 16;
 bool groups_rows(int combos, int hidden, int inter, bool f32) {
     return combos >= GROUP_COMBOS || (combos >= (f32 ? GROUP_LEAST : 24) && (long long)combos * hidden * inter >= (f32 ? 47000000 : 80000000));
 }
+// Blocks of the grouping kernel that make records at most: one to an SM (1024 threads of 56 registers) beside the one that groups.
+constexpr int DIGIT_BLOCKS = 148 - 1;
 // Bytes of a plan's store of digits at most.
 constexpr size_t DIGITS_MOST = (size_t)64 << 20;
 
@@ -269,7 +301,8 @@ int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int c
     CN_ALLOW_SMEM(moe_group_kernel, 160 * 1024);
     const size_t listed = smem + (size_t)combos * sizeof(int);
     const bool fits = listed <= 160 * 1024;
-    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3(1u + (unsigned)((digits.chunks + 31) / 32)), dim3(1024), fits ? listed : smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax, (int)fits, digits));
+    const int more = (digits.chunks + 31) / 32, blocks = 1 + (more < DIGIT_BLOCKS ? more : DIGIT_BLOCKS);
+    CN_CUDA(cn_launch_pdl(moe_group_kernel, dim3((unsigned)blocks), dim3(1024), fits ? listed : smem, stream, ids, tab, combos, experts, order, ga, gb, gbrows, counts, gmax, (int)fits, digits));
     return CN_OK;
 }
 
@@ -360,6 +393,17 @@ bool grouped(const MoePlan* p, int combos, bool f32) {
     return groups_rows(combos, p->hidden, p->inter, f32) && p->hidden <= MAX_ROW && p->inter <= MAX_ROW && (size_t)(3 * (p->experts + 1) + combos) * sizeof(int) <= 160 * 1024;
 }
 
+}  // namespace
+
+extern "C" int cn_moe_nvfp4_plan_digits(void* plan, void** records, size_t* bytes) {
+    const MoePlan* p = (const MoePlan*)plan;
+    if (!p || !records || !bytes) CN_FAIL(CN_ERR_SHAPE, "cn_moe_nvfp4_plan_digits: null argument");
+    *records = p->xd, *bytes = p->xd_bytes;
+    return CN_OK;
+}
+
+namespace {
+
 // the shared expert on every token, up to 8 rows per pass, on the plan's side stream between the fork and join events:
 // whatever happens after the fork, the side stream is joined again (a capture of the caller's stream stays valid)
 int shared_branch(MoePlan* p, const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs, const void* x,
@@ -446,7 +490,7 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
         // a launch of their own in front of the down projection: 64 tokens 167 / 175, 108 tokens 129 / 122, 128 tokens 234 / 232.
         DigitsCall dx = {};
         if (!((uintptr_t)x & 15) && x_chunks * digit_record(f32) <= (long long)p->xd_bytes) {
-            dx.x = x, dx.chunks = (int)x_chunks, dx.f32 = f32, dx.out = p->xd;
+            dx.x = x, dx.chunks = (int)x_chunks, dx.row_chunks = p->hidden / 256, dx.x_div = x_div, dx.f32 = f32, dx.out = p->xd;
             u.digits = p->xd;
         }
         if (int rc = cn_moe_group_launch(ids, table_gu, combos, p->experts, p->order, ga, gb, gbrows, counts, 8, stream, dx)) return rc;

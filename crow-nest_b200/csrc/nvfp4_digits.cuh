@@ -154,12 +154,17 @@ __device__ __forceinline__ void to_digits(const uint4* raw, int lane, uint8_t* b
 // The same kept in global memory, for matrices of many tiles, which would each make the digits of their rows: the lines as of row 0, four words of scales, factor and blocks without digits.
 __host__ __device__ constexpr int digit_record(bool f32) { return digits_of(f32) * 128 + 32; }
 template <bool F32>
-__device__ __forceinline__ void put_record(const void* x, int lane, uint8_t* rec) {  // x: the chunk's 256 values
-    constexpr int XR = F32 ? 2 : 1;
-    uint4 raw[XR];
+struct ChunkValues {  // a lane's eight values of a chunk
+    static constexpr int XR = F32 ? 2 : 1;
+    uint4 v[XR];
+    __device__ __forceinline__ void load(const void* x, int lane) {  // x: the chunk's 256 values
 #pragma unroll
-    for (int j = 0; j < XR; j++) raw[j] = __ldcg((const uint4*)x + lane * XR + j);
-    to_digits<F32, true>(raw, lane, rec, rec + digits_of(F32) * 128, 0, (float2*)(rec + digits_of(F32) * 128 + 16));
+        for (int j = 0; j < XR; j++) v[j] = __ldcg((const uint4*)x + lane * XR + j);
+    }
+};
+template <bool F32>
+__device__ __forceinline__ void put_record(const ChunkValues<F32>& c, int lane, uint8_t* rec) {
+    to_digits<F32, true>(c.v, lane, rec, rec + digits_of(F32) * 128, 0, (float2*)(rec + digits_of(F32) * 128 + 16));
 }
 template <bool F32>
 struct DigitRecord {  // a lane's part of one

@@ -46,10 +46,11 @@ unsigned long long* cn_trace_slot();  // diagnostic build: where the next launch
 
 // Sort combos by expert and cut every expert's run into groups (moe.cu): order [combos]; ga = positions (in order) of the
 // one-row groups, counts[0] of them; gb / gbrows = positions and row counts (2..gmax, gmax 4 or 8) of the larger groups,
-// counts[1]. Combos without a resident expert are in no group. Beside it, where given, chunks of activations into records of digits (nvfp4_digits.cuh).
+// counts[1]. Combos without a resident expert are in no group. Beside it, where given, chunks of activations into records of digits (nvfp4_digits.cuh), but for
+// rows that no such combo reads.
 struct DigitsCall {
     const void* x;  // rows one after another
-    int chunks, f32;
+    int chunks, row_chunks, x_div, f32;  // in all, of a row; combos that read a row (those from row x x_div on)
     uint8_t* out;
 };
 int cn_moe_group_launch(const int32_t* ids, const unsigned long long* tab, int combos, int experts, int32_t* order, int* ga, int* gb, int* gbrows,

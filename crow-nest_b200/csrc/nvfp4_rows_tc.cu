@@ -46,15 +46,6 @@ struct Unit {
 };
 static_assert(UNIT_OFF + NU * sizeof(Unit) <= HEADER && NBAR * 8 + 8 <= FS_OFF, "header");
 
-template <int XR>
-struct Values {  // a lane's eight values of a chunk
-    uint4 v[XR];
-    __device__ __forceinline__ void load(const void* x, int lane) {
-#pragma unroll
-        for (int j = 0; j < XR; j++) v[j] = __ldcg((const uint4*)x + lane * XR + j);
-    }
-};
-
 template <bool F32, bool KEPT>
 __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCall c) {
     constexpr int D = depth_of(F32), LV = digits_of(F32), ES = F32 ? 4 : 2, N = ncol(F32), B_CODES = N * 128, B_STAGE = b_stage(F32);
@@ -189,10 +180,9 @@ __global__ void __launch_bounds__(THREADS, 2) nvfp4_rows_tc_kernel(const RowsCal
         }
     } else if (warp >= 8) {
         // ------------------------------------------------------------ activations -> digits: rows of a chunk and the next chunk's go round the four warps
-        constexpr int XR = F32 ? 2 : 1;
         const int w = warp - 8;
         int q = 0, ch = 0, nrows = 0;
-        using Held = typename std::conditional<KEPT, DigitRecord<F32>, Values<XR>>::type;
+        using Held = typename std::conditional<KEPT, DigitRecord<F32>, ChunkValues<F32>>::type;
         Held nx[2];
         bool ok = true;
         auto unit = [&](int n) -> int {  // rows of unit n

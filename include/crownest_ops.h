@@ -189,6 +189,10 @@ int cn_moe_combine(const float* eo, const float* wts, const int32_t* ids, const 
  * null) and hands its partial sums to a reduction across ranks. */
 int cn_moe_nvfp4_plan_create(void** plan_out, int hidden, int inter, int shared_inter, int experts, int topk, int max_tokens);
 int cn_moe_nvfp4_plan_destroy(void* plan);
+/* Where a plan keeps its rows of activations in fixed point for a grouped step (device memory of the plan; null and 0: nowhere), row by row, hidden / 256 records of
+ * 1056 bytes (f32 rows: 1440) each. A step writes those of the rows that have a resident expert; of the others no more
+ * than the first 4704 (one for every warp that makes them). Exported so that this can be checked. */
+int cn_moe_nvfp4_plan_digits(void* plan, void** records, size_t* bytes);
 int cn_moe_nvfp4_run(void* plan, const unsigned long long* table_gu, const unsigned long long* table_up,
                      const unsigned long long* table_dn, const float* gs_gu, const float* gs_up, const float* gs_dn,
                      const void* shared_gate, const void* shared_up, const void* shared_down, const float* shared_gs,

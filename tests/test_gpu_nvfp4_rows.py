@@ -1,10 +1,13 @@
 """Experts with their rows in groups (48 combos and more): k that ends in a part of a chunk, row counts that end in a part of a tile,
 groups of one, two and eight rows and what is left over, f32 and bf16 rows, the shared expert beyond eight rows."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 from crownest_b200 import CrownestError, device_status, moe, ops, synth
+from crownest_b200._lib import check, lib
 
 pytestmark = pytest.mark.gpu
 
@@ -264,6 +267,50 @@ def test_digits_made_once_are_those_made_in_each_tile(hidden, inter, rows, dtype
         plan.experts_only(w, ids, x, eo=eo)
         out.append(eo.view(torch.int32).clone())
     assert torch.equal(*out)
+    assert device_status() == 0
+
+
+def _records(plan, rows, hidden, dtype):
+    """A plan's records of `rows` rows, as a view of its memory."""
+    at, size = C.c_void_p(), C.c_size_t()
+    check(lib().cn_moe_nvfp4_plan_digits(plan.handle, C.byref(at), C.byref(size)))
+    each = hidden // 256 * (1440 if dtype == torch.float32 else 1056)
+    assert rows * each <= size.value
+
+    class View:
+        __cuda_array_interface__ = {"shape": (rows, each), "typestr": "|u1", "data": (at.value, False), "version": 3}
+    return torch.as_tensor(View(), device="cuda")
+
+
+@pytest.mark.parametrize("hidden,rows,topk", [(256, 49, 1), (768, 5000, 1), (2048, 3000, 1), (4096, 800, 9), (2560, 600, 17)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rows_that_no_resident_expert_reads_get_no_digits(hidden, rows, topk, dtype):
+    """A rank of an expert-parallel group: ids of -1 (inbox slots that nobody filled), ids beyond the experts, experts that live elsewhere. Rows with a combo of this rank are in the plan's
+    store, the others' places beyond a chunk for every warp are as they were; one, two and more rounds of the warps, picks up to eight and beyond. The results are those of a step without a
+    store."""
+    experts, held, inter = 24, 3, 256
+    rng = np.random.default_rng(rows + topk)
+
+    def matrix(n, k):
+        return torch.from_numpy(synth.nvfp4_matrix(n, k, rng)).cuda()
+
+    gu, dn = [matrix(2 * inter, hidden) for _ in range(held)], [matrix(hidden, inter) for _ in range(held)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 0.03, 0.7, gate_up=gu + [None] * (experts - held), down=dn + [None] * (experts - held), device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, topk, rows)
+    x = torch.from_numpy(rng.standard_normal((rows, hidden)).astype(np.float32)).cuda().to(dtype)
+    ids = torch.from_numpy(rng.integers(-6, experts + 4, (rows, topk)).astype(np.int32)).cuda()
+    store = _records(plan, rows, hidden, dtype)
+    store.fill_(0xA5)
+    eo = plan.experts_only(w, ids, x, eo=torch.zeros((rows * topk, hidden), device="cuda"), x_div=topk)
+    read = ((ids >= 0) & (ids < held)).any(dim=1)
+    written = (store != 0xA5).view(rows * hidden // 256, -1).any(dim=1)
+    read = read[:, None].expand(-1, hidden // 256).reshape(-1)
+    warps = min(147, -(-read.numel() // 32)) * 32
+    assert written[:warps].all() and torch.equal(written[warps:], read[warps:])
+    assert read.numel() <= 4704 or (read[4704:].any() and not read[4704:].all())
+    few = moe.GpuMoePlan(hidden, inter, experts, rows * topk, 1)  # (a store of one row)
+    again = few.experts_only(w, ids, x, eo=torch.zeros_like(eo), x_div=topk)
+    assert torch.equal(eo.view(torch.int32), again.view(torch.int32))
     assert device_status() == 0
 
 
