@@ -11,7 +11,7 @@
 //   gemv     y' = xh W_hat over a k-split: each CTA owns 8 adjacent tile columns (128 outputs) and
 //            k/(16 S) tile rows; the 768-byte run of 8 tiles per tile row arrives by 1-D bulk copy
 //            (TMA) into a shared-memory ring; warp w decodes tile column w: lane g extracts its 8
-//            states from two 32-bit windows (compile-time shifts at K = 2, 3, 3.5, 4), multiplies by 0x83DCD12D,
+//            states from one to three 32-bit windows (every bitrate has its shifts at compile time), multiplies by 0x83DCD12D,
 //            sums the bytes with dp4a (+0x6400 = the f16 pattern of 1024 + s), maps pairs through
 //            one HFMA2 to the codec's f16 weights (bit-exact) and accumulates with f16 x f16 -> f32
 //            mixed FMAs; partial sums of the k-split go to scratch
@@ -19,8 +19,10 @@
 // The first step is part of the GEMV launch for x where there are few rows (every CTA transforms its k-split) and a launch of its own for more
 // (staged_rows), and a kernel of its own, with the activation, for h; the last one carries the weighted combine of a routed step. One token, four experts
 // of 4096 x 1536: eight launches 52.5 us, five 43.4.
-// The inner loop is instruction-bound, not HBM-bound: about 6 issue slots per weight. us per step of 16 tokens, 64 experts of 4096 x 1536, top 4: K = 3 257.7 with three words a lane and two loads a
-// B operand, 249.7 with two and one; K = 3.5 480 with the words of every state looked up on their own, 290 with two windows; K = 4 439 / 256; one token at K = 2 61.9 / 41.4. Measured and not kept: pairs
+// The inner loop is instruction-bound, not HBM-bound: about 6 issue slots per weight. us per step in a graph of six, 64 experts of 4096 x 1536, top 4, the words of every state looked up on their own
+// (at K = 3: three words a lane) and two loads a B operand / so, one token and 16: K = 1 58.9 / 36.3 and 416 / 238, 1.5 58.3 / 36.7 and 429 / 246, 2 58.9 / 37.8 and 437 / 251, 2.5 59.2 / 38.6 and 422 / 246,
+// 3 40.8 / 39.0 and 258.5 / 248.2, 3.5 59.8 / 40.0 and 436 / 261, 4 59.4 / 38.2 and 425 / 239, 5 63.0 / 40.7 and 467 / 266, 6 62.9 / 41.4 and 473 / 280, 7 63.6 / 42.0 and 453 / 269, 8 63.7 / 40.1 and 472 / 262;
+// gate of 16 slots of eight rows, K = 2.5 78.9 / 48.0, K = 6 88.2 / 51.8. Measured and not kept: pairs
 // of sums put together by a multiplication in place of a byte permute (260.1 at K = 3), shifts by multiplications (270 and more): IMAD and dp4a share a pipe that is as full as the one
 // of shifts and masks. A stage is a whole 128-row block of eight tiles: with
 // four the waits and counters of a stage took a step of 16 tokens from 280 to 296 us.
@@ -214,14 +216,20 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t s0, uint32_t s1) {
     return w;
 }
 
-// A lane's eight states at a bitrate of K2 / 2 that is known at compile time. They lie in 16 + off(7) bits of the tile, which start at one of a few bits of a word: those that end within
-// the first 32 of them are cut out of the window `hi` of these, the others out of the last 32, `lw`. Where no lane starts so late that the second window goes beyond the next word (ALONE), both
-// come from the same two words; else the second has two of its own.
+// A lane's eight states at a bitrate of K2 / 2. They lie in 16 + off(7) bits of the tile, which start at one of a few bits of a word: those that end within the first 32 of them are cut out of
+// the window `hi` of these, those within the last 32 out of `lw`, and what neither has (above five bits) out of a third, `md`, that starts with the first of them. Where no lane starts so late that the second
+// window goes beyond the next word (ALONE), both come from the same two words; else each has two of its own.
 template <int K2>
 struct Rate {
     static constexpr int words = 4 * K2;  // of a tile
     __host__ __device__ static constexpr int off(int j) { return K2 % 2 == 0 ? K2 / 2 * j : j / 2 * K2 + (j & 1 ? K2 / 2 + 1 : 0); }
     static constexpr int second = off(7) > 16 ? off(7) - 16 : 0;  // first bit of `lw`
+    __host__ __device__ static constexpr int between() {          // of `md`; 0: none
+        for (int j = 0; j < 8; j++)
+            if (off(j) > 16 && off(j) < second) return off(j);
+        return 0;
+    }
+    static constexpr int third = between();
     __host__ __device__ static constexpr bool alone() {
         for (int g = 0; g < 32; g++)
             if (((4 * K2 * g + K2 / 2 - 16) & 31) + second > 32) return false;
@@ -229,7 +237,7 @@ struct Rate {
     }
     __host__ __device__ static constexpr bool fits() {
         for (int j = 0; j < 8; j++)
-            if (off(j) > 16 && off(j) < second) return false;
+            if (off(j) > 16 && off(j) < second && off(j) - third > 16) return false;
         return true;
     }
 };
@@ -239,18 +247,11 @@ __device__ __forceinline__ uint32_t field(uint32_t x) {
     return AT == 0 ? x >> 16 : (x >> (16 - AT)) & 0xffffu;
 }
 template <int K2, int J>
-__device__ __forceinline__ uint32_t state(uint32_t hi, uint32_t lw) {
+__device__ __forceinline__ uint32_t state(uint32_t hi, uint32_t md, uint32_t lw) {
     using R = Rate<K2>;
-    constexpr bool first = R::off(J) <= 16;
-    return field<first ? R::off(J) : R::off(J) - R::second>(first ? hi : lw);
-}
-// The same at any bitrate.
-__device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const int lo[8], uint32_t st[8]) {
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int i = lo[j] >> 5, o = lo[j] & 31, i1 = i + 1 == n32 ? 0 : i + 1;
-        st[j] = __funnelshift_l(tile[i1], tile[i], o) >> 16;
-    }
+    constexpr int at = R::off(J);
+    constexpr bool first = at <= 16, last = at >= R::second;
+    return field<first ? at : last ? at - R::second : at - R::third>(first ? hi : last ? lw : md);
 }
 
 // y' partials of one k-split. grid (matrices n/128, S, slots), block 288 = 8 decode warps + 1 copy warp.
@@ -259,7 +260,7 @@ __device__ __forceinline__ void lane_states(const uint32_t* tile, int n32, const
 // HAD: the input transform is part of the launch: xh = H128(x * suh) per 128-block as hi / lo planes and 1 / scale, one warp per (row, block), straight
 // into shared memory. The CTAs of one k-split repeat it (some 150 instructions a block), which costs less than a launch before this one
 // and the planes' way through memory.
-// K2: twice the bitrate where the kernel is built for it, 0: any
+// K2: twice the bitrate
 template <int K2, int MT, bool HAD>
 __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* __restrict__ ptrs, Mul1Side side_a, Mul1Side side_b, Mul1Spec sp_,
                                                         int S, int T, size_t plane, int SPC, Mul1In in) {
@@ -351,15 +352,10 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
 
-    int lo[8];
-    const int sbits = n32 * 32;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const int tpos = 8 * lane + j;
-        const int eb = !sp_.half ? (tpos + 1) * sp_.bits : ((tpos & 1) ? (tpos / 2 + 1) * (2 * sp_.bits + 1) : (tpos / 2) * (2 * sp_.bits + 1) + sp_.bits);
-        lo[j] = (eb - 16 + sbits) % sbits;
-    }
-    const int wi0 = lo[0] >> 5, sh0 = lo[0] & 31;
+    using R = Rate<K2>;
+    static_assert(R::fits(), "states that lie in no window");
+    constexpr int TW = R::words;  // words of a tile
+    const int first_bit = (4 * K2 * lane + K2 / 2 - 16 + 32 * TW) % (32 * TW), wi0 = first_bit >> 5, sh0 = first_bit & 31;
     // Multiply-accumulate on the tensor cores. The eight weights a lane decodes from a tile are the A fragment of one
     // mma.m16n8k16 as they stand (MMA row = output column g / g + 8 of the tile, MMA k = the tile's k): w01 | w45 | w23 |
     // w67. Column c of the B operand is activation row c >> 1, plane c & 1 (hi, lo), so one MMA serves four activation
@@ -378,16 +374,13 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
     float acc[NM][4], tot0[NM], tot1[NM];
 #pragma unroll
     for (int i = 0; i < NM; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = tot0[i] = tot1[i] = 0.0f;
-    // Everything a tile needs beyond its own words is a constant offset from pointers that move once per stage: where the bitrate
-    // is known a tile's words are (24 at K = 3), and a split is a whole number of stages and of 128-row blocks (tps % 8 == 0, which
-    // the launcher guarantees), so the loop carries no division, no bounds test and no address arithmetic per tile.
-    using R = Rate<K2 ? K2 : 6>;
-    static_assert(R::fits(), "states that lie in neither window");
-    constexpr int TW = K2 ? R::words : 0;  // words of a tile when known at compile time
+    // Everything a tile needs beyond its own words is a constant offset from pointers that move once per stage, and a split is a whole number of stages and of 128-row
+    // blocks (tps % 8 == 0, which the launcher guarantees), so the loop carries no division, no bounds test and no address arithmetic per tile.
     constexpr bool ALONE = R::alone();
-    const int tw = K2 ? TW : n32;
-    const int o1 = wi0 + 1 == tw ? 0 : wi0 + 1, wi1 = (wi0 + ((sh0 + R::second) >> 5)) % tw, o2 = wi1 + 1 == tw ? 0 : wi1 + 1, sh1 = ALONE ? sh0 + R::second : (sh0 + R::second) & 31;
-    const uint32_t* lane_tile = ring + (size_t)warp * tw;  // this warp's tile of the ring's first tile row
+    auto after = [](int w) { return w + 1 == TW ? 0 : w + 1; };
+    const int o1 = after(wi0), wi1 = (wi0 + ((sh0 + R::second) >> 5)) % TW, o2 = after(wi1), sh1 = ALONE ? sh0 + R::second : (sh0 + R::second) & 31;
+    const int wi2 = (wi0 + ((sh0 + R::third) >> 5)) % TW, o3 = after(wi2), sh2 = (sh0 + R::third) & 31;
+    const uint32_t* lane_tile = ring + (size_t)warp * TW;  // this warp's tile of the ring's first tile row
     int s = 0, cs = 0, spi = 0;
     uint32_t ph = 0;
     for (int c = 0; c < nst; c++) {
@@ -395,23 +388,17 @@ __global__ void __launch_bounds__(288, 4) mul1_gemv_kernel(unsigned long long* _
             cn_dev_fail(CN_DEV_WAIT_FULL);
             return;
         }
-        const uint32_t* tb = lane_tile + (size_t)s * (UROWS * 8) * tw;
+        const uint32_t* tb = lane_tile + (size_t)s * (UROWS * 8) * TW;
         const int kx = (spi * tps + cs * UROWS) * 16;  // first k of the stage within the staged activations
 #pragma unroll
         for (int u = 0; u < UROWS; u++) {
-            uint32_t st[8];
-            if (K2) {
-                const uint32_t* tl = tb + u * 8 * TW;
-                const uint32_t w0 = tl[wi0], w1 = tl[o1];
-                // (a shift of 32 is the second word itself)
-                const uint32_t hi = __funnelshift_l(w1, w0, sh0), lw = R::second == 0 ? hi : ALONE ? __funnelshift_lc(w1, w0, sh1) : __funnelshift_l(tl[o2], tl[wi1], sh1);
-                st[0] = state<R::words / 4, 0>(hi, lw), st[1] = state<R::words / 4, 1>(hi, lw), st[2] = state<R::words / 4, 2>(hi, lw), st[3] = state<R::words / 4, 3>(hi, lw);
-                st[4] = state<R::words / 4, 4>(hi, lw), st[5] = state<R::words / 4, 5>(hi, lw), st[6] = state<R::words / 4, 6>(hi, lw), st[7] = state<R::words / 4, 7>(hi, lw);
-            } else {
-                lane_states(tb + (size_t)u * 8 * tw, n32, lo, st);
-            }
-            const uint32_t w01 = mul1_pair(st[0], st[1]), w23 = mul1_pair(st[2], st[3]);
-            const uint32_t w45 = mul1_pair(st[4], st[5]), w67 = mul1_pair(st[6], st[7]);
+            const uint32_t* tl = tb + u * 8 * TW;
+            const uint32_t w0 = tl[wi0], w1 = tl[o1];
+            // (a shift of 32 is the second word itself)
+            const uint32_t hi = __funnelshift_l(w1, w0, sh0), lw = R::second == 0 ? hi : ALONE ? __funnelshift_lc(w1, w0, sh1) : __funnelshift_l(tl[o2], tl[wi1], sh1);
+            const uint32_t md = R::third == 0 ? hi : __funnelshift_l(tl[o3], tl[wi2], sh2);
+            const uint32_t w01 = mul1_pair(state<K2, 0>(hi, md, lw), state<K2, 1>(hi, md, lw)), w23 = mul1_pair(state<K2, 2>(hi, md, lw), state<K2, 3>(hi, md, lw));
+            const uint32_t w45 = mul1_pair(state<K2, 4>(hi, md, lw), state<K2, 5>(hi, md, lw)), w67 = mul1_pair(state<K2, 6>(hi, md, lw), state<K2, 7>(hi, md, lw));
 #pragma unroll
             for (int i = 0; i < NM; i++) {
                 const uint2 xr = *(const uint2*)(xb[i] + kx + u * 16);
@@ -652,7 +639,7 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     const size_t smem = 128 + (size_t)RING * UROWS * 32 * s.n32 + (size_t)2 * T * (rows + XPAD) * 2 + 8 + (size_t)T * (rows / 128) * 4;
     dim3 grid(mats * (s.n / 128), S / spc, slots);
     if (smem > most) CN_FAIL(CN_ERR_LIMIT, "mul1 gemv: %zu B of shared memory per block", smem);
-    const int rate = 2 * s.bits + (s.half ? 1 : 0), k2 = rate == 4 || rate == 6 || rate == 7 || rate == 8 ? rate : 0;
+    const int k2 = 2 * s.bits + (s.half ? 1 : 0);
     const int mt = T == 1 ? 1 : (T == 2 ? 2 : (T <= 4 ? 4 : 8));
     const Mul1In none = {};
 #define CN_MUL1_CASE(K2V, MTV, HADV)                                                                                                \
@@ -662,7 +649,8 @@ int launch_gemv(const unsigned long long* ptrs, const Mul1Side& sa, const Mul1Si
     }
 #define CN_MUL1_CASES(K2V) CN_MUL1_CASE(K2V, 1, true) CN_MUL1_CASE(K2V, 2, true) CN_MUL1_CASE(K2V, 4, true) CN_MUL1_CASE(K2V, 8, true) \
     CN_MUL1_CASE(K2V, 1, false) CN_MUL1_CASE(K2V, 2, false) CN_MUL1_CASE(K2V, 4, false) CN_MUL1_CASE(K2V, 8, false)
-    CN_MUL1_CASES(0) CN_MUL1_CASES(4) CN_MUL1_CASES(6) CN_MUL1_CASES(7) CN_MUL1_CASES(8)
+    CN_MUL1_CASES(2) CN_MUL1_CASES(3) CN_MUL1_CASES(4) CN_MUL1_CASES(5) CN_MUL1_CASES(6) CN_MUL1_CASES(7) CN_MUL1_CASES(8) CN_MUL1_CASES(10) CN_MUL1_CASES(12) CN_MUL1_CASES(14)
+    CN_MUL1_CASES(16)
 #undef CN_MUL1_CASES
 #undef CN_MUL1_CASE
     CN_CUDA(cudaGetLastError());

@@ -69,11 +69,11 @@ def test_gemv_matches_the_cpu_reference(K, hidden, inter, t):
     plan.free()
 
 
-@pytest.mark.parametrize("K", [1.0, 1.5, 2.0, 2.5, 3.0, 3.5, 4.0, 5.0, 8.0])
+@pytest.mark.parametrize("K", [1.0, 1.5, 2.0, 2.5, 3.0, 3.5, 4.0, 5.0, 6.0, 7.0, 8.0])
 @pytest.mark.parametrize("t", [1, 2, 4, 7])
 @pytest.mark.parametrize("slots", [1, 520])
 def test_every_bitrate_at_every_row_count(K, t, slots):
-    """Rates whose states come out of windows known at compile time (2, 3, 3.5, 4) and the others, each with its words of a tile and the lane whose window goes round the tile's end; rows
+    """Rates whose states come out of one window of the bit stream, of two from the same words or from words of their own, and of three, each with the lane whose window goes round the tile's end; rows
     transformed inside the GEMV (few slots) and staged by a launch of their own (many; the rows of the last slots are looked at). The other records are null."""
     hidden, inter = 768, 512
     rec = tk.mul1_record(int(2 * K) + t, hidden, inter, K)
