@@ -52,9 +52,9 @@ def test_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
     assert device_status() == 0
 
 
-# bf16: the smallest matrices that come here: 74 tiles, 64 of few chunks, 40 of two chunks, long rows (gate / up: pairs of rows count twice)
-@pytest.mark.parametrize("rows,k,gu", [(9345, 512, False), (8065, 1024, False), (4993, 512, False), (1400, 5120, False), (520, 8192, False), (4673, 512, True), (4065, 1024, True),
-                                       (260, 8192, True)])
+# bf16: the smallest matrices that come here: 74 tiles, 64 of four to six chunks, 40 of one to three, long rows (gate / up: pairs of rows count twice, and 74 up to three chunks)
+@pytest.mark.parametrize("rows,k,gu", [(9345, 1792, False), (8065, 1024, False), (8065, 1536, False), (4993, 256, False), (4993, 512, False), (4993, 768, False), (1400, 5120, False),
+                                       (520, 8192, False), (4673, 256, True), (4673, 512, True), (4673, 768, True), (4065, 1024, True), (260, 8192, True)])
 @pytest.mark.parametrize("m", [1, 3, 8])
 def test_smallest_matrices_of_the_rule(rows, k, gu, m):
     rng, g, g64 = _make(rows, k, rows + k)
