@@ -61,19 +61,17 @@ static int encode_map(CUtensorMap* map, CUtensorMapDataType type, unsigned rank,
     return CN_OK;
 }
 
-int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
-               unsigned box_cols, unsigned box_rows) {
-    const CUtensorMapDataType type = elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : elem == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_cols, box_rows};
-    return encode_map(map, type, 2, base, dims, strides, box, elem == 4 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B);
+int cn_tmap_words(CUtensorMap* map, const void* base, unsigned long long words, unsigned long long rows, unsigned box_words, unsigned box_rows) {
+    const cuuint64_t dims[2] = {words, rows}, strides[1] = {words * 4};
+    const cuuint32_t box[2] = {box_words, box_rows};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-int cn_tmap_blocks(CUtensorMap* map, const void* base, int elem, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
+int cn_tmap_blocks(CUtensorMap* map, const void* base, bool bf16, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
                    unsigned box_blocks) {
     const cuuint64_t dims[3] = {64, rows, blocks}, strides[2] = {row_bytes, 128};
     const cuuint32_t box[3] = {64, box_rows, box_blocks};
-    return encode_map(map, elem == 3 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    return encode_map(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 extern "C" const char* cn_last_error_string(void) { return t_err; }

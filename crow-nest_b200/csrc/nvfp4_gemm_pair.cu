@@ -549,8 +549,8 @@ int cn_gemm_pair_launch(const GemmCall& c, cudaStream_t stream) {
     p.row_tiles = (c.rows + 255) / 256;
     p.tiles = p.row_tiles * ((c.m + p.tn - 1) / p.tn);
     if (!c.packed)
-        if (int rc = cn_tmap_2d(&wmap, c.w, 4, (unsigned long long)nk * 9, c.rows, (unsigned long long)nk * 36, 36, 128)) return rc;
-    if (int rc = cn_tmap_blocks(&xmap, c.x, c.x_f16 ? 2 : 3, nk, c.m, (unsigned long long)c.k * 2, p.tn / 2, box)) return rc;
+        if (int rc = cn_tmap_words(&wmap, c.w, (unsigned long long)nk * 9, c.rows, 36, 128)) return rc;
+    if (int rc = cn_tmap_blocks(&xmap, c.x, !c.x_f16, nk, c.m, (unsigned long long)c.k * 2, p.tn / 2, box)) return rc;
     const size_t smem = HDR + 1024 + (size_t)p.nws * W_STAGE + (size_t)p.nb * bslot;
     const int units = p.tiles * p.ksplits, grid = 2 * (units < PAIRS ? units : PAIRS);
     int rc = CN_ERR_SHAPE;

@@ -833,8 +833,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // has a single team; and 22 for meeting in the first CTA, 44 for four. A CTA of two teams comes before two CTAs (us of the two, two / four rows: 17408 x
     // 5120 gate / up 27.3 / 30.2 and 27.4 / 31.0, 7168 x 5120 8.5 / 9.8 and 9.3 / 11.1, 3000 x 9216 8.6 / 10.0 and 9.6 / 11.8; eight rows of gate / up
     // 46.6, one team 59.6), but not in clusters of four, which fill the SMs of a GPC badly with one CTA each (640 x 17408 10.3 / 12.0 and
-    // 6.8 / 8.3), nor where tiles are short (two rows of 20246 x 1536 10.1 and 9.2,
-    // eight of 248000 x 2048 154 and 147). Eight rows in two teams spill 20 to 44 bytes a thread (18 warps leave each 96 registers); the figure
+    // 6.8 / 8.3), nor where tiles are short (two rows of 20246 x 1536 10.1 and 9.2). Eight rows in two teams spill 20 to 44 bytes a thread (18 warps leave each 96 registers); the figure
     // for eight rows above has that in it. 5120 x 17408, two, four and eight rows: 18.6 / 21.3 / 34.8 in clusters of two; 22.0 / 26.7 / 53.1 with
     // parts one after another and a single team.
     int ksplit = mt == 1 ? parts : 1, teams = 1, waves = 1;
@@ -844,7 +843,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
         for (int ks = 1; ks <= parts; ks *= 2) {
             if (ks > 1 && (long long)ROWS * (bpr / ks) * 36 < 32 * 1024) continue;
             const int n = parts / ks;
-            const bool ctas = ks == 4 || (tx == 16 && mt < 8) || (mt == 8 && gap(n) == 1 && ntiles > 8 * 148);
+            const bool ctas = ks == 4 || (tx == 16 && mt < 8);
             for (int f = 0; f < 3; f++) {
                 const int form = !ctas && f < 2 ? 1 - f : f;  // 0: two CTAs per SM, 1: one of two teams, 2: one of one
                 const int c = form == 0 ? 2 : 1, nt = form == 1 ? 2 : 1, per_sm = c * nt, clusters = 148 * c / ks * nt, wv = (ntiles + clusters - 1) / clusters;
@@ -950,7 +949,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     if (tx == TXV && cps == CPSV && mt == MTV && teams == 1) return launch_m1<TXV, CPSV, MTV>(cfg, p);
     CN_M1_CASE(32, 2, 1) CN_M1_CASE(32, 3, 1) CN_M1_CASE(16, 4, 1)
     CN_M1_CASE(32, 1, 2) CN_M1_CASE(32, 1, 4) CN_M1_CASE(32, 1, 8)
-    CN_M1_CASE(16, 2, 2) CN_M1_CASE(16, 2, 4) CN_M1_CASE(16, 2, 8)
+    CN_M1_CASE(16, 2, 2) CN_M1_CASE(16, 2, 4)
     if (tx == 16 && teams == 2 && mt == 8) return launch_m1<16, 1, 8, 1, false, 1, 2>(cfg, p);
 #undef CN_M1_CASE
     CN_FAIL(CN_ERR_SHAPE, "%s: no kernel for %d blocks per stage, %d CTAs per SM, %d rows", who, tx, cps, mt);

@@ -596,10 +596,10 @@ int cn_gemv_tc_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
 #endif
     CUtensorMap map0, map1;
     const unsigned long long row_bytes = (unsigned long long)nk * 144;
-    if (int rc = cn_tmap_2d(&map0, a.w0, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, (unsigned)per_tile)) return rc;
+    if (int rc = cn_tmap_words(&map0, a.w0, row_bytes / 4, (unsigned long long)a.rows, 36, (unsigned)per_tile)) return rc;
     if (!gu)
         map1 = map0;
-    else if (int rc = cn_tmap_2d(&map1, a.w1, 4, row_bytes / 4, (unsigned long long)a.rows, row_bytes, 36, 64))
+    else if (int rc = cn_tmap_words(&map1, a.w1, row_bytes / 4, (unsigned long long)a.rows, 36, 64))
         return rc;
     // A CTA asks for half of an SM's shared memory, as of its tensor memory: as many of these kernels (or of nvfp4_rows_tc.cu's) as fit an SM find tensor memory there. The pair
     // GEMM, which takes all of it, stands apart by its registers: 640 threads of 72 leave no room for 448 of 64.

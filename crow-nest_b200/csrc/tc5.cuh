@@ -5,15 +5,12 @@
 
 #include "common.cuh"
 
-// ---------------------------------------------------------------- host: 2-D tensor maps
-// A row-major matrix of `rows` rows, `row_bytes` apart (a multiple of 16), read in boxes of box_cols elements x box_rows
-// rows; elements beyond the matrix read as zero. elem: 2 = f16, 3 = bf16, 128-byte swizzle (the K-major operand tile of an MMA),
-// 4 = 32-bit, no swizzle (NVFP4 container bytes).
-int cn_tmap_2d(CUtensorMap* map, const void* base, int elem, unsigned long long cols, unsigned long long rows, unsigned long long row_bytes,
-               unsigned box_cols, unsigned box_rows);
-// A row-major matrix of 16-bit values (elem 2 or 3) as blocks of 64 columns: coordinates (column of a block, row, block), boxes of box_rows rows and box_blocks blocks, each block
-// the operand tile that a 2-D box of it would be.
-int cn_tmap_blocks(CUtensorMap* map, const void* base, int elem, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
+// ---------------------------------------------------------------- host: tensor maps (elements beyond the matrix read as zero)
+// Rows of `words` 32-bit words (a multiple of four) one after another, in boxes of box_words words x box_rows rows, no swizzle: NVFP4 container bytes.
+int cn_tmap_words(CUtensorMap* map, const void* base, unsigned long long words, unsigned long long rows, unsigned box_words, unsigned box_rows);
+// A row-major matrix of 16-bit values (bf16 or f16), rows row_bytes apart (a multiple of 16), as blocks of 64 columns: coordinates (column of a block, row, block), boxes of box_rows rows
+// and box_blocks blocks with 128-byte swizzle, each block a K-major operand tile of an MMA.
+int cn_tmap_blocks(CUtensorMap* map, const void* base, bool bf16, unsigned long long blocks, unsigned long long rows, unsigned long long row_bytes, unsigned box_rows,
                    unsigned box_blocks);
 
 // ---------------------------------------------------------------- device: TMA and clusters
