@@ -84,33 +84,38 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
 constexpr int LONG_RUN = 64;
 __device__ __forceinline__ bool resident(int e, const unsigned long long* __restrict__ tab, int E) { return e >= 0 && e < E && !(tab && tab[e] == 0ull); }
 // Records of the chunks of activations, by warp `w` of `warps`. Rows none of whose combos has a resident expert are left out, since nothing reads them and most inbox slots of an
-// expert-parallel rank are such rows: one rank of eight, 512 experts of 2048 x 512, top 10, 64 tokens a rank (620 of 5120 slots in use), routed experts 88.7 -> 78.4 us. A lane looks one of the
-// warp's chunks up, the ids and then the entries of eight combos at a time. The first chunk of a warp is made without a look: up to a chunk for every warp they are made beside
+// expert-parallel rank are such rows: one rank of eight, 512 experts of 2048 x 512, top 10, 64 tokens a rank (620 of 5120 slots in use), routed experts 88.0 -> 76.5 us. A lane looks one of the
+// warp's chunks up, the ids and then the entries of four combos at a time. The first chunk of a warp is made without a look: up to a chunk for every warp they are made beside
 // the grouping on SMs that have nothing else to do, and two more trips to memory in front of them show (160 slots 23.0 -> 23.3 us).
+// (a function of its own: inlined into the loop of put_records the kernel has 56 registers, not 40, and a block of it an SM to itself; seven tokens of 128 experts of 2560 x 768, top 6, 43.1 us, 42.7 so)
+template <bool F32>
+__device__ __noinline__ void one_record(const char* x, int lane, uint8_t* rec) {
+    ChunkValues<F32> v;
+    v.load(x, lane);
+    put_record<F32>(v, lane, rec);
+}
 template <bool F32>
 __device__ __forceinline__ void put_records(const DigitsCall& dc, const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E, int w, int warps, int lane) {
     const char* x = (const char*)dc.x;
     constexpr size_t BYTES = 256 * (F32 ? 4 : 2);
     for (int i0 = w; i0 < dc.chunks; i0 += 32 * warps) {
-        ChunkValues<F32> v;
-        v.load(x + i0 * BYTES, lane);
         const int at = i0 + lane * warps;
         bool read = at == w;
         if (!read && at < dc.chunks) {
             const int c0 = at / dc.row_chunks * dc.x_div, c1 = min(c0 + dc.x_div, n);
-            for (int c = c0; c < c1 && !read; c += 8) {
-                int e[8];
+#pragma unroll 1
+            for (int c = c0; c < c1 && !read; c += 4) {
+                int e[4];
 #pragma unroll
-                for (int j = 0; j < 8; j++) e[j] = c + j < c1 ? ids[c + j] : -1;
+                for (int j = 0; j < 4; j++) e[j] = c + j < c1 ? ids[c + j] : -1;
 #pragma unroll
-                for (int j = 0; j < 8; j++) read |= resident(e[j], tab, E);
+                for (int j = 0; j < 4; j++) read |= resident(e[j], tab, E);
             }
         }
+#pragma unroll 1
         for (uint32_t todo = __ballot_sync(0xffffffffu, read); todo; todo &= todo - 1u) {
-            const int j = __ffs(todo) - 1;
-            const size_t i = (size_t)(i0 + j * warps);
-            if (j > 0) v.load(x + i * BYTES, lane);
-            put_record<F32>(v, lane, dc.out + i * digit_record(F32));
+            const size_t i = (size_t)(i0 + (__ffs(todo) - 1) * warps);
+            one_record<F32>(x + i * BYTES, lane, dc.out + i * digit_record(F32));
         }
     }
 }
@@ -267,7 +272,7 @@ constexpr int GROUP_COMBOS = 48, GROUP_LEAST = 16;
 bool groups_rows(int combos, int hidden, int inter, bool f32) {
     return combos >= GROUP_COMBOS || (combos >= (f32 ? GROUP_LEAST : 24) && (long long)combos * hidden * inter >= (f32 ? 47000000 : 80000000));
 }
-// Blocks of the grouping kernel that make records at most: one to an SM (1024 threads of 56 registers) beside the one that groups.
+// Blocks of the grouping kernel that make records at most: one to an SM (1024 threads of 40 registers) beside the one that groups.
 constexpr int DIGIT_BLOCKS = 148 - 1;
 // Bytes of a plan's store of digits at most.
 constexpr size_t DIGITS_MOST = (size_t)64 << 20;
