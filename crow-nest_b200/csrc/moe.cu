@@ -265,12 +265,14 @@ __global__ void moe_combine_kernel(const float* __restrict__ eo, const float* __
 }
 
 // Combos from which the routed step groups the rows of an expert (measured: see routed_experts), and fewer of larger experts: one by one, each combo streams its expert, and f32 rows take CUDA
-// cores. us per step one by one / grouped: 288 experts of 4096 x 2048, top 8, 3 tokens 93.5 / 87, 5 tokens 136 / 114, f32 2 tokens 93 / 75, 5 tokens 191 / 120; 128 of 2560 x 1280, top 6,
-// 4 tokens 55.7 / 55.7, 7 tokens 81 / 73, f32 3 tokens 66 / 53, 7 tokens 106 / 75; 512 of 2048 x 768, top 10, 4 tokens 51 / 54, f32 3 tokens 53.6 / 50.9; 64 of 1024 x 1280, top 8, f32 5 tokens
-// 59 / 41.5; 512 of 2048 x 512, top 10, 4 tokens 35.5 / 49, f32 45 / 50.
+// cores. The line is where grouping is no slower with or without a shared expert, in combos x hidden x inter. us per step without / with one of 512, one by one / grouped, f32 rows: 31.5 M (30 combos of 2048 x 512, 512
+// experts) 29.9 / 30.9 and 30.9 / 34.2, 37.7 M (36) 31.9 / 30.5 and 38.1 / 39.4, 41.9 M (40) 37.4 / 35.7 and 39.3 / 39.1, 41.9 M (32 of 2560 x 512) 35.5 / 34.0 and 39.3 / 39.0, 47.2 M (30 of 2048 x 768) 47.6 / 37.5 and
+// 47.3 / 39.5, 52.4 M (40 of 1024 x 1280, 64 experts) 53.6 / 33.9 and 61.1 / 39.2. bf16 rows: 62.9 M (40 of 2048 x 768) 36.9 / 40.9 and 40.0 / 42.3, 70.8 M (36 of 2560 x 768, 128 experts) 39.1 / 41.0 and 47.5 / 48.1, 78.6 M
+// (30 of 2048 x 1280, 64 experts) 40.8 / 41.4 and 47.0 / 46.2, 82.6 M (42 of 2560 x 768) 43.7 / 42.9 and 51.6 / 50.0, 98.3 M (30 of 2560 x 1280) 50.1 / 46.5 and 56.6 / 54.0; 16 combos of 4096 x 2048 (134 M) 56.5 / 61.6 and 58.2 / 63.1.
+// A rank that holds an eighth of the experts gains more, since dead combos are in no group: 24 combos of 4096 x 2048, three of them live, 44.9 / 31.7, f32 36.1 / 31.6; 16 of f32 29.2 / 28.2.
 constexpr int GROUP_COMBOS = 48, GROUP_LEAST = 16;
 bool groups_rows(int combos, int hidden, int inter, bool f32) {
-    return combos >= GROUP_COMBOS || (combos >= (f32 ? GROUP_LEAST : 24) && (long long)combos * hidden * inter >= (f32 ? 47000000 : 80000000));
+    return combos >= GROUP_COMBOS || (combos >= (f32 ? GROUP_LEAST : 24) && (long long)combos * hidden * inter >= (f32 ? 40000000 : 80000000));
 }
 // Blocks of the grouping kernel that make records at most: one to an SM (1024 threads of 40 registers) beside the one that groups.
 constexpr int DIGIT_BLOCKS = 148 - 1;

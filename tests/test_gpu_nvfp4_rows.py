@@ -63,6 +63,14 @@ def test_fewer_combos_of_large_experts_against_64_bits(tokens, dtype):
     test_grouped_experts_against_64_bits(4096, 2048, 3, 2, tokens, 256, dtype)
 
 
+# ... and with as many combos x hidden x inter as it takes (40 M of f32 rows: 19 and 20 tokens; 80 M of bf16 rows: 15 and 16)
+@pytest.mark.parametrize("hidden,inter,topk,tokens,dtype", [(2048, 512, 2, 19, torch.float32), (2048, 512, 2, 20, torch.float32), (2048, 1280, 2, 15, torch.bfloat16),
+                                                            (2048, 1280, 2, 16, torch.bfloat16)])
+@pytest.mark.parametrize("shared", [0, 512])
+def test_either_side_of_the_grouping_line_against_64_bits(hidden, inter, topk, tokens, dtype, shared):
+    test_grouped_experts_against_64_bits(hidden, inter, 5, topk, tokens, shared, dtype)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [56, 64, 125])
 def test_full_groups_repeat_bit_for_bit(tokens, dtype):
