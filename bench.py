@@ -274,6 +274,21 @@ MOE_SHAPES = {"moe": "hidden 2048, 512 experts, inter 512, shared expert 512, so
               "mul1": "hidden 4096, 64 experts, inter 1536, top-4, EXL3 MUL1 K=3"}
 
 
+def graph_kernels(graph):
+    """Kernels of a captured graph (kept with keep_graph=True), counted node by node."""
+    import ctypes as C
+    rt, n, kind = C.CDLL("libcudart.so.12"), C.c_size_t(), C.c_int()
+    raw = C.c_void_p(graph.raw_cuda_graph())
+    assert rt.cudaGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert rt.cudaGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    kernels = 0
+    for node in nodes:
+        assert rt.cudaGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        kernels += kind.value == 0  # cudaGraphNodeTypeKernel
+    return kernels
+
+
 def moe_measure(kind, tokens, rank, world, local, steps, warmup, cpu=False, e2e=True):
     """One routed-expert decode configuration: `tokens` rows per rank, experts spread over the ranks (all-to-all dispatch
     and return over peer memory when world > 1). Returns the figures of one block of the JSON line (rank 0) or None."""
@@ -288,9 +303,11 @@ def moe_measure(kind, tokens, rank, world, local, steps, warmup, cpu=False, e2e=
     with torch.cuda.stream(st):
         wl.step()
         st.synchronize()
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(graph, stream=st):
             wl.step()
+    launches = graph_kernels(graph)
+    graph.instantiate()
     torch.cuda.synchronize()
     tm = Timer(world)
     t = tm.run(graph.replay, steps, warmup)
@@ -329,7 +346,7 @@ def moe_measure(kind, tokens, rank, world, local, steps, warmup, cpu=False, e2e=
                "roofline": {"bound": "hbm", "achieved": gbs / world, "peak": peak, "unit": "GB/s", "frac": gbs / world / peak, "peak_kind": peak_kind,
                             "scope": "per GPU", "kernel": "mul1_gemv_kernel" if kind != "moe" else "nvfp4_rows_tc_kernel" if tokens * wl.topk >= 48 else "nvfp4_gemv_m1_kernel (routed form)"},
                "parallelism": f"ep{world}: all-to-all dispatch / return over peer memory" if world > 1 else "none",
-               "launches_per_step": wl.launches_per_step, "device_status": status}
+               "launches_per_step": launches, "device_status": status}
         if e2e_s is not None:
             out["e2e_tok_s"] = tokens * world / e2e_s
             out["h2d_bytes_per_step"] = x_host.numel() * 2

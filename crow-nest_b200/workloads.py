@@ -51,10 +51,6 @@ class MoeDecode:
             self.ep = EpExchange(tokens, topk, hidden, experts, rank, world, device, group)
             # the rows a rank receives are one combo each: a second plan with top-1 geometry over all inbox slots
             self.plan_in = moe.GpuMoePlan(hidden, inter, experts, 1, max_tokens=self.ep.slots)
-        # router, gate/up and down (grouped from 48 combos on: one more), the shared expert's two, combine; sort, dispatch, targets and return
-        # of the exchange
-        combos = tokens * topk if world == 1 else self.ep.slots
-        self.launches_per_step = 6 + (1 if combos >= 48 else 0) + (4 if world > 1 else 0)
 
     def step(self):
         """One decode step over this rank's tokens; returns y [tokens][hidden] bf16."""
@@ -117,10 +113,6 @@ class Mul1MoeDecode:
         if world > 1:
             self.ep = EpExchange(tokens, topk, hidden, experts, rank, world, device, group)
             self.eo = torch.empty((self.ep.slots, hidden), dtype=torch.float32, device=device)
-        # router, records (two launches when grouped: two combos for every expert and more), Hadamard in, gate and up, activation, down,
-        # Hadamard out, combine; sort, dispatch, targets and return of the exchange
-        combos = tokens * topk if world == 1 else self.ep.slots
-        self.launches_per_step = 8 + (1 if 2 * combos >= experts else 0) + (4 if world > 1 else 0)
 
     def step(self):
         ids, wts = moe.route_softmax_topk(self.logits, self.topk)

@@ -187,3 +187,20 @@ def test_grouped_experts_with_f32_rows_and_short_rows(hidden, inter, experts, k,
     from crownest_b200 import device_status
     assert device_status() == 0
     plan.free()
+
+
+@pytest.mark.parametrize("kind,tokens,kernels", [("moe", 1, 3), ("moe", 4, 3), ("moe", 64, 7), ("mul1", 1, 5), ("mul1", 16, 8)])
+def test_benchmark_counts_the_kernels_of_a_captured_step(kind, tokens, kernels):
+    """NVFP4: router, gate / up and down + combine in a small step; router, grouping, two for the experts, two for the shared expert and the combine in a grouped one. MUL1: router, gate / up,
+    activation, down, output + combine; sorting, slots and the input transform more with sixteen tokens."""
+    import bench
+    from crownest_b200 import workloads
+    wl = (workloads.MoeDecode if kind == "moe" else workloads.Mul1MoeDecode)(tokens, device="cuda", experts=64)
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        wl.step()
+        st.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph, stream=st):
+            wl.step()
+    assert bench.graph_kernels(graph) == kernels
