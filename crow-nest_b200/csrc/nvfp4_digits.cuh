@@ -202,7 +202,7 @@ __device__ __forceinline__ double power_of_two(float f) { return __hiloint2doubl
 // ---------------------------------------------------------------- container blocks -> operand layout (a lane: the four blocks of a row)
 constexpr int A_COLS = 32, A_SCALES = 4 * 512;  // a chunk of 128 rows as operand A: columns of tensor memory with its codes, bytes of the four MMAs' scales
 
-// A row's 144 bytes at src into registers, scale bytes as the tensor core is to read them; which lanes' rows have one of 0xFF: that stands for 480, which it does not know, and is
+// A row's 144 bytes at src into registers, scale bytes as the tensor core is to read them; whether any row of the warp has one of 0xFF: that stands for 480, which it does not know, and is
 // nothing here (`whole_blocks` multiplies the block out).
 __device__ __forceinline__ uint32_t load_row(const uint4* src, uint32_t (&v)[36]) {
 #pragma unroll
@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t load_row(const uint4* src, uint32_t (&v)[36]
     uint32_t odd = 0u;
 #pragma unroll
     for (int b = 0; b < 4; b++) odd |= v[9 * b] & ((v[9 * b] & 0x7f7f7f7fu) + 0x01010101u);
-    odd = __ballot_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
+    odd = __any_sync(0xffffffffu, (odd & 0x80808080u) != 0u);
 #pragma unroll
     for (int b = 0; b < 4; b++) {
         const uint32_t sc = v[9 * b];

@@ -45,7 +45,8 @@ constexpr int FS_OFF = 512, WF_OFF = 1536, HEADER = 2048;  // barriers; chunk fa
 __host__ __device__ constexpr int ncol(int mt, bool f32) { return (mt * digits_of(f32) + 15) / 16 * 16; }  // columns of the MMA
 __host__ __device__ constexpr int b_codes(int mt, bool f32) { return ncol(mt, f32) * 128; }
 __host__ __device__ constexpr int b_stage(int mt, bool f32) { return b_codes(mt, f32) + 4 * 512; }
-// chunks of digits (us with two / four: four rows of gate / up 17408 x 5120 22.0 / 21.6, eight 31.6 / 30.7; where they fit beside three container stages)
+// chunks of digits (us with two / four: four rows of gate / up 17408 x 5120 22.0 / 21.6, eight 31.6 / 30.7). They leave room for three container stages or four, but for two where eight rows of either type
+// have the sums of three tiles on their way
 __host__ __device__ constexpr int nb_of(int mt, bool f32) { return mt == 8 && f32 ? 2 : 4; }
 // accumulators, in half of an SM's tensor memory beside the codes of two chunks and the scales: those of two chunks where they fit (all but eight f32 rows)
 constexpr int TMEM = 256, TM_FIXED = NA * A_COLS + 64;

@@ -182,7 +182,7 @@ def test_scale_bytes_that_the_tensor_core_reads_differently():
 @pytest.mark.parametrize("gu", [False, True])
 @pytest.mark.parametrize("m,dtype", [(1, torch.bfloat16), (8, torch.bfloat16), (4, torch.float32), (8, torch.float32)])
 def test_one_row_of_a_tile_with_such_scale_bytes(gu, m, dtype):
-    """Row t of tile t alone has 0xFF: the lane that meets it and the thread that sums the row are in different warps."""
+    """Row t of tile t alone has 0xFF, so every lane of every weight warp meets one, and the adding warp of the same rows learns of it by the warp's word."""
     per = 64 if gu else 128
     rng, g, _ = _make(per * per, 1024, 11)
     sel = torch.arange(per, device="cuda") * (per + 1)
