@@ -332,6 +332,21 @@ int launch_m(const GemvParams& p, int mp, int rt, int grid, int gy, size_t smem,
 
 }  // namespace
 
+// f32 activations on the fifth-generation tensor cores where a row is long, a matrix large, or a row no whole number of this kernel's steps of 512 values. us a call in a stream of
+// dependent ones, there / here for one and eight rows: 12288 x 512 3.0 / 3.4 and 5.7 / 12.6, 8192 x 512 2.9 / 3.1 and 5.4 / 6.4, 4096 x 512 2.8 / 2.3 and 5.0 / 6.0, 2048 x 1024 3.4 / 2.4 and 5.3 / 6.8,
+// 256 x 1792 3.2 / 5.3 and 5.4 / 14.7, 256 x 1280 3.2 / 4.1 and 5.5 / 11.4, 256 x 768 3.0 / 3.0 and 5.6 / 8.1; gate / up of 256 x 1280 3.5 / 4.2 and 5.6 / 12.2, of 256 x 768 3.5 / 3.1 and
+// 7.4 / 8.8. Against 64 bits a row is 2.7e-8 off there, 1.0e-7 here (normally distributed rows, SiLU rows, cubes, a few channels of a hundred times the rest); where
+// three and more of a block's sixteen values are 1e4 times the others and meet zero weights, 3e-6 there, 9e-8 here. The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
+// A rule of the matrix alone: a row's result does not depend on how many rows the call has.
+static bool f32_digits(int rows, int k, bool gu) {
+    const bool odd_steps = k % 512 != 0 && (k >= 1280 || (k >= 768 && rows >= 64 && !gu));
+    return k >= 2048 || odd_steps || (k >= 512 && rows >= 8192 && !gu) || (long long)rows * k * (gu ? 2 : 1) >= 6000000;
+}
+extern "C" int cn_nvfp4_gemv_fixed_bits(int rows, int k, int gate_up, int dtype) {
+    if (rows < 1 || k < 256 || k % 256 != 0) return 0;
+    return dtype == CN_F32 ? (f32_digits(rows, k, gate_up != 0) ? 31 : 0) : dtype == CN_BF16 && cn_gemv_bf16_digits(rows, k, gate_up != 0) ? 22 : 0;
+}
+
 // One launch of the GEMV family (declared in nvfp4_gemv.cuh for the MoE operator).
 int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int rows = a.rows, k = a.k, m = a.m;
@@ -346,13 +361,7 @@ int cn_gemv_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     // bf16 activations: the tensor-core kernel
     if (a.dtype == CN_BF16) return cn_gemv_m1_launch(a, stream, who);
     if (a.line_bases) CN_FAIL(CN_ERR_SHAPE, "%s: line output takes bf16 activations", who);
-    // f32 activations on the fifth-generation tensor cores where a row is long, a matrix large, or a row no whole number of this kernel's steps of 512 values. us a call in a stream of
-    // dependent ones, there / here for one and eight rows: 12288 x 512 3.0 / 3.4 and 5.7 / 12.6, 8192 x 512 2.9 / 3.1 and 5.4 / 6.4, 4096 x 512 2.8 / 2.3 and 5.0 / 6.0, 2048 x 1024 3.4 / 2.4 and 5.3 / 6.8,
-    // 256 x 1792 3.2 / 5.3 and 5.4 / 14.7, 256 x 1280 3.2 / 4.1 and 5.5 / 11.4, 256 x 768 3.0 / 3.0 and 5.6 / 8.1; gate / up of 256 x 1280 3.5 / 4.2 and 5.6 / 12.2, of 256 x 768 3.5 / 3.1 and
-    // 7.4 / 8.8. Against 64 bits a row is 2.7e-8 off there, 1.0e-7 here (normally distributed rows, SiLU rows, cubes). The routed form stays here at any k (its rows are as short); from 16 combos on nvfp4_rows_tc.cu takes what it can of it (moe.cu).
-    // A rule of the matrix alone: a row's result does not depend on how many rows the call has.
-    const bool odd_steps = k % 512 != 0 && (k >= 1280 || (k >= 768 && rows >= 64 && !a.w1));
-    if (!routed && (k >= 2048 || odd_steps || (k >= 512 && rows >= 8192 && !a.w1) || (long long)rows * k * (a.w1 ? 2 : 1) >= 6000000)) {
+    if (!routed && f32_digits(rows, k, a.w1 != nullptr)) {
         if (k > 108544) CN_FAIL(CN_ERR_LIMIT,  // (the library's limit for f32 rows, as it was; this kernel has none)
                                  "%s: k = %d, f32 rows have up to 108544 values", who, k);
         return cn_gemv_tc_launch(a, stream, who);

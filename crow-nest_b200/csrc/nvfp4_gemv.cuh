@@ -111,6 +111,8 @@ __device__ __forceinline__ float act_gu(float g, float u, float limit) {
 
 
 // bf16 activation rows (1..8): persistent CTAs, tensor-core inner loop in word form (nvfp4_gemv_m1.cu)
+// whether bf16 rows of a matrix go to nvfp4_gemv_tc.cu from there
+bool cn_gemv_bf16_digits(int rows, int k, bool gu);
 int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who);
 
 // bf16 or f32 activation rows (1..8) of a plain or gate / up call: tcgen05, block scale (nvfp4_gemv_tc.cu)

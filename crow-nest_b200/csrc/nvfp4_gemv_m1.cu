@@ -761,6 +761,27 @@ Split one_row_split(int ntiles, int bpr, int tx) {
     return r;
 }
 
+// Larger matrices go to the fifth-generation tensor cores, whatever the number of rows (a rule of the matrix alone: a row's bits are those of a one-row
+// call), where that is no slower for any. us a call in a stream of dependent ones, here / there, for one, two, four and eight rows. Long rows: 4096 x 4096 4.7 / 4.2, 4.9 / 4.5, 5.6 / 5.6, 8.2 / 8.2;
+// 2048 x 4096 4.2 / 3.5, 4.2 / 3.7, 4.7 / 3.9, 6.7 / 5.4; 1500 x 5120 4.2 / 3.8, 4.5 / 3.8, 5.3 / 4.6, 8.3 / 6.5; 512 x 8192 4.0 / 3.8, 4.2 / 3.9, 5.2 / 4.6, 7.6 / 6.6; below these sizes its longer way
+// from the activations to the first product shows with one row: 1792 x 4096 3.0 / 3.4, 4.1 / 3.6, 4.6 / 3.8, 6.7 / 5.3; 1300 x 5120 3.6 / 3.7, 4.4 / 3.8, 5.2 / 4.3, 8.2 / 5.8; 2048 x 2048 2.8 / 3.4, 3.2 / 3.4, 3.5 / 3.5,
+// 4.7 / 4.7. With shorter rows the kernel here has parts of K to share only late, until the tiles of 128 rows there, a pair of CTAs each, fill the 148 SMs: 9728 x 2048 5.0 / 4.6, 5.5 / 4.9, 6.7 / 6.1, 10.2 /
+// 8.7; 9728 x 3584 7.1 / 6.0, 7.9 / 6.5, 9.2 / 8.7, 13.9 / 13.1; but 9216 x 3072 5.8 / 5.1, 6.6 / 5.7, 7.3 / 8.1, 10.4 / 11.1 and 5632 x 2048 3.5 / 4.1, 4.3 / 4.2, 5.0 / 4.5, 7.4 / 6.1. Few chunks want fewer tiles, four to
+// six of them 64: 8192 x 1536 4.3 / 3.8, 5.0 / 3.9, 5.7 / 4.8, 7.4 / 7.3; 8192 x 1024 3.5 / 3.4, 3.9 / 3.6, 4.5 / 4.0, 6.3 / 6.0; but 7168 x 1536 4.1 / 4.6, 4.8 / 4.7, 5.6 / 5.1, 7.3 / 6.7 and 7168 x 1024 3.3 / 4.2, 3.7 /
+// 4.2, 4.5 / 4.4, 6.2 / 5.2. Up to three, which no cluster shares, 40: 5120 x 768 2.9 / 2.8, 3.5 / 2.9, 4.2 / 3.3, 5.3 / 4.6; 5120 x 512 2.8 / 2.5, 3.0 / 2.6, 3.6 / 2.8, 4.8 / 3.7; 5120 x 256 2.5 / 2.4, 3.0 / 2.3, 3.4 / 2.4,
+// 4.5 / 3.0; but 3840 x 768 2.9 / 2.8, 2.8 / 2.9, 3.2 / 3.3, 4.0 / 4.4 and 2560 x 256 2.1 / 2.2, 2.3 / 2.3, 2.6 / 2.3, 3.6 / 2.9; or those that fill half of the SMs where gate and up meet in one tile: 5120 x 768 3.7 / 3.5, 5.0 / 3.7, 5.7 / 4.5, 8.8 / 6.4;
+// 5120 x 256 3.3 / 3.0, 4.3 / 2.9, 5.1 / 3.2, 7.9 / 4.5; but 4096 x 768 3.2 / 3.5, 4.0 / 3.6, 4.9 / 4.3, 7.2 / 5.8 and 4096 x 256 2.8 / 2.9, 3.5 / 2.9, 4.2 / 3.2, 6.4 / 4.5. Few long rows stay, too: its clusters end at eight CTAs a tile of 128 rows
+// (640 x 17408 6.4 / 5.9, 512 x 16384 6.0 / 5.0
+// there / here). A row that does not fit here is refused as it was, and so are lines of rows shorter than 2048 values, below.
+bool takes_digits(int rows, int k, bool gu, Split one) {
+    const long long all_rows = (long long)rows * (gu ? 2 : 1), weights = all_rows * k, tiles128 = (all_rows + 127) / 128;
+    const bool long_rows = k >= 4096 && weights >= (k >= 8192 ? 4100000 : k >= 5120 ? 7000000 : 8000000) && !(all_rows <= 1280 && k > 14336);
+    const bool many_tiles = tiles128 >= (k <= 768 ? (gu ? 74 : 40) : k <= 1536 ? 64 : 74);
+    if (!long_rows && !many_tiles) return false;
+    const int tx = k >= 2048 ? 32 : 16, bp = k / 64 / one.parts;
+    return front_bytes(2, (bp + tx - 1) / tx, 1, 1, bp, 0) + 2 * stage_bytes_of(tx) <= sm_share(one.cps);
+}
+
 }  // namespace
 
 #ifdef CN_M1_TRACE
@@ -770,6 +791,11 @@ static int g_m1_trace_n = 0, g_m1_trace_i = 0;
 extern "C" void cn_m1_trace(unsigned long long* buf, int launches) { g_m1_trace = buf, g_m1_trace_n = launches, g_m1_trace_i = 0; }
 unsigned long long* cn_trace_slot() { return g_m1_trace && g_m1_trace_i < g_m1_trace_n ? g_m1_trace + (size_t)(g_m1_trace_i++) * 512 * 8 : nullptr; }
 #endif
+
+bool cn_gemv_bf16_digits(int rows, int k, bool gu) {
+    const int per_cta = gu ? ROWS / 2 : ROWS;
+    return takes_digits(rows, k, gu, one_row_split((rows + per_cta - 1) / per_cta, k / 64, k >= 2048 ? 32 : 16));
+}
 
 int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int rows = a.rows, k = a.k, m = a.m;
@@ -786,25 +812,7 @@ int cn_gemv_m1_launch(const GemvCall& a, cudaStream_t stream, const char* who) {
     const int combos = a.combos + (routed ? a.side_tokens : 0);
     Split one = {1, 0};
     if (!routed) one = one_row_split(ntiles, bpr, tx);
-    // Larger matrices go to the fifth-generation tensor cores, whatever the number of rows (a rule of the matrix alone: a row's bits are those of a one-row
-    // call), where that is no slower for any. us a call in a stream of dependent ones, here / there, for one, two, four and eight rows. Long rows: 4096 x 4096 4.7 / 4.2, 4.9 / 4.5, 5.6 / 5.6, 8.2 / 8.2;
-    // 2048 x 4096 4.2 / 3.5, 4.2 / 3.7, 4.7 / 3.9, 6.7 / 5.4; 1500 x 5120 4.2 / 3.8, 4.5 / 3.8, 5.3 / 4.6, 8.3 / 6.5; 512 x 8192 4.0 / 3.8, 4.2 / 3.9, 5.2 / 4.6, 7.6 / 6.6; below these sizes its longer way
-    // from the activations to the first product shows with one row: 1792 x 4096 3.0 / 3.4, 4.1 / 3.6, 4.6 / 3.8, 6.7 / 5.3; 1300 x 5120 3.6 / 3.7, 4.4 / 3.8, 5.2 / 4.3, 8.2 / 5.8; 2048 x 2048 2.8 / 3.4, 3.2 / 3.4, 3.5 / 3.5,
-    // 4.7 / 4.7. With shorter rows the kernel here has parts of K to share only late, until the tiles of 128 rows there, a pair of CTAs each, fill the 148 SMs: 9728 x 2048 5.0 / 4.6, 5.5 / 4.9, 6.7 / 6.1, 10.2 /
-    // 8.7; 9728 x 3584 7.1 / 6.0, 7.9 / 6.5, 9.2 / 8.7, 13.9 / 13.1; but 9216 x 3072 5.8 / 5.1, 6.6 / 5.7, 7.3 / 8.1, 10.4 / 11.1 and 5632 x 2048 3.5 / 4.1, 4.3 / 4.2, 5.0 / 4.5, 7.4 / 6.1. Few chunks want fewer tiles, four to
-    // six of them 64: 8192 x 1536 4.3 / 3.8, 5.0 / 3.9, 5.7 / 4.8, 7.4 / 7.3; 8192 x 1024 3.5 / 3.4, 3.9 / 3.6, 4.5 / 4.0, 6.3 / 6.0; but 7168 x 1536 4.1 / 4.6, 4.8 / 4.7, 5.6 / 5.1, 7.3 / 6.7 and 7168 x 1024 3.3 / 4.2, 3.7 /
-    // 4.2, 4.5 / 4.4, 6.2 / 5.2. Up to three, which no cluster shares, 40: 5120 x 768 2.9 / 2.8, 3.5 / 2.9, 4.2 / 3.3, 5.3 / 4.6; 5120 x 512 2.8 / 2.5, 3.0 / 2.6, 3.6 / 2.8, 4.8 / 3.7; 5120 x 256 2.5 / 2.4, 3.0 / 2.3, 3.4 / 2.4,
-    // 4.5 / 3.0; but 3840 x 768 2.9 / 2.8, 2.8 / 2.9, 3.2 / 3.3, 4.0 / 4.4 and 2560 x 256 2.1 / 2.2, 2.3 / 2.3, 2.6 / 2.3, 3.6 / 2.9; or those that fill half of the SMs where gate and up meet in one tile: 5120 x 768 3.7 / 3.5, 5.0 / 3.7, 5.7 / 4.5, 8.8 / 6.4;
-    // 5120 x 256 3.3 / 3.0, 4.3 / 2.9, 5.1 / 3.2, 7.9 / 4.5; but 4096 x 768 3.2 / 3.5, 4.0 / 3.6, 4.9 / 4.3, 7.2 / 5.8 and 4096 x 256 2.8 / 2.9, 3.5 / 2.9, 4.2 / 3.2, 6.4 / 4.5. Few long rows stay, too: its clusters end at eight CTAs a tile of 128 rows
-    // (640 x 17408 6.4 / 5.9, 512 x 16384 6.0 / 5.0
-    // there / here). A row that does not fit here is refused as it was, and so are lines of rows shorter than 2048 values, below.
-    const long long all_rows = (long long)rows * (gu ? 2 : 1), weights = all_rows * k, tiles128 = (all_rows + 127) / 128;
-    const bool long_rows = k >= 4096 && weights >= (k >= 8192 ? 4100000 : k >= 5120 ? 7000000 : 8000000) && !(all_rows <= 1280 && k > 14336);
-    const bool many_tiles = tiles128 >= (k <= 768 ? (gu ? 74 : 40) : k <= 1536 ? 64 : 74);
-    if (!routed && (long_rows || many_tiles) && !(a.line_bases && tx != 32)) {
-        const int bp = bpr / one.parts;
-        if (front_bytes(2, (bp + tx - 1) / tx, 1, 1, bp, 0) + 2 * stage_bytes <= sm_share(one.cps)) return cn_gemv_tc_launch(a, stream, who);
-    }
+    if (!routed && !(a.line_bases && tx != 32) && takes_digits(rows, k, gu, one)) return cn_gemv_tc_launch(a, stream, who);
     const int parts = one.parts, bpp = bpr / parts;  // parts of K (each longer than a chunk where there are several), blocks of one
     // chunks from one part's end to the next where a CTA has n of them: a row is cut into whole chunks from its first part's start
     auto gap = [&](int n) { return n > 1 ? bpp / tx : (bpp + tx - 1) / tx; };

@@ -72,6 +72,9 @@ int cn_smem_book(const void* kernel, int device, int bytes, int commit);
  * the matrix alone - rows, values of a row, gate / up or plain - whatever the device and the number of activation rows. Makes no CUDA call; exported so that it
  * can be checked without a GPU. */
 int cn_nvfp4_gemv_cut(int rows, int k, int gate_up);
+/* Bits below the largest of 16 values to which the GEMV keeps activations of `dtype` for a matrix (see cn_nvfp4_gemv): 31 or 22 in fixed point, 0 where it keeps them whole. Whatever
+ * the device and the number of activation rows. Makes no CUDA call. */
+int cn_nvfp4_gemv_fixed_bits(int rows, int k, int gate_up, int dtype);
 
 /* ---------------------------------------------------------------- NVFP4 GEMV, M = 1..8
  * y[m][r] = sum_k W[r][k] * x[m][k], m < M.
@@ -82,8 +85,11 @@ int cn_nvfp4_gemv_cut(int rows, int k, int gate_up);
  * x row m at x + m*k elements, y row m at y + m*ldy elements (ldy >= rows). gs: device pointer to
  * the f32 tensor scale. Row m of a call with M rows is bit-identical to a call with M = 1 on that
  * row (the batch invariance of engine/src/kernels_p2.rs:391-396).
- * What is kept of an activation where the tensor cores multiply it in fixed point (larger matrices; also routed experts in groups): of every 16 values, f32 ones to 2^-31 and bf16
- * ones to 2^-22 of the largest, unless one half of the sixteen has none that reaches 2^-8 of it and the other fewer than three; then all of them whole. Smaller matrices: f32 ones whole, bf16 ones as f16 planes. */
+ * What is kept of an activation is a rule of the matrix (cn_nvfp4_gemv_fixed_bits). 0: f32 values whole, bf16 ones as f16 values x a power of two for every 64. Else the rows go to the
+ * tensor cores in fixed point of that many bits: a value is off by 2^-31 (f32) or 2^-22 (bf16) of the largest of its block of 16 at most, a result by the sum over the blocks of that
+ * much times the sum of the block's |weights|. Values are whole where a half of the sixteen has none that reaches 2^-8 of the largest and the other half fewer than three, and, in any block, from 2^-7 (f32) or 2^-14
+ * (bf16) of the largest on. Of a block's smaller values, where three and more of the others outweigh them by that and meet zero weights, low bits are lost, or all of them. Rows of routed experts go the same
+ * way where they run in groups, and to down projections from 16 combos on. */
 int cn_nvfp4_gemv(const void* w, const float* gs, const void* x, void* y, int rows, int k, int m, int ldy, int dtype,
                   cn_stream_t stream);
 

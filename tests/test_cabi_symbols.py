@@ -46,6 +46,20 @@ def test_shared_memory_attribute_is_booked_per_kernel_and_device():
     assert L.cn_smem_book(k1, 1, 100 * 1024, 1) == 0
 
 
+def test_where_activations_are_held_in_fixed_point():
+    """A rule of the matrix and the type alone: both sides of each of its lines (rows, k, gate / up)."""
+    from crownest_b200 import CN_BF16, CN_F32
+    bits = _lib.lib().cn_nvfp4_gemv_fixed_bits
+    # bf16: 40 tiles of 128 rows up to three chunks of 256 values (74 with gate / up), 64 up to six, 74 beyond; long rows from a size on; few long rows never
+    for yes, no in [((4993, 256, 0), (4992, 256, 0)), ((4993, 512, 0), (4992, 512, 0)), ((4993, 768, 0), (4992, 768, 0)), ((4673, 256, 1), (4672, 256, 1)), ((4673, 768, 1), (4672, 768, 1)),
+                    ((8065, 1024, 0), (8064, 1024, 0)), ((8065, 1536, 0), (8064, 1536, 0)), ((9345, 1792, 0), (9344, 1792, 0)), ((4033, 1024, 1), (4032, 1024, 1)), ((1954, 4096, 0), (1953, 4096, 0)),
+                    ((1368, 5120, 0), (1367, 5120, 0)), ((501, 8192, 0), (500, 8192, 0)), ((1281, 17408, 0), (1280, 17408, 0))]:
+        assert bits(*yes, CN_BF16) == 22 and bits(*no, CN_BF16) == 0, (yes, no)
+    for yes, no in [((1, 2048, 0), (1, 1024, 0)), ((1, 1280, 1), (1, 1024, 1)), ((64, 768, 0), (63, 768, 0)), ((64, 1792, 0), (64, 768, 1)), ((8192, 512, 0), (8191, 512, 0)), ((5860, 512, 1), (5859, 512, 1))]:
+        assert bits(*yes, CN_F32) == 31 and bits(*no, CN_F32) == 0, (yes, no)
+    assert bits(0, 4096, 0, CN_F32) == bits(4096, 100, 0, CN_F32) == bits(4096, 4096, 0, 2) == 0
+
+
 def test_the_cut_of_a_row_needs_no_device():
     """Into how many parts a row is cut fixes the order of its sum: a rule of the matrix alone, the same on every GPU and on none."""
     cut = _lib.lib().cn_nvfp4_gemv_cut

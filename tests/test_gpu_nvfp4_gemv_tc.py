@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from crownest_b200 import device_status, ops, synth
+from crownest_b200 import CN_BF16, CN_F32, device_status, lib, ops, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -98,6 +98,38 @@ def test_f32_rows_against_64_bits_and_one_row_calls(rows, k, gu, m):
 @pytest.mark.parametrize("m", [1, 3, 8])
 def test_f32_rows_of_short_matrices(rows, k, gu, m):
     test_f32_rows_against_64_bits_and_one_row_calls(rows, k, gu, m)
+
+
+# the smallest matrices in fixed point of either type, and neighbours that hold values whole
+@pytest.mark.parametrize("rows,k,dtype", [(1500, 5120, torch.bfloat16), (4993, 256, torch.bfloat16), (8192, 1024, torch.bfloat16), (9728, 2048, torch.bfloat16), (4992, 256, torch.bfloat16),
+                                          (256, 1280, torch.float32), (8192, 512, torch.float32), (64, 768, torch.float32), (16, 1792, torch.float32), (256, 1024, torch.float32)])
+@pytest.mark.parametrize("large", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("size", [1e3, 1e4, 1e7])
+def test_large_values_over_zero_weights(rows, k, dtype, large, size):
+    """`large` values of every sixteen are `size` times the others and meet zero weights, so that the others alone make the result: it is off by the last bit kept of the largest value at most, block by
+    block, and by nothing where values are held whole, or one or two alone outweigh the rest."""
+    rng, w, _ = _make(rows, k, rows + k)
+    codes = w.w.view(-1, 36)[:, 4:].view(-1, 4, 8)  # sixteen values in eight bytes
+    codes[:, :, :large // 2] = 0
+    if large % 2:
+        codes[:, :, large // 2] &= 0xF0
+    w64 = ops.dequant(w, rule=True).double().view(rows, k)
+    blocks = w64.view(rows, k // 16, 16)
+    assert not blocks[:, :, :large].any()
+    x = torch.from_numpy(rng.standard_normal((3, k)).astype(np.float32)).cuda()
+    x.view(3, k // 16, 16)[:, :, :large] *= size
+    x = x.to(dtype)
+    want, y = x.double() @ w64.t(), ops.launch_gemv(w, x)
+    bits = lib().cn_nvfp4_gemv_fixed_bits(rows, k, 0, CN_BF16 if dtype == torch.bfloat16 else CN_F32)
+    top = x.double().abs().view(3, k // 16, 16)
+    held = 2.0 ** -bits * (top.amax(dim=2) @ blocks.abs().sum(dim=2).t()) if bits else 0.0
+    # f32 sums of some thousand products, each addition off by 2^-24 of a part of the sum of their sizes (they add up as their root); a bf16 result by 2^-9 of itself more
+    sums = 2e-6 * (x.double().abs() @ w64.abs().t()) + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()
+    assert ((y.double() - want).abs() <= held + sums).all()
+    if large <= 2 and size >= 1e4:  # (below, or where a half's largest is near the others, a block keeps its digits; 2^-8 of the largest decides)
+        near = 2.0 ** -24 * (top.amax(dim=2) @ blocks.abs().sum(dim=2).t()) / size
+        assert ((y.double() - want).abs() <= near + sums).double().mean() >= 0.9
+    assert device_status() == 0
 
 
 def test_f32_rows_of_any_magnitude():

@@ -72,6 +72,58 @@ def test_either_side_of_the_grouping_line_against_64_bits(hidden, inter, topk, t
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("large", [3, 8])
+@pytest.mark.parametrize("size", [1e4, 1e7])
+def test_large_values_over_zero_weights_of_grouped_rows(large, size, dtype):
+    """As for the GEMV: `large` values of every sixteen are `size` times the others and meet zero weights of gate and up, in steps of 16 (f32) and 24 combos of large experts. What fixed point
+    loses of a block, 2^-31 (bf16: 2^-22) of its largest value, goes through the activation and the down projection, whose rows are held the same way."""
+    hidden, inter, experts, topk = 4096, 2048, 8, 8
+    tokens = 2 if dtype == torch.float32 else 3
+    rng = np.random.default_rng(large)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(large)
+
+    def matrix(rows, k, zeros):
+        m = torch.randint(0, 256, (rows * k // 64, 36), dtype=torch.uint8, device="cuda", generator=gen)
+        m[:, :4] = (torch.randn((rows * k // 64, 4), device="cuda", generator=gen).abs_() * 0.05).to(torch.float8_e4m3fn).view(torch.uint8)
+        codes = m[:, 4:].view(-1, 4, 8)
+        codes[:, :, :zeros // 2] = 0
+        if zeros % 2:
+            codes[:, :, zeros // 2] &= 0xF0
+        return m.view(-1)
+
+    gu, dn = [matrix(2 * inter, hidden, large) for _ in range(experts)], [matrix(hidden, inter, 0) for _ in range(experts)]
+    w = moe.GpuMoeWeights(hidden, inter, experts, 0.03, 0.7, gate_up=gu, down=dn, device="cuda")
+    plan = moe.GpuMoePlan(hidden, inter, experts, topk, tokens)
+    x = torch.from_numpy(rng.standard_normal((tokens, hidden)).astype(np.float32)).cuda()
+    x.view(tokens, hidden // 16, 16)[:, :, :large] *= size
+    x = x.to(dtype)
+    ids = torch.stack([torch.randperm(experts, device="cuda", generator=gen) for _ in range(tokens)]).int()
+    eo = plan.experts_only(w, ids, x, eo=torch.zeros((tokens * topk, hidden), device="cuda"), x_div=topk).double().view(tokens, topk, hidden)
+
+    def deq(m, rows, k, gs):
+        return ops.dequant(ops.Fp4(m, torch.tensor([gs], dtype=torch.float32, device="cuda"), rows, k), rule=True).double().view(rows, k)
+
+    def product(v, m, bits):
+        """v times a matrix, and how far off a row in fixed point may be: the last bit of each block's largest value, and f32 sums."""
+        blocks = lambda t: t.abs().view(t.shape[0], -1, 16)
+        return v @ m.t(), 2.0 ** -bits * (blocks(v).amax(dim=2) @ blocks(m).sum(dim=2).t()) + 2e-6 * (v.abs() @ m.abs().t())
+
+    x64, bits = x.double(), 31 if dtype == torch.float32 else 22
+    for e in range(experts):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        full, down = deq(gu[e], 2 * inter, hidden, 0.03), deq(dn[e], hidden, inter, 0.7)
+        a, da = product(x64[t], full[:inter], bits)
+        b, db = product(x64[t], full[inter:], bits)
+        s = a / (1 + torch.exp(-a))
+        h = s * b
+        dh = 1.1 * da * (b.abs() + db) + s.abs() * db + 1e-6 * h.abs()  # the slope of SiLU is 1.1 at most
+        y, dy = product(h, down, 31)
+        assert ((eo[t, j] - y).abs() <= dy + (1 + 1e-6) * (dh @ down.abs().t())).all()
+    assert device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [56, 64, 125])
 def test_full_groups_repeat_bit_for_bit(tokens, dtype):
     """Every expert has all tokens: groups of eight rows (and of seven or five at the end), one chunk right behind the other. The accumulators of two chunks in flight lie side by side in
