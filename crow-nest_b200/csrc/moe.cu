@@ -72,32 +72,26 @@ __global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int32_t* __rest
     }
 }
 
-// Sort the combos by expert and cut every expert's run into groups of up to gmax rows, gmax 4 or 8 (one CTA of 1024 threads):
-//   order[]           the combos sorted by expert, stable; combos without a resident expert (id outside 0..E-1, or a
-//                     null entry of `tab`) last, in any order, and in no group
-//   ga[] / counts[0]  positions (in order[]) of the one-row groups: an expert's single row, or the one left over after
-//                     its groups of gmax
-//   gb[], gbrows[] / counts[1]  first positions and row counts (2..gmax) of the other groups
-// Placement: every combo counts the earlier ones among its expert's (the list in shared memory, in the order of the counting atomics), which keeps the sort
-// stable; where an expert has more than LONG_RUN rows, or the list does not fit (listed = 0), one warp walks the combos in order instead (match.any finds the lanes of a
-// step that share an expert; 20 dependent steps for 640 combos). A step of 64 tokens, top 10 of 512 experts: 203.0 -> 199.9 us, replayed 199.5 -> 198.8.
-constexpr int LONG_RUN = 64;
 __device__ __forceinline__ bool resident(int e, const unsigned long long* __restrict__ tab, int E) { return e >= 0 && e < E && !(tab && tab[e] == 0ull); }
-// Records of the chunks of activations, by warp `w` of `warps`. Rows none of whose combos has a resident expert are left out, since nothing reads them and most inbox slots of an
-// expert-parallel rank are such rows: one rank of eight, 512 experts of 2048 x 512, top 10, 64 tokens a rank (620 of 5120 slots in use), routed experts 88.0 -> 76.5 us. A lane looks one of the
-// warp's chunks up, the ids and then the entries of four combos at a time. The first chunk of a warp is made without a look: up to a chunk for every warp they are made beside
-// the grouping on SMs that have nothing else to do, and two more trips to memory in front of them show (160 slots 23.0 -> 23.3 us).
-// (a function of its own: inlined into the loop of put_records the kernel has 56 registers, not 40, and a block of it an SM to itself; seven tokens of 128 experts of 2560 x 768, top 6, 43.1 us, 42.7 so)
+
 template <bool F32>
-__device__ __noinline__ void one_record(const char* x, int lane, uint8_t* rec) {
+__device__ __forceinline__ void one_chunk(const DigitsCall& dc, size_t i, int lane) {
     ChunkValues<F32> v;
-    v.load(x, lane);
-    put_record<F32>(v, lane, rec);
+    v.load((const char*)dc.x + i * (256 * (F32 ? 4 : 2)), lane);
+    put_record<F32>(v, lane, dc.out + i * digit_record(F32));
+}
+// Records of the chunks of activations, more than there are warps. Rows none of whose combos has a resident expert are left out, since nothing reads them and most inbox slots of an
+// expert-parallel rank are such rows: one rank of eight, 512 experts of 2048 x 512, top 10, 64 tokens a rank (637 of 5120 slots in use), routed experts 91.9 -> 80.1 us. A lane looks one of the
+// warp's chunks up, the ids and then the entries of four combos at a time. The first chunk of a warp is made without a look, as are all where every warp has one at most: they are made beside
+// the grouping on SMs that have nothing else to do, and two more trips to memory in front of them show (160 slots 23.0 -> 23.3 us).
+// A chunk is a call here (inlined into the loop the kernel has 56 registers, not 40, and a block of it an SM to itself: seven tokens of 128 experts of 2560 x 768, top 6, 43.0 -> 43.5 us), and inline code where a
+// warp has one.
+template <bool F32>
+__device__ __noinline__ void far_chunk(const DigitsCall& dc, size_t i, int lane) {
+    one_chunk<F32>(dc, i, lane);
 }
 template <bool F32>
 __device__ __forceinline__ void put_records(const DigitsCall& dc, const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E, int w, int warps, int lane) {
-    const char* x = (const char*)dc.x;
-    constexpr size_t BYTES = 256 * (F32 ? 4 : 2);
     for (int i0 = w; i0 < dc.chunks; i0 += 32 * warps) {
         const int at = i0 + lane * warps;
         bool read = at == w;
@@ -113,12 +107,20 @@ __device__ __forceinline__ void put_records(const DigitsCall& dc, const int32_t*
             }
         }
 #pragma unroll 1
-        for (uint32_t todo = __ballot_sync(0xffffffffu, read); todo; todo &= todo - 1u) {
-            const size_t i = (size_t)(i0 + (__ffs(todo) - 1) * warps);
-            one_record<F32>(x + i * BYTES, lane, dc.out + i * digit_record(F32));
-        }
+        for (uint32_t todo = __ballot_sync(0xffffffffu, read); todo; todo &= todo - 1u) far_chunk<F32>(dc, (size_t)(i0 + (__ffs(todo) - 1) * warps), lane);
     }
 }
+
+// Sort the combos by expert and cut every expert's run into groups of up to gmax rows, gmax 4 or 8 (one CTA of 1024 threads):
+//   order[]           the combos sorted by expert, stable; combos without a resident expert (id outside 0..E-1, or a
+//                     null entry of `tab`) last, in any order, and in no group
+//   ga[] / counts[0]  positions (in order[]) of the one-row groups: an expert's single row, or the one left over after
+//                     its groups of gmax
+//   gb[], gbrows[] / counts[1]  first positions and row counts (2..gmax) of the other groups
+// Placement: every combo counts the earlier ones among its expert's (the list in shared memory, in the order of the counting atomics), which keeps the sort
+// stable; where an expert has more than LONG_RUN rows, or the list does not fit (listed = 0), one warp walks the combos in order instead (match.any finds the lanes of a
+// step that share an expert; 20 dependent steps for 640 combos). A step of 64 tokens, top 10 of 512 experts: 203.0 -> 199.9 us, replayed 199.5 -> 198.8.
+constexpr int LONG_RUN = 64;
 __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restrict__ ids, const unsigned long long* __restrict__ tab, int n, int E,
                                                          int32_t* __restrict__ order, int* __restrict__ ga, int* __restrict__ gb,
                                                          int* __restrict__ gbrows, int* __restrict__ counts, int gmax, int listed, const DigitsCall dc) {
@@ -136,10 +138,17 @@ __global__ void __launch_bounds__(1024) moe_group_kernel(const int32_t* __restri
     pdl_wait();
     if (blockIdx.x > 0) {  // not the grouping
         const int w = ((int)blockIdx.x - 1) * 32 + wid, warps = ((int)gridDim.x - 1) * 32;
-        if (dc.f32)
-            put_records<true>(dc, ids, tab, n, E, w, warps, lane);
-        else
-            put_records<false>(dc, ids, tab, n, E, w, warps, lane);
+        if (dc.chunks > warps) {
+            if (dc.f32)
+                put_records<true>(dc, ids, tab, n, E, w, warps, lane);
+            else
+                put_records<false>(dc, ids, tab, n, E, w, warps, lane);
+        } else if (w < dc.chunks) {
+            if (dc.f32)
+                one_chunk<true>(dc, w, lane);
+            else
+                one_chunk<false>(dc, w, lane);
+        }
         return;
     }
     for (int i = tid; i <= E; i += blockDim.x) cnt[i] = 0;
@@ -492,9 +501,9 @@ int routed_experts(MoePlan* p, const unsigned long long* table_gu, const unsigne
         d.count1 = counts, d.pos1 = ga, d.count2 = counts + 1, d.pos2 = gb, d.rows2 = gbrows;
         const bool f32 = dtype == CN_F32;
         const long long x_chunks = (long long)((combos + x_div - 1) / x_div) * (p->hidden / 256);
-        // The digits of x are made once, beside the grouping, and not by every tile of gate / up: us per step, in each tile / so: 64 tokens 169 / 167, 128 tokens 247 / 234, 64 tokens of f32
-        // 187 / 179, 288 experts of 4096 x 2048, 32 tokens 369 / 339, 10 tokens 180 / 176, 64 experts of 1024 x 1280, 108 tokens 140 / 129; 16 and 24 tokens of 512 experts the same. Those of h,
-        // a launch of their own in front of the down projection: 64 tokens 167 / 175, 108 tokens 129 / 122, 128 tokens 234 / 232.
+        // The digits of x are made once, beside the grouping, and not by every tile of gate / up: us per step without a shared expert, a graph of twelve with other picks, in each tile / so: 64 tokens 153 / 148,
+        // 128 tokens 221 / 203, 64 tokens of f32 165 / 158, 288 experts of 4096 x 2048, 32 tokens 517 / 495, 10 tokens 198 / 197, 64 experts of 1024 x 1280, 108 tokens 137 / 126, 16 tokens of 512 experts 67.3 / 67.7; one rank
+        // of eight with 64 tokens 91.8 / 79.8. Those of h, a launch of their own in front of the down projection: 64 tokens 167 / 175, 108 tokens 129 / 122, 128 tokens 234 / 232.
         DigitsCall dx = {};
         if (!((uintptr_t)x & 15) && x_chunks * digit_record(f32) <= (long long)p->xd_bytes) {
             dx.x = x, dx.chunks = (int)x_chunks, dx.row_chunks = p->hidden / 256, dx.x_div = x_div, dx.f32 = f32, dx.out = p->xd;
